@@ -61,7 +61,10 @@ struct DevBuf {
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
-psb_status check_device(int device, cudaDeviceProp* prop_out = nullptr) {
+// Runs at every operator call.  The full property block (cudaGetDeviceProperties) takes milliseconds on some hosts - 10 of the
+// 18 ms of a psb_pq_encode call on 1M rows went there - so two attributes are asked once per device and the SM count is remembered.
+psb_status check_device(int device, int* sm_count = nullptr) {
+    static std::atomic<int> known_sms[64];
     int n = 0;
     cudaError_t e = cudaGetDeviceCount(&n);
     if (e != cudaSuccess || n <= 0) {
@@ -69,35 +72,15 @@ psb_status check_device(int device, cudaDeviceProp* prop_out = nullptr) {
         return fail(PSB_NO_DEVICE, "no CUDA device is usable; this library has no CPU path");
     }
     if (device < 0 || device >= n) return fail(PSB_INVALID_ARGUMENT, "device ordinal out of range");
-    cudaDeviceProp prop;
-    PSB_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10) return fail(PSB_NO_DEVICE, "device is not sm_100 (kernels are built for sm_100a only)");
-    if (prop_out) *prop_out = prop;
-    PSB_CUDA(cudaSetDevice(device));
-    return PSB_OK;
-}
-
-// The same check for operators called once per batch: attribute queries (microseconds) instead of the full property
-// block (milliseconds), and the SM count remembered per device.
-psb_status check_device_quick(int device, int* sm_count) {
-    static int known_sms[64] = {0};
-    int n = 0;
-    cudaError_t e = cudaGetDeviceCount(&n);
-    if (e != cudaSuccess || n <= 0) {
-        cudaGetLastError();
-        return fail(PSB_NO_DEVICE, "no CUDA device is usable; this library has no CPU path");
-    }
-    if (device < 0 || device >= n) return fail(PSB_INVALID_ARGUMENT, "device ordinal out of range");
-    if (device >= 64 || known_sms[device] == 0) {
-        int major = 0, sms = 0;
+    int sms = device < 64 ? known_sms[device].load(std::memory_order_relaxed) : 0;
+    if (sms == 0) {
+        int major = 0;
         PSB_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
         PSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         if (major != 10) return fail(PSB_NO_DEVICE, "device is not sm_100 (kernels are built for sm_100a only)");
-        if (device < 64) known_sms[device] = sms;
-        if (sm_count) *sm_count = sms;
-    } else if (sm_count) {
-        *sm_count = known_sms[device];
+        if (device < 64) known_sms[device].store(sms, std::memory_order_relaxed);
     }
+    if (sm_count) *sm_count = sms;
     PSB_CUDA(cudaSetDevice(device));
     return PSB_OK;
 }
@@ -771,8 +754,8 @@ int psb_device_count(void) {
     if (cudaGetDeviceCount(&n) != cudaSuccess) { cudaGetLastError(); return 0; }
     int ok = 0;
     for (int i = 0; i < n; ++i) {
-        cudaDeviceProp p;
-        if (cudaGetDeviceProperties(&p, i) == cudaSuccess && p.major == 10) ++ok;
+        int major = 0;
+        if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, i) == cudaSuccess && major == 10) ++ok;
     }
     return ok;
 }
@@ -813,11 +796,11 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
     if (opt.gather_ctas < 0 || opt.gather_ctas > 1024) return fail(PSB_INVALID_ARGUMENT, "gather_ctas must be in 0..1024");
     if (opt.adc_mode == 1 && !index->exact.fp32 && !index->exact.u8)
         return fail(PSB_INVALID_ARGUMENT, "residual mode always reranks: exact rows are required");
-    cudaDeviceProp prop;
-    PSB_TRY(check_device(opt.device, &prop));
+    int sms = 0;
+    PSB_TRY(check_device(opt.device, &sms));
     std::unique_ptr<psb_session> s(new (std::nothrow) psb_session());
     if (!s) return fail(PSB_OUT_OF_MEMORY, "host allocation failed");
-    s->device = opt.device; s->sm_count = prop.multiProcessorCount; s->opt = opt;
+    s->device = opt.device; s->sm_count = sms; s->opt = opt;
     s->nlist = nlist; s->dim = index->coarse.dim; s->m = index->pq.subvectors; s->k = index->pq.codebook_size;
     s->n_vectors = index->lists.n_vectors; s->list_begin = lb; s->list_end = le;
     s->row_base = index->lists.offsets[lb];
@@ -986,7 +969,7 @@ psb_status psb_sign_rotate(const float* d_rows, int64_t n, int dim, int padded_d
                            uint32_t* d_codes, float* d_norms, float* d_norm_sq, int device, void* stream) {
     if (!d_rows || n < 0 || (!d_rotated && !d_codes && !d_norms && !d_norm_sq)) return fail(PSB_INVALID_ARGUMENT, "invalid sign rotation request");
     int sms = 0;
-    PSB_TRY(check_device_quick(device, &sms));
+    PSB_TRY(check_device(device, &sms));
     return launch_sign_rotate(d_rows, n, dim, padded_dim, seed, d_rotated, d_codes, d_norms, d_norm_sq, sms,
                               static_cast<cudaStream_t>(stream));
 }
@@ -998,7 +981,7 @@ psb_status psb_sign_encode_database(const void* d_rows, int elem_bytes, int64_t 
         return fail(PSB_INVALID_ARGUMENT, "invalid sign database encoding request");
     if (elem_bytes != 1 && elem_bytes != 4) return fail(PSB_INVALID_ARGUMENT, "rows must be u8 (1) or fp32 (4)");
     int sms = 0;
-    PSB_TRY(check_device_quick(device, &sms));
+    PSB_TRY(check_device(device, &sms));
     return launch_sign_encode_database(d_rows, elem_bytes, n, d_centroids, reinterpret_cast<const long long*>(d_list_offsets), nlist,
                                        dim, padded_dim, seed, row_offset, d_codes, d_scales, sms,
                                        static_cast<cudaStream_t>(stream));
@@ -1010,7 +993,7 @@ psb_status psb_sign_encode_queries(const float* d_queries, const float* d_centro
     if (!d_queries || !d_centroids || !d_probes || nq < 0 || nprobe <= 0 || nlist <= 0 || (!d_states && !d_state_codes))
         return fail(PSB_INVALID_ARGUMENT, "invalid sign query encoding request");
     int sms = 0;
-    PSB_TRY(check_device_quick(device, &sms));
+    PSB_TRY(check_device(device, &sms));
     return launch_sign_encode_queries(d_queries, d_centroids, d_probes, nq, nprobe, nlist, dim, padded_dim, seed, d_states, d_norm_sq,
                                       d_state_codes, d_norms, sms, static_cast<cudaStream_t>(stream));
 }
@@ -1027,7 +1010,7 @@ psb_status psb_sign_search_candidates(int mode, const float* d_states, const flo
     if (!d_codes || !d_row_params || !d_list_offsets || !d_probes || !d_rows_out || nq < 0 || nprobe <= 0 || nlist <= 0)
         return fail(PSB_INVALID_ARGUMENT, "invalid sign candidate search request");
     int sms = 0;
-    PSB_TRY(check_device_quick(device, &sms));
+    PSB_TRY(check_device(device, &sms));
     return launch_sign_candidates(mode, d_states, d_norm_sq, d_state_codes, d_norms, d_codes, d_row_params,
                                   reinterpret_cast<const long long*>(d_list_offsets), nlist, d_probes, nq, nprobe, padded_dim,
                                   candidate_count, d_rows_out, d_dist_out, sms, static_cast<cudaStream_t>(stream));
@@ -1581,12 +1564,12 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
     psb_options opt{};
     if (options) opt = *options;
     if (opt.max_batch <= 0) opt.max_batch = 10000;
-    cudaDeviceProp prop;
-    PSB_TRY(check_device(opt.device, &prop));
+    int sms = 0;
+    PSB_TRY(check_device(opt.device, &sms));
     std::unique_ptr<psb_session> s(new (std::nothrow) psb_session());
     if (!s) return fail(PSB_OUT_OF_MEMORY, "host allocation failed");
     s->flat = true;
-    s->device = opt.device; s->sm_count = prop.multiProcessorCount; s->opt = opt;
+    s->device = opt.device; s->sm_count = sms; s->opt = opt;
     s->nlist = index->lists.nlist; s->dim = index->coarse.dim; s->n_vectors = index->lists.n_vectors;
     s->list_begin = 0; s->list_end = s->nlist; s->row_base = 0; s->shard_rows = s->n_vectors;
     if (opt.stream) s->stream = static_cast<cudaStream_t>(opt.stream);
@@ -1721,8 +1704,8 @@ psb_status psb_rerank_host(const psb_host_storage_view* storage, const uint8_t* 
             if (h_candidate_counts[q] < 0 || h_candidate_counts[q] > candidate_count)
                 return fail(PSB_INVALID_ARGUMENT, "host rerank candidate count exceeds row width");
     if (candidate_count > kMaxRerankWidth || topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "rerank width above 4096 or topk above 2048");
-    cudaDeviceProp prop;
-    PSB_TRY(check_device(device, &prop));
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
     const int elem = use_float ? 4 : 1;
     const int dim = storage->dim;
     const size_t base_bytes = (size_t)storage->count * dim * elem;
@@ -1746,7 +1729,7 @@ psb_status psb_rerank_host(const psb_host_storage_view* storage, const uint8_t* 
     DevBuf score;
     PSB_TRY(score.reserve(sizeof(float) * (size_t)batch_n * candidate_count));
     PSB_TRY(launch_gather_rows(base.p, mp, dim, elem, cand.as<int>(), batch_n, candidate_count, candidate_stride,
-                               d_counts, stage.p, st, prop.multiProcessorCount));
+                               d_counts, stage.p, st, sms));
     PSB_TRY(launch_rerank_score(stage.p, mp, dim, elem, q.p, cand.as<int>(), batch_n, candidate_count, candidate_stride,
                                 d_counts, score.as<float>(), st));
     PSB_TRY(launch_topk_select(score.as<float>(), cand.as<int>(), batch_n, candidate_count, candidate_stride, d_counts,
@@ -1761,7 +1744,8 @@ psb_status psb_coarse_host(const float* h_queries, int nq, const float* h_centro
     if (!h_queries || !h_centroids || !h_ids || nq < 0 || nlist <= 0 || dim <= 0) return fail(PSB_INVALID_ARGUMENT, "invalid coarse request");
     if (nprobe <= 0 || nprobe > nlist) return fail(PSB_INVALID_ARGUMENT, "nprobe must be in 1..nlist");
     if (nprobe > kMaxProbe) return fail(PSB_UNSUPPORTED_SHAPE, "nprobe above 4096 is not supported");
-    PSB_TRY(check_device(device));
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
     if (nq == 0) return PSB_OK;
     DevBuf q, c, tile, ids, ids64, dist;
     PSB_TRY(q.reserve(sizeof(float) * (size_t)nq * dim)); PSB_TRY(c.reserve(sizeof(float) * (size_t)nlist * dim));
@@ -1772,14 +1756,12 @@ psb_status psb_coarse_host(const float* h_queries, int nq, const float* h_centro
     const bool tc_ok = coarse_tc_supported(nq, nlist, dim, nprobe);
     if (coarse_mode == 2 && !tc_ok) return fail(PSB_UNSUPPORTED_SHAPE, "tensor-core coarse stage does not support this shape");
     if (coarse_mode != 1 && tc_ok) {
-        cudaDeviceProp prop;
-        PSB_CUDA(cudaGetDeviceProperties(&prop, device));
         TcIndexBuffers tix;
         TcWorkBuffers twk;
         PSB_TRY(tix.prepare(h_centroids, c.as<float>(), nlist, dim, nullptr));
         PSB_TRY(twk.ensure(nq, nlist, dim, nprobe, nullptr));
         PSB_TRY(launch_coarse_tc(tix.view(c.as<float>(), nlist, dim), twk.view(), q.as<float>(), nq, nprobe, ids.as<int>(),
-                                 dist.as<float>(), prop.multiProcessorCount, nullptr));
+                                 dist.as<float>(), sms, nullptr));
         PSB_CUDA(cudaDeviceSynchronize());
         PSB_TRY(twk.check_status());
     } else {
@@ -1844,8 +1826,8 @@ psb_status psb_knn_exact(const float* d_queries, int nq, const float* d_base, in
 psb_status psb_kmeans_train(const float* d_data, int64_t n, int dim, float* d_centroids, int k, int iters,
                             int* d_assign, double* h_objective, int device, void* stream) {
     if (!d_data || !d_centroids || n <= 0 || dim <= 0 || k <= 0 || iters < 0) return fail(PSB_INVALID_ARGUMENT, "invalid k-means request");
-    cudaDeviceProp prop;
-    PSB_TRY(check_device(device, &prop));
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     DevBuf tile, assign, best, sums, counts, obj;
     const size_t row_bytes = sizeof(float) * (size_t)k;
@@ -1887,10 +1869,10 @@ psb_status psb_kmeans_train(const float* d_data, int64_t n, int dim, float* d_ce
                 // centroid is now - and the filter GEMM runs once instead of twice.
                 if (it > 0)
                     PSB_TRY(launch_coarse_tc_assign(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, d_as + r0,
-                                                    d_as + r0, best.as<float>() + r0, prop.multiProcessorCount, st));
+                                                    d_as + r0, best.as<float>() + r0, sms, st));
                 else
                     PSB_TRY(launch_coarse_tc(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, 1,
-                                             d_as + r0, best.as<float>() + r0, prop.multiProcessorCount, st));
+                                             d_as + r0, best.as<float>() + r0, sms, st));
             } else {
                 PSB_TRY(tile.reserve(row_bytes * (size_t)nn));
                 PSB_TRY(launch_coarse_dist_exact(d_data + (size_t)r0 * dim, nn, d_centroids, k, dim, tile.as<float>(), st));
@@ -1919,8 +1901,8 @@ psb_status psb_kmeans_assign_bounded(const float* d_data, int64_t n, int dim, co
                                      float* d_best, int have_previous, int device, void* stream) {
     if (!d_data || !d_centroids || !d_assign || !d_best || n <= 0 || dim <= 0 || k <= 0)
         return fail(PSB_INVALID_ARGUMENT, "invalid k-means assignment request");
-    cudaDeviceProp prop;
-    PSB_TRY(check_device(device, &prop));
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t row_bytes = sizeof(float) * (size_t)k;
     long long chunk = std::min<long long>((long long)std::max<size_t>(64, ((size_t)1 << 30) / row_bytes), n);
@@ -1942,10 +1924,10 @@ psb_status psb_kmeans_assign_bounded(const float* d_data, int64_t n, int dim, co
             PSB_TRY(tcw.ensure(nn, k, dim, 1, st));
             if (have_previous)
                 PSB_TRY(launch_coarse_tc_assign(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, d_assign + r0,
-                                                d_assign + r0, d_best + r0, prop.multiProcessorCount, st));
+                                                d_assign + r0, d_best + r0, sms, st));
             else
                 PSB_TRY(launch_coarse_tc(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, 1, d_assign + r0,
-                                         d_best + r0, prop.multiProcessorCount, st));
+                                         d_best + r0, sms, st));
         } else {
             PSB_TRY(tile.reserve(row_bytes * (size_t)nn));
             PSB_TRY(launch_coarse_dist_exact(d_data + (size_t)r0 * dim, nn, d_centroids, k, dim, tile.as<float>(), st));
