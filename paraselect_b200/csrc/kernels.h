@@ -280,12 +280,15 @@ psb_status launch_pq_encode(const float* d_data, long long n, int dim, const flo
                             uint8_t* d_codes, cudaStream_t s);
 psb_status launch_pq_accumulate(const float* d_data, long long n, int dim, const uint8_t* d_codes, int m, int k,
                                 double* d_sums, int* d_counts, cudaStream_t s);
-psb_status launch_pq_update(const double* d_sums, const int* d_counts, int m, int k, int dsub, float* d_codebook,
-                            cudaStream_t s);
+// Codewords = sums / counts (no rows: kept); leaves the sums and counts zeroed.
+psb_status launch_pq_update(double* d_sums, int* d_counts, int m, int k, int dsub, float* d_codebook, cudaStream_t s);
 // Initial codewords taken from given data rows: d_rows [m][k] (row of the data for codeword c of subspace sub).
 psb_status launch_pq_init_rows(const float* d_data, int dim, int m, int k, const long long* d_rows, float* d_codebook, cudaStream_t s);
-psb_status launch_pq_init(const float* d_data, long long n, int dim, int m, int k, uint64_t seed,
-                          float* d_codebook, cudaStream_t s);
+// k-means++ rows of every subspace: d_draws [m][k - 1] uniform in [0, 1), d_first [m] first rows; d_rows [m][k] out, d_status [m]
+// (zeroed by the caller) = 1 where a sum of distances is not a positive finite number and the host has to pick.
+bool pq_seed_fits(long long n);
+psb_status launch_pq_seed(const float* d_data, int n, int dim, int m, int k, const double* d_draws, const int* d_first, long long* d_rows,
+                          int* d_status, cudaStream_t s);
 // Workspace of the k-means accumulation: rows grouped by centroid (order [n], offsets [k + 1], cursor [k], all int32).
 struct KmeansAccumWs { int* order = nullptr; int* offsets = nullptr; int* cursor = nullptr; };
 // d_counts [k] and *d_obj zeroed by the caller; d_sums [k][dim] is written whole (zeros for a centroid without rows).

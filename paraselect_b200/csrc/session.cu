@@ -19,6 +19,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 namespace psb {
@@ -84,6 +85,53 @@ psb_status check_device(int device, int* sm_count = nullptr) {
     PSB_CUDA(cudaSetDevice(device));
     return PSB_OK;
 }
+
+// Work memory of the operators that allocate, run and free within one call (training, one-shot searches): from a memory pool of
+// the library per device, stream-ordered, so that a call pays neither cudaMalloc nor the device synchronisation of cudaFree (about
+// a third of a small training call).  The pool keeps at most kPoolKeep bytes between calls; what is above goes back to the device at
+// the next synchronisation.
+constexpr unsigned long long kPoolKeep = 1ull << 30;
+psb_status work_pool(int device, cudaMemPool_t* out) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    if (device < 0 || device >= 64) return fail(PSB_UNSUPPORTED_SHAPE, "device ordinal above 63");
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pools[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t p = nullptr;
+        PSB_CUDA(cudaMemPoolCreate(&p, &props));
+        unsigned long long keep = kPoolKeep;
+        PSB_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+        pools[device] = p;
+    }
+    *out = pools[device];
+    return PSB_OK;
+}
+
+// Stream-ordered buffer from the pool; freed on the same stream, so work queued there before may still use it.
+struct PoolBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+    cudaStream_t st = nullptr;
+    PoolBuf() = default;
+    PoolBuf(const PoolBuf&) = delete;
+    PoolBuf& operator=(const PoolBuf&) = delete;
+    ~PoolBuf() { release(); }
+    void release() { if (p) cudaFreeAsync(p, st); p = nullptr; bytes = 0; }
+    psb_status reserve(size_t need, int device, cudaStream_t stream) {
+        if (p && need <= bytes) return PSB_OK;
+        release();
+        cudaMemPool_t pool;
+        PSB_TRY(work_pool(device, &pool));
+        PSB_CUDA(cudaMallocFromPoolAsync(&p, need ? need : 1, pool, stream));
+        bytes = need; st = stream;
+        return PSB_OK;
+    }
+    template <typename T> T* as() const { return static_cast<T*>(p); }
+};
 
 // Persistent fork-join pool of host threads for the staged rerank transport (the reference keeps a persistent rerank pool
 // too: src/search/ivf_common/ivf_host_rerank.cpp:42-51).  run(job) calls job(t) on every thread t and returns when all are done.
@@ -1991,13 +2039,16 @@ void kmeans_init_rows(long long n, int dim, int k, int seed, int policy, RowFn r
     std::mt19937 rng((unsigned)seed);
     const bool plusplus = policy == 2 || (policy == 0 && (long long)ni * k_eff <= 20000000LL);
     if (!plusplus) {
-        std::vector<int> idx((size_t)ni);
-        for (int i = 0; i < ni; ++i) idx[(size_t)i] = i;
+        // the identity permutation is kept implicit: only the places the shuffle has touched are stored
+        std::unordered_map<int, int> moved;
+        auto at = [&](int i) { const auto it = moved.find(i); return it == moved.end() ? i : it->second; };
         for (int i = 0; i < k_eff; ++i) {
             std::uniform_int_distribution<int> dist(i, ni - 1);
-            std::swap(idx[(size_t)i], idx[(size_t)dist(rng)]);
+            const int j = dist(rng), x = at(i), y = at(j);
+            moved[j] = x;
+            moved[i] = y;
         }
-        for (int c = 0; c < k; ++c) picked[(size_t)c] = idx[(size_t)(c < k_eff ? c : 0)];
+        for (int c = 0; c < k; ++c) picked[(size_t)c] = at(c < k_eff ? c : 0);
         return;
     }
     auto dist2 = [&](const float* x, const float* c) {
@@ -2057,43 +2108,70 @@ psb_status psb_pq_train(const float* d_data, int64_t n, int dim, int subvectors,
         codebook_size > kMaxCodebook || iters < 0)
         return fail(PSB_INVALID_ARGUMENT, "invalid PQ training request");
     PSB_TRY(check_device(device));
+    if (n > INT_MAX) return fail(PSB_UNSUPPORTED_SHAPE, "PQ training on more than 2^31-1 rows");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int dsub = dim / subvectors;
-    DevBuf codes, sums, counts;
-    PSB_TRY(codes.reserve((size_t)n * subvectors));
-    PSB_TRY(sums.reserve(sizeof(double) * (size_t)subvectors * codebook_size * dsub));
-    PSB_TRY(counts.reserve(sizeof(int) * (size_t)subvectors * codebook_size));
+    const int dsub = dim / subvectors, words = subvectors * codebook_size;
+    // One block: codes, sums, counts (with the seeding's status words behind them), rows, draws, first rows.
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t b_codes = up((size_t)n * subvectors), b_sums = up(sizeof(double) * (size_t)words * dsub),
+                 b_counts = up(sizeof(int) * ((size_t)words + subvectors)), b_rows = up(sizeof(long long) * (size_t)words),
+                 b_draws = up(sizeof(double) * (size_t)words), b_first = up(sizeof(int) * (size_t)subvectors);
+    PoolBuf block;
+    PSB_TRY(block.reserve(b_codes + b_sums + b_counts + b_rows + b_draws + b_first, device, st));
+    uint8_t* codes = block.as<uint8_t>();
+    double* sums = reinterpret_cast<double*>(codes + b_codes);
+    int* counts = reinterpret_cast<int*>(codes + b_codes + b_sums);
+    int* status = counts + words;
+    long long* d_rows = reinterpret_cast<long long*>(codes + b_codes + b_sums + b_counts);
+    double* d_draws = reinterpret_cast<double*>(codes + b_codes + b_sums + b_counts + b_rows);
+    int* d_first = reinterpret_cast<int*>(codes + b_codes + b_sums + b_counts + b_rows + b_draws);
+    PSB_CUDA(cudaMemsetAsync(sums, 0, b_sums + b_counts, st));
     // Initial codewords as the reference's GPU trainer picks them (src/quantization/pq/pq_trainer.cu:30-95): subspace `sub`
     // runs the k-means initialisation with seed + sub * 104729 on its own sub-vectors.  The random-rows policy needs no data;
-    // the k-means++ policy (small training sets only: n * K <= 2e7) works on a host copy of the subspace.
-    if (n > INT_MAX) return fail(PSB_UNSUPPORTED_SHAPE, "PQ training on more than 2^31-1 rows");
-    {
-        std::vector<long long> rows((size_t)subvectors * codebook_size), picked;
-        const bool plusplus = (long long)n * std::min<long long>(codebook_size, n) <= 20000000LL;
-        std::vector<float> sub_host;
-        if (plusplus) sub_host.resize((size_t)n * dsub);
+    // the k-means++ policy (small training sets only: n * K <= 2e7) runs on the device with the draws made here.
+    const bool plusplus = (long long)n * std::min<long long>(codebook_size, n) <= 20000000LL;
+    const bool on_device = plusplus && pq_seed_fits(n);
+    auto sub_seed = [&](int sub) { return (int)((unsigned)seed + (unsigned)sub * 104729u); };
+    std::vector<long long> rows((size_t)words), picked;
+    std::vector<double> draws;
+    std::vector<int> first, to_host((size_t)subvectors, plusplus ? 1 : 0);
+    if (on_device) {
+        draws.assign((size_t)words, 0.0);
+        first.resize((size_t)subvectors);
+        const int keff = (int)std::min<long long>(codebook_size, n);
         for (int sub = 0; sub < subvectors; ++sub) {
-            const int sub_seed = (int)((unsigned)seed + (unsigned)sub * 104729u);
+            std::mt19937 rng((unsigned)sub_seed(sub));
+            first[(size_t)sub] = std::uniform_int_distribution<int>(0, (int)n - 1)(rng);
+            for (int c = 1; c < keff; ++c)
+                draws[(size_t)sub * (codebook_size - 1) + (c - 1)] = std::generate_canonical<double, std::numeric_limits<double>::digits>(rng);
+        }
+        PSB_CUDA(cudaMemcpyAsync(d_draws, draws.data(), sizeof(double) * draws.size(), cudaMemcpyHostToDevice, st));
+        PSB_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, st));
+        PSB_TRY(launch_pq_seed(d_data, (int)n, dim, subvectors, codebook_size, d_draws, d_first, d_rows, status, st));
+        PSB_CUDA(cudaMemcpyAsync(to_host.data(), status, sizeof(int) * to_host.size(), cudaMemcpyDeviceToHost, st));
+        PSB_CUDA(cudaStreamSynchronize(st));
+    }
+    {
+        std::vector<float> sub_host;
+        for (int sub = 0; sub < subvectors; ++sub) {
+            if (on_device && !to_host[(size_t)sub]) continue;
             if (plusplus) {
+                sub_host.resize((size_t)n * dsub);
                 PSB_CUDA(cudaMemcpy2DAsync(sub_host.data(), sizeof(float) * (size_t)dsub, d_data + (size_t)sub * dsub, sizeof(float) * (size_t)dim,
                                            sizeof(float) * (size_t)dsub, (size_t)n, cudaMemcpyDeviceToHost, st));
                 PSB_CUDA(cudaStreamSynchronize(st));
             }
-            kmeans_init_rows(n, dsub, codebook_size, sub_seed, 0, [&](long long i) { return sub_host.data() + (size_t)i * dsub; }, picked);
+            kmeans_init_rows(n, dsub, codebook_size, sub_seed(sub), 0, [&](long long i) { return sub_host.data() + (size_t)i * dsub; }, picked);
             std::copy(picked.begin(), picked.end(), rows.begin() + (size_t)sub * codebook_size);
+            PSB_CUDA(cudaMemcpyAsync(d_rows + (size_t)sub * codebook_size, rows.data() + (size_t)sub * codebook_size, sizeof(long long) * (size_t)codebook_size,
+                                     cudaMemcpyHostToDevice, st));
         }
-        DevBuf d_rows;
-        PSB_TRY(d_rows.reserve(sizeof(long long) * rows.size()));
-        PSB_CUDA(cudaMemcpyAsync(d_rows.p, rows.data(), sizeof(long long) * rows.size(), cudaMemcpyHostToDevice, st));
-        PSB_TRY(launch_pq_init_rows(d_data, dim, subvectors, codebook_size, d_rows.as<long long>(), d_codebook, st));
-        PSB_CUDA(cudaStreamSynchronize(st));   // rows and d_rows go out of scope
     }
+    PSB_TRY(launch_pq_init_rows(d_data, dim, subvectors, codebook_size, d_rows, d_codebook, st));
     for (int it = 0; it < iters; ++it) {
-        PSB_TRY(launch_pq_encode(d_data, n, dim, d_codebook, subvectors, codebook_size, codes.as<uint8_t>(), st));
-        PSB_CUDA(cudaMemsetAsync(sums.p, 0, sums.bytes, st));
-        PSB_CUDA(cudaMemsetAsync(counts.p, 0, counts.bytes, st));
-        PSB_TRY(launch_pq_accumulate(d_data, n, dim, codes.as<uint8_t>(), subvectors, codebook_size, sums.as<double>(), counts.as<int>(), st));
-        PSB_TRY(launch_pq_update(sums.as<double>(), counts.as<int>(), subvectors, codebook_size, dsub, d_codebook, st));
+        PSB_TRY(launch_pq_encode(d_data, n, dim, d_codebook, subvectors, codebook_size, codes, st));
+        PSB_TRY(launch_pq_accumulate(d_data, n, dim, codes, subvectors, codebook_size, sums, counts, st));
+        PSB_TRY(launch_pq_update(sums, counts, subvectors, codebook_size, dsub, d_codebook, st));
     }
     PSB_CUDA(cudaStreamSynchronize(st));
     return PSB_OK;
