@@ -4,11 +4,13 @@
 //   pass 1  epilogue keeps, per query and per group of G consecutive centroids, the minimum approximate distance
 //           a = |c'|^2 - 2 q'.c'  (q', c' = inputs minus the mean centroid, rounded to bf16).  The nprobe-th smallest
 //           group minimum T is an upper bound of the nprobe-th smallest approximate distance.
-//   pass 2  epilogue appends every centroid with a <= T + 2E to the query's candidate list, E >= |a - exact| being
-//           the bf16 rounding bound 4.1 * 2^-8 * |q'| * max|c'| (plus fp32 slack).  Every centroid of the exact top-nprobe
-//           is then a candidate: the nprobe approximately-nearest have exact distance <= T + E, so the exact
-//           nprobe-th distance is <= T + E and its members have a <= T + 2E.
-// k_coarse_refine re-scores the candidates (typically 1.2-2 x nprobe) in the CPU path's arithmetic (sequential
+//   pass 2  epilogue appends every centroid with a <= T + 2E to the query's candidate list, E >= |a - exact|.
+//           Every centroid of the exact top-nprobe is then a candidate: the nprobe approximately-nearest have exact
+//           distance <= T + E, so the exact nprobe-th distance is <= T + E and its members have a <= T + 2E.
+// E comes from the rounding that happened, not from the format's worst case: with qb, cb the bf16 operands,
+//     |q'.c' - qb.cb| <= |q' - qb| |c'| + |qb| |c' - cb|,   E = 2 (|q' - qb| max|c'| + |qb| max|c' - cb|) plus fp32 slack,
+// four to five times below 2^-7 |q'| max|c'|.
+// k_coarse_refine re-scores the candidates (typically 1.1-1.3 x nprobe) in the CPU path's arithmetic (sequential
 // non-fused fp32, reference src/cpu/utils/cpu_distance.h:74-81) and sorts by (distance, id): results are bit-identical
 // to the exact kernels in coarse.cu.  A query whose list overflowed is redone by k_coarse_exact_query.
 //
@@ -54,7 +56,22 @@ __device__ __forceinline__ void group_mins(const float (&v)[32], float* __restri
     }
 }
 
+__device__ __forceinline__ float max32(const float (&v)[32]) {   // three-input maxima, two chains
+    float m0 = v[0], m1 = v[1];
+#pragma unroll
+    for (int j = 2; j < 32; j += 4) {
+        asm("max.f32 %0, %0, %1, %2;" : "+f"(m0) : "f"(v[j]), "f"(v[j + 1]));
+        if (j + 3 < 32) asm("max.f32 %0, %0, %1, %2;" : "+f"(m1) : "f"(v[j + 2]), "f"(v[j + 3]));
+    }
+    return fmaxf(m0, m1);
+}
+__device__ __forceinline__ void add_f32x2(float& o0, float& o1, float a0, float a1, float b0, float b1) {
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(o0), "=f"(o1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+
 struct TcArgs {
+    const int* nq_dev;      // when set: the number of rows is min(*nq_dev, nq), known on the device only
     int nq, nlist, katoms;  // katoms = padded dim / 64
     int ntiles;             // centroid tiles of TCOL
     int group;              // G: centroids per minimum in pass 1 (power of two <= 32)
@@ -62,8 +79,8 @@ struct TcArgs {
     int ngroups;            // minima per query row = ntiles * (TCOL / G)
     int nprobe;
     const float* cn2;       // [ntiles * TCOL] |c'|^2, +inf beyond nlist
-    const float* qnorm;     // [nq] |q'|
-    float cmax;             // max |c'|
+    const float2* qnorm;    // [nq] |q'| and |q' - qb|
+    const float* cmax;      // [2] max |c'| and max |c' - cb|
     float* gmin;            // pass 1 out: [nq][ngroups]
     const float* seltop;    // pass 2 in: [nq][nprobe] ascending group minima (T = last)
     uint32_t* mask;         // pass 2 out: [nq][mwords] one bit per centroid (zeroed before the launch; only non-zero words are written)
@@ -73,6 +90,7 @@ struct TcArgs {
     int* cand_cnt;          // pass 2, list form (nearest-centroid assignment with a known bound): [nq] candidates found so far
     int* cand_list;         //   [nq][cand_cap] their ids; null: the bit mask above is written instead
     int cand_cap;
+    float band;             // pass 2: cut = T + band * E; 2, or 1 when T bounds the exact distance itself (a previous assignment)
     int wait_limit;         // polls before a wait gives up (0: kWaitLimit)
     int skip_loads;         // test hook of the time-out path: the producer issues no load at all, so nothing is in flight when
                             // the other roles give up
@@ -87,7 +105,7 @@ __device__ __forceinline__ void cta_range(const TcArgs& a, long long& l0, long l
     l1 = total * (blockIdx.x + 1) / gridDim.x;
 }
 __device__ __forceinline__ int seg_count(const TcArgs& a, long long l0, long long l1) {
-    return l1 > l0 ? (int)((l1 - 1) / a.qtiles - l0 / a.qtiles) + 1 : 0;
+    return l1 > l0 && a.qtiles > 0 ? (int)((l1 - 1) / a.qtiles - l0 / a.qtiles) + 1 : 0;
 }
 __device__ __forceinline__ void seg_get(const TcArgs& a, long long l0, long long l1, int i, int& cblock, int& t0, int& t1) {
     cblock = (int)(l0 / a.qtiles) + i;
@@ -116,7 +134,9 @@ constexpr int kBlockCols = 2 * TCOL;  // centroids per work unit
 // centroid side), so the accumulator already holds w = q'.c' - |c'|^2 / 2 and the epilogue needs no norm arithmetic.
 template <bool kSecondPass, bool kAug>
 __global__ void __launch_bounds__(kTcThreadsV2, 1)
-k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_c, const TcArgs a) {
+k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_c, const TcArgs args) {
+    TcArgs a = args;
+    if (a.nq_dev) { a.nq = min(*a.nq_dev, a.nq); a.qtiles = (a.nq + TQ - 1) / TQ; }
     extern __shared__ __align__(1024) unsigned char s_tc[];
     unsigned char* s_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_tc) + 1023) & ~uintptr_t(1023));
     const size_t a_bytes = (size_t)a.katoms * TQ * 128, b_bytes = (size_t)a.katoms * TCOL * 128;
@@ -203,16 +223,17 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
             int cblock, t0, t1;
             seg_get(a, l0, l1, u, cblock, t0, t1);
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");  // previous unit's readers of s_cn2 are done
-            for (int i = tid; i < kBlockCols; i += kEpiThreads) s_cn2[i] = a.cn2[(size_t)cblock * kBlockCols + i];
+            for (int i = tid; i < kBlockCols; i += kEpiThreads) s_cn2[i] = -0.5f * a.cn2[(size_t)cblock * kBlockCols + i];
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
             for (int t = t0; t < t1 && !failed; ++t) {
                 const int q = t * TQ + row;
                 float cut = 0.0f;
                 if (kSecondPass && q < a.nq) {
                     const float T = a.seltop[(size_t)q * a.nprobe + a.nprobe - 1];
-                    const float qn = a.qnorm[q];
-                    const float E = 4.1f * 0.00390625f * qn * a.cmax;  // |a - exact| <= 2 |q'.c' - qb.cb| <= 2 * 2.01 * 2^-8 |q'||c'|
-                    cut = -0.5f * (T + 2.0f * E + 4e-5f * (qn + a.cmax) * (qn + a.cmax));  // candidates: w >= cut
+                    const float2 qn = a.qnorm[q];
+                    const float cm = a.cmax[0], ce = a.cmax[1];
+                    const float E = 2.0001f * (qn.y * cm + (qn.x + qn.y) * ce);
+                    cut = -0.5f * (T + a.band * E + 6e-5f * (qn.x + cm) * (qn.x + cm));  // candidates: w >= cut
                 }
                 const bool partial = (cblock + 1) * kBlockCols > a.nlist;  // block reaches past the last centroid
                 for (int h = 0; h < 2; ++h) {
@@ -244,12 +265,10 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
                                 }
                             } else {
 #pragma unroll
-                                for (int j = 0; j < 32; j += 4) {
+                                for (int j = 0; j < 32; j += 4) {   // s_cn2 holds -|c'|^2 / 2
                                     const float4 n4 = *reinterpret_cast<const float4*>(&s_cn2[h * TCOL + cb + j]);
-                                    v[j] = fmaf(-0.5f, n4.x, __uint_as_float(rr[j]));
-                                    v[j + 1] = fmaf(-0.5f, n4.y, __uint_as_float(rr[j + 1]));
-                                    v[j + 2] = fmaf(-0.5f, n4.z, __uint_as_float(rr[j + 2]));
-                                    v[j + 3] = fmaf(-0.5f, n4.w, __uint_as_float(rr[j + 3]));
+                                    add_f32x2(v[j], v[j + 1], __uint_as_float(rr[j]), __uint_as_float(rr[j + 1]), n4.x, n4.y);
+                                    add_f32x2(v[j + 2], v[j + 3], __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 3]), n4.z, n4.w);
                                 }
                             }
                             if (!kSecondPass) {
@@ -263,11 +282,12 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
                                     default: group_mins<1>(v, out); break;
                                 }
                             } else {
-                                // one bit per centroid of this 32-column chunk; most chunks hold none and write nothing
-                                uint32_t bits = 0;
+                                // one bit per centroid of this 32-column chunk; most chunks hold none, which their maximum tells in a
+                                // quarter of the instructions the bits take
+                                if (max32(v) >= cut) {
+                                    uint32_t bits = 0;
 #pragma unroll
-                                for (int j = 0; j < 32; ++j) bits |= (v[j] >= cut ? 1u : 0u) << j;
-                                if (bits) {
+                                    for (int j = 0; j < 32; ++j) bits |= (v[j] >= cut ? 1u : 0u) << j;
                                     if (a.cand_list) {   // a handful of candidates per row: a short list instead of a mask to scan
                                         while (bits) {
                                             const int j = __ffs((int)bits) - 1;
@@ -293,35 +313,59 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     if (warp == 0) tmem_dealloc(tmem, 2 * TCOL);
 }
 
-// q' = q - mu as bf16 rows padded with zeros to dimp, and |q'|.
+// q' = q - mu as bf16 rows padded with zeros to dimp, |q'|^2 (sq), |q'| with the rounding error |q' - qb| (norm), and the largest of
+// each over all rows (maxima [2], zeroed by the caller).
 // aug: 0 = no extra slots, 1 = query rows (slots dim..dim+2 hold 1), 2 = centroid rows (slots hold minus the bf16
 // three-term split of |c'|^2 / 2).
-__global__ void k_tc_prep_rows(const float* __restrict__ x, int n, int dim, int dimp, const float* __restrict__ mu,
-                               __nv_bfloat16* __restrict__ out, float* __restrict__ norm, float* __restrict__ sq, int aug) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    float s = 0.0f;
+__global__ void k_tc_prep_rows(const float* __restrict__ x, long long n, int dim, int dimp, const float* __restrict__ mu,
+                               __nv_bfloat16* __restrict__ out, float2* __restrict__ norm, float* __restrict__ sq, float* __restrict__ maxima, int aug) {
+    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (row >= n) return;
+    float s = 0.0f, e = 0.0f;
     for (int d = lane; d < dimp; d += 32) {
         float v = 0.0f;
-        if (d < dim) v = x[(size_t)warp * dim + d] - mu[d];
-        if (!(aug && d >= dim && d < dim + 3)) out[(size_t)warp * dimp + d] = __float2bfloat16_rn(v);
+        if (d < dim) v = x[(size_t)row * dim + d] - mu[d];
+        const __nv_bfloat16 h = __float2bfloat16_rn(v);
+        if (!(aug && d >= dim && d < dim + 3)) out[(size_t)row * dimp + d] = h;
+        const float r = v - __bfloat162float(h);
         s += v * v;
+        e += r * r;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    for (int o = 16; o > 0; o >>= 1) { s += __shfl_xor_sync(0xffffffffu, s, o); e += __shfl_xor_sync(0xffffffffu, e, o); }
     if (lane == 0) {
-        if (norm) norm[warp] = sqrtf(s);
-        if (sq) sq[warp] = s;
+        const float nrm = sqrtf(s), err = sqrtf(e) * 1.0001f;
+        if (norm) norm[row] = make_float2(nrm, err);
+        if (sq) sq[row] = s;
+        if (maxima) {   // non-negative floats order like their bits
+            atomicMax(reinterpret_cast<int*>(maxima), __float_as_int(nrm * 1.0001f));
+            atomicMax(reinterpret_cast<int*>(maxima) + 1, __float_as_int(err));
+        }
         if (aug == 1) {
-            for (int i = 0; i < 3; ++i) out[(size_t)warp * dimp + dim + i] = __float2bfloat16_rn(1.0f);
+            for (int i = 0; i < 3; ++i) out[(size_t)row * dimp + dim + i] = __float2bfloat16_rn(1.0f);
         } else if (aug == 2) {
             float rest = 0.5f * s;
             for (int i = 0; i < 3; ++i) {
                 const __nv_bfloat16 h = __float2bfloat16_rn(rest);
-                out[(size_t)warp * dimp + dim + i] = __hneg(h);
+                out[(size_t)row * dimp + dim + i] = __hneg(h);
                 rest -= __bfloat162float(h);
             }
         }
+    }
+}
+
+// Mean of n rows, one CTA per 32 dimensions, a warp per 32nd row: the point the operands are centred on.
+__global__ void __launch_bounds__(1024) k_mean_row(const float* __restrict__ x, int n, int dim, float* __restrict__ mu) {
+    __shared__ double s_part[32][33];
+    const int d = blockIdx.x * 32 + (threadIdx.x & 31), w = threadIdx.x >> 5;
+    double acc = 0.0;
+    if (d < dim) for (int r = w; r < n; r += 32) acc += (double)x[(size_t)r * dim + d];
+    s_part[w][threadIdx.x & 31] = acc;
+    __syncthreads();
+    if (w == 0 && d < dim) {
+        for (int i = 1; i < 32; ++i) acc += s_part[i][threadIdx.x & 31];
+        mu[d] = (float)(acc / n);
     }
 }
 
@@ -330,53 +374,123 @@ __global__ void k_fill_inf(float* p, long long n) {
     if (i < n) p[i] = __int_as_float(0x7f800000);
 }
 
-// Per query row the k-th smallest of n <= 2048 values, written to out[q * out_stride + out_stride - 1].  One warp per row:
-// the values sit in registers as order-preserving integer keys and the answer is found by bisection on the key (32
-// counting rounds), which is exact.
-constexpr int kKthPerLane = 64;
+// Per query row a value that at least k of its n <= 2048 values do not exceed - the k-th smallest or a little more - written to
+// out[q * out_stride + out_stride - 1].  One warp per row, the values in registers; bisection between the row's extremes that ends
+// when exactly k values lie below or after kKthRounds rounds: the filter's cut may be a little high, never low, and a
+// 2^14th of the row's range is far below the band E that is added to it.  (An exact k-th smallest took 32 rounds.)
+constexpr int kKthPerLane = 64, kKthRounds = 14;
 __global__ void __launch_bounds__(256)
 k_kth_smallest(const float* __restrict__ vals, int nq, int n, int k, float* __restrict__ out, int out_stride) {
     const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (q >= nq) return;
-    uint32_t key[kKthPerLane];
+    float v[kKthPerLane];
+    const float inf = __int_as_float(0x7f800000);
+    float mn = inf, mx = -inf;
 #pragma unroll
     for (int j = 0; j < kKthPerLane; ++j) {
         const int i = j * 32 + lane;
-        key[j] = i < n ? f2o(vals[(size_t)q * n + i]) : 0xffffffffu;
+        v[j] = i < n ? vals[(size_t)q * n + i] : inf;
+        mn = fminf(mn, v[j]);
+        if (v[j] < inf) mx = fmaxf(mx, v[j]);
     }
-    uint32_t lo = 0u, hi = 0xffffffffu;
-    while (lo < hi) {
-        const uint32_t mid = lo + ((hi - lo) >> 1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    float lo = mn, hi = mx;   // at most k values <= lo is not known yet; all finite values <= hi
+    for (int it = 0; it < kKthRounds; ++it) {
+        const float mid = lo + 0.5f * (hi - lo);
         int c = 0;
 #pragma unroll
-        for (int j = 0; j < kKthPerLane; ++j) c += key[j] <= mid ? 1 : 0;
+        for (int j = 0; j < kKthPerLane; ++j) c += v[j] <= mid ? 1 : 0;
         c = __reduce_add_sync(0xffffffffu, c);
-        if (c >= k) hi = mid; else lo = mid + 1;
+        if (c >= k) hi = mid; else lo = mid;
+        if (c == k) break;
     }
-    if (lane == 0) out[(size_t)q * out_stride + out_stride - 1] = o2f(lo);
+    // fewer than k finite values: no cut at all
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < kKthPerLane; ++j) c += v[j] <= hi ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) out[(size_t)q * out_stride + out_stride - 1] = c >= k ? hi : inf;
+}
+
+// k = 1: the row minimum of any number of values, one warp per row.
+__global__ void __launch_bounds__(256) k_row_min(const float* __restrict__ vals, long long nq, const int* __restrict__ nq_dev, int n, float* __restrict__ out) {
+    const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (q >= nq || (nq_dev && q >= *nq_dev)) return;
+    float mn = __int_as_float(0x7f800000);
+    for (int i = lane; i < n; i += 32) mn = fminf(mn, vals[(size_t)q * n + i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    if (lane == 0) out[q] = mn;
+}
+
+// Distance of a centroid row to a query in the CPU path's arithmetic (sequential, non-fused); both rows 16-byte aligned when vec.
+__device__ __forceinline__ float l2_sequential(const float* q, const float* c, int dim, bool vec) {
+    float sum = 0.0f;
+    if (vec) {
+        const float4* c4 = reinterpret_cast<const float4*>(c);
+        const float4* q4 = reinterpret_cast<const float4*>(q);
+#pragma unroll 8
+        for (int d = 0; d < dim / 4; ++d) {
+            const float4 x = c4[d];
+            const float4 y = q4[d];
+            float diff = __fsub_rn(y.x, x.x); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+            diff = __fsub_rn(y.y, x.y); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+            diff = __fsub_rn(y.z, x.z); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+            diff = __fsub_rn(y.w, x.w); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+        }
+    } else {
+        for (int d = 0; d < dim; ++d) {
+            const float diff = __fsub_rn(q[d], c[d]);
+            sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+        }
+    }
+    return sum;
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
 // Exact re-scoring of a query's candidates in the CPU path's arithmetic, sort by (distance, id), first nprobe out.
-constexpr int kRefineThreads = 256;
+// 128 threads per query.  The candidates' rows come through shared memory, kRefineTile at a time, loaded whole by warps; a thread
+// then walks its own row (a row per thread straight from L2 read each 32-byte sector four times over: 600 us for 20,000 queries
+// x 65,536 centroids x 96, top 64).
+constexpr int kRefineThreads = 128;
+constexpr int kRefineTile = 64;
+__host__ __device__ __forceinline__ int refine_pitch(int dim) { return (dim + 3) / 4 * 4 + 4; }   // rows spread over the banks
 __global__ void __launch_bounds__(kRefineThreads)
 k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ centroids, int dim, int nlist, int nprobe,
                 const uint32_t* __restrict__ mask, int mwords, int* __restrict__ out_ids,
                 float* __restrict__ out_dist, int* __restrict__ fail_list, int* __restrict__ n_fail) {
     extern __shared__ __align__(16) unsigned char s_ref[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_ref);                        // [kCandCap]
-    float* s_q = reinterpret_cast<float*>(s_ref + (size_t)kCandCap * 8);         // [dim]
-    int* s_cand = reinterpret_cast<int*>(s_ref + (size_t)kCandCap * 8 + (size_t)((dim + 3) & ~3) * 4);  // [kCandCap]
+    const int pitch = refine_pitch(dim);
+    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_ref);                        // [kCandCap]; the low words hold the ids first
+    float* s_q = reinterpret_cast<float*>(s_ref + (size_t)kCandCap * 8);         // [pitch]
+    float* s_row = s_q + pitch;                                                   // [kRefineTile][pitch]
     __shared__ int s_n;
-    const int q = blockIdx.x;
+    const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) s_n = 0;
+    for (int d = threadIdx.x; d < dim; d += kRefineThreads) s_q[d] = queries[(size_t)q * dim + d];
     __syncthreads();
-    for (int w = threadIdx.x; w < mwords; w += blockDim.x) {  // the candidate bits of this query -> list of centroid ids
-        uint32_t bits = mask[(size_t)q * mwords + w];
-        while (bits) {
-            const int j = __ffs((int)bits) - 1;
-            bits &= bits - 1;
-            const int pos = atomicAdd(&s_n, 1);
-            if (pos < kCandCap) s_cand[pos] = w * 32 + j;
+    const uint4* m4 = reinterpret_cast<const uint4*>(mask + (size_t)q * mwords);   // mwords is a multiple of 16
+#pragma unroll 4
+    for (int w = threadIdx.x; w < mwords / 4; w += kRefineThreads) {  // the candidate bits of this query -> list of centroid ids
+        const uint4 x = m4[w];
+        const unsigned long long bw[2] = {((unsigned long long)x.y << 32) | x.x, ((unsigned long long)x.w << 32) | x.z};
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            unsigned long long bits = bw[i];
+            while (bits) {
+                const int j = __ffsll((long long)bits) - 1;
+                bits &= bits - 1;
+                const int pos = atomicAdd(&s_n, 1);
+                if (pos < kCandCap) s_keys[pos] = (uint64_t)(w * 128 + i * 64 + j);
+            }
         }
     }
     __syncthreads();
@@ -388,39 +502,54 @@ k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ cen
         }
         return;
     }
-    for (int d = threadIdx.x; d < dim; d += blockDim.x) s_q[d] = queries[(size_t)q * dim + d];
-    __syncthreads();
-    const int np = next_pow2(max(n, 2));
-    for (int i = threadIdx.x; i < np; i += blockDim.x) {
-        uint64_t key = KEY_MAX;
-        if (i < n) {
-            const int c = s_cand[i];
-            const float* cp = centroids + (size_t)c * dim;
-            float sum = 0.0f;
-            if ((dim & 3) == 0) {  // 16-byte loads: a row's 32-byte sectors are fetched once or twice, not eight times
-                const float4* cp4 = reinterpret_cast<const float4*>(cp);
-                const float4* q4 = reinterpret_cast<const float4*>(s_q);
-                for (int d = 0; d < dim / 4; ++d) {
-                    const float4 x = __ldg(cp4 + d);
-                    const float4 y = q4[d];
-                    float diff = __fsub_rn(y.x, x.x); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                    diff = __fsub_rn(y.y, x.y); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                    diff = __fsub_rn(y.z, x.z); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                    diff = __fsub_rn(y.w, x.w); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                }
-            } else {
-                for (int d = 0; d < dim; ++d) {
-                    const float diff = __fsub_rn(s_q[d], __ldg(cp + d));
-                    sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                }
+    const bool vec = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(centroids) & 15) == 0;
+    for (int t0 = 0; t0 < n; t0 += kRefineTile) {
+        const int cnt = min(kRefineTile, n - t0);
+        if (vec) {
+            const int n4 = dim >> 2;
+            for (int i = warp; i < cnt; i += kRefineThreads / 32) {
+                const float4* src = reinterpret_cast<const float4*>(centroids + (size_t)(uint32_t)s_keys[t0 + i] * dim);
+                for (int d = lane; d < n4; d += 32) cp_async16(s_row + i * pitch + d * 4, src + d);   // all rows in flight at once
             }
-            key = make_key(sum, (uint32_t)c);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        } else {
+            for (int i = warp; i < cnt; i += kRefineThreads / 32) {
+                const float* src = centroids + (size_t)(uint32_t)s_keys[t0 + i] * dim;
+                for (int d = lane; d < dim; d += 32) s_row[i * pitch + d] = __ldg(src + d);
+            }
         }
-        s_keys[i] = key;
+        __syncthreads();
+        if (threadIdx.x < cnt) {
+            const uint32_t c = (uint32_t)s_keys[t0 + threadIdx.x];
+            s_keys[t0 + threadIdx.x] = make_key(l2_sequential(s_q, s_row + threadIdx.x * pitch, dim, vec), c);
+        }
+        __syncthreads();
     }
+    if (n <= 2 * kRefineThreads) {   // a key's place is the number of smaller ones: no barriers, a third of the sort's instructions
+        const uint64_t k0 = threadIdx.x < n ? s_keys[threadIdx.x] : KEY_MAX;
+        const uint64_t k1 = threadIdx.x + kRefineThreads < n ? s_keys[threadIdx.x + kRefineThreads] : KEY_MAX;
+        int rank0 = 0, rank1 = 0;
+        if (n > kRefineThreads) {
+            for (int j = 0; j < n; ++j) { const uint64_t o = s_keys[j]; rank0 += o < k0 ? 1 : 0; rank1 += o < k1 ? 1 : 0; }
+        } else if ((threadIdx.x & ~31) < n) {
+#pragma unroll 4
+            for (int j = 0; j < n; ++j) rank0 += s_keys[j] < k0 ? 1 : 0;
+        }
+        if (threadIdx.x < n && rank0 < nprobe) {
+            out_ids[(size_t)q * nprobe + rank0] = (int)key_idx(k0);
+            if (out_dist) out_dist[(size_t)q * nprobe + rank0] = key_dist(k0);
+        }
+        if (threadIdx.x + kRefineThreads < n && rank1 < nprobe) {
+            out_ids[(size_t)q * nprobe + rank1] = (int)key_idx(k1);
+            if (out_dist) out_dist[(size_t)q * nprobe + rank1] = key_dist(k1);
+        }
+        return;
+    }
+    const int np = next_pow2(n);
+    for (int i = n + threadIdx.x; i < np; i += kRefineThreads) s_keys[i] = KEY_MAX;
     __syncthreads();
     block_bitonic_sort(s_keys, np);
-    for (int i = threadIdx.x; i < nprobe; i += blockDim.x) {
+    for (int i = threadIdx.x; i < nprobe; i += kRefineThreads) {
         out_ids[(size_t)q * nprobe + i] = (int)key_idx(s_keys[i]);
         if (out_dist) out_dist[(size_t)q * nprobe + i] = key_dist(s_keys[i]);
     }
@@ -431,79 +560,151 @@ k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ cen
 // distance to the nearest centroid from above.  With that bound in place of pass 1's group minimum the GEMM runs once: the
 // candidates (every centroid whose bf16 estimate is within the bound plus the rounding slack - the nearest one and all its
 // ties among them) go to a short per-row list, and k_coarse_refine1 picks the exact nearest in the CPU path's arithmetic.
-constexpr int kAssignCap = 32;   // candidates kept per row (one per lane of the refining warp); more: the exact per-row kernel
-// seltop[row] = (bound on the squared distance) - |q'|^2, the quantity pass 2 compares a = |c'|^2 - 2 q'.c' against.
-__global__ void k_prev_bound(const float* __restrict__ rows, long long n, int dim, const float* __restrict__ centroids, int nlist,
-                             const int* __restrict__ prev, const float* __restrict__ qnorm, float* __restrict__ seltop) {
-    const long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (r >= n) return;
-    const int c = prev[r];
-    float acc = 0.0f;
-    const bool ok = c >= 0 && c < nlist;
-    if (ok) {
-        const float* x = rows + (size_t)r * dim;
-        const float* cp = centroids + (size_t)c * dim;
-        for (int d = lane; d < dim; d += 32) { const float diff = x[d] - __ldg(cp + d); acc = fmaf(diff, diff, acc); }
-    }
+constexpr int kAssignCap = 32;   // candidates kept per row; more: the exact per-row kernel
+// seltop[row] = (bound on the squared distance) - |q'|^2, the quantity pass 2 compares a = |c'|^2 - 2 q'.c' against.  A warp takes four
+// rows, so that their loads, each behind the row's previous id, are in flight together.
+__global__ void __launch_bounds__(256) k_prev_bound(const float* __restrict__ rows, int n, int dim, const float* __restrict__ centroids, int nlist,
+                                                    const int* __restrict__ prev, const float2* __restrict__ qnorm, float* __restrict__ seltop) {
+    const int r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 4, lane = threadIdx.x & 31;
+    if (r0 >= n) return;
+    const bool vec = (dim & 3) == 0 && ((reinterpret_cast<uintptr_t>(centroids) | reinterpret_cast<uintptr_t>(rows)) & 15) == 0;
+    int mine = -1;
+    float qn = 0.0f;
+    if (lane < 4 && r0 + lane < n) { mine = prev[r0 + lane]; qn = qnorm[r0 + lane].x; if (mine < 0 || mine >= nlist) mine = -1; }
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    int c[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-        const float qn = qnorm[r];
-        // a bound, not a result: one part in 1e5 covers the different summation order
-        seltop[r] = ok ? acc * (1.0f + 1e-5f) - qn * qn : __int_as_float(0x7f800000);
+    for (int i = 0; i < 4; ++i) c[i] = __shfl_sync(0xffffffffu, mine, i);
+    if (vec) {
+        for (int d = lane; d < dim >> 2; d += 32) {
+            float4 a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c[i] >= 0) {
+                    a[i] = __ldg(reinterpret_cast<const float4*>(rows + (size_t)(r0 + i) * dim) + d);
+                    b[i] = __ldg(reinterpret_cast<const float4*>(centroids + (size_t)c[i] * dim) + d);
+                }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c[i] >= 0) {
+                    float diff = a[i].x - b[i].x; acc[i] = fmaf(diff, diff, acc[i]);
+                    diff = a[i].y - b[i].y; acc[i] = fmaf(diff, diff, acc[i]);
+                    diff = a[i].z - b[i].z; acc[i] = fmaf(diff, diff, acc[i]);
+                    diff = a[i].w - b[i].w; acc[i] = fmaf(diff, diff, acc[i]);
+                }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c[i] >= 0)
+                for (int d = lane; d < dim; d += 32) {
+                    const float diff = __ldg(rows + (size_t)(r0 + i) * dim + d) - __ldg(centroids + (size_t)c[i] * dim + d);
+                    acc[i] = fmaf(diff, diff, acc[i]);
+                }
     }
+    float bound = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        if (lane == i) bound = acc[i];
+    }
+    // a bound, not a result: one part in 1e5 covers the different summation order
+    if (lane < 4 && r0 + lane < n) seltop[r0 + lane] = mine >= 0 ? bound * (1.0f + 1e-5f) - qn * qn : __int_as_float(0x7f800000);
 }
-// One warp per row: lane i re-scores candidate i exactly (sequential non-fused fp32, the CPU path's arithmetic), the warp
-// takes the smallest (distance, id).  No candidate or too many: the row goes to the exact per-row kernel.
-__global__ void __launch_bounds__(256) k_coarse_refine1(const float* __restrict__ rows, const float* __restrict__ centroids, int dim,
-                                                        long long n, const int* __restrict__ cand_cnt, const int* __restrict__ cand_list,
-                                                        int* __restrict__ out_ids, float* __restrict__ out_dist,
-                                                        int* __restrict__ fail_list, int* __restrict__ n_fail) {
-    const long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (r >= n) return;
-    const int cnt = cand_cnt[r];
-    if (cnt <= 0 || cnt > kAssignCap) {
-        if (lane == 0) {
-            fail_list[atomicAdd(n_fail, 1)] = (int)r;
-            atomicAdd(n_fail + 3, 1);
+// One lane per row: its candidates (one or two as a rule) exactly (sequential non-fused fp32, the CPU path's arithmetic), the smallest
+// (distance, id).  The rows and the candidates' centroids pass through shared memory 32 dimensions at a time, a row's 128 bytes
+// loaded by eight lanes: every line is fetched once (32 rows walked by 32 threads straight from L1 took 1.7 times as long, a warp
+// per row left 30 of 32 lanes without a candidate).  No candidate or too many: the row goes on the fail list.
+// index: the rows' numbers when the candidates belong to a gathered subset (*n_dev of them, at most n).
+constexpr int kR1Warps = 4, kR1Pitch = 36;
+__global__ void __launch_bounds__(kR1Warps * 32)
+k_coarse_refine1(const float* __restrict__ rows, const float* __restrict__ centroids, int dim, int n, const int* __restrict__ n_dev,
+                 const int* __restrict__ index, const int* __restrict__ cand_cnt, const int* __restrict__ cand_list,
+                 int* __restrict__ out_ids, float* __restrict__ out_dist, int* __restrict__ fail_list, int* __restrict__ n_fail,
+                 int* __restrict__ fail_total) {
+    __shared__ __align__(16) float s_tile[kR1Warps][2][32 * kR1Pitch];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (n_dev) n = min(n, *n_dev);
+    const int at = (blockIdx.x * kR1Warps + warp) * 32 + lane;
+    if (at - lane >= n) return;
+    int r = -1, cnt = 0;
+    if (at < n) {
+        r = index ? index[at] : at;
+        cnt = cand_cnt[at];
+        if (cnt <= 0 || cnt > kAssignCap) {
+            fail_list[atomicAdd(n_fail, 1)] = r;
+            if (fail_total) atomicAdd(fail_total, 1);
+            cnt = 0;
         }
-        return;
     }
+    const bool vec = (dim & 3) == 0 && ((reinterpret_cast<uintptr_t>(centroids) | reinterpret_cast<uintptr_t>(rows)) & 15) == 0;
+    float* xs = s_tile[warp][0];
+    float* cs = s_tile[warp][1];
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
     uint64_t key = KEY_MAX;
-    if (lane < cnt) {
-        const int c = cand_list[(size_t)r * kAssignCap + lane];
-        const float* x = rows + (size_t)r * dim;
-        const float* cp = centroids + (size_t)c * dim;
+    for (int i = 0; i < most; ++i) {
+        const int c = i < cnt ? cand_list[(size_t)at * kAssignCap + i] : -1;
         float sum = 0.0f;
-        if ((dim & 3) == 0) {
-            const float4* cp4 = reinterpret_cast<const float4*>(cp);
-            const float4* x4 = reinterpret_cast<const float4*>(x);
-            for (int d = 0; d < dim / 4; ++d) {
-                const float4 a = __ldg(cp4 + d);
-                const float4 b = __ldg(x4 + d);
-                float diff = __fsub_rn(b.x, a.x); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                diff = __fsub_rn(b.y, a.y); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                diff = __fsub_rn(b.z, a.z); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                diff = __fsub_rn(b.w, a.w); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-            }
-        } else {
-            for (int d = 0; d < dim; ++d) {
-                const float diff = __fsub_rn(__ldg(x + d), __ldg(cp + d));
-                sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-            }
-        }
-        key = make_key(sum, (uint32_t)c);
-    }
+        for (int d0 = 0; d0 < dim; d0 += 32) {
+            const int w = min(32, dim - d0);
+            if (vec) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const uint64_t other = __shfl_xor_sync(0xffffffffu, key, o);
-        key = other < key ? other : key;
+                for (int j = 0; j < 8; ++j) {   // four rows and their centroids per step, eight lanes each
+                    const int o = j * 4 + (lane >> 3), v = (lane & 7) * 4;
+                    const int ro = __shfl_sync(0xffffffffu, r, o), co = __shfl_sync(0xffffffffu, c, o);
+                    if (co >= 0 && v < w) {
+                        *reinterpret_cast<float4*>(xs + o * kR1Pitch + v) = __ldg(reinterpret_cast<const float4*>(rows + (size_t)ro * dim + d0 + v));
+                        *reinterpret_cast<float4*>(cs + o * kR1Pitch + v) = __ldg(reinterpret_cast<const float4*>(centroids + (size_t)co * dim + d0 + v));
+                    }
+                }
+            } else {
+                for (int o = 0; o < 32; ++o) {
+                    const int ro = __shfl_sync(0xffffffffu, r, o), co = __shfl_sync(0xffffffffu, c, o);
+                    if (co >= 0 && lane < w) {
+                        xs[o * kR1Pitch + lane] = __ldg(rows + (size_t)ro * dim + d0 + lane);
+                        cs[o * kR1Pitch + lane] = __ldg(centroids + (size_t)co * dim + d0 + lane);
+                    }
+                }
+            }
+            __syncwarp();
+            if (c >= 0) {
+                const float* x = xs + lane * kR1Pitch;
+                const float* y = cs + lane * kR1Pitch;
+                if (w == 32) {
+#pragma unroll
+                    for (int d = 0; d < 32; d += 4) {
+                        const float4 a = *reinterpret_cast<const float4*>(x + d), b = *reinterpret_cast<const float4*>(y + d);
+                        float diff = __fsub_rn(a.x, b.x); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+                        diff = __fsub_rn(a.y, b.y); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+                        diff = __fsub_rn(a.z, b.z); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+                        diff = __fsub_rn(a.w, b.w); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
+                    }
+                } else {
+                    for (int d = 0; d < w; ++d) { const float diff = __fsub_rn(x[d], y[d]); sum = __fadd_rn(sum, __fmul_rn(diff, diff)); }
+                }
+            }
+            __syncwarp();
+        }
+        if (c >= 0) { const uint64_t kk = make_key(sum, (uint32_t)c); key = kk < key ? kk : key; }
     }
-    if (lane == 0) {
+    if (cnt > 0) {
         out_ids[r] = (int)key_idx(key);
         if (out_dist) out_dist[r] = key_dist(key);
+    }
+}
+
+// The operands of the rows on the fail list, gathered for a two-pass search of their own; rows beyond `cap` go straight to `rest`.
+__global__ void k_gather_failed(const int* __restrict__ fail_list, const int* __restrict__ n_fail, int cap, const uint4* __restrict__ qb,
+                                const float2* __restrict__ qnorm, int row16, uint4* __restrict__ qb_out, float2* __restrict__ qnorm_out,
+                                int* __restrict__ rest, int* __restrict__ n_rest) {
+    const int n = *n_fail, lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+        const int r = fail_list[i];
+        if (i >= cap) { if (lane == 0) rest[atomicAdd(n_rest, 1)] = r; continue; }
+        if (lane < row16) qb_out[(size_t)i * row16 + lane] = qb[(size_t)r * row16 + lane];
+        if (lane == 0) qnorm_out[i] = qnorm[r];
     }
 }
 
@@ -592,7 +793,8 @@ psb_status encode_rows_map(CUtensorMap* map, const void* base, long long rows, i
 
 int coarse_tc_padded_dim(int dim) { return (dim + KATOM - 1) / KATOM * KATOM; }
 int coarse_tc_tiles(int nlist) { return (nlist + kBlockCols - 1) / kBlockCols * 2; }  // whole 512-centroid blocks
-int coarse_tc_cand_cap() { return kCandCap; }
+int coarse_tc_list_cap() { return kAssignCap; }
+int coarse_tc_retry_rows() { return 65536; }
 int coarse_tc_mask_words(int nlist) { return coarse_tc_tiles(nlist) * TCOL / 32; }
 
 int coarse_tc_group(int nlist, int nprobe) {
@@ -607,65 +809,134 @@ bool coarse_tc_supported(int nq, int nlist, int dim, int nprobe) {
            nlist / coarse_tc_group(nlist, nprobe) >= 4 * nprobe;
 }
 
-psb_status launch_tc_prep_centroids(const float* d_centroids, int nlist, int dim, const float* d_mu, void* d_cb,
-                                    float* d_cn2, float* d_cnorm, cudaStream_t s) {
-    const int dimp = coarse_tc_padded_dim(dim);
-    const long long padded = (long long)coarse_tc_tiles(nlist) * TCOL;
-    k_fill_inf<<<(unsigned)((padded + 255) / 256), 256, 0, s>>>(d_cn2, padded);
+psb_status launch_mean_row(const float* d_rows, int n, int dim, float* d_mu, cudaStream_t s) {
+    k_mean_row<<<(dim + 31) / 32, 1024, 0, s>>>(d_rows, n, dim, d_mu);
     count_launch();
     PSB_LAUNCH_CHECK();
-    k_tc_prep_rows<<<(nlist * 32 + 255) / 256, 256, 0, s>>>(d_centroids, nlist, dim, dimp, d_mu,
-                                                            static_cast<__nv_bfloat16*>(d_cb), d_cnorm, d_cn2,
+    return PSB_OK;
+}
+
+psb_status launch_tc_prep_centroids(const float* d_centroids, int nlist, int dim, const float* d_mu, void* d_cb,
+                                    float* d_cn2, float* d_maxima, cudaStream_t s) {
+    const int dimp = coarse_tc_padded_dim(dim);
+    const long long padded = (long long)coarse_tc_tiles(nlist) * TCOL;
+    if (padded > nlist) {
+        k_fill_inf<<<(unsigned)((padded - nlist + 255) / 256), 256, 0, s>>>(d_cn2 + nlist, padded - nlist);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+    }
+    PSB_CUDA(cudaMemsetAsync(d_maxima, 0, 2 * sizeof(float), s));
+    k_tc_prep_rows<<<(unsigned)(((long long)nlist * 32 + 255) / 256), 256, 0, s>>>(d_centroids, nlist, dim, dimp, d_mu,
+                                                            static_cast<__nv_bfloat16*>(d_cb), nullptr, d_cn2, d_maxima,
                                                             dimp - dim >= 3 ? 2 : 0);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
 }
 
+psb_status launch_tc_prep_queries(const CoarseTcIndex& ix, const float* d_rows, long long n, void* d_qb, void* d_qnorm, cudaStream_t s) {
+    const int dimp = coarse_tc_padded_dim(ix.dim);
+    k_tc_prep_rows<<<(unsigned)((n * 32 + 255) / 256), 256, 0, s>>>(d_rows, n, ix.dim, dimp, ix.mu, static_cast<__nv_bfloat16*>(d_qb),
+                                                                     static_cast<float2*>(d_qnorm), nullptr, nullptr, dimp - ix.dim >= 3 ? 1 : 0);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+
+namespace {
+// The kernel arguments both entry points share, the tensor maps and the launch shape.
+struct TcPlan {
+    TcArgs a;
+    CUtensorMap map_q, map_c;
+    size_t smem;
+    unsigned grid;
+    bool aug;
+};
+psb_status plan_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, int nq, int nprobe, int group, int sm_count, TcPlan* pl) {
+    const int dimp = coarse_tc_padded_dim(ix.dim);
+    TcArgs& a = pl->a;
+    a.nq_dev = nullptr; a.nq = nq; a.nlist = ix.nlist; a.katoms = dimp / KATOM; a.ntiles = coarse_tc_tiles(ix.nlist);
+    a.group = group; a.ngroups = a.ntiles * (TCOL / group);
+    a.lg_group = 0;
+    while ((1 << a.lg_group) < group) ++a.lg_group;
+    a.nprobe = nprobe; a.cn2 = ix.cn2; a.qnorm = static_cast<const float2*>(ws.qnorm); a.cmax = ix.cmax; a.gmin = ws.gmin; a.seltop = ws.seltop;
+    a.mwords = coarse_tc_mask_words(ix.nlist); a.status = ws.status;
+    a.mask = nullptr; a.cand_cnt = nullptr; a.cand_list = nullptr; a.cand_cap = 0; a.band = 2.0f;
+    a.wait_limit = ws.test_wait_limit; a.skip_loads = ws.test_skip_loads;
+    a.qtiles = (nq + TQ - 1) / TQ;
+    a.cblocks = a.ntiles / 2;
+    pl->aug = dimp - ix.dim >= 3;
+    pl->smem = (size_t)a.katoms * (kStagesA * TQ + 2 * TCOL) * 128 + 1024;
+    const long long pairs = (long long)a.cblocks * a.qtiles;
+    pl->grid = (unsigned)(pairs < sm_count ? pairs : sm_count);
+    PSB_TRY(encode_rows_map(&pl->map_q, ws.qb, nq, dimp, TQ));
+    return encode_rows_map(&pl->map_c, ix.cb, ix.nlist, dimp, TCOL);
+}
+template <bool kSecondPass>
+psb_status run_tc(const TcPlan& pl, cudaEvent_t begin, cudaEvent_t end, cudaStream_t s) {
+    auto go = [&](auto kernel) -> psb_status {
+        PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        if (begin) PSB_CUDA(cudaEventRecord(begin, s));
+        kernel<<<pl.grid, kTcThreadsV2, pl.smem, s>>>(pl.map_q, pl.map_c, pl.a);
+        if (end) PSB_CUDA(cudaEventRecord(end, s));
+        return PSB_OK;
+    };
+    if (pl.aug) PSB_TRY(go(k_coarse_tc<kSecondPass, true>));
+    else PSB_TRY(go(k_coarse_tc<kSecondPass, false>));
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+// Queries whose candidates overflowed, one CTA each.
+psb_status run_exact_queries(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, const float* d_queries, int nprobe, int* d_ids, float* d_dist,
+                             int sm_count, cudaStream_t s) {
+    int buf_n = 2048;
+    while (buf_n < nprobe + kExactThreads) buf_n <<= 1;
+    const size_t esmem = (size_t)buf_n * 8 + (size_t)ix.dim * sizeof(float);
+    if (esmem > 32 * 1024)
+        PSB_CUDA(cudaFuncSetAttribute(k_coarse_exact_query, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem));
+    k_coarse_exact_query<<<sm_count, kExactThreads, esmem, s>>>(d_queries, ix.centroids, ix.dim, ix.nlist, nprobe, buf_n,
+                                                                ws.fail_list, ws.n_fail, ws.fail_cursor ? ws.fail_cursor : ws.n_fail + 1, d_ids, d_dist);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+psb_status run_refine1(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, const float* d_rows, int n, const int* n_dev, const int* index,
+                       int* d_ids, float* d_dist, int* fail_list, int* n_fail, int* fail_total, cudaStream_t s) {
+    k_coarse_refine1<<<(unsigned)((n + kR1Warps * 32 - 1) / (kR1Warps * 32)), kR1Warps * 32, 0, s>>>(
+        d_rows, ix.centroids, ix.dim, n, n_dev, index, ws.cand_cnt, ws.cand, d_ids, d_dist, fail_list, n_fail, fail_total);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+// Pass 2 with short candidate lists, one or two per row, and the exact nearest of each row (nprobe 1).
+psb_status nearest_by_lists(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, TcPlan& pl, const float* d_rows, int nq, float band, int* d_ids,
+                            float* d_dist, int* fail_total, cudaStream_t s) {
+    pl.a.cand_cnt = ws.cand_cnt; pl.a.cand_list = ws.cand; pl.a.cand_cap = kAssignCap; pl.a.band = band;
+    PSB_CUDA(cudaMemsetAsync(ws.cand_cnt, 0, sizeof(int) * (size_t)nq, s));
+    PSB_TRY(run_tc<true>(pl, ws.ev[2], ws.ev[3], s));
+    return run_refine1(ix, ws, d_rows, nq, nullptr, nullptr, d_ids, d_dist, ws.fail_list, ws.n_fail, fail_total, s);
+}
+}  // namespace
+
 psb_status launch_coarse_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, const float* d_queries, int nq,
                             int nprobe, int* d_ids, float* d_dist, int sm_count, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
-    const int dimp = coarse_tc_padded_dim(ix.dim);
-    const int katoms = dimp / KATOM;
-    const int ntiles = coarse_tc_tiles(ix.nlist);
-    const int group = coarse_tc_group(ix.nlist, nprobe);
-    const int ngroups = ntiles * (TCOL / group);
-    const bool aug = dimp - ix.dim >= 3;
     // query side: centre, round to bf16, norms
-    k_tc_prep_rows<<<(nq * 32 + 255) / 256, 256, 0, s>>>(d_queries, nq, ix.dim, dimp, ix.mu,
-                                                         static_cast<__nv_bfloat16*>(ws.qb), ws.qnorm, nullptr, aug ? 1 : 0);
-    count_launch();
-    PSB_LAUNCH_CHECK();
-    CUtensorMap map_q, map_c;
-    PSB_TRY(encode_rows_map(&map_q, ws.qb, nq, dimp, TQ));
-    PSB_TRY(encode_rows_map(&map_c, ix.cb, ix.nlist, dimp, TCOL));
-    TcArgs a;
-    a.nq = nq; a.nlist = ix.nlist; a.katoms = katoms; a.ntiles = ntiles; a.group = group; a.ngroups = ngroups;
-    a.lg_group = 0;
-    while ((1 << a.lg_group) < group) ++a.lg_group;
-    a.nprobe = nprobe; a.cn2 = ix.cn2; a.qnorm = ws.qnorm; a.cmax = ix.cmax; a.gmin = ws.gmin; a.seltop = ws.seltop;
-    a.mask = reinterpret_cast<uint32_t*>(ws.cand); a.mwords = coarse_tc_mask_words(ix.nlist); a.status = ws.status;
-    a.cand_cnt = nullptr; a.cand_list = nullptr; a.cand_cap = 0;
-    a.wait_limit = ws.test_wait_limit; a.skip_loads = ws.test_skip_loads;
-    const size_t smem = (size_t)katoms * (kStagesA * TQ + 2 * TCOL) * 128 + 1024;
-    PSB_CUDA(cudaFuncSetAttribute(k_coarse_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PSB_CUDA(cudaFuncSetAttribute(k_coarse_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PSB_CUDA(cudaFuncSetAttribute(k_coarse_tc<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PSB_CUDA(cudaFuncSetAttribute(k_coarse_tc<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    a.qtiles = (nq + TQ - 1) / TQ;
-    a.cblocks = ntiles / 2;
-    const long long pairs = (long long)a.cblocks * a.qtiles;
-    const dim3 grid((unsigned)(pairs < sm_count ? pairs : sm_count));
-    constexpr int kTcThreads = kTcThreadsV2;
-    PSB_CUDA(cudaMemsetAsync(ws.cand, 0, sizeof(uint32_t) * (size_t)nq * a.mwords, s));
+    if (!ws.queries_ready) PSB_TRY(launch_tc_prep_queries(ix, d_queries, nq, ws.qb, ws.qnorm, s));
+    TcPlan pl;
+    PSB_TRY(plan_tc(ix, ws, nq, nprobe, coarse_tc_group(ix.nlist, nprobe), sm_count, &pl));
     PSB_CUDA(cudaMemsetAsync(ws.n_fail, 0, 2 * sizeof(int), s));  // n_fail, cursor
-    if (ws.ev[0]) PSB_CUDA(cudaEventRecord(ws.ev[0], s));
-    if (aug) k_coarse_tc<false, true><<<grid, kTcThreads, smem, s>>>(map_q, map_c, a);
-    else k_coarse_tc<false, false><<<grid, kTcThreads, smem, s>>>(map_q, map_c, a);
-    if (ws.ev[1]) PSB_CUDA(cudaEventRecord(ws.ev[1], s));
-    count_launch();
-    PSB_LAUNCH_CHECK();
-    // pass 2 needs only T = the nprobe-th smallest group minimum of each query
+    PSB_TRY(run_tc<false>(pl, ws.ev[0], ws.ev[1], s));
+    // pass 2 needs only T = an upper bound of the nprobe-th smallest group minimum of each query
+    const int ngroups = pl.a.ngroups;
+    if (nprobe == 1) {
+        k_row_min<<<(unsigned)(((long long)nq * 32 + 255) / 256), 256, 0, s>>>(ws.gmin, nq, nullptr, ngroups, ws.seltop);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        PSB_TRY(nearest_by_lists(ix, ws, pl, d_queries, nq, 2.0f, d_ids, d_dist, ws.n_fail + 3, s));
+        return run_exact_queries(ix, ws, d_queries, 1, d_ids, d_dist, sm_count, s);
+    }
     if (ngroups <= kKthPerLane * 32) {
         k_kth_smallest<<<(unsigned)(((long long)nq * 32 + 255) / 256), 256, 0, s>>>(ws.gmin, nq, ngroups, nprobe, ws.seltop, nprobe);
         count_launch();
@@ -673,91 +944,57 @@ psb_status launch_coarse_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws
     } else {
         PSB_TRY(launch_select_rows(ws.gmin, nq, ngroups, nprobe, ws.selids, ws.seltop, s));
     }
-    if (ws.ev[2]) PSB_CUDA(cudaEventRecord(ws.ev[2], s));
-    if (aug) k_coarse_tc<true, true><<<grid, kTcThreads, smem, s>>>(map_q, map_c, a);
-    else k_coarse_tc<true, false><<<grid, kTcThreads, smem, s>>>(map_q, map_c, a);
-    if (ws.ev[3]) PSB_CUDA(cudaEventRecord(ws.ev[3], s));
+    pl.a.mask = reinterpret_cast<uint32_t*>(ws.cand);
+    PSB_CUDA(cudaMemsetAsync(ws.cand, 0, sizeof(uint32_t) * (size_t)nq * pl.a.mwords, s));
+    PSB_TRY(run_tc<true>(pl, ws.ev[2], ws.ev[3], s));
+    const size_t rsmem = (size_t)kCandCap * 8 + (size_t)(kRefineTile + 1) * refine_pitch(ix.dim) * sizeof(float);
+    PSB_CUDA(cudaFuncSetAttribute(k_coarse_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem));
+    k_coarse_refine<<<nq, kRefineThreads, rsmem, s>>>(d_queries, ix.centroids, ix.dim, ix.nlist, nprobe, pl.a.mask, pl.a.mwords, d_ids, d_dist,
+                                                      ws.fail_list, ws.n_fail);
     count_launch();
     PSB_LAUNCH_CHECK();
-    {
-        const size_t rsmem = (size_t)kCandCap * 8 + (size_t)((ix.dim + 3) & ~3) * sizeof(float) + (size_t)kCandCap * sizeof(int);
-        k_coarse_refine<<<nq, kRefineThreads, rsmem, s>>>(d_queries, ix.centroids, ix.dim, ix.nlist, nprobe,
-                                                          reinterpret_cast<const uint32_t*>(ws.cand), a.mwords, d_ids, d_dist,
-                                                          ws.fail_list, ws.n_fail);
-        count_launch();
-        PSB_LAUNCH_CHECK();
-    }
-    {
-        int buf_n = 2048;
-        while (buf_n < nprobe + kExactThreads) buf_n <<= 1;
-        const size_t esmem = (size_t)buf_n * 8 + (size_t)ix.dim * sizeof(float);
-        if (esmem > 32 * 1024)
-            PSB_CUDA(cudaFuncSetAttribute(k_coarse_exact_query, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem));
-        k_coarse_exact_query<<<sm_count, kExactThreads, esmem, s>>>(d_queries, ix.centroids, ix.dim, ix.nlist, nprobe, buf_n,
-                                                                    ws.fail_list, ws.n_fail, ws.n_fail + 1, d_ids, d_dist);
-        count_launch();
-        PSB_LAUNCH_CHECK();
-    }
-    return PSB_OK;
+    return run_exact_queries(ix, ws, d_queries, nprobe, d_ids, d_dist, sm_count, s);
 }
 
 // Nearest centroid of every row when a previous assignment is known (d_prev [nq], may alias d_ids): ONE GEMM pass.
 psb_status launch_coarse_tc_assign(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, const float* d_rows, int nq, const int* d_prev,
                                    int* d_ids, float* d_dist, int sm_count, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
-    const int dimp = coarse_tc_padded_dim(ix.dim);
-    const int katoms = dimp / KATOM;
-    const int ntiles = coarse_tc_tiles(ix.nlist);
-    const bool aug = dimp - ix.dim >= 3;
-    if (coarse_tc_mask_words(ix.nlist) < kAssignCap) return fail(PSB_INTERNAL, "candidate buffer too small for the list form");
-    k_tc_prep_rows<<<(nq * 32 + 255) / 256, 256, 0, s>>>(d_rows, nq, ix.dim, dimp, ix.mu, static_cast<__nv_bfloat16*>(ws.qb), ws.qnorm,
-                                                         nullptr, aug ? 1 : 0);
+    if (!ws.queries_ready) PSB_TRY(launch_tc_prep_queries(ix, d_rows, nq, ws.qb, ws.qnorm, s));
+    k_prev_bound<<<(unsigned)((nq + 31) / 32), 256, 0, s>>>(d_rows, nq, ix.dim, ix.centroids, ix.nlist, d_prev,
+                                                                              static_cast<const float2*>(ws.qnorm), ws.seltop);
     count_launch();
     PSB_LAUNCH_CHECK();
-    k_prev_bound<<<(unsigned)(((long long)nq * 32 + 255) / 256), 256, 0, s>>>(d_rows, nq, ix.dim, ix.centroids, ix.nlist, d_prev, ws.qnorm,
-                                                                              ws.seltop);
-    count_launch();
-    PSB_LAUNCH_CHECK();
-    CUtensorMap map_q, map_c;
-    PSB_TRY(encode_rows_map(&map_q, ws.qb, nq, dimp, TQ));
-    PSB_TRY(encode_rows_map(&map_c, ix.cb, ix.nlist, dimp, TCOL));
-    TcArgs a;
-    a.nq = nq; a.nlist = ix.nlist; a.katoms = katoms; a.ntiles = ntiles; a.group = 32; a.lg_group = 5; a.ngroups = ntiles * (TCOL / 32);
-    a.nprobe = 1; a.cn2 = ix.cn2; a.qnorm = ws.qnorm; a.cmax = ix.cmax; a.gmin = ws.gmin; a.seltop = ws.seltop;
-    a.mask = nullptr; a.mwords = coarse_tc_mask_words(ix.nlist); a.status = ws.status;
-    a.cand_cnt = ws.cand_cnt; a.cand_list = ws.cand; a.cand_cap = kAssignCap;
-    a.wait_limit = ws.test_wait_limit; a.skip_loads = ws.test_skip_loads;
-    const size_t smem = (size_t)katoms * (kStagesA * TQ + 2 * TCOL) * 128 + 1024;
-    PSB_CUDA(cudaFuncSetAttribute(k_coarse_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PSB_CUDA(cudaFuncSetAttribute(k_coarse_tc<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    a.qtiles = (nq + TQ - 1) / TQ;
-    a.cblocks = ntiles / 2;
-    const long long pairs = (long long)a.cblocks * a.qtiles;
-    const dim3 grid((unsigned)(pairs < sm_count ? pairs : sm_count));
-    PSB_CUDA(cudaMemsetAsync(ws.cand_cnt, 0, sizeof(int) * (size_t)nq, s));
+    TcPlan pl;
+    PSB_TRY(plan_tc(ix, ws, nq, 1, 32, sm_count, &pl));
     PSB_CUDA(cudaMemsetAsync(ws.n_fail, 0, 2 * sizeof(int), s));  // n_fail, cursor
-    if (ws.ev[2]) PSB_CUDA(cudaEventRecord(ws.ev[2], s));
-    if (aug) k_coarse_tc<true, true><<<grid, kTcThreadsV2, smem, s>>>(map_q, map_c, a);
-    else k_coarse_tc<true, false><<<grid, kTcThreadsV2, smem, s>>>(map_q, map_c, a);
-    if (ws.ev[3]) PSB_CUDA(cudaEventRecord(ws.ev[3], s));
+    PSB_CUDA(cudaMemsetAsync(ws.n_fail2, 0, sizeof(int), s));
+    PSB_TRY(nearest_by_lists(ix, ws, pl, d_rows, nq, 1.0f, d_ids, d_dist, nullptr, s));
+    // Rows whose bound was too loose (their centroid has moved far away: the second iteration of a training, rows of clusters that
+    // had drawn no initial centroid) are gathered and get the two passes of a row without a bound; how many they are is known on
+    // the device only.  Searched one CTA per row, 13 % of 400,000 rows took 10 ms.
+    const int cap = nq < coarse_tc_retry_rows() ? nq : coarse_tc_retry_rows();
+    const int row16 = coarse_tc_padded_dim(ix.dim) / 8;
+    k_gather_failed<<<sm_count * 4, 256, 0, s>>>(ws.fail_list, ws.n_fail, cap, static_cast<const uint4*>(ws.qb), static_cast<const float2*>(ws.qnorm),
+                                                 row16, static_cast<uint4*>(ws.retry_qb), static_cast<float2*>(ws.retry_qnorm), ws.fail_list2, ws.n_fail2);
     count_launch();
     PSB_LAUNCH_CHECK();
-    k_coarse_refine1<<<(unsigned)(((long long)nq * 32 + 255) / 256), 256, 0, s>>>(d_rows, ix.centroids, ix.dim, nq, ws.cand_cnt, ws.cand, d_ids,
-                                                                                  d_dist, ws.fail_list, ws.n_fail);
+    CoarseTcWorkspace w2 = ws;
+    w2.qb = ws.retry_qb; w2.qnorm = ws.retry_qnorm;
+    TcPlan p2;
+    PSB_TRY(plan_tc(ix, w2, cap, 1, 32, sm_count, &p2));
+    p2.a.nq_dev = ws.n_fail;
+    PSB_TRY(run_tc<false>(p2, nullptr, nullptr, s));
+    k_row_min<<<(unsigned)(((long long)cap * 32 + 255) / 256), 256, 0, s>>>(ws.gmin, cap, ws.n_fail, p2.a.ngroups, ws.seltop);
     count_launch();
     PSB_LAUNCH_CHECK();
-    {
-        int buf_n = 2048;
-        while (buf_n < 1 + kExactThreads) buf_n <<= 1;
-        const size_t esmem = (size_t)buf_n * 8 + (size_t)ix.dim * sizeof(float);
-        if (esmem > 32 * 1024)
-            PSB_CUDA(cudaFuncSetAttribute(k_coarse_exact_query, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem));
-        k_coarse_exact_query<<<sm_count, kExactThreads, esmem, s>>>(d_rows, ix.centroids, ix.dim, ix.nlist, 1, buf_n, ws.fail_list, ws.n_fail,
-                                                                    ws.n_fail + 1, d_ids, d_dist);
-        count_launch();
-        PSB_LAUNCH_CHECK();
-    }
-    return PSB_OK;
+    p2.a.cand_cnt = ws.cand_cnt; p2.a.cand_list = ws.cand; p2.a.cand_cap = kAssignCap;
+    PSB_CUDA(cudaMemsetAsync(ws.cand_cnt, 0, sizeof(int) * (size_t)cap, s));
+    PSB_TRY(run_tc<true>(p2, nullptr, nullptr, s));
+    PSB_TRY(run_refine1(ix, ws, d_rows, cap, ws.n_fail, ws.fail_list, d_ids, d_dist, ws.fail_list2, ws.n_fail2, nullptr, s));
+    CoarseTcWorkspace w3 = ws;
+    w3.fail_list = ws.fail_list2; w3.n_fail = ws.n_fail2; w3.fail_cursor = ws.n_fail + 1;
+    return run_exact_queries(ix, w3, d_rows, 1, d_ids, d_dist, sm_count, s);
 }
 
 }  // namespace psb

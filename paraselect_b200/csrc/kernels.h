@@ -39,32 +39,44 @@ struct CoarseTcIndex {
     const void* cb;          // [nlist][dimp] bf16, centred on mu
     const float* cn2;        // [tiles * 256] |c'|^2 (+inf padding)
     const float* mu;         // [dim] mean centroid
-    float cmax;              // max |c'|
+    const float* cmax;       // device [2]: max |c'| and max |c' - bf16(c')|
     int nlist, dim;
 };
 struct CoarseTcWorkspace {
     void* qb;        // [nq][dimp] bf16
-    float* qnorm;    // [nq]
+    void* qnorm;     // [nq] float2: |q'| and |q' - bf16(q')|
+    bool queries_ready = false;   // qb and qnorm hold these rows already (launch_tc_prep_queries)
     float* gmin;     // [nq][groups]
     float* seltop;   // [nq][nprobe]
     int* selids;     // [nq][nprobe]
     int* cand_cnt;   // [nq]
     int* cand;       // [nq][mask words]: pass 2's candidate bit mask, one bit per (padded) centroid
     int* fail_list;  // [nq]
-    int* n_fail;     // [2]: count, cursor
+    // bounded assignment only: the rows that failed get a second, two-pass search (coarse_tc_retry_rows() of them at most)
+    int* fail_list2 = nullptr;       // [nq] rows that failed again, and their count
+    int* n_fail2 = nullptr;
+    void* retry_qb = nullptr;        // [retry rows][dimp] bf16
+    void* retry_qnorm = nullptr;     // [retry rows] float2
+    int* n_fail;     // count, cursor, (status), cumulative count of failed queries
+    int* fail_cursor = nullptr;   // null: n_fail + 1
     int* status;     // [1]
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // optional: begin/end of GEMM pass 1 and pass 2
     int test_wait_limit = 0, test_skip_loads = 0;              // test hooks of the time-out path (0: off)
 };
 int coarse_tc_padded_dim(int dim);
 int coarse_tc_tiles(int nlist);
-int coarse_tc_cand_cap();
+int coarse_tc_list_cap();   // candidate ids per row of the list form (nprobe 1)
+int coarse_tc_retry_rows(); // rows a bounded assignment searches again with two passes, at most
 int coarse_tc_mask_words(int nlist);
 int coarse_tc_group(int nlist, int nprobe);
 bool coarse_tc_supported(int nq, int nlist, int dim, int nprobe);
-// d_cb [nlist][dimp] bf16, d_cn2 [tiles*256], d_cnorm [nlist] out.
+// d_mu [dim] = mean of n rows: the point the operands are centred on.
+psb_status launch_mean_row(const float* d_rows, int n, int dim, float* d_mu, cudaStream_t s);
+// d_cb [nlist][dimp] bf16, d_cn2 [tiles*256], d_maxima [2] (CoarseTcIndex::cmax) out.
 psb_status launch_tc_prep_centroids(const float* d_centroids, int nlist, int dim, const float* d_mu, void* d_cb,
-                                    float* d_cn2, float* d_cnorm, cudaStream_t s);
+                                    float* d_cn2, float* d_maxima, cudaStream_t s);
+// The query side of the same: d_qb [n][dimp] bf16, d_qnorm [n] float2.
+psb_status launch_tc_prep_queries(const CoarseTcIndex& ix, const float* d_rows, long long n, void* d_qb, void* d_qnorm, cudaStream_t s);
 psb_status launch_coarse_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, const float* d_queries, int nq,
                             int nprobe, int* d_ids, float* d_dist, int sm_count, cudaStream_t s);
 

@@ -59,6 +59,7 @@ struct DevBuf {
         bytes = need;
         return PSB_OK;
     }
+    psb_status reserve(size_t need, int, cudaStream_t) { return reserve(need); }   // the signature of PoolBuf
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
@@ -198,72 +199,76 @@ struct EventTimer {
     }
 };
 
-// Centroid-side buffers of the tensor-core coarse filter (built once per index).
+// Centroid-side buffers of the tensor-core coarse filter (built once per index; rebuilt per iteration in training).
+template <typename Buf>
 struct TcIndexBuffers {
-    DevBuf cb, cn2, cnorm, mu;
-    float cmax = 0.f;
+    Buf cb, cn2, cmax, mu;
     bool ready = false;
-    psb_status prepare(const float* h_centroids, const float* d_centroids, int nlist, int dim, cudaStream_t st) {
-        std::vector<double> acc((size_t)dim, 0.0);
-        for (int c = 0; c < nlist; ++c)
-            for (int d = 0; d < dim; ++d) acc[(size_t)d] += h_centroids[(size_t)c * dim + d];
-        std::vector<float> mean((size_t)dim);
-        for (int d = 0; d < dim; ++d) mean[(size_t)d] = (float)(acc[(size_t)d] / nlist);
+    // keep_mean: the operands stay centred on the mean of an earlier call (queries prepared then stay valid).
+    psb_status prepare(const float* d_centroids, int nlist, int dim, int device, cudaStream_t st, bool keep_mean = false) {
         const int dimp = coarse_tc_padded_dim(dim);
-        PSB_TRY(mu.reserve(sizeof(float) * (size_t)dim));
-        PSB_TRY(cb.reserve((size_t)2 * nlist * dimp));
-        PSB_TRY(cn2.reserve(sizeof(float) * (size_t)coarse_tc_tiles(nlist) * 256));
-        PSB_TRY(cnorm.reserve(sizeof(float) * (size_t)nlist));
-        PSB_CUDA(cudaMemcpyAsync(mu.p, mean.data(), sizeof(float) * (size_t)dim, cudaMemcpyHostToDevice, st));
-        PSB_TRY(launch_tc_prep_centroids(d_centroids, nlist, dim, mu.as<float>(), cb.p, cn2.as<float>(), cnorm.as<float>(), st));
-        std::vector<float> norms((size_t)nlist);
-        PSB_CUDA(cudaMemcpyAsync(norms.data(), cnorm.p, sizeof(float) * (size_t)nlist, cudaMemcpyDeviceToHost, st));
-        PSB_CUDA(cudaStreamSynchronize(st));
-        cmax = 0.f;
-        for (float v : norms) cmax = std::max(cmax, v);
+        PSB_TRY(mu.reserve(sizeof(float) * (size_t)dim, device, st));
+        PSB_TRY(cb.reserve((size_t)2 * nlist * dimp, device, st));
+        PSB_TRY(cn2.reserve(sizeof(float) * (size_t)coarse_tc_tiles(nlist) * 256, device, st));
+        PSB_TRY(cmax.reserve(sizeof(float) * 2, device, st));
+        if (!keep_mean) PSB_TRY(launch_mean_row(d_centroids, nlist, dim, mu.template as<float>(), st));
+        PSB_TRY(launch_tc_prep_centroids(d_centroids, nlist, dim, mu.template as<float>(), cb.p, cn2.template as<float>(), cmax.template as<float>(), st));
         ready = true;
         return PSB_OK;
     }
     CoarseTcIndex view(const float* d_centroids, int nlist, int dim) const {
         CoarseTcIndex ix;
-        ix.centroids = d_centroids; ix.cb = cb.p; ix.cn2 = cn2.as<float>(); ix.mu = mu.as<float>(); ix.cmax = cmax;
+        ix.centroids = d_centroids; ix.cb = cb.p; ix.cn2 = cn2.template as<float>(); ix.mu = mu.template as<float>(); ix.cmax = cmax.template as<float>();
         ix.nlist = nlist; ix.dim = dim;
         return ix;
     }
 };
 
 // Per-batch buffers of the tensor-core coarse filter.
+template <typename Buf>
 struct TcWorkBuffers {
-    DevBuf qb, qnorm, gmin, seltop, selids, cand_cnt, cand, fail_list, scalars;
-    psb_status ensure(int nq, int nlist, int dim, int nprobe, cudaStream_t st) {
+    Buf qb, qnorm, gmin, seltop, selids, cand_cnt, cand, fail_list, scalars, fail_list2, retry_qb, retry_qnorm;
+    // own_queries: qb and qnorm are needed (not when the caller keeps prepared rows); bounded: rows come with a previous assignment
+    // (launch_coarse_tc_assign), which needs group minima for the rows it searches again only.
+    psb_status ensure(int nq, int nlist, int dim, int nprobe, int device, cudaStream_t st, bool own_queries = true, bool bounded = false) {
         const int dimp = coarse_tc_padded_dim(dim);
         const int groups = coarse_tc_tiles(nlist) * (256 / coarse_tc_group(nlist, nprobe));
-        PSB_TRY(qb.reserve((size_t)2 * nq * dimp));
-        PSB_TRY(qnorm.reserve(sizeof(float) * (size_t)nq));
-        PSB_TRY(gmin.reserve(sizeof(float) * (size_t)nq * groups));
-        PSB_TRY(seltop.reserve(sizeof(float) * (size_t)nq * nprobe));
-        PSB_TRY(selids.reserve(sizeof(int) * (size_t)nq * nprobe));
-        PSB_TRY(cand_cnt.reserve(sizeof(int) * (size_t)nq));
-        PSB_TRY(cand.reserve(sizeof(int) * (size_t)nq * coarse_tc_mask_words(nlist)));
-        PSB_TRY(fail_list.reserve(sizeof(int) * (size_t)nq));
+        if (own_queries) {
+            PSB_TRY(qb.reserve((size_t)2 * nq * dimp, device, st));
+            PSB_TRY(qnorm.reserve(sizeof(float) * 2 * (size_t)nq, device, st));
+        }
+        const int retry = std::min(nq, coarse_tc_retry_rows());
+        PSB_TRY(gmin.reserve(sizeof(float) * (size_t)(bounded ? retry : nq) * groups, device, st));
+        if (bounded) {
+            PSB_TRY(fail_list2.reserve(sizeof(int) * (size_t)nq, device, st));
+            PSB_TRY(retry_qb.reserve((size_t)2 * retry * dimp, device, st));
+            PSB_TRY(retry_qnorm.reserve(sizeof(float) * 2 * (size_t)retry, device, st));
+        }
+        PSB_TRY(seltop.reserve(sizeof(float) * (size_t)nq * nprobe, device, st));
+        if (nprobe > 1) PSB_TRY(selids.reserve(sizeof(int) * (size_t)nq * nprobe, device, st));
+        PSB_TRY(cand_cnt.reserve(sizeof(int) * (size_t)nq, device, st));
+        PSB_TRY(cand.reserve(sizeof(int) * (size_t)nq * (nprobe == 1 ? coarse_tc_list_cap() : coarse_tc_mask_words(nlist)), device, st));
+        PSB_TRY(fail_list.reserve(sizeof(int) * (size_t)nq, device, st));
         if (!scalars.p) {
-            PSB_TRY(scalars.reserve(sizeof(int) * 4));
-            PSB_CUDA(cudaMemsetAsync(scalars.p, 0, sizeof(int) * 4, st));
+            PSB_TRY(scalars.reserve(sizeof(int) * 8, device, st));
+            PSB_CUDA(cudaMemsetAsync(scalars.p, 0, sizeof(int) * 8, st));
         }
         return PSB_OK;
     }
     CoarseTcWorkspace view() const {
         CoarseTcWorkspace w;
-        w.qb = qb.p; w.qnorm = qnorm.as<float>(); w.gmin = gmin.as<float>(); w.seltop = seltop.as<float>();
-        w.selids = selids.as<int>(); w.cand_cnt = cand_cnt.as<int>(); w.cand = cand.as<int>();
-        w.fail_list = fail_list.as<int>(); w.n_fail = scalars.as<int>(); w.status = scalars.as<int>() + 2;
+        w.qb = qb.p; w.qnorm = qnorm.p; w.gmin = gmin.template as<float>(); w.seltop = seltop.template as<float>();
+        w.selids = selids.template as<int>(); w.cand_cnt = cand_cnt.template as<int>(); w.cand = cand.template as<int>();
+        w.fail_list = fail_list.template as<int>(); w.n_fail = scalars.template as<int>(); w.status = scalars.template as<int>() + 2;
+        w.fail_list2 = fail_list2.template as<int>(); w.n_fail2 = scalars.template as<int>() + 4;
+        w.retry_qb = retry_qb.p; w.retry_qnorm = retry_qnorm.p;
         return w;
     }
     // Reads the sticky time-out word (the stream must be idle).
     psb_status check_status() const {
         if (!scalars.p) return PSB_OK;
         int st = 0;
-        PSB_CUDA(cudaMemcpy(&st, scalars.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost));
+        PSB_CUDA(cudaMemcpy(&st, scalars.template as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost));
         if (st) return fail(PSB_TIMEOUT, "a bounded wait in the tensor-core coarse kernel gave up");
         return PSB_OK;
     }
@@ -275,8 +280,8 @@ struct TcWorkBuffers {
 using namespace psb;
 
 struct psb_session {
-    TcIndexBuffers tc_index;
-    TcWorkBuffers tc_work;
+    TcIndexBuffers<DevBuf> tc_index;
+    TcWorkBuffers<DevBuf> tc_work;
     int device = 0;
     int sm_count = 148;
     cudaStream_t stream = nullptr;
@@ -549,7 +554,7 @@ psb_status coarse_exact(psb_session* s, const float* d_queries, int nq, int npro
     const bool tc_ok = s->tc_index.ready && coarse_tc_supported(nq, s->nlist, s->dim, nprobe);
     if (mode == 2 && !tc_ok) return fail(PSB_UNSUPPORTED_SHAPE, "tensor-core coarse stage does not support this shape");
     if (mode != 1 && tc_ok) {
-        PSB_TRY(s->tc_work.ensure(nq, s->nlist, s->dim, nprobe, s->stream));
+        PSB_TRY(s->tc_work.ensure(nq, s->nlist, s->dim, nprobe, s->device, s->stream));
         CoarseTcWorkspace tw = s->tc_work.view();
         tw.test_wait_limit = s->opt.test_wait_limit; tw.test_skip_loads = (s->opt.test_skip_mma & 2) ? 1 : 0;
         if (s->opt.time_kernels) {
@@ -870,7 +875,7 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
     PSB_TRY(s->centroids.reserve(sizeof(float) * (size_t)nlist * s->dim));
     PSB_CUDA(cudaMemcpyAsync(s->centroids.p, index->coarse.centroids, sizeof(float) * (size_t)nlist * s->dim, cudaMemcpyHostToDevice, st));
     if (opt.coarse_mode != 1 && nlist >= 1024 && coarse_tc_padded_dim(s->dim) <= 128)
-        PSB_TRY(s->tc_index.prepare(index->coarse.centroids, s->centroids.as<float>(), nlist, s->dim, st));
+        PSB_TRY(s->tc_index.prepare(s->centroids.as<float>(), nlist, s->dim, s->device, st));
     PSB_TRY(s->offsets.reserve(sizeof(long long) * ((size_t)nlist + 1)));
     PSB_CUDA(cudaMemcpyAsync(s->offsets.p, index->lists.offsets, sizeof(long long) * ((size_t)nlist + 1), cudaMemcpyHostToDevice, st));
     PSB_TRY(s->reordered.reserve(sizeof(long long) * (size_t)std::max<long long>(1, s->n_vectors)));
@@ -1627,7 +1632,7 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
     PSB_TRY(s->centroids.reserve(sizeof(float) * nl * s->dim));
     PSB_CUDA(cudaMemcpyAsync(s->centroids.p, index->coarse.centroids, sizeof(float) * nl * s->dim, cudaMemcpyHostToDevice, st));
     if (opt.coarse_mode != 1 && s->nlist >= 1024 && coarse_tc_padded_dim(s->dim) <= 128)
-        PSB_TRY(s->tc_index.prepare(index->coarse.centroids, s->centroids.as<float>(), s->nlist, s->dim, st));
+        PSB_TRY(s->tc_index.prepare(s->centroids.as<float>(), s->nlist, s->dim, s->device, st));
     PSB_TRY(s->offsets.reserve(sizeof(long long) * (nl + 1)));
     PSB_CUDA(cudaMemcpyAsync(s->offsets.p, index->lists.offsets, sizeof(long long) * (nl + 1), cudaMemcpyHostToDevice, st));
     PSB_TRY(s->reordered.reserve(sizeof(long long) * n));
@@ -1804,10 +1809,10 @@ psb_status psb_coarse_host(const float* h_queries, int nq, const float* h_centro
     const bool tc_ok = coarse_tc_supported(nq, nlist, dim, nprobe);
     if (coarse_mode == 2 && !tc_ok) return fail(PSB_UNSUPPORTED_SHAPE, "tensor-core coarse stage does not support this shape");
     if (coarse_mode != 1 && tc_ok) {
-        TcIndexBuffers tix;
-        TcWorkBuffers twk;
-        PSB_TRY(tix.prepare(h_centroids, c.as<float>(), nlist, dim, nullptr));
-        PSB_TRY(twk.ensure(nq, nlist, dim, nprobe, nullptr));
+        TcIndexBuffers<PoolBuf> tix;
+        TcWorkBuffers<PoolBuf> twk;
+        PSB_TRY(tix.prepare(c.as<float>(), nlist, dim, device, nullptr));
+        PSB_TRY(twk.ensure(nq, nlist, dim, nprobe, device, nullptr));
         PSB_TRY(launch_coarse_tc(tix.view(c.as<float>(), nlist, dim), twk.view(), q.as<float>(), nq, nprobe, ids.as<int>(),
                                  dist.as<float>(), sms, nullptr));
         PSB_CUDA(cudaDeviceSynchronize());
@@ -1871,62 +1876,99 @@ psb_status psb_knn_exact(const float* d_queries, int nq, const float* d_base, in
 
 // ---- training ---------------------------------------------------------------------------------------------
 
+namespace {
+// Nearest-centroid assignment of n device rows: the coarse stage with nprobe 1.  Large problems take the tensor-core filter with
+// exact refinement (identical assignments and distances: ties go to the lower centroid id on both paths), others the exact kernels.
+// One object serves all iterations of a training: the rows' bf16 operand is made once (centred on the first iteration's mean
+// centroid - any point will do) and kept when it takes at most kKeepRows bytes, and nothing is copied to the host in between.
+class Assigner {
+public:
+    Assigner(const float* d_data, int64_t n, int dim, int k, int device, int sms, cudaStream_t st)
+        : data_(d_data), n_(n), dim_(dim), k_(k), device_(device), sms_(sms), st_(st) {
+        tc_ = coarse_tc_supported((int)std::min<int64_t>(n, 1 << 30), k, dim, 1);
+    }
+    // d_assign [n], d_best [n] out; bounded: d_assign holds an assignment on entry, whose distances bound the nearest ones (one
+    // filter pass instead of two).
+    psb_status run(const float* d_centroids, int* d_assign, float* d_best, bool bounded) {
+        if (!tc_) return exact(d_centroids, d_assign, d_best);
+        PSB_TRY(index_.prepare(d_centroids, k_, dim_, device_, st_, index_.ready));
+        const CoarseTcIndex ix = index_.view(d_centroids, k_, dim_);
+        const int dimp = coarse_tc_padded_dim(dim_);
+        const bool keep = (size_t)n_ * dimp * 2 <= kKeepRows;
+        if (keep && !rows_.p) {
+            PSB_TRY(rows_.reserve((size_t)n_ * dimp * 2, device_, st_));
+            PSB_TRY(norms_.reserve((size_t)n_ * 8, device_, st_));
+            PSB_TRY(launch_tc_prep_queries(ix, data_, n_, rows_.p, norms_.p, st_));
+        }
+        // Rows per launch: the group minima of a first pass (k / 32 floats a row) or the candidate lists (32 ids a row) bound it;
+        // equal parts, so that no part falls below the filter's smallest batch.
+        const int64_t most = bounded ? 2097152 : 262144;
+        const int64_t parts = (n_ + most - 1) / most;
+        const int64_t chunk = ((n_ + parts - 1) / parts + 127) / 128 * 128;
+        for (int64_t r0 = 0; r0 < n_; r0 += chunk) {
+            const int nn = (int)std::min<int64_t>(chunk, n_ - r0);
+            PSB_TRY(work_.ensure((int)std::min<int64_t>(chunk, n_), k_, dim_, 1, device_, st_, !keep, bounded));
+            CoarseTcWorkspace w = work_.view();
+            if (keep) {
+                w.qb = rows_.as<unsigned char>() + (size_t)r0 * dimp * 2;
+                w.qnorm = norms_.as<unsigned char>() + (size_t)r0 * 8;
+                w.queries_ready = true;
+            }
+            const float* rows = data_ + (size_t)r0 * dim_;
+            if (bounded) PSB_TRY(launch_coarse_tc_assign(ix, w, rows, nn, d_assign + r0, d_assign + r0, d_best + r0, sms_, st_));
+            else PSB_TRY(launch_coarse_tc(ix, w, rows, nn, 1, d_assign + r0, d_best + r0, sms_, st_));
+        }
+        if (!bounded) work_.gmin.release();
+        return PSB_OK;
+    }
+    psb_status check_status() const { return tc_ ? work_.check_status() : PSB_OK; }
+private:
+    static constexpr size_t kKeepRows = (size_t)4 << 30;
+    psb_status exact(const float* d_centroids, int* d_assign, float* d_best) {
+        const size_t row_bytes = sizeof(float) * (size_t)k_;
+        const int64_t chunk = std::min<int64_t>((int64_t)std::max<size_t>(64, ((size_t)1 << 30) / row_bytes), n_);
+        PSB_TRY(tile_.reserve(row_bytes * (size_t)chunk, device_, st_));
+        for (int64_t r0 = 0; r0 < n_; r0 += chunk) {
+            const int nn = (int)std::min<int64_t>(chunk, n_ - r0);
+            PSB_TRY(launch_coarse_dist_exact(data_ + (size_t)r0 * dim_, nn, d_centroids, k_, dim_, tile_.as<float>(), st_));
+            PSB_TRY(launch_select_rows(tile_.as<float>(), nn, k_, 1, d_assign + r0, d_best + r0, st_));
+        }
+        return PSB_OK;
+    }
+    const float* data_;
+    int64_t n_;
+    int dim_, k_, device_, sms_;
+    cudaStream_t st_;
+    bool tc_;
+    TcIndexBuffers<PoolBuf> index_;
+    TcWorkBuffers<PoolBuf> work_;
+    PoolBuf rows_, norms_, tile_;
+};
+}  // namespace
+
 psb_status psb_kmeans_train(const float* d_data, int64_t n, int dim, float* d_centroids, int k, int iters,
                             int* d_assign, double* h_objective, int device, void* stream) {
     if (!d_data || !d_centroids || n <= 0 || dim <= 0 || k <= 0 || iters < 0) return fail(PSB_INVALID_ARGUMENT, "invalid k-means request");
     int sms = 0;
     PSB_TRY(check_device(device, &sms));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    DevBuf tile, assign, best, sums, counts, obj;
-    const size_t row_bytes = sizeof(float) * (size_t)k;
-    long long chunk = (long long)std::max<size_t>(64, ((size_t)1 << 30) / row_bytes);
-    chunk = std::min<long long>(chunk, n);
-    // Assignment = nearest centroid = the coarse stage with nprobe 1.  Large problems take the tensor-core filter with
-    // exact refinement (identical assignments and distances: ties go to the lower centroid id on both paths); the bf16
-    // centroid operand is rebuilt from the current centroids at the start of every iteration.
-    const long long chunk_tc = std::min<long long>(n, 262144);
-    const bool tc = coarse_tc_supported((int)chunk_tc, k, dim, 1);
-    TcIndexBuffers tci;
-    TcWorkBuffers tcw;
-    std::vector<float> h_centroids;
-    if (tc) { chunk = chunk_tc; h_centroids.resize((size_t)k * dim); }
-    else PSB_TRY(tile.reserve(row_bytes * (size_t)chunk));
-    PSB_TRY(best.reserve(sizeof(float) * (size_t)n));
+    PoolBuf assign, best, sums, counts, obj, acc_order, acc_offsets, acc_cursor;   // the last three: rows grouped by centroid
+    PSB_TRY(best.reserve(sizeof(float) * (size_t)n, device, st));
     int* d_as = d_assign;
-    if (!d_as) { PSB_TRY(assign.reserve(sizeof(int) * (size_t)n)); d_as = assign.as<int>(); }
-    PSB_TRY(sums.reserve(sizeof(double) * (size_t)k * dim)); PSB_TRY(counts.reserve(sizeof(int) * (size_t)k));
-    PSB_TRY(obj.reserve(sizeof(double) * ((size_t)iters + 1)));
-    DevBuf acc_order, acc_offsets, acc_cursor;   // rows grouped by centroid for the accumulation
-    PSB_TRY(acc_order.reserve(sizeof(int) * (size_t)n));
-    PSB_TRY(acc_offsets.reserve(sizeof(int) * ((size_t)k + 1)));
-    PSB_TRY(acc_cursor.reserve(sizeof(int) * (size_t)k));
+    if (!d_as) { PSB_TRY(assign.reserve(sizeof(int) * (size_t)n, device, st)); d_as = assign.as<int>(); }
+    PSB_TRY(sums.reserve(sizeof(double) * (size_t)k * dim, device, st)); PSB_TRY(counts.reserve(sizeof(int) * (size_t)k, device, st));
+    PSB_TRY(obj.reserve(sizeof(double) * ((size_t)iters + 1), device, st));
+    PSB_TRY(acc_order.reserve(sizeof(int) * (size_t)n, device, st));
+    PSB_TRY(acc_offsets.reserve(sizeof(int) * ((size_t)k + 1), device, st));
+    PSB_TRY(acc_cursor.reserve(sizeof(int) * (size_t)k, device, st));
     KmeansAccumWs acc_ws;
     acc_ws.order = acc_order.as<int>(); acc_ws.offsets = acc_offsets.as<int>(); acc_ws.cursor = acc_cursor.as<int>();
     PSB_CUDA(cudaMemsetAsync(obj.p, 0, sizeof(double) * ((size_t)iters + 1), st));
+    Assigner assigner(d_data, n, dim, k, device, sms, st);
     for (int it = 0; it <= iters; ++it) {
-        if (tc) {
-            PSB_CUDA(cudaMemcpyAsync(h_centroids.data(), d_centroids, sizeof(float) * (size_t)k * dim, cudaMemcpyDeviceToHost, st));
-            PSB_CUDA(cudaStreamSynchronize(st));
-            PSB_TRY(tci.prepare(h_centroids.data(), d_centroids, k, dim, st));
-        }
-        for (long long r0 = 0; r0 < n; r0 += chunk) {
-            const int nn = (int)std::min<long long>(chunk, n - r0);
-            if (tc && coarse_tc_supported(nn, k, dim, 1)) {
-                PSB_TRY(tcw.ensure(nn, k, dim, 1, st));
-                // After the first iteration every row brings a bound along - its distance to the centroid it had, where that
-                // centroid is now - and the filter GEMM runs once instead of twice.
-                if (it > 0)
-                    PSB_TRY(launch_coarse_tc_assign(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, d_as + r0,
-                                                    d_as + r0, best.as<float>() + r0, sms, st));
-                else
-                    PSB_TRY(launch_coarse_tc(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, 1,
-                                             d_as + r0, best.as<float>() + r0, sms, st));
-            } else {
-                PSB_TRY(tile.reserve(row_bytes * (size_t)nn));
-                PSB_TRY(launch_coarse_dist_exact(d_data + (size_t)r0 * dim, nn, d_centroids, k, dim, tile.as<float>(), st));
-                PSB_TRY(launch_select_rows(tile.as<float>(), nn, k, 1, d_as + r0, best.as<float>() + r0, st));
-            }
-        }
+        // After the first iteration every row brings a bound along - its distance to the centroid it had, where that centroid
+        // is now - and the filter GEMM runs once instead of twice.
+        PSB_TRY(assigner.run(d_centroids, d_as, best.as<float>(), it > 0));
         PSB_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * (size_t)k, st));
         PSB_TRY(launch_kmeans_accumulate(d_data, n, dim, d_as, best.as<float>(), k, sums.as<double>(), counts.as<int>(),
                                          obj.as<double>() + it, acc_ws, st));
@@ -1934,8 +1976,7 @@ psb_status psb_kmeans_train(const float* d_data, int64_t n, int dim, float* d_ce
     }
     if (h_objective) PSB_CUDA(cudaMemcpyAsync(h_objective, obj.p, sizeof(double) * ((size_t)iters + 1), cudaMemcpyDeviceToHost, st));
     PSB_CUDA(cudaStreamSynchronize(st));
-    if (tc) PSB_TRY(tcw.check_status());
-    return PSB_OK;
+    return assigner.check_status();
 }
 
 // ---- one Lloyd iteration in three calls (data-parallel training: the caller all-reduces sums and counts in between) ----
@@ -1952,39 +1993,10 @@ psb_status psb_kmeans_assign_bounded(const float* d_data, int64_t n, int dim, co
     int sms = 0;
     PSB_TRY(check_device(device, &sms));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t row_bytes = sizeof(float) * (size_t)k;
-    long long chunk = std::min<long long>((long long)std::max<size_t>(64, ((size_t)1 << 30) / row_bytes), n);
-    const long long chunk_tc = std::min<long long>(n, 262144);
-    const bool tc = coarse_tc_supported((int)chunk_tc, k, dim, 1);
-    TcIndexBuffers tci;
-    TcWorkBuffers tcw;
-    DevBuf tile;
-    if (tc) {
-        chunk = chunk_tc;
-        std::vector<float> h_centroids((size_t)k * dim);
-        PSB_CUDA(cudaMemcpyAsync(h_centroids.data(), d_centroids, sizeof(float) * (size_t)k * dim, cudaMemcpyDeviceToHost, st));
-        PSB_CUDA(cudaStreamSynchronize(st));
-        PSB_TRY(tci.prepare(h_centroids.data(), d_centroids, k, dim, st));
-    }
-    for (long long r0 = 0; r0 < n; r0 += chunk) {
-        const int nn = (int)std::min<long long>(chunk, n - r0);
-        if (tc && coarse_tc_supported(nn, k, dim, 1)) {
-            PSB_TRY(tcw.ensure(nn, k, dim, 1, st));
-            if (have_previous)
-                PSB_TRY(launch_coarse_tc_assign(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, d_assign + r0,
-                                                d_assign + r0, d_best + r0, sms, st));
-            else
-                PSB_TRY(launch_coarse_tc(tci.view(d_centroids, k, dim), tcw.view(), d_data + (size_t)r0 * dim, nn, 1, d_assign + r0,
-                                         d_best + r0, sms, st));
-        } else {
-            PSB_TRY(tile.reserve(row_bytes * (size_t)nn));
-            PSB_TRY(launch_coarse_dist_exact(d_data + (size_t)r0 * dim, nn, d_centroids, k, dim, tile.as<float>(), st));
-            PSB_TRY(launch_select_rows(tile.as<float>(), nn, k, 1, d_assign + r0, d_best + r0, st));
-        }
-    }
-    PSB_CUDA(cudaStreamSynchronize(st));  // the work buffers above are released on return
-    if (tc) PSB_TRY(tcw.check_status());
-    return PSB_OK;
+    Assigner assigner(d_data, n, dim, k, device, sms, st);
+    PSB_TRY(assigner.run(d_centroids, d_assign, d_best, have_previous != 0));
+    PSB_CUDA(cudaStreamSynchronize(st));
+    return assigner.check_status();
 }
 
 psb_status psb_kmeans_accumulate(const float* d_data, int64_t n, int dim, const int* d_assign, const float* d_best, int k,
@@ -1995,10 +2007,10 @@ psb_status psb_kmeans_accumulate(const float* d_data, int64_t n, int dim, const 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     PSB_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(int) * (size_t)k, st));
     PSB_CUDA(cudaMemsetAsync(d_objective, 0, sizeof(double), st));
-    DevBuf order, offsets, cursor;   // rows grouped by centroid: freed after the stream has drained below
-    PSB_TRY(order.reserve(sizeof(int) * (size_t)std::max<int64_t>(n, 1)));
-    PSB_TRY(offsets.reserve(sizeof(int) * ((size_t)k + 1)));
-    PSB_TRY(cursor.reserve(sizeof(int) * (size_t)k));
+    PoolBuf order, offsets, cursor;   // rows grouped by centroid
+    PSB_TRY(order.reserve(sizeof(int) * (size_t)std::max<int64_t>(n, 1), device, st));
+    PSB_TRY(offsets.reserve(sizeof(int) * ((size_t)k + 1), device, st));
+    PSB_TRY(cursor.reserve(sizeof(int) * (size_t)k, device, st));
     KmeansAccumWs ws;
     ws.order = order.as<int>(); ws.offsets = offsets.as<int>(); ws.cursor = cursor.as<int>();
     PSB_TRY(launch_kmeans_accumulate(d_data, n, dim, d_assign, d_best, k, d_sums, d_counts, d_objective, ws, st));

@@ -602,9 +602,11 @@ __host__ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 // 1. k_km_count:   counts[c] (one int atomic per row) and the objective (one fp64 atomic per CTA)
 // 2. k_km_offsets: exclusive prefix of the counts, one CTA in coalesced rounds
 // 3. k_km_fill:    order[offset[c] + slot] = row (one int atomic per row)
-// 4. k_km_sums:    CTA c sums its rows in fp64, eight rows at a time (one per warp), and writes sums[c][:] - no atomics; a
-//                  group of at most 1,024 rows is sorted first, so that its sum does not depend on the order the slots were taken
-constexpr int kKmSumThreads = 256;
+// 4. k_km_sums:    CTA c sums its rows in fp64, two threads per dimension, and writes sums[c][:]; a group of more than 1,024 rows (the
+//                  nearest of a crowd without a centroid of its own) is cut over kKmSplit CTAs that add atomically, or it alone
+//                  takes most of the pass.  The rows of a group of at most 1,024 are put in order first (each finds its rank among the others: one barrier where a bitonic sort of
+//                  64 rows has 21), so that the sum does not depend on the order the slots were taken
+constexpr int kKmSumThreads = 256, kKmSplit = 8;
 __global__ void k_km_count(const int* __restrict__ assign, const float* __restrict__ best, long long n, int* __restrict__ counts,
                            double* __restrict__ obj) {
     __shared__ double s_part[8];
@@ -647,39 +649,62 @@ __global__ void k_km_fill(const int* __restrict__ assign, long long n, const int
     order[offsets[c] + atomicAdd(&cursor[c], 1)] = (int)i;
 }
 __global__ void __launch_bounds__(kKmSumThreads) k_km_sums(const float* __restrict__ data, int dim, const int* __restrict__ offsets,
-                                                           int* __restrict__ order, double* __restrict__ sums) {
-    __shared__ int s_rows[1024];
-    __shared__ double s_part[kKmSumThreads / 32][256];
+                                                           const int* __restrict__ order, double* __restrict__ sums) {
+    __shared__ int s_in[1024], s_rows[1024];
+    __shared__ double s_part[kKmSumThreads / 2];
     const int c = blockIdx.x;
-    const int b0 = offsets[c], cnt = offsets[c + 1] - b0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int b0 = offsets[c], cnt = offsets[c + 1] - b0;
+    const bool split = cnt > 1024;
+    if (split) {
+        const int b = (int)((long long)cnt * blockIdx.y / kKmSplit), e = (int)((long long)cnt * (blockIdx.y + 1) / kKmSplit);
+        b0 += b; cnt = e - b;
+    } else if (blockIdx.y) {
+        return;
+    }
     const int* rows = order + b0;
-    if (cnt > 1 && cnt <= 1024) {   // canonical order for the usual, small group
-        int np = 2;
-        while (np < cnt) np <<= 1;
-        for (int i = threadIdx.x; i < np; i += blockDim.x) s_rows[i] = i < cnt ? rows[i] : 0x7fffffff;
+    if (!split && cnt > 1) {   // canonical order for the usual, small group
+        for (int i = threadIdx.x; i < cnt; i += kKmSumThreads) s_in[i] = rows[i];
         __syncthreads();
-        block_bitonic_sort(s_rows, np);
+        for (int i = threadIdx.x; i < cnt; i += kKmSumThreads) {
+            const int mine = s_in[i];
+            int rank = 0;
+            for (int j = 0; j < cnt; ++j) rank += s_in[j] < mine ? 1 : 0;
+            s_rows[rank] = mine;
+        }
+        __syncthreads();
         rows = s_rows;
     }
-    for (int d0 = 0; d0 < dim; d0 += 256) {   // 256 dimensions at a time: eight per lane
-        double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int j = warp; j < cnt; j += kKmSumThreads / 32) {
-            const float* x = data + (size_t)rows[j] * dim + d0;
+    constexpr int kHalf = kKmSumThreads / 2;
+    const int half = threadIdx.x / kHalf;   // even and odd rows
+    for (int d0 = 0; d0 < dim; d0 += kHalf) {
+        const int d = d0 + (threadIdx.x - half * kHalf);
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        if (d < dim) {
+            const float* x = data + d;
+            int j = half;
+            for (; j + 30 < cnt; j += 32) {   // sixteen loads in flight
+                float v[16];
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                const int d = lane + 32 * t;
-                if (d0 + d < dim) acc[t] += (double)x[d];
+                for (int t = 0; t < 16; ++t) v[t] = __ldg(x + (size_t)rows[j + 2 * t] * dim);
+#pragma unroll
+                for (int t = 0; t < 16; ++t) acc[t & 3] += (double)v[t];
             }
+            for (; j + 6 < cnt; j += 8) {
+                float v[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) v[t] = __ldg(x + (size_t)rows[j + 2 * t] * dim);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) acc[t] += (double)v[t];
+            }
+            for (; j < cnt; j += 2) acc[0] += (double)__ldg(x + (size_t)rows[j] * dim);
         }
-#pragma unroll
-        for (int t = 0; t < 8; ++t) s_part[warp][lane + 32 * t] = acc[t];
+        const double sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        if (half) s_part[threadIdx.x - kHalf] = sum;
         __syncthreads();
-        for (int d = threadIdx.x; d < 256 && d0 + d < dim; d += blockDim.x) {
-            double t = 0.0;
-#pragma unroll
-            for (int w = 0; w < kKmSumThreads / 32; ++w) t += s_part[w][d];
-            sums[(size_t)c * dim + d0 + d] = t;
+        if (!half && d < dim) {
+            const double total = sum + s_part[threadIdx.x];
+            if (split) atomicAdd(&sums[(size_t)c * dim + d], total);
+            else sums[(size_t)c * dim + d] = total;
         }
         __syncthreads();
     }
@@ -847,7 +872,8 @@ psb_status launch_kmeans_accumulate(const float* d_data, long long n, int dim, c
         count_launch();
         PSB_LAUNCH_CHECK();
     }
-    k_km_sums<<<k, kKmSumThreads, 0, s>>>(d_data, dim, ws.offsets, ws.order, d_sums);
+    PSB_CUDA(cudaMemsetAsync(d_sums, 0, sizeof(double) * (size_t)k * dim, s));   // what the split groups add to
+    k_km_sums<<<dim3((unsigned)k, kKmSplit), kKmSumThreads, 0, s>>>(d_data, dim, ws.offsets, ws.order, d_sums);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
