@@ -3,9 +3,14 @@
 // (distance, id) pairs.  The tensor-core filter in coarse_tc.cu narrows the centroid set first; what it keeps
 // is scored by the kernels here, so results are bit-identical with or without it.
 #include "common.cuh"
+#include "dist_tile.cuh"
 #include "kernels.h"
+#include "select.cuh"
 
 namespace psb {
+
+using namespace tile;
+
 namespace {
 
 constexpr int BQ = 64, BC = 128, KC = 16, kDistThreads = 256;
@@ -62,70 +67,46 @@ k_coarse_dist_exact(const float* __restrict__ queries, int nq, const float* __re
     }
 }
 
-// Per row: the k smallest (value, index) pairs, ascending.  64-bit radix select (8-bit digits, most significant
-// first, stopping as soon as the chosen bucket is taken whole), gather, bitonic sort.
-constexpr int kSelThreads = 512;
-__global__ void __launch_bounds__(kSelThreads)
-k_select_rows(const float* __restrict__ dist, int n, int k, int* __restrict__ out_ids, float* __restrict__ out_dist) {
-    extern __shared__ __align__(16) uint64_t s_sel[];  // [pow2 >= k]
-    __shared__ unsigned int s_hist[256];
-    __shared__ uint64_t s_prefix;
-    __shared__ unsigned int s_rank;
-    __shared__ int s_done, s_cnt;
-    const float* row = dist + (size_t)blockIdx.x * n;
-    if (threadIdx.x == 0) { s_prefix = 0; s_rank = (unsigned)k; s_done = 0; s_cnt = 0; }
-    uint64_t mask = 0;
-    uint64_t cut = KEY_MAX;
-    if (k < n) {
-        for (int pass = 7; pass >= 0; --pass) {
-            const int shift = pass * 8;
-            for (int i = threadIdx.x; i < 256; i += blockDim.x) s_hist[i] = 0;
-            __syncthreads();
-            if (s_done) break;
-            const uint64_t prefix = s_prefix;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                const uint64_t key = make_key(row[i], (uint32_t)i);
-                if ((key & mask) == prefix) atomicAdd(&s_hist[(key >> shift) & 255], 1u);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                unsigned cum = 0;
-                const unsigned rank = s_rank;
-                for (int b = 0; b < 256; ++b) {
-                    const unsigned h = s_hist[b];
-                    if (cum + h >= rank) {
-                        s_prefix = prefix | ((uint64_t)b << shift);
-                        s_rank = rank - cum;
-                        if (h == rank - cum) s_done = 1;  // the whole bucket is selected
-                        break;
-                    }
-                    cum += h;
-                }
-            }
-            mask |= 255ull << shift;
-            __syncthreads();
-        }
-        __syncthreads();
-        // keys <= cut are exactly the k smallest: cut = prefix with every undecided low bit set
-        cut = s_prefix | ~mask;
-    }
-    const int np = next_pow2(max(k, 2));
-    for (int i = threadIdx.x; i < np; i += blockDim.x) s_sel[i] = KEY_MAX;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint64_t key = make_key(row[i], (uint32_t)i);
-        if (key <= cut) {
-            const int slot = atomicAdd(&s_cnt, 1);
-            if (slot < np) s_sel[slot] = key;
+// The same for batches whose BQ x BC tiles do not fill the chip: 32 queries x 64 centroids per CTA of 128 threads (4 x 4 each), all
+// dimensions staged at once by 16-byte loads, one barrier.  A batch of 333 queries x 700 centroids x 100 dimensions is 36 of the large
+// tiles, each a chain of load, barrier and compute steps (38 us); a single query against 1,024 centroids took 24 us the same way.
+__global__ void __launch_bounds__(kSmallThreads)
+k_coarse_dist_small(const float* __restrict__ queries, int nq, const float* __restrict__ centroids, int nlist, int dim, float* __restrict__ dist) {
+    extern __shared__ __align__(16) float s_small[];
+    const int pitch = small_pitch(dim);
+    float* qs = s_small;                  // [SQ][pitch]
+    float* cs = s_small + SQ * pitch;     // [SC][pitch]
+    const int q0 = blockIdx.y * SQ, c0 = blockIdx.x * SC;
+    stage_rows<kSmallThreads>(qs, pitch, queries + (size_t)q0 * dim, min(SQ, nq - q0), dim);
+    stage_rows<kSmallThreads>(cs, pitch, centroids + (size_t)c0 * dim, min(SC, nlist - c0), dim);
+    stage_wait();
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    if (q0 + ty * 4 >= nq) return;
+    float acc[4][4];
+    tile_distances(qs + ty * 4 * pitch, cs + tx * pitch, pitch, dim, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int q = q0 + ty * 4 + i;
+        if (q >= nq) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int c = c0 + tx + 16 * j;
+            if (c < nlist) dist[(size_t)q * nlist + c] = acc[i][j];
         }
     }
-    __syncthreads();
-    block_bitonic_sort(s_sel, np);
+}
+
+// Per row: the k smallest (value, index) pairs, ascending.
+__global__ void __launch_bounds__(sel::kThreads)
+k_select_rows(const float* __restrict__ dist, int n, int k, int buffer, int* __restrict__ out_ids, float* __restrict__ out_dist) {
+    extern __shared__ __align__(16) uint64_t s_sel[];  // [buffer] keys, then the group minima
+    __shared__ sel::Words w;
+    const int keep = sel::smallest(dist + (size_t)blockIdx.x * n, n, k, [](int i) { return (uint32_t)i; }, s_sel, buffer,
+                                   reinterpret_cast<float*>(s_sel + buffer), &w);
     for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        const uint64_t key = s_sel[i];
-        const bool ok = key != KEY_MAX;
-        out_ids[(size_t)blockIdx.x * k + i] = ok ? (int)key_idx(key) : -1;
-        if (out_dist) out_dist[(size_t)blockIdx.x * k + i] = ok ? key_dist(key) : FLT_MAX;
+        const bool ok = i < keep;
+        out_ids[(size_t)blockIdx.x * k + i] = ok ? (int)key_idx(s_sel[i]) : -1;
+        if (out_dist) out_dist[(size_t)blockIdx.x * k + i] = ok ? key_dist(s_sel[i]) : FLT_MAX;
     }
 }
 
@@ -135,6 +116,17 @@ psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float*
                                     int dim, float* d_dist, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
     dim3 grid((nlist + BC - 1) / BC, (nq + BQ - 1) / BQ);
+    // Small tiles while the large ones would leave SMs without one (two waves of small tiles still beat one of large ones), if
+    // their rows fit.
+    const size_t small = small_tile_bytes(dim);
+    if ((long long)grid.x * grid.y < 148 && small <= (size_t)200 * 1024) {
+        const dim3 g2((nlist + SC - 1) / SC, (nq + SQ - 1) / SQ);
+        PSB_CUDA(cudaFuncSetAttribute(k_coarse_dist_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small));
+        k_coarse_dist_small<<<g2, kSmallThreads, small, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        return PSB_OK;
+    }
     k_coarse_dist_exact<<<grid, kDistThreads, 0, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist);
     count_launch();
     PSB_LAUNCH_CHECK();
@@ -144,9 +136,9 @@ psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float*
 psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_ids, float* d_out, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
     if (k <= 0 || k > kMaxProbe) return fail(PSB_UNSUPPORTED_SHAPE, "row selection supports 1..4096 results");
-    int np = 2;
-    while (np < k) np <<= 1;
-    k_select_rows<<<nq, kSelThreads, (size_t)np * sizeof(uint64_t), s>>>(d_dist, n, k, d_ids, d_out);
+    const size_t smem = sel::shared_bytes(k);
+    PSB_CUDA(cudaFuncSetAttribute(k_select_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_select_rows<<<nq, sel::kThreads, smem, s>>>(d_dist, n, k, sel::buffer_entries(k), d_ids, d_out);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

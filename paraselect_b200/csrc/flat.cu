@@ -1,187 +1,246 @@
 // IVF-Flat fine scan over device-resident rows: for every query the exact fp32 squared L2 distance to every row of its
-// probed lists, and the topk nearest by (distance, row).
+// probed lists, and the topk nearest by (distance, row), as original ids.
 //
-// One CTA per query.  Rows are staged through shared memory in tiles (coalesced loads, one padded row per thread afterwards),
-// each thread sums one row in the CPU path's arithmetic - sequential, sub / mul / add without FMA, the reference's
-// l2_distance_squared (src/cpu/utils/cpu_distance.h:74-81) - and a running top-k keeps the best: keys below the current cutoff
-// are appended to a buffer that is sorted and cut back to topk whenever it could overflow.  Results equal the reference's
-// cpu_ivf_search (src/cpu/search/cpu_search.h:226-332) with ties by row; the kernel reads each probed row once per visiting
-// query, so its bound is HBM: bytes = sum over (query, probe) of rows * dim * 4.
+// Two halves with a distance row per query between them.  The distances: every (query, probe) pair owns a stretch of the query's
+// row; when lists have enough visitors they are computed list by list in tiles of 32 visiting queries x 64 rows (dist_tile.cuh), so
+// that a list's rows are read once per 32 visitors and the arithmetic - sequential, sub / mul / add without FMA, the reference's
+// l2_distance_squared (src/cpu/utils/cpu_distance.h:74-81) - runs at its issue limit; with few visitors a thread takes one row of
+// one query and the rows of a query are spread over the whole chip.  The selection reads each query's distances twice (select.cuh).
+// One CTA per query that did both took 872 us for 1,000 queries x 16 lists of 390 rows x 128 (L2 traffic of every visit) and
+// 573 us for 4 queries (four CTAs).  Results equal the reference's cpu_ivf_search (src/cpu/search/cpu_search.h:226-332) with ties
+// by row.
 //
 // Reference counterpart: the GPU-resident fine kernels of src/search/kernels/fine/gpu_fine/resident/resident_full_l2_topk.cu:19-178
 // behind ivfflat_search (src/search/ivfflat/ivfflat_search.cuh:41-51).
+#include <algorithm>
+
 #include "common.cuh"
+#include "dist_tile.cuh"
 #include "kernels.h"
+#include "scan_common.cuh"
+#include "select.cuh"
 
 namespace psb {
+
+using namespace tile;
+
 namespace {
 
-constexpr int kFlatThreads = 256;
-constexpr int kFlatTile = 128;  // rows per shared-memory tile
-
-__global__ void __launch_bounds__(kFlatThreads)
-k_flat_scan(const float* __restrict__ queries, int dim, const int* __restrict__ probes, int nprobe,
-            const long long* __restrict__ offsets, int nlist, const float* __restrict__ rows, long long row_base, int topk,
-            int buf_n, int* __restrict__ out_rows, float* __restrict__ out_dist, unsigned long long* __restrict__ counters) {
-    extern __shared__ __align__(16) unsigned char s_flat[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_flat);                         // [buf_n]
-    float* s_q = reinterpret_cast<float*>(s_flat + (size_t)buf_n * 8);             // [dim]
-    float* s_tile = s_q + ((dim + 3) & ~3);                                         // [kFlatTile][dim + 1]
-    __shared__ int s_cnt;
-    __shared__ uint64_t s_cut;
-    const int q = blockIdx.x;
-    const int pitch = dim + 1;
-    for (int d = threadIdx.x; d < dim; d += blockDim.x) s_q[d] = queries[(size_t)q * dim + d];
-    if (threadIdx.x == 0) { s_cnt = 0; s_cut = KEY_MAX; }
-    __syncthreads();
-    long long scanned = 0;
-    for (int p = 0; p < nprobe; ++p) {
-        const int l = probes[(size_t)q * nprobe + p];
-        if (l < 0 || l >= nlist) continue;  // uniform
-        const long long b = offsets[l], e = offsets[l + 1];
-        scanned += e - b;
-        for (long long r0 = b; r0 < e; r0 += kFlatTile) {
-            const int n = (int)min((long long)kFlatTile, e - r0);
-            const float* src = rows + (size_t)(r0 - row_base) * dim;
-            for (int i = threadIdx.x; i < n * dim; i += blockDim.x) s_tile[(i / dim) * pitch + (i % dim)] = __ldg(src + i);
-            const int c_now = s_cnt;  // stable since the barrier that ended the previous tile
-            __syncthreads();
-            if (c_now + kFlatTile > buf_n) {  // uniform
-                for (int i = c_now + threadIdx.x; i < buf_n; i += blockDim.x) s_keys[i] = KEY_MAX;
-                __syncthreads();
-                block_bitonic_sort(s_keys, buf_n);
-                if (threadIdx.x == 0) {
-                    const int keep = c_now < topk ? c_now : topk;
-                    s_cnt = keep;
-                    s_cut = keep == topk ? s_keys[topk - 1] : KEY_MAX;
-                }
-                __syncthreads();
-            }
-            if (threadIdx.x < n) {
-                const float* t = s_tile + threadIdx.x * pitch;
-                float sum = 0.0f;
-                for (int d = 0; d < dim; ++d) {
-                    const float diff = __fsub_rn(s_q[d], t[d]);
-                    sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                }
-                const uint64_t key = make_key(sum, (uint32_t)(r0 + threadIdx.x));
-                if (key < s_cut) s_keys[atomicAdd(&s_cnt, 1)] = key;
-            }
-            __syncthreads();
+// One warp per query: where each probe's distances start in the query's row, the rows it scans, and (list form) the pair's place
+// among its list's visitors.
+__global__ void __launch_bounds__(128) k_flat_pairs(const int* __restrict__ probes, int nq, int nprobe, const long long* __restrict__ offsets, int nlist,
+                                                    int* __restrict__ seg, int* __restrict__ vis_count, int* __restrict__ slot,
+                                                    unsigned long long* __restrict__ counters) {
+    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (q >= nq) return;
+    int* s = seg + (size_t)q * (nprobe + 1);
+    int carry = 0;
+    for (int p0 = 0; p0 < nprobe; p0 += 32) {
+        const int p = p0 + lane;
+        int len = 0, l = -1;
+        if (p < nprobe) {
+            l = probes[(size_t)q * nprobe + p];
+            if (l >= 0 && l < nlist) len = (int)(offsets[l + 1] - offsets[l]); else l = -1;
         }
+        int in = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int up = __shfl_up_sync(0xffffffffu, in, o); if (lane >= o) in += up; }
+        if (p < nprobe) {
+            s[p] = carry + in - len;
+            if (slot) slot[(size_t)q * nprobe + p] = l >= 0 ? atomicAdd(&vis_count[l], 1) : -1;
+        }
+        carry += __shfl_sync(0xffffffffu, in, 31);
     }
-    const int c = s_cnt;
-    for (int i = c + threadIdx.x; i < buf_n; i += blockDim.x) s_keys[i] = KEY_MAX;
-    __syncthreads();
-    block_bitonic_sort(s_keys, buf_n);
-    for (int i = threadIdx.x; i < topk; i += blockDim.x) {
-        const uint64_t key = s_keys[i];
-        const bool ok = key != KEY_MAX;
-        out_rows[(size_t)q * topk + i] = ok ? (int)key_idx(key) : -1;
-        out_dist[(size_t)q * topk + i] = ok ? key_dist(key) : FLT_MAX;
+    if (lane == 0) {
+        s[nprobe] = carry;
+        if (counters) atomicAdd(&counters[0], (unsigned long long)carry);
     }
-    if (threadIdx.x == 0 && counters) atomicAdd(&counters[0], (unsigned long long)scanned);
 }
 
-// The same scan without the shared-memory tile, for dim % 4 == 0 and 16-byte aligned rows: every thread reads its own row
-// straight from global memory with 16-byte loads (a row is a run of whole 128-byte lines, and the lines of a warp's 32 rows
-// stay in L1 from one load to the next), so all 256 threads score rows, nothing is staged and re-read, and a step needs
-// barriers only for the key buffer.  Same arithmetic in the same order, same keys.
-constexpr int kFlatStep = kFlatThreads;   // rows per step
-__global__ void __launch_bounds__(kFlatThreads)
-k_flat_scan_direct(const float* __restrict__ queries, int dim, const int* __restrict__ probes, int nprobe,
-                   const long long* __restrict__ offsets, int nlist, const float* __restrict__ rows, long long row_base, int topk,
-                   int buf_n, int* __restrict__ out_rows, float* __restrict__ out_dist, unsigned long long* __restrict__ counters) {
-    extern __shared__ __align__(16) unsigned char s_flat[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_flat);                         // [buf_n]
-    float4* s_q = reinterpret_cast<float4*>(s_flat + (size_t)buf_n * 8);           // [dim / 4]
-    __shared__ int s_cnt;
-    __shared__ uint64_t s_cut;
-    const int q = blockIdx.x;
-    const int dim4 = dim >> 2;
-    for (int d = threadIdx.x; d < dim4; d += blockDim.x) s_q[d] = reinterpret_cast<const float4*>(queries + (size_t)q * dim)[d];
-    if (threadIdx.x == 0) { s_cnt = 0; s_cut = KEY_MAX; }
-    __syncthreads();
-    long long scanned = 0;
-    for (int p = 0; p < nprobe; ++p) {
-        const int l = probes[(size_t)q * nprobe + p];
-        if (l < 0 || l >= nlist) continue;  // uniform
-        const long long b = offsets[l], e = offsets[l + 1];
-        scanned += e - b;
-        for (long long r0 = b; r0 < e; r0 += kFlatStep) {
-            const int c_now = s_cnt;  // stable since the barrier that ended the previous step
-            __syncthreads();
-            if (c_now + kFlatStep > buf_n) {  // uniform
-                for (int i = c_now + threadIdx.x; i < buf_n; i += blockDim.x) s_keys[i] = KEY_MAX;
-                __syncthreads();
-                block_bitonic_sort(s_keys, buf_n);
-                if (threadIdx.x == 0) {
-                    const int keep = c_now < topk ? c_now : topk;
-                    s_cnt = keep;
-                    s_cut = keep == topk ? s_keys[topk - 1] : KEY_MAX;
-                }
-                __syncthreads();
+// Single CTA: exclusive scans over the lists (visitor offsets, tiles).
+__global__ void __launch_bounds__(1024) k_flat_lists(const int* __restrict__ vis_count, const long long* __restrict__ offsets, int nlist,
+                                                     int* __restrict__ vis_off, long long* __restrict__ item_off) {
+    __shared__ int s_warp[32];
+    __shared__ int s_total;
+    __shared__ long long s_items[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;
+    long long items = 0;
+    for (int base = 0; base < nlist; base += blockDim.x) {
+        const int l = base + threadIdx.x;
+        const int v = l < nlist ? vis_count[l] : 0;
+        const long long len = l < nlist ? offsets[l + 1] - offsets[l] : 0;
+        const long long it = (long long)((v + SQ - 1) / SQ) * ((len + SC - 1) / SC);
+        const int ex = block_exclusive_scan(v, s_warp, &s_total);
+        long long in = it;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const long long up = __shfl_up_sync(0xffffffffu, in, o); if (lane >= o) in += up; }
+        if (lane == 31) s_items[warp] = in;
+        __syncthreads();
+        long long before = 0, all = 0;
+        for (int w = 0; w < 32; ++w) { const long long x = s_items[w]; if (w < warp) before += x; all += x; }
+        if (l < nlist) { vis_off[l] = carry + ex; item_off[l] = items + before + in - it; }
+        carry += s_total;
+        items += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) { vis_off[nlist] = carry; item_off[nlist] = items; }
+}
+
+__global__ void k_flat_visitors(const int* __restrict__ probes, long long pairs, const int* __restrict__ slot, const int* __restrict__ vis_off,
+                                int* __restrict__ visitors) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= pairs || slot[i] < 0) return;
+    visitors[vis_off[probes[i]] + slot[i]] = (int)i;
+}
+
+// Persistent CTAs over the tiles: (list, 32 of its visitors, 64 of its rows).
+__global__ void __launch_bounds__(kSmallThreads)
+k_flat_tiles(const float* __restrict__ queries, int dim, int nprobe, const long long* __restrict__ offsets, int nlist, const float* __restrict__ rows,
+             const int* __restrict__ vis_off, const long long* __restrict__ item_off, const int* __restrict__ visitors, const int* __restrict__ seg,
+             long long stride, float* __restrict__ dist) {
+    extern __shared__ __align__(16) float s_flat[];
+    __shared__ int s_list, s_pair[SQ];
+    __shared__ long long s_dst[SQ];
+    const int pitch = small_pitch(dim);
+    float* qs = s_flat;
+    float* cs = s_flat + SQ * pitch;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long total = item_off[nlist];
+    const bool vec = rows_vec(queries, dim);
+    for (long long item = blockIdx.x; item < total; item += gridDim.x) {
+        __syncthreads();   // the previous tile is done with shared memory
+        if (warp == 0) { const int l = scan::find_list(item_off, nlist, item); if (lane == 0) s_list = l; }
+        __syncthreads();
+        const int l = s_list;
+        const int v0 = vis_off[l], nvis = vis_off[l + 1] - v0;
+        const int groups = (nvis + SQ - 1) / SQ;
+        const long long local = item - item_off[l];
+        const int g = (int)(local % groups);
+        const long long r0 = local / groups * SC, len = offsets[l + 1] - offsets[l];
+        const int nv = min(SQ, nvis - g * SQ), nr = (int)min((long long)SC, len - r0);
+        if (threadIdx.x < SQ) {
+            const int pair = threadIdx.x < nv ? visitors[v0 + g * SQ + threadIdx.x] : -1;
+            s_pair[threadIdx.x] = pair;
+            if (pair >= 0) { const int q = pair / nprobe; s_dst[threadIdx.x] = (long long)q * stride + seg[(size_t)q * (nprobe + 1) + (pair - q * nprobe)] + r0; }
+        }
+        stage_rows<kSmallThreads>(cs, pitch, rows + (size_t)(offsets[l] + r0) * dim, nr, dim);
+        __syncthreads();
+        for (int i = warp; i < nv; i += kSmallThreads / 32) stage_row(qs + i * pitch, queries + (size_t)(s_pair[i] / nprobe) * dim, dim, vec, lane);
+        stage_wait();
+        if (ty * 4 < nv) {
+            float acc[4][4];
+            tile_distances(qs + ty * 4 * pitch, cs + tx * pitch, pitch, dim, acc);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (ty * 4 + i >= nv) continue;
+                float* out = dist + s_dst[ty * 4 + i];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) if (tx + 16 * j < nr) out[tx + 16 * j] = acc[i][j];
             }
-            const uint64_t cut = s_cut;
-            const long long row = r0 + threadIdx.x;
-            if (row < e) {
-                const float4* src = reinterpret_cast<const float4*>(rows + (size_t)(row - row_base) * dim);
-                float sum = 0.0f;
-#pragma unroll 8
-                for (int d = 0; d < dim4; ++d) {
-                    const float4 v = __ldg(src + d);
-                    const float4 qv = s_q[d];
-                    float diff = __fsub_rn(qv.x, v.x); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                    diff = __fsub_rn(qv.y, v.y); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                    diff = __fsub_rn(qv.z, v.z); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                    diff = __fsub_rn(qv.w, v.w); sum = __fadd_rn(sum, __fmul_rn(diff, diff));
-                }
-                const uint64_t key = make_key(sum, (uint32_t)row);
-                if (key < cut) s_keys[atomicAdd(&s_cnt, 1)] = key;
-            }
-            __syncthreads();
         }
     }
-    const int c = s_cnt;
-    for (int i = c + threadIdx.x; i < buf_n; i += blockDim.x) s_keys[i] = KEY_MAX;
+}
+
+// Few visitors per list: a thread per (query, row).  grid (row blocks, queries).
+__global__ void __launch_bounds__(128)
+k_flat_rows(const float* __restrict__ queries, int dim, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
+            const float* __restrict__ rows, const int* __restrict__ seg, long long stride, float* __restrict__ dist) {
+    extern __shared__ __align__(16) float s_q[];
+    const int q = blockIdx.y;
+    const int* s = seg + (size_t)q * (nprobe + 1);
+    const int n = s[nprobe];
+    if ((int)(blockIdx.x * 128) >= n) return;
+    for (int d = threadIdx.x; d < dim; d += 128) s_q[d] = queries[(size_t)q * dim + d];
     __syncthreads();
-    block_bitonic_sort(s_keys, buf_n);
-    for (int i = threadIdx.x; i < topk; i += blockDim.x) {
-        const uint64_t key = s_keys[i];
-        const bool ok = key != KEY_MAX;
-        out_rows[(size_t)q * topk + i] = ok ? (int)key_idx(key) : -1;
-        out_dist[(size_t)q * topk + i] = ok ? key_dist(key) : FLT_MAX;
+    const bool vec = rows_vec(rows, dim);
+    for (int i = blockIdx.x * 128 + threadIdx.x; i < n; i += gridDim.x * 128) {
+        int lo = 0, hi = nprobe;   // largest p with s[p] <= i
+        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
+        const float* x = rows + (size_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo])) * dim;
+        float sum = 0.0f;
+        if (vec) {
+#pragma unroll 8
+            for (int d = 0; d < dim; d += 4) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(x + d));
+                const float4 y = *reinterpret_cast<const float4*>(s_q + d);
+                float t = __fsub_rn(y.x, v.x); sum = __fadd_rn(sum, __fmul_rn(t, t));
+                t = __fsub_rn(y.y, v.y); sum = __fadd_rn(sum, __fmul_rn(t, t));
+                t = __fsub_rn(y.z, v.z); sum = __fadd_rn(sum, __fmul_rn(t, t));
+                t = __fsub_rn(y.w, v.w); sum = __fadd_rn(sum, __fmul_rn(t, t));
+            }
+        } else {
+#pragma unroll 8
+            for (int d = 0; d < dim; ++d) { const float t = __fsub_rn(s_q[d], __ldg(x + d)); sum = __fadd_rn(sum, __fmul_rn(t, t)); }
+        }
+        dist[(size_t)q * stride + i] = sum;
     }
-    if (threadIdx.x == 0 && counters) atomicAdd(&counters[0], (unsigned long long)scanned);
+}
+
+// One CTA per query: the topk nearest of its distances, ties by row; original ids out.
+__global__ void __launch_bounds__(sel::kThreads)
+k_flat_select(const float* __restrict__ dist, long long stride, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
+              const int* __restrict__ seg, int topk, int buffer, const long long* __restrict__ ids, long long* __restrict__ out_ids,
+              float* __restrict__ out_dist) {
+    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, then the group minima
+    __shared__ sel::Words w;
+    const int q = blockIdx.x;
+    const int* s = seg + (size_t)q * (nprobe + 1);
+    auto row_of = [&](int i) -> uint32_t {
+        int lo = 0, hi = nprobe;
+        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
+        return (uint32_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo]));
+    };
+    const int keep = sel::smallest(dist + (size_t)q * stride, s[nprobe], topk, row_of, s_key, buffer, reinterpret_cast<float*>(s_key + buffer), &w);
+    for (int i = threadIdx.x; i < topk; i += sel::kThreads) {
+        const bool ok = i < keep;
+        out_ids[(size_t)q * topk + i] = ok ? ids[key_idx(s_key[i])] : -1;
+        out_dist[(size_t)q * topk + i] = ok ? key_dist(s_key[i]) : FLT_MAX;
+    }
 }
 
 }  // namespace
 
-psb_status launch_flat_scan(const float* d_queries, int nq, int dim, const int* d_probes, int nprobe, const long long* d_offsets,
-                            int nlist, const float* d_rows, long long row_base, int topk, int* d_out_rows, float* d_out_dist,
-                            unsigned long long* d_counters, cudaStream_t s) {
+bool flat_list_form(int nq, int nprobe, int nlist, int dim) {
+    // From eight visitors per list on, a tile's rows serve enough queries to be worth the schedule's three small kernels; the tile's
+    // rows have to fit.
+    return (long long)nq * nprobe >= 8ll * nlist && small_tile_bytes(dim) <= (size_t)200 * 1024;
+}
+
+psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
-    if (topk <= 0 || topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "flat scan supports topk in 1..2048");
-    if (dim % 4 == 0 && reinterpret_cast<uintptr_t>(d_rows) % 16 == 0 && reinterpret_cast<uintptr_t>(d_queries) % 16 == 0) {
-        int buf = 1024;
-        while (buf < topk + kFlatStep) buf <<= 1;
-        const size_t bytes = (size_t)buf * 8 + (size_t)dim * 4;
-        if (bytes <= (size_t)220 * 1024) {
-            if (bytes > 32 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_flat_scan_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-            k_flat_scan_direct<<<nq, kFlatThreads, bytes, s>>>(d_queries, dim, d_probes, nprobe, d_offsets, nlist, d_rows, row_base, topk,
-                                                               buf, d_out_rows, d_out_dist, d_counters);
-            count_launch();
-            PSB_LAUNCH_CHECK();
-            return PSB_OK;
-        }
+    if (f.topk <= 0 || f.topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "flat scan supports topk in 1..2048");
+    const bool lists = flat_list_form(nq, f.nprobe, f.nlist, f.dim);
+    const long long pairs = (long long)nq * f.nprobe;
+    if (lists) PSB_CUDA(cudaMemsetAsync(f.vis_count, 0, sizeof(int) * (size_t)f.nlist, s));
+    k_flat_pairs<<<(unsigned)((nq + 3) / 4), 128, 0, s>>>(f.probes, nq, f.nprobe, f.offsets, f.nlist, f.seg, f.vis_count, lists ? f.slot : nullptr, f.counters);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    if (lists) {
+        k_flat_lists<<<1, 1024, 0, s>>>(f.vis_count, f.offsets, f.nlist, f.vis_off, f.item_off);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        k_flat_visitors<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(f.probes, pairs, f.slot, f.vis_off, f.visitors);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        const size_t smem = small_tile_bytes(f.dim);
+        PSB_CUDA(cudaFuncSetAttribute(k_flat_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)220 * 1024 / (smem + 1024)));
+        k_flat_tiles<<<(unsigned)(f.sm_count * per_sm), kSmallThreads, smem, s>>>(f.queries, f.dim, f.nprobe, f.offsets, f.nlist, f.rows, f.vis_off,
+                                                                                  f.item_off, f.visitors, f.seg, f.stride, f.dist);
+    } else {
+        const long long blocks = std::min<long long>((f.stride + 127) / 128, 8192);
+        const size_t smem = (size_t)((f.dim + 3) & ~3) * sizeof(float);
+        if (smem > 48 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_flat_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_flat_rows<<<dim3((unsigned)std::max<long long>(1, blocks), (unsigned)nq), 128, smem, s>>>(f.queries, f.dim, f.probes, f.nprobe, f.offsets, f.rows,
+                                                                                                    f.seg, f.stride, f.dist);
     }
-    int buf_n = 1024;
-    while (buf_n < topk + kFlatTile) buf_n <<= 1;
-    const size_t smem = (size_t)buf_n * 8 + (size_t)((dim + 3) & ~3) * 4 + (size_t)kFlatTile * (dim + 1) * 4;
-    if (smem > (size_t)220 * 1024) return fail(PSB_UNSUPPORTED_SHAPE, "flat scan: dim too large for the shared-memory tile");
-    if (smem > 32 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_flat_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_flat_scan<<<nq, kFlatThreads, smem, s>>>(d_queries, dim, d_probes, nprobe, d_offsets, nlist, d_rows, row_base, topk, buf_n,
-                                               d_out_rows, d_out_dist, d_counters);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    const size_t smem = sel::shared_bytes(f.topk);
+    PSB_CUDA(cudaFuncSetAttribute(k_flat_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_flat_select<<<nq, sel::kThreads, smem, s>>>(f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids,
+                                                  f.out_dist);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

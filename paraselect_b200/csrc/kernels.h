@@ -248,10 +248,23 @@ psb_status launch_scan(const ScanIndex& ix, const ScanWorkspace& ws, const float
 
 // ---- IVF-Flat fine scan (flat.cu) ------------------------------------------------------------------------------
 // Exact fp32 distances of every query to the rows of its probed lists (device-resident rows, list-contiguous) and the topk
-// nearest by (distance, row).  d_out_rows [nq][topk] list-contiguous rows (-1 pad), d_out_dist (FLT_MAX pad).
-psb_status launch_flat_scan(const float* d_queries, int nq, int dim, const int* d_probes, int nprobe, const long long* d_offsets,
-                            int nlist, const float* d_rows, long long row_base, int topk, int* d_out_rows, float* d_out_dist,
-                            unsigned long long* d_counters, cudaStream_t s);
+// nearest by (distance, row), as original ids (-1 / FLT_MAX pad).
+struct FlatScan {
+    const float* queries; int dim;             // [nq][dim]
+    const int* probes; int nprobe;             // [nq][nprobe] list ids (outside [0, nlist): skipped)
+    const long long* offsets; int nlist;       // [nlist + 1]
+    const float* rows; const long long* ids;   // [n][dim], [n]
+    int topk;
+    long long* out_ids; float* out_dist;       // [nq][topk]
+    float* dist; long long stride;             // [nq][stride] workspace, stride >= the rows of any nprobe lists
+    int* seg;                                  // [nq][nprobe + 1]
+    // list form only (flat_list_form): [nlist], [nq * nprobe], [nlist + 1], [nlist + 1], [nq * nprobe]
+    int* vis_count; int* slot; int* vis_off; long long* item_off; int* visitors;
+    unsigned long long* counters;
+    int sm_count;
+};
+bool flat_list_form(int nq, int nprobe, int nlist, int dim);
+psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s);
 
 // ---- rerank ------------------------------------------------------------------------------------------------
 // Which rows of the index-wide (list-contiguous) numbering a session's exact store and id table hold.

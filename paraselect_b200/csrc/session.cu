@@ -316,7 +316,8 @@ struct psb_session {
     DevBuf opq, q_rot;                     // OPQ rotation [dim][dim] and the rotated queries of the batch in flight
     bool row_bias_is_u16 = false;          // row_bias holds the caller's affine u16 row correction
     bool flat = false;                     // IVF-Flat session: exact rows resident in flat_rows, no PQ parts
-    DevBuf flat_rows;
+    DevBuf flat_rows, flat_dist, flat_seg, flat_slot;
+    std::vector<long long> flat_longest;   // [p] = rows of the p longest lists together
     std::unique_ptr<HostPool> host_pool;   // gather threads of the staged transport (created on first use)
     double staged_gather_s = 0.0;          // host time spent gathering rows, and the bytes gathered (reported by the bench)
     long long staged_gather_bytes = 0;
@@ -1641,6 +1642,13 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
         PSB_CUDA(cudaMemcpyAsync(s->reordered.p, index->lists.reordered_ids, sizeof(long long) * n, cudaMemcpyHostToDevice, st));
         PSB_CUDA(cudaMemcpyAsync(s->flat_rows.p, index->rowmajor_fp32, sizeof(float) * n * s->dim, cudaMemcpyHostToDevice, st));
     }
+    {
+        std::vector<long long> len(nl);
+        for (size_t l = 0; l < nl; ++l) len[l] = index->lists.offsets[l + 1] - index->lists.offsets[l];
+        std::sort(len.begin(), len.end(), std::greater<long long>());
+        s->flat_longest.assign(nl + 1, 0);
+        for (size_t l = 0; l < nl; ++l) s->flat_longest[l + 1] = s->flat_longest[l] + len[l];
+    }
     PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
     PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, st));
     PSB_CUDA(cudaStreamSynchronize(st));
@@ -1656,19 +1664,39 @@ psb_status psb_flat_session_destroy(psb_flat_session* s) {
 namespace {
 psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe, int topk, long long* d_ids, float* d_dist) {
     PSB_TRY(s->probes.reserve(sizeof(int) * (size_t)n * nprobe));
-    PSB_TRY(s->out_rows.reserve(sizeof(int) * (size_t)n * topk));
     PSB_TRY(coarse_exact(s, dq, n, nprobe, s->probes.as<int>(), nullptr));
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    if (s->opt.time_kernels) {  // bracket the fine-scan kernel (read back by psb_session_counters)
+    if (s->opt.time_kernels) {  // bracket the fine scan (read back by psb_session_counters)
         PSB_CUDA(cudaEventCreate(&ev0));
         PSB_CUDA(cudaEventCreate(&ev1));
         s->scan_events.emplace_back(ev0, ev1);
         PSB_CUDA(cudaEventRecord(ev0, s->stream));
     }
-    PSB_TRY(launch_flat_scan(dq, n, s->dim, s->probes.as<int>(), nprobe, s->offsets.as<long long>(), s->nlist, s->flat_rows.as<float>(),
-                             0, topk, s->out_rows.as<int>(), d_dist, s->scalars.as<unsigned long long>(), s->stream));
+    // A row of distances per query, as long as the nprobe longest lists; queries in parts of at most 1 GiB of them.
+    FlatScan f{};
+    f.stride = std::max<long long>(1, s->flat_longest[(size_t)nprobe]);
+    const long long most = std::max<long long>(1, std::min<long long>(32768, ((long long)1 << 28) / f.stride));
+    const int parts = (int)((n + most - 1) / most), per = (n + parts - 1) / parts;
+    PSB_TRY(s->flat_dist.reserve(sizeof(float) * (size_t)per * f.stride));
+    PSB_TRY(s->flat_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
+    if (flat_list_form(per, nprobe, s->nlist, s->dim)) {
+        PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
+        PSB_TRY(s->flat_slot.reserve(sizeof(int) * (size_t)per * nprobe));
+        PSB_TRY(s->vis_off.reserve(sizeof(int) * ((size_t)s->nlist + 1)));
+        PSB_TRY(s->item_off.reserve(sizeof(long long) * ((size_t)s->nlist + 1)));
+        PSB_TRY(s->visitors.reserve(sizeof(int) * (size_t)per * nprobe));
+    }
+    f.dim = s->dim; f.nprobe = nprobe; f.offsets = s->offsets.as<long long>(); f.nlist = s->nlist; f.rows = s->flat_rows.as<float>();
+    f.ids = s->reordered.as<long long>(); f.topk = topk; f.dist = s->flat_dist.as<float>(); f.seg = s->flat_seg.as<int>();
+    f.vis_count = s->vis_count.as<int>(); f.slot = s->flat_slot.as<int>(); f.vis_off = s->vis_off.as<int>(); f.item_off = s->item_off.as<long long>();
+    f.visitors = s->visitors.as<int>(); f.counters = s->scalars.as<unsigned long long>(); f.sm_count = s->sm_count;
+    for (int q0 = 0; q0 < n; q0 += per) {
+        f.queries = dq + (size_t)q0 * s->dim; f.probes = s->probes.as<int>() + (size_t)q0 * nprobe;
+        f.out_ids = d_ids + (size_t)q0 * topk; f.out_dist = d_dist + (size_t)q0 * topk;
+        PSB_TRY(launch_flat_scan(f, std::min(per, n - q0), s->stream));
+    }
     if (ev1) PSB_CUDA(cudaEventRecord(ev1, s->stream));
-    return launch_map_ids(s->out_rows.as<int>(), (long long)n * topk, s->reordered.as<long long>(), s->row_map(), d_ids, s->stream);
+    return PSB_OK;
 }
 psb_status flat_check(const psb_session* s, const psb_search_params* p) {
     if (!s || !s->flat) return fail(PSB_INVALID_ARGUMENT, "not an IVF-Flat session");

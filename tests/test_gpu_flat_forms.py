@@ -1,0 +1,40 @@
+"""IVF-Flat: the list form (many visitors per list) and the row form (few), tiles and row blocks that do not fill, dimensions that are no
+multiple of four, and every way the selection can go - all values gathered, cut by the group minima, radix passes for equal values and
+for more results than the minima cover - against the CPU checker."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,dim,nlist,nq,nprobe,topk,values", [
+    (3000, 33, 5, 97, 5, 10, "normal"), (3000, 100, 5, 1, 3, 7, "normal"), (4000, 64, 3, 33, 2, 300, "normal"), (9000, 16, 7, 2, 7, 300, "normal"),
+    (6000, 8, 4, 40, 4, 1100, "normal"), (6000, 8, 4, 3, 4, 2048, "normal"), (7000, 12, 3, 40, 3, 50, "grid"), (5000, 4, 2, 2, 2, 20, "equal"),
+    (64, 300, 2, 20, 2, 5, "normal"), (40, 7, 20, 33, 20, 64, "normal")])
+def test_flat_forms(psb, n, dim, nlist, nq, nprobe, topk, values):
+    rng = np.random.default_rng(n + dim + nq)
+    draw = {"normal": lambda *s: rng.standard_normal(s), "grid": lambda *s: rng.integers(-1, 2, s), "equal": lambda *s: np.ones(s)}[values]
+    cuts = np.sort(rng.integers(0, n + 1, nlist - 1))
+    off = np.concatenate([[0], cuts, [n]]).astype(np.int64)
+    fx = dict(centroids=rng.standard_normal((nlist, dim)).astype(np.float32), offsets=off, reordered_ids=rng.permutation(n).astype(np.int64),
+              vectors=draw(n, dim).astype(np.float32))
+    q = draw(nq, dim).astype(np.float32)
+    wi, wd = oracle.ivfflat_search(fx["centroids"], off, fx["reordered_ids"], fx["vectors"], q, nprobe, topk)
+    with psb.FlatSession(fx) as s:
+        got = s.search(q, nprobe, topk)
+    assert np.array_equal(got["indices"], wi) and np.array_equal(got["distances"], wd)
+
+
+@pytest.mark.parametrize("nq,nlist,dim,k", [(1, 3, 5, 3), (33, 65, 12, 20), (2, 3000, 40, 1), (3, 5000, 8, 700), (40, 513, 6, 130), (2, 9000, 4, 1500)])
+@pytest.mark.parametrize("equal", [False, True])
+def test_coarse_small_batches(psb, nq, nlist, dim, k, equal):
+    rng = np.random.default_rng(nlist)
+    c = rng.standard_normal((nlist, dim)).astype(np.float32)
+    if equal:
+        c[:] = c[0]
+    q = rng.standard_normal((nq, dim)).astype(np.float32)
+    ids, dist = psb.coarse_host(q, c, k, coarse_mode=1)
+    wi, wd = oracle.coarse(q, c, k)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
