@@ -97,11 +97,12 @@ k_coarse_dist_small(const float* __restrict__ queries, int nq, const float* __re
 }
 
 // Per row: the k smallest (value, index) pairs, ascending.
-__global__ void __launch_bounds__(sel::kThreads)
+constexpr int kSelThreads = 256;
+__global__ void __launch_bounds__(kSelThreads)
 k_select_rows(const float* __restrict__ dist, int n, int k, int buffer, int* __restrict__ out_ids, float* __restrict__ out_dist) {
     extern __shared__ __align__(16) uint64_t s_sel[];  // [buffer] keys, then the group minima
     __shared__ sel::Words w;
-    const int keep = sel::smallest(dist + (size_t)blockIdx.x * n, n, k, [](int i) { return (uint32_t)i; }, s_sel, buffer,
+    const int keep = sel::smallest<kSelThreads>(dist + (size_t)blockIdx.x * n, n, k, [](int i) { return (uint32_t)i; }, s_sel, buffer,
                                    reinterpret_cast<float*>(s_sel + buffer), &w);
     for (int i = threadIdx.x; i < k; i += blockDim.x) {
         const bool ok = i < keep;
@@ -138,7 +139,7 @@ psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_
     if (k <= 0 || k > kMaxProbe) return fail(PSB_UNSUPPORTED_SHAPE, "row selection supports 1..4096 results");
     const size_t smem = sel::shared_bytes(k);
     PSB_CUDA(cudaFuncSetAttribute(k_select_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_select_rows<<<nq, sel::kThreads, smem, s>>>(d_dist, n, k, sel::buffer_entries(k), d_ids, d_out);
+    k_select_rows<<<nq, kSelThreads, smem, s>>>(d_dist, n, k, sel::buffer_entries(k), d_ids, d_out);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

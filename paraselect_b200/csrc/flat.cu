@@ -28,7 +28,7 @@ namespace {
 
 // One warp per query: where each probe's distances start in the query's row, the rows it scans, and (list form) the pair's place
 // among its list's visitors.
-__global__ void __launch_bounds__(128) k_flat_pairs(const int* __restrict__ probes, int nq, int nprobe, const long long* __restrict__ offsets, int nlist,
+__global__ void __launch_bounds__(128) k_row_segments(const int* __restrict__ probes, int nq, int nprobe, const long long* __restrict__ offsets, int lb, int le,
                                                     int* __restrict__ seg, int* __restrict__ vis_count, int* __restrict__ slot,
                                                     unsigned long long* __restrict__ counters) {
     const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(128) k_flat_pairs(const int* __restrict__ prob
         int len = 0, l = -1;
         if (p < nprobe) {
             l = probes[(size_t)q * nprobe + p];
-            if (l >= 0 && l < nlist) len = (int)(offsets[l + 1] - offsets[l]); else l = -1;
+            if (l >= lb && l < le) len = (int)(offsets[l + 1] - offsets[l]); else l = -1;
         }
         int in = len;
 #pragma unroll
@@ -178,7 +178,8 @@ k_flat_rows(const float* __restrict__ queries, int dim, const int* __restrict__ 
 }
 
 // One CTA per query: the topk nearest of its distances, ties by row; original ids out.
-__global__ void __launch_bounds__(sel::kThreads)
+template <int T>
+__global__ void __launch_bounds__(T)
 k_flat_select(const float* __restrict__ dist, long long stride, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
               const int* __restrict__ seg, int topk, int buffer, const long long* __restrict__ ids, long long* __restrict__ out_ids,
               float* __restrict__ out_dist) {
@@ -191,8 +192,8 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
         while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
         return (uint32_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo]));
     };
-    const int keep = sel::smallest(dist + (size_t)q * stride, s[nprobe], topk, row_of, s_key, buffer, reinterpret_cast<float*>(s_key + buffer), &w);
-    for (int i = threadIdx.x; i < topk; i += sel::kThreads) {
+    const int keep = sel::smallest<T>(dist + (size_t)q * stride, s[nprobe], topk, row_of, s_key, buffer, reinterpret_cast<float*>(s_key + buffer), &w);
+    for (int i = threadIdx.x; i < topk; i += T) {
         const bool ok = i < keep;
         out_ids[(size_t)q * topk + i] = ok ? ids[key_idx(s_key[i])] : -1;
         out_dist[(size_t)q * topk + i] = ok ? key_dist(s_key[i]) : FLT_MAX;
@@ -200,6 +201,14 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
 }
 
 }  // namespace
+
+psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const long long* d_offsets, int list_begin, int list_end, int* d_seg,
+                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s) {
+    k_row_segments<<<(unsigned)((nq + 3) / 4), 128, 0, s>>>(d_probes, nq, nprobe, d_offsets, list_begin, list_end, d_seg, d_vis_count, d_slot, d_counters);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
 
 bool flat_list_form(int nq, int nprobe, int nlist, int dim) {
     // From eight visitors per list on, a tile's rows serve enough queries to be worth the schedule's three small kernels; the tile's
@@ -213,9 +222,7 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     const bool lists = flat_list_form(nq, f.nprobe, f.nlist, f.dim);
     const long long pairs = (long long)nq * f.nprobe;
     if (lists) PSB_CUDA(cudaMemsetAsync(f.vis_count, 0, sizeof(int) * (size_t)f.nlist, s));
-    k_flat_pairs<<<(unsigned)((nq + 3) / 4), 128, 0, s>>>(f.probes, nq, f.nprobe, f.offsets, f.nlist, f.seg, f.vis_count, lists ? f.slot : nullptr, f.counters);
-    count_launch();
-    PSB_LAUNCH_CHECK();
+    PSB_TRY(launch_row_segments(f.probes, nq, f.nprobe, f.offsets, 0, f.nlist, f.seg, f.vis_count, lists ? f.slot : nullptr, f.counters, s));
     if (lists) {
         k_flat_lists<<<1, 1024, 0, s>>>(f.vis_count, f.offsets, f.nlist, f.vis_off, f.item_off);
         count_launch();
@@ -238,9 +245,14 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     count_launch();
     PSB_LAUNCH_CHECK();
     const size_t smem = sel::shared_bytes(f.topk);
-    PSB_CUDA(cudaFuncSetAttribute(k_flat_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_flat_select<<<nq, sel::kThreads, smem, s>>>(f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids,
-                                                  f.out_dist);
+    auto select = [&](auto kernel, int threads) -> psb_status {   // fewer queries than SMs: large blocks
+        PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<nq, threads, smem, s>>>(f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids,
+                                         f.out_dist);
+        return PSB_OK;
+    };
+    if (nq <= f.sm_count) PSB_TRY(select(k_flat_select<1024>, 1024));
+    else PSB_TRY(select(k_flat_select<256>, 256));
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

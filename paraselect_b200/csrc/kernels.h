@@ -190,6 +190,8 @@ struct ScanIndex {
     int dim = 0;
 };
 
+bool scan_tree_order(const ScanIndex& ix);   // whether ADC sums run as a pairwise tree (residual mode, m = 8 or 16, k = 256)
+
 // ---- tensor-core pre-filter scan (scan_tc.cu) ------------------------------------------------------------------
 // Whether the tensor-core scan supports the shape (dsub 2, 4 or 8, dim a multiple of 8, m of 4, operands within shared memory).
 bool scan_tc_supported(int dim, int m, int k);
@@ -245,6 +247,27 @@ psb_status launch_build_tables_residual(const float* d_queries, int nq, int dim,
 psb_status launch_scan(const ScanIndex& ix, const ScanWorkspace& ws, const float* d_lut, int nq,
                        const int* d_probes, int nprobe, int stage1_k, int* d_rows, float* d_dist,
                        int* d_count, int sm_count, cudaStream_t s, const float* d_queries = nullptr);
+
+// ---- rows of distances (flat.cu, adc_rows.cu) --------------------------------------------------------------------
+// d_seg [nq][nprobe + 1]: where the distances of each probe start in the query's row of distances, then the rows it scans (lists
+// outside [list_begin, list_end) have none).  d_slot (may be null) [nq * nprobe]: the pair's place among its list's visitors, counted in
+// d_vis_count.  d_counters[0] += rows.
+psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const long long* d_offsets, int list_begin, int list_end, int* d_seg,
+                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s);
+// The ADC scan in its row form: all distances, then the stage1_k smallest.
+struct AdcRows {
+    const float* queries; const int* probes; int nprobe;
+    const float* centroids; const float* codebook; const uint8_t* codes; const long long* offsets; long long row_base; const long long* row_delta;
+    int list_begin, list_end, dim, m, k;
+    bool residual, tree;
+    int stage1_k;
+    int* out_rows; float* out_dist; int* out_count;
+    int* seg; float* dist; long long stride;        // workspace: [nq][nprobe + 1], [nq][stride]
+    double expected_rows; long long longest_list;   // rows a query is expected to scan; rows of the longest list
+    unsigned long long* counters;
+    int sm_count;
+};
+psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s);
 
 // ---- IVF-Flat fine scan (flat.cu) ------------------------------------------------------------------------------
 // Exact fp32 distances of every query to the rows of its probed lists (device-resident rows, list-contiguous) and the topk

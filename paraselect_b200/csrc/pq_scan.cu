@@ -1157,7 +1157,7 @@ bool half_scan_fits(int m, int k) {
 
 // The reference's residual CPU scan sums M = 16 and M = 8 (K = 256) rows as a balanced pairwise tree and every other
 // shape sequentially (src/search/ivfrespq/stage/ivfrespq_cpu_rerank.cpp:307-341); the plain mode is always sequential.
-bool tree_order(const ScanIndex& ix) { return ix.residual && ix.k == 256 && (ix.m == 16 || ix.m == 8); }
+bool tree_order(const ScanIndex& ix) { return scan_tree_order(ix); }
 
 template <typename F>
 psb_status set_smem(F kernel, size_t bytes) {
@@ -1256,6 +1256,8 @@ psb_status run_fallback(const ScanIndex& ix, const ScanWorkspace& ws, const floa
     }
 
 }  // namespace
+
+bool scan_tree_order(const ScanIndex& ix) { return ix.residual && ix.k == 256 && (ix.m == 16 || ix.m == 8); }
 
 int seed_record_keys(int stage1_k, float sigma) {
     const float s = sigma >= 6.f && sigma <= 10.f ? sigma : 6.0f;   // the margin of the shared cutoff

@@ -6,8 +6,7 @@
 namespace psb {
 namespace sel {
 
-constexpr int kThreads = 256;     // threads of a selecting block
-constexpr int kMaxGroups = 2048;  // group minima: up to eight per thread
+constexpr int kMaxGroups = 2048;  // group minima
 
 // Entries the key buffer needs: a power of two that holds the keys gathered at the usual cut several times over.
 inline int buffer_entries(int k) { return k <= 256 ? 1024 : (k <= 1024 ? 4096 : 8192); }
@@ -23,7 +22,7 @@ struct Words { unsigned int hist[256]; uint64_t prefix; unsigned int rank; int d
 // that cut are gathered and put in order by rank or, above 256, by a bitonic sort.  A radix selection over the whole keys
 // (up to eight passes with a histogram each, 12 us for 1,024 values and one row) is left for the rows the cut does not serve: too
 // many equal values, fewer than k comparable ones, or k above what the group minima cover.
-template <typename Payload>
+template <int kThreads, typename Payload>   // kThreads: the block's threads, 256 or more
 __device__ int smallest(const float* __restrict__ vals, int n, int k, Payload payload, uint64_t* s_keys, int buffer, float* s_min, Words* w) {
     const int tid = threadIdx.x, lane = tid & 31;
     const float inf = __int_as_float(0x7f800000);
@@ -88,7 +87,7 @@ __device__ int smallest(const float* __restrict__ vals, int n, int k, Payload pa
         __syncthreads();
         for (int pass = 7; pass >= 0; --pass) {
             const int shift = pass * 8;
-            w->hist[tid] = 0;
+            if (tid < 256) w->hist[tid] = 0;
             __syncthreads();
             if (w->done) break;
             const uint64_t prefix = w->prefix;

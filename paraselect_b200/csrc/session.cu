@@ -316,8 +316,10 @@ struct psb_session {
     DevBuf opq, q_rot;                     // OPQ rotation [dim][dim] and the rotated queries of the batch in flight
     bool row_bias_is_u16 = false;          // row_bias holds the caller's affine u16 row correction
     bool flat = false;                     // IVF-Flat session: exact rows resident in flat_rows, no PQ parts
-    DevBuf flat_rows, flat_dist, flat_seg, flat_slot;
-    std::vector<long long> flat_longest;   // [p] = rows of the p longest lists together
+    DevBuf flat_rows, flat_slot;
+    DevBuf row_dist, row_seg;              // a row of distances per query (IVF-Flat, row form of the ADC scan)
+    std::vector<long long> longest;        // [p] = rows of this shard's p longest lists together
+    double own_list_rows = 0.0;            // expected length of the list a random row lies in
     std::unique_ptr<HostPool> host_pool;   // gather threads of the staged transport (created on first use)
     double staged_gather_s = 0.0;          // host time spent gathering rows, and the bytes gathered (reported by the bench)
     long long staged_gather_bytes = 0;
@@ -475,12 +477,44 @@ size_t table_count(const psb_session* s, int nq, int nprobe) {
     return s->opt.adc_mode == 1 ? (size_t)nq * nprobe : (size_t)nq;
 }
 
+void note_list_lengths(psb_session* s, const int64_t* offsets) {
+    std::vector<long long> len;
+    double sq = 0.0;
+    for (int l = s->list_begin; l < s->list_end; ++l) { len.push_back(offsets[l + 1] - offsets[l]); sq += (double)len.back() * (double)len.back(); }
+    std::sort(len.begin(), len.end(), std::greater<long long>());
+    s->longest.assign((size_t)s->nlist + 1, 0);
+    for (size_t p = 0; p < (size_t)s->nlist; ++p) s->longest[p + 1] = s->longest[p] + (p < len.size() ? len[p] : 0);
+    s->own_list_rows = s->shard_rows > 0 ? sq / (double)s->shard_rows : 0.0;
+}
+
+constexpr long long kRowDistFloats = 1ll << 28;   // distances kept at a time in the row forms: 1 GiB
+
+// Rows a query is expected to scan: its own list's, found in proportion to its length, and those of nprobe - 1 others.
+double expected_rows(const psb_session* s, int nprobe) {
+    return std::min((double)s->longest[(size_t)std::min(nprobe, s->nlist)], s->own_list_rows + (nprobe - 1) * (double)s->shard_rows / std::max(1, s->nlist));
+}
+
+// Whether the ADC scan of nq queries takes its row form (adc_rows.cu): when its work - m shared-memory gathers per visited row, 50 G
+// row visits/s at m = 48 - takes less than the list-centric scan's chain of kernels, which costs about 180 us before its first row and
+// runs at 66 G visits/s with the tensor-core filter.  Shapes the filter does not take stay with the row form at any size.
+// any_probes: the caller's own probes, which may name a list more than once.
+long long row_stride(const psb_session* s, int nprobe, bool any_probes) {
+    return std::max<long long>(1, any_probes ? s->longest[1] * nprobe : s->longest[(size_t)nprobe]);
+}
+bool rows_form(const psb_session* s, int nq, int nprobe, bool any_probes = false) {
+    if (s->opt.scan_mode != 0 || s->opt.tc_min_visitors > 1 || s->opt.test_wait_limit || s->opt.test_skip_mma || s->longest.empty()) return false;
+    const long long stride = row_stride(s, nprobe, any_probes);
+    const size_t smem = ((size_t)s->m * s->k + s->dim + nprobe + 1) * 4;
+    if (stride > kRowDistFloats || smem > (size_t)220 * 1024) return false;
+    return s->row_aug.p == nullptr || (double)nq * expected_rows(s, nprobe) * s->m <= 4.8e8;
+}
+
 // Queries per sub-batch of the pipeline: a quarter of the batch when the rerank overlaps the scan, and in residual mode
 // few enough that the per-(query, probe) tables stay below ~16 GiB.
 int sub_batch_rows(const psb_session* s, int n, int nprobe, bool overlap) {
     const int pipeline_parts = s->opt.pipeline_parts >= 2 && s->opt.pipeline_parts <= 32 ? s->opt.pipeline_parts : 4;
     int parts = overlap ? pipeline_parts : 1;
-    if (s->opt.adc_mode == 1 && !residual_table_free(s, stage1_width(s, 1))) {
+    if (s->opt.adc_mode == 1 && !residual_table_free(s, stage1_width(s, 1)) && !rows_form(s, n, nprobe)) {
         const double bytes = (double)n * nprobe * s->m * s->k * sizeof(float);
         parts = std::max(parts, (int)std::ceil(bytes / (16.0 * 1024 * 1024 * 1024)));
     }
@@ -496,7 +530,8 @@ bool overlap_enabled(const psb_session* s, int n, bool rerank) {
 }
 
 // Grows the scan workspace to hold nq queries (never shrinks; a growing buffer is freed first, which waits for the device).
-psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k) {
+// own_tables: the scan's row form takes this call (it needs no tables).
+psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool own_tables) {
     const size_t tables = table_count(s, nq, nprobe);
     s->ws_scan_queries = 0; s->ws_scan_tables = 0;  // set again below once every buffer has its size
     PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
@@ -513,7 +548,7 @@ psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k) {
     s->pool_cap = cap;
     PSB_TRY(s->fail_list.reserve(sizeof(int) * (size_t)nq));
     PSB_TRY(s->fallback_partial.reserve(fallback_partial_bytes(stage1_k)));
-    const bool half_tables = s->opt.scan_mode != 1 && !residual_table_free(s, stage1_k);
+    const bool half_tables = s->opt.scan_mode != 1 && !residual_table_free(s, stage1_k) && !own_tables;
     if (half_tables) {
         PSB_TRY(s->lut_h.reserve(sizeof(unsigned short) * tables * s->m * s->k));
         PSB_TRY(s->lut_scale.reserve(sizeof(float) * tables));
@@ -533,19 +568,46 @@ psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k) {
     return PSB_OK;
 }
 
+// The ADC scan of one sub-batch.  d_lut may be null in the row form (it builds its tables in shared memory) and as launch_scan allows.
+psb_status run_scan(psb_session* s, const ScanWorkspace& ws, const float* d_queries, const float* d_lut, int nq, const int* d_probes, int nprobe,
+                    int stage1_k, int* d_rows, float* d_dist, int* d_count, cudaStream_t st, bool any_probes = false) {
+    if (!d_queries || ws.phase != 0 || !rows_form(s, nq, nprobe, any_probes))
+        return launch_scan(s->scan_index(), ws, d_lut, nq, d_probes, nprobe, stage1_k, d_rows, d_dist, d_count, s->sm_count, st, d_queries);
+    AdcRows g{};
+    g.stride = row_stride(s, nprobe, any_probes);
+    const int most = (int)std::max<long long>(1, std::min<long long>(32768, kRowDistFloats / g.stride));
+    const int parts = (nq + most - 1) / most, per = (nq + parts - 1) / parts;
+    PSB_TRY(s->row_dist.reserve(sizeof(float) * (size_t)per * g.stride));
+    PSB_TRY(s->row_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
+    const ScanIndex ix = s->scan_index();
+    g.nprobe = nprobe; g.centroids = ix.centroids; g.codebook = ix.codebook; g.codes = ix.codes; g.offsets = ix.offsets; g.row_base = ix.row_base;
+    g.row_delta = ix.row_delta; g.list_begin = ix.list_begin; g.list_end = ix.list_end; g.dim = ix.dim; g.m = ix.m; g.k = ix.k;
+    g.residual = ix.residual; g.tree = scan_tree_order(ix); g.stage1_k = stage1_k; g.seg = s->row_seg.as<int>(); g.dist = s->row_dist.as<float>();
+    g.expected_rows = expected_rows(s, nprobe); g.longest_list = s->longest[1]; g.counters = ws.counters; g.sm_count = s->sm_count;
+    if (ws.ev_begin) PSB_CUDA(cudaEventRecord(ws.ev_begin, st));
+    for (int q0 = 0; q0 < nq; q0 += per) {
+        g.queries = d_queries + (size_t)q0 * s->dim; g.probes = d_probes + (size_t)q0 * nprobe;
+        g.out_rows = d_rows + (size_t)q0 * stage1_k; g.out_dist = d_dist ? d_dist + (size_t)q0 * stage1_k : nullptr;
+        g.out_count = d_count ? d_count + q0 : nullptr;
+        PSB_TRY(launch_adc_rows(g, std::min(per, nq - q0), st));
+    }
+    if (ws.ev_end) PSB_CUDA(cudaEventRecord(ws.ev_end, st));
+    return PSB_OK;
+}
+
 psb_status ensure_pipeline_ws(psb_session* s, int nq, int nprobe, int topk, int stage1_k) {
     const int sb = sub_batch_rows(s, nq, nprobe, overlap_enabled(s, nq, rerank_enabled(s, topk)));
     PSB_TRY(s->q.reserve(sizeof(float) * (size_t)nq * s->dim));
     PSB_TRY(s->probes.reserve(sizeof(int) * (size_t)nq * nprobe));
     PSB_TRY(s->probe_dist.reserve(sizeof(float) * (size_t)nq * nprobe));
-    if (!residual_table_free(s, stage1_k)) PSB_TRY(s->lut.reserve(sizeof(float) * table_count(s, sb, nprobe) * s->m * s->k));
+    if (!residual_table_free(s, stage1_k) && !rows_form(s, sb, nprobe)) PSB_TRY(s->lut.reserve(sizeof(float) * table_count(s, sb, nprobe) * s->m * s->k));
     PSB_TRY(s->cand_rows.reserve(sizeof(int) * (size_t)nq * stage1_k));
     PSB_TRY(s->cand_dist.reserve(sizeof(float) * (size_t)nq * stage1_k));
     PSB_TRY(s->cand_count.reserve(sizeof(int) * (size_t)nq));
     PSB_TRY(s->out_rows.reserve(sizeof(int) * (size_t)nq * topk));
     PSB_TRY(s->out_dist.reserve(sizeof(float) * (size_t)nq * topk));
     PSB_TRY(s->out_ids.reserve(sizeof(long long) * (size_t)nq * topk));
-    return ensure_scan_ws(s, sb, nprobe, stage1_k);  // the scan runs one sub-batch at a time
+    return ensure_scan_ws(s, sb, nprobe, stage1_k, rows_form(s, sb, nprobe));  // the scan runs one sub-batch at a time
 }
 
 // Coarse stage on device queries: exact distance tiles + row selection, query-chunked so the distance tile
@@ -923,6 +985,7 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
         PSB_TRY(s->cb_maxnorm.reserve(sizeof(float) * (size_t)s->m));
         PSB_CUDA(cudaMemcpy(s->cb_maxnorm.p, mx.data(), sizeof(float) * (size_t)s->m, cudaMemcpyHostToDevice));
     }
+    note_list_lengths(s.get(), index->lists.offsets);
     // exact rows
     const auto& E = index->exact;
     if (E.fp32 || E.u8) {
@@ -1113,11 +1176,10 @@ psb_status psb_stage_scan_queries(psb_session* s, const float* d_queries, const 
     if (nprobe <= 0 || stage1_k <= 0) return fail(PSB_INVALID_ARGUMENT, "nprobe and stage1_k must be positive");
     if (nprobe > kMaxProbe || stage1_k > kMaxStage1) return fail(PSB_UNSUPPORTED_SHAPE, "nprobe above 4096 or stage1_k above 2048");
     PSB_CUDA(cudaSetDevice(s->device));
-    PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k));
+    PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, d_queries != nullptr && rows_form(s, nq, nprobe, true)));
     ScanWorkspace ws;
     PSB_TRY(s->timed_scan_ws(&ws));
-    return launch_scan(s->scan_index(), ws, d_lut, nq, d_probes, nprobe, stage1_k, d_rows, d_dist, d_count,
-                       s->sm_count, s->stream, d_queries);
+    return run_scan(s, ws, d_queries, d_lut, nq, d_probes, nprobe, stage1_k, d_rows, d_dist, d_count, s->stream, true);
 }
 
 int psb_scan_sample_words(const psb_session* s, int stage1_k) {
@@ -1140,7 +1202,7 @@ psb_status psb_stage_scan_sample(psb_session* s, const float* d_queries, const f
     PSB_TRY(check_scan_stage(s, d_probes, nprobe, stage1_k));
     if (!d_samples) return fail(PSB_INVALID_ARGUMENT, "null argument");
     PSB_CUDA(cudaSetDevice(s->device));
-    PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k));
+    PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, false));
     ScanWorkspace ws;
     PSB_TRY(s->timed_scan_ws(&ws));
     ws.phase = 1; ws.seed_export = d_samples; ws.seed_keys = seed_record_keys(stage1_k, s->opt.seed_sigma);
@@ -1277,9 +1339,9 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     for (size_t ci = 0; ci + 1 < cuts.size(); ++ci) sb_max = std::max(sb_max, cuts[ci + 1] - cuts[ci]);
     // The sub-batch size depends on this batch's own n (a short tail batch may run in one piece where the full batch ran
     // in four), so the tables and the scan workspace are sized here, for the largest sub-batch of THIS batch.
-    const bool table_free = residual_table_free(s, stage1_k);
+    const bool table_free = residual_table_free(s, stage1_k) || rows_form(s, sb_max, nprobe);
     if (!table_free) PSB_TRY(s->lut.reserve(sizeof(float) * table_count(s, sb_max, nprobe) * s->m * s->k));
-    PSB_TRY(ensure_scan_ws(s, sb_max, nprobe, stage1_k));
+    PSB_TRY(ensure_scan_ws(s, sb_max, nprobe, stage1_k, rows_form(s, sb_max, nprobe)));
     if ((overlap || staged_overlap) && !s->aux_stream) {
         int lo = 0, hi = 0;  // lowest priority: the scan's CTAs get the SMs first, the transfer fills the gaps
         PSB_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
@@ -1411,8 +1473,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         if (rc == PSB_OK && times) rc = tm_s.mark(st);
         if (rc == PSB_OK) {
             PSB_RANGE("pq_adc_scan");
-            rc = launch_scan(s->scan_index(), sws, table_free ? nullptr : s->lut.as<float>(), m, probes, nprobe, stage1_k,
-                             rows_out, dist_out, cnt_out, s->sm_count, st, q);
+            rc = run_scan(s, sws, q, table_free ? nullptr : s->lut.as<float>(), m, probes, nprobe, stage1_k, rows_out, dist_out, cnt_out, st);
         }
         if (rc == PSB_OK && times) rc = tm_s.mark(st);
         if (rc != PSB_OK) break;
@@ -1642,13 +1703,7 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
         PSB_CUDA(cudaMemcpyAsync(s->reordered.p, index->lists.reordered_ids, sizeof(long long) * n, cudaMemcpyHostToDevice, st));
         PSB_CUDA(cudaMemcpyAsync(s->flat_rows.p, index->rowmajor_fp32, sizeof(float) * n * s->dim, cudaMemcpyHostToDevice, st));
     }
-    {
-        std::vector<long long> len(nl);
-        for (size_t l = 0; l < nl; ++l) len[l] = index->lists.offsets[l + 1] - index->lists.offsets[l];
-        std::sort(len.begin(), len.end(), std::greater<long long>());
-        s->flat_longest.assign(nl + 1, 0);
-        for (size_t l = 0; l < nl; ++l) s->flat_longest[l + 1] = s->flat_longest[l] + len[l];
-    }
+    note_list_lengths(s.get(), index->lists.offsets);
     PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
     PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, st));
     PSB_CUDA(cudaStreamSynchronize(st));
@@ -1674,11 +1729,11 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     }
     // A row of distances per query, as long as the nprobe longest lists; queries in parts of at most 1 GiB of them.
     FlatScan f{};
-    f.stride = std::max<long long>(1, s->flat_longest[(size_t)nprobe]);
+    f.stride = std::max<long long>(1, s->longest[(size_t)nprobe]);
     const long long most = std::max<long long>(1, std::min<long long>(32768, ((long long)1 << 28) / f.stride));
     const int parts = (int)((n + most - 1) / most), per = (n + parts - 1) / parts;
-    PSB_TRY(s->flat_dist.reserve(sizeof(float) * (size_t)per * f.stride));
-    PSB_TRY(s->flat_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
+    PSB_TRY(s->row_dist.reserve(sizeof(float) * (size_t)per * f.stride));
+    PSB_TRY(s->row_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
     if (flat_list_form(per, nprobe, s->nlist, s->dim)) {
         PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
         PSB_TRY(s->flat_slot.reserve(sizeof(int) * (size_t)per * nprobe));
@@ -1687,7 +1742,7 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
         PSB_TRY(s->visitors.reserve(sizeof(int) * (size_t)per * nprobe));
     }
     f.dim = s->dim; f.nprobe = nprobe; f.offsets = s->offsets.as<long long>(); f.nlist = s->nlist; f.rows = s->flat_rows.as<float>();
-    f.ids = s->reordered.as<long long>(); f.topk = topk; f.dist = s->flat_dist.as<float>(); f.seg = s->flat_seg.as<int>();
+    f.ids = s->reordered.as<long long>(); f.topk = topk; f.dist = s->row_dist.as<float>(); f.seg = s->row_seg.as<int>();
     f.vis_count = s->vis_count.as<int>(); f.slot = s->flat_slot.as<int>(); f.vis_off = s->vis_off.as<int>(); f.item_off = s->item_off.as<long long>();
     f.visitors = s->visitors.as<int>(); f.counters = s->scalars.as<unsigned long long>(); f.sm_count = s->sm_count;
     for (int q0 = 0; q0 < n; q0 += per) {
