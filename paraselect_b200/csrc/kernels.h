@@ -301,21 +301,28 @@ struct RowMap {
     long long base = 0;
     long long count = 0;
 };
-// Copies the candidate rows held here (fp32 or u8, elem_bytes 4 or 1) from src (device-visible: mapped host or
-// device) to stage [nq][candidate_count][dim].  Candidates are global rows.  compact_ctas > 0: the kernel runs beside a scan
-// on another stream as that many lean CTAs; owned_sms > 0 (takes precedence): as that many CTAs that each keep an SM to
-// themselves.
-psb_status launch_gather_rows(const void* src, const RowMap& mp, int dim, int elem_bytes, const int* d_candidates,
-                              int nq, int candidate_count, int candidate_stride, const int* d_counts,
-                              void* d_stage, cudaStream_t s, int sm_count, int compact_ctas = 0, int owned_sms = 0);
-// d_out_dist [nq][candidate_count]: exact distance of each staged candidate, +inf for rows not held here.
-psb_status launch_rerank_score(const void* d_stage, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
+// Each row a batch's candidates name gets a slot: d_slot_of [count] (-1: none yet), d_unique [slots] = the row of each, d_n_unique their
+// number so far (the caller zeroes it once per batch; a batch may claim in several launches).  launch_release_rows puts d_slot_of back.
+psb_status launch_claim_rows(const RowMap& mp, const int* d_candidates, int nq, int candidate_count, int candidate_stride, const int* d_counts,
+                             int* d_slot_of, int* d_unique, int* d_n_unique, cudaStream_t s);
+psb_status launch_release_rows(const int* d_unique, const int* d_n_unique, int* d_slot_of, int sm_count, cudaStream_t s);
+// Of the slots [begin, end) the host threads fill those below this, the gather kernel the others.
+__host__ __device__ __forceinline__ int host_share_end(int begin, int end, int host_pct) { return begin + (int)((long long)(end - begin) * host_pct / 100); }
+// Copies the rows (src: device-visible, by row) of slots [*d_begin, *d_end) to d_stage (by slot).  compact_ctas > 0: the kernel runs
+// beside a scan on another stream as that many lean CTAs; owned_sms > 0 (takes precedence): as that many CTAs that each keep an SM
+// to themselves.
+psb_status launch_gather_unique(const void* src, int row_bytes, const int* d_unique, const int* d_begin, const int* d_end, int host_pct,
+                                void* d_stage, cudaStream_t s, int sm_count, int compact_ctas = 0, int owned_sms = 0);
+// d_out_dist [nq][candidate_count]: exact distance of each candidate, +inf for rows not held here.  d_slot_of null: rows at d_src by
+// their number, else by their slot.
+psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
                                const int* d_candidates, int nq, int candidate_count, int candidate_stride,
                                const int* d_counts, float* d_out_dist, cudaStream_t s);
-// Per query the topk (distance,row) pairs without duplicates from d_dist [nq][candidate_count].
+// Per query the topk (distance,row) pairs without duplicates from d_dist [nq][candidate_count]; with d_ids (original ids by row)
+// d_out_ids [nq][topk] is written instead of d_out_rows.
 psb_status launch_topk_select(const float* d_dist, const int* d_candidates, int nq, int candidate_count,
                               int candidate_stride, const int* d_counts, int topk, int* d_out_rows,
-                              float* d_out_dist, cudaStream_t s);
+                              float* d_out_dist, cudaStream_t s, const long long* d_ids = nullptr, long long* d_out_ids = nullptr);
 psb_status launch_map_ids(const int* d_rows, long long n, const long long* d_reordered, const RowMap& mp,
                           long long* d_out, cudaStream_t s);
 psb_status launch_merge(const int* d_rows, const float* d_dist, int parts, int nq, int k, int* d_out_rows,

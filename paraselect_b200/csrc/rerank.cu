@@ -1,18 +1,22 @@
 // Exact rerank of the ADC candidates, id mapping and the multi-shard candidate merge.
 //
-//   k_gather_rows     copies each candidate's exact row (fp32 or u8) from the exact store - host memory mapped
-//                     into the device address space and read over PCIe, or device memory - into a dense staging
-//                     buffer in HBM; one warp per row, 16-byte loads.  Rows this session does not hold (other
-//                     shards' rows, invalid ids) are skipped.
-//   k_rerank_score    half-warps score staged rows in the accumulation order of the CPU kernel the reference uses
-//                     (four 16-lane FMA accumulators, pairwise combine, halving tree:
+// Rows in device memory, and the rows of a small batch, are scored where they lie.  The rows of a large batch in host memory cross
+// PCIe once each, whatever the number of queries that ask for them (a third of the requests of a 10,000-query batch over 1M
+// rows, two thirds and more on skewed lists, name a row another query has asked for):
+//   k_claim_rows      the first candidate to name a row claims it and gives it the next slot of the staging buffer
+//   k_gather_unique   copies the claimed rows - host memory mapped into the device address space, read over PCIe - to their
+//                     slots; a warp keeps eight rows in flight.  Host threads fill a range of the slots instead or besides.
+//   k_rerank_score    half-warps score rows - from the slots or from where they lie - in the accumulation order of the CPU kernel
+//                     the reference uses (four 16-lane FMA accumulators, pairwise combine, halving tree:
 //                     src/cpu/distance/fp32_l2_avx512.h:16-53); rows not held here score +inf
-//   k_topk_select     one CTA per query: bitonic sort of (distance,row) keys, duplicate rows collapse, the first
-//                     topk are written (reference semantics: src/search/ivf_common/ivf_host_rerank.cpp:152-177,
-//                     src/search/ivf_common/ivf_exact_topk.h:12-22)
-#include <cstdlib>
+//   k_topk_select     one CTA per query: the topk smallest (distance,row), duplicate rows once (reference semantics:
+//                     src/search/ivf_common/ivf_host_rerank.cpp:152-177, src/search/ivf_common/ivf_exact_topk.h:12-22)
+//   k_release_rows    the claims of a batch are taken back
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
+#include "select.cuh"
 
 namespace psb {
 namespace {
@@ -40,95 +44,106 @@ __device__ __forceinline__ long long local_row(const RowMap& mp, long long r) {
     return l < mp.local_offsets[lo + 1] ? l : -1;
 }
 
-// Gathers candidate rows into the staging buffer.  A warp takes 32 candidates at a time: every lane resolves one candidate
-// to a local row (for a striped shard that is a binary search of 16 dependent loads - done for 32 candidates at once), then
-// the warp copies the rows four at a time, all four rows' loads issued before the first store, so that a few hundred KB
-// of PCIe reads stay in flight even on a small grid.
-template <int U = 4>
-__device__ __forceinline__ void gather_rows_body(const unsigned char* __restrict__ src, const RowMap& mp, int row_bytes,
-                                                 const int* __restrict__ cand, int nq, int candidate_count, int candidate_stride,
-                                                 const int* __restrict__ counts, unsigned char* __restrict__ stage) {
-    const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+// One thread per candidate.  slot_of [rows held here], -1: unclaimed; -2 while the claimer of this launch has not stored its slot (the
+// slots are read by later kernels only).
+__global__ void __launch_bounds__(256) k_claim_rows(RowMap mp, const int* __restrict__ cand, int nq, int candidate_count, int candidate_stride,
+                                                    const int* __restrict__ counts, int* __restrict__ slot_of, int* __restrict__ unique, int* __restrict__ n_unique) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const long long total = (long long)nq * candidate_count;
+    bool won = false;
+    long long row = -1;
+    if (i < (long long)nq * candidate_count) {
+        const int q = (int)(i / candidate_count), c = (int)(i - (long long)q * candidate_count);
+        if (c < cand_count(counts, q, candidate_count)) row = local_row(mp, cand[(size_t)q * candidate_stride + c]);
+        if (row >= 0 && *(volatile int*)(slot_of + row) == -1) won = atomicCAS(slot_of + row, -1, -2) == -1;
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, won);
+    if (!bal) return;
+    int base = 0;
+    if (lane == __ffs((int)bal) - 1) base = atomicAdd(n_unique, __popc(bal));
+    base = __shfl_sync(0xffffffffu, base, __ffs((int)bal) - 1);
+    if (won) {
+        const int slot = base + __popc(bal & ((1u << lane) - 1u));
+        unique[slot] = (int)row;
+        *(volatile int*)(slot_of + row) = slot;
+    }
+}
+
+__global__ void k_release_rows(const int* __restrict__ unique, const int* __restrict__ n_unique, int* __restrict__ slot_of) {
+    const int n = *n_unique;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) slot_of[unique[i]] = -1;
+}
+
+// Copies the rows of slots [*begin, *end), from the end of the host threads' share (host_pct) on, into the staging buffer; a warp takes eight slots
+// at a time, all eight rows' loads issued before the first store.
+__device__ __forceinline__ void gather_unique_body(const unsigned char* __restrict__ src, int row_bytes, const int* __restrict__ unique,
+                                                   const int* __restrict__ begin, const int* __restrict__ end, int host_pct,
+                                                   unsigned char* __restrict__ stage) {
+    constexpr int U = 8;
+    const int lane = threadIdx.x & 31;
+    const int warp0 = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
+    const int e = *end, b = host_share_end(*begin, e, host_pct);
     const uintptr_t both = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(stage);
-    const bool vec16 = (row_bytes % 16) == 0 && (both % 16) == 0;
-    const bool vec4 = (row_bytes % 4) == 0 && (both % 4) == 0;
-    const int n16 = row_bytes / 16;
-    for (long long base = warp0 * 32; base < total; base += nwarps * 32) {
-        long long mine = -1;
-        const long long w = base + lane;
-        if (w < total) {
-            const int q = (int)(w / candidate_count), i = (int)(w % candidate_count);
-            if (i < cand_count(counts, q, candidate_count)) mine = local_row(mp, cand[(size_t)q * candidate_stride + i]);
-        }
-        if (vec16 && n16 <= 32) {
-            // The rows held here, four at a time whatever their positions among the 32 candidates: on a shard most candidates
-            // belong to other shards, and the reads in flight must not thin out with them.
-            unsigned present = __ballot_sync(0xffffffffu, mine >= 0);
-#pragma unroll 1
-            while (present) {
-                int at[U];
-                long long r[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    at[u] = present ? __ffs(present) - 1 : -1;   // uniform across the warp
-                    if (present) present &= present - 1;
-                    r[u] = __shfl_sync(0xffffffffu, mine, at[u] < 0 ? 0 : at[u]);
-                }
+    const bool vec16 = (row_bytes % 16) == 0 && (both % 16) == 0, vec4 = (row_bytes % 4) == 0 && (both % 4) == 0;
+    for (int s0 = b + warp0 * U; s0 < e; s0 += nwarps * U) {
+        const int mine = lane < U && s0 + lane < e ? unique[s0 + lane] : -1;
+        if (vec16) {
+            for (int j0 = 0; j0 < row_bytes / 16; j0 += 32) {
+                const int j = j0 + lane;
                 uint4 v[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (at[u] >= 0 && lane < n16) v[u] = reinterpret_cast<const uint4*>(src + (size_t)r[u] * row_bytes)[lane];
+                for (int u = 0; u < U; ++u) {
+                    const int r = __shfl_sync(0xffffffffu, mine, u);
+                    if (r >= 0 && j < row_bytes / 16) v[u] = reinterpret_cast<const uint4*>(src + (size_t)r * row_bytes)[j];
+                }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
-                    if (at[u] >= 0 && lane < n16) reinterpret_cast<uint4*>(stage + (size_t)(base + at[u]) * row_bytes)[lane] = v[u];
+                    if (__shfl_sync(0xffffffffu, mine, u) >= 0 && j < row_bytes / 16) reinterpret_cast<uint4*>(stage + (size_t)(s0 + u) * row_bytes)[j] = v[u];
+            }
+        } else if (vec4) {
+            for (int j0 = 0; j0 < row_bytes / 4; j0 += 32) {
+                const int j = j0 + lane;
+                uint32_t v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int r = __shfl_sync(0xffffffffu, mine, u);
+                    if (r >= 0 && j < row_bytes / 4) v[u] = reinterpret_cast<const uint32_t*>(src + (size_t)r * row_bytes)[j];
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (__shfl_sync(0xffffffffu, mine, u) >= 0 && j < row_bytes / 4) reinterpret_cast<uint32_t*>(stage + (size_t)(s0 + u) * row_bytes)[j] = v[u];
             }
         } else {
-            for (int k = 0; k < 32; ++k) {
-                const long long row = __shfl_sync(0xffffffffu, mine, k);
-                if (row < 0) continue;
-                const unsigned char* sp = src + (size_t)row * row_bytes;
-                unsigned char* d = stage + (size_t)(base + k) * row_bytes;
-                if (vec16) {
-                    for (int j = lane; j < n16; j += 32) reinterpret_cast<uint4*>(d)[j] = reinterpret_cast<const uint4*>(sp)[j];
-                } else if (vec4) {
-                    for (int j = lane; j < row_bytes / 4; j += 32) reinterpret_cast<uint32_t*>(d)[j] = reinterpret_cast<const uint32_t*>(sp)[j];
-                } else {
-                    for (int j = lane; j < row_bytes; j += 32) d[j] = sp[j];
-                }
+            for (int u = 0; u < U; ++u) {
+                const int r = __shfl_sync(0xffffffffu, mine, u);
+                if (r < 0) continue;
+                for (int j = lane; j < row_bytes; j += 32) stage[(size_t)(s0 + u) * row_bytes + j] = src[(size_t)r * row_bytes + j];
             }
         }
     }
 }
 
-__global__ void k_gather_rows(const unsigned char* __restrict__ src, RowMap mp, int row_bytes,
-                              const int* __restrict__ cand, int nq, int candidate_count, int candidate_stride,
-                              const int* __restrict__ counts, unsigned char* __restrict__ stage) {
-    gather_rows_body(src, mp, row_bytes, cand, nq, candidate_count, candidate_stride, counts, stage);
+__global__ void __launch_bounds__(256) k_gather_unique(const unsigned char* __restrict__ src, int row_bytes, const int* __restrict__ unique,
+                                                       const int* __restrict__ begin, const int* __restrict__ end, int host_pct,
+                                                       unsigned char* __restrict__ stage) {
+    gather_unique_body(src, row_bytes, unique, begin, end, host_pct, stage);
 }
 // The same gather built to sit BESIDE a scan kernel that owns nearly a whole SM (one 576-thread CTA with ~55K registers and
 // ~200 KB of shared memory): 128-thread CTAs capped at 40 registers and no shared memory, two of which fit into what the
-// scan leaves of every SM.  Spread over all SMs they keep far more PCIe reads in flight than the link's bandwidth-delay
-// product while taking almost no issue slots (their warps wait on loads).
-__global__ void __launch_bounds__(256, 6) k_gather_rows_beside(const unsigned char* __restrict__ src, RowMap mp, int row_bytes,
-                                                               const int* __restrict__ cand, int nq, int candidate_count,
-                                                               int candidate_stride, const int* __restrict__ counts,
-                                                               unsigned char* __restrict__ stage) {
-    gather_rows_body(src, mp, row_bytes, cand, nq, candidate_count, candidate_stride, counts, stage);
+// scan leaves of every SM.
+__global__ void __launch_bounds__(256, 6) k_gather_unique_beside(const unsigned char* __restrict__ src, int row_bytes, const int* __restrict__ unique,
+                                                                 const int* __restrict__ begin, const int* __restrict__ end, int host_pct,
+                                                                 unsigned char* __restrict__ stage) {
+    gather_unique_body(src, row_bytes, unique, begin, end, host_pct, stage);
 }
-
 // The same gather on SMs of its own: CTAs of 1,024 threads that also claim (without using it) nearly all the shared memory of
 // an SM, so that no kernel with a shared-memory footprint - the scan, the cutoff sampling, the selections - shares an SM with
 // them.  Reads of host memory stay in flight for microseconds; next to another kernel's warps they held up that kernel's own
-// memory traffic (its stages ran at half speed), on separate SMs they do not.  Eight such CTAs keep ~800 KB of reads in
-// flight.
-__global__ void __launch_bounds__(1024, 1) k_gather_rows_owned(const unsigned char* __restrict__ src, RowMap mp, int row_bytes,
-                                                               const int* __restrict__ cand, int nq, int candidate_count,
-                                                               int candidate_stride, const int* __restrict__ counts,
-                                                               unsigned char* __restrict__ stage) {
-    gather_rows_body<8>(src, mp, row_bytes, cand, nq, candidate_count, candidate_stride, counts, stage);   // eight rows per warp in flight
+// memory traffic (its stages ran at half speed), on separate SMs they do not.
+__global__ void __launch_bounds__(1024, 1) k_gather_unique_owned(const unsigned char* __restrict__ src, int row_bytes, const int* __restrict__ unique,
+                                                                 const int* __restrict__ begin, const int* __restrict__ end, int host_pct,
+                                                                 unsigned char* __restrict__ stage) {
+    gather_unique_body(src, row_bytes, unique, begin, end, host_pct, stage);
 }
 
 // fp32 squared L2 by a half-warp (16 lanes), bit-identical to the AVX-512 kernel's order.
@@ -158,7 +173,16 @@ __device__ __forceinline__ float l2_halfwarp(const float* __restrict__ q, const 
 __device__ __forceinline__ float l2_u8_halfwarp(const unsigned char* __restrict__ q, const unsigned char* __restrict__ v,
                                                 int dim, int j, unsigned hmask) {
     int s = 0;
-    for (int i = j; i < dim; i += 16) { const int d = (int)q[i] - (int)v[i]; s += d * d; }
+    if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(v) | (uintptr_t)dim) & 3) == 0) {   // whole numbers: any order
+        unsigned acc = 0;
+        for (int i = j; i < dim / 4; i += 16) {
+            const unsigned d = __vabsdiffu4(reinterpret_cast<const unsigned*>(q)[i], reinterpret_cast<const unsigned*>(v)[i]);
+            acc = __dp4a(d, d, acc);
+        }
+        s = (int)acc;
+    } else {
+        for (int i = j; i < dim; i += 16) { const int d = (int)q[i] - (int)v[i]; s += d * d; }
+    }
     s += __shfl_xor_sync(hmask, s, 8);
     s += __shfl_xor_sync(hmask, s, 4);
     s += __shfl_xor_sync(hmask, s, 2);
@@ -167,81 +191,138 @@ __device__ __forceinline__ float l2_u8_halfwarp(const unsigned char* __restrict_
 }
 
 constexpr int kScoreThreads = 256;
-// grid (nq, ceil(candidate_count / 16 half-warps)): dist[q][i] = exact distance of candidate i, +inf when the row is
-// invalid, beyond the query's count, or not held by this session.
+constexpr int kScoreRows = 4;                                       // rows a warp has in flight
+constexpr int kScoreBlock = kScoreThreads / 32 * kScoreRows;        // candidates per CTA
+__host__ __device__ __forceinline__ int score_pitch(int row_bytes) { return (row_bytes + 15) / 16 * 16 + 16; }
+// grid (nq, candidate_count / kScoreBlock): dist[q][i] = exact distance of candidate i, +inf when the row is invalid, beyond the
+// query's count, or not held by this session.  slot_of null: the rows lie at src by their number (device memory, or host memory
+// mapped here); else at src by their slot.  Rows are fetched whole, 16 bytes per lane, into shared memory (through = 0: too long
+// for it, read in place).
 __global__ void __launch_bounds__(kScoreThreads)
-k_rerank_score(const unsigned char* __restrict__ stage, RowMap mp, int dim, int elem_bytes,
+k_rerank_score(const unsigned char* __restrict__ src, const int* __restrict__ slot_of, RowMap mp, int dim, int elem_bytes, int through,
                const unsigned char* __restrict__ queries, const int* __restrict__ cand, int candidate_count,
                int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist) {
-    extern __shared__ __align__(16) unsigned char s_q[];
-    const int q = blockIdx.x;
-    const int row_bytes = dim * elem_bytes;
-    for (int i = threadIdx.x; i < row_bytes; i += blockDim.x) s_q[i] = queries[(size_t)q * row_bytes + i];
-    __syncthreads();
+    extern __shared__ __align__(16) unsigned char s_score[];
+    const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row_bytes = dim * elem_bytes, pitch = score_pitch(row_bytes);
+    unsigned char* s_q = s_score;
+    unsigned char* s_row = s_score + pitch + (size_t)warp * kScoreRows * pitch;
+    if ((row_bytes & 3) == 0)
+        for (int i = threadIdx.x; i < row_bytes / 4; i += kScoreThreads) reinterpret_cast<uint32_t*>(s_q)[i] = reinterpret_cast<const uint32_t*>(queries + (size_t)q * row_bytes)[i];
+    else
+        for (int i = threadIdx.x; i < row_bytes; i += kScoreThreads) s_q[i] = queries[(size_t)q * row_bytes + i];
     const int n = cand_count(counts, q, candidate_count);
-    const int hw = threadIdx.x >> 4, j = threadIdx.x & 15;
-    const unsigned hmask = 0xffffu << (threadIdx.x & 16);
-    const int i = blockIdx.y * (kScoreThreads / 16) + hw;
-    if (i >= candidate_count) return;
-    float d = __int_as_float(0x7f800000);
-    const long long row = i < n ? local_row(mp, cand[(size_t)q * candidate_stride + i]) : -1;
-    if (row >= 0) {
-        const unsigned char* v = stage + ((size_t)q * candidate_count + i) * row_bytes;
-        d = elem_bytes == 4
-            ? l2_halfwarp(reinterpret_cast<const float*>(s_q), reinterpret_cast<const float*>(v), dim, j, hmask)
-            : l2_u8_halfwarp(s_q, v, dim, j, hmask);
+    const int i0 = blockIdx.y * kScoreBlock + warp * kScoreRows;
+    int at = -1;
+    if (lane < kScoreRows && i0 + lane < n) {
+        const long long row = local_row(mp, cand[(size_t)q * candidate_stride + i0 + lane]);
+        if (row >= 0) at = slot_of ? slot_of[row] : (int)row;
     }
-    if (j == 0) out_dist[(size_t)q * candidate_count + i] = d;
+    if (through) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(src) | (uintptr_t)row_bytes;
+        const int unit = (a & 15) == 0 ? 16 : ((a & 3) == 0 ? 4 : 1);
+        const int units = row_bytes / unit;
+        for (int j0 = 0; j0 < units; j0 += 32) {
+            const int j = j0 + lane;
+            uint4 v[kScoreRows];
+#pragma unroll
+            for (int u = 0; u < kScoreRows; ++u) {
+                const int r = __shfl_sync(0xffffffffu, at, u);
+                if (r < 0 || j >= units) continue;
+                const unsigned char* p = src + (size_t)r * row_bytes + (size_t)j * unit;
+                if (unit == 16) v[u] = __ldg(reinterpret_cast<const uint4*>(p));
+                else if (unit == 4) v[u].x = __ldg(reinterpret_cast<const uint32_t*>(p));
+                else v[u].x = __ldg(p);
+            }
+#pragma unroll
+            for (int u = 0; u < kScoreRows; ++u) {
+                if (__shfl_sync(0xffffffffu, at, u) < 0 || j >= units) continue;
+                unsigned char* d = s_row + u * pitch + j * unit;
+                if (unit == 16) *reinterpret_cast<uint4*>(d) = v[u];
+                else if (unit == 4) *reinterpret_cast<uint32_t*>(d) = v[u].x;
+                else *d = (unsigned char)v[u].x;
+            }
+        }
+    }
+    __syncthreads();
+    const int half = lane >> 4, j = lane & 15;
+    const unsigned hmask = 0xffffu << (lane & 16);
+#pragma unroll
+    for (int u0 = 0; u0 < kScoreRows; u0 += 2) {
+        const int u = u0 + half;
+        const int r = __shfl_sync(0xffffffffu, at, u);
+        float d = __int_as_float(0x7f800000);
+        if (r >= 0) {
+            const unsigned char* v = through ? s_row + u * pitch : src + (size_t)r * row_bytes;
+            d = elem_bytes == 4 ? l2_halfwarp(reinterpret_cast<const float*>(s_q), reinterpret_cast<const float*>(v), dim, j, hmask)
+                                : l2_u8_halfwarp(s_q, v, dim, j, hmask);
+        }
+        if (j == 0 && i0 + u < candidate_count) out_dist[(size_t)q * candidate_count + i0 + u] = d;
+    }
 }
 
 constexpr int kSelectThreads = 256;
-// dist [nq][candidate_count] (dense), cand [nq][candidate_stride] global rows.
+// dist [nq][candidate_count] (dense), cand [nq][candidate_stride] global rows.  ids: original ids by row (out_ids is written
+// instead of out_rows).  The smallest come from select.cuh; when a row turns up twice among them - the ADC stage names a row once, a
+// caller's own candidates need not - everything is sorted and duplicates, equal keys next to each other, are dropped.
 __global__ void __launch_bounds__(kSelectThreads)
 k_topk_select(const float* __restrict__ dist, const int* __restrict__ cand, int candidate_count, int candidate_stride,
-              const int* __restrict__ counts, int topk, int np, int* __restrict__ out_rows, float* __restrict__ out_dist) {
+              const int* __restrict__ counts, int topk, int np, int buffer, int* __restrict__ out_rows, float* __restrict__ out_dist,
+              const long long* __restrict__ ids, long long* __restrict__ out_ids) {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_raw);         // [np]
-    int* s_rank = reinterpret_cast<int*>(s_raw + (size_t)np * 8);  // [np]
+    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_raw);            // [max(np, buffer)]
+    int* s_rank = reinterpret_cast<int*>(s_raw + (size_t)max(np, buffer) * 8);  // [max(np, kMaxGroups)]: ranks, or the group minima
+    __shared__ sel::Words w;
     __shared__ int s_warp[32];
-    __shared__ int s_total;
+    __shared__ int s_total, s_twice;
     const int q = blockIdx.x;
     const int n = cand_count(counts, q, candidate_count);
-    for (int i = threadIdx.x; i < np; i += blockDim.x) {
+    const int* rows = cand + (size_t)q * candidate_stride;
+    const float inf = __int_as_float(0x7f800000);
+    auto put = [&](int r, uint64_t key) {
+        if (out_ids) out_ids[(size_t)q * topk + r] = key == KEY_MAX ? -1 : ids[key_idx(key)];
+        else out_rows[(size_t)q * topk + r] = key == KEY_MAX ? -1 : (int)key_idx(key);
+        out_dist[(size_t)q * topk + r] = key == KEY_MAX ? FLT_MAX : key_dist(key);
+    };
+    const int keep = sel::smallest<kSelectThreads>(dist + (size_t)q * candidate_count, n, topk, [&](int i) { return (uint32_t)rows[i]; }, s_keys, buffer,
+                                                   reinterpret_cast<float*>(s_rank), &w);
+    if (threadIdx.x == 0) s_twice = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < keep; i += kSelectThreads)   // a row twice, or a distance without a row
+        if (key_dist(s_keys[i]) != inf && ((i && s_keys[i] == s_keys[i - 1]) || (int)key_idx(s_keys[i]) < 0)) s_twice = 1;
+    __syncthreads();
+    if (!s_twice) {
+        for (int r = threadIdx.x; r < topk; r += kSelectThreads) put(r, r < keep && key_dist(s_keys[r]) != inf ? s_keys[r] : KEY_MAX);
+        return;
+    }
+    for (int i = threadIdx.x; i < np; i += kSelectThreads) {
         uint64_t key = KEY_MAX;
         if (i < n) {
-            const int row = cand[(size_t)q * candidate_stride + i];
             const float d = dist[(size_t)q * candidate_count + i];
-            if (row >= 0 && d != __int_as_float(0x7f800000)) key = make_key(d, (uint32_t)row);
+            if (rows[i] >= 0 && d != inf) key = make_key(d, (uint32_t)rows[i]);
         }
         s_keys[i] = key;
     }
     __syncthreads();
     block_bitonic_sort(s_keys, np);
-    // duplicates are adjacent (same row -> same distance -> same key): keep the first of each run
     int base = 0;
-    for (int c0 = 0; c0 < np; c0 += blockDim.x) {
+    for (int c0 = 0; c0 < np; c0 += kSelectThreads) {
         const int i = c0 + threadIdx.x;
-        int keep = 0;
+        int fresh = 0;
         if (i < np) {
             const uint64_t key = s_keys[i];
-            keep = key != KEY_MAX && (i == 0 || s_keys[i - 1] != key);
+            fresh = key != KEY_MAX && (i == 0 || s_keys[i - 1] != key);
         }
-        const int ex = block_exclusive_scan(keep, s_warp, &s_total);
-        if (i < np) s_rank[i] = keep ? base + ex : -1;
+        const int ex = block_exclusive_scan(fresh, s_warp, &s_total);
+        if (i < np) s_rank[i] = fresh ? base + ex : -1;
         base += s_total;
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < np; i += blockDim.x) {
+    for (int i = threadIdx.x; i < np; i += kSelectThreads) {
         const int r = s_rank[i];
-        if (r >= 0 && r < topk) {
-            out_rows[(size_t)q * topk + r] = (int)key_idx(s_keys[i]);
-            out_dist[(size_t)q * topk + r] = key_dist(s_keys[i]);
-        }
+        if (r >= 0 && r < topk) put(r, s_keys[i]);
     }
-    for (int r = base + threadIdx.x; r < topk; r += blockDim.x) {
-        out_rows[(size_t)q * topk + r] = -1;
-        out_dist[(size_t)q * topk + r] = FLT_MAX;
-    }
+    for (int r = base + threadIdx.x; r < topk; r += kSelectThreads) put(r, KEY_MAX);
 }
 
 // out[i] = original id of global row rows[i] when this session holds the row, else -1.
@@ -292,49 +373,61 @@ k_merge(const int* __restrict__ rows, const float* __restrict__ dist, int parts,
 
 }  // namespace
 
-psb_status launch_gather_rows(const void* src, const RowMap& mp, int dim, int elem_bytes, const int* d_candidates,
-                              int nq, int candidate_count, int candidate_stride, const int* d_counts,
-                              void* d_stage, cudaStream_t s, int sm_count, int compact_ctas, int owned_sms) {
+psb_status launch_claim_rows(const RowMap& mp, const int* d_candidates, int nq, int candidate_count, int candidate_stride, const int* d_counts,
+                             int* d_slot_of, int* d_unique, int* d_n_unique, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
     const long long total = (long long)nq * candidate_count;
-    PSB_TRY(prefer_max_shared(k_gather_rows));
+    PSB_TRY(prefer_max_shared(k_claim_rows));
+    k_claim_rows<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(mp, d_candidates, nq, candidate_count, candidate_stride, d_counts, d_slot_of, d_unique,
+                                                                 d_n_unique);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+
+psb_status launch_release_rows(const int* d_unique, const int* d_n_unique, int* d_slot_of, int sm_count, cudaStream_t s) {
+    PSB_TRY(prefer_max_shared(k_release_rows));
+    k_release_rows<<<sm_count * 2, 256, 0, s>>>(d_unique, d_n_unique, d_slot_of);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+
+psb_status launch_gather_unique(const void* src, int row_bytes, const int* d_unique, const int* d_begin, const int* d_end, int host_pct,
+                                void* d_stage, cudaStream_t s, int sm_count, int compact_ctas, int owned_sms) {
+    const unsigned char* from = static_cast<const unsigned char*>(src);
+    unsigned char* to = static_cast<unsigned char*>(d_stage);
     if (owned_sms > 0) {
         constexpr int kOwnedSmem = 200 * 1024;   // claimed, not used: keeps every kernel that needs shared memory off the SM
-        PSB_TRY(prefer_max_shared(k_gather_rows_owned));
-        PSB_CUDA(cudaFuncSetAttribute(k_gather_rows_owned, cudaFuncAttributeMaxDynamicSharedMemorySize, kOwnedSmem));
-        long long blocks = (total * 32 + 1023) / 1024;
-        if (blocks > owned_sms) blocks = owned_sms;
-        k_gather_rows_owned<<<(unsigned)blocks, 1024, kOwnedSmem, s>>>(static_cast<const unsigned char*>(src), mp, dim * elem_bytes,
-                                                                        d_candidates, nq, candidate_count, candidate_stride, d_counts,
-                                                                        static_cast<unsigned char*>(d_stage));
+        PSB_TRY(prefer_max_shared(k_gather_unique_owned));
+        PSB_CUDA(cudaFuncSetAttribute(k_gather_unique_owned, cudaFuncAttributeMaxDynamicSharedMemorySize, kOwnedSmem));
+        k_gather_unique_owned<<<owned_sms, 1024, kOwnedSmem, s>>>(from, row_bytes, d_unique, d_begin, d_end, host_pct, to);
     } else if (compact_ctas > 0) {
-        // Beside a scan kernel on the other stream of the overlapped pipeline: small lean CTAs on every SM (compact_ctas of them).
-        PSB_TRY(prefer_max_shared(k_gather_rows_beside));
-        long long blocks = (total * 32 + 127) / 128;
-        if (blocks > compact_ctas) blocks = compact_ctas;
-        k_gather_rows_beside<<<(unsigned)blocks, 128, 0, s>>>(static_cast<const unsigned char*>(src), mp, dim * elem_bytes,
-                                                              d_candidates, nq, candidate_count, candidate_stride, d_counts,
-                                                              static_cast<unsigned char*>(d_stage));
+        PSB_TRY(prefer_max_shared(k_gather_unique_beside));
+        k_gather_unique_beside<<<compact_ctas, 128, 0, s>>>(from, row_bytes, d_unique, d_begin, d_end, host_pct, to);
     } else {
-        long long blocks = (total * 32 + 255) / 256;
-        if (blocks > (long long)sm_count * 8) blocks = (long long)sm_count * 8;
-        k_gather_rows<<<(unsigned)blocks, 256, 0, s>>>(static_cast<const unsigned char*>(src), mp, dim * elem_bytes,
-                                                       d_candidates, nq, candidate_count, candidate_stride, d_counts,
-                                                       static_cast<unsigned char*>(d_stage));
+        PSB_TRY(prefer_max_shared(k_gather_unique));
+        k_gather_unique<<<sm_count * 2, 256, 0, s>>>(from, row_bytes, d_unique, d_begin, d_end, host_pct, to);
     }
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
 }
 
-psb_status launch_rerank_score(const void* d_stage, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
+psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
                                const int* d_candidates, int nq, int candidate_count, int candidate_stride,
                                const int* d_counts, float* d_out_dist, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
-    dim3 grid(nq, (candidate_count + kScoreThreads / 16 - 1) / (kScoreThreads / 16));
+    const dim3 grid(nq, (candidate_count + kScoreBlock - 1) / kScoreBlock);
+    const size_t pitch = (size_t)score_pitch(dim * elem_bytes);
+    size_t smem = pitch * (1 + kScoreBlock);
+    const int through = smem <= (size_t)200 * 1024 ? 1 : 0;
+    if (!through) smem = pitch;
+    if (smem > (size_t)220 * 1024) return fail(PSB_UNSUPPORTED_SHAPE, "rows too long for the exact rerank");
+    if (smem > 48 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_rerank_score, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     PSB_TRY(prefer_max_shared(k_rerank_score));
-    k_rerank_score<<<grid, kScoreThreads, (size_t)dim * elem_bytes, s>>>(
-        static_cast<const unsigned char*>(d_stage), mp, dim, elem_bytes, static_cast<const unsigned char*>(d_queries),
+    k_rerank_score<<<grid, kScoreThreads, smem, s>>>(
+        static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, elem_bytes, through, static_cast<const unsigned char*>(d_queries),
         d_candidates, candidate_count, candidate_stride, d_counts, d_out_dist);
     count_launch();
     PSB_LAUNCH_CHECK();
@@ -343,17 +436,18 @@ psb_status launch_rerank_score(const void* d_stage, const RowMap& mp, int dim, i
 
 psb_status launch_topk_select(const float* d_dist, const int* d_candidates, int nq, int candidate_count,
                               int candidate_stride, const int* d_counts, int topk, int* d_out_rows,
-                              float* d_out_dist, cudaStream_t s) {
+                              float* d_out_dist, cudaStream_t s, const long long* d_ids, long long* d_out_ids) {
     if (nq <= 0) return PSB_OK;
     if (candidate_count > kMaxRerankWidth) return fail(PSB_UNSUPPORTED_SHAPE, "rerank accepts at most 4096 candidates per query");
     int np = 32;
     while (np < candidate_count) np <<= 1;
-    const size_t smem = (size_t)np * 12;
+    const int buffer = sel::buffer_entries(topk);
+    const size_t smem = (size_t)std::max(np, buffer) * 8 + (size_t)std::max(np, sel::kMaxGroups) * 4;
     if (smem > 32 * 1024)
         PSB_CUDA(cudaFuncSetAttribute(k_topk_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     PSB_TRY(prefer_max_shared(k_topk_select));
     k_topk_select<<<nq, kSelectThreads, smem, s>>>(d_dist, d_candidates, candidate_count, candidate_stride, d_counts,
-                                                   topk, np, d_out_rows, d_out_dist);
+                                                   topk, np, buffer, d_out_rows, d_out_dist, d_ids, d_out_ids);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

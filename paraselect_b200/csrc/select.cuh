@@ -128,7 +128,7 @@ __device__ int smallest(const float* __restrict__ vals, int n, int k, Payload pa
         int rank = 0;
         if ((tid & ~31) < c) {
 #pragma unroll 4
-            for (int j = 0; j < c; ++j) rank += s_keys[j] < mine ? 1 : 0;
+            for (int j = 0; j < c; ++j) { const uint64_t o = s_keys[j]; rank += o < mine || (o == mine && j < tid) ? 1 : 0; }   // a key may occur twice
         }
         __syncthreads();
         if (tid < c) s_keys[rank] = mine;

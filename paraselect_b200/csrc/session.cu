@@ -323,10 +323,15 @@ struct psb_session {
     std::unique_ptr<HostPool> host_pool;   // gather threads of the staged transport (created on first use)
     double staged_gather_s = 0.0;          // host time spent gathering rows, and the bytes gathered (reported by the bench)
     long long staged_gather_bytes = 0;
-    std::vector<int> h_cand;
-    int* h_cand_pinned = nullptr;        // candidates of the whole batch on the host (overlapped staged transport)
-    size_t h_cand_pinned_count = 0;
-    std::vector<long long> h_global_begin, h_offsets;  // striped shards: host copies for the staged transport
+    // Rows of a large batch cross to the device once each: the slot of every row held here, the rows by slot, the number of slots and
+    // where each sub-batch's begin (kMarks: count, 0, end of part 0, end of part 1, ...).
+    DevBuf slot_of, unique, marks;
+    bool slots_dirty = true;             // slot_of is not all -1 (never used, or a batch was left half done)
+    int* h_unique = nullptr;             // pinned: the slots the host threads fill
+    size_t h_unique_count = 0;
+    int* h_marks = nullptr;              // pinned [2 * kMaxParts]
+    cudaStream_t list_stream = nullptr;  // brings the slot lists to the host thread beside the row copies
+    std::vector<long long> h_global_begin;  // striped shards: host copy of the slices' first rows
     // workspaces
     DevBuf q, q_u8, dist_tile, probes, probe_dist, lut, vis_count, vis_off, vis_cursor, item_off, item_off_tc, visitors, q_rows, thr,
         pool_cnt, pool, fail_list, fallback_partial, scalars, lut_h, lut_scale, cand_rows, cand_dist, cand_count, stage, score, out_rows, out_dist, out_ids;
@@ -358,7 +363,9 @@ struct psb_session {
             if (pinned[i]) cudaFreeHost(pinned[i]);
             if (pinned_ev[i]) cudaEventDestroy(pinned_ev[i]);
         }
-        if (h_cand_pinned) cudaFreeHost(h_cand_pinned);
+        if (h_unique) cudaFreeHost(h_unique);
+        if (h_marks) cudaFreeHost(h_marks);
+        if (list_stream) { cudaStreamSynchronize(list_stream); cudaStreamDestroy(list_stream); }
         if (aux_stream) { cudaStreamSynchronize(aux_stream); cudaStreamDestroy(aux_stream); }
         if (zc_stream) { cudaStreamSynchronize(zc_stream); cudaStreamDestroy(zc_stream); }
         if (zc_ev_a) cudaEventDestroy(zc_ev_a);
@@ -688,25 +695,17 @@ psb_status validate_params(const psb_session* s, const psb_query_batch_view* qv,
     return PSB_OK;
 }
 
-// Host-side twin of the device row mapping (staged transport only).
-long long host_local_row(const psb_session* s, long long r) {
-    if (r < 0) return -1;
-    if (!s->striped) return r < s->n_vectors ? r : -1;
-    const auto& gb = s->h_global_begin;
-    auto it = std::upper_bound(gb.begin(), gb.end(), r);
-    if (it == gb.begin()) return -1;
-    const size_t l = (size_t)(it - gb.begin()) - 1;
-    const long long loc = s->h_offsets[l] + (r - gb[l]);
-    return loc < s->h_offsets[l + 1] ? loc : -1;
-}
+constexpr int kMaxParts = 1024;           // sub-batches of a batch
+constexpr long long kClaimRequests = 65536;   // candidates from which a batch's rows are fetched once each
 
-// Staged rerank transport: candidate rows come back to the host, host threads gather the exact rows into two
-// pinned buffers, and cudaMemcpyAsync moves each filled buffer while the other is being filled.
-// h_cand: the candidates on the host; d_stage: destination [nq][width][row bytes]; copies are queued on `stream`.
-psb_status staged_gather_host(psb_session* s, const int* h_cand, int nq, int width, int stride, void* d_stage, cudaStream_t stream) {
+// Staged rerank transport: host threads gather exact rows into two pinned buffers, and cudaMemcpyAsync moves each filled buffer
+// while the other is being filled.  h_rows: the rows of `count` consecutive slots; d_stage: the first slot's place; copies are queued
+// on `stream`.
+psb_status staged_gather_host(psb_session* s, const int* h_rows, size_t count, void* d_stage, cudaStream_t stream) {
+    if (count == 0) return PSB_OK;
     const size_t row_bytes = (size_t)s->dim * s->exact_elem;
-    const size_t chunk_q = std::max<size_t>(1, ((size_t)64 << 20) / std::max<size_t>(1, row_bytes * width));
-    const size_t need = chunk_q * width * row_bytes;
+    const size_t chunk = std::max<size_t>(1, ((size_t)64 << 20) / std::max<size_t>(1, row_bytes));
+    const size_t need = std::min(chunk, std::max<size_t>(count, 4096)) * row_bytes;
     if (s->pinned_bytes < need) {
         for (int i = 0; i < 2; ++i) {
             if (s->pinned_used[i]) PSB_CUDA(cudaEventSynchronize(s->pinned_ev[i]));  // no copy may still read the old buffer
@@ -723,59 +722,85 @@ psb_status staged_gather_host(psb_session* s, const int* h_cand, int nq, int wid
         s->host_pool.reset(new HostPool((int)std::min<unsigned>(hc, 64)));
     }
     const int nthreads = s->host_pool->size();
+    const size_t per = s->pinned_bytes / row_bytes;
     // The ring state outlives the call: the next call may start while this call's last copy is still in flight.
-    for (size_t q0 = 0; q0 < (size_t)nq; q0 += chunk_q, s->pinned_slot ^= 1) {
+    for (size_t i0 = 0; i0 < count; i0 += per, s->pinned_slot ^= 1) {
         const int slot = s->pinned_slot;
-        const size_t n = std::min(chunk_q, (size_t)nq - q0);
+        const size_t total = std::min(per, count - i0);
         if (s->pinned_used[slot]) PSB_CUDA(cudaEventSynchronize(s->pinned_ev[slot]));
         unsigned char* dst = static_cast<unsigned char*>(s->pinned[slot]);
         const unsigned char* src = static_cast<const unsigned char*>(s->exact_host);
-        const size_t total = n * width;
+        const int* rows = h_rows + i0;
         const auto t_begin = std::chrono::steady_clock::now();
         s->host_pool->run([&](int t) {
-            // Rows sit at random places of a host array far larger than the caches: each copy would wait for DRAM.  The rows of
-            // the next kAhead candidates are resolved and prefetched while the current one is copied, so a thread keeps
-            // several misses in flight.
-            constexpr int kAhead = 8;
+            // Rows sit at random places of a host array far larger than the caches: each copy would wait for DRAM.  The row kAhead
+            // places on is prefetched while the current one is copied, so a thread keeps several misses in flight.
+            constexpr size_t kAhead = 8;
             const size_t b = total * t / nthreads, e = total * (t + 1) / nthreads;
-            long long rows[kAhead];
-            auto resolve = [&](size_t i) -> long long {
-                const size_t q = q0 + i / width, c = i % width;
-                const long long row = host_local_row(s, h_cand[q * stride + c]);
-                return (row >= 0 && row < s->exact_count) ? row : -1;
+            auto prefetch = [&](size_t i) {
+                for (size_t off = 0; off < row_bytes; off += 64) __builtin_prefetch(src + (size_t)rows[i] * row_bytes + off, 0, 0);
             };
-            for (size_t i = b; i < std::min(e, b + kAhead); ++i) {
-                rows[i % kAhead] = resolve(i);
-                if (rows[i % kAhead] >= 0)
-                    for (size_t off = 0; off < row_bytes; off += 64) __builtin_prefetch(src + (size_t)rows[i % kAhead] * row_bytes + off, 0, 0);
-            }
+            for (size_t i = b; i < std::min(e, b + kAhead); ++i) prefetch(i);
             for (size_t i = b; i < e; ++i) {
-                const long long row = rows[i % kAhead];
-                if (i + kAhead < e) {
-                    const long long nx = resolve(i + kAhead);
-                    rows[i % kAhead] = nx;
-                    if (nx >= 0)
-                        for (size_t off = 0; off < row_bytes; off += 64) __builtin_prefetch(src + (size_t)nx * row_bytes + off, 0, 0);
-                }
-                if (row >= 0) std::memcpy(dst + i * row_bytes, src + (size_t)row * row_bytes, row_bytes);
+                if (i + kAhead < e) prefetch(i + kAhead);
+                std::memcpy(dst + i * row_bytes, src + (size_t)rows[i] * row_bytes, row_bytes);
             }
         });
         s->staged_gather_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - t_begin).count();
         s->staged_gather_bytes += (long long)(total * row_bytes);
-        PSB_CUDA(cudaMemcpyAsync(static_cast<unsigned char*>(d_stage) + q0 * width * row_bytes, dst, total * row_bytes,
-                                 cudaMemcpyHostToDevice, stream));
+        PSB_CUDA(cudaMemcpyAsync(static_cast<unsigned char*>(d_stage) + i0 * row_bytes, dst, total * row_bytes, cudaMemcpyHostToDevice, stream));
         PSB_CUDA(cudaEventRecord(s->pinned_ev[slot], stream));
         s->pinned_used[slot] = true;
     }
     return PSB_OK;
 }
 
-psb_status staged_gather(psb_session* s, const int* d_cand, int nq, int width, int stride, const int* d_counts) {
-    (void)d_counts;
-    s->h_cand.resize((size_t)nq * stride);
-    PSB_CUDA(cudaMemcpyAsync(s->h_cand.data(), d_cand, sizeof(int) * (size_t)nq * stride, cudaMemcpyDeviceToHost, s->stream));
-    PSB_CUDA(cudaStreamSynchronize(s->stream));
-    return staged_gather_host(s, s->h_cand.data(), nq, width, stride, s->stage.p, s->stream);
+// The rows of one batch (of one rerank call): claimed part by part, fetched once each, released at the end.  All of a batch's claims,
+// fetches and scores are ordered by the caller's streams and events.
+psb_status rows_begin(psb_session* s, long long requests, cudaStream_t st) {
+    const size_t slots = (size_t)std::max<long long>(1, std::min(requests, s->exact_count));
+    PSB_TRY(s->unique.reserve(sizeof(int) * slots));
+    PSB_TRY(s->marks.reserve(sizeof(int) * (kMaxParts + 2)));
+    PSB_TRY(s->stage.reserve(slots * s->dim * s->exact_elem));
+    const bool fresh = s->slot_of.p == nullptr;
+    PSB_TRY(s->slot_of.reserve(sizeof(int) * (size_t)std::max<long long>(1, s->exact_count)));
+    if (fresh || s->slots_dirty) PSB_CUDA(cudaMemsetAsync(s->slot_of.p, 0xff, s->slot_of.bytes, st));
+    s->slots_dirty = true;
+    PSB_CUDA(cudaMemsetAsync(s->marks.p, 0, sizeof(int) * (kMaxParts + 2), st));
+    return PSB_OK;
+}
+int* part_begin(const psb_session* s, int part) { return s->marks.as<int>() + 1 + part; }
+int* part_end(const psb_session* s, int part) { return s->marks.as<int>() + 2 + part; }
+psb_status rows_claim(psb_session* s, int part, const int* d_cand, int nq, int width, int stride, const int* d_counts, cudaStream_t st) {
+    PSB_TRY(launch_claim_rows(s->row_map(), d_cand, nq, width, stride, d_counts, s->slot_of.as<int>(), s->unique.as<int>(), s->marks.as<int>(), st));
+    PSB_CUDA(cudaMemcpyAsync(part_end(s, part), s->marks.p, sizeof(int), cudaMemcpyDeviceToDevice, st));
+    return PSB_OK;
+}
+psb_status rows_end(psb_session* s, cudaStream_t st) {
+    PSB_TRY(launch_release_rows(s->unique.as<int>(), s->marks.as<int>(), s->slot_of.as<int>(), s->sm_count, st));
+    s->slots_dirty = false;
+    return PSB_OK;
+}
+// Queues the copy of a part's slot range to the host behind its claim (h_marks[2 part], [2 part + 1] once `st` gets there).
+psb_status rows_tell_host(psb_session* s, int part, cudaStream_t st) {
+    if (!s->h_marks) PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_marks), sizeof(int) * 2 * kMaxParts, cudaHostAllocDefault));
+    PSB_CUDA(cudaMemcpyAsync(s->h_marks + 2 * part, part_begin(s, part), sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+    return PSB_OK;
+}
+// The host threads' share of a part whose claim is done: slot list to the host, rows to their slots (copies on `st`).
+psb_status rows_from_host(psb_session* s, int part, int host_pct, cudaStream_t st) {
+    const int b = s->h_marks[2 * part], e = host_share_end(b, s->h_marks[2 * part + 1], host_pct);
+    if (e <= b) return PSB_OK;
+    if (!s->list_stream) PSB_CUDA(cudaStreamCreateWithFlags(&s->list_stream, cudaStreamNonBlocking));
+    if (s->h_unique_count < (size_t)(e - b)) {
+        if (s->h_unique) cudaFreeHost(s->h_unique);
+        s->h_unique = nullptr; s->h_unique_count = 0;
+        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_unique), sizeof(int) * (size_t)(e - b), cudaHostAllocDefault));
+        s->h_unique_count = (size_t)(e - b);
+    }
+    PSB_CUDA(cudaMemcpyAsync(s->h_unique, s->unique.as<int>() + b, sizeof(int) * (size_t)(e - b), cudaMemcpyDeviceToHost, s->list_stream));
+    PSB_CUDA(cudaStreamSynchronize(s->list_stream));
+    return staged_gather_host(s, s->h_unique, (size_t)(e - b), static_cast<unsigned char*>(s->stage.p) + (size_t)b * s->dim * s->exact_elem, st);
 }
 
 // The stream of the hybrid transport's gather kernel.  Highest priority: its few CTAs each need an SM to themselves and must be
@@ -788,53 +813,72 @@ psb_status ensure_zc_stream(psb_session* s) {
     return PSB_OK;
 }
 
+// The host threads' share of the rows, in percent.
+int host_share(const psb_session* s) {
+    if (s->opt.exact_mode == PSB_EXACT_HOST_STAGED || !s->exact_dev) return 100;
+    return s->opt.exact_mode == PSB_EXACT_HOST_HYBRID ? 100 - (s->opt.zero_copy_pct > 0 ? s->opt.zero_copy_pct : 45) : 0;
+}
+bool device_rows(const psb_session* s) { return s->opt.exact_mode == PSB_EXACT_RESIDENT || s->opt.exact_mode == PSB_EXACT_HOST_CACHED; }
+// Rows scored where they lie: in device memory, or so few that fetching each once would not pay for its launches.
+bool rows_in_place(const psb_session* s, long long requests) {
+    return device_rows(s) || (s->exact_dev && s->opt.exact_mode != PSB_EXACT_HOST_STAGED && requests < kClaimRequests);
+}
+
+// Scores and selection of one part, the rows being in place or in their slots.  d_ids_out: original ids instead of rows.
+psb_status score_and_select(psb_session* s, bool in_place, const void* d_queries, int nq, const int* d_cand, int width, int stride, const int* d_counts,
+                            int topk, int* d_out_rows, float* d_out_dist, long long* d_out_ids, float* d_score, cudaStream_t st) {
+    PSB_TRY(launch_rerank_score(in_place ? s->exact_dev : s->stage.p, in_place ? nullptr : s->slot_of.as<int>(), s->row_map(), s->dim, s->exact_elem,
+                                d_queries, d_cand, nq, width, stride, d_counts, d_score, st));
+    if (!d_out_rows && !d_out_ids) return PSB_OK;  // partial rerank: the caller combines the scores of all shards
+    return launch_topk_select(d_score, d_cand, nq, width, stride, d_counts, topk, d_out_rows, d_out_dist, st, s->reordered.as<long long>(), d_out_ids);
+}
+
 psb_status rerank_impl(psb_session* s, const void* d_queries, int nq, const int* d_cand, int width, int stride,
-                       const int* d_counts, int topk, int* d_out_rows, float* d_out_dist, float* d_score = nullptr) {
+                       const int* d_counts, int topk, int* d_out_rows, float* d_out_dist, float* d_score = nullptr, long long* d_out_ids = nullptr) {
     if (!s->exact_elem) return fail(PSB_INVALID_ARGUMENT, "session has no exact rows for the rerank");
     if (width <= 0 || stride < width || topk <= 0) return fail(PSB_INVALID_ARGUMENT, "invalid rerank request");
     if (width > kMaxRerankWidth || topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "rerank width above 4096 or topk above 2048");
-    PSB_TRY(s->stage.reserve((size_t)nq * width * s->dim * s->exact_elem));
-    const int zc_pct = s->opt.zero_copy_pct > 0 ? s->opt.zero_copy_pct : 45;
-    const int mz = (int)((long long)nq * zc_pct / 100);
-    if (s->opt.exact_mode == PSB_EXACT_HOST_HYBRID && s->exact_dev && mz > 0 && mz < nq && (long long)nq * width >= 65536) {
-        // Both transports for one stage call (the sharded step's exchange half): the kernel gathers the rows of the last mz
-        // queries on a stream of its own while this thread gathers the others through the pinned rings.  The call blocks for
-        // the host gather; a caller that overlaps it with a scan queues that scan first.
-        const int mh = nq - mz;
-        const size_t row_bytes = (size_t)s->dim * s->exact_elem;
-        const bool beside = s->background || (s->aux_stream != nullptr && s->stream == s->aux_stream);
-        PSB_TRY(ensure_zc_stream(s));
-        if (!s->zc_ev_a) PSB_CUDA(cudaEventCreateWithFlags(&s->zc_ev_a, cudaEventDisableTiming));
-        if (!s->zc_ev_b) PSB_CUDA(cudaEventCreateWithFlags(&s->zc_ev_b, cudaEventDisableTiming));
-        PSB_CUDA(cudaEventRecord(s->zc_ev_a, s->stream));
-        PSB_CUDA(cudaStreamWaitEvent(s->zc_stream, s->zc_ev_a, 0));
-        PSB_TRY(launch_gather_rows(s->exact_dev, s->row_map(), s->dim, s->exact_elem, d_cand + (size_t)mh * stride, mz, width, stride,
-                                   d_counts ? d_counts + mh : nullptr, static_cast<unsigned char*>(s->stage.p) + (size_t)mh * width * row_bytes,
-                                   s->zc_stream, s->sm_count, 0, beside && s->opt.gather_ctas == 0 ? (s->opt.reserve_sms > 0 ? s->opt.reserve_sms : 8) : 0));
-        PSB_CUDA(cudaEventRecord(s->zc_ev_b, s->zc_stream));
-        PSB_TRY(staged_gather(s, d_cand, mh, width, stride, d_counts));
-        PSB_CUDA(cudaStreamWaitEvent(s->stream, s->zc_ev_b, 0));
-    } else if (staged_mode(s) && !(s->opt.exact_mode == PSB_EXACT_HOST_HYBRID && s->exact_dev && mz >= nq)) {
-        PSB_TRY(staged_gather(s, d_cand, nq, width, stride, d_counts));
-    } else {
-        // Beside a scan on the other stream the gather runs on SMs of its own: the ones the scan's persistent grid leaves free
-        // (reserve_sms), or gather_ctas lean CTAs spread over all SMs when the caller asks for that.
-        const bool beside = s->background || (s->aux_stream != nullptr && s->stream == s->aux_stream);
-        const bool host_rows = s->opt.exact_mode == PSB_EXACT_HOST_MAPPED || s->opt.exact_mode == PSB_EXACT_HOST_HYBRID;
-        const int owned = beside && host_rows && s->opt.gather_ctas == 0 ? (s->opt.reserve_sms > 0 ? s->opt.reserve_sms : 8) : 0;
-        PSB_TRY(launch_gather_rows(s->exact_dev, s->row_map(), s->dim, s->exact_elem, d_cand, nq, width, stride, d_counts,
-                                   s->stage.p, s->stream, s->sm_count,
-                                   beside ? (s->opt.gather_ctas > 0 ? s->opt.gather_ctas : 2 * s->sm_count) : 0, owned));
-    }
+    if (nq <= 0) return PSB_OK;
     float* score = d_score;
     if (!score) {
         PSB_TRY(s->score.reserve(sizeof(float) * (size_t)nq * width));
         score = s->score.as<float>();
     }
-    PSB_TRY(launch_rerank_score(s->stage.p, s->row_map(), s->dim, s->exact_elem, d_queries, d_cand, nq, width, stride,
-                                d_counts, score, s->stream));
-    if (!d_out_rows) return PSB_OK;  // partial rerank: the caller combines the scores of all shards
-    return launch_topk_select(score, d_cand, nq, width, stride, d_counts, topk, d_out_rows, d_out_dist, s->stream);
+    const bool in_place = rows_in_place(s, (long long)nq * width);
+    if (!in_place) {
+        PSB_TRY(rows_begin(s, (long long)nq * width, s->stream));
+        PSB_TRY(rows_claim(s, 0, d_cand, nq, width, stride, d_counts, s->stream));
+        const int host_pct = host_share(s);
+        const int row_bytes = s->dim * s->exact_elem;
+        // Beside a scan on the other stream the gather kernel runs on SMs of its own: the ones the scan's persistent grid leaves free
+        // (reserve_sms), or gather_ctas lean CTAs spread over all SMs when the caller asks for that.
+        const bool beside = s->background || (s->aux_stream != nullptr && s->stream == s->aux_stream);
+        const int owned = beside && s->opt.gather_ctas == 0 ? (s->opt.reserve_sms > 0 ? s->opt.reserve_sms : 8) : 0;
+        const int lean = beside ? s->opt.gather_ctas : 0;
+        if (host_pct == 0) {
+            PSB_TRY(launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, 0), part_end(s, 0), 0, s->stage.p, s->stream,
+                                         s->sm_count, lean, owned));
+        } else {
+            // This thread and the host pool bring their share while the kernel, on a stream of its own, brings the rest.  The call
+            // blocks for the host gather; a caller that overlaps it with a scan queues that scan first.
+            PSB_TRY(rows_tell_host(s, 0, s->stream));
+            if (host_pct < 100) {
+                PSB_TRY(ensure_zc_stream(s));
+                if (!s->zc_ev_a) PSB_CUDA(cudaEventCreateWithFlags(&s->zc_ev_a, cudaEventDisableTiming));
+                if (!s->zc_ev_b) PSB_CUDA(cudaEventCreateWithFlags(&s->zc_ev_b, cudaEventDisableTiming));
+                PSB_CUDA(cudaEventRecord(s->zc_ev_a, s->stream));
+                PSB_CUDA(cudaStreamWaitEvent(s->zc_stream, s->zc_ev_a, 0));
+                PSB_TRY(launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, 0), part_end(s, 0), host_pct, s->stage.p,
+                                             s->zc_stream, s->sm_count, 0, owned));
+                PSB_CUDA(cudaEventRecord(s->zc_ev_b, s->zc_stream));
+            }
+            PSB_CUDA(cudaStreamSynchronize(s->stream));
+            PSB_TRY(rows_from_host(s, 0, host_pct, s->stream));
+            if (host_pct < 100) PSB_CUDA(cudaStreamWaitEvent(s->stream, s->zc_ev_b, 0));
+        }
+    }
+    PSB_TRY(score_and_select(s, in_place, d_queries, nq, d_cand, width, stride, d_counts, topk, d_out_rows, d_out_dist, d_out_ids, score, s->stream));
+    return in_place ? PSB_OK : rows_end(s, s->stream);
 }
 
 }  // namespace
@@ -927,7 +971,6 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
     if (gb) {
         s->striped = true;
         s->h_global_begin.assign(gb, gb + nlist);
-        s->h_offsets.assign(index->lists.offsets, index->lists.offsets + nlist + 1);
         std::vector<long long> delta((size_t)nlist);
         for (int l = 0; l < nlist; ++l) delta[(size_t)l] = gb[l] - index->lists.offsets[l];
         PSB_TRY(s->global_begin.reserve(sizeof(long long) * (size_t)nlist));
@@ -1362,7 +1405,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         PSB_CUDA(cudaStreamWaitEvent(sx, e0, 0));
     }
     psb_status rc = PSB_OK;
-    struct Job { int p0, m; cudaEvent_t ready; int mz; cudaEvent_t gathered; };
+    struct Job { int part, p0, m; cudaEvent_t ready; cudaEvent_t gathered; };
     std::mutex mu;
     std::condition_variable cv;
     std::deque<Job> jobs;
@@ -1370,45 +1413,45 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     psb_status worker_rc = PSB_OK;
     std::string worker_msg;
     std::thread worker;
-    const bool hybrid = staged_overlap && s->opt.exact_mode == PSB_EXACT_HOST_HYBRID && s->exact_dev != nullptr;
-    const int zc_pct = s->opt.zero_copy_pct > 0 ? s->opt.zero_copy_pct : 45;
+    // The rows of the whole batch are claimed and fetched once each, sub-batch by sub-batch (a row an earlier sub-batch has fetched is
+    // in its slot already), unless they are scored in place.
+    const int host_pct = host_share(s);
+    const bool hybrid = staged_overlap && host_pct < 100;
+    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k) && cuts.size() <= (size_t)kMaxParts);
+    const int row_bytes = s->dim * s->exact_elem;
     if (hybrid) PSB_TRY(ensure_zc_stream(s));
-    if (staged_overlap) {
-        const size_t cand_count = (size_t)n * stage1_k;
-        if (s->h_cand_pinned_count < cand_count) {
-            if (s->h_cand_pinned) cudaFreeHost(s->h_cand_pinned);
-            s->h_cand_pinned = nullptr; s->h_cand_pinned_count = 0;
-            PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_cand_pinned), sizeof(int) * cand_count, cudaHostAllocDefault));
-            s->h_cand_pinned_count = cand_count;
-        }
-        // Hybrid transport: every sub-batch has a staging region of its own (the whole batch: nq * stage1_k rows of device
-        // memory), so that the gather kernel of a sub-batch depends on nothing but that sub-batch's scan.
-        PSB_TRY(s->stage.reserve((size_t)(hybrid ? n : sb_max) * stage1_k * s->dim * s->exact_elem));
+    if (shared_rows) {
         PSB_TRY(s->score.reserve(sizeof(float) * (size_t)sb_max * stage1_k));
+        PSB_TRY(rows_begin(s, (long long)n * stage1_k, st));
+        cudaEvent_t e0;
+        PSB_CUDA(cudaEventCreateWithFlags(&e0, cudaEventDisableTiming));
+        deps.push_back(e0);
+        PSB_CUDA(cudaEventRecord(e0, st));
+        PSB_CUDA(cudaStreamWaitEvent(sx, e0, 0));
+    }
+    auto score_part = [&](int p0, int m) {
+        const unsigned char* qe = static_cast<const unsigned char*>(dq_exact) + (size_t)p0 * row_bytes;
+        return score_and_select(s, false, qe, m, s->cand_rows.as<int>() + (size_t)p0 * stage1_k, stage1_k, stage1_k, s->cand_count.as<int>() + p0, topk,
+                                s->striped ? s->out_rows.as<int>() + (size_t)p0 * topk : nullptr, d_dist + (size_t)p0 * topk,
+                                s->striped ? nullptr : d_ids + (size_t)p0 * topk, s->score.as<float>(), sx);
+    };
+    if (staged_overlap) {
         worker = std::thread([&]() {
             cudaSetDevice(s->device);
             auto process = [&](const Job& j) -> psb_status {
                 PSB_RANGE("pq_rerank");
                 PSB_CUDA(cudaEventSynchronize(j.ready));
-                const int* cand_d = s->cand_rows.as<int>() + (size_t)j.p0 * stage1_k;
-                const int* cnt_d = s->cand_count.as<int>() + j.p0;
                 if (times) PSB_TRY(tm_x.mark(sx));
-                // Hybrid transport: the rows of the last j.mz queries come through the gather kernel, which the main thread queued
-                // right behind this sub-batch's scan (j.gathered marks its end); the host threads and the copy engine bring the
-                // others; the scoring waits for both.
-                const int mh = j.m - j.mz;
-                unsigned char* region = static_cast<unsigned char*>(s->stage.p) +
-                                        (hybrid ? (size_t)j.p0 * stage1_k * s->dim * s->exact_elem : 0);
-                if (mh > 0) PSB_TRY(staged_gather_host(s, s->h_cand_pinned + (size_t)j.p0 * stage1_k, mh, stage1_k, stage1_k, region, sx));
-                if (j.mz > 0) PSB_CUDA(cudaStreamWaitEvent(sx, j.gathered, 0));
-                const unsigned char* qe = static_cast<const unsigned char*>(dq_exact) + (size_t)j.p0 * s->dim * s->exact_elem;
-                PSB_TRY(launch_rerank_score(region, s->row_map(), s->dim, s->exact_elem, qe, cand_d, j.m, stage1_k, stage1_k,
-                                            cnt_d, s->score.as<float>(), sx));
-                PSB_TRY(launch_topk_select(s->score.as<float>(), cand_d, j.m, stage1_k, stage1_k, cnt_d, topk,
-                                           s->out_rows.as<int>() + (size_t)j.p0 * topk, d_dist + (size_t)j.p0 * topk, sx));
+                // Hybrid transport: the kernel's share of the slots comes through the gather kernel, which the main thread queued right
+                // behind this sub-batch's claim (j.gathered marks its end); the host threads and the copy engine bring the others; the
+                // scoring waits for both.
+                PSB_TRY(rows_from_host(s, j.part, host_pct, sx));
+                if (j.gathered) PSB_CUDA(cudaStreamWaitEvent(sx, j.gathered, 0));
+                PSB_TRY(score_part(j.p0, j.m));
                 if (times) PSB_TRY(tm_x.mark(sx));
-                PSB_TRY(launch_map_ids(s->out_rows.as<int>() + (size_t)j.p0 * topk, (long long)j.m * topk,
-                                       s->reordered.as<long long>(), s->row_map(), d_ids + (size_t)j.p0 * topk, sx));
+                if (s->striped)
+                    PSB_TRY(launch_map_ids(s->out_rows.as<int>() + (size_t)j.p0 * topk, (long long)j.m * topk, s->reordered.as<long long>(), s->row_map(),
+                                           d_ids + (size_t)j.p0 * topk, sx));
                 if (times) PSB_TRY(tm_x.mark(sx));
                 return PSB_OK;
             };
@@ -1477,33 +1520,25 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         }
         if (rc == PSB_OK && times) rc = tm_s.mark(st);
         if (rc != PSB_OK) break;
-        if (staged_overlap) {  // hand the sub-batch to the worker: candidates to the host, an event marks them ready
-            cudaEvent_t e;
+        if (staged_overlap) {  // claim the sub-batch's rows and hand it to the worker: an event marks the slot range ready
+            cudaEvent_t e, gathered = nullptr;
             if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) { rc = fail(PSB_CUDA_ERROR, "event creation failed"); break; }
             deps.push_back(e);
-            const int mz = hybrid ? (int)((long long)m * zc_pct / 100) : 0;
-            cudaEvent_t gathered = nullptr;
-            if (mz > 0) {   // the kernel's share of the transfer, queued now: it starts the moment this sub-batch's scan stage ends
-                cudaEvent_t scanned;
-                if (cudaEventCreateWithFlags(&scanned, cudaEventDisableTiming) != cudaSuccess ||
-                    cudaEventCreateWithFlags(&gathered, cudaEventDisableTiming) != cudaSuccess) { rc = fail(PSB_CUDA_ERROR, "event creation failed"); break; }
-                deps.push_back(scanned);
+            rc = rows_claim(s, (int)ci, rows_out, m, stage1_k, stage1_k, cnt_out, st);
+            if (rc == PSB_OK) rc = rows_tell_host(s, (int)ci, st);
+            if (rc != PSB_OK) break;
+            cudaEventRecord(e, st);
+            if (hybrid) {   // the kernel's share of the transfer, queued now: it starts the moment the rows are claimed
+                if (cudaEventCreateWithFlags(&gathered, cudaEventDisableTiming) != cudaSuccess) { rc = fail(PSB_CUDA_ERROR, "event creation failed"); break; }
                 deps.push_back(gathered);
-                cudaEventRecord(scanned, st);
-                cudaStreamWaitEvent(s->zc_stream, scanned, 0);
-                const int mh = m - mz;
+                cudaStreamWaitEvent(s->zc_stream, e, 0);
                 // on the SMs the scan's grid leaves free (reserve_sms), unless the caller asked for lean CTAs on all SMs
-                rc = launch_gather_rows(s->exact_dev, s->row_map(), s->dim, s->exact_elem, rows_out + (size_t)mh * stage1_k, mz, stage1_k, stage1_k,
-                                        cnt_out + mh,
-                                        static_cast<unsigned char*>(s->stage.p) + (size_t)(p0 + mh) * stage1_k * s->dim * s->exact_elem,
-                                        s->zc_stream, s->sm_count, s->opt.gather_ctas > 0 ? s->opt.gather_ctas : 2 * s->sm_count,
-                                        s->opt.gather_ctas > 0 ? 0 : s->opt.reserve_sms);
+                rc = launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, (int)ci), part_end(s, (int)ci), host_pct, s->stage.p,
+                                          s->zc_stream, s->sm_count, s->opt.gather_ctas, s->opt.gather_ctas > 0 ? 0 : s->opt.reserve_sms);
                 if (rc != PSB_OK) break;
                 cudaEventRecord(gathered, s->zc_stream);
             }
-            cudaMemcpyAsync(s->h_cand_pinned + (size_t)p0 * stage1_k, rows_out, sizeof(int) * (size_t)m * stage1_k, cudaMemcpyDeviceToHost, st);
-            cudaEventRecord(e, st);
-            { std::lock_guard<std::mutex> lk(mu); jobs.push_back(Job{p0, m, e, mz, gathered}); }
+            { std::lock_guard<std::mutex> lk(mu); jobs.push_back(Job{(int)ci, p0, m, e, gathered}); }
             cv.notify_all();
             continue;
         }
@@ -1518,14 +1553,24 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         cudaStream_t keep = s->stream;
         s->stream = sx;  // rerank_impl and the launchers below run on s->stream
         if (times) rc = tm_x.mark(sx);
+        bool mapped_ids = false;
         if (rc == PSB_OK && rerank) {
             PSB_RANGE("pq_rerank");
-            const unsigned char* qe = static_cast<const unsigned char*>(dq_exact) + (size_t)p0 * s->dim * s->exact_elem;
-            rc = rerank_impl(s, qe, m, rows_out, stage1_k, stage1_k, cnt_out, topk, s->out_rows.as<int>() + (size_t)p0 * topk,
-                             d_dist + (size_t)p0 * topk);
+            mapped_ids = !s->striped;
+            if (shared_rows) {
+                rc = rows_claim(s, (int)ci, rows_out, m, stage1_k, stage1_k, cnt_out, sx);
+                if (rc == PSB_OK)
+                    rc = launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, (int)ci), part_end(s, (int)ci), 0, s->stage.p, sx,
+                                              s->sm_count, s->opt.gather_ctas, s->opt.gather_ctas > 0 ? 0 : (s->opt.reserve_sms > 0 ? s->opt.reserve_sms : 8));
+                if (rc == PSB_OK) rc = score_part(p0, m);
+            } else {
+                const unsigned char* qe = static_cast<const unsigned char*>(dq_exact) + (size_t)p0 * row_bytes;
+                rc = rerank_impl(s, qe, m, rows_out, stage1_k, stage1_k, cnt_out, topk, mapped_ids ? nullptr : s->out_rows.as<int>() + (size_t)p0 * topk,
+                                 d_dist + (size_t)p0 * topk, nullptr, mapped_ids ? d_ids + (size_t)p0 * topk : nullptr);
+            }
         }
         if (rc == PSB_OK && times) rc = tm_x.mark(sx);
-        if (rc == PSB_OK) {
+        if (rc == PSB_OK && !mapped_ids) {
             PSB_RANGE("pq_map_ids");
             rc = launch_map_ids(s->out_rows.as<int>() + (size_t)p0 * topk, (long long)m * topk, s->reordered.as<long long>(),
                                 s->row_map(), d_ids + (size_t)p0 * topk, sx);
@@ -1535,6 +1580,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     }
     finish_worker();
     if (worker_rc != PSB_OK && rc == PSB_OK) rc = fail(worker_rc, "rerank worker: " + worker_msg);
+    if (shared_rows && rc == PSB_OK) rc = rows_end(s, sx);
     if (overlap || staged_overlap) {  // the main stream continues only after the second stream has finished this batch
         cudaEvent_t e;
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) {
@@ -1840,15 +1886,13 @@ psb_status psb_rerank_host(const psb_host_storage_view* storage, const uint8_t* 
             if (h_candidate_counts[q] < 0 || h_candidate_counts[q] > candidate_count)
                 return fail(PSB_INVALID_ARGUMENT, "host rerank candidate count exceeds row width");
     if (candidate_count > kMaxRerankWidth || topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "rerank width above 4096 or topk above 2048");
-    int sms = 0;
-    PSB_TRY(check_device(device, &sms));
+    PSB_TRY(check_device(device));
     const int elem = use_float ? 4 : 1;
     const int dim = storage->dim;
     const size_t base_bytes = (size_t)storage->count * dim * elem;
-    DevBuf base, q, cand, counts, stage, out_rows, out_dist;
+    DevBuf base, q, cand, counts, out_rows, out_dist;
     PSB_TRY(base.reserve(base_bytes)); PSB_TRY(q.reserve((size_t)batch_n * dim * elem));
     PSB_TRY(cand.reserve(sizeof(int) * (size_t)batch_n * candidate_stride));
-    PSB_TRY(stage.reserve((size_t)batch_n * candidate_count * dim * elem));
     PSB_TRY(out_rows.reserve(sizeof(int) * (size_t)batch_n * topk)); PSB_TRY(out_dist.reserve(sizeof(float) * (size_t)batch_n * topk));
     cudaStream_t st = nullptr;
     PSB_CUDA(cudaMemcpy(base.p, use_float ? (const void*)storage->fp32 : (const void*)storage->u8, base_bytes, cudaMemcpyHostToDevice));
@@ -1864,9 +1908,7 @@ psb_status psb_rerank_host(const psb_host_storage_view* storage, const uint8_t* 
     mp.count = storage->count;
     DevBuf score;
     PSB_TRY(score.reserve(sizeof(float) * (size_t)batch_n * candidate_count));
-    PSB_TRY(launch_gather_rows(base.p, mp, dim, elem, cand.as<int>(), batch_n, candidate_count, candidate_stride,
-                               d_counts, stage.p, st, sms));
-    PSB_TRY(launch_rerank_score(stage.p, mp, dim, elem, q.p, cand.as<int>(), batch_n, candidate_count, candidate_stride,
+    PSB_TRY(launch_rerank_score(base.p, nullptr, mp, dim, elem, q.p, cand.as<int>(), batch_n, candidate_count, candidate_stride,
                                 d_counts, score.as<float>(), st));
     PSB_TRY(launch_topk_select(score.as<float>(), cand.as<int>(), batch_n, candidate_count, candidate_stride, d_counts,
                                topk, out_rows.as<int>(), out_dist.as<float>(), st));

@@ -1,0 +1,53 @@
+"""Exact rerank of batches whose queries name the same rows many times over: every transport fetches a row once, whether in one call, in
+overlapped sub-batches or in a sharded session, batch after batch; rows no 16-byte load can take; candidates given twice."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def index(n, dim, u8, seed):
+    rng = np.random.default_rng(seed)
+    vec = rng.integers(0, 256, (n, dim)).astype(np.uint8) if u8 else rng.standard_normal((n, dim)).astype(np.float32)
+    cen = rng.standard_normal((4, dim)).astype(np.float32)
+    m = 4 if dim % 4 == 0 else 3
+    return dict(centroids=cen, offsets=np.array([0, n // 4, n // 2, n // 2, n], np.int64), reordered_ids=rng.permutation(n).astype(np.int64),
+                codes=rng.integers(0, 16, (n, m)).astype(np.uint8), codebook=rng.standard_normal((m, 16, dim // m)).astype(np.float32), vectors=vec)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 3, 4])
+@pytest.mark.parametrize("dim,u8,nq,width", [(32, False, 700, 100), (33, False, 700, 100), (30, True, 70, 1000), (100, True, 700, 100), (9, True, 20, 64)])
+def test_rows_named_many_times(psb, mode, dim, u8, nq, width):
+    import torch
+    ix = index(1500, dim, u8, dim + mode)
+    rng = np.random.default_rng(nq)
+    with psb.Session(ix, n_rerank=width, exact_mode=mode, max_batch=nq) as s:
+        for again in range(3):
+            q = rng.integers(0, 256, (nq, dim)).astype(np.uint8) if u8 else rng.standard_normal((nq, dim)).astype(np.float32)
+            cand = np.stack([rng.permutation(1500)[:width] for _ in range(nq)]).astype(np.int32)
+            cand[:, 5] = -1
+            cand[::3, 7] = cand[::3, 3]          # a candidate twice
+            cand[1, :] = cand[1, 0]              # only one row
+            cnt = rng.integers(0, width + 1, nq).astype(np.int32)
+            rows = torch.empty((nq, 10), dtype=torch.int32, device="cuda"); dist = torch.empty((nq, 10), device="cuda")
+            s.stage_rerank(torch.from_numpy(q).cuda(), nq, torch.from_numpy(cand).cuda(), width, width, torch.from_numpy(cnt).cuda(), 10, rows, dist)
+            s.sync()
+            masked = np.where(np.arange(width)[None, :] < cnt[:, None], cand, -1)
+            wi, wd = oracle.rerank(ix["vectors"], q, masked, 10)
+            assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 4])
+def test_overlapped_batches_share_rows(psb, mode):
+    ix = index(3000, 32, False, 7)
+    q = np.random.default_rng(8).standard_normal((2500, 32)).astype(np.float32)
+    want = oracle.ivfpq_search(ix, q[:200], 3, 10, 60)
+    with psb.Session(ix, n_rerank=60, exact_mode=3) as s:
+        ref = s.search(q, 3, 10, batch_size=2500)
+    with psb.Session(ix, n_rerank=60, exact_mode=mode) as s:
+        for _ in range(2):
+            got = s.search(q, 3, 10, batch_size=2500)
+            assert np.array_equal(got["indices"], ref["indices"]) and np.array_equal(got["distances"], ref["distances"])
+    assert np.array_equal(ref["indices"][:200], want["indices"]) and np.array_equal(ref["distances"][:200], want["distances"])
