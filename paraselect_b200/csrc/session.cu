@@ -182,12 +182,28 @@ private:
     bool stop_ = false;
 };
 
-struct EventTimer {
+// Timing events of a session, used over and over (creating and destroying the fifteen of a search took longer than recording them).
+struct EventPool {
     std::vector<cudaEvent_t> ev;
-    ~EventTimer() { for (auto e : ev) cudaEventDestroy(e); }
+    size_t used = 0;
+    ~EventPool() { for (auto e : ev) cudaEventDestroy(e); }
+    psb_status get(cudaEvent_t* out) {
+        if (used == ev.size()) {
+            cudaEvent_t e;
+            PSB_CUDA(cudaEventCreate(&e));
+            ev.push_back(e);
+        }
+        *out = ev[used++];
+        return PSB_OK;
+    }
+};
+struct EventTimer {
+    EventPool* pool;
+    std::vector<cudaEvent_t> ev;
+    explicit EventTimer(EventPool* p) : pool(p) {}
     psb_status mark(cudaStream_t s) {
         cudaEvent_t e;
-        PSB_CUDA(cudaEventCreate(&e));
+        PSB_TRY(pool->get(&e));
         ev.push_back(e);
         PSB_CUDA(cudaEventRecord(e, s));
         return PSB_OK;
@@ -317,6 +333,14 @@ struct psb_session {
     bool row_bias_is_u16 = false;          // row_bias holds the caller's affine u16 row correction
     bool flat = false;                     // IVF-Flat session: exact rows resident in flat_rows, no PQ parts
     DevBuf flat_rows, flat_slot;
+    EventPool timing, timing_aux;          // events of the main stream's marks and of the second stream's (set from one thread each)
+    // Host side of a search call: one pinned block through which a small batch's queries and results pass, and the device's counters
+    // and status words with the results, so that a call waits for the GPU once.
+    unsigned char* h_io = nullptr;
+    size_t h_io_bytes = 0;
+    struct Tail { unsigned long long c[16]; int tc[8]; };
+    Tail* h_tail = nullptr;                // pinned
+    bool counters_known = false;           // h_tail->c is what the device's counters hold
     DevBuf row_dist, row_seg;              // a row of distances per query (IVF-Flat, row form of the ADC scan)
     std::vector<long long> longest;        // [p] = rows of this shard's p longest lists together
     double own_list_rows = 0.0;            // expected length of the list a random row lies in
@@ -363,6 +387,8 @@ struct psb_session {
             if (pinned[i]) cudaFreeHost(pinned[i]);
             if (pinned_ev[i]) cudaEventDestroy(pinned_ev[i]);
         }
+        if (h_io) cudaFreeHost(h_io);
+        if (h_tail) cudaFreeHost(h_tail);
         if (h_unique) cudaFreeHost(h_unique);
         if (h_marks) cudaFreeHost(h_marks);
         if (list_stream) { cudaStreamSynchronize(list_stream); cudaStreamDestroy(list_stream); }
@@ -1218,6 +1244,7 @@ psb_status psb_stage_scan_queries(psb_session* s, const float* d_queries, const 
     if (!s || !d_probes || !d_rows) return fail(PSB_INVALID_ARGUMENT, "null argument");
     if (nprobe <= 0 || stage1_k <= 0) return fail(PSB_INVALID_ARGUMENT, "nprobe and stage1_k must be positive");
     if (nprobe > kMaxProbe || stage1_k > kMaxStage1) return fail(PSB_UNSUPPORTED_SHAPE, "nprobe above 4096 or stage1_k above 2048");
+    s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, d_queries != nullptr && rows_form(s, nq, nprobe, true)));
     ScanWorkspace ws;
@@ -1244,6 +1271,7 @@ psb_status psb_stage_scan_sample(psb_session* s, const float* d_queries, const f
     PSB_RANGE("pq_adc_scan_sample");
     PSB_TRY(check_scan_stage(s, d_probes, nprobe, stage1_k));
     if (!d_samples) return fail(PSB_INVALID_ARGUMENT, "null argument");
+    s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, false));
     ScanWorkspace ws;
@@ -1258,6 +1286,7 @@ psb_status psb_stage_scan_shared(psb_session* s, const float* d_queries, const f
     PSB_RANGE("pq_adc_scan");
     PSB_TRY(check_scan_stage(s, d_probes, nprobe, stage1_k));
     if (!d_all_samples || !d_rows || shards <= 0) return fail(PSB_INVALID_ARGUMENT, "null argument or no shards");
+    s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     if (nq > s->ws_scan_queries) return fail(PSB_INVALID_ARGUMENT, "psb_stage_scan_shared follows psb_stage_scan_sample of the same queries");
     ScanWorkspace ws;
@@ -1313,6 +1342,7 @@ psb_status psb_stage_merge(psb_session* s, const int* d_rows, const float* d_dis
 
 psb_status psb_session_counters(psb_session* s, psb_stats* stats, int reset) {
     if (!s || !stats) return fail(PSB_INVALID_ARGUMENT, "null argument");
+    s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (s->scalars.p) {
@@ -1350,7 +1380,62 @@ psb_status psb_session_counters(psb_session* s, psb_stats* stats, int reset) {
 
 namespace {
 
-struct StageTimes { double coarse = 0, lut = 0, scan = 0, rerank = 0, map = 0; };
+// Stage times of one search call: marks are left by search_device and read once the stream has drained.
+struct StageTimes {
+    double coarse = 0, lut = 0, scan = 0, rerank = 0, map = 0;
+    EventTimer tm_s, tm_x;
+    explicit StageTimes(psb_session* s) : tm_s(&s->timing), tm_x(&s->timing_aux) {}
+    void collect() {
+        if (tm_s.ev.size() >= 2) coarse += tm_s.ms(0, 1);
+        for (size_t i = 2; i + 2 < tm_s.ev.size(); i += 3) { lut += tm_s.ms(i, i + 1); scan += tm_s.ms(i + 1, i + 2); }
+        for (size_t i = 0; i + 2 < tm_x.ev.size(); i += 3) { rerank += tm_x.ms(i, i + 1); map += tm_x.ms(i + 1, i + 2); }
+        tm_s.ev.clear(); tm_x.ev.clear();
+        tm_s.pool->used = 0; tm_x.pool->used = 0;
+    }
+};
+
+constexpr size_t kSmallIo = 256 * 1024;   // queries and results of a call that pass through the pinned block
+
+// The pinned block and the tail, large enough; `bytes` of the block are asked for.
+psb_status ensure_host_io(psb_session* s, size_t bytes) {
+    if (s->h_io_bytes < bytes) {
+        if (s->h_io) cudaFreeHost(s->h_io);
+        s->h_io = nullptr; s->h_io_bytes = 0;
+        const size_t want = std::max<size_t>(bytes, 16 * 1024);
+        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_io), want, cudaHostAllocMapped | cudaHostAllocPortable));
+        s->h_io_bytes = want;
+    }
+    if (!s->h_tail) {
+        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_tail), sizeof(psb_session::Tail), cudaHostAllocPortable));
+        std::memset(s->h_tail, 0, sizeof(*s->h_tail));
+    }
+    return PSB_OK;
+}
+// Queues the device's counters and status words behind the work on `st`.
+psb_status queue_tail(psb_session* s, cudaStream_t st) {
+    PSB_CUDA(cudaMemcpyAsync(s->h_tail->c, s->scalars.p, sizeof(s->h_tail->c), cudaMemcpyDeviceToHost, st));
+    if (s->tc_work.scalars.p) PSB_CUDA(cudaMemcpyAsync(s->h_tail->tc, s->tc_work.scalars.p, sizeof(s->h_tail->tc), cudaMemcpyDeviceToHost, st));
+    return PSB_OK;
+}
+// The counters as they are before a call: what the last call left, unless others have run in between.
+psb_status counters_before(psb_session* s, cudaStream_t st, unsigned long long (&c)[4]) {
+    if (!s->counters_known) {
+        PSB_TRY(queue_tail(s, st));
+        PSB_CUDA(cudaStreamSynchronize(st));
+    }
+    std::memcpy(c, s->h_tail->c, sizeof(c));
+    return PSB_OK;
+}
+// Once the stream has drained: the status words the tail brought.
+psb_status check_tail(psb_session* s) {
+    s->counters_known = true;
+    if (s->h_tail->tc[2]) return fail(PSB_TIMEOUT, "a bounded wait in the tensor-core coarse kernel gave up");
+    if ((int)s->h_tail->c[12]) {
+        s->counters_known = false;
+        return s->check_scan_status();
+    }
+    return PSB_OK;
+}
 
 // One batch, device in / device out.  With a rerank from mapped or resident exact rows the batch is cut into
 // sub-batches: coarse + LUT + scan of sub-batch i run on the session's stream while the PCIe gather, exact scoring,
@@ -1396,7 +1481,6 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         ~EventList() { for (auto e : v) cudaEventDestroy(e); }
         void push_back(cudaEvent_t e) { v.push_back(e); }
     } deps;
-    EventTimer tm_s, tm_x;
     if (overlap || staged_overlap) {  // the second stream starts after everything already queued on the main stream
         cudaEvent_t e0;
         PSB_CUDA(cudaEventCreateWithFlags(&e0, cudaEventDisableTiming));
@@ -1441,18 +1525,18 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
             auto process = [&](const Job& j) -> psb_status {
                 PSB_RANGE("pq_rerank");
                 PSB_CUDA(cudaEventSynchronize(j.ready));
-                if (times) PSB_TRY(tm_x.mark(sx));
+                if (times) PSB_TRY(times->tm_x.mark(sx));
                 // Hybrid transport: the kernel's share of the slots comes through the gather kernel, which the main thread queued right
                 // behind this sub-batch's claim (j.gathered marks its end); the host threads and the copy engine bring the others; the
                 // scoring waits for both.
                 PSB_TRY(rows_from_host(s, j.part, host_pct, sx));
                 if (j.gathered) PSB_CUDA(cudaStreamWaitEvent(sx, j.gathered, 0));
                 PSB_TRY(score_part(j.p0, j.m));
-                if (times) PSB_TRY(tm_x.mark(sx));
+                if (times) PSB_TRY(times->tm_x.mark(sx));
                 if (s->striped)
                     PSB_TRY(launch_map_ids(s->out_rows.as<int>() + (size_t)j.p0 * topk, (long long)j.m * topk, s->reordered.as<long long>(), s->row_map(),
                                            d_ids + (size_t)j.p0 * topk, sx));
-                if (times) PSB_TRY(tm_x.mark(sx));
+                if (times) PSB_TRY(times->tm_x.mark(sx));
                 return PSB_OK;
             };
             for (;;) {
@@ -1478,7 +1562,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     };
     // Coarse stage for the whole batch first: one large GEMM is more efficient than four small ones, and the tensor-core
     // kernel (a full SM's shared and tensor memory per CTA) then never has to share SMs with the transfer stream.
-    if (times) rc = tm_s.mark(st);
+    if (times) rc = times->tm_s.mark(st);
     if (rc == PSB_OK) { PSB_RANGE("coarse_search"); rc = coarse_exact(s, dq, n, nprobe, d_probes, nullptr); }
     // OPQ index: the PQ side works on the rotated queries (counted with the coarse stage's time)
     const float* dq_pq = dq;
@@ -1487,7 +1571,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         if (rc == PSB_OK) rc = launch_rotate_rows(dq, s->opq.as<float>(), n, s->dim, s->q_rot.as<float>(), st);
         dq_pq = s->q_rot.as<float>();
     }
-    if (rc == PSB_OK && times) rc = tm_s.mark(st);
+    if (rc == PSB_OK && times) rc = times->tm_s.mark(st);
     for (size_t ci = 0; ci + 1 < cuts.size() && rc == PSB_OK; ++ci) {
         const int p0 = cuts[ci];
         const int m = cuts[ci + 1] - p0;
@@ -1496,7 +1580,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         int* rows_out = rerank ? s->cand_rows.as<int>() + (size_t)p0 * stage1_k : s->out_rows.as<int>() + (size_t)p0 * topk;
         float* dist_out = rerank ? s->cand_dist.as<float>() + (size_t)p0 * stage1_k : d_dist + (size_t)p0 * topk;
         int* cnt_out = s->cand_count.as<int>() + p0;
-        if (times) rc = tm_s.mark(st);
+        if (times) rc = times->tm_s.mark(st);
         ScanWorkspace sws;
         if (rc == PSB_OK) rc = s->timed_scan_ws(&sws);
         if (rc == PSB_OK && !table_free) {
@@ -1513,12 +1597,12 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
                 rc = launch_build_lut(q, m, s->dim, s->codebook.as<float>(), s->m, s->k, s->lut.as<float>(), st);
             }
         }
-        if (rc == PSB_OK && times) rc = tm_s.mark(st);
+        if (rc == PSB_OK && times) rc = times->tm_s.mark(st);
         if (rc == PSB_OK) {
             PSB_RANGE("pq_adc_scan");
             rc = run_scan(s, sws, q, table_free ? nullptr : s->lut.as<float>(), m, probes, nprobe, stage1_k, rows_out, dist_out, cnt_out, st);
         }
-        if (rc == PSB_OK && times) rc = tm_s.mark(st);
+        if (rc == PSB_OK && times) rc = times->tm_s.mark(st);
         if (rc != PSB_OK) break;
         if (staged_overlap) {  // claim the sub-batch's rows and hand it to the worker: an event marks the slot range ready
             cudaEvent_t e, gathered = nullptr;
@@ -1552,7 +1636,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         // second half of the sub-batch (on the second stream when overlapping)
         cudaStream_t keep = s->stream;
         s->stream = sx;  // rerank_impl and the launchers below run on s->stream
-        if (times) rc = tm_x.mark(sx);
+        if (times) rc = times->tm_x.mark(sx);
         bool mapped_ids = false;
         if (rc == PSB_OK && rerank) {
             PSB_RANGE("pq_rerank");
@@ -1569,13 +1653,13 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
                                  d_dist + (size_t)p0 * topk, nullptr, mapped_ids ? d_ids + (size_t)p0 * topk : nullptr);
             }
         }
-        if (rc == PSB_OK && times) rc = tm_x.mark(sx);
+        if (rc == PSB_OK && times) rc = times->tm_x.mark(sx);
         if (rc == PSB_OK && !mapped_ids) {
             PSB_RANGE("pq_map_ids");
             rc = launch_map_ids(s->out_rows.as<int>() + (size_t)p0 * topk, (long long)m * topk, s->reordered.as<long long>(),
                                 s->row_map(), d_ids + (size_t)p0 * topk, sx);
         }
-        if (rc == PSB_OK && times) rc = tm_x.mark(sx);
+        if (rc == PSB_OK && times) rc = times->tm_x.mark(sx);
         s->stream = keep;
     }
     finish_worker();
@@ -1588,16 +1672,6 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
             cudaEventRecord(e, sx);
             cudaStreamWaitEvent(st, e, 0);
         } else if (rc == PSB_OK) rc = fail(PSB_CUDA_ERROR, "event creation failed");
-    }
-    if (times && rc == PSB_OK) {
-        if (cudaStreamSynchronize(st) != cudaSuccess) rc = fail(PSB_CUDA_ERROR, "stream synchronisation failed");
-        if (tm_s.ev.size() >= 2) times->coarse += tm_s.ms(0, 1);
-        for (size_t i = 2; i + 2 < tm_s.ev.size() + 0 && rc == PSB_OK; i += 3) {
-            times->lut += tm_s.ms(i, i + 1); times->scan += tm_s.ms(i + 1, i + 2);
-        }
-        for (size_t i = 0; i + 2 < tm_x.ev.size() + 0 && rc == PSB_OK; i += 3) {
-            times->rerank += tm_x.ms(i, i + 1); times->map += tm_x.ms(i + 1, i + 2);
-        }
     }
     return rc;
 }
@@ -1613,6 +1687,7 @@ psb_status psb_session_search_device(psb_session* s, const float* d_queries, con
     if (params->nprobe > kMaxProbe || params->topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "nprobe above 4096 or topk above 2048");
     if (params->distance != 0) return fail(PSB_UNSUPPORTED_SHAPE, "only squared L2 is supported on this path");
     if (nq == 0) return PSB_OK;
+    s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     const int topk = params->topk;
     const int stage1_k = stage1_width(s, topk);
@@ -1641,53 +1716,70 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
     const bool rerank = rerank_enabled(s, topk);
     if (stage1_k > kMaxStage1) return fail(PSB_UNSUPPORTED_SHAPE, "candidate width above 2048 is not supported");
     PSB_TRY(ensure_pipeline_ws(s, batch, nprobe, topk, stage1_k));
-    if (rerank && s->exact_elem == 1) PSB_TRY(s->q_u8.reserve((size_t)batch * s->dim));
+    const bool u8 = rerank && s->exact_elem == 1;
+    if (u8) PSB_TRY(s->q_u8.reserve((size_t)batch * s->dim));
     cudaStream_t st = s->stream;
+    // A small call's queries go to the device from the pinned block, and its results are written there by the kernels themselves.
+    const size_t b_q = (sizeof(float) * (size_t)total * s->dim + 255) / 256 * 256, b_u8 = u8 ? ((size_t)total * s->dim + 255) / 256 * 256 : 0,
+                 b_ids = sizeof(long long) * (size_t)total * topk, b_dist = sizeof(float) * (size_t)total * topk;
+    const bool small = batch == total && b_q + b_u8 + b_ids + b_dist <= kSmallIo;
+    PSB_TRY(ensure_host_io(s, small ? b_q + b_u8 + b_ids + b_dist : 0));
     const long long launches0 = launches_total();
     unsigned long long c0[4] = {0, 0, 0, 0};
-    if (stats) {
-        PSB_CUDA(cudaMemcpyAsync(c0, s->scalars.p, sizeof(c0), cudaMemcpyDeviceToHost, st));
-        PSB_CUDA(cudaStreamSynchronize(st));
-    }
+    if (stats) PSB_TRY(counters_before(s, st, c0));
+    s->counters_known = false;
     s->collect_scan_events();
     const double scan_ms0 = s->scan_ms_total;
     const long long scan_n0 = s->scan_launches_total;
-    StageTimes times;
+    s->timing.used = s->timing_aux.used = 0;
+    StageTimes times(s);
     double t_h2d = 0, t_d2h = 0, t_total = 0;
     long long h2d = 0, d2h = 0;
     int nb = 0;
     for (int q0 = 0; q0 < total; q0 += batch, ++nb) {
         const int n = std::min(batch, total - q0);
-        EventTimer tm;
+        EventTimer tm(&s->timing);
         if (stats) PSB_TRY(tm.mark(st));
-        PSB_CUDA(cudaMemcpyAsync(s->q.p, queries->fp32 + (size_t)q0 * s->dim, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
+        const void* from = queries->fp32 + (size_t)q0 * s->dim;
+        const void* from_u8 = u8 ? queries->u8 + (size_t)q0 * s->dim : nullptr;
+        if (small) {
+            std::memcpy(s->h_io, from, sizeof(float) * (size_t)n * s->dim);
+            from = s->h_io;
+            if (u8) { std::memcpy(s->h_io + b_q, from_u8, (size_t)n * s->dim); from_u8 = s->h_io + b_q; }
+        }
+        PSB_CUDA(cudaMemcpyAsync(s->q.p, from, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
         h2d += (long long)sizeof(float) * n * s->dim;
-        if (rerank && s->exact_elem == 1) {
-            PSB_CUDA(cudaMemcpyAsync(s->q_u8.p, queries->u8 + (size_t)q0 * s->dim, (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
+        if (u8) {
+            PSB_CUDA(cudaMemcpyAsync(s->q_u8.p, from_u8, (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
             h2d += (long long)n * s->dim;
         }
         if (stats) PSB_TRY(tm.mark(st));
         const void* qe = s->exact_elem == 1 ? s->q_u8.p : s->q.p;
-        PSB_TRY(search_device(s, s->q.as<float>(), qe, n, nprobe, topk, stage1_k, rerank, s->out_ids.as<long long>(),
-                              s->out_dist.as<float>(), s->probes.as<int>(), stats ? &times : nullptr));
+        long long* ids = small ? reinterpret_cast<long long*>(s->h_io + b_q + b_u8) : s->out_ids.as<long long>();
+        float* dist = small ? reinterpret_cast<float*>(s->h_io + b_q + b_u8 + b_ids) : s->out_dist.as<float>();
+        PSB_TRY(search_device(s, s->q.as<float>(), qe, n, nprobe, topk, stage1_k, rerank, ids, dist, s->probes.as<int>(), stats ? &times : nullptr));
         if (stats) PSB_TRY(tm.mark(st));
-        PSB_CUDA(cudaMemcpyAsync(output->indices + (size_t)q0 * topk, s->out_ids.p, sizeof(long long) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
-        PSB_CUDA(cudaMemcpyAsync(output->distances + (size_t)q0 * topk, s->out_dist.p, sizeof(float) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
+        if (!small) {
+            PSB_CUDA(cudaMemcpyAsync(output->indices + (size_t)q0 * topk, ids, sizeof(long long) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
+            PSB_CUDA(cudaMemcpyAsync(output->distances + (size_t)q0 * topk, dist, sizeof(float) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
+        }
         d2h += (long long)(sizeof(long long) + sizeof(float)) * n * topk;
         if (output->coarse_ids) {
             PSB_CUDA(cudaMemcpyAsync(output->coarse_ids + (size_t)q0 * nprobe, s->probes.p, sizeof(int) * (size_t)n * nprobe, cudaMemcpyDeviceToHost, st));
             d2h += (long long)sizeof(int) * n * nprobe;
         }
+        if (q0 + batch >= total) PSB_TRY(queue_tail(s, st));
         if (stats) PSB_TRY(tm.mark(st));
         PSB_CUDA(cudaStreamSynchronize(st));
-        if (stats) { t_h2d += tm.ms(0, 1); t_d2h += tm.ms(2, 3); t_total += tm.ms(0, 3); }
+        if (small) {
+            std::memcpy(output->indices, ids, b_ids);
+            std::memcpy(output->distances, dist, b_dist);
+        }
+        if (stats) { t_h2d += tm.ms(0, 1); t_d2h += tm.ms(2, 3); t_total += tm.ms(0, 3); times.collect(); }
     }
-    PSB_TRY(s->tc_work.check_status());
-    PSB_TRY(s->check_scan_status());
+    PSB_TRY(check_tail(s));
     if (stats) {
-        unsigned long long c1[4];
-        PSB_CUDA(cudaMemcpyAsync(c1, s->scalars.p, sizeof(c1), cudaMemcpyDeviceToHost, st));
-        PSB_CUDA(cudaStreamSynchronize(st));
+        const unsigned long long* c1 = s->h_tail->c;
         stats->h2d_ms = t_h2d; stats->coarse_search_ms = times.coarse; stats->pq_lut_build_ms = times.lut;
         stats->pq_adc_scan_ms = times.scan; stats->pq_rerank_ms = times.rerank; stats->pq_map_ids_ms = times.map; stats->d2h_ms = t_d2h;
         stats->total_ms = t_total;  // stage times can overlap: their sum may exceed the total
@@ -1817,6 +1909,7 @@ psb_status psb_flat_session_search_device(psb_flat_session* s, const float* d_qu
     if (!d_queries || !d_indices || !d_distances) return fail(PSB_INVALID_ARGUMENT, "null argument");
     if (nq < 0 || nq > s->opt.max_batch) return fail(PSB_INVALID_ARGUMENT, "nq must be in 0..max_batch");
     if (nq == 0) return PSB_OK;
+    s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     return flat_search_device(s, d_queries, nq, params->nprobe, params->topk, reinterpret_cast<long long*>(d_indices), d_distances);
 }
@@ -1837,29 +1930,46 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
     PSB_TRY(s->q.reserve(sizeof(float) * (size_t)batch * s->dim));
     PSB_TRY(s->out_ids.reserve(sizeof(long long) * (size_t)batch * topk));
     PSB_TRY(s->out_dist.reserve(sizeof(float) * (size_t)batch * topk));
+    const size_t b_q = (sizeof(float) * (size_t)total * s->dim + 255) / 256 * 256, b_ids = sizeof(long long) * (size_t)total * topk,
+                 b_dist = sizeof(float) * (size_t)total * topk;
+    const bool small = batch == total && b_q + b_ids + b_dist <= kSmallIo;   // through the pinned block, as psb_session_search
+    PSB_TRY(ensure_host_io(s, small ? b_q + b_ids + b_dist : 0));
     const long long launches0 = launches_total();
-    unsigned long long c0 = 0, c1 = 0;
-    PSB_CUDA(cudaMemcpyAsync(&c0, s->scalars.p, sizeof(c0), cudaMemcpyDeviceToHost, st));
-    EventTimer tm;
-    PSB_TRY(tm.mark(st));
+    unsigned long long c0[4] = {0, 0, 0, 0};
+    if (stats) PSB_TRY(counters_before(s, st, c0));
+    s->counters_known = false;
+    s->timing.used = 0;
+    EventTimer tm(&s->timing);
+    if (stats) PSB_TRY(tm.mark(st));
     int nb = 0;
     for (int q0 = 0; q0 < total; q0 += batch, ++nb) {
         const int n = std::min(batch, total - q0);
-        PSB_CUDA(cudaMemcpyAsync(s->q.p, queries->fp32 + (size_t)q0 * s->dim, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
-        PSB_TRY(flat_search_device(s, s->q.as<float>(), n, nprobe, topk, s->out_ids.as<long long>(), s->out_dist.as<float>()));
-        PSB_CUDA(cudaMemcpyAsync(output->indices + (size_t)q0 * topk, s->out_ids.p, sizeof(long long) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
-        PSB_CUDA(cudaMemcpyAsync(output->distances + (size_t)q0 * topk, s->out_dist.p, sizeof(float) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
+        const void* from = queries->fp32 + (size_t)q0 * s->dim;
+        if (small) { std::memcpy(s->h_io, from, sizeof(float) * (size_t)n * s->dim); from = s->h_io; }
+        PSB_CUDA(cudaMemcpyAsync(s->q.p, from, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
+        long long* ids = small ? reinterpret_cast<long long*>(s->h_io + b_q) : s->out_ids.as<long long>();
+        float* dist = small ? reinterpret_cast<float*>(s->h_io + b_q + b_ids) : s->out_dist.as<float>();
+        PSB_TRY(flat_search_device(s, s->q.as<float>(), n, nprobe, topk, ids, dist));
+        if (!small) {
+            PSB_CUDA(cudaMemcpyAsync(output->indices + (size_t)q0 * topk, ids, sizeof(long long) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
+            PSB_CUDA(cudaMemcpyAsync(output->distances + (size_t)q0 * topk, dist, sizeof(float) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
+        }
         if (output->coarse_ids)
             PSB_CUDA(cudaMemcpyAsync(output->coarse_ids + (size_t)q0 * nprobe, s->probes.p, sizeof(int) * (size_t)n * nprobe, cudaMemcpyDeviceToHost, st));
+        if (q0 + batch >= total) {
+            PSB_TRY(queue_tail(s, st));
+            if (stats) PSB_TRY(tm.mark(st));
+        }
         PSB_CUDA(cudaStreamSynchronize(st));  // the batch buffers are reused
+        if (small) {
+            std::memcpy(output->indices, ids, b_ids);
+            std::memcpy(output->distances, dist, b_dist);
+        }
     }
-    PSB_TRY(tm.mark(st));
-    PSB_CUDA(cudaMemcpyAsync(&c1, s->scalars.p, sizeof(c1), cudaMemcpyDeviceToHost, st));
-    PSB_CUDA(cudaStreamSynchronize(st));
-    PSB_TRY(s->tc_work.check_status());
+    PSB_TRY(check_tail(s));
     if (stats) {
         stats->total_ms = tm.ms(0, 1);
-        stats->pq_scanned_codes = (long long)(c1 - c0);  // rows scanned
+        stats->pq_scanned_codes = (long long)(s->h_tail->c[0] - c0[0]);  // rows scanned
         stats->h2d_bytes = (long long)sizeof(float) * total * s->dim;
         stats->d2h_bytes = (long long)(sizeof(long long) + sizeof(float)) * total * topk;
         stats->kernel_launches = launches_total() - launches0;
