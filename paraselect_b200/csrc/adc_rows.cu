@@ -26,6 +26,7 @@ constexpr int kRowsThreads = 256;
 __device__ __forceinline__ void build_table(float* __restrict__ s_tab, const float* __restrict__ s_q, const float* __restrict__ codebook, int m, int k, int dsub) {
     auto add = [](float e, float q, float c) { const float t = __fsub_rn(q, c); return __fadd_rn(e, __fmul_rn(t, t)); };
     const bool wide = (reinterpret_cast<uintptr_t>(codebook) & 15) == 0;
+#pragma unroll 8
     for (int e = threadIdx.x; e < m * k; e += kRowsThreads) {
         const int sub = k == 256 ? e >> 8 : e / k;
         const float* q = s_q + sub * dsub;
@@ -138,11 +139,11 @@ psb_status run_rows(const AdcRows& g, int nq, cudaStream_t s) {
         const int chunks = (int)std::max<long long>(1, (g.longest_list + block - 1) / block);
         const long long blocks = (long long)nq * g.nprobe * chunks;
         if (blocks > 0x7fffffffLL) return fail(PSB_UNSUPPORTED_SHAPE, "too many (query, probe) pairs in one batch");
-        PSB_CUDA(cudaFuncSetAttribute(k_adc_pair_rows<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_adc_pair_rows<M>), tab));
         k_adc_pair_rows<M><<<(unsigned)blocks, kRowsThreads, tab, s>>>(g, block, chunks);
     } else {
         const size_t smem = tab + ((size_t)g.nprobe + 1) * sizeof(int);
-        PSB_CUDA(cudaFuncSetAttribute(k_adc_rows<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_adc_rows<M>), smem));
         k_adc_rows<M><<<dim3((unsigned)((g.stride + block - 1) / block), (unsigned)nq), kRowsThreads, smem, s>>>(g, block);
     }
     count_launch();
@@ -169,7 +170,7 @@ psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s) {
     const size_t smem = sel::shared_bytes(g.stage1_k);
     // Fewer queries than SMs: one selecting block per SM at most, so a large one.
     auto select = [&](auto kernel, int threads) -> psb_status {
-        PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
         kernel<<<nq, threads, smem, s>>>(g, buffer);
         return PSB_OK;
     };

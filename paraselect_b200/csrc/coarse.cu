@@ -122,7 +122,7 @@ psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float*
     const size_t small = small_tile_bytes(dim);
     if ((long long)grid.x * grid.y < 148 && small <= (size_t)200 * 1024) {
         const dim3 g2((nlist + SC - 1) / SC, (nq + SQ - 1) / SQ);
-        PSB_CUDA(cudaFuncSetAttribute(k_coarse_dist_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_coarse_dist_small), small));
         k_coarse_dist_small<<<g2, kSmallThreads, small, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist);
         count_launch();
         PSB_LAUNCH_CHECK();
@@ -138,7 +138,7 @@ psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_
     if (nq <= 0) return PSB_OK;
     if (k <= 0 || k > kMaxProbe) return fail(PSB_UNSUPPORTED_SHAPE, "row selection supports 1..4096 results");
     const size_t smem = sel::shared_bytes(k);
-    PSB_CUDA(cudaFuncSetAttribute(k_select_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_select_rows), smem));
     k_select_rows<<<nq, kSelThreads, smem, s>>>(d_dist, n, k, sel::buffer_entries(k), d_ids, d_out);
     count_launch();
     PSB_LAUNCH_CHECK();

@@ -875,7 +875,7 @@ psb_status plan_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, int nq,
 template <bool kSecondPass>
 psb_status run_tc(const TcPlan& pl, cudaEvent_t begin, cudaEvent_t end, cudaStream_t s) {
     auto go = [&](auto kernel) -> psb_status {
-        PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), pl.smem));
         if (begin) PSB_CUDA(cudaEventRecord(begin, s));
         kernel<<<pl.grid, kTcThreadsV2, pl.smem, s>>>(pl.map_q, pl.map_c, pl.a);
         if (end) PSB_CUDA(cudaEventRecord(end, s));
@@ -894,7 +894,7 @@ psb_status run_exact_queries(const CoarseTcIndex& ix, const CoarseTcWorkspace& w
     while (buf_n < nprobe + kExactThreads) buf_n <<= 1;
     const size_t esmem = (size_t)buf_n * 8 + (size_t)ix.dim * sizeof(float);
     if (esmem > 32 * 1024)
-        PSB_CUDA(cudaFuncSetAttribute(k_coarse_exact_query, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_coarse_exact_query), esmem));
     k_coarse_exact_query<<<sm_count, kExactThreads, esmem, s>>>(d_queries, ix.centroids, ix.dim, ix.nlist, nprobe, buf_n,
                                                                 ws.fail_list, ws.n_fail, ws.fail_cursor ? ws.fail_cursor : ws.n_fail + 1, d_ids, d_dist);
     count_launch();
@@ -948,7 +948,7 @@ psb_status launch_coarse_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws
     PSB_CUDA(cudaMemsetAsync(ws.cand, 0, sizeof(uint32_t) * (size_t)nq * pl.a.mwords, s));
     PSB_TRY(run_tc<true>(pl, ws.ev[2], ws.ev[3], s));
     const size_t rsmem = (size_t)kCandCap * 8 + (size_t)(kRefineTile + 1) * refine_pitch(ix.dim) * sizeof(float);
-    PSB_CUDA(cudaFuncSetAttribute(k_coarse_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem));
+    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_coarse_refine), rsmem));
     k_coarse_refine<<<nq, kRefineThreads, rsmem, s>>>(d_queries, ix.centroids, ix.dim, ix.nlist, nprobe, pl.a.mask, pl.a.mwords, d_ids, d_dist,
                                                       ws.fail_list, ws.n_fail);
     count_launch();

@@ -91,6 +91,11 @@ __host__ __device__ __forceinline__ uint32_t key_idx(uint64_t k) { return static
 
 constexpr uint64_t KEY_MAX = ~0ull;
 
+// Function attributes are set once per kernel and device: a cudaFuncSetAttribute at every launch cost a small search more than a
+// microsecond per kernel.  kernel_shared: the launch may use `bytes` of dynamic shared memory (remembers the largest).
+psb_status kernel_shared(const void* kernel, size_t bytes);
+psb_status kernel_carveout_max(const void* kernel);
+
 #ifdef __CUDACC__
 // Asks for the maximum shared-memory carve-out for a kernel, whether or not it uses much shared memory.  An SM runs kernels of
 // one carve-out at a time; the scan, coarse and selection kernels need nearly all of it, so every kernel that may run beside
@@ -98,8 +103,7 @@ constexpr uint64_t KEY_MAX = ~0ull;
 // carve-out - otherwise the SMs drain between kernels instead of sharing.
 template <typename F>
 inline psb_status prefer_max_shared(F kernel) {
-    PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    return PSB_OK;
+    return kernel_carveout_max(reinterpret_cast<const void*>(kernel));
 }
 
 // ---- device: block-wide bitonic sort of n (power of two) keys in shared memory, ascending ---------

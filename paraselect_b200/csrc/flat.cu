@@ -231,14 +231,14 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
         count_launch();
         PSB_LAUNCH_CHECK();
         const size_t smem = small_tile_bytes(f.dim);
-        PSB_CUDA(cudaFuncSetAttribute(k_flat_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_tiles), smem));
         const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)220 * 1024 / (smem + 1024)));
         k_flat_tiles<<<(unsigned)(f.sm_count * per_sm), kSmallThreads, smem, s>>>(f.queries, f.dim, f.nprobe, f.offsets, f.nlist, f.rows, f.vis_off,
                                                                                   f.item_off, f.visitors, f.seg, f.stride, f.dist);
     } else {
         const long long blocks = std::min<long long>((f.stride + 127) / 128, 8192);
         const size_t smem = (size_t)((f.dim + 3) & ~3) * sizeof(float);
-        if (smem > 48 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_flat_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_rows), smem));
         k_flat_rows<<<dim3((unsigned)std::max<long long>(1, blocks), (unsigned)nq), 128, smem, s>>>(f.queries, f.dim, f.probes, f.nprobe, f.offsets, f.rows,
                                                                                                     f.seg, f.stride, f.dist);
     }
@@ -246,7 +246,7 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     PSB_LAUNCH_CHECK();
     const size_t smem = sel::shared_bytes(f.topk);
     auto select = [&](auto kernel, int threads) -> psb_status {   // fewer queries than SMs: large blocks
-        PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
         kernel<<<nq, threads, smem, s>>>(f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids,
                                          f.out_dist);
         return PSB_OK;

@@ -1138,7 +1138,7 @@ psb_status run_scan_h(const ScanArgsH& ah, int sm_count, cudaStream_t s) {
     } else {
         const size_t smem = (size_t)ah.a.m * ah.a.k * 16 + (size_t)(kScanThreads / 32) * kQueuePerWarp * 8;
         if (smem > 32 * 1024)
-            PSB_CUDA(cudaFuncSetAttribute(k_scan_h<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_scan_h<M>), smem));
         int occ = 0;
         PSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_scan_h<M>, kScanThreads, smem));
         if (occ < 1) return fail(PSB_UNSUPPORTED_SHAPE, "half scan kernel does not fit an SM");
@@ -1161,7 +1161,7 @@ bool tree_order(const ScanIndex& ix) { return scan_tree_order(ix); }
 
 template <typename F>
 psb_status set_smem(F kernel, size_t bytes) {
-    if (bytes > 32 * 1024) PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (bytes > 32 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), bytes));
     return PSB_OK;
 }
 

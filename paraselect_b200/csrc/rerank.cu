@@ -400,7 +400,7 @@ psb_status launch_gather_unique(const void* src, int row_bytes, const int* d_uni
     if (owned_sms > 0) {
         constexpr int kOwnedSmem = 200 * 1024;   // claimed, not used: keeps every kernel that needs shared memory off the SM
         PSB_TRY(prefer_max_shared(k_gather_unique_owned));
-        PSB_CUDA(cudaFuncSetAttribute(k_gather_unique_owned, cudaFuncAttributeMaxDynamicSharedMemorySize, kOwnedSmem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_gather_unique_owned), kOwnedSmem));
         k_gather_unique_owned<<<owned_sms, 1024, kOwnedSmem, s>>>(from, row_bytes, d_unique, d_begin, d_end, host_pct, to);
     } else if (compact_ctas > 0) {
         PSB_TRY(prefer_max_shared(k_gather_unique_beside));
@@ -424,7 +424,7 @@ psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const Ro
     const int through = smem <= (size_t)200 * 1024 ? 1 : 0;
     if (!through) smem = pitch;
     if (smem > (size_t)220 * 1024) return fail(PSB_UNSUPPORTED_SHAPE, "rows too long for the exact rerank");
-    if (smem > 48 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_rerank_score, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_rerank_score), smem));
     PSB_TRY(prefer_max_shared(k_rerank_score));
     k_rerank_score<<<grid, kScoreThreads, smem, s>>>(
         static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, elem_bytes, through, static_cast<const unsigned char*>(d_queries),
@@ -444,7 +444,7 @@ psb_status launch_topk_select(const float* d_dist, const int* d_candidates, int 
     const int buffer = sel::buffer_entries(topk);
     const size_t smem = (size_t)std::max(np, buffer) * 8 + (size_t)std::max(np, sel::kMaxGroups) * 4;
     if (smem > 32 * 1024)
-        PSB_CUDA(cudaFuncSetAttribute(k_topk_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_topk_select), smem));
     PSB_TRY(prefer_max_shared(k_topk_select));
     k_topk_select<<<nq, kSelectThreads, smem, s>>>(d_dist, d_candidates, candidate_count, candidate_stride, d_counts,
                                                    topk, np, buffer, d_out_rows, d_out_dist, d_ids, d_out_ids);
@@ -487,7 +487,7 @@ psb_status launch_merge(const int* d_rows, const float* d_dist, int parts, int n
     int np = 2;
     while (np < total) np <<= 1;
     const size_t smem = (size_t)np * 8;
-    if (smem > 32 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 32 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_merge), smem));
     k_merge<<<nq, 1024, smem, s>>>(d_rows, d_dist, parts, nq, k, np, d_out_rows, d_out_dist);
     count_launch();
     PSB_LAUNCH_CHECK();

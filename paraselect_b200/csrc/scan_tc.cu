@@ -738,7 +738,7 @@ psb_status launch_row_aug(const uint8_t* d_codes, long long rows, int dim, int m
     const unsigned grid = (unsigned)std::min<long long>((rows + 255) / 256, 148 * 16);
 #define PSB_AUG(D)                                                                                                      \
     do {                                                                                                                \
-        if (smem > 32 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_row_aug<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        if (smem > 32 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_row_aug<D>), smem)); \
         k_row_aug<D><<<grid, 256, smem, s>>>(d_codes, rows, m, k, d_codebook, cw2, static_cast<uint2*>(d_out));          \
     } while (0)
     if (dsub == 2) PSB_AUG(2);
@@ -754,7 +754,7 @@ psb_status launch_row_aug(const uint8_t* d_codes, long long rows, int dim, int m
 namespace {
 template <int DSUB, int M>
 psb_status run_scan_tc(const ScanTcArgs& g, unsigned grid, size_t smem, cudaStream_t s) {
-    PSB_CUDA(cudaFuncSetAttribute(k_scan_tc<DSUB, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_scan_tc<DSUB, M>), smem));
     k_scan_tc<DSUB, M><<<grid, kTcScanThreads, smem, s>>>(g);
     count_launch();
     PSB_LAUNCH_CHECK();
@@ -809,7 +809,7 @@ template <int M>
 psb_status run_select_rescore(const RescoreArgs& g, int nq, cudaStream_t s) {
     const size_t smem = (size_t)g.pool_cap * 8 + (g.residual ? (size_t)g.dim * 4 : (size_t)g.m * g.k * 4);
     if (smem > (size_t)226 * 1024) return fail(PSB_UNSUPPORTED_SHAPE, "re-scoring selection does not fit shared memory");
-    if (smem > 32 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_select_rescore<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 32 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_select_rescore<M>), smem));
     PSB_TRY(prefer_max_shared(k_select_rescore<M>));
     k_select_rescore<M><<<nq, kRescoreThreads, smem, s>>>(g);
     count_launch();

@@ -69,7 +69,7 @@ __device__ int smallest(const float* __restrict__ vals, int n, int k, Payload pa
     __syncthreads();
     const float cut = w->cut;
     if (cut < inf || n <= buffer) {
-#pragma unroll 4
+#pragma unroll 8
         for (int i = tid; i < n; i += kThreads) {
             const float v = vals[i];
             if (cut == inf || v <= cut) {

@@ -45,6 +45,44 @@ void count_launch(long long n) { g_launches.fetch_add(n, std::memory_order_relax
 long long launches_total() { return g_launches.load(std::memory_order_relaxed); }
 
 namespace {
+// One word per (kernel, device): bit 31 the carve-out is set, the rest the shared memory allowed so far.  Open addressing; a full table
+// (never: the library has fewer kernels) just sets the attribute every time.
+struct KernelAttr { std::atomic<uintptr_t> key{0}; std::atomic<unsigned> word{0}; };
+KernelAttr g_attr[2048];
+KernelAttr* kernel_attr(const void* kernel) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    const uintptr_t key = (reinterpret_cast<uintptr_t>(kernel) << 6) ^ (uintptr_t)(dev & 63) ^ ((uintptr_t)1 << 63);
+    size_t h = (key * 0x9E3779B97F4A7C15ull) >> 53;
+    for (int i = 0; i < 64; ++i, h = (h + 1) & 2047) {
+        uintptr_t seen = g_attr[h].key.load(std::memory_order_acquire);
+        if (seen == 0 && g_attr[h].key.compare_exchange_strong(seen, key, std::memory_order_acq_rel)) return &g_attr[h];
+        if (seen == key) return &g_attr[h];
+    }
+    return nullptr;
+}
+}  // namespace
+psb_status kernel_shared(const void* kernel, size_t bytes) {
+    KernelAttr* a = kernel_attr(kernel);
+    const unsigned need = (unsigned)bytes;
+    if (a && need <= (a->word.load(std::memory_order_acquire) & 0x7fffffffu)) return PSB_OK;
+    static std::mutex mu;   // the attribute only ever grows, whichever threads ask for how much
+    std::lock_guard<std::mutex> lk(mu);
+    const unsigned have = a ? a->word.load(std::memory_order_relaxed) & 0x7fffffffu : 0;
+    if (a && need <= have) return PSB_OK;
+    PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+    if (a) a->word.fetch_add(need - have, std::memory_order_release);
+    return PSB_OK;
+}
+psb_status kernel_carveout_max(const void* kernel) {
+    KernelAttr* a = kernel_attr(kernel);
+    if (a && (a->word.load(std::memory_order_relaxed) & 0x80000000u)) return PSB_OK;
+    PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (a) a->word.fetch_or(0x80000000u);
+    return PSB_OK;
+}
+
+namespace {
 
 // Device buffer that grows on demand (contents are not preserved).
 struct DevBuf {
@@ -1380,17 +1418,32 @@ psb_status psb_session_counters(psb_session* s, psb_stats* stats, int reset) {
 
 namespace {
 
-// Stage times of one search call: marks are left by search_device and read once the stream has drained.
+// Stage times of one search call: spans between events, read once the stream has drained.  A recorded time costs the GPU about five
+// microseconds between two kernels, so stages that follow one another on a stream share the event between them.
 struct StageTimes {
-    double coarse = 0, lut = 0, scan = 0, rerank = 0, map = 0;
+    enum Stage { kCoarse, kLut, kScan, kRerank, kMap, kStages };
+    double ms[kStages] = {0, 0, 0, 0, 0};
     EventTimer tm_s, tm_x;
+    struct Span { Stage stage; cudaEvent_t a, b; };
+    std::vector<Span> spans, spans_x;   // of the main thread, of the thread that drives the second stream
+    cudaEvent_t last = nullptr;         // the main stream's latest mark; null once something else may have been queued behind it
     explicit StageTimes(psb_session* s) : tm_s(&s->timing), tm_x(&s->timing_aux) {}
+    psb_status mark(cudaStream_t st) { PSB_TRY(tm_s.mark(st)); last = tm_s.ev.back(); return PSB_OK; }
+    psb_status begin(cudaStream_t st) { return last ? PSB_OK : mark(st); }
+    psb_status end(Stage stage, cudaStream_t st) {   // of a stage that began at `last`
+        const cudaEvent_t from = last;
+        PSB_TRY(mark(st));
+        spans.push_back({stage, from, last});
+        return PSB_OK;
+    }
+    psb_status mark_x(cudaStream_t st, cudaEvent_t* e) { PSB_TRY(tm_x.mark(st)); *e = tm_x.ev.back(); return PSB_OK; }
     void collect() {
-        if (tm_s.ev.size() >= 2) coarse += tm_s.ms(0, 1);
-        for (size_t i = 2; i + 2 < tm_s.ev.size(); i += 3) { lut += tm_s.ms(i, i + 1); scan += tm_s.ms(i + 1, i + 2); }
-        for (size_t i = 0; i + 2 < tm_x.ev.size(); i += 3) { rerank += tm_x.ms(i, i + 1); map += tm_x.ms(i + 1, i + 2); }
+        for (const auto* v : {&spans, &spans_x})
+            for (const Span& sp : *v) { float t = 0.f; cudaEventElapsedTime(&t, sp.a, sp.b); ms[sp.stage] += t; }
+        spans.clear(); spans_x.clear();
         tm_s.ev.clear(); tm_x.ev.clear();
         tm_s.pool->used = 0; tm_x.pool->used = 0;
+        last = nullptr;
     }
 };
 
@@ -1525,18 +1578,20 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
             auto process = [&](const Job& j) -> psb_status {
                 PSB_RANGE("pq_rerank");
                 PSB_CUDA(cudaEventSynchronize(j.ready));
-                if (times) PSB_TRY(times->tm_x.mark(sx));
+                cudaEvent_t t0 = nullptr, t1 = nullptr;
+                if (times) PSB_TRY(times->mark_x(sx, &t0));
                 // Hybrid transport: the kernel's share of the slots comes through the gather kernel, which the main thread queued right
                 // behind this sub-batch's claim (j.gathered marks its end); the host threads and the copy engine bring the others; the
                 // scoring waits for both.
                 PSB_TRY(rows_from_host(s, j.part, host_pct, sx));
                 if (j.gathered) PSB_CUDA(cudaStreamWaitEvent(sx, j.gathered, 0));
                 PSB_TRY(score_part(j.p0, j.m));
-                if (times) PSB_TRY(times->tm_x.mark(sx));
-                if (s->striped)
+                if (times) { PSB_TRY(times->mark_x(sx, &t1)); times->spans_x.push_back({StageTimes::kRerank, t0, t1}); }
+                if (s->striped) {
                     PSB_TRY(launch_map_ids(s->out_rows.as<int>() + (size_t)j.p0 * topk, (long long)j.m * topk, s->reordered.as<long long>(), s->row_map(),
                                            d_ids + (size_t)j.p0 * topk, sx));
-                if (times) PSB_TRY(times->tm_x.mark(sx));
+                    if (times) { PSB_TRY(times->mark_x(sx, &t0)); times->spans_x.push_back({StageTimes::kMap, t1, t0}); }
+                }
                 return PSB_OK;
             };
             for (;;) {
@@ -1562,7 +1617,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     };
     // Coarse stage for the whole batch first: one large GEMM is more efficient than four small ones, and the tensor-core
     // kernel (a full SM's shared and tensor memory per CTA) then never has to share SMs with the transfer stream.
-    if (times) rc = times->tm_s.mark(st);
+    if (times) rc = times->begin(st);
     if (rc == PSB_OK) { PSB_RANGE("coarse_search"); rc = coarse_exact(s, dq, n, nprobe, d_probes, nullptr); }
     // OPQ index: the PQ side works on the rotated queries (counted with the coarse stage's time)
     const float* dq_pq = dq;
@@ -1571,7 +1626,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         if (rc == PSB_OK) rc = launch_rotate_rows(dq, s->opq.as<float>(), n, s->dim, s->q_rot.as<float>(), st);
         dq_pq = s->q_rot.as<float>();
     }
-    if (rc == PSB_OK && times) rc = times->tm_s.mark(st);
+    if (rc == PSB_OK && times) rc = times->end(StageTimes::kCoarse, st);
     for (size_t ci = 0; ci + 1 < cuts.size() && rc == PSB_OK; ++ci) {
         const int p0 = cuts[ci];
         const int m = cuts[ci + 1] - p0;
@@ -1580,7 +1635,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         int* rows_out = rerank ? s->cand_rows.as<int>() + (size_t)p0 * stage1_k : s->out_rows.as<int>() + (size_t)p0 * topk;
         float* dist_out = rerank ? s->cand_dist.as<float>() + (size_t)p0 * stage1_k : d_dist + (size_t)p0 * topk;
         int* cnt_out = s->cand_count.as<int>() + p0;
-        if (times) rc = times->tm_s.mark(st);
+        if (times) rc = times->begin(st);
         ScanWorkspace sws;
         if (rc == PSB_OK) rc = s->timed_scan_ws(&sws);
         if (rc == PSB_OK && !table_free) {
@@ -1597,12 +1652,12 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
                 rc = launch_build_lut(q, m, s->dim, s->codebook.as<float>(), s->m, s->k, s->lut.as<float>(), st);
             }
         }
-        if (rc == PSB_OK && times) rc = times->tm_s.mark(st);
+        if (rc == PSB_OK && times && !table_free) rc = times->end(StageTimes::kLut, st);
         if (rc == PSB_OK) {
             PSB_RANGE("pq_adc_scan");
             rc = run_scan(s, sws, q, table_free ? nullptr : s->lut.as<float>(), m, probes, nprobe, stage1_k, rows_out, dist_out, cnt_out, st);
         }
-        if (rc == PSB_OK && times) rc = times->tm_s.mark(st);
+        if (rc == PSB_OK && times) rc = times->end(StageTimes::kScan, st);
         if (rc != PSB_OK) break;
         if (staged_overlap) {  // claim the sub-batch's rows and hand it to the worker: an event marks the slot range ready
             cudaEvent_t e, gathered = nullptr;
@@ -1636,7 +1691,8 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         // second half of the sub-batch (on the second stream when overlapping)
         cudaStream_t keep = s->stream;
         s->stream = sx;  // rerank_impl and the launchers below run on s->stream
-        if (times) rc = times->tm_x.mark(sx);
+        cudaEvent_t t0 = nullptr, t1 = nullptr;   // second stream
+        if (times && overlap) rc = times->mark_x(sx, &t0);
         bool mapped_ids = false;
         if (rc == PSB_OK && rerank) {
             PSB_RANGE("pq_rerank");
@@ -1653,18 +1709,21 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
                                  d_dist + (size_t)p0 * topk, nullptr, mapped_ids ? d_ids + (size_t)p0 * topk : nullptr);
             }
         }
-        if (rc == PSB_OK && times) rc = times->tm_x.mark(sx);
+        if (rc == PSB_OK && times && rerank && !overlap) rc = times->end(StageTimes::kRerank, st);
+        if (rc == PSB_OK && times && overlap) { rc = times->mark_x(sx, &t1); times->spans_x.push_back({StageTimes::kRerank, t0, t1}); }
         if (rc == PSB_OK && !mapped_ids) {
             PSB_RANGE("pq_map_ids");
             rc = launch_map_ids(s->out_rows.as<int>() + (size_t)p0 * topk, (long long)m * topk, s->reordered.as<long long>(),
                                 s->row_map(), d_ids + (size_t)p0 * topk, sx);
         }
-        if (rc == PSB_OK && times) rc = times->tm_x.mark(sx);
+        if (rc == PSB_OK && times && !overlap && !mapped_ids) rc = times->end(StageTimes::kMap, st);
+        if (rc == PSB_OK && times && overlap && !mapped_ids) { rc = times->mark_x(sx, &t0); times->spans_x.push_back({StageTimes::kMap, t1, t0}); }
         s->stream = keep;
     }
     finish_worker();
     if (worker_rc != PSB_OK && rc == PSB_OK) rc = fail(worker_rc, "rerank worker: " + worker_msg);
     if (shared_rows && rc == PSB_OK) rc = rows_end(s, sx);
+    if (times && (overlap || staged_overlap)) times->last = nullptr;
     if (overlap || staged_overlap) {  // the main stream continues only after the second stream has finished this batch
         cudaEvent_t e;
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) {
@@ -1738,8 +1797,8 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
     int nb = 0;
     for (int q0 = 0; q0 < total; q0 += batch, ++nb) {
         const int n = std::min(batch, total - q0);
-        EventTimer tm(&s->timing);
-        if (stats) PSB_TRY(tm.mark(st));
+        cudaEvent_t t_begin = nullptr, t_in = nullptr, t_done = nullptr;
+        if (stats) { PSB_TRY(times.mark(st)); t_begin = times.last; }
         const void* from = queries->fp32 + (size_t)q0 * s->dim;
         const void* from_u8 = u8 ? queries->u8 + (size_t)q0 * s->dim : nullptr;
         if (small) {
@@ -1753,12 +1812,12 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
             PSB_CUDA(cudaMemcpyAsync(s->q_u8.p, from_u8, (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
             h2d += (long long)n * s->dim;
         }
-        if (stats) PSB_TRY(tm.mark(st));
+        if (stats) { PSB_TRY(times.mark(st)); t_in = times.last; }
         const void* qe = s->exact_elem == 1 ? s->q_u8.p : s->q.p;
         long long* ids = small ? reinterpret_cast<long long*>(s->h_io + b_q + b_u8) : s->out_ids.as<long long>();
         float* dist = small ? reinterpret_cast<float*>(s->h_io + b_q + b_u8 + b_ids) : s->out_dist.as<float>();
         PSB_TRY(search_device(s, s->q.as<float>(), qe, n, nprobe, topk, stage1_k, rerank, ids, dist, s->probes.as<int>(), stats ? &times : nullptr));
-        if (stats) PSB_TRY(tm.mark(st));
+        if (stats) { PSB_TRY(times.begin(st)); t_done = times.last; }
         if (!small) {
             PSB_CUDA(cudaMemcpyAsync(output->indices + (size_t)q0 * topk, ids, sizeof(long long) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
             PSB_CUDA(cudaMemcpyAsync(output->distances + (size_t)q0 * topk, dist, sizeof(float) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
@@ -1769,19 +1828,24 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
             d2h += (long long)sizeof(int) * n * nprobe;
         }
         if (q0 + batch >= total) PSB_TRY(queue_tail(s, st));
-        if (stats) PSB_TRY(tm.mark(st));
+        if (stats) PSB_TRY(times.mark(st));
         PSB_CUDA(cudaStreamSynchronize(st));
         if (small) {
             std::memcpy(output->indices, ids, b_ids);
             std::memcpy(output->distances, dist, b_dist);
         }
-        if (stats) { t_h2d += tm.ms(0, 1); t_d2h += tm.ms(2, 3); t_total += tm.ms(0, 3); times.collect(); }
+        if (stats) {
+            auto span = [](cudaEvent_t a, cudaEvent_t b) { float t = 0.f; cudaEventElapsedTime(&t, a, b); return (double)t; };
+            t_h2d += span(t_begin, t_in); t_d2h += span(t_done, times.last); t_total += span(t_begin, times.last);
+            times.collect();
+        }
     }
     PSB_TRY(check_tail(s));
     if (stats) {
         const unsigned long long* c1 = s->h_tail->c;
-        stats->h2d_ms = t_h2d; stats->coarse_search_ms = times.coarse; stats->pq_lut_build_ms = times.lut;
-        stats->pq_adc_scan_ms = times.scan; stats->pq_rerank_ms = times.rerank; stats->pq_map_ids_ms = times.map; stats->d2h_ms = t_d2h;
+        stats->h2d_ms = t_h2d; stats->coarse_search_ms = times.ms[StageTimes::kCoarse]; stats->pq_lut_build_ms = times.ms[StageTimes::kLut];
+        stats->pq_adc_scan_ms = times.ms[StageTimes::kScan]; stats->pq_rerank_ms = times.ms[StageTimes::kRerank];
+        stats->pq_map_ids_ms = times.ms[StageTimes::kMap]; stats->d2h_ms = t_d2h;
         stats->total_ms = t_total;  // stage times can overlap: their sum may exceed the total
         stats->pq_scanned_codes = (long long)(c1[0] - c0[0]);
         stats->pq_adc_lookups = stats->pq_scanned_codes * s->m;

@@ -779,7 +779,7 @@ psb_status dispatch_encode(const SignEncodeArgs& args, int padded, int sm_count,
 template <int W, int MODE>
 psb_status run_scan(const SignScanArgs& a, size_t smem, cudaStream_t s) {
     PSB_TRY(prefer_max_shared(k_sign_scan<W, MODE>));
-    PSB_CUDA(cudaFuncSetAttribute(k_sign_scan<W, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_sign_scan<W, MODE>), smem));
     k_sign_scan<W, MODE><<<(unsigned)(a.nq * a.split), kScanThreads, smem, s>>>(a);
     PSB_LAUNCH_CHECK();
     count_launch();

@@ -749,7 +749,7 @@ psb_status run_pq_nearest(const float* d_data, long long n, int dim, const float
     const int ranges = (int)std::max<long long>(1, std::min<long long>(m, (2 * 148 + blocks - 1) / blocks));
     const int per = (m + ranges - 1) / ranges;
     const size_t smem = near_smem<D>(per);
-    PSB_CUDA(cudaFuncSetAttribute(k_pq_nearest<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_nearest<D>), smem));
     k_pq_nearest<D><<<dim3((unsigned)blocks, (unsigned)((m + per - 1) / per)), kNearWarps * 32, smem, s>>>(d_data, n, dim, d_codebook, m, k, per, d_codes);
     count_launch();
     PSB_LAUNCH_CHECK();
@@ -780,11 +780,11 @@ psb_status launch_pq_encode(const float* d_data, long long n, int dim, const flo
     const unsigned grid = (unsigned)((n + kEncThreads - 1) / kEncThreads);
     const size_t tile = (size_t)kEncThreads * (dim + 1) * sizeof(float) + (size_t)k * dsub * sizeof(float) + (size_t)kEncThreads * m;
     if (tile <= 200 * 1024) {  // rows staged in shared memory
-        PSB_CUDA(cudaFuncSetAttribute(k_pq_encode_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_encode_tile), tile));
         k_pq_encode_tile<<<grid, kEncThreads, tile, s>>>(d_data, n, dim, d_codebook, m, k, d_codes);
     } else {
         const size_t smem = (size_t)k * dsub * sizeof(float) + (size_t)kEncThreads * m;
-        if (smem > 32 * 1024) PSB_CUDA(cudaFuncSetAttribute(k_pq_encode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 32 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_encode), smem));
         k_pq_encode<<<grid, kEncThreads, smem, s>>>(d_data, n, dim, d_codebook, m, k, d_codes);
     }
     count_launch();
@@ -819,7 +819,7 @@ psb_status launch_pq_seed(const float* d_data, int n, int dim, int m, int k, con
     const int staged = mins + rows <= (size_t)200 * 1024 ? 1 : 0;
     const size_t smem = mins + (staged ? rows : 0);
     auto run = [&](auto kernel) -> psb_status {
-        PSB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
         kernel<<<dim3(kSeedCluster, (unsigned)m), kSeedCtaThreads, smem, s>>>(d_data, n, dim, dsub, k, per, staged, d_draws, d_first, d_rows, d_status);
         return PSB_OK;
     };
