@@ -55,7 +55,7 @@ constexpr int kWarpSched = kWarpMma + 1;            // warp 17: fetches work ite
 constexpr int kTcScanThreads = (kWarpSched + 1) * 32;
 constexpr int kProducers = kDecodeWarps * 32;
 constexpr int kItemRing = 4;       // work items in flight
-constexpr int kQueueCap = 256;     // survivors a warp collects before it pushes them to the pools
+constexpr int kQueueCap = 16;      // survivors a thread (its visitor) collects before its warp pushes them to the pools
 constexpr int kAugSlots = 4;
 constexpr float kBeta = 0.001953125f * 1.001f;  // 2^-9 (1 + 1e-3)
 
@@ -183,8 +183,10 @@ __device__ __forceinline__ void decode_row(const RowCodes<M>& codes, const uint8
 //   warps 0-7   producers: build the item's query tile (A operand, ring of `na` slots) and its per-visitor constants, then
 //               decode code rows into the ring of `ns` row tiles (B operand), one tile in flight per warp group
 //   warp 16     MMA issuer: kp / 16 tcgen05.mma per tile into accumulator `stage`, tcgen05.commit -> mbarriers
-//   warps 8-15  epilogue: tcgen05.ld the accumulator (two 32-column loads in flight), one comparison per (visitor, row); survivors go to a per-warp queue in
-//               shared memory that is pushed to the visitors' pools 32 at a time (one round of global atomics per push)
+//   warps 8-15  epilogue: tcgen05.ld the accumulator (two 32-column loads in flight), one comparison per (visitor, row); a visitor's survivors
+//               collect in its thread's own 16 places in shared memory, and when one of them fills up the warp pushes all to the pools:
+//               one global atomic per visitor and push, all in flight together.  (A queue per warp, with an atomic per survivor to
+//               enter it and another to leave it, took most of the kernel where one row in sixty survives: 990 us for 62M pairs.)
 template <int DSUB, int M>
 __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs g) {
     const ScanArgs& a = g.a;
@@ -200,8 +202,7 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
     __shared__ ItemDesc s_desc[kItemRing];
     __shared__ float s_P[kItemRing][TV];
     __shared__ int s_pq[kItemRing][TV], s_hi[kItemRing][TV];
-    __shared__ uint32_t s_queue[kEpiWarps][kQueueCap];
-    __shared__ int s_qcnt[kEpiWarps];
+    __shared__ uint16_t s_queue[kEpiWarps][kQueueCap][32];   // rows of the item (a chunk has at most 16,384)
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -225,7 +226,6 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (tid < kEpiWarps) s_qcnt[tid] = 0;
     // the codebook rounded to bf16, once per CTA (all threads)
     for (int e = tid; e < a.m * a.k; e += kTcScanThreads) {
         const float* cb = g.codebook + (size_t)e * DSUB;
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
         const int e = warp - kDecodeWarps, quad = warp & 3, eg = e >> 2;  // warp % 4 == quad: the tensor-memory lanes this warp may read
         const int i = quad * 32 + lane;
         const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
-        uint32_t* queue = s_queue[e];
+        uint16_t (*queue)[32] = s_queue[e];
         uint32_t it0 = 0;
         for (uint32_t n = 0;; ++n) {
             const int islot = n % kItemRing;
@@ -398,23 +398,22 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
             if (!__all_sync(0xffffffffu, wait_or_abort(&vis_full[islot], (n / kItemRing) & 1u, abort_flag, limit))) { failed = true; break; }
             const float P = s_P[islot][i];
             const uint32_t nrows = (uint32_t)(d.r1 - d.r0);  // rows of the item
+            const int pq = s_pq[islot][i];
+            const uint64_t hi = (uint64_t)(uint32_t)s_hi[islot][i] << 32;
+            int held = 0;   // survivors in this thread's queue
             // pushes the queued survivors of this item to their visitors' pools
             auto flush = [&]() {
-                const int cnt = min(s_qcnt[e], kQueueCap);
-                for (int x = lane; x < cnt; x += 32) {
-                    const uint32_t en = queue[x];
-                    const int vi = (int)(en >> 24);
-                    const int pq = s_pq[islot][vi];
-                    const int slot = atomicAdd(&a.pool_cnt[pq], 1);
-                    if (slot < a.pool_cap)
-                        a.pool[(size_t)pq * a.pool_cap + slot] = ((uint64_t)(uint32_t)s_hi[islot][vi] << 32) | (uint32_t)(d.r0 + (en & 0xFFFFFFu));
+                if (held) {
+                    const int slot = atomicAdd(&a.pool_cnt[pq], held);
+                    uint64_t* out = a.pool + (size_t)pq * a.pool_cap + slot;
+                    for (int x = 0; x < held; ++x)
+                        if (slot + x < a.pool_cap) out[x] = hi | (uint32_t)(d.r0 + queue[x][lane]);
+                    passes += held;
+                    held = 0;
                 }
-                __syncwarp();
-                if (lane == 0) s_qcnt[e] = 0;
-                __syncwarp();
             };
             // 32 accumulator columns (rows rel .. rel + 31 of the item) against this thread's visitor: the maximum by three-input
-            // max, and only when it reaches the visitor's bound the hit mask and one queue entry per hit (no branch per column)
+            // max, and only when it reaches the visitor's bound in some thread the hit masks
             auto scan32 = [&](const uint32_t (&v)[32], uint32_t rel) {
                 float m0 = __uint_as_float(v[0]), m1 = __uint_as_float(v[1]);
 #pragma unroll
@@ -422,28 +421,22 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
                     asm("max.f32 %0, %0, %1, %2;" : "+f"(m0) : "f"(__uint_as_float(v[j])), "f"(__uint_as_float(v[j + 1])));
                     if (j + 3 < 32) asm("max.f32 %0, %0, %1, %2;" : "+f"(m1) : "f"(__uint_as_float(v[j + 2])), "f"(__uint_as_float(v[j + 3])));
                 }
-                if (fmaxf(m0, m1) >= P) {
-                    uint32_t mask = 0;
+                const bool any = fmaxf(m0, m1) >= P;
+                if (!__any_sync(0xffffffffu, any)) return;
+                uint32_t mask = 0;
+                if (any) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) mask |= (__uint_as_float(v[j]) >= P ? 1u : 0u) << j;
                     if (rel + 32 > nrows) mask &= rel < nrows ? (0xffffffffu >> (rel + 32 - nrows)) : 0u;  // padding rows of the last tile
-                    while (mask) {
-                        const uint32_t j = (uint32_t)__ffs((int)mask) - 1u;
-                        mask &= mask - 1u;
-                        ++passes;
-                        const int pos = atomicAdd(&s_qcnt[e], 1);
-                        if (pos < kQueueCap) {
-                            queue[pos] = ((uint32_t)i << 24) | (rel + j);
-                        } else {  // queue full (a visitor without cutoff admits whole lists): straight to the pool
-                            const int pq = s_pq[islot][i];
-                            const int slot = atomicAdd(&a.pool_cnt[pq], 1);
-                            if (slot < a.pool_cap)
-                                a.pool[(size_t)pq * a.pool_cap + slot] = ((uint64_t)(uint32_t)s_hi[islot][i] << 32) | (uint32_t)(d.r0 + rel + j);
-                        }
-                    }
                 }
-                __syncwarp();  // reconverged: the tcgen05 loads and waits that follow are warp-aligned
-                if (s_qcnt[e] >= kQueueCap / 2) flush();  // warp-uniform
+                while (__any_sync(0xffffffffu, mask != 0)) {
+                    if (__any_sync(0xffffffffu, held + __popc(mask) > kQueueCap)) flush();   // (a visitor without cutoff takes whole lists: 16 at a time)
+                    while (mask && held < kQueueCap) {
+                        queue[held++][lane] = (uint16_t)(rel + (uint32_t)__ffs((int)mask) - 1u);
+                        mask &= mask - 1u;
+                    }
+                    __syncwarp();
+                }
             };
             for (int k = 0; k < d.ntiles; ++k) {
                 const uint32_t gi = it0 + (uint32_t)k;
