@@ -221,6 +221,7 @@ struct SelectRescoreLaunch {
     int m, k; bool residual, tree;
     int* out_rows; float* out_dist; int* out_count; int* fail_list; int* n_fail; unsigned long long* counters;
     bool shared_cut = false;
+    int sm_count = 148;
 };
 psb_status launch_select_rescore(const SelectRescoreLaunch& L, int nq, cudaStream_t s);
 

@@ -1449,7 +1449,7 @@ psb_status launch_scan(const ScanIndex& ix, const ScanWorkspace& ws, const float
         R.nprobe = nprobe; R.dim = ix.dim; R.nlist = ix.nlist; R.codes = ix.codes; R.row_base = ix.row_base; R.row_delta = ix.row_delta;
         R.m = ix.m; R.k = ix.k; R.residual = ix.residual; R.tree = tree_order(ix);
         R.out_rows = d_rows; R.out_dist = d_dist; R.out_count = d_count; R.fail_list = ws.fail_list; R.n_fail = ws.n_fail;
-        R.counters = ws.counters; R.shared_cut = ws.phase == 2;
+        R.counters = ws.counters; R.shared_cut = ws.phase == 2; R.sm_count = sm_count;
         PSB_TRY(launch_select_rescore(R, nq, s));
     } else {
         const size_t smem = (size_t)ws.pool_cap * sizeof(uint64_t);

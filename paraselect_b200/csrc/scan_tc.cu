@@ -1,4 +1,4 @@
-// ADC scan, tensor-core pre-filter (sm_100a tcgen05) and the re-scoring selection that follows it.
+// ADC scan, tensor-core pre-filter (sm_100a tcgen05); the re-scoring selection that follows it is in rescore.cu.
 //
 // The ADC distance of a code row against a query is |q - recon(row)|^2, recon(row) = the row's codewords laid side by
 // side.  For a list visited by many queries that is a GEMM: a tile of 128 visiting queries (A operand, centred on the
@@ -554,103 +554,6 @@ __global__ void k_row_aug(const uint8_t* __restrict__ codes, long long rows, int
     }
 }
 
-// ------------------------------------------------------------------------------------------------------
-// Selection with re-scoring.  A pool entry is either an exact key (distance bits with the top bit set: written by the SIMT
-// scans) or an unscored survivor of the tensor-core filter: (list id, or in residual mode the (query, probe) pair) << 32 |
-// scanned row.  Unscored entries get their exact fp32 ADC distance here - plain mode from the query's fp32 table staged in
-// shared memory, residual mode from the pair's residual and the codebook, both in the CPU path's summation order - and are
-// dropped when it exceeds the cutoff.  Then the pool is sorted by (distance, row) and the first stage1_k rows go out.  A pool
-// that overflowed, or holds fewer than min(stage1_k, rows scanned) entries within the cutoff, sends the query to the exact
-// fallback.
-constexpr int kRescoreThreads = 1024;
-
-struct RescoreArgs {
-    const uint64_t* pool; const int* pool_cnt; int pool_cap;
-    const long long* q_rows; const float* thr; int stage1_k;
-    const float* lut;          // plain mode: [nq][m * k]
-    const float* queries; const float* centroids; const float* codebook; const int* probes; int nprobe, dim, nlist;  // residual mode
-    const uint8_t* codes; long long row_base; const long long* row_delta;
-    int m, k, residual, tree;
-    int* out_rows; float* out_dist; int* out_count;
-    int* fail_list; int* n_fail; unsigned long long* counters;
-    int shared_cut;   // the cutoff covers the rows of all shards: this shard need not reach stage1_k rows
-};
-
-template <int M>
-__global__ void __launch_bounds__(kRescoreThreads) k_select_rescore(const RescoreArgs g) {
-    extern __shared__ __align__(16) unsigned char s_sel[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_sel);                      // [pool_cap]
-    float* s_tab = reinterpret_cast<float*>(s_sel + (size_t)g.pool_cap * 8);   // plain: the table [m * k]; residual: the query [dim]
-    __shared__ int s_valid;
-    const int q = blockIdx.x;
-    const int c = g.pool_cnt[q];
-    const long long N = g.q_rows[q];
-    long long need = N < g.stage1_k ? N : g.stage1_k;
-    if (g.shared_cut && g.thr[q] < __int_as_float(0x7f800000)) need = 0;   // sharded search: the shards owe stage1_k rows together
-    if (c > g.pool_cap || c < need) {
-        if (threadIdx.x == 0) g.fail_list[atomicAdd(g.n_fail, 1)] = q;
-        return;  // the fallback writes this query's outputs
-    }
-    const int mk = g.m * g.k;
-    const int dsub = g.dim / g.m;
-    if (!g.residual) {
-        for (int e = threadIdx.x; e < mk; e += blockDim.x) s_tab[e] = g.lut[(size_t)q * mk + e];
-    } else {
-        for (int d = threadIdx.x; d < g.dim; d += blockDim.x) s_tab[d] = g.queries[(size_t)q * g.dim + d];
-    }
-    if (threadIdx.x == 0) s_valid = 0;
-    __syncthreads();
-    const float cut = g.thr[q];
-    const int n = next_pow2(max(c, 2));
-    int valid = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        uint64_t key = KEY_MAX;
-        if (i < c) {
-            const uint64_t e = g.pool[(size_t)q * g.pool_cap + i];
-            if (e >> 63) {
-                key = e;  // exact already, and within the cutoff
-                ++valid;
-            } else {
-                const long long r = (long long)(uint32_t)e;
-                const int hi = (int)(e >> 32);
-                const uint8_t* row = g.codes + (size_t)(r - g.row_base) * g.m;
-                float d;
-                int l;
-                if (!g.residual) {
-                    l = hi;
-                    d = adc_row<M>(row, s_tab, g.m, g.k, false);
-                } else {
-                    l = g.probes[hi];
-                    const float* cen = g.centroids + (size_t)l * g.dim;
-                    d = adc_row_direct<M>(row, s_tab, g.codebook, g.m, g.k, dsub, g.tree != 0, cen);
-                }
-                if (d <= cut) {
-                    const long long delta = g.row_delta ? g.row_delta[l] : 0;
-                    key = make_key(d, (uint32_t)(r + delta));
-                    ++valid;
-                }
-            }
-        }
-        s_keys[i] = key;
-    }
-    if (valid) atomicAdd(&s_valid, valid);
-    __syncthreads();
-    const int nv = s_valid;
-    if (nv < need) {
-        if (threadIdx.x == 0) g.fail_list[atomicAdd(g.n_fail, 1)] = q;
-        return;
-    }
-    if (threadIdx.x == 0) atomicAdd(&g.counters[1], (unsigned long long)nv);
-    block_bitonic_sort(s_keys, n);
-    const int keep = nv < g.stage1_k ? nv : g.stage1_k;
-    for (int i = threadIdx.x; i < g.stage1_k; i += blockDim.x) {
-        const bool ok = i < keep;
-        g.out_rows[(size_t)q * g.stage1_k + i] = ok ? (int)key_idx(s_keys[i]) : -1;
-        if (g.out_dist) g.out_dist[(size_t)q * g.stage1_k + i] = ok ? key_dist(s_keys[i]) : FLT_MAX;
-    }
-    if (g.out_count && threadIdx.x == 0) g.out_count[q] = keep;
-}
-
 // Shared-memory plan of k_scan_tc for a shape: query-tile slots, row-tile stages and the dynamic bytes; false when the
 // shape is outside the kernel's range or does not fit.
 bool tc_scan_plan(int dim, int m, int k, int* na, int* ns, size_t* bytes) {
@@ -794,39 +697,6 @@ psb_status launch_scan_tc(const ScanTcLaunch& L, cudaStream_t s) {
             case 16: return run_scan_tc<8, 16>(g, grid, smem, s);
             default: return run_scan_tc<8, 0>(g, grid, smem, s);
         }
-    }
-}
-
-namespace {
-template <int M>
-psb_status run_select_rescore(const RescoreArgs& g, int nq, cudaStream_t s) {
-    const size_t smem = (size_t)g.pool_cap * 8 + (g.residual ? (size_t)g.dim * 4 : (size_t)g.m * g.k * 4);
-    if (smem > (size_t)226 * 1024) return fail(PSB_UNSUPPORTED_SHAPE, "re-scoring selection does not fit shared memory");
-    if (smem > 32 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_select_rescore<M>), smem));
-    PSB_TRY(prefer_max_shared(k_select_rescore<M>));
-    k_select_rescore<M><<<nq, kRescoreThreads, smem, s>>>(g);
-    count_launch();
-    PSB_LAUNCH_CHECK();
-    return PSB_OK;
-}
-}  // namespace
-
-psb_status launch_select_rescore(const SelectRescoreLaunch& L, int nq, cudaStream_t s) {
-    if (nq <= 0) return PSB_OK;
-    RescoreArgs g;
-    g.pool = L.pool; g.pool_cnt = L.pool_cnt; g.pool_cap = L.pool_cap; g.q_rows = L.q_rows; g.thr = L.thr; g.stage1_k = L.stage1_k;
-    g.lut = L.lut; g.queries = L.queries; g.centroids = L.centroids; g.codebook = L.codebook; g.probes = L.probes;
-    g.nprobe = L.nprobe; g.dim = L.dim; g.nlist = L.nlist; g.codes = L.codes; g.row_base = L.row_base; g.row_delta = L.row_delta;
-    g.m = L.m; g.k = L.k; g.residual = L.residual ? 1 : 0; g.tree = L.tree ? 1 : 0;
-    g.out_rows = L.out_rows; g.out_dist = L.out_dist; g.out_count = L.out_count; g.fail_list = L.fail_list; g.n_fail = L.n_fail;
-    g.counters = L.counters; g.shared_cut = L.shared_cut ? 1 : 0;
-    switch (L.m) {
-        case 8: return run_select_rescore<8>(g, nq, s);
-        case 16: return run_select_rescore<16>(g, nq, s);
-        case 32: return run_select_rescore<32>(g, nq, s);
-        case 48: return run_select_rescore<48>(g, nq, s);
-        case 64: return run_select_rescore<64>(g, nq, s);
-        default: return run_select_rescore<0>(g, nq, s);
     }
 }
 
