@@ -226,9 +226,46 @@ __device__ __forceinline__ void stage_residual_table(float* __restrict__ s_lut, 
 //   all, and the cutoff is the r-th smallest sample distance with r = ceil(mu + 4 sqrt(mu) + 2), mu = stage1_k * n_s / N:
 //   the stage1_k-th smallest of all N distances lies below it except with negligible probability, and about r * stride
 //   rows (2-4 x stage1_k) pass it.  The selection kernel verifies that each pool holds at least stage1_k rows and did
-//   not overflow; the exact fallback handles the rest.  The r smallest sample keys are kept with a running cutoff:
-//   keys below it go to a 2048-entry buffer that is sorted and cut back to r whenever it could overflow.
-constexpr int kSeedBuf = 2048;
+//   not overflow; the exact fallback handles the rest.  The smallest sample keys are kept with a running cutoff: keys up to it go
+//   to a 4,096-entry buffer that is cut back to little more than r whenever it could overflow.  The cuts, the last one among them,
+//   are bisections over the keys (a cutoff that lets an r / 8th more through does no harm; sorting the buffer for the r-th key took
+//   a quarter of the kernel), and a thread takes four samples at a time, whose chains of dependent loads - probe, list, row - overlap.
+constexpr int kSeedBuf = 4096;
+constexpr int kSeedUnroll = 4;
+// Block-wide: a value that at least r and, equal keys aside, at most r + r / 8 of the c >= r keys do not exceed.  s_cnt [2 * warps].
+__device__ __forceinline__ uint32_t seed_bound(const uint32_t* __restrict__ s_keys, int c, int r, int* s_cnt) {
+    constexpr int kPer = kSeedBuf / kSeedThreads, kWarps = kSeedThreads / 32;
+    uint32_t v[kPer];
+    uint32_t mn = 0xffffffffu, mx = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int i = threadIdx.x + j * kSeedThreads;
+        v[j] = i < c ? s_keys[i] : 0xffffffffu;
+        if (i < c) { mn = min(mn, v[j]); mx = max(mx, v[j]); }
+    }
+    int flip = 0;
+    auto all = [&](uint32_t x, bool add, bool low) -> uint32_t {   // block-wide sum, minimum or maximum, one barrier
+        const uint32_t w = add ? __reduce_add_sync(0xffffffffu, x) : (low ? __reduce_min_sync(0xffffffffu, x) : __reduce_max_sync(0xffffffffu, x));
+        int* s = s_cnt + kWarps * (flip ^= 1);
+        if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = (int)w;
+        __syncthreads();
+        const uint32_t t = (uint32_t)s[threadIdx.x & (kWarps - 1)];
+        return add ? __reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < kWarps ? t : 0u) : (low ? __reduce_min_sync(0xffffffffu, t) : __reduce_max_sync(0xffffffffu, t));
+    };
+    uint32_t lo = all(mn, false, true), hi = all(mx, false, false);
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        int n = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) n += v[j] <= mid ? 1 : 0;
+        n = (int)all((uint32_t)n, true, false);
+        if (n < r) { lo = mid + 1; continue; }
+        hi = mid;
+        if (n <= r + (r >> 3)) break;
+    }
+    __syncthreads();
+    return hi;
+}
 template <int M>
 __global__ void __launch_bounds__(kSeedThreads)
 k_seed_threshold(const float* __restrict__ lut, const int* __restrict__ probes, int nprobe,
@@ -244,7 +281,7 @@ k_seed_threshold(const float* __restrict__ lut, const int* __restrict__ probes, 
     uint32_t* s_keys = reinterpret_cast<uint32_t*>(s_seed_raw + (size_t)m * k * 4);       // [kSeedBuf]
     int* s_pref = reinterpret_cast<int*>(s_seed_raw + (size_t)m * k * 4 + kSeedBuf * 4);  // [nprobe + 1]
     __shared__ int s_warp[32];
-    __shared__ int s_total, s_cnt;
+    __shared__ int s_total, s_cnt, s_bound[2 * kSeedThreads / 32];
     __shared__ uint32_t s_cut;
     const int q = blockIdx.x;
     const long long N = q_rows[q];
@@ -272,15 +309,31 @@ k_seed_threshold(const float* __restrict__ lut, const int* __restrict__ probes, 
     const bool flat_bias = per_probe && lut == nullptr;
     float* s_pk = reinterpret_cast<float*>(s_pref + nprobe + 1);  // [nprobe] |q - c|^2 per probe (flat_bias only)
     if (!per_probe) {
-        for (int e = threadIdx.x; e < m * k; e += blockDim.x) s_lut[e] = lut[(size_t)q * m * k + e];
+        const float* src = lut + (size_t)q * m * k;
+        if (((m * k) & 3) == 0) {
+#pragma unroll 4
+            for (int e = threadIdx.x; e < m * k / 4; e += kSeedThreads) reinterpret_cast<float4*>(s_lut)[e] = __ldg(reinterpret_cast<const float4*>(src) + e);
+        } else {
+            for (int e = threadIdx.x; e < m * k; e += kSeedThreads) s_lut[e] = src[e];
+        }
     } else if (flat_bias) {
         const int dsub = rs.dim / m;
         const float* qv = rs.queries + (size_t)q * rs.dim;
-        for (int e = threadIdx.x; e < m * k; e += blockDim.x) {
-            const int sub = e / k;
+        const bool pairs = (dsub & 1) == 0 && (reinterpret_cast<uintptr_t>(rs.codebook) & 7) == 0;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < m * k; e += kSeedThreads) {
+            const int sub = k == 256 ? e >> 8 : e / k;
             const float* c = rs.codebook + (size_t)e * dsub;
             float dot = 0.0f;
-            for (int d = 0; d < dsub; ++d) dot = fmaf(__ldg(qv + sub * dsub + d), __ldg(c + d), dot);
+            if (pairs) {
+                for (int d = 0; d < dsub; d += 2) {
+                    const float2 w = __ldg(reinterpret_cast<const float2*>(c + d));
+                    dot = fmaf(__ldg(qv + sub * dsub + d), w.x, dot);
+                    dot = fmaf(__ldg(qv + sub * dsub + d + 1), w.y, dot);
+                }
+            } else {
+                for (int d = 0; d < dsub; ++d) dot = fmaf(__ldg(qv + sub * dsub + d), __ldg(c + d), dot);
+            }
             s_lut[e] = -2.0f * dot;
         }
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -322,7 +375,7 @@ k_seed_threshold(const float* __restrict__ lut, const int* __restrict__ probes, 
         for (int it = 0; it < 6; ++it) c = mu + margin_sigma * sqrtf(c) + 2.0f;
         r = (int)ceilf(c) + 8;
     }
-    if ((r >= ns && !rec) || r + (int)blockDim.x > kSeedBuf) { if (threadIdx.x == 0) thr[q] = inf; empty_record(0); return; }
+    if ((r >= ns && !rec) || r + (r >> 3) + kSeedUnroll * kSeedThreads > kSeedBuf) { if (threadIdx.x == 0) thr[q] = inf; empty_record(0); return; }
     __syncthreads();
     const bool staged_probes = per_probe && !flat_bias;  // one table per probe, staged one after the other
     const int nseg = staged_probes ? nprobe : 1;
@@ -334,42 +387,69 @@ k_seed_threshold(const float* __restrict__ lut, const int* __restrict__ probes, 
             stage_residual_table(s_lut, lut, rs, q, sg, nprobe, probes[(size_t)q * nprobe + sg], m, k);
             __syncthreads();
         }
-        for (int base = b0; base < b1; base += blockDim.x) {
+        for (int base = b0; base < b1; base += kSeedUnroll * kSeedThreads) {
             const int c_now = s_cnt;  // stable since the barrier that ended the previous round
             __syncthreads();
-            if (c_now + (int)blockDim.x > kSeedBuf) {  // uniform
-                for (int i = c_now + threadIdx.x; i < kSeedBuf; i += blockDim.x) s_keys[i] = 0xffffffffu;
+            if (c_now + kSeedUnroll * kSeedThreads > kSeedBuf) {  // uniform; c_now >= r here
+                const uint32_t bound = seed_bound(s_keys, c_now, r, s_bound);
+                uint32_t v[kSeedBuf / kSeedThreads];
+#pragma unroll
+                for (int j = 0; j < kSeedBuf / kSeedThreads; ++j) {
+                    const int i = threadIdx.x + j * kSeedThreads;
+                    v[j] = i < c_now ? s_keys[i] : 0xffffffffu;
+                }
+                if (threadIdx.x == 0) { s_cnt = 0; s_cut = bound; }
                 __syncthreads();
-                block_bitonic_sort(s_keys, kSeedBuf);
-                if (threadIdx.x == 0) { s_cnt = r; s_cut = s_keys[r - 1]; }  // c_now >= r here
+#pragma unroll
+                for (int j = 0; j < kSeedBuf / kSeedThreads; ++j)   // equal keys beyond the room left are copies of the bound: they may go
+                    if (v[j] < bound) s_keys[atomicAdd(&s_cnt, 1)] = v[j];
+                __syncthreads();
+                const int less = s_cnt;
+                __syncthreads();
+                for (int i = less + threadIdx.x; i < r; i += kSeedThreads) s_keys[i] = bound;
+                if (threadIdx.x == 0) s_cnt = less > r ? less : r;
                 __syncthreads();
             }
-            const int idx = base + threadIdx.x;
-            if (idx < b1) {
-                int lo = sg, hi = nprobe;  // largest p with s_pref[p] <= idx
-                if (!staged_probes) {
-                    lo = 0;
-                    while (hi - lo > 1) {
-                        const int mid = (lo + hi) >> 1;
-                        if (s_pref[mid] <= idx) lo = mid; else hi = mid;
+            const uint32_t cut = s_cut;
+            float sd[kSeedUnroll];
+#pragma unroll
+            for (int u = 0; u < kSeedUnroll; ++u) {
+                const int idx = base + u * kSeedThreads + threadIdx.x;
+                sd[u] = inf;
+                if (idx < b1) {
+                    int lo = sg, hi = nprobe;  // largest p with s_pref[p] <= idx
+                    if (!staged_probes) {
+                        lo = 0;
+                        while (hi - lo > 1) {
+                            const int mid = (lo + hi) >> 1;
+                            if (s_pref[mid] <= idx) lo = mid; else hi = mid;
+                        }
                     }
+                    const int l = probes[(size_t)q * nprobe + lo];
+                    const long long row = offsets[l] + (long long)(idx - s_pref[lo]) * stride;
+                    float d = adc_row<M>(codes + (size_t)(row - row_base) * m, s_lut, m, k, tree != 0);
+                    if (flat_bias) {
+                        const float corr = rs.row_bias ? __ldg(rs.row_bias + (row - row_base))
+                                                       : fmaf(rs.rc_scale, (float)__ldg(rs.row_bias_u16 + (row - row_base)), rs.rc_offset);
+                        d = fmaxf(d + s_pk[lo] + corr, 0.0f);
+                    }
+                    sd[u] = d;
                 }
-                const int l = probes[(size_t)q * nprobe + lo];
-                const long long row = offsets[l] + (long long)(idx - s_pref[lo]) * stride;
-                const uint8_t* rp = codes + (size_t)(row - row_base) * m;
-                float sd = adc_row<M>(rp, s_lut, m, k, tree != 0);
-                if (flat_bias) {
-                    const float corr = rs.row_bias ? __ldg(rs.row_bias + (row - row_base))
-                                                   : fmaf(rs.rc_scale, (float)__ldg(rs.row_bias_u16 + (row - row_base)), rs.rc_offset);
-                    sd = fmaxf(sd + s_pk[lo] + corr, 0.0f);
-                }
-                const uint32_t key = f2o(sd);
-                if (key < s_cut) s_keys[atomicAdd(&s_cnt, 1)] = key;
+            }
+#pragma unroll
+            for (int u = 0; u < kSeedUnroll; ++u) {
+                const uint32_t key = f2o(sd[u]);
+                if (base + u * kSeedThreads + (int)threadIdx.x < b1 && key < cut) s_keys[atomicAdd(&s_cnt, 1)] = key;
             }
             __syncthreads();
         }
     }
     const int c = s_cnt;
+    if (!rec) {
+        const uint32_t bound = c >= r ? seed_bound(s_keys, c, r, s_bound) : 0u;
+        if (threadIdx.x == 0) thr[q] = c >= r ? o2f(bound) : inf;
+        return;
+    }
     for (int i = c + threadIdx.x; i < kSeedBuf; i += blockDim.x) s_keys[i] = 0xffffffffu;
     __syncthreads();
     block_bitonic_sort(s_keys, kSeedBuf);
