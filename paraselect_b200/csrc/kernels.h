@@ -334,6 +334,10 @@ psb_status launch_widen_ids(const int* d_in, long long n, long long* d_out, cuda
 // ---- training ------------------------------------------------------------------------------------------------
 psb_status launch_pq_encode(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
                             uint8_t* d_codes, cudaStream_t s);
+// The assignment of PQ training's Lloyd iterations: |c|^2 - 2 x.c in fused multiply-adds for sub-vectors of 2, 4 or 8 (else the encoder's
+// arithmetic).
+psb_status launch_pq_assign_train(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
+                                  uint8_t* d_codes, cudaStream_t s);
 psb_status launch_pq_accumulate(const float* d_data, long long n, int dim, const uint8_t* d_codes, int m, int k,
                                 double* d_sums, int* d_counts, cudaStream_t s);
 // Codewords = sums / counts (no rows: kept); leaves the sums and counts zeroed.

@@ -2480,7 +2480,7 @@ psb_status psb_pq_train(const float* d_data, int64_t n, int dim, int subvectors,
     }
     PSB_TRY(launch_pq_init_rows(d_data, dim, subvectors, codebook_size, d_rows, d_codebook, st));
     for (int it = 0; it < iters; ++it) {
-        PSB_TRY(launch_pq_encode(d_data, n, dim, d_codebook, subvectors, codebook_size, codes, st));
+        PSB_TRY(launch_pq_assign_train(d_data, n, dim, d_codebook, subvectors, codebook_size, codes, st));
         PSB_TRY(launch_pq_accumulate(d_data, n, dim, codes, subvectors, codebook_size, sums, counts, st));
         PSB_TRY(launch_pq_update(sums, counts, subvectors, codebook_size, dsub, d_codebook, st));
     }

@@ -103,6 +103,8 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
 //   E: bf16 splits 3.1 * 2^-18 |x||c|; accumulation and norm split (16 KS) 2^-22 (|x||c| + |c|^2 / 2); rounding of the exact fp32
 //   distance (2 dsub + 2) 2^-24 (|x| + |c|)^2: together 2E <= 2^-15 |x| cmax + (KS + 1) 2^-18 (|x| + cmax)^2.
 // The nearest codeword in the exact arithmetic and all its ties are among the evaluated ones; the lowest index wins a tie.
+// kTrain: the evaluated ones are compared by |c|^2 - 2 x.c in fused multiply-adds, as the trainer's Lloyd iterations always have (the
+// reference's trainer assigns with a TF32 GEMM: src/quantization/pq/pq_trainer.cu:97-170); its rounding is within the same bound.
 // A warp takes 32 rows at a time (two 16-row tiles share every B fragment); a group's maximum is kept, not its values, so that the
 // 256 products of a row cost 16 registers; hits are queued and evaluated by full warps, one group per lane.  Rows pass through a
 // shared-memory tile of 32 floats each (read by 8 rows per request straight from global memory they took two thirds of the
@@ -189,7 +191,7 @@ __device__ __forceinline__ float near_a_words(const float* __restrict__ x, int t
     return n2;
 }
 
-template <int D>
+template <int D, bool kTrain>
 __global__ void __launch_bounds__(kNearWarps * 32, 2)
 k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* __restrict__ codebook, int m, int k, int subs_per_cta,
              uint8_t* __restrict__ codes) {
@@ -316,13 +318,20 @@ k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* 
                     const int c = c0 + (j & 1) + (j >> 1) * 8;
                     float cv[D], dist = 0.0f;
                     near_load<D>(cv, s_cb + c * D);
+                    if constexpr (kTrain) {
 #pragma unroll
-                    for (int d = 0; d < D; ++d) {
-                        const float diff = __fsub_rn(xv[d], cv[d]);
-                        dist = __fadd_rn(dist, __fmul_rn(diff, diff));
+                        for (int d = 0; d < D; ++d) dist = fmaf(cv[d], cv[d], dist);
+#pragma unroll
+                        for (int d = 0; d < D; ++d) dist = fmaf(xv[d], -2.0f * cv[d], dist);
+                    } else {
+#pragma unroll
+                        for (int d = 0; d < D; ++d) {
+                            const float diff = __fsub_rn(xv[d], cv[d]);
+                            dist = __fadd_rn(dist, __fmul_rn(diff, diff));
+                        }
                     }
                     if (c < k && dist < FLT_MAX) {
-                        const unsigned long long kk = ((unsigned long long)__float_as_uint(dist) << 32) | (unsigned)c;
+                        const unsigned long long kk = make_key(dist, (unsigned)c);
                         key = kk < key ? kk : key;
                     }
                 }
@@ -741,7 +750,7 @@ __global__ void k_gen_normal(uint64_t seed, long long first, long long n, float 
 }  // namespace
 
 namespace {
-template <int D>
+template <int D, bool kTrain = false>
 psb_status run_pq_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, uint8_t* d_codes, cudaStream_t s) {
     // A CTA walks its sub-quantisers one after the other; with few row blocks they are cut into ranges so that two CTAs per SM
     // have work, down to one sub-quantiser each.
@@ -749,8 +758,8 @@ psb_status run_pq_nearest(const float* d_data, long long n, int dim, const float
     const int ranges = (int)std::max<long long>(1, std::min<long long>(m, (2 * 148 + blocks - 1) / blocks));
     const int per = (m + ranges - 1) / ranges;
     const size_t smem = near_smem<D>(per);
-    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_nearest<D>), smem));
-    k_pq_nearest<D><<<dim3((unsigned)blocks, (unsigned)((m + per - 1) / per)), kNearWarps * 32, smem, s>>>(d_data, n, dim, d_codebook, m, k, per, d_codes);
+    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_nearest<D, kTrain>), smem));
+    k_pq_nearest<D, kTrain><<<dim3((unsigned)blocks, (unsigned)((m + per - 1) / per)), kNearWarps * 32, smem, s>>>(d_data, n, dim, d_codebook, m, k, per, d_codes);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
@@ -790,6 +799,20 @@ psb_status launch_pq_encode(const float* d_data, long long n, int dim, const flo
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
+}
+
+psb_status launch_pq_assign_train(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
+                                  uint8_t* d_codes, cudaStream_t s) {
+    if (n <= 0) return PSB_OK;
+    if (k > 32 && m <= 192) {
+        switch (dim / m) {
+            case 2: return run_pq_nearest<2, true>(d_data, n, dim, d_codebook, m, k, d_codes, s);
+            case 4: return run_pq_nearest<4, true>(d_data, n, dim, d_codebook, m, k, d_codes, s);
+            case 8: return run_pq_nearest<8, true>(d_data, n, dim, d_codebook, m, k, d_codes, s);
+            default: break;
+        }
+    }
+    return launch_pq_encode(d_data, n, dim, d_codebook, m, k, d_codes, s);
 }
 
 psb_status launch_pq_accumulate(const float* d_data, long long n, int dim, const uint8_t* d_codes, int m, int k,
