@@ -7,13 +7,13 @@
 //                   widths from 32 up are register pairs.  Every butterfly still computes (lhs + rhs, lhs - rhs) on the same
 //                   pairs, the per-row statistic goes through the same two shuffle-down trees, so the bits are the same; a row
 //                   costs no barrier and the loads of 8 rows per CTA are in flight together.
-//   k_sign_scan     one CTA per (query, slice of its probes): rows of the probed lists are scored against the state of their
+//   k_sign_scan_*   one CTA per (query, slice of its probes): rows of the probed lists are scored against the state of their
 //                   (query, probe) - one chain over d = 0..dim-1 of +-state[d] for float states, a popcount for sign-coded
 //                   ones (src/quantization/turboquant/turboquant_1bit_score.cuh:17-72) - and the candidate_count smallest
 //                   (score, row) keys are kept in shared memory: a row enters the buffer only below the current cutoff, a full
 //                   buffer is cut back to candidate_count by a radix selection, and the survivors are sorted once at the end.
-//                   For float states a table of partial sums gives every row a score with a known error bound first; only
-//                   rows that could be below the cutoff get the exact chain (see the kernel).  The reference sorts every
+//                   For float states the tensor cores give every row a score with a known error bound first; only rows that
+//                   could be among the candidate_count get the exact chain (see the kernel).  The reference sorts every
 //                   group of 8 chunks of 2,048 rows and merges the groups' lists per query
 //                   (turboquant_1bit_grouped_scan.cu:92-190, 45-90); the result, the exact candidate_count smallest keys in
 //                   ascending order, is the same.
@@ -341,6 +341,7 @@ struct SignScanArgs {
     const long long* offsets;     // [nlist + 1]
     const int* probes;            // [nq][nprobe]
     int nlist, nq, nprobe, dim, k, kp2, cap, split;
+    int seg;                      // waiting rows per warp (float states)
     uint64_t* partial;            // [nq][split][k] when split > 1
     int* rows_out;                // [nq][k]
     float* dist_out;              // [nq][k] or null
@@ -470,7 +471,7 @@ __device__ __forceinline__ int sign_finish(uint64_t* keys, uint64_t* spill, int 
 
 // The exact scores of up to kScanRows rows per thread, each against the float state `state[r]` points to (global memory: the
 // rows of a thread may belong to different probes): one chain over d = 0..dim-1 per row, the chains interleaved.
-template <int W>
+template <int W, bool WIDE>   // WIDE: the states are 16-byte aligned
 __device__ __forceinline__ void exact_float_scores(const CodeWords<W> (&c)[kScanRows], const float (&param)[kScanRows],
                                                    const float* const (&state)[kScanRows], const float (&norm_sq)[kScanRows],
                                                    float (&score)[kScanRows]) {
@@ -480,9 +481,22 @@ __device__ __forceinline__ void exact_float_scores(const CodeWords<W> (&c)[kScan
 #pragma unroll
     for (int w = 0; w < W; ++w) {
 #pragma unroll
-        for (int bit = 0; bit < 32; ++bit) {
+        for (int bit = 0; bit < 32; bit += 4) {
+            float4 v[kScanRows];
 #pragma unroll
-            for (int r = 0; r < kScanRows; ++r) dot[r] = sign_step(dot[r], __ldg(state[r] + 32 * w + bit), c[r].w[w], 1u << bit);
+            for (int r = 0; r < kScanRows; ++r) {
+                const float* x = state[r] + 32 * w + bit;
+                if (WIDE) v[r] = __ldg(reinterpret_cast<const float4*>(x));
+                else v[r] = make_float4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
+            }
+#pragma unroll
+            for (int r = 0; r < kScanRows; ++r) dot[r] = sign_step(dot[r], v[r].x, c[r].w[w], 1u << bit);
+#pragma unroll
+            for (int r = 0; r < kScanRows; ++r) dot[r] = sign_step(dot[r], v[r].y, c[r].w[w], 2u << bit);
+#pragma unroll
+            for (int r = 0; r < kScanRows; ++r) dot[r] = sign_step(dot[r], v[r].z, c[r].w[w], 4u << bit);
+#pragma unroll
+            for (int r = 0; r < kScanRows; ++r) dot[r] = sign_step(dot[r], v[r].w, c[r].w[w], 8u << bit);
         }
     }
     const float dimf = (float)(32 * W);
@@ -493,152 +507,95 @@ __device__ __forceinline__ void exact_float_scores(const CodeWords<W> (&c)[kScan
     }
 }
 
-// The signed sum of a row from a table of the 16 possible sums of every group of four dimensions: dim / 4 look-ups instead of
-// dim additions.  The order of the additions differs from the chain's, so the value may differ from the exact dot in the last
-// bits; the caller allows for that.  lut[g * 16 + v], v = the four sign bits of group g: the 16 entries of a group lie in 16
-// different banks, so a warp's look-ups never collide.
+constexpr int kUnitRows = 64, kStepUnits = 2;   // rows a warp takes at a time, and how often between two looks at the queue
+
+// The filter's dot products, on the integer tensor cores.  A row's sign bits b_d are bytes of the left operand: a code word masked with
+// 0x01010101 << p holds four of them as 0 or 2^p, p < 4, and the word shifted right by 4 the other half, so an operand register costs
+// one mask.  The state is two columns of bytes, w_d = 256 hi_d + lo_d = state[d] / (2^p delta) to the nearest, p = d mod 4, and
+//   sum +-state[d] = delta (2 (256 sum b 2^p hi + sum b 2^p lo) - sum 2^p w)   within  delta / 2 (1 + 2 + 4 + 8) dim / 4.
+// The sums are exact whole numbers.  All four column pairs of mma.m16n8k32 hold the same two columns: after four tiles of 16 rows
+// every thread picks the tile of its own and has two rows.
+// Which bits make which K slots is free as long as the state's bytes follow: thread t of a quad takes word t (padded_dim 128; its half
+// of word t / 2 for 64, a quarter of the only word for 32, words t and t + 4 for 256), byte positions p and p + 1 of it per step.
+__device__ __forceinline__ void imma_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <int W> __device__ __forceinline__ int slot_word(int s, int t) { return W >= 4 ? t + 4 * (s >> 2) : (W == 2 ? t >> 1 : 0); }
+template <int W> __device__ __forceinline__ int slot_bit(int s, int t) { return W >= 4 ? 2 * (s & 3) : (W == 2 ? 4 * (t & 1) + 2 * s : 2 * t); }
+// out[0], out[1]: sum b 2^p w of rows base + 16 t + g and + 8 (t, g: lane % 4, lane / 4); rows past `last`, the last of all, repeat it.
 template <int W>
-__device__ __forceinline__ float table_dot(const CodeWords<W>& c, const float* lut) {
-    float a0 = 0.f, a1 = 0.f;
+__device__ __forceinline__ void tile_dots(const uint32_t* __restrict__ codes, int base, int last, const uint2 (&b)[W], int (&out)[2]) {
+    constexpr int WPT = W >= 4 ? W / 4 : 1;
+    const int lane = threadIdx.x & 31, t = lane & 3, g = lane >> 2;
+    uint32_t x[4][2][WPT];
+    if (base + kUnitRows - 1 <= last) {   // warp-uniform; one address, for padded_dim 128 consecutive words in every load
+        const uint32_t* code = codes + (size_t)(base + g) * W + slot_word<W>(0, t);
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-        const uint32_t word = c.w[w];
+        for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int t = 0; t < 8; t += 2) {
-            a0 += lut[(8 * w + t) * 16 + ((word >> (4 * t)) & 15u)];
-            a1 += lut[(8 * w + t + 1) * 16 + ((word >> (4 * t + 4)) & 15u)];
-        }
+            for (int i = 0; i < WPT; ++i) x[j >> 1][j & 1][i] = __ldg(code + 8 * j * W + 4 * i);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int i = 0; i < WPT; ++i) x[j >> 1][j & 1][i] = __ldg(codes + (size_t)min(base + 8 * j + g, last) * W + slot_word<W>(4 * i, t));
     }
-    return a0 + a1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        int acc[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int s = 0; s < W; ++s) {
+            const int p = slot_bit<W>(s, t), i = W >= 4 ? s >> 2 : 0;
+            const uint32_t u = x[j][0][i] >> (p & 4), v = x[j][1][i] >> (p & 4);
+            const uint32_t m0 = 0x01010101u << (p & 3), m1 = m0 << 1;
+            imma_16832(acc, u & m0, v & m0, u & m1, v & m1, b[s].x, b[s].y);
+        }
+        if (t == j) { out[0] = 256 * acc[0] + acc[1]; out[1] = 256 * acc[2] + acc[3]; }
+    }
 }
 
-constexpr int kQueueCap = 2 * kScanStep;   // rows waiting for their exact score
+// The kept keys to the query's output, or to its slice's place for k_sign_merge.
+__device__ __forceinline__ void sign_output(const SignScanArgs& a, int q, int slice, const uint64_t* keys, int n) {
+    if (a.split > 1) {
+        uint64_t* out = a.partial + ((size_t)q * a.split + slice) * a.k;
+        for (int i = threadIdx.x; i < a.k; i += kScanThreads) out[i] = i < n ? keys[i] : KEY_MAX;
+    } else {
+        for (int i = threadIdx.x; i < a.k; i += kScanThreads) {
+            a.rows_out[(size_t)q * a.k + i] = i < n ? (int)key_idx(keys[i]) : -1;
+            if (a.dist_out) a.dist_out[(size_t)q * a.k + i] = i < n ? key_dist(keys[i]) : FLT_MAX;
+        }
+    }
+}
 
-// Scan of one (query, slice of probes) per CTA.
-//
-// Sign-coded states (MODE 1): every row's score is a popcount; keys below the cutoff go to the buffer.
-//
-// Float states (MODE 0): a row's score is first taken from the table (table_dot), and only rows whose score could still be
-// below the cutoff - the table score minus a bound on its error against the exact chain - are queued, (row, probe), for the
-// exact chain.  The queue is worked off 1,024 rows at a time, four interleaved chains per thread on all threads, whenever it
-// holds that many (and once at the end), so the chains - 128 dependent additions each - always run with full warps.  Until
-// the first cutoff exists every row is queued.  A queued row is tested against the cutoff of the time its exact score is
-// taken; cutoffs only fall, so nothing is lost by waiting.
-// Error bound of the table score: with A = sum |state[d]|, every partial sum on either path is at most A in magnitude and
-// every rounding at most 2^-24 of it; the chain has dim <= 256 roundings, the table path fewer than 80 (3 per entry,
-// dim / 4 + 1 additions), so |table - chain| < 336 * 2^-24 * A < 2^-15 * A for every dim here.  The queue test uses
-// 2^-14 * A (twice that) on the dot and 2^-20 relative on the final fused multiply-adds.
-template <int W, int MODE>
-__global__ void __launch_bounds__(kScanThreads, W > 4 ? 2 : (MODE == 1 ? 6 : 4)) k_sign_scan(const SignScanArgs a) {
+// Sign-coded states: every row's score is a popcount; keys below the cutoff go to the buffer.  One CTA per (query, slice of probes).
+template <int W>
+__global__ void __launch_bounds__(kScanThreads, W > 4 ? 2 : 6) k_sign_scan_codes(const SignScanArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     uint64_t* keys = reinterpret_cast<uint64_t*>(s_raw);
-    uint64_t* spill = keys + a.cap;                                       // k keys
-    float* s_state = reinterpret_cast<float*>(spill + ((a.k + 1) & ~1));  // 256 floats: the state (MODE 0), 16-byte aligned
-    float* s_lut = s_state + 256;                                         // W * 128 floats: the table (MODE 0)
+    uint64_t* spill = keys + a.cap;   // k keys
     __shared__ SignSelectScratch s_sel;
-    __shared__ uint32_t s_qrow[MODE == 0 ? kQueueCap : 1];
-    __shared__ uint16_t s_qprobe[MODE == 0 ? kQueueCap : 1];
-    __shared__ int s_qn;
     __shared__ int s_cnt;
     __shared__ unsigned long long s_thr;
     const int q = blockIdx.x / a.split, slice = blockIdx.x % a.split;
     const int tid = threadIdx.x;
     const float dimf = (float)(32 * W);
-    if (tid == 0) { s_cnt = 0; s_thr = KEY_MAX; s_qn = 0; }
+    if (tid == 0) { s_cnt = 0; s_thr = KEY_MAX; }
     __syncthreads();
-
-    // MODE 0: takes the exact scores of queued rows, 1,024 per round; with `all` also the last, partial round.  Called by
-    // all threads after a barrier that follows the last append to the queue.
-    auto work_off_queue = [&](bool all) {
-        const int queued = s_qn;
-        int done = 0;
-        while (queued - done >= (all ? 1 : kScanStep)) {
-            const int take = min(kScanStep, queued - done);
-            const int held = s_cnt;
-            __syncthreads();
-            if (held > a.cap - kScanStep) sign_compact(keys, spill, a.k, &s_cnt, &s_thr, &s_sel);   // uniform
-            const unsigned long long thr = s_thr;
-            CodeWords<W> c[kScanRows];
-            float param[kScanRows], norm_sq[kScanRows], score[kScanRows];
-            const float* state[kScanRows];
-            uint32_t row[kScanRows];
-            bool ok[kScanRows];
-#pragma unroll
-            for (int r = 0; r < kScanRows; ++r) {   // four consecutive entries per thread: whole warps work or rest
-                const int at = kScanRows * tid + r;
-                ok[r] = at < take;
-                row[r] = 0u; param[r] = 0.f; norm_sq[r] = 0.f; state[r] = a.states;
-#pragma unroll
-                for (int w = 0; w < W; ++w) c[r].w[w] = 0u;
-                if (ok[r]) {
-                    row[r] = s_qrow[done + at];
-                    const long long st = (long long)q * a.nprobe + s_qprobe[done + at];
-                    c[r] = load_code<W>(a.codes, row[r]);
-                    param[r] = __ldg(a.row_params + row[r]);
-                    norm_sq[r] = __ldg(a.norm_sq + st);
-                    state[r] = a.states + (size_t)st * (32 * W);
-                }
-            }
-            if (ok[0]) {
-                exact_float_scores<W>(c, param, state, norm_sq, score);
-#pragma unroll
-                for (int r = 0; r < kScanRows; ++r) {
-                    if (!ok[r]) continue;
-                    const uint64_t key = make_key(score[r], row[r]);
-                    if (key < thr) keys[atomicAdd(&s_cnt, 1)] = key;   // room for a whole round was made above
-                }
-            }
-            __syncthreads();
-            done += take;
-        }
-        const int rest = queued - done;   // < 1,024 <= done whenever done > 0: source and destination do not overlap
-        if (done > 0) {
-            for (int i = tid; i < rest; i += kScanThreads) { s_qrow[i] = s_qrow[done + i]; s_qprobe[i] = s_qprobe[done + i]; }
-            __syncthreads();
-            if (tid == 0) s_qn = rest;
-            __syncthreads();
-        }
-    };
-
     for (int p = slice; p < a.nprobe; p += a.split) {
         const long long st = (long long)q * a.nprobe + p;
         const int list = a.probes[st];
         if (list < 0 || list >= a.nlist) continue;   // uniform
-        __syncthreads();
-        float abs_sum = 0.f;   // MODE 0: sum |state[d]|, rounded up a little
-        uint32_t qcode[W];     // MODE 1: the state's sign words
-        if (MODE == 0) {
-            for (int d = tid; d < 32 * W; d += kScanThreads) s_state[d] = a.states[(size_t)st * (32 * W) + d];
-            __syncthreads();
-            for (int e = tid; e < W * 128; e += kScanThreads) {   // entry v of group g: ((+-x0 +- x1) +- x2) +- x3
-                const int g = e >> 4, v = e & 15;
-                const float* x = s_state + 4 * g;
-                float t = (v & 1) ? x[0] : -x[0];
-                t += (v & 2) ? x[1] : -x[1];
-                t += (v & 4) ? x[2] : -x[2];
-                t += (v & 8) ? x[3] : -x[3];
-                s_lut[e] = t;
-            }
-            const int lane = tid & 31;
+        uint32_t qcode[W];   // the state's sign words, the same in every thread
 #pragma unroll
-            for (int j = 0; j < W; ++j) abs_sum += fabsf(s_state[lane + 32 * j]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) abs_sum += __shfl_xor_sync(kFull, abs_sum, o);
-            abs_sum *= 1.001f;
-        }
-#pragma unroll
-        for (int w = 0; w < W; ++w) qcode[w] = MODE == 1 ? __ldg(a.state_codes + (size_t)st * W + w) : 0u;   // same in every thread
-        const float qparam = MODE == 0 ? a.norm_sq[st] : a.norms[st];
-        __syncthreads();
+        for (int w = 0; w < W; ++w) qcode[w] = __ldg(a.state_codes + (size_t)st * W + w);
+        const float qparam = a.norms[st];
         const long long beg = a.offsets[list], end = a.offsets[list + 1];
         for (long long row0 = beg; row0 < end; row0 += kScanStep) {
-            unsigned long long thr;
-            if (MODE == 1) {
-                const int held = s_cnt;   // settled: the previous step ended with a barrier
-                __syncthreads();          // ... and nobody appends before everybody has read it
-                if (held > a.cap - kScanStep) sign_compact(keys, spill, a.k, &s_cnt, &s_thr, &s_sel);   // uniform
-            }
-            thr = s_thr;   // MODE 0: changed only inside work_off_queue, between barriers
+            const int held = s_cnt;   // settled: the previous step ended with a barrier
+            __syncthreads();          // ... and nobody appends before everybody has read it
+            if (held > a.cap - kScanStep) sign_compact(keys, spill, a.k, &s_cnt, &s_thr, &s_sel);   // uniform
+            const unsigned long long thr = s_thr;
             CodeWords<W> c[kScanRows];
             float param[kScanRows];
             bool ok[kScanRows];
@@ -654,62 +611,293 @@ __global__ void __launch_bounds__(kScanThreads, W > 4 ? 2 : (MODE == 1 ? 6 : 4))
                     param[r] = 0.f;
                 }
             }
-            if (MODE == 0) {
-                const bool have_cut = thr != KEY_MAX;   // uniform
-                const float cut = key_dist(thr);
-                const float dot_slack = abs_sum * (1.0f / 16384.0f);
-                bool filled = false;   // one of this thread's rows took the queue's 1,024th place
+#pragma unroll
+            for (int r = 0; r < kScanRows; ++r) {
+                if (!ok[r]) continue;
+                int h = 0;
+#pragma unroll
+                for (int w = 0; w < W; ++w) h += __popc(qcode[w] ^ c[r].w[w]);
+                const float cosine = __fdiv_rn(__fsub_rn(dimf, __fmul_rn(2.0f, (float)h)), dimf);
+                const float dn = param[r];
+                const float score = __fmaf_rn(-__fmul_rn(__fmul_rn(2.0f, qparam), dn), cosine, __fmaf_rn(dn, dn, __fmul_rn(qparam, qparam)));
+                const uint64_t key = make_key(score, (uint32_t)rows[r]);
+                if (key < thr) keys[atomicAdd(&s_cnt, 1)] = key;   // room for a whole step was checked above
+            }
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    sign_output(a, q, slice, keys, sign_finish(keys, spill, a.k, a.kp2, &s_cnt, &s_thr, &s_sel));
+}
+
+// Float states.  One CTA per (query, slice of probes); its probes are taken kProbeChunk at a time, their states' bytes and bounds laid
+// out in shared memory together (a warp per state), and the chunk's rows are dealt to the warps in units of 64 of one list.
+// A row first gets a bound: rough - slack <= exact score <= rough + slack, rough from the filter's dot product.  Rows whose
+// lower bound is not above the cut wait, (bound, row, probe), in their warp's part of the queue.  The cut never is below the k-th
+// smallest exact score: k waiting rows have upper bounds, lower + 2 x the largest slack seen, of at most it.  When a warp's part
+// runs full the cut is moved down (a histogram of the bounds finds a value that k of them do not exceed) and what lies above it goes;
+// only if that does not make room - many equal scores, or a k beyond the queue - the waiting rows are scored exactly, into the key
+// buffer, whose k-th key is a cut too.  What still waits at the end, little more than k rows, gets the exact chain.
+//
+// Slack: with A = sum |state[d]| and delta = max |state| / 32,500, the filter's dot is within 1.875 dim delta of the true sum (above), and
+// the exact chain too rounds: every partial sum is at most A in magnitude and each of its dim <= 256 roundings at most 2^-24 of it,
+// less than 2^-15 A in all; a few more come from the multiplications by delta.  Taken: 2 dim delta + 2^-14 A on the dot and
+// 2^-20 relative on the final multiply-adds.
+//
+// The earlier form scored rows from a table of partial sums (32 look-ups of 8 warp instructions per row and warp) and, its cut coming from
+// exact keys alone, sent a third of all rows through the chain.  4,000 queries x 32 of 2,048 lists, 2M rows, k = 512: 1,556 -> 1,041 us.
+constexpr int kProbeChunk = 32;
+constexpr int kScanWarps = kScanThreads / 32;
+template <int W> struct ProbeChunk { static constexpr int value = W > 4 ? kProbeChunk / 2 : kProbeChunk; };
+
+struct SignProbe { int beg, end, probe; float delta2, offset, slack, norm_sq; };   // dot = delta2 x (sum of bytes) + offset
+struct WarpBounds { float lo, hi, slack, kth; int n; };
+
+template <int W>
+__global__ void __launch_bounds__(kScanThreads, W > 4 ? 2 : 4) k_sign_scan_float(const SignScanArgs a) {
+    constexpr int CHUNK = ProbeChunk<W>::value, DIM = 32 * W;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    uint64_t* keys = reinterpret_cast<uint64_t*>(s_raw);
+    uint64_t* spill = keys + a.cap;                                              // k keys
+    int8_t* s_bytes = reinterpret_cast<int8_t*>(spill + ((a.k + 1) & ~1));       // [CHUNK][2][DIM]: high and low bytes, in slot order
+    float* q_low = reinterpret_cast<float*>(s_bytes + CHUNK * 2 * DIM);          // the waiting rows, a.seg per warp
+    uint32_t* q_row = reinterpret_cast<uint32_t*>(q_low + kScanWarps * a.seg);
+    uint16_t* q_probe = reinterpret_cast<uint16_t*>(q_row + kScanWarps * a.seg);
+    __shared__ SignSelectScratch s_sel;
+    __shared__ SignProbe s_probe[CHUNK];
+    __shared__ WarpBounds s_bounds[kScanWarps];
+    __shared__ int s_cnt;
+    __shared__ unsigned long long s_thr;
+    const int q = blockIdx.x / a.split, slice = blockIdx.x % a.split;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = lane & 3, g = lane >> 2;
+    const float dimf = (float)DIM;
+    float* w_low = q_low + warp * a.seg;   // this warp's
+    uint32_t* w_row = q_row + warp * a.seg;
+    uint16_t* w_probe = q_probe + warp * a.seg;
+    if (tid == 0) { s_cnt = 0; s_thr = KEY_MAX; }
+    __syncthreads();
+    int waiting = 0;            // rows in this warp's part
+    float cut = __int_as_float(0x7f800000);   // the same in every thread
+    float max_slack = 0.f, low_min = cut, low_max = -cut;   // over the rows this lane has queued
+
+    // Moves the cut down and drops the waiting rows above it.  Called by all threads after a barrier.
+    auto prune = [&]() {
+        float lo = low_min, hi = low_max, slack = max_slack;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(kFull, lo, o)); hi = fmaxf(hi, __shfl_xor_sync(kFull, hi, o));
+            slack = fmaxf(slack, __shfl_xor_sync(kFull, slack, o));
+        }
+        if (lane == 0) { WarpBounds& b = s_bounds[warp]; b.lo = lo; b.hi = hi; b.slack = slack; b.n = waiting; }
+        s_sel.hist[tid] = 0;
+        if (tid == 0) s_sel.bucket = -1;
+        __syncthreads();
+        int n = 0;
+#pragma unroll
+        for (int i = 0; i < kScanWarps; ++i) {
+            const WarpBounds b = s_bounds[i];
+            lo = fminf(lo, b.lo); hi = fmaxf(hi, b.hi); slack = fmaxf(slack, b.slack); n += b.n;
+        }
+        hi = fminf(hi, cut);   // of those that wait
+        if (n < a.k) return;   // uniform
+        const float scale = 255.0f / (hi - lo);   // no spread, or one beyond float: everything in bin 0
+        auto bin = [&](float x) { return max(0, min(255, __float2int_rz((x - lo) * scale))); };
+        for (int i = lane; i < waiting; i += 32) {
+            const float x = w_low[i];
+            if (fabsf(x) < __int_as_float(0x7f800000)) atomicAdd(&s_sel.hist[bin(x)], 1);
+        }
+        __syncthreads();
+        const int c = s_sel.hist[tid];
+        const int before = block_exclusive_scan(c, s_sel.warp_sums, nullptr);
+        if (before < a.k && a.k <= before + c) s_sel.bucket = tid;
+        __syncthreads();
+        const int bucket = s_sel.bucket;
+        if (bucket < 0) return;   // uniform; fewer than k numbers
+        float kth = -__int_as_float(0x7f800000);
+        for (int i = lane; i < waiting; i += 32) {
+            const float x = w_low[i];
+            if (fabsf(x) < __int_as_float(0x7f800000) && bin(x) <= bucket) kth = fmaxf(kth, x);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) kth = fmaxf(kth, __shfl_xor_sync(kFull, kth, o));
+        if (lane == 0) s_bounds[warp].kth = kth;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kScanWarps; ++i) kth = fmaxf(kth, s_bounds[i].kth);
+        cut = fminf(cut, kth + 2.0f * slack);
+        int kept = 0;
+        for (int i0 = 0; i0 < waiting; i0 += 32) {
+            const int i = i0 + lane;
+            const bool in = i < waiting;
+            const float x = in ? w_low[i] : 0.f;
+            const uint32_t row = in ? w_row[i] : 0u;
+            const uint16_t pr = in ? w_probe[i] : (uint16_t)0;
+            const bool keep = in && !(x > cut);
+            const unsigned mask = __ballot_sync(kFull, keep);   // everyone has read before anyone writes, at or before i
+            if (keep) {
+                const int at = kept + __popc(mask & ((1u << lane) - 1u));
+                w_low[at] = x; w_row[at] = row; w_probe[at] = pr;
+            }
+            kept += __popc(mask);
+            __syncwarp();
+        }
+        waiting = kept;
+    };
+
+    // Exact scores of all waiting rows, up to 1,024 per round.  Called by all threads after a barrier.
+    auto work_off = [&]() {
+        if (lane == 0) s_bounds[warp].n = waiting;
+        __syncthreads();
+        int all = 0;
+#pragma unroll
+        for (int i = 0; i < kScanWarps; ++i) all += s_bounds[i].n;
+        const bool wide = reinterpret_cast<uintptr_t>(a.states) % 16 == 0;
+#pragma unroll 1
+        for (int done = 0; done < all; done += kScanStep) {
+            const int held = s_cnt;
+            __syncthreads();
+            if (held > a.cap - kScanStep) sign_compact(keys, spill, a.k, &s_cnt, &s_thr, &s_sel);   // uniform
+            const unsigned long long thr = s_thr;
+            CodeWords<W> c[kScanRows];
+            float param[kScanRows], norm_sq[kScanRows], score[kScanRows];
+            const float* state[kScanRows];
+            uint32_t row[kScanRows];
+            bool ok[kScanRows];
+#pragma unroll
+            for (int r = 0; r < kScanRows; ++r) {
+                int at = done + kScanRows * tid + r;   // four consecutive rows per thread: whole warps work or rest
+                ok[r] = at < all;
+                row[r] = 0u; param[r] = 0.f; norm_sq[r] = 0.f; state[r] = a.states;
+#pragma unroll
+                for (int w = 0; w < W; ++w) c[r].w[w] = 0u;
+                if (ok[r]) {
+                    int part = 0;
+                    while (at >= s_bounds[part].n) { at -= s_bounds[part].n; ++part; }
+                    at += part * a.seg;
+                    row[r] = q_row[at];
+                    const long long st = (long long)q * a.nprobe + q_probe[at];
+                    c[r] = load_code<W>(a.codes, row[r]);
+                    param[r] = __ldg(a.row_params + row[r]);
+                    norm_sq[r] = __ldg(a.norm_sq + st);
+                    state[r] = a.states + (size_t)st * DIM;
+                }
+            }
+            if (ok[0]) {
+                if (wide) exact_float_scores<W, true>(c, param, state, norm_sq, score);
+                else exact_float_scores<W, false>(c, param, state, norm_sq, score);
 #pragma unroll
                 for (int r = 0; r < kScanRows; ++r) {
                     if (!ok[r]) continue;
-                    bool queue = true;
-                    if (have_cut) {
-                        const float s = param[r], two_s = fabsf(2.0f * s);
-                        const float base = __fmaf_rn(__fmul_rn(dimf, s), s, qparam);
-                        const float rough = __fmaf_rn(-__fmul_rn(2.0f, s), table_dot<W>(c[r], s_lut), base);
-                        const float slack = two_s * dot_slack + (fabsf(base) + two_s * abs_sum) * (1.0f / 1048576.0f);
-                        queue = !(rough - slack > cut);   // NaN queues too
-                    }
-                    if (queue) {
-                        const int at = atomicAdd(&s_qn, 1);   // at most 1,024 join a queue that held fewer than 1,024
-                        s_qrow[at] = (uint32_t)rows[r];
-                        s_qprobe[at] = (uint16_t)p;
-                        filled |= at == kScanStep - 1;
-                    }
+                    const uint64_t key = make_key(score[r], row[r]);
+                    if (key < thr) keys[atomicAdd(&s_cnt, 1)] = key;   // room for a whole round was made above
                 }
-                // The queue held fewer than 1,024 rows before this step, so it holds that many now exactly when that place
-                // was taken in this step: every thread learns it from the barrier itself (reading the counter after the
-                // barrier would race with the next step's appends).
-                if (__syncthreads_or(filled)) work_off_queue(false);
-            } else {
+            }
+            __syncthreads();
+        }
+        waiting = 0;
+        if (s_thr != KEY_MAX) cut = fminf(cut, key_dist(s_thr));
+    };
+
+    const int probes = (a.nprobe - slice + a.split - 1) / a.split;   // of this slice
+    const int last = (int)a.offsets[a.nlist] - 1;
+#pragma unroll 1
+    for (int c0 = 0; c0 < probes; c0 += CHUNK) {
+        const int np = min(CHUNK, probes - c0);
+        __syncthreads();
+        for (int i = warp; i < np; i += kScanWarps) {
+            const int p = slice + (c0 + i) * a.split;
+            const long long st = (long long)q * a.nprobe + p;
+            const int list = a.probes[st];
+            if (list < 0 || list >= a.nlist) {   // warp-uniform
+                if (lane == 0) { s_probe[i].beg = 0; s_probe[i].end = 0; }
+                continue;
+            }
+            float x[W], abs_sum = 0.f, top = 0.f;   // abs_sum: rounded up a little
 #pragma unroll
-                for (int r = 0; r < kScanRows; ++r) {
-                    if (!ok[r]) continue;
-                    int h = 0;
+            for (int j = 0; j < W; ++j) { x[j] = __ldg(a.states + (size_t)st * DIM + lane + 32 * j); abs_sum += fabsf(x[j]); top = fmaxf(top, fabsf(x[j])); }
 #pragma unroll
-                    for (int w = 0; w < W; ++w) h += __popc(qcode[w] ^ c[r].w[w]);
-                    const float cosine = __fdiv_rn(__fsub_rn(dimf, __fmul_rn(2.0f, (float)h)), dimf);
-                    const float dn = param[r];
-                    const float score = __fmaf_rn(-__fmul_rn(__fmul_rn(2.0f, qparam), dn), cosine, __fmaf_rn(dn, dn, __fmul_rn(qparam, qparam)));
-                    const uint64_t key = make_key(score, (uint32_t)rows[r]);
-                    if (key < thr) keys[atomicAdd(&s_cnt, 1)] = key;   // room for a whole step was checked above
+            for (int o = 16; o > 0; o >>= 1) { abs_sum += __shfl_xor_sync(kFull, abs_sum, o); top = fmaxf(top, __shfl_xor_sync(kFull, top, o)); }
+            abs_sum *= 1.001f;
+            const float delta = fmaxf(top, 1e-30f) * (1.0f / 32500.0f);   // never so small that the division leaves its range
+            const float unit = delta * (float)(1 << (lane & 3));
+            int part = 0;
+            int8_t* out = s_bytes + i * 2 * DIM + 4 * (lane & 7) + (lane >> 3);   // slot order: the four bits of a byte position side by side
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                const int v = __float2int_rn(__fdividef(x[j], unit));
+                const int lo = (int)(int8_t)(v & 255), hi = (int)(int8_t)((v - lo) >> 8);
+                out[32 * j] = (int8_t)hi;
+                out[32 * j + DIM] = (int8_t)lo;
+                part += (256 * hi + lo) << (lane & 3);
+            }
+            part = __reduce_add_sync(kFull, part);
+            if (lane == 0)
+                s_probe[i] = SignProbe{(int)a.offsets[list], (int)a.offsets[list + 1], p, 2.0f * delta, -delta * (float)part,
+                                       2.0f * (abs_sum * (1.0f / 16384.0f + 1.0f / 1048576.0f) + 2.0f * dimf * delta), __ldg(a.norm_sq + st)};
+        }
+        __syncthreads();
+        const int units = lane < np ? (s_probe[lane < CHUNK ? lane : 0].end - s_probe[lane < CHUNK ? lane : 0].beg + kUnitRows - 1) / kUnitRows : 0;
+        int upto = units;   // units of this lane's probe and those before it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const int total = __shfl_sync(kFull, upto, 31);
+#pragma unroll 1
+        for (int u0 = 0; u0 < total; u0 += kStepUnits * kScanWarps) {
+#pragma unroll 1
+            for (int h = 0; h < kStepUnits; ++h) {
+                const int u = u0 + h * kScanWarps + warp;
+                if (u >= total) break;   // warp-uniform
+                const int i = __popc(__ballot_sync(kFull, upto <= u));
+                const SignProbe pr = s_probe[i];
+                const int base = pr.beg + (u - __shfl_sync(kFull, upto - units, i)) * kUnitRows;
+                const int mine = base + 16 * t + g;
+                float param[2];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) param[r] = __ldg(a.row_params + min(mine + 8 * r, last));
+                uint2 b[W];   // even columns: high bytes, odd ones: low bytes
+                const uint2* col = reinterpret_cast<const uint2*>(s_bytes + (2 * i + (g & 1)) * DIM);
+#pragma unroll
+                for (int s = 0; s < W; ++s) b[s] = col[slot_word<W>(s, t) * 4 + slot_bit<W>(s, t) / 2];
+                int dots[2];
+                tile_dots<W>(a.codes, base, last, b, dots);
+                float low[2], slack[2];
+                bool wait[2];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const float s = param[r];
+                    const float base_score = __fmaf_rn(__fmul_rn(dimf, s), s, pr.norm_sq);
+                    const float rough = __fmaf_rn(-2.0f * s, __fmaf_rn(pr.delta2, (float)dots[r], pr.offset), base_score);
+                    slack[r] = fabsf(s) * pr.slack + fabsf(base_score) * (1.0f / 1048576.0f);
+                    low[r] = rough - slack[r];
+                    wait[r] = mine + 8 * r < pr.end && !(low[r] > cut);   // NaN waits too
                 }
-                __syncthreads();
+                if (!__any_sync(kFull, wait[0] || wait[1])) continue;
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const unsigned mask = __ballot_sync(kFull, wait[r]);
+                    if (wait[r]) {
+                        const int at = waiting + __popc(mask & ((1u << lane) - 1u));   // room for two units was left
+                        w_low[at] = low[r]; w_row[at] = (uint32_t)(mine + 8 * r); w_probe[at] = (uint16_t)pr.probe;
+                        max_slack = fmaxf(max_slack, slack[r]); low_min = fminf(low_min, low[r]); low_max = fmaxf(low_max, low[r]);
+                    }
+                    waiting += __popc(mask);
+                }
+            }
+            if (__syncthreads_or(waiting > a.seg - kStepUnits * kUnitRows)) {
+                prune();
+                if (__syncthreads_or(waiting > a.seg - kStepUnits * kUnitRows)) work_off();
             }
         }
     }
     __syncthreads();
-    if (MODE == 0) work_off_queue(true);
-    const int n = sign_finish(keys, spill, a.k, a.kp2, &s_cnt, &s_thr, &s_sel);
-    if (a.split > 1) {
-        uint64_t* out = a.partial + ((size_t)q * a.split + slice) * a.k;
-        for (int i = tid; i < a.k; i += kScanThreads) out[i] = i < n ? keys[i] : KEY_MAX;
-    } else {
-        for (int i = tid; i < a.k; i += kScanThreads) {
-            a.rows_out[(size_t)q * a.k + i] = i < n ? (int)key_idx(keys[i]) : -1;
-            if (a.dist_out) a.dist_out[(size_t)q * a.k + i] = i < n ? key_dist(keys[i]) : FLT_MAX;
-        }
-    }
+    prune();
+    __syncthreads();
+    work_off();
+    __syncthreads();
+    sign_output(a, q, slice, keys, sign_finish(keys, spill, a.k, a.kp2, &s_cnt, &s_thr, &s_sel));
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_sign_merge(const uint64_t* __restrict__ partial, int split, int k, int cap,
@@ -776,23 +964,34 @@ psb_status dispatch_encode(const SignEncodeArgs& args, int padded, int sm_count,
     return fail(PSB_INVALID_ARGUMENT, "padded_dim must be 32, 64, 128 or 256");
 }
 
-template <int W, int MODE>
-psb_status run_scan(const SignScanArgs& a, size_t smem, cudaStream_t s) {
-    PSB_TRY(prefer_max_shared(k_sign_scan<W, MODE>));
-    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_sign_scan<W, MODE>), smem));
-    k_sign_scan<W, MODE><<<(unsigned)(a.nq * a.split), kScanThreads, smem, s>>>(a);
+template <int W>
+psb_status run_scan(int mode, SignScanArgs& a, cudaStream_t s) {
+    size_t smem = sizeof(uint64_t) * ((size_t)a.cap + ((a.k + 1) & ~1));
+    auto kernel = k_sign_scan_codes<W>;
+    if (mode == 0) {
+        kernel = k_sign_scan_float<W>;
+        smem += (size_t)ProbeChunk<W>::value * 64 * W;
+        // Room for k waiting rows and two full steps more, so that the bounds alone can move the cut; a k for which that does not fit
+        // beside its key buffer (above 4,096) leaves the cut to the exact keys.
+        const size_t per_row = kScanWarps * (sizeof(float) + sizeof(uint32_t) + sizeof(uint16_t));
+        a.seg = ((a.k + 2 * kScanStep) / kScanWarps + 31) / 32 * 32;
+        if (smem + a.seg * per_row > 222 * 1024) a.seg = 2 * kScanStep / kScanWarps;
+        smem += a.seg * per_row;
+    }
+    PSB_TRY(prefer_max_shared(kernel));
+    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
+    kernel<<<(unsigned)(a.nq * a.split), kScanThreads, smem, s>>>(a);
     PSB_LAUNCH_CHECK();
     count_launch();
     return PSB_OK;
 }
 
-template <int MODE>
-psb_status dispatch_scan(const SignScanArgs& a, size_t smem, cudaStream_t s) {
+psb_status dispatch_scan(int mode, SignScanArgs& a, cudaStream_t s) {
     switch (a.dim) {
-        case 32: return run_scan<1, MODE>(a, smem, s);
-        case 64: return run_scan<2, MODE>(a, smem, s);
-        case 128: return run_scan<4, MODE>(a, smem, s);
-        case 256: return run_scan<8, MODE>(a, smem, s);
+        case 32: return run_scan<1>(mode, a, s);
+        case 64: return run_scan<2>(mode, a, s);
+        case 128: return run_scan<4>(mode, a, s);
+        case 256: return run_scan<8>(mode, a, s);
     }
     return fail(PSB_INVALID_ARGUMENT, "padded_dim must be 32, 64, 128 or 256");
 }
@@ -875,13 +1074,13 @@ psb_status launch_sign_candidates(int mode, const float* d_states, const float* 
         PSB_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&partial), sizeof(uint64_t) * (size_t)nq * split * candidate_count, s));
         a.partial = partial;
     }
-    const size_t smem = sizeof(uint64_t) * ((size_t)a.cap + ((candidate_count + 1) & ~1)) + sizeof(float) * (256 + 1024);
-    psb_status rc = mode == 0 ? dispatch_scan<0>(a, smem, s) : dispatch_scan<1>(a, smem, s);
+    psb_status rc = dispatch_scan(mode, a, s);
     if (rc == PSB_OK && split > 1) {
         const int mcap = pow2_at_least(split * candidate_count);
         const size_t msmem = sizeof(uint64_t) * (size_t)mcap;
-        cudaError_t e = cudaFuncSetAttribute(k_sign_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem);
-        if (e == cudaSuccess) {
+        cudaError_t e = cudaSuccess;
+        rc = kernel_shared(reinterpret_cast<const void*>(k_sign_merge), msmem);
+        if (rc == PSB_OK) {
             k_sign_merge<<<(unsigned)nq, kScanThreads, msmem, s>>>(partial, split, candidate_count, mcap, d_rows_out, d_dist_out);
             e = cudaGetLastError();
             count_launch();
