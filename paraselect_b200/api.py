@@ -681,6 +681,24 @@ class SignIndex:
         self.scales.copy_(t.from_numpy(scales))
         return self
 
+    # Host arrays of a search go through page-locked memory that torch keeps and reuses, so that the copies neither stage nor wait and
+    # the results land in pages that exist already: a fresh 8 MB result took longer to fault in than to copy.  Larger ones go
+    # through pageable memory, so that no caller's results hold much page-locked memory.
+    PINNED_LIMIT_BYTES = 32 << 20
+
+    def _upload(self, array):
+        t = self._t
+        src = t.from_numpy(array)
+        if array.nbytes > self.PINNED_LIMIT_BYTES:
+            return src.to(self.dev)
+        return t.empty(src.shape, dtype=src.dtype, pin_memory=True).copy_(src).to(self.dev, non_blocking=True)
+
+    def _download(self, tensor):
+        t = self._t
+        if tensor.numel() * tensor.element_size() > self.PINNED_LIMIT_BYTES:
+            return tensor.cpu()
+        return t.empty(tensor.shape, dtype=tensor.dtype, pin_memory=True).copy_(tensor, non_blocking=True)
+
     def search_candidates(self, host_queries, host_probe_ids, candidate_count=512, score_mode=SIGN_FLOAT_STATES,
                           want_distances=False):
         """host_queries [nq][dim] fp32, host_probe_ids [nq][nprobe] (ids outside the index are skipped); candidate rows
@@ -694,9 +712,12 @@ class SignIndex:
                 or probes.shape[1] <= 0 or candidate_count <= 0:
             raise InvalidArgument(1, "IVFResTurboQuant search received invalid input")
         nq, nprobe = probes.shape
-        bad = (probes < 0) | (probes >= self.n_clusters)
-        d_probes = t.from_numpy(np.where(bad, -1, probes).astype(np.int32)).to(self.dev)
-        d_q = t.from_numpy(q).to(self.dev)
+        if probes.dtype != np.int32:   # 32-bit ids go as they are: the kernels skip those outside the index
+            bad = (probes < 0) | (probes >= self.n_clusters)
+            probes = np.where(bad, -1, probes).astype(np.int32)
+        stream = t.cuda.current_stream(self.dev)
+        raw = stream.cuda_stream
+        d_probes, d_q = self._upload(probes), self._upload(q)
         words = self.padded_dim // 32
         st = nsq = sc = nm = None
         if score_mode == SIGN_FLOAT_STATES:
@@ -706,14 +727,16 @@ class SignIndex:
             sc = t.empty((nq * nprobe, words), dtype=t.int32, device=self.dev)
             nm = t.empty(nq * nprobe, dtype=t.float32, device=self.dev)
         sign_encode_queries(d_q, self.centroids, d_probes, nq, nprobe, self.n_clusters, self.dim, self.padded_dim, d_states=st,
-                            d_norm_sq=nsq, d_state_codes=sc, d_norms=nm, seed=self.rotation_seed, device=self.device)
+                            d_norm_sq=nsq, d_state_codes=sc, d_norms=nm, seed=self.rotation_seed, device=self.device, stream=raw)
         rows = t.empty((nq, candidate_count), dtype=t.int32, device=self.dev)
         dist = t.empty((nq, candidate_count), dtype=t.float32, device=self.dev) if want_distances else None
         sign_search_candidates(score_mode, self.codes, self.scales, self.offsets, self.n_clusters, d_probes, nq, nprobe,
                                self.padded_dim, candidate_count, rows, dist, d_states=st, d_norm_sq=nsq, d_state_codes=sc,
-                               d_norms=nm, device=self.device)
-        t.cuda.synchronize(self.dev)
-        return (rows.cpu().numpy(), dist.cpu().numpy()) if want_distances else rows.cpu().numpy()
+                               d_norms=nm, device=self.device, stream=raw)
+        rows = self._download(rows)
+        dist = self._download(dist) if want_distances else None
+        stream.synchronize()
+        return (rows.numpy(), dist.numpy()) if want_distances else rows.numpy()
 
     def search(self, host_queries, host_vectors, nprobe, topk, n_rerank=512, reordered_ids=None, queries_u8=None,
                score_mode=SIGN_FLOAT_STATES):
