@@ -42,7 +42,7 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TCO
 
 // Per group of G consecutive values of a 32-value chunk: out = -2 * max(w), i.e. the minimum of a = -2 w.
 template <int G>
-__device__ __forceinline__ void group_mins(const float (&v)[32], float* __restrict__ out) {
+__device__ __forceinline__ void group_mins(const float (&v)[32], float* __restrict__ out, size_t stride) {
 #pragma unroll
     for (int g = 0; g < 32 / G; ++g) {
         float t[G];
@@ -52,19 +52,20 @@ __device__ __forceinline__ void group_mins(const float (&v)[32], float* __restri
         for (int w = G / 2; w >= 1; w >>= 1)  // pairwise tree: short dependency chains
 #pragma unroll
             for (int j = 0; j < w; ++j) t[j] = fmaxf(t[j], t[j + w]);
-        out[g] = -2.0f * t[0];
+        out[g * stride] = -2.0f * t[0];
     }
 }
 
-__device__ __forceinline__ float max32(const float (&v)[32]) {   // three-input maxima, two chains
-    float m0 = v[0], m1 = v[1];
-#pragma unroll
-    for (int j = 2; j < 32; j += 4) {
-        asm("max.f32 %0, %0, %1, %2;" : "+f"(m0) : "f"(v[j]), "f"(v[j + 1]));
-        if (j + 3 < 32) asm("max.f32 %0, %0, %1, %2;" : "+f"(m1) : "f"(v[j + 2]), "f"(v[j + 3]));
-    }
-    return fmaxf(m0, m1);
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float m;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
 }
+template <int FROM>
+__device__ __forceinline__ float max8(const float (&v)[32]) {   // of eight values
+    return fmaxf(max3(max3(v[FROM], v[FROM + 1], v[FROM + 2]), v[FROM + 3], v[FROM + 4]), max3(v[FROM + 5], v[FROM + 6], v[FROM + 7]));
+}
+
 __device__ __forceinline__ void add_f32x2(float& o0, float& o1, float a0, float a1, float b0, float b1) {
     asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
         : "=f"(o0), "=f"(o1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
@@ -81,7 +82,8 @@ struct TcArgs {
     const float* cn2;       // [ntiles * TCOL] |c'|^2, +inf beyond nlist
     const float2* qnorm;    // [nq] |q'| and |q' - qb|
     const float* cmax;      // [2] max |c'| and max |c' - cb|
-    float* gmin;            // pass 1 out: [nq][ngroups]
+    float* gmin;            // pass 1 out: the minimum of row q and group g at [q * gmin_q + g * gmin_g]
+    int gmin_q, gmin_g;
     const float* seltop;    // pass 2 in: [nq][nprobe] ascending group minima (T = last)
     uint32_t* mask;         // pass 2 out: [nq][mwords] one bit per centroid (zeroed before the launch; only non-zero words are written)
     int mwords;             // ntiles * TCOL / 32
@@ -150,7 +152,7 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     if (tid == 0) {
         for (int i = 0; i < kStagesA; ++i) { mbar_init(&a_full[i], 1); mbar_init(&a_empty[i], 1); }
         mbar_init(&b_full, 1); mbar_init(&b_empty, 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpiThreads); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpiWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -248,7 +250,8 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
                     tmem_ld_wait();
                     // the accumulators are in registers: hand the tensor memory back before the arithmetic
                     tc_fence_before();
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[h])) : "memory");
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[h])) : "memory");
                     if (q < a.nq) {
 #pragma unroll
                         for (int half = 0; half < 2; ++half) {
@@ -272,22 +275,27 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
                                 }
                             }
                             if (!kSecondPass) {
-                                float* out = a.gmin + (size_t)q * a.ngroups + (c0 >> a.lg_group);
+                                float* out = a.gmin + (size_t)q * a.gmin_q + (size_t)(c0 >> a.lg_group) * a.gmin_g;
                                 switch (a.lg_group) {  // uniform
-                                    case 5: group_mins<32>(v, out); break;
-                                    case 4: group_mins<16>(v, out); break;
-                                    case 3: group_mins<8>(v, out); break;
-                                    case 2: group_mins<4>(v, out); break;
-                                    case 1: group_mins<2>(v, out); break;
-                                    default: group_mins<1>(v, out); break;
+                                    case 5: out[0] = -2.0f * fmaxf(max3(max8<0>(v), max8<8>(v), max8<16>(v)), max8<24>(v)); break;
+                                    case 4: group_mins<16>(v, out, a.gmin_g); break;
+                                    case 3: group_mins<8>(v, out, a.gmin_g); break;
+                                    case 2: group_mins<4>(v, out, a.gmin_g); break;
+                                    case 1: group_mins<2>(v, out, a.gmin_g); break;
+                                    default: group_mins<1>(v, out, a.gmin_g); break;
                                 }
                             } else {
                                 // one bit per centroid of this 32-column chunk; most chunks hold none, which their maximum tells in a
-                                // quarter of the instructions the bits take
-                                if (max32(v) >= cut) {
+                                // quarter of the instructions the bits take, and so it is with the eighths of a chunk that does
+                                const float m[4] = {max8<0>(v), max8<8>(v), max8<16>(v), max8<24>(v)};
+                                if (fmaxf(max3(m[0], m[1], m[2]), m[3]) >= cut) {
                                     uint32_t bits = 0;
 #pragma unroll
-                                    for (int j = 0; j < 32; ++j) bits |= (v[j] >= cut ? 1u : 0u) << j;
+                                    for (int g = 0; g < 4; ++g) {
+                                        if (m[g] < cut) continue;
+#pragma unroll
+                                        for (int j = 8 * g; j < 8 * g + 8; ++j) bits |= (v[j] >= cut ? 1u : 0u) << j;
+                                    }
                                     if (a.cand_list) {   // a handful of candidates per row: a short list instead of a mask to scan
                                         while (bits) {
                                             const int j = __ffs((int)bits) - 1;
@@ -379,9 +387,22 @@ __global__ void k_fill_inf(float* p, long long n) {
 // when exactly k values lie below or after kKthRounds rounds: the filter's cut may be a little high, never low, and a
 // 2^14th of the row's range is far below the band E that is added to it.  (An exact k-th smallest took 32 rounds.)
 constexpr int kKthPerLane = 64, kKthRounds = 14;
-__global__ void __launch_bounds__(256)
-k_kth_smallest(const float* __restrict__ vals, int nq, int n, int k, float* __restrict__ out, int out_stride) {
-    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+// The values of a query lie `pitch` apart (pass 1 stores 32 queries' minima of a group side by side; one query's side by side made
+// every 4-byte store a memory sector of its own, and those, not the products, set pass 1's pace: 298 us for 20,000 x 65,536 x 96),
+// so a CTA takes eight queries, a sector, and turns them over in shared memory.
+constexpr int kKthQueries = 8;
+__global__ void __launch_bounds__(kKthQueries * 32)
+k_kth_smallest(const float* __restrict__ vals, int nq, int pitch, int n, int k, float* __restrict__ out, int out_stride) {
+    extern __shared__ __align__(16) float s_vals[];   // [kKthQueries][n]
+    const int q0 = blockIdx.x * kKthQueries, w = threadIdx.x >> 5, lane = threadIdx.x & 31, q = q0 + w;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += kKthQueries * 32) {
+        const float4* src = reinterpret_cast<const float4*>(vals + (size_t)i * pitch + q0);   // pitch is a multiple of 8
+        const float4 a = __ldg(src), b = __ldg(src + 1);
+        s_vals[i] = a.x; s_vals[n + i] = a.y; s_vals[2 * n + i] = a.z; s_vals[3 * n + i] = a.w;
+        s_vals[4 * n + i] = b.x; s_vals[5 * n + i] = b.y; s_vals[6 * n + i] = b.z; s_vals[7 * n + i] = b.w;
+    }
+    __syncthreads();
     if (q >= nq) return;
     float v[kKthPerLane];
     const float inf = __int_as_float(0x7f800000);
@@ -389,7 +410,7 @@ k_kth_smallest(const float* __restrict__ vals, int nq, int n, int k, float* __re
 #pragma unroll
     for (int j = 0; j < kKthPerLane; ++j) {
         const int i = j * 32 + lane;
-        v[j] = i < n ? vals[(size_t)q * n + i] : inf;
+        v[j] = i < n ? s_vals[w * n + i] : inf;
         mn = fminf(mn, v[j]);
         if (v[j] < inf) mx = fmaxf(mx, v[j]);
     }
@@ -416,16 +437,23 @@ k_kth_smallest(const float* __restrict__ vals, int nq, int n, int k, float* __re
     if (lane == 0) out[(size_t)q * out_stride + out_stride - 1] = c >= k ? hi : inf;
 }
 
-// k = 1: the row minimum of any number of values, one warp per row.
-__global__ void __launch_bounds__(256) k_row_min(const float* __restrict__ vals, long long nq, const int* __restrict__ nq_dev, int n, float* __restrict__ out) {
-    const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (q >= nq || (nq_dev && q >= *nq_dev)) return;
+// k = 1: the minimum of any number of values per query, `pitch` apart; a CTA takes 32 queries, each warp every eighth value of them.
+__global__ void __launch_bounds__(256) k_row_min(const float* __restrict__ vals, int nq, const int* __restrict__ nq_dev, int pitch, int n, float* __restrict__ out) {
+    __shared__ float s_min[8][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * 32 + lane;
+    if (nq_dev) nq = min(nq, *nq_dev);
+    if (blockIdx.x * 32 >= nq) return;   // uniform
     float mn = __int_as_float(0x7f800000);
-    for (int i = lane; i < n; i += 32) mn = fminf(mn, vals[(size_t)q * n + i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if (lane == 0) out[q] = mn;
+    if (q < nq) {
+#pragma unroll 4
+        for (int i = w; i < n; i += 8) mn = fminf(mn, __ldg(vals + (size_t)i * pitch + q));
+    }
+    s_min[w][lane] = mn;
+    __syncthreads();
+    if (w == 0 && q < nq) {
+        for (int i = 1; i < 8; ++i) mn = fminf(mn, s_min[i][lane]);
+        out[q] = mn;
+    }
 }
 
 // Distance of a centroid row to a query in the CPU path's arithmetic (sequential, non-fused); both rows 16-byte aligned when vec.
@@ -462,6 +490,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // x 65,536 centroids x 96, top 64).
 constexpr int kRefineThreads = 128;
 constexpr int kRefineTile = 64;
+constexpr int kRefineFew = 2 * kRefineThreads;   // with at most this many candidates their keys leave room for more rows at a time
 __host__ __device__ __forceinline__ int refine_pitch(int dim) { return (dim + 3) / 4 * 4 + 4; }   // rows spread over the banks
 __global__ void __launch_bounds__(kRefineThreads)
 k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ centroids, int dim, int nlist, int nprobe,
@@ -470,8 +499,7 @@ k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ cen
     extern __shared__ __align__(16) unsigned char s_ref[];
     const int pitch = refine_pitch(dim);
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_ref);                        // [kCandCap]; the low words hold the ids first
-    float* s_q = reinterpret_cast<float*>(s_ref + (size_t)kCandCap * 8);         // [pitch]
-    float* s_row = s_q + pitch;                                                   // [kRefineTile][pitch]
+    float* s_q = reinterpret_cast<float*>(s_ref + (size_t)kCandCap * 8) + kRefineTile * pitch;   // [pitch]
     __shared__ int s_n;
     const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) s_n = 0;
@@ -503,8 +531,11 @@ k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ cen
         return;
     }
     const bool vec = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(centroids) & 15) == 0;
-    for (int t0 = 0; t0 < n; t0 += kRefineTile) {
-        const int cnt = min(kRefineTile, n - t0);
+    // [tile][pitch]: all the candidates at once as a rule, since every tile costs a memory latency and a chain of dim additions
+    float* s_row = reinterpret_cast<float*>(s_ref + (size_t)(n <= kRefineFew ? kRefineFew : kCandCap) * 8);
+    const int tile = n <= kRefineFew ? min(kRefineThreads, kRefineTile + (kCandCap - kRefineFew) * 2 / pitch) : kRefineTile;
+    for (int t0 = 0; t0 < n; t0 += tile) {
+        const int cnt = min(tile, n - t0);
         if (vec) {
             const int n4 = dim >> 2;
             for (int i = warp; i < cnt; i += kRefineThreads / 32) {
@@ -525,7 +556,7 @@ k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ cen
         }
         __syncthreads();
     }
-    if (n <= 2 * kRefineThreads) {   // a key's place is the number of smaller ones: no barriers, a third of the sort's instructions
+    if (n <= kRefineFew) {   // a key's place is the number of smaller ones: no barriers, a third of the sort's instructions
         const uint64_t k0 = threadIdx.x < n ? s_keys[threadIdx.x] : KEY_MAX;
         const uint64_t k1 = threadIdx.x + kRefineThreads < n ? s_keys[threadIdx.x + kRefineThreads] : KEY_MAX;
         int rank0 = 0, rank1 = 0;
@@ -795,6 +826,7 @@ int coarse_tc_padded_dim(int dim) { return (dim + KATOM - 1) / KATOM * KATOM; }
 int coarse_tc_tiles(int nlist) { return (nlist + kBlockCols - 1) / kBlockCols * 2; }  // whole 512-centroid blocks
 int coarse_tc_list_cap() { return kAssignCap; }
 int coarse_tc_retry_rows() { return 65536; }
+int coarse_tc_pitch(int nq) { return (nq + 7) / 8 * 8; }
 int coarse_tc_mask_words(int nlist) { return coarse_tc_tiles(nlist) * TCOL / 32; }
 
 int coarse_tc_group(int nlist, int nprobe) {
@@ -863,6 +895,7 @@ psb_status plan_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, int nq,
     a.mwords = coarse_tc_mask_words(ix.nlist); a.status = ws.status;
     a.mask = nullptr; a.cand_cnt = nullptr; a.cand_list = nullptr; a.cand_cap = 0; a.band = 2.0f;
     a.wait_limit = ws.test_wait_limit; a.skip_loads = ws.test_skip_loads;
+    a.gmin_q = 1; a.gmin_g = coarse_tc_pitch(nq);
     a.qtiles = (nq + TQ - 1) / TQ;
     a.cblocks = a.ntiles / 2;
     pl->aug = dimp - ix.dim >= 3;
@@ -927,18 +960,22 @@ psb_status launch_coarse_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws
     TcPlan pl;
     PSB_TRY(plan_tc(ix, ws, nq, nprobe, coarse_tc_group(ix.nlist, nprobe), sm_count, &pl));
     PSB_CUDA(cudaMemsetAsync(ws.n_fail, 0, 2 * sizeof(int), s));  // n_fail, cursor
+    const int ngroups = pl.a.ngroups;
+    const bool own_kth = ngroups <= kKthPerLane * 32;
+    if (nprobe > 1 && !own_kth) { pl.a.gmin_q = ngroups; pl.a.gmin_g = 1; }   // the general row selection wants rows
     PSB_TRY(run_tc<false>(pl, ws.ev[0], ws.ev[1], s));
     // pass 2 needs only T = an upper bound of the nprobe-th smallest group minimum of each query
-    const int ngroups = pl.a.ngroups;
     if (nprobe == 1) {
-        k_row_min<<<(unsigned)(((long long)nq * 32 + 255) / 256), 256, 0, s>>>(ws.gmin, nq, nullptr, ngroups, ws.seltop);
+        k_row_min<<<(unsigned)((nq + 31) / 32), 256, 0, s>>>(ws.gmin, nq, nullptr, pl.a.gmin_g, ngroups, ws.seltop);
         count_launch();
         PSB_LAUNCH_CHECK();
         PSB_TRY(nearest_by_lists(ix, ws, pl, d_queries, nq, 2.0f, d_ids, d_dist, ws.n_fail + 3, s));
         return run_exact_queries(ix, ws, d_queries, 1, d_ids, d_dist, sm_count, s);
     }
-    if (ngroups <= kKthPerLane * 32) {
-        k_kth_smallest<<<(unsigned)(((long long)nq * 32 + 255) / 256), 256, 0, s>>>(ws.gmin, nq, ngroups, nprobe, ws.seltop, nprobe);
+    if (own_kth) {
+        const size_t ksmem = (size_t)kKthQueries * ngroups * sizeof(float);
+        PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_kth_smallest), ksmem));
+        k_kth_smallest<<<(unsigned)((nq + kKthQueries - 1) / kKthQueries), kKthQueries * 32, ksmem, s>>>(ws.gmin, nq, pl.a.gmin_g, ngroups, nprobe, ws.seltop, nprobe);
         count_launch();
         PSB_LAUNCH_CHECK();
     } else {
@@ -985,7 +1022,7 @@ psb_status launch_coarse_tc_assign(const CoarseTcIndex& ix, const CoarseTcWorksp
     PSB_TRY(plan_tc(ix, w2, cap, 1, 32, sm_count, &p2));
     p2.a.nq_dev = ws.n_fail;
     PSB_TRY(run_tc<false>(p2, nullptr, nullptr, s));
-    k_row_min<<<(unsigned)(((long long)cap * 32 + 255) / 256), 256, 0, s>>>(ws.gmin, cap, ws.n_fail, p2.a.ngroups, ws.seltop);
+    k_row_min<<<(unsigned)((cap + 31) / 32), 256, 0, s>>>(ws.gmin, cap, ws.n_fail, p2.a.gmin_g, p2.a.ngroups, ws.seltop);
     count_launch();
     PSB_LAUNCH_CHECK();
     p2.a.cand_cnt = ws.cand_cnt; p2.a.cand_list = ws.cand; p2.a.cand_cap = kAssignCap;

@@ -46,7 +46,7 @@ struct CoarseTcWorkspace {
     void* qb;        // [nq][dimp] bf16
     void* qnorm;     // [nq] float2: |q'| and |q' - bf16(q')|
     bool queries_ready = false;   // qb and qnorm hold these rows already (launch_tc_prep_queries)
-    float* gmin;     // [nq][groups]
+    float* gmin;     // [groups][coarse_tc_pitch(nq)]
     float* seltop;   // [nq][nprobe]
     int* selids;     // [nq][nprobe]
     int* cand_cnt;   // [nq]
@@ -66,7 +66,8 @@ struct CoarseTcWorkspace {
 int coarse_tc_padded_dim(int dim);
 int coarse_tc_tiles(int nlist);
 int coarse_tc_list_cap();   // candidate ids per row of the list form (nprobe 1)
-int coarse_tc_retry_rows(); // rows a bounded assignment searches again with two passes, at most
+int coarse_tc_pitch(int nq);   // queries rounded up to a memory sector
+int coarse_tc_retry_rows();   // rows a bounded assignment searches again with two passes, at most
 int coarse_tc_mask_words(int nlist);
 int coarse_tc_group(int nlist, int nprobe);
 bool coarse_tc_supported(int nq, int nlist, int dim, int nprobe);

@@ -292,7 +292,7 @@ struct TcWorkBuffers {
             PSB_TRY(qnorm.reserve(sizeof(float) * 2 * (size_t)nq, device, st));
         }
         const int retry = std::min(nq, coarse_tc_retry_rows());
-        PSB_TRY(gmin.reserve(sizeof(float) * (size_t)(bounded ? retry : nq) * groups, device, st));
+        PSB_TRY(gmin.reserve(sizeof(float) * (size_t)coarse_tc_pitch(bounded ? retry : nq) * groups, device, st));
         if (bounded) {
             PSB_TRY(fail_list2.reserve(sizeof(int) * (size_t)nq, device, st));
             PSB_TRY(retry_qb.reserve((size_t)2 * retry * dimp, device, st));
