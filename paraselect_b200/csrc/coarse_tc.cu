@@ -506,18 +506,24 @@ k_coarse_refine(const float* __restrict__ queries, const float* __restrict__ cen
     for (int d = threadIdx.x; d < dim; d += kRefineThreads) s_q[d] = queries[(size_t)q * dim + d];
     __syncthreads();
     const uint4* m4 = reinterpret_cast<const uint4*>(mask + (size_t)q * mwords);   // mwords is a multiple of 16
-#pragma unroll 4
-    for (int w = threadIdx.x; w < mwords / 4; w += kRefineThreads) {  // the candidate bits of this query -> list of centroid ids
-        const uint4 x = m4[w];
-        const unsigned long long bw[2] = {((unsigned long long)x.y << 32) | x.x, ((unsigned long long)x.w << 32) | x.z};
+    // the candidate bits of this query -> list of centroid ids; four loads in flight per thread
+    for (int w0 = threadIdx.x; w0 < mwords / 4; w0 += 4 * kRefineThreads) {
+        uint4 x[4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            unsigned long long bits = bw[i];
-            while (bits) {
-                const int j = __ffsll((long long)bits) - 1;
-                bits &= bits - 1;
-                const int pos = atomicAdd(&s_n, 1);
-                if (pos < kCandCap) s_keys[pos] = (uint64_t)(w * 128 + i * 64 + j);
+        for (int i = 0; i < 4; ++i) x[i] = w0 + i * kRefineThreads < mwords / 4 ? __ldg(m4 + w0 + i * kRefineThreads) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t words[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+            if ((words[0] | words[1] | words[2] | words[3]) == 0u) continue;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                uint32_t bits = words[h];
+                while (bits) {
+                    const int j = __ffs((int)bits) - 1;
+                    bits &= bits - 1;
+                    const int pos = atomicAdd(&s_n, 1);
+                    if (pos < kCandCap) s_keys[pos] = (uint64_t)((w0 + i * kRefineThreads) * 128 + h * 32 + j);
+                }
             }
         }
     }
