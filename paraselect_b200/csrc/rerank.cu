@@ -6,7 +6,7 @@
 //   k_claim_rows      the first candidate to name a row claims it and gives it the next slot of the staging buffer
 //   k_gather_unique   copies the claimed rows - host memory mapped into the device address space, read over PCIe - to their
 //                     slots; a warp keeps eight rows in flight.  Host threads fill a range of the slots instead or besides.
-//   k_rerank_score    half-warps score rows - from the slots or from where they lie - in the accumulation order of the CPU kernel
+//   k_rerank_score*   eight lanes (half-warps, for rows that are not whole 16-byte units) score rows - from the slots or from where they lie - in the accumulation order of the CPU kernel
 //                     the reference uses (four 16-lane FMA accumulators, pairwise combine, halving tree:
 //                     src/cpu/distance/fp32_l2_avx512.h:16-53); rows not held here score +inf
 //   k_topk_select     one CTA per query: the topk smallest (distance,row), duplicate rows once (reference semantics:
@@ -261,6 +261,81 @@ k_rerank_score(const unsigned char* __restrict__ src, const int* __restrict__ sl
     }
 }
 
+// The same scores for rows of whole 16-byte units.  Eight lanes a row: lane l stands for lanes 4 (l % 4) .. + 3 of the CPU kernel's 16 and
+// for its accumulators l / 4 and l / 4 + 2, so the row comes in as 128-byte lines straight into registers, the additions are
+// the CPU kernel's own, and a row takes 73 warp instructions where a half-warp and a trip through shared memory took 160, which is
+// what bound it: 2,000 queries x 500 rows of 384 bytes 165 -> 122 us.
+// Two rows per lane group at a time cost the occupancy more than they brought (72 registers: 136 us).
+template <bool U8>
+__global__ void __launch_bounds__(kScoreThreads, 6)
+k_rerank_score_wide(const unsigned char* __restrict__ src, const int* __restrict__ slot_of, RowMap mp, int dim,
+                    const unsigned char* __restrict__ queries, const int* __restrict__ cand, int candidate_count,
+                    int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist) {
+    extern __shared__ __align__(16) unsigned char s_score[];
+    const int q = blockIdx.x, lane = threadIdx.x & 31, l = lane & 7;
+    const int units = (U8 ? dim : dim * 4) >> 4;
+    const int i = (blockIdx.y * (kScoreThreads / 32) + (threadIdx.x >> 5)) * 4 + (lane >> 3);
+    long long at = i < cand_count(counts, q, candidate_count) ? local_row(mp, cand[(size_t)q * candidate_stride + i]) : -1;
+    if (at >= 0 && slot_of) at = slot_of[at];
+    const uint4* own = reinterpret_cast<const uint4*>(queries) + (size_t)q * units;
+    const uint4* row = at >= 0 ? reinterpret_cast<const uint4*>(src) + (size_t)at * units : own;   // no row: any will do
+    uint4* query = reinterpret_cast<uint4*>(s_score);
+    for (int u = threadIdx.x; u < units; u += kScoreThreads) query[u] = own[u];
+    __syncthreads();
+    float result;
+    if constexpr (U8) {
+        unsigned acc = 0;
+#pragma unroll 4
+        for (int u = l; u < units; u += 8) {
+            const uint4 v = __ldg(row + u), y = query[u];
+            unsigned d = __vabsdiffu4(v.x, y.x); acc = __dp4a(d, d, acc);
+            d = __vabsdiffu4(v.y, y.y); acc = __dp4a(d, d, acc);
+            d = __vabsdiffu4(v.z, y.z); acc = __dp4a(d, d, acc);
+            d = __vabsdiffu4(v.w, y.w); acc = __dp4a(d, d, acc);
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        result = (float)(int)acc;
+    } else {
+        float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};   // accumulators l / 4 and l / 4 + 2
+        auto fold = [](float (&acc)[4], const uint4& x, const uint4& y) {   // y: the query
+            float d = __fsub_rn(__uint_as_float(y.x), __uint_as_float(x.x)); acc[0] = __fmaf_rn(d, d, acc[0]);
+            d = __fsub_rn(__uint_as_float(y.y), __uint_as_float(x.y)); acc[1] = __fmaf_rn(d, d, acc[1]);
+            d = __fsub_rn(__uint_as_float(y.z), __uint_as_float(x.z)); acc[2] = __fmaf_rn(d, d, acc[2]);
+            d = __fsub_rn(__uint_as_float(y.w), __uint_as_float(x.w)); acc[3] = __fmaf_rn(d, d, acc[3]);
+        };
+        const int full = units & ~15;   // 16-byte units in whole blocks of 64 elements
+#pragma unroll 2
+        for (int u = l; u < full; u += 16) {
+            const uint4 v0 = __ldg(row + u), v1 = __ldg(row + u + 8);
+            fold(a0, v0, query[u]);
+            fold(a1, v1, query[u + 8]);
+        }
+        if (l < 4) {   // what is left goes to accumulator 0, 16 elements at a time
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                if (full + 4 * c + 4 <= units) fold(a0, __ldg(row + full + 4 * c + l), query[full + 4 * c + l]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)   // (a0 + a1) + (a2 + a3)
+            a0[e] = __fadd_rn(__fadd_rn(a0[e], __shfl_xor_sync(0xffffffffu, a0[e], 4)), __fadd_rn(a1[e], __shfl_xor_sync(0xffffffffu, a1[e], 4)));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a0[e] = __fadd_rn(a0[e], __shfl_xor_sync(0xffffffffu, a0[e], 2));   // halving tree: 8 apart,
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a0[e] = __fadd_rn(a0[e], __shfl_xor_sync(0xffffffffu, a0[e], 1));   // 4,
+        result = __fadd_rn(__fadd_rn(a0[0], a0[2]), __fadd_rn(a0[1], a0[3]));                           // 2 and 1
+        if (l == 0) {
+#pragma unroll 1
+            for (int d = dim & ~15; d < dim; ++d) {
+                const float diff = __fsub_rn(reinterpret_cast<const float*>(s_score)[d], __ldg(reinterpret_cast<const float*>(row) + d));
+                result = __fmaf_rn(diff, diff, result);
+            }
+        }
+    }
+    if (l == 0 && i < candidate_count) out_dist[(size_t)q * candidate_count + i] = at >= 0 ? result : __int_as_float(0x7f800000);
+}
+
 constexpr int kSelectThreads = 256;
 // dist [nq][candidate_count] (dense), cand [nq][candidate_stride] global rows.  ids: original ids by row (out_ids is written
 // instead of out_rows).  The smallest come from select.cuh; when a row turns up twice among them - the ADC stage names a row once, a
@@ -418,7 +493,18 @@ psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const Ro
                                const int* d_candidates, int nq, int candidate_count, int candidate_stride,
                                const int* d_counts, float* d_out_dist, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
+    const int row_bytes = dim * elem_bytes;
     const dim3 grid(nq, (candidate_count + kScoreBlock - 1) / kScoreBlock);
+    if (((reinterpret_cast<uintptr_t>(d_src) | reinterpret_cast<uintptr_t>(d_queries) | row_bytes) & 15) == 0 && row_bytes <= 48 * 1024) {
+        auto kernel = elem_bytes == 4 ? k_rerank_score_wide<false> : k_rerank_score_wide<true>;
+        PSB_TRY(prefer_max_shared(kernel));
+        kernel<<<grid, kScoreThreads, row_bytes, s>>>(
+            static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, static_cast<const unsigned char*>(d_queries), d_candidates, candidate_count,
+            candidate_stride, d_counts, d_out_dist);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        return PSB_OK;
+    }
     const size_t pitch = (size_t)score_pitch(dim * elem_bytes);
     size_t smem = pitch * (1 + kScoreBlock);
     const int through = smem <= (size_t)200 * 1024 ? 1 : 0;

@@ -51,3 +51,23 @@ def test_overlapped_batches_share_rows(psb, mode):
             got = s.search(q, 3, 10, batch_size=2500)
             assert np.array_equal(got["indices"], ref["indices"]) and np.array_equal(got["distances"], ref["distances"])
     assert np.array_equal(ref["indices"][:200], want["indices"]) and np.array_equal(ref["distances"][:200], want["distances"])
+
+
+@pytest.mark.parametrize("dim,u8", [(16, False), (4, False), (20, False), (60, False), (64, False), (68, False), (112, False), (124, False), (128, False),
+                                    (200, False), (960, False), (16, True), (128, True), (144, True), (272, True)])
+@pytest.mark.parametrize("nq,width", [(2, 33), (90, 700)])
+def test_rows_of_whole_units(psb, dim, u8, nq, width):
+    import torch
+    ix = index(900, dim, u8, dim)
+    rng = np.random.default_rng(dim)
+    with psb.Session(ix, n_rerank=width, exact_mode=3, max_batch=nq) as s:
+        q = rng.integers(0, 256, (nq, dim)).astype(np.uint8) if u8 else rng.standard_normal((nq, dim)).astype(np.float32)
+        cand = np.stack([rng.permutation(900)[:width] for _ in range(nq)]).astype(np.int32)
+        cand[:, 5] = -1
+        cnt = rng.integers(0, width + 1, nq).astype(np.int32)
+        rows = torch.empty((nq, 10), dtype=torch.int32, device="cuda"); dist = torch.empty((nq, 10), device="cuda")
+        s.stage_rerank(torch.from_numpy(q).cuda(), nq, torch.from_numpy(cand).cuda(), width, width, torch.from_numpy(cnt).cuda(), 10, rows, dist)
+        s.sync()
+        masked = np.where(np.arange(width)[None, :] < cnt[:, None], cand, -1)
+        wi, wd = oracle.rerank(ix["vectors"], q, masked, 10)
+        assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
