@@ -391,6 +391,7 @@ struct psb_session {
     bool slots_dirty = true;             // slot_of is not all -1 (never used, or a batch was left half done)
     int* h_unique = nullptr;             // pinned: the slots the host threads fill
     size_t h_unique_count = 0;
+    size_t slots = 0;                    // of the batch at work, at most
     int* h_marks = nullptr;              // pinned [2 * kMaxParts]
     cudaStream_t list_stream = nullptr;  // brings the slot lists to the host thread beside the row copies
     std::vector<long long> h_global_begin;  // striped shards: host copy of the slices' first rows
@@ -768,8 +769,10 @@ constexpr long long kClaimRequests = 65536;   // candidates from which a batch's
 psb_status staged_gather_host(psb_session* s, const int* h_rows, size_t count, void* d_stage, cudaStream_t stream) {
     if (count == 0) return PSB_OK;
     const size_t row_bytes = (size_t)s->dim * s->exact_elem;
+    // Sized for the batch, not for the part: growing the buffers from part to part waits for the device every time.  (Buffers of 16 MB, so
+    // that a part's first copy starts sooner, cost more in handing out the work: 4,096 queries x 1,000 rows 18.9 -> 25.0 ms.)
     const size_t chunk = std::max<size_t>(1, ((size_t)64 << 20) / std::max<size_t>(1, row_bytes));
-    const size_t need = std::min(chunk, std::max<size_t>(count, 4096)) * row_bytes;
+    const size_t need = std::min(chunk, std::max<size_t>(std::max(count, s->slots), 4096)) * row_bytes;
     if (s->pinned_bytes < need) {
         for (int i = 0; i < 2; ++i) {
             if (s->pinned_used[i]) PSB_CUDA(cudaEventSynchronize(s->pinned_ev[i]));  // no copy may still read the old buffer
@@ -823,6 +826,7 @@ psb_status staged_gather_host(psb_session* s, const int* h_rows, size_t count, v
 // fetches and scores are ordered by the caller's streams and events.
 psb_status rows_begin(psb_session* s, long long requests, cudaStream_t st) {
     const size_t slots = (size_t)std::max<long long>(1, std::min(requests, s->exact_count));
+    s->slots = slots;
     PSB_TRY(s->unique.reserve(sizeof(int) * slots));
     PSB_TRY(s->marks.reserve(sizeof(int) * (kMaxParts + 2)));
     PSB_TRY(s->stage.reserve(slots * s->dim * s->exact_elem));
@@ -856,15 +860,21 @@ psb_status rows_from_host(psb_session* s, int part, int host_pct, cudaStream_t s
     const int b = s->h_marks[2 * part], e = host_share_end(b, s->h_marks[2 * part + 1], host_pct);
     if (e <= b) return PSB_OK;
     if (!s->list_stream) PSB_CUDA(cudaStreamCreateWithFlags(&s->list_stream, cudaStreamNonBlocking));
-    if (s->h_unique_count < (size_t)(e - b)) {
+    constexpr size_t kListChunk = (size_t)1 << 18;   // ids on the host at a time
+    const size_t room = std::min(kListChunk, std::max(s->slots, (size_t)(e - b)));
+    if (s->h_unique_count < room) {
         if (s->h_unique) cudaFreeHost(s->h_unique);
         s->h_unique = nullptr; s->h_unique_count = 0;
-        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_unique), sizeof(int) * (size_t)(e - b), cudaHostAllocDefault));
-        s->h_unique_count = (size_t)(e - b);
+        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_unique), sizeof(int) * room, cudaHostAllocDefault));
+        s->h_unique_count = room;
     }
-    PSB_CUDA(cudaMemcpyAsync(s->h_unique, s->unique.as<int>() + b, sizeof(int) * (size_t)(e - b), cudaMemcpyDeviceToHost, s->list_stream));
-    PSB_CUDA(cudaStreamSynchronize(s->list_stream));
-    return staged_gather_host(s, s->h_unique, (size_t)(e - b), static_cast<unsigned char*>(s->stage.p) + (size_t)b * s->dim * s->exact_elem, st);
+    for (size_t i = b; i < (size_t)e; i += s->h_unique_count) {
+        const size_t count = std::min(s->h_unique_count, (size_t)e - i);
+        PSB_CUDA(cudaMemcpyAsync(s->h_unique, s->unique.as<int>() + i, sizeof(int) * count, cudaMemcpyDeviceToHost, s->list_stream));
+        PSB_CUDA(cudaStreamSynchronize(s->list_stream));
+        PSB_TRY(staged_gather_host(s, s->h_unique, count, static_cast<unsigned char*>(s->stage.p) + i * s->dim * s->exact_elem, st));
+    }
+    return PSB_OK;
 }
 
 // The stream of the hybrid transport's gather kernel.  Highest priority: its few CTAs each need an SM to themselves and must be
