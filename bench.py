@@ -892,7 +892,7 @@ def flat_search(args, cfg, torch, api, device):
               e2e=dict(value=round(nq / (ms_e2e * 1e-3), 1), unit="queries/s", ms_per_step=round(ms_e2e, 4),
                        h2d_bytes_per_step=int(stats["h2d_bytes"]), d2h_bytes_per_step=int(stats["d2h_bytes"])),
               gpu_launches=int(c["kernel_launches"]),
-              roofline=dict(bound="hbm", kernel="k_flat_scan_direct", achieved=round(achieved, 1), peak=peak, unit="GB/s",
+              roofline=dict(bound="hbm", kernel="k_flat_tiles", achieved=round(achieved, 1), peak=peak, unit="GB/s",
                             frac=round(achieved / peak, 4), peak_source="measured" if peaks else "fallback",
                             algorithmic_bytes_per_launch=int(rows_per_launch * dim * 4), rows_per_launch=int(rows_per_launch),
                             ms_per_launch=round(scan_ms, 4), traffic=None,
@@ -1188,7 +1188,7 @@ def sign_codec(args, cfg, torch, api, device):
               e2e=dict(value=round(nq / (ms_e2e * 1e-3), 1), unit="queries/s", ms_per_step=round(ms_e2e, 3),
                        h2d_bytes_per_step=nq * dim * 4 + nq * nprobe * 4, d2h_bytes_per_step=nq * k * 4),
               gpu_launches=2 * args.steps,
-              roofline=dict(bound="hbm", kernel="k_sign_scan<4,0>", achieved=round(achieved, 1), peak=peak, unit="GB/s",
+              roofline=dict(bound="hbm", kernel="k_sign_scan_float<4>", achieved=round(achieved, 1), peak=peak, unit="GB/s",
                             frac=round(achieved / peak, 4), peak_source="measured" if peaks else "fallback",
                             ms_per_launch=round(scan_ms, 3), algorithmic_bytes_per_launch=bytes_per_launch,
                             bytes_per_row_visit=words * 4 + 4, row_visits_per_s=round(visits / (scan_ms * 1e-3), 1), traffic=None,

@@ -118,7 +118,7 @@ enum {
                                   there (refused with PSB_OUT_OF_MEMORY when they do not fit); no counterpart in the reference,
                                   whose rerank rows stay on the host */
     PSB_EXACT_HOST_HYBRID = 4  /* both host transports at once: the rows are registered and mapped as in HOST_MAPPED, and of every
-                                  sub-batch psb_options.zero_copy_pct percent of the queries have their rows gathered by a kernel
+                                  sub-batch psb_options.zero_copy_pct percent of the rows fetched are gathered by a kernel
                                   over PCIe - on reserve_sms SMs of its own (default 32), which the scan's grid leaves free -
                                   while host threads stage the others through the pinned rings; neither the host cores nor
                                   the kernel's reads fill the link alone */
