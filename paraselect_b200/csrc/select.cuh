@@ -14,14 +14,51 @@ inline size_t shared_bytes(int k) { return (size_t)buffer_entries(k) * 8 + (size
 
 struct Words { unsigned int hist[256]; uint64_t prefix; unsigned int rank; int done, cnt; float cut; };
 
+// The rank-th smallest of the words get(i, word) gives for i = 0..n-1 (false: none), most significant byte first; returns its rank
+// among those equal to it.  At least `rank` words.  All threads of the block.
+template <int kThreads, typename Get>
+__device__ unsigned smallest_word(int n, unsigned rank, Get get, uint32_t* out, Words* w) {
+    uint32_t prefix = 0, mask = 0;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+        if (threadIdx.x < 256) w->hist[threadIdx.x] = 0;
+        __syncthreads();
+#pragma unroll 4
+        for (int i = threadIdx.x; i < n; i += kThreads) {
+            uint32_t word = 0;
+            if (get(i, word) && (word & mask) == prefix) atomicAdd(&w->hist[(word >> shift) & 255u], 1u);
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {   // eight bins a lane
+            unsigned mine = 0;
+            for (int j = 0; j < 8; ++j) mine += w->hist[threadIdx.x * 8 + j];
+            unsigned upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const unsigned v = __shfl_up_sync(0xffffffffu, upto, o); if ((int)threadIdx.x >= o) upto += v; }
+            unsigned before = upto - mine;
+            if (before < rank && rank <= upto) {
+                int j = 0;
+                while (before + w->hist[threadIdx.x * 8 + j] < rank) before += w->hist[threadIdx.x * 8 + j++];
+                w->prefix = prefix | (uint32_t)(threadIdx.x * 8 + j) << shift;
+                w->rank = rank - before;
+            }
+        }
+        __syncthreads();
+        prefix = (uint32_t)w->prefix;
+        rank = w->rank;
+        mask |= 255u << shift;
+        __syncthreads();
+    }
+    *out = prefix;
+    return rank;
+}
+
 // Leaves the min(k, n) smallest keys (vals[i], payload(i)) of i = 0..n-1 at the front of s_keys, ascending, and returns their number.  s_keys [buffer], s_min [kMaxGroups], one Words in shared memory; k <= buffer.
 //
 // Reads the values twice.  First every thread takes the minima of a few of its strided subsets; the k-th smallest of all these
 // minima - there are at least 2 k of them - bounds the k-th smallest value from above, and not much more than k values lie below
 // it.  One warp finds it by bisection (14 rounds or until exactly k lie below; a little high does no harm).  Then the values up to
-// that cut are gathered and put in order by rank or, above 256, by a bitonic sort.  A radix selection over the whole keys
-// (up to eight passes with a histogram each, 12 us for 1,024 values and one row) is left for the rows the cut does not serve: too
-// many equal values, fewer than k comparable ones, or k above what the group minima cover.
+// that cut are gathered and put in order by rank or, above 256, by a bitonic sort.  A radix selection is left for
+// the rows the cut does not serve: too many equal values, fewer than k comparable ones, or k above what the group minima cover.
 template <int kThreads, typename Payload>   // kThreads: the block's threads, 256 or more
 __device__ int smallest(const float* __restrict__ vals, int n, int k, Payload payload, uint64_t* s_keys, int buffer, float* s_min, Words* w) {
     const int tid = threadIdx.x, lane = tid & 31;
@@ -81,46 +118,50 @@ __device__ int smallest(const float* __restrict__ vals, int n, int k, Payload pa
     __syncthreads();
     int c = w->cnt;
     __syncthreads();
-    if (c < keep || c > buffer) {   // radix selection over the whole keys, most significant byte first
-        if (tid == 0) { w->prefix = 0; w->rank = (unsigned)keep; w->done = keep == n ? 1 : 0; w->cnt = 0; }
-        uint64_t mask = 0;
+    if (c < keep || c > buffer) {
+        // The keep-th smallest value by radix over the values up to the cut, then all below it and of the equal ones those with the
+        // smallest payloads.  Rows of one code have one distance, so this happens; payloads, a search each, are asked of the chosen only
+        // (whole keys, eight passes with a payload per value: 980 us for one row of 62,500 in a batch that takes 110).
+        const bool all = c < keep;
+        auto taken = [&](float v) { return all || cut == inf || v <= cut; };
+        if (tid == 0) { w->cnt = 0; w->done = 0; }
         __syncthreads();
-        for (int pass = 7; pass >= 0; --pass) {
-            const int shift = pass * 8;
-            if (tid < 256) w->hist[tid] = 0;
-            __syncthreads();
-            if (w->done) break;
-            const uint64_t prefix = w->prefix;
+        if (keep == n) {
+            for (int i = tid; i < n; i += kThreads) s_keys[i] = make_key(vals[i], payload(i));
+            c = n;
+        } else {
+            uint32_t value = 0;
+            const unsigned rank = smallest_word<kThreads>(n, (unsigned)keep, [&](int i, uint32_t& word) {
+                const float v = vals[i];
+                word = (uint32_t)(make_key(v, 0u) >> 32);
+                return taken(v);
+            }, &value, w);
+#pragma unroll 4
             for (int i = tid; i < n; i += kThreads) {
-                const uint64_t key = make_key(vals[i], payload(i));
-                if ((key & mask) == prefix) atomicAdd(&w->hist[(key >> shift) & 255], 1u);
+                const float v = vals[i];
+                const uint32_t word = (uint32_t)(make_key(v, 0u) >> 32);
+                if (word < value) { const int pos = atomicAdd(&w->cnt, 1); if (pos < buffer) s_keys[pos] = make_key(v, payload(i)); }
+                else if (word == value) atomicAdd(&w->done, 1);
             }
             __syncthreads();
-            if (tid == 0) {
-                unsigned cum = 0;
-                const unsigned rank = w->rank;
-                for (int b = 0; b < 256; ++b) {
-                    const unsigned h = w->hist[b];
-                    if (cum + h >= rank) {
-                        w->prefix = prefix | ((uint64_t)b << shift);
-                        w->rank = rank - cum;
-                        if (h == rank - cum) w->done = 1;  // the whole bucket is selected
-                        break;
-                    }
-                    cum += h;
-                }
-            }
-            mask |= 255ull << shift;
+            uint32_t last = 0xffffffffu;   // the largest payload wanted of the equal ones
+            if (w->cnt + w->done > buffer)
+                smallest_word<kThreads>(n, rank, [&](int i, uint32_t& word) {
+                    if ((uint32_t)(make_key(vals[i], 0u) >> 32) != value) return false;
+                    word = (uint32_t)payload(i);
+                    return true;
+                }, &last, w);
             __syncthreads();
+#pragma unroll 4
+            for (int i = tid; i < n; i += kThreads) {
+                const float v = vals[i];
+                if ((uint32_t)(make_key(v, 0u) >> 32) != value) continue;
+                const uint32_t x = (uint32_t)payload(i);
+                if (x <= last) { const int pos = atomicAdd(&w->cnt, 1); if (pos < buffer) s_keys[pos] = make_key(v, x); }
+            }
+            __syncthreads();
+            c = w->cnt < buffer ? w->cnt : buffer;
         }
-        __syncthreads();
-        const uint64_t most = keep == n ? KEY_MAX : (w->prefix | ~mask);   // keys <= most are exactly the smallest
-        for (int i = tid; i < n; i += kThreads) {
-            const uint64_t key = make_key(vals[i], payload(i));
-            if (key <= most) { const int pos = atomicAdd(&w->cnt, 1); if (pos < buffer) s_keys[pos] = key; }
-        }
-        __syncthreads();
-        c = w->cnt;
         __syncthreads();
     }
     if (c <= kThreads) {   // a key's place is the number of smaller ones

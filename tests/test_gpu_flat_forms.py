@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n,dim,nlist,nq,nprobe,topk,values", [
     (3000, 33, 5, 97, 5, 10, "normal"), (3000, 100, 5, 1, 3, 7, "normal"), (4000, 64, 3, 33, 2, 300, "normal"), (9000, 16, 7, 2, 7, 300, "normal"),
     (6000, 8, 4, 40, 4, 1100, "normal"), (6000, 8, 4, 3, 4, 2048, "normal"), (7000, 12, 3, 40, 3, 50, "grid"), (5000, 4, 2, 2, 2, 20, "equal"),
-    (64, 300, 2, 20, 2, 5, "normal"), (40, 7, 20, 33, 20, 64, "normal")])
+    (64, 300, 2, 20, 2, 5, "normal"), (40, 7, 20, 33, 20, 64, "normal"), (30000, 2, 4, 200, 4, 300, "grid"), (30000, 1, 4, 3, 4, 900, "grid")])
 def test_flat_forms(psb, n, dim, nlist, nq, nprobe, topk, values):
     rng = np.random.default_rng(n + dim + nq)
     draw = {"normal": lambda *s: rng.standard_normal(s), "grid": lambda *s: rng.integers(-1, 2, s), "equal": lambda *s: np.ones(s)}[values]
