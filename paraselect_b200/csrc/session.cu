@@ -566,9 +566,13 @@ double expected_rows(const psb_session* s, int nprobe) {
     return std::min((double)s->longest[(size_t)std::min(nprobe, s->nlist)], s->own_list_rows + (nprobe - 1) * (double)s->shard_rows / std::max(1, s->nlist));
 }
 
-// Whether the ADC scan of nq queries takes its row form (adc_rows.cu): when its work - m shared-memory gathers per visited row, 50 G
-// row visits/s at m = 48 - takes less than the list-centric scan's chain of kernels, which costs about 180 us before its first row and
-// runs at 66 G visits/s with the tensor-core filter.  Shapes the filter does not take stay with the row form at any size.
+// Whether the ADC scan of nq queries takes its row form (adc_rows.cu).  It starts some 130 us (residual 170) before the list-centric
+// scan, a chain of a dozen kernels more, has seen its first row; but its cost per query grows with the visited rows, 4 ns a thousand more
+// than the tensor-core filter's and 0.32 ns per sub-space's look-up, and in residual mode with a table per probe, while the
+// list-centric scan takes 0.1 us (residual 0.35) a query whatever it visits.  Fitted to both forms at 128 to 4,096 queries over 0.3 to
+// 2 million rows, m = 8 to 48, 16 to 64 probes: the line lies where they meet to within 10 % of the time - at 240 queries for 31,000
+// rows of m = 48 each, 1,200 for m = 8; lists so short that a query's rows cost less than its fixed share stay with the row form.
+// So do shapes the filter does not take, at any size.
 // any_probes: the caller's own probes, which may name a list more than once.
 long long row_stride(const psb_session* s, int nprobe, bool any_probes) {
     return std::max<long long>(1, any_probes ? s->longest[1] * nprobe : s->longest[(size_t)nprobe]);
@@ -578,7 +582,9 @@ bool rows_form(const psb_session* s, int nq, int nprobe, bool any_probes = false
     const long long stride = row_stride(s, nprobe, any_probes);
     const size_t smem = ((size_t)s->m * s->k + s->dim + nprobe + 1) * 4;
     if (stride > kRowDistFloats || smem > (size_t)220 * 1024) return false;
-    return s->row_aug.p == nullptr || (double)nq * expected_rows(s, nprobe) * s->m <= 4.8e8;
+    const bool residual = s->opt.adc_mode == 1;
+    const double per_query = expected_rows(s, nprobe) * (4e-6 + 3.2e-7 * s->m) + (residual ? nprobe * (0.008 + 2.3e-4 * s->m) - 0.35 : -0.1);   // us
+    return s->row_aug.p == nullptr || nq * per_query <= (residual ? 170.0 : 130.0);
 }
 
 // Queries per sub-batch of the pipeline: a quarter of the batch when the rerank overlaps the scan, and in residual mode
