@@ -683,8 +683,10 @@ class SignIndex:
 
     # Host arrays of a search go through page-locked memory that torch keeps and reuses, so that the copies neither stage nor wait and
     # the results land in pages that exist already: a fresh 8 MB result took longer to fault in than to copy.  Larger ones go
-    # through pageable memory, so that no caller's results hold much page-locked memory.
+    # through pageable memory, so that no caller's results hold much page-locked memory, and so do results below a megabyte, which a
+    # caller that keeps them would make torch page-lock anew on every call for the few microseconds the copy takes.
     PINNED_LIMIT_BYTES = 32 << 20
+    PINNED_RESULT_BYTES = 1 << 20
 
     def _upload(self, array):
         t = self._t
@@ -695,7 +697,7 @@ class SignIndex:
 
     def _download(self, tensor):
         t = self._t
-        if tensor.numel() * tensor.element_size() > self.PINNED_LIMIT_BYTES:
+        if not self.PINNED_RESULT_BYTES <= tensor.numel() * tensor.element_size() <= self.PINNED_LIMIT_BYTES:
             return tensor.cpu()
         return t.empty(tensor.shape, dtype=tensor.dtype, pin_memory=True).copy_(tensor, non_blocking=True)
 

@@ -106,10 +106,12 @@ psb_status launch_sign_encode_queries(const float* d_queries, const float* d_cen
                                       int nlist, int dim, int padded_dim, uint32_t seed, float* d_states, float* d_norm_sq,
                                       uint32_t* d_state_codes, float* d_norms, int sm_count, cudaStream_t s);
 // mode 0: float states + norm_sq against reconstruction scales; mode 1: sign-coded states + norms against row norms.
+// d_partial: sign_partial_bytes of device memory (none when that is 0).
+size_t sign_partial_bytes(int nq, int nprobe, int candidate_count, int sm_count);
 psb_status launch_sign_candidates(int mode, const float* d_states, const float* d_norm_sq, const uint32_t* d_state_codes,
                                   const float* d_norms, const uint32_t* d_codes, const float* d_row_params,
                                   const long long* d_offsets, int nlist, const int* d_probes, int nq, int nprobe, int padded_dim,
-                                  int candidate_count, int* d_rows_out, float* d_dist_out, int sm_count, cudaStream_t s);
+                                  int candidate_count, int* d_rows_out, float* d_dist_out, void* d_partial, int sm_count, cudaStream_t s);
 
 // ---- PQ lookup tables --------------------------------------------------------------------------------
 psb_status launch_build_lut(const float* d_queries, int nq, int dim, const float* d_codebook, int m, int k,

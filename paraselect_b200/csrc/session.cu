@@ -1251,9 +1251,12 @@ psb_status psb_sign_search_candidates(int mode, const float* d_states, const flo
         return fail(PSB_INVALID_ARGUMENT, "invalid sign candidate search request");
     int sms = 0;
     PSB_TRY(check_device(device, &sms));
+    PoolBuf partial;   // the slices of queries whose probes go to several CTAs
+    const size_t bytes = sign_partial_bytes(nq, nprobe, candidate_count, sms);
+    if (bytes) PSB_TRY(partial.reserve(bytes, device, static_cast<cudaStream_t>(stream)));
     return launch_sign_candidates(mode, d_states, d_norm_sq, d_state_codes, d_norms, d_codes, d_row_params,
                                   reinterpret_cast<const long long*>(d_list_offsets), nlist, d_probes, nq, nprobe, padded_dim,
-                                  candidate_count, d_rows_out, d_dist_out, sms, static_cast<cudaStream_t>(stream));
+                                  candidate_count, d_rows_out, d_dist_out, partial.p, sms, static_cast<cudaStream_t>(stream));
 }
 
 psb_status psb_stage_rotate_queries(psb_session* s, const float* d_queries, int nq, float* d_rotated) {

@@ -1046,10 +1046,23 @@ psb_status launch_sign_encode_queries(const float* d_queries, const float* d_cen
     return dispatch_encode(a, padded_dim, sm_count, s);
 }
 
+// Few queries: the probes of one query go to several CTAs so that the grid covers the SMs twice over.
+static int sign_split(int nq, int nprobe, int candidate_count, int sm_count) {
+    int split = 1;
+    if (nq < 2 * sm_count) split = std::min(nprobe, (2 * sm_count + nq - 1) / nq);
+    return std::max(1, std::min(split, kMergeMaxKeys / pow2_at_least(candidate_count)));
+}
+
+size_t sign_partial_bytes(int nq, int nprobe, int candidate_count, int sm_count) {
+    if (nq <= 0 || nprobe <= 0 || candidate_count <= 0 || candidate_count > kSignMaxCandidates) return 0;
+    const int split = sign_split(nq, nprobe, candidate_count, sm_count);
+    return split > 1 ? sizeof(uint64_t) * (size_t)nq * split * candidate_count : 0;
+}
+
 psb_status launch_sign_candidates(int mode, const float* d_states, const float* d_norm_sq, const uint32_t* d_state_codes,
                                   const float* d_norms, const uint32_t* d_codes, const float* d_row_params,
                                   const long long* d_offsets, int nlist, const int* d_probes, int nq, int nprobe, int padded_dim,
-                                  int candidate_count, int* d_rows_out, float* d_dist_out, int sm_count, cudaStream_t s) {
+                                  int candidate_count, int* d_rows_out, float* d_dist_out, void* d_partial, int sm_count, cudaStream_t s) {
     if (!sign_shape_ok(padded_dim, padded_dim)) return fail(PSB_INVALID_ARGUMENT, "sign codec: padded_dim must be 32, 64, 128 or 256");
     if (nprobe > 65535) return fail(PSB_INVALID_ARGUMENT, "sign codec: at most 65,535 probes per query");
     if (candidate_count <= 0 || candidate_count > kSignMaxCandidates)
@@ -1063,17 +1076,11 @@ psb_status launch_sign_candidates(int mode, const float* d_states, const float* 
     const int kp2 = pow2_at_least(candidate_count);
     a.kp2 = kp2;
     a.cap = std::max(2 * kp2, 2 * kScanStep);   // a whole step always fits after a cut back to candidate_count
-    // Few queries: the probes of one query go to several CTAs so that the grid covers the SMs twice over.
-    int split = 1;
-    if (nq < 2 * sm_count) split = std::min(nprobe, (2 * sm_count + nq - 1) / nq);
-    split = std::max(1, std::min(split, kMergeMaxKeys / kp2));
+    const int split = sign_split(nq, nprobe, candidate_count, sm_count);
     a.split = split;
     a.rows_out = d_rows_out; a.dist_out = d_dist_out;
-    uint64_t* partial = nullptr;
-    if (split > 1) {
-        PSB_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&partial), sizeof(uint64_t) * (size_t)nq * split * candidate_count, s));
-        a.partial = partial;
-    }
+    uint64_t* partial = static_cast<uint64_t*>(d_partial);
+    a.partial = split > 1 ? partial : nullptr;
     psb_status rc = dispatch_scan(mode, a, s);
     if (rc == PSB_OK && split > 1) {
         const int mcap = pow2_at_least(split * candidate_count);
@@ -1086,10 +1093,6 @@ psb_status launch_sign_candidates(int mode, const float* d_states, const float* 
             count_launch();
         }
         if (e != cudaSuccess) rc = cuda_fail(e, "k_sign_merge", __FILE__, __LINE__);
-    }
-    if (partial) {
-        const cudaError_t e = cudaFreeAsync(partial, s);
-        if (rc == PSB_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaFreeAsync", __FILE__, __LINE__);
     }
     return rc;
 }
