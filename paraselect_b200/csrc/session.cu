@@ -1,5 +1,6 @@
 // Host side of the C ABI: sessions (device copies of the index, workspaces, the batch pipeline), the
 // stage-level and one-shot operator entry points, training drivers and the synthetic-data entry points.
+#include "batch_parts.h"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -386,13 +387,15 @@ struct psb_session {
     double staged_gather_s = 0.0;          // host time spent gathering rows, and the bytes gathered (reported by the bench)
     long long staged_gather_bytes = 0;
     // Rows of a large batch cross to the device once each: the slot of every row held here, the rows by slot, the number of slots and
-    // where each sub-batch's begin (kMarks: count, 0, end of part 0, end of part 1, ...).
+    // where each sub-batch's begin (PartMarks).
     DevBuf slot_of, unique, marks;
     bool slots_dirty = true;             // slot_of is not all -1 (never used, or a batch was left half done)
     int* h_unique = nullptr;             // pinned: the slots the host threads fill
     size_t h_unique_count = 0;
     size_t slots = 0;                    // of the batch at work, at most
-    int* h_marks = nullptr;              // pinned [2 * kMaxParts]
+    size_t parts = 0;                    // of the batch at work
+    int* h_marks = nullptr;              // pinned
+    size_t h_marks_words = 0;
     cudaStream_t list_stream = nullptr;  // brings the slot lists to the host thread beside the row copies
     std::vector<long long> h_global_begin;  // striped shards: host copy of the slices' first rows
     // workspaces
@@ -591,13 +594,8 @@ bool rows_form(const psb_session* s, int nq, int nprobe, bool any_probes = false
 // few enough that the per-(query, probe) tables stay below ~16 GiB.
 int sub_batch_rows(const psb_session* s, int n, int nprobe, bool overlap) {
     const int pipeline_parts = s->opt.pipeline_parts >= 2 && s->opt.pipeline_parts <= 32 ? s->opt.pipeline_parts : 4;
-    int parts = overlap ? pipeline_parts : 1;
-    if (s->opt.adc_mode == 1 && !residual_table_free(s, stage1_width(s, 1)) && !rows_form(s, n, nprobe)) {
-        const double bytes = (double)n * nprobe * s->m * s->k * sizeof(float);
-        parts = std::max(parts, (int)std::ceil(bytes / (16.0 * 1024 * 1024 * 1024)));
-    }
-    parts = std::min(parts, std::max(n, 1));
-    return (n + parts - 1) / parts;
+    const bool tables = s->opt.adc_mode == 1 && !residual_table_free(s, stage1_width(s, 1)) && !rows_form(s, n, nprobe);
+    return part_rows(n, overlap ? pipeline_parts : 1, tables ? (double)nprobe * s->m * s->k * sizeof(float) : 0.0);
 }
 
 // The staged transport (host gather threads + pinned rings), alone or with the kernel gather beside it.
@@ -766,7 +764,6 @@ psb_status validate_params(const psb_session* s, const psb_query_batch_view* qv,
     return PSB_OK;
 }
 
-constexpr int kMaxParts = 1024;           // sub-batches of a batch
 constexpr long long kClaimRequests = 65536;   // candidates from which a batch's rows are fetched once each
 
 // Staged rerank transport: host threads gather exact rows into two pinned buffers, and cudaMemcpyAsync moves each filled buffer
@@ -830,21 +827,22 @@ psb_status staged_gather_host(psb_session* s, const int* h_rows, size_t count, v
 
 // The rows of one batch (of one rerank call): claimed part by part, fetched once each, released at the end.  All of a batch's claims,
 // fetches and scores are ordered by the caller's streams and events.
-psb_status rows_begin(psb_session* s, long long requests, cudaStream_t st) {
+psb_status rows_begin(psb_session* s, long long requests, size_t parts, cudaStream_t st) {
     const size_t slots = (size_t)std::max<long long>(1, std::min(requests, s->exact_count));
     s->slots = slots;
+    s->parts = parts;
     PSB_TRY(s->unique.reserve(sizeof(int) * slots));
-    PSB_TRY(s->marks.reserve(sizeof(int) * (kMaxParts + 2)));
+    PSB_TRY(s->marks.reserve(sizeof(int) * PartMarks::device_words(parts)));
     PSB_TRY(s->stage.reserve(slots * s->dim * s->exact_elem));
     const bool fresh = s->slot_of.p == nullptr;
     PSB_TRY(s->slot_of.reserve(sizeof(int) * (size_t)std::max<long long>(1, s->exact_count)));
     if (fresh || s->slots_dirty) PSB_CUDA(cudaMemsetAsync(s->slot_of.p, 0xff, s->slot_of.bytes, st));
     s->slots_dirty = true;
-    PSB_CUDA(cudaMemsetAsync(s->marks.p, 0, sizeof(int) * (kMaxParts + 2), st));
+    PSB_CUDA(cudaMemsetAsync(s->marks.p, 0, sizeof(int) * PartMarks::device_words(parts), st));
     return PSB_OK;
 }
-int* part_begin(const psb_session* s, int part) { return s->marks.as<int>() + 1 + part; }
-int* part_end(const psb_session* s, int part) { return s->marks.as<int>() + 2 + part; }
+int* part_begin(const psb_session* s, int part) { return s->marks.as<int>() + PartMarks::device_begin((size_t)part); }
+int* part_end(const psb_session* s, int part) { return part_begin(s, part) + 1; }
 psb_status rows_claim(psb_session* s, int part, const int* d_cand, int nq, int width, int stride, const int* d_counts, cudaStream_t st) {
     PSB_TRY(launch_claim_rows(s->row_map(), d_cand, nq, width, stride, d_counts, s->slot_of.as<int>(), s->unique.as<int>(), s->marks.as<int>(), st));
     PSB_CUDA(cudaMemcpyAsync(part_end(s, part), s->marks.p, sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -855,15 +853,22 @@ psb_status rows_end(psb_session* s, cudaStream_t st) {
     s->slots_dirty = false;
     return PSB_OK;
 }
-// Queues the copy of a part's slot range to the host behind its claim (h_marks[2 part], [2 part + 1] once `st` gets there).
+// Queues the copy of a part's slot range to the host behind its claim (there once `st` gets to it).
 psb_status rows_tell_host(psb_session* s, int part, cudaStream_t st) {
-    if (!s->h_marks) PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_marks), sizeof(int) * 2 * kMaxParts, cudaHostAllocDefault));
-    PSB_CUDA(cudaMemcpyAsync(s->h_marks + 2 * part, part_begin(s, part), sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+    if (s->h_marks_words < PartMarks::host_words(s->parts)) {   // part 0: the worker of this batch has nothing to read yet
+        if (s->h_marks) { PSB_CUDA(cudaDeviceSynchronize()); cudaFreeHost(s->h_marks); }
+        s->h_marks = nullptr; s->h_marks_words = 0;
+        const size_t words = std::max(PartMarks::host_words(s->parts), (size_t)64);
+        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_marks), sizeof(int) * words, cudaHostAllocDefault));
+        s->h_marks_words = words;
+    }
+    PSB_CUDA(cudaMemcpyAsync(s->h_marks + PartMarks::host_begin((size_t)part), part_begin(s, part), sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
     return PSB_OK;
 }
 // The host threads' share of a part whose claim is done: slot list to the host, rows to their slots (copies on `st`).
 psb_status rows_from_host(psb_session* s, int part, int host_pct, cudaStream_t st) {
-    const int b = s->h_marks[2 * part], e = host_share_end(b, s->h_marks[2 * part + 1], host_pct);
+    const int* range = s->h_marks + PartMarks::host_begin((size_t)part);
+    const int b = range[0], e = host_share_end(b, range[1], host_pct);
     if (e <= b) return PSB_OK;
     if (!s->list_stream) PSB_CUDA(cudaStreamCreateWithFlags(&s->list_stream, cudaStreamNonBlocking));
     constexpr size_t kListChunk = (size_t)1 << 18;   // ids on the host at a time
@@ -926,7 +931,7 @@ psb_status rerank_impl(psb_session* s, const void* d_queries, int nq, const int*
     }
     const bool in_place = rows_in_place(s, (long long)nq * width);
     if (!in_place) {
-        PSB_TRY(rows_begin(s, (long long)nq * width, s->stream));
+        PSB_TRY(rows_begin(s, (long long)nq * width, 1, s->stream));
         PSB_TRY(rows_claim(s, 0, d_cand, nq, width, stride, d_counts, s->stream));
         const int host_pct = host_share(s);
         const int row_bytes = s->dim * s->exact_elem;
@@ -1532,8 +1537,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         if (plan == 2) cuts = {0, (int)(0.32 * n), (int)(0.64 * n), (int)(0.90 * n), n};  // short last sub-batch (scan-bound hosts)
         else cuts = {0, (int)(0.10 * n), (int)(0.40 * n), (int)(0.70 * n), n};
     } else {
-        for (int p0 = 0; p0 < n; p0 += sb) cuts.push_back(p0);
-        cuts.push_back(n);
+        cuts = even_cuts(n, sb);
     }
     int sb_max = 0;
     for (size_t ci = 0; ci + 1 < cuts.size(); ++ci) sb_max = std::max(sb_max, cuts[ci + 1] - cuts[ci]);
@@ -1573,12 +1577,12 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     // in its slot already), unless they are scored in place.
     const int host_pct = host_share(s);
     const bool hybrid = staged_overlap && host_pct < 100;
-    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k) && cuts.size() <= (size_t)kMaxParts);
+    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k));
     const int row_bytes = s->dim * s->exact_elem;
     if (hybrid) PSB_TRY(ensure_zc_stream(s));
     if (shared_rows) {
         PSB_TRY(s->score.reserve(sizeof(float) * (size_t)sb_max * stage1_k));
-        PSB_TRY(rows_begin(s, (long long)n * stage1_k, st));
+        PSB_TRY(rows_begin(s, (long long)n * stage1_k, cuts.size() - 1, st));
         cudaEvent_t e0;
         PSB_CUDA(cudaEventCreateWithFlags(&e0, cudaEventDisableTiming));
         deps.push_back(e0);
