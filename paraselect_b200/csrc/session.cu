@@ -1304,8 +1304,9 @@ psb_status psb_stage_scan_queries(psb_session* s, const float* d_queries, const 
                                   int nprobe, int stage1_k, int* d_rows, float* d_dist, int* d_count) {
     PSB_RANGE("pq_adc_scan");
     if (!s || !d_probes || !d_rows) return fail(PSB_INVALID_ARGUMENT, "null argument");
-    if (nprobe <= 0 || stage1_k <= 0) return fail(PSB_INVALID_ARGUMENT, "nprobe and stage1_k must be positive");
+    if (nq < 0 || nprobe <= 0 || stage1_k <= 0) return fail(PSB_INVALID_ARGUMENT, "nprobe and stage1_k must be positive, nq not negative");
     if (nprobe > kMaxProbe || stage1_k > kMaxStage1) return fail(PSB_UNSUPPORTED_SHAPE, "nprobe above 4096 or stage1_k above 2048");
+    if (nq == 0) return PSB_OK;
     s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, d_queries != nullptr && rows_form(s, nq, nprobe, true)));
