@@ -328,11 +328,13 @@ psb_status psb_stage_quantize_lut_u8(psb_session* session, const float* d_lut, i
  * d_count [nq] (may be NULL). */
 psb_status psb_stage_scan(psb_session* session, const float* d_lut, int nq, const int* d_probes, int nprobe,
                           int stage1_k, int* d_rows, float* d_dist, int* d_count);
-/* The same stage with the queries at hand (d_queries [nq][dim]): lets the scan take the tensor-core pre-filter, which
- * needs the query vectors besides their tables.  Same results as psb_stage_scan.  In residual mode d_lut may be NULL when
- * the tensor-core scan takes every list (scan_mode 0 or 3 on a supported shape): no per-(query, probe) table is then
- * materialised at all - the scan works on q - centroid directly, and the cutoff, re-scoring and fallback kernels compute
- * the table entries they need from the query, the centroid and the codebook. */
+/* The same stage with the queries at hand (d_queries [nq][dim]): lets the scan take the tensor-core pre-filter, which needs the
+ * query vectors besides their tables, or, for a small batch, score every row without a filter.  Same results as psb_stage_scan:
+ * whichever form runs, distances are sums of entries of d_lut, so d_lut has to be the tables of d_queries (a filter that works
+ * on the queries would otherwise drop rows by other distances than the tables give).  In residual mode d_lut may be NULL where
+ * the tensor-core scan is possible for every list (scan_mode 0 or 3 on a supported shape): no per-(query, probe) table is then
+ * materialised at all - the kernels build the entries they need from the query, the centroid and the codebook, with the same
+ * rounding. */
 psb_status psb_stage_scan_queries(psb_session* session, const float* d_queries, const float* d_lut, int nq,
                                   const int* d_probes, int nprobe, int stage1_k, int* d_rows, float* d_dist, int* d_count);
 

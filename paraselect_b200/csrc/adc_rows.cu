@@ -2,9 +2,10 @@
 //
 // The list-centric scans (pq_scan.cu, scan_tc.cu) sample a cutoff, schedule the visitors of every list, filter, re-score and sort pools:
 // about 180 us of kernels that a small batch pays in full, most of them one CTA per query.  Here a CTA builds the query's table in shared
-// memory (residual mode: the table of a (query, probe) pair), scores its share of the query's rows with it and writes the distances
-// out; nothing is sampled, scheduled or re-scored, and a query's rows spread over the chip.  Bound: shared-memory gathers, m per row
-// visit, about 3.5 cycles per warp-wide gather of random banks.  The selection is select.cuh's, reading each distance twice.
+// memory (residual mode: the table of a (query, probe) pair; a caller's own tables are read instead), scores its share of the query's rows
+// with it and writes the distances out; nothing is sampled, scheduled or re-scored, and a query's rows spread over the chip.  Bound:
+// shared-memory gathers, m per row visit, about 3.5 cycles per warp-wide gather of random banks.  The selection is select.cuh's, reading
+// each distance twice.
 // Same arithmetic and order as the other scans (reference: src/search/ivfpq/stage/ivfpq_fine_cpu_lut.cpp:51-63,76-80;
 // src/search/ivfrespq/stage/ivfrespq_cpu_rerank.cpp:87-130,226-259,440-451), so the same candidates.
 #include <algorithm>
@@ -48,6 +49,17 @@ __device__ __forceinline__ void build_table(float* __restrict__ s_tab, const flo
     }
 }
 
+// The table of a block: the caller's where there is one, else built on the (residual) query in s_q.
+__device__ __forceinline__ void block_table(float* __restrict__ s_tab, const float* __restrict__ s_q, const AdcRows& g, long long table) {
+    if (g.lut) {
+        const float* from = g.lut + (size_t)table * g.m * g.k;
+#pragma unroll 8
+        for (int e = threadIdx.x; e < g.m * g.k; e += kRowsThreads) s_tab[e] = __ldg(from + e);
+    } else {
+        build_table(s_tab, s_q, g.codebook, g.m, g.k, g.dim / g.m);
+    }
+}
+
 // Plain mode: grid (row blocks, queries); a block takes `block_rows` consecutive rows of the query's probed lists laid end to end.
 template <int M>
 __global__ void __launch_bounds__(kRowsThreads)
@@ -64,7 +76,7 @@ k_adc_rows(const AdcRows g, int block_rows) {
     for (int d = threadIdx.x; d < g.dim; d += kRowsThreads) s_q[d] = g.queries[(size_t)q * g.dim + d];
     for (int p = threadIdx.x; p <= g.nprobe; p += kRowsThreads) s_seg[p] = seg[p];
     __syncthreads();
-    build_table(s_tab, s_q, g.codebook, g.m, g.k, g.dim / g.m);
+    block_table(s_tab, s_q, g, q);
     __syncthreads();
     float* out = g.dist + (size_t)q * g.stride;
     for (int i = i0 + threadIdx.x; i < i1; i += kRowsThreads) {
@@ -92,7 +104,7 @@ k_adc_pair_rows(const AdcRows g, int block_rows, int chunks) {
     for (int d = threadIdx.x; d < g.dim; d += kRowsThreads)
         s_q[d] = __fsub_rn(g.queries[(size_t)q * g.dim + d], __ldg(g.centroids + (size_t)l * g.dim + d));
     __syncthreads();
-    build_table(s_tab, s_q, g.codebook, g.m, g.k, g.dim / g.m);
+    block_table(s_tab, s_q, g, pair);
     __syncthreads();
     float* out = g.dist + (size_t)q * g.stride + g.seg[(size_t)q * (g.nprobe + 1) + p];
     for (long long r = r0 + threadIdx.x; r < r1; r += kRowsThreads)

@@ -261,6 +261,7 @@ psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const lo
 // The ADC scan in its row form: all distances, then the stage1_k smallest.
 struct AdcRows {
     const float* queries; const int* probes; int nprobe;
+    const float* lut;   // the caller's tables, [nq][m * k] or, residual, [nq][nprobe][m * k]; null: each block builds its own
     const float* centroids; const float* codebook; const uint8_t* codes; const long long* offsets; long long row_base; const long long* row_delta;
     int list_begin, list_end, dim, m, k;
     bool residual, tree;

@@ -547,6 +547,13 @@ bool residual_table_free(const psb_session* s, int stage1_k) {
            (size_t)pool_capacity(stage1_k) * 8 + (size_t)s->dim * 4 <= (size_t)226 * 1024;
 }
 
+// Whether a stage call may leave its tables out: residual mode on a shape the tensor-core scan takes (a shard without rows scans
+// nothing), whichever form the scan then runs in.
+bool tables_optional(const psb_session* s, int stage1_k) {
+    if (residual_table_free(s, stage1_k)) return true;
+    return s->opt.adc_mode == 1 && s->shard_rows == 0 && scan_tc_supported(s->dim, s->m, s->k);
+}
+
 // Tables one scan call needs for nq queries.
 size_t table_count(const psb_session* s, int nq, int nprobe) {
     return s->opt.adc_mode == 1 ? (size_t)nq * nprobe : (size_t)nq;
@@ -644,7 +651,8 @@ psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool
     return PSB_OK;
 }
 
-// The ADC scan of one sub-batch.  d_lut may be null in the row form (it builds its tables in shared memory) and as launch_scan allows.
+// The ADC scan of one sub-batch.  d_lut may be null in the row form (it then builds its tables in shared memory) and as launch_scan
+// allows; tables that are given are what every form scores from.
 psb_status run_scan(psb_session* s, const ScanWorkspace& ws, const float* d_queries, const float* d_lut, int nq, const int* d_probes, int nprobe,
                     int stage1_k, int* d_rows, float* d_dist, int* d_count, cudaStream_t st, bool any_probes = false) {
     if (!d_queries || ws.phase != 0 || !rows_form(s, nq, nprobe, any_probes))
@@ -663,6 +671,7 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, const float* d_quer
     if (ws.ev_begin) PSB_CUDA(cudaEventRecord(ws.ev_begin, st));
     for (int q0 = 0; q0 < nq; q0 += per) {
         g.queries = d_queries + (size_t)q0 * s->dim; g.probes = d_probes + (size_t)q0 * nprobe;
+        g.lut = d_lut ? d_lut + (size_t)q0 * table_count(s, 1, nprobe) * s->m * s->k : nullptr;
         g.out_rows = d_rows + (size_t)q0 * stage1_k; g.out_dist = d_dist ? d_dist + (size_t)q0 * stage1_k : nullptr;
         g.out_count = d_count ? d_count + q0 : nullptr;
         PSB_TRY(launch_adc_rows(g, std::min(per, nq - q0), st));
@@ -1307,6 +1316,8 @@ psb_status psb_stage_scan_queries(psb_session* s, const float* d_queries, const 
     if (nq < 0 || nprobe <= 0 || stage1_k <= 0) return fail(PSB_INVALID_ARGUMENT, "nprobe and stage1_k must be positive, nq not negative");
     if (nprobe > kMaxProbe || stage1_k > kMaxStage1) return fail(PSB_UNSUPPORTED_SHAPE, "nprobe above 4096 or stage1_k above 2048");
     if (nq == 0) return PSB_OK;
+    if (!d_lut && !tables_optional(s, stage1_k))
+        return fail(PSB_INVALID_ARGUMENT, "the scan needs the lookup tables (they may be left out only in residual mode with the tensor-core scan)");
     s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, d_queries != nullptr && rows_form(s, nq, nprobe, true)));

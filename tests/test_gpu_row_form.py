@@ -33,3 +33,28 @@ def test_empty_batch(psb, M, dim, residual):
             s.stage_scan_queries(dev(q), lut, -1, dev(probes.astype(np.int32)), 3, 20, rows, dist, cnt)
         s.sync()
     assert (rows.cpu().numpy() == -9).all()
+
+
+@pytest.mark.parametrize("M,dim", [(48, 96), (20, 100)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_scores_come_from_the_callers_tables(psb, M, dim, residual):
+    """Tables that are not the queries' own: the row form's distances are their entries' sums, as those of the call without queries."""
+    nq, nprobe, width = 5, 4, 60
+    ix = synth.make_index(4000, dim, 8, M, seed=M + 5, residual=residual)
+    q = synth.make_queries(ix, nq, seed=2)
+    probes, _ = oracle.coarse(q, ix["centroids"], nprobe)
+    dp, dq = dev(probes.astype(np.int32)), dev(q)
+    lut = dev(np.random.default_rng(M).random((nq * (nprobe if residual else 1), M * 256)).astype(np.float32))
+    want, got = outputs(nq, width), outputs(nq, width)
+    with psb.Session(ix, residual=residual) as s:
+        s.stage_scan(lut, nq, dp, nprobe, width, *want)
+        s.stage_scan_queries(dq, lut, nq, dp, nprobe, width, *got)
+        s.sync()
+        for a, b in zip(got, want):
+            assert np.array_equal(a.cpu().numpy(), b.cpu().numpy())
+        if residual and M == 48:
+            s.stage_scan_queries(dq, None, nq, dp, nprobe, width, *got)
+        else:   # nothing to score with: refused whatever the batch's size
+            with pytest.raises(psb.InvalidArgument):
+                s.stage_scan_queries(dq, None, nq, dp, nprobe, width, *got)
+        s.sync()
