@@ -349,7 +349,7 @@ k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* 
                 uint32_t hit = 0;
 #pragma unroll
                 for (int u = 0; u < 16; ++u) hit |= (gm[i][u] >= thr ? 1u : 0u) << u;
-                if (!(mx == mx)) hit = 0xffffu;   // not a number somewhere: no bound holds, evaluate everything
+                if (!(fabsf(thr) <= FLT_MAX)) hit = 0xffffu;   // a product or a norm overflowed or is not a number: no bound holds, evaluate everything
                 while (hit) {
                     const int u = __ffs((int)hit) - 1;
                     hit &= hit - 1;

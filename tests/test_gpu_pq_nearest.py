@@ -26,3 +26,24 @@ def test_encode_matches_checker(n, dim, M, K):
     api.pq_encode(torch.from_numpy(x).cuda(), n, dim, torch.from_numpy(cb).cuda(), M, K, codes)
     torch.cuda.synchronize()
     assert np.array_equal(codes.cpu().numpy(), oracle.pq_encode(x, cb))
+
+
+@pytest.mark.parametrize("dim,M", [(8, 4), (16, 4), (32, 4), (20, 4), (64, 4)])   # two to sixteen dimensions a sub-vector
+@pytest.mark.parametrize("scale", [3e18, 1e19, 1.8e19, 1e20])
+def test_encode_where_products_overflow(dim, M, scale):
+    """Magnitudes whose products pass the range of fp32 although distances to near codewords do not: rows are codewords or lie beside them."""
+    import torch
+    from paraselect_b200 import api
+    rng = np.random.default_rng(dim)
+    n, K = 700, 256
+    cb = (rng.standard_normal((M, K, dim // M)) * scale).astype(np.float32)
+    pick = rng.integers(0, K, (n, M))
+    x = (cb[np.arange(M)[None, :], pick] * (1 + 1e-3 * rng.standard_normal((n, M, 1)))).astype(np.float32).reshape(n, dim)
+    x[: n // 2] = cb[np.arange(M)[None, :], pick[: n // 2]].reshape(-1, dim)
+    x[-20:] = 0.0
+    codes = torch.full((n, M), 99, dtype=torch.uint8, device="cuda")
+    api.pq_encode(torch.from_numpy(x).cuda(), n, dim, torch.from_numpy(cb).cuda(), M, K, codes)
+    torch.cuda.synchronize()
+    want = oracle.pq_encode(x, cb)
+    assert np.array_equal(codes.cpu().numpy(), want)
+    assert np.array_equal(want[: n // 2], pick[: n // 2])
