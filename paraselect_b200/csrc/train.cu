@@ -112,6 +112,7 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
 constexpr int kNearWarps = 8;
 constexpr int kNearSets = 2;                     // sets of 32 rows a warp takes one after the other against one codebook
 constexpr int kNearRows = kNearWarps * 32 * kNearSets;   // rows per CTA
+constexpr float kFarNorm = 3.0e38f;              // in place of |c|^2 / 2 for codewords past k: below every score a threshold is taken from
 constexpr int kNearQueue = 384;                  // hits a warp queues (32 rows: usually 33 or 34); any beyond are evaluated on the spot
 
 __device__ __forceinline__ uint32_t bf16_word(float lo, float hi) {
@@ -244,7 +245,7 @@ k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* 
                 const float h = bf16_round(v[d]);
                 slot[d] = h; slot[D + d] = v[d] - h; slot[2 * D + d] = h;
             }
-            float rest = c < k ? 0.5f * n2 : 1.0e30f;   // codewords past k are never near
+            float rest = c < k ? 0.5f * n2 : kFarNorm;   // codewords past k are never near
 #pragma unroll
             for (int i = 0; i < 3; ++i) { const float h = bf16_round(rest); slot[3 * D + i] = -h; rest -= h; }
             uint4* dst = reinterpret_cast<uint4*>(s_b + ((size_t)(c >> 3) * KS) * 32 + (c & 7) * 4);   // fragment lane = (column % 8) * 4 + t
@@ -349,7 +350,7 @@ k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* 
                 uint32_t hit = 0;
 #pragma unroll
                 for (int u = 0; u < 16; ++u) hit |= (gm[i][u] >= thr ? 1u : 0u) << u;
-                if (!(fabsf(thr) <= FLT_MAX)) hit = 0xffffu;   // a product or a norm overflowed or is not a number: no bound holds, evaluate everything
+                if (!(fabsf(thr) <= 0.9f * kFarNorm)) hit = 0xffffu;   // a product or a norm overflowed or is not a number, or the codewords past k came first: evaluate everything
                 while (hit) {
                     const int u = __ffs((int)hit) - 1;
                     hit &= hit - 1;

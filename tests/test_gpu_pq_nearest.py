@@ -47,3 +47,20 @@ def test_encode_where_products_overflow(dim, M, scale):
     want = oracle.pq_encode(x, cb)
     assert np.array_equal(codes.cpu().numpy(), want)
     assert np.array_equal(want[: n // 2], pick[: n // 2])
+
+
+@pytest.mark.parametrize("dim,M,K", [(8, 4, 100), (16, 4, 33), (32, 4, 255), (20, 4, 64), (64, 4, 40)])
+@pytest.mark.parametrize("scale", [1e14, 1e16, 1e18, 1e19])
+def test_encode_fewer_codewords_far_away(dim, M, K, scale):
+    """Rows near the origin, fewer than 256 codewords all far from it: every score is a large negative number."""
+    import torch
+    from paraselect_b200 import api
+    rng = np.random.default_rng(dim + K)
+    n = 300
+    cb = (np.sign(rng.standard_normal((M, K, dim // M))) * scale * (1 + 0.1 * rng.random((M, K, dim // M)))).astype(np.float32)
+    x = (rng.standard_normal((n, dim)) * scale * 1e-3).astype(np.float32)
+    x[: n // 3] = 0.0
+    codes = torch.full((n, M), 99, dtype=torch.uint8, device="cuda")
+    api.pq_encode(torch.from_numpy(x).cuda(), n, dim, torch.from_numpy(cb).cuda(), M, K, codes)
+    torch.cuda.synchronize()
+    assert np.array_equal(codes.cpu().numpy(), oracle.pq_encode(x, cb))
