@@ -101,7 +101,8 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
 // accumulators of mma.sync lie in registers where the maximum is taken; the contraction is so short (one K step for dsub 4) that
 // a tcgen05 accumulator would have to be read back from tensor memory, one value per pair, for a single K step of work.
 //   E: bf16 splits 3.1 * 2^-18 |x||c|; accumulation and norm split (16 KS) 2^-22 (|x||c| + |c|^2 / 2); rounding of the exact fp32
-//   distance (2 dsub + 2) 2^-24 (|x| + |c|)^2: together 2E <= 2^-15 |x| cmax + (KS + 1) 2^-18 (|x| + cmax)^2.
+//   distance (2 dsub + 2) 2^-24 (|x| + |c|)^2: together 2E <= 2^-15 |x| cmax + (KS + 1) 2^-18 (|x| + cmax)^2, and where products
+//   are subnormal or vanish, 2^-126 for each of the 16 KS products and three norm terms: 2 (16 KS + 3) 2^-126 <= 2^-118.
 // The nearest codeword in the exact arithmetic and all its ties are among the evaluated ones; the lowest index wins a tie.
 // kTrain: the evaluated ones are compared by |c|^2 - 2 x.c in fused multiply-adds, as the trainer's Lloyd iterations always have (the
 // reference's trainer assigns with a TF32 GEMM: src/quantization/pq/pq_trainer.cu:97-170); its rounding is within the same bound.
@@ -112,6 +113,7 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
 constexpr int kNearWarps = 8;
 constexpr int kNearSets = 2;                     // sets of 32 rows a warp takes one after the other against one codebook
 constexpr int kNearRows = kNearWarps * 32 * kNearSets;   // rows per CTA
+constexpr float kNearTiny = 3.1e-36f;            // above 2^-118
 constexpr float kFarNorm = 3.0e38f;              // in place of |c|^2 / 2 for codewords past k: below every score a threshold is taken from
 constexpr int kNearQueue = 384;                  // hits a warp queues (32 rows: usually 33 or 34); any beyond are evaluated on the spot
 
@@ -346,7 +348,7 @@ k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* 
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
                 const float nx = sqrtf(xn[i]) * 1.000001f, both = nx + cmax;
-                const float thr = mx - (3.0517578125e-5f * nx * cmax + (float)(KS + 1) * 3.814697265625e-6f * both * both);
+                const float thr = mx - (3.0517578125e-5f * nx * cmax + (float)(KS + 1) * 3.814697265625e-6f * both * both + kNearTiny);
                 uint32_t hit = 0;
 #pragma unroll
                 for (int u = 0; u < 16; ++u) hit |= (gm[i][u] >= thr ? 1u : 0u) << u;

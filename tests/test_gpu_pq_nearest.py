@@ -64,3 +64,19 @@ def test_encode_fewer_codewords_far_away(dim, M, K, scale):
     api.pq_encode(torch.from_numpy(x).cuda(), n, dim, torch.from_numpy(cb).cuda(), M, K, codes)
     torch.cuda.synchronize()
     assert np.array_equal(codes.cpu().numpy(), oracle.pq_encode(x, cb))
+
+
+@pytest.mark.parametrize("dim,M", [(8, 4), (16, 4), (32, 4), (20, 4), (64, 4)])
+@pytest.mark.parametrize("scale", [1e-16, 1e-18, 1e-19, 1e-20, 1e-22])
+def test_encode_where_products_underflow(dim, M, scale):
+    """Magnitudes whose products are subnormal or vanish: the filter's rounding is absolute there, not relative."""
+    import torch
+    from paraselect_b200 import api
+    rng = np.random.default_rng(dim)
+    n, K = 700, 256
+    cb = (rng.standard_normal((M, K, dim // M)) * scale).astype(np.float32)
+    x = (rng.standard_normal((n, dim)) * scale).astype(np.float32)
+    codes = torch.full((n, M), 99, dtype=torch.uint8, device="cuda")
+    api.pq_encode(torch.from_numpy(x).cuda(), n, dim, torch.from_numpy(cb).cuda(), M, K, codes)
+    torch.cuda.synchronize()
+    assert np.array_equal(codes.cpu().numpy(), oracle.pq_encode(x, cb))
