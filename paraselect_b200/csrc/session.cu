@@ -613,8 +613,13 @@ bool overlap_enabled(const psb_session* s, int n, bool rerank) {
 }
 
 // Grows the scan workspace to hold nq queries (never shrinks; a growing buffer is freed first, which waits for the device).
-// own_tables: the scan's row form takes this call (it needs no tables).
-psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool own_tables) {
+// row_form: the scan's row form takes this call.  It uses the counters alone of all that follows; its distances are run_scan's.
+psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool row_form) {
+    if (!s->scalars.p) {
+        PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
+        PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, s->stream));
+    }
+    if (row_form) return PSB_OK;
     const size_t tables = table_count(s, nq, nprobe);
     s->ws_scan_queries = 0; s->ws_scan_tables = 0;  // set again below once every buffer has its size
     PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
@@ -631,14 +636,10 @@ psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool
     s->pool_cap = cap;
     PSB_TRY(s->fail_list.reserve(sizeof(int) * (size_t)nq));
     PSB_TRY(s->fallback_partial.reserve(fallback_partial_bytes(stage1_k)));
-    const bool half_tables = s->opt.scan_mode != 1 && !residual_table_free(s, stage1_k) && !own_tables;
+    const bool half_tables = s->opt.scan_mode != 1 && !residual_table_free(s, stage1_k);
     if (half_tables) {
         PSB_TRY(s->lut_h.reserve(sizeof(unsigned short) * tables * s->m * s->k));
         PSB_TRY(s->lut_scale.reserve(sizeof(float) * tables));
-    }
-    if (!s->scalars.p) {
-        PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
-        PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, s->stream));
     }
     // what the buffers hold now (reserve() keeps a larger buffer from an earlier call)
     s->ws_scan_queries = (int)std::min<size_t>({s->q_rows.bytes / sizeof(long long), s->thr.bytes / sizeof(float),
@@ -652,10 +653,11 @@ psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool
 }
 
 // The ADC scan of one sub-batch.  d_lut may be null in the row form (it then builds its tables in shared memory) and as launch_scan
-// allows; tables that are given are what every form scores from.
-psb_status run_scan(psb_session* s, const ScanWorkspace& ws, const float* d_queries, const float* d_lut, int nq, const int* d_probes, int nprobe,
-                    int stage1_k, int* d_rows, float* d_dist, int* d_count, cudaStream_t st, bool any_probes = false) {
-    if (!d_queries || ws.phase != 0 || !rows_form(s, nq, nprobe, any_probes))
+// allows; tables that are given are what every form scores from.  rows_only: ensure_scan_ws was told of the row form, so nothing else
+// has its buffers.
+psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, const float* d_queries, const float* d_lut, int nq, const int* d_probes,
+                    int nprobe, int stage1_k, int* d_rows, float* d_dist, int* d_count, cudaStream_t st, bool any_probes = false) {
+    if (!rows_only && (!d_queries || !rows_form(s, nq, nprobe, any_probes)))
         return launch_scan(s->scan_index(), ws, d_lut, nq, d_probes, nprobe, stage1_k, d_rows, d_dist, d_count, s->sm_count, st, d_queries);
     AdcRows g{};
     g.stride = row_stride(s, nprobe, any_probes);
@@ -1320,10 +1322,11 @@ psb_status psb_stage_scan_queries(psb_session* s, const float* d_queries, const 
         return fail(PSB_INVALID_ARGUMENT, "the scan needs the lookup tables (they may be left out only in residual mode with the tensor-core scan)");
     s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
-    PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, d_queries != nullptr && rows_form(s, nq, nprobe, true)));
+    const bool rows_only = d_queries != nullptr && rows_form(s, nq, nprobe, true);
+    PSB_TRY(ensure_scan_ws(s, nq, nprobe, stage1_k, rows_only));
     ScanWorkspace ws;
     PSB_TRY(s->timed_scan_ws(&ws));
-    return run_scan(s, ws, d_queries, d_lut, nq, d_probes, nprobe, stage1_k, d_rows, d_dist, d_count, s->stream, true);
+    return run_scan(s, ws, rows_only, d_queries, d_lut, nq, d_probes, nprobe, stage1_k, d_rows, d_dist, d_count, s->stream, true);
 }
 
 int psb_scan_sample_words(const psb_session* s, int stage1_k) {
@@ -1555,9 +1558,9 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     for (size_t ci = 0; ci + 1 < cuts.size(); ++ci) sb_max = std::max(sb_max, cuts[ci + 1] - cuts[ci]);
     // The sub-batch size depends on this batch's own n (a short tail batch may run in one piece where the full batch ran
     // in four), so the tables and the scan workspace are sized here, for the largest sub-batch of THIS batch.
-    const bool table_free = residual_table_free(s, stage1_k) || rows_form(s, sb_max, nprobe);
+    const bool rows_only = rows_form(s, sb_max, nprobe), table_free = residual_table_free(s, stage1_k) || rows_only;
     if (!table_free) PSB_TRY(s->lut.reserve(sizeof(float) * table_count(s, sb_max, nprobe) * s->m * s->k));
-    PSB_TRY(ensure_scan_ws(s, sb_max, nprobe, stage1_k, rows_form(s, sb_max, nprobe)));
+    PSB_TRY(ensure_scan_ws(s, sb_max, nprobe, stage1_k, rows_only));
     if ((overlap || staged_overlap) && !s->aux_stream) {
         int lo = 0, hi = 0;  // lowest priority: the scan's CTAs get the SMs first, the transfer fills the gaps
         PSB_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
@@ -1690,7 +1693,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         if (rc == PSB_OK && times && !table_free) rc = times->end(StageTimes::kLut, st);
         if (rc == PSB_OK) {
             PSB_RANGE("pq_adc_scan");
-            rc = run_scan(s, sws, q, table_free ? nullptr : s->lut.as<float>(), m, probes, nprobe, stage1_k, rows_out, dist_out, cnt_out, st);
+            rc = run_scan(s, sws, rows_only, q, table_free ? nullptr : s->lut.as<float>(), m, probes, nprobe, stage1_k, rows_out, dist_out, cnt_out, st);
         }
         if (rc == PSB_OK && times) rc = times->end(StageTimes::kScan, st);
         if (rc != PSB_OK) break;

@@ -58,3 +58,20 @@ def test_scores_come_from_the_callers_tables(psb, M, dim, residual):
             with pytest.raises(psb.InvalidArgument):
                 s.stage_scan_queries(dq, None, nq, dp, nprobe, width, *got)
         s.sync()
+
+
+def test_row_form_takes_no_list_workspace(psb):
+    """A batch in the row form leaves the admission pools (131 MB for 1,000 queries of 1,000 candidates) and the fallback's lists alone."""
+    import torch
+    ix = synth.make_index(4000, 100, 8, 20, seed=9, residual=True)
+    q = synth.make_queries(ix, 1000, seed=3)
+    want = oracle.ivfrespq_search(ix, q[:50], 4, 10, 1000)
+    used = []
+    for _ in range(2):   # the first session also brings the kernels in
+        with psb.Session(ix, n_rerank=1000, residual=True, max_batch=1000) as s:
+            torch.cuda.synchronize()
+            before = torch.cuda.mem_get_info()[0]
+            got = s.search(q, 4, 10)
+            used.append(before - torch.cuda.mem_get_info()[0])
+        assert np.array_equal(got["indices"][:50], want["indices"]) and np.array_equal(got["distances"][:50], want["distances"])
+    assert used[1] < 100e6, used
