@@ -173,6 +173,54 @@ struct PoolBuf {
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Host rows mapped for the device, counted over the sessions that read them: several sessions may lie over one array (a session per
+// query thread, or per view of it), and the mapping ends with the last of them, whichever made it.
+class MappedRows {
+public:
+    static MappedRows& get() { static MappedRows* one = new MappedRows; return *one; }   // never destroyed: the driver may end first
+    // *counted: give() has to follow.  False when the caller itself has the range registered, which is then the caller's to end.
+    psb_status take(const void* rows, size_t bytes, bool* counted) {
+        const uintptr_t b = reinterpret_cast<uintptr_t>(rows), e = b + bytes;
+        std::lock_guard<std::mutex> lk(mu_);
+        *counted = false;
+        for (Range& r : ranges_) {
+            if (r.begin <= b && e <= r.end) { ++r.users; *counted = true; return PSB_OK; }
+            if (r.begin < e && b < r.end)
+                return fail(PSB_CUDA_ERROR, "the exact rows overlap rows another session has mapped; use PSB_EXACT_HOST_STAGED");
+        }
+        cudaError_t err = cudaHostRegister(const_cast<void*>(rows), bytes, cudaHostRegisterMapped | cudaHostRegisterReadOnly);
+        if (err == cudaErrorHostMemoryAlreadyRegistered) { cudaGetLastError(); return PSB_OK; }
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            err = cudaHostRegister(const_cast<void*>(rows), bytes, cudaHostRegisterMapped);
+        }
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            return fail(PSB_CUDA_ERROR, std::string("cannot map the exact rows into the device address space (") + cudaGetErrorString(err) +
+                                            "); use PSB_EXACT_HOST_STAGED");
+        }
+        ranges_.push_back(Range{b, e, 1});
+        *counted = true;
+        return PSB_OK;
+    }
+    void give(const void* rows, size_t bytes) {
+        const uintptr_t b = reinterpret_cast<uintptr_t>(rows), e = b + bytes;
+        std::lock_guard<std::mutex> lk(mu_);
+        for (size_t i = 0; i < ranges_.size(); ++i) {
+            if (b < ranges_[i].begin || ranges_[i].end < e) continue;
+            if (--ranges_[i].users == 0) {
+                cudaHostUnregister(reinterpret_cast<void*>(ranges_[i].begin));
+                ranges_.erase(ranges_.begin() + (ptrdiff_t)i);
+            }
+            return;
+        }
+    }
+private:
+    struct Range { uintptr_t begin, end; int users; };
+    std::mutex mu_;
+    std::vector<Range> ranges_;
+};
+
 // Persistent fork-join pool of host threads for the staged rerank transport (the reference keeps a persistent rerank pool
 // too: src/search/ivf_common/ivf_host_rerank.cpp:42-51).  run(job) calls job(t) on every thread t and returns when all are done.
 class HostPool {
@@ -360,7 +408,7 @@ struct psb_session {
     int exact_elem = 0;            // 4 = fp32, 1 = u8, 0 = rerank disabled
     const void* exact_host = nullptr;
     const void* exact_dev = nullptr;  // device-visible pointer (mapped host or resident)
-    bool registered = false;
+    bool mapped = false;           // exact_host is counted in MappedRows
     long long exact_count = 0;
     // staged mode
     void* pinned[2] = {nullptr, nullptr};
@@ -424,7 +472,7 @@ struct psb_session {
             stream = home_stream;
         }
         collect_scan_events();
-        if (registered) cudaHostUnregister(const_cast<void*>(exact_host));
+        if (mapped) MappedRows::get().give(exact_host, (size_t)exact_count * dim * exact_elem);
         for (int i = 0; i < 2; ++i) {
             if (pinned[i]) cudaFreeHost(pinned[i]);
             if (pinned_ev[i]) cudaEventDestroy(pinned_ev[i]);
@@ -1148,18 +1196,7 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
                                          cudaMemcpyHostToDevice, st));
             s->exact_dev = s->exact_cache.p;
         } else if ((opt.exact_mode == PSB_EXACT_HOST_MAPPED || opt.exact_mode == PSB_EXACT_HOST_HYBRID) && bytes > 0) {
-            cudaError_t e = cudaHostRegister(const_cast<void*>(s->exact_host), bytes, cudaHostRegisterMapped | cudaHostRegisterReadOnly);
-            if (e == cudaErrorHostMemoryAlreadyRegistered) { cudaGetLastError(); e = cudaSuccess; }
-            else if (e != cudaSuccess) {
-                cudaGetLastError();
-                e = cudaHostRegister(const_cast<void*>(s->exact_host), bytes, cudaHostRegisterMapped);
-                if (e == cudaSuccess) s->registered = true;
-            } else s->registered = true;
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                return fail(PSB_CUDA_ERROR, std::string("cannot map the exact rows into the device address space (") +
-                                                cudaGetErrorString(e) + "); use PSB_EXACT_HOST_STAGED");
-            }
+            PSB_TRY(MappedRows::get().take(s->exact_host, bytes, &s->mapped));
             void* dp = nullptr;
             PSB_CUDA(cudaHostGetDevicePointer(&dp, const_cast<void*>(s->exact_host), 0));
             s->exact_dev = dp;
