@@ -221,6 +221,36 @@ private:
     std::vector<Range> ranges_;
 };
 
+// Page-locked blocks through which small calls pass, one to a session from its first search to its end, handed on from session to
+// session.  A process's first page-locked memory takes 0.8 to 3 ms whatever its size, and again whenever all of it has been given back
+// in between: four fifths of the first search of a session that answers single queries.  At most kIdle blocks (2 MiB) stay with the library.
+constexpr size_t kSmallIo = 256 * 1024;   // queries and results of a call that passes through the block
+constexpr size_t kHostBlock = kSmallIo + 4096;
+class HostBlocks {
+public:
+    static HostBlocks& get() { static HostBlocks* one = new HostBlocks; return *one; }   // never destroyed: the driver may end first
+    psb_status take(unsigned char** out) {
+        for (;;) {
+            unsigned char* p = nullptr;
+            { std::lock_guard<std::mutex> lk(mu_); if (!idle_.empty()) { p = idle_.back(); idle_.pop_back(); } }
+            if (!p) break;
+            cudaPointerAttributes at{};   // a block from before a device reset is no longer the driver's, nor ours to free
+            if (cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost) { *out = p; return PSB_OK; }
+            cudaGetLastError();
+        }
+        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(out), kHostBlock, cudaHostAllocMapped | cudaHostAllocPortable));
+        return PSB_OK;
+    }
+    void give(unsigned char* p) {   // nothing on the device may still use it
+        { std::lock_guard<std::mutex> lk(mu_); if (idle_.size() < kIdle) { idle_.push_back(p); return; } }
+        cudaFreeHost(p);
+    }
+private:
+    static constexpr size_t kIdle = 8;
+    std::mutex mu_;
+    std::vector<unsigned char*> idle_;
+};
+
 // Persistent fork-join pool of host threads for the staged rerank transport (the reference keeps a persistent rerank pool
 // too: src/search/ivf_common/ivf_host_rerank.cpp:42-51).  run(job) calls job(t) on every thread t and returns when all are done.
 class HostPool {
@@ -423,10 +453,10 @@ struct psb_session {
     EventPool timing, timing_aux;          // events of the main stream's marks and of the second stream's (set from one thread each)
     // Host side of a search call: one pinned block through which a small batch's queries and results pass, and the device's counters
     // and status words with the results, so that a call waits for the GPU once.
-    unsigned char* h_io = nullptr;
-    size_t h_io_bytes = 0;
+    unsigned char* h_io = nullptr;         // a block of HostBlocks: kSmallIo bytes, then the tail
     struct Tail { unsigned long long c[16]; int tc[8]; };
-    Tail* h_tail = nullptr;                // pinned
+    Tail* h_tail = nullptr;
+    static_assert(kSmallIo + sizeof(Tail) <= kHostBlock, "the tail lies behind the block's data");
     bool counters_known = false;           // h_tail->c is what the device's counters hold
     DevBuf row_dist, row_seg;              // a row of distances per query (IVF-Flat, row form of the ADC scan)
     std::vector<long long> longest;        // [p] = rows of this shard's p longest lists together
@@ -471,19 +501,18 @@ struct psb_session {
             cudaStreamSynchronize(home_stream);
             stream = home_stream;
         }
+        // A search that returned an error may have left work on its other streams: nothing they use is given back before they have drained.
+        for (cudaStream_t other : {list_stream, aux_stream, zc_stream})
+            if (other) { cudaStreamSynchronize(other); cudaStreamDestroy(other); }
         collect_scan_events();
         if (mapped) MappedRows::get().give(exact_host, (size_t)exact_count * dim * exact_elem);
         for (int i = 0; i < 2; ++i) {
             if (pinned[i]) cudaFreeHost(pinned[i]);
             if (pinned_ev[i]) cudaEventDestroy(pinned_ev[i]);
         }
-        if (h_io) cudaFreeHost(h_io);
-        if (h_tail) cudaFreeHost(h_tail);
         if (h_unique) cudaFreeHost(h_unique);
         if (h_marks) cudaFreeHost(h_marks);
-        if (list_stream) { cudaStreamSynchronize(list_stream); cudaStreamDestroy(list_stream); }
-        if (aux_stream) { cudaStreamSynchronize(aux_stream); cudaStreamDestroy(aux_stream); }
-        if (zc_stream) { cudaStreamSynchronize(zc_stream); cudaStreamDestroy(zc_stream); }
+        if (h_io) HostBlocks::get().give(h_io);
         if (zc_ev_a) cudaEventDestroy(zc_ev_a);
         if (zc_ev_b) cudaEventDestroy(zc_ev_b);
 
@@ -1523,21 +1552,12 @@ struct StageTimes {
     }
 };
 
-constexpr size_t kSmallIo = 256 * 1024;   // queries and results of a call that pass through the pinned block
-
-// The pinned block and the tail, large enough; `bytes` of the block are asked for.
-psb_status ensure_host_io(psb_session* s, size_t bytes) {
-    if (s->h_io_bytes < bytes) {
-        if (s->h_io) cudaFreeHost(s->h_io);
-        s->h_io = nullptr; s->h_io_bytes = 0;
-        const size_t want = std::max<size_t>(bytes, 16 * 1024);
-        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_io), want, cudaHostAllocMapped | cudaHostAllocPortable));
-        s->h_io_bytes = want;
-    }
-    if (!s->h_tail) {
-        PSB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->h_tail), sizeof(psb_session::Tail), cudaHostAllocPortable));
-        std::memset(s->h_tail, 0, sizeof(*s->h_tail));
-    }
+// The session's page-locked block.
+psb_status ensure_host_io(psb_session* s) {
+    if (s->h_io) return PSB_OK;
+    PSB_TRY(HostBlocks::get().take(&s->h_io));
+    s->h_tail = reinterpret_cast<psb_session::Tail*>(s->h_io + kSmallIo);
+    std::memset(s->h_tail, 0, sizeof(*s->h_tail));
     return PSB_OK;
 }
 // Queues the device's counters and status words behind the work on `st`.
@@ -1857,7 +1877,7 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
     const size_t b_q = (sizeof(float) * (size_t)total * s->dim + 255) / 256 * 256, b_u8 = u8 ? ((size_t)total * s->dim + 255) / 256 * 256 : 0,
                  b_ids = sizeof(long long) * (size_t)total * topk, b_dist = sizeof(float) * (size_t)total * topk;
     const bool small = batch == total && b_q + b_u8 + b_ids + b_dist <= kSmallIo;
-    PSB_TRY(ensure_host_io(s, small ? b_q + b_u8 + b_ids + b_dist : 0));
+    PSB_TRY(ensure_host_io(s));
     const long long launches0 = launches_total();
     unsigned long long c0[4] = {0, 0, 0, 0};
     if (stats) PSB_TRY(counters_before(s, st, c0));
@@ -2072,7 +2092,7 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
     const size_t b_q = (sizeof(float) * (size_t)total * s->dim + 255) / 256 * 256, b_ids = sizeof(long long) * (size_t)total * topk,
                  b_dist = sizeof(float) * (size_t)total * topk;
     const bool small = batch == total && b_q + b_ids + b_dist <= kSmallIo;   // through the pinned block, as psb_session_search
-    PSB_TRY(ensure_host_io(s, small ? b_q + b_ids + b_dist : 0));
+    PSB_TRY(ensure_host_io(s));
     const long long launches0 = launches_total();
     unsigned long long c0[4] = {0, 0, 0, 0};
     if (stats) PSB_TRY(counters_before(s, st, c0));

@@ -1,0 +1,52 @@
+"""Sessions hand their page-locked block on: many at once, in threads, one after the other, on other streams, with calls that pass their
+queries and results through the block and calls too large for it."""
+import threading
+
+import numpy as np
+import pytest
+
+import oracle
+import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def test_blocks_pass_between_sessions(psb):
+    ix = synth.make_index(4000, 32, 16, 8, seed=5)
+    q = synth.make_queries(ix, 3000, seed=6)
+    want = oracle.ivfpq_search(ix, q, 4, 10, 40)
+    fx = dict(centroids=ix["centroids"], offsets=ix["offsets"], reordered_ids=ix["reordered_ids"], vectors=ix["vectors"])
+    fi, fd = oracle.ivfflat_search(fx["centroids"], fx["offsets"], fx["reordered_ids"], fx["vectors"], q, 4, 10)
+    wrong = []
+
+    def check(s, lo, n, flat):
+        got = s.search(q[lo:lo + n], 4, 10)
+        wi, wd = (fi, fd) if flat else (want["indices"], want["distances"])
+        if not (np.array_equal(got["indices"], wi[lo:lo + n]) and np.array_equal(got["distances"], wd[lo:lo + n])):
+            wrong.append((lo, n, flat))
+
+    def work(t):
+        try:
+            rng = np.random.default_rng(t)
+            for i in range(6):
+                flat = (t + i) % 3 == 0
+                with (psb.FlatSession(fx, max_batch=3000) if flat else psb.Session(ix, n_rerank=40, max_batch=3000)) as s:
+                    for n in (1, 300, 3000 if i == 2 else 7, 1):
+                        check(s, int(rng.integers(0, 3001 - n)), n, flat)
+        except Exception as e:  # noqa: BLE001 - reported by the test below
+            wrong.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
+    held = [psb.Session(ix, n_rerank=40, max_batch=64) for _ in range(12)]   # more than are kept between sessions
+    for i, s in enumerate(held):
+        check(s, i * 50, 50, False)
+    for s in held:
+        s.close()
+    with psb.Session(ix, n_rerank=40, max_batch=64) as s:
+        check(s, 0, 64, False)
+    assert not wrong, wrong
