@@ -89,8 +89,9 @@ namespace {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool part = false;   // a part of a group's allocation
     ~DevBuf() { release(); }
-    void release() { if (p) cudaFree(p); p = nullptr; bytes = 0; }
+    void release() { if (p && !part) cudaFree(p); p = nullptr; bytes = 0; part = false; }
     psb_status reserve(size_t need) {
         if (need <= bytes) return PSB_OK;
         release();
@@ -101,6 +102,34 @@ struct DevBuf {
     psb_status reserve(size_t need, int, cudaStream_t) { return reserve(need); }   // the signature of PoolBuf
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
+
+// Buffers that a call sizes together, in one allocation: every cudaMalloc above 1 MB takes about 0.35 ms, and a session's first call made
+// up to eight of them in a row.  When one has to grow, all are laid out anew (*moved): none shrinks, contents are not preserved.
+psb_status reserve_together(DevBuf* whole, std::initializer_list<std::pair<DevBuf*, size_t>> want, int = 0, cudaStream_t = nullptr, bool* moved = nullptr) {
+    auto padded = [](size_t n) { return (n + 255) / 256 * 256; };
+    bool grow = false;
+    for (const auto& w : want) grow = grow || w.second > w.first->bytes;
+    if (moved) *moved = grow;
+    if (!grow) return PSB_OK;
+    std::vector<size_t> sizes;
+    size_t total = 0;
+    for (const auto& w : want) {
+        sizes.push_back(std::max(w.second, w.first->bytes));
+        total += padded(sizes.back());
+        w.first->release();
+    }
+    whole->release();
+    PSB_TRY(whole->reserve(total));
+    unsigned char* at = whole->as<unsigned char>();
+    size_t i = 0;
+    for (const auto& w : want) {
+        const size_t n = sizes[i++];
+        if (n == 0) continue;
+        w.first->p = at; w.first->bytes = n; w.first->part = true;
+        at += padded(n);
+    }
+    return PSB_OK;
+}
 
 // Runs at every operator call.  The full property block (cudaGetDeviceProperties) takes milliseconds on some hosts - 10 of the
 // 18 ms of a psb_pq_encode call on 1M rows went there - so two attributes are asked once per device and the SM count is remembered.
@@ -251,6 +280,13 @@ private:
     std::vector<unsigned char*> idle_;
 };
 
+// The pool serves these from what it holds, one by one.
+psb_status reserve_together(PoolBuf*, std::initializer_list<std::pair<PoolBuf*, size_t>> want, int device, cudaStream_t st) {
+    for (const auto& w : want)
+        if (w.second) PSB_TRY(w.first->reserve(w.second, device, st));
+    return PSB_OK;
+}
+
 // Persistent fork-join pool of host threads for the staged rerank transport (the reference keeps a persistent rerank pool
 // too: src/search/ivf_common/ivf_host_rerank.cpp:42-51).  run(job) calls job(t) on every thread t and returns when all are done.
 class HostPool {
@@ -360,28 +396,19 @@ struct TcIndexBuffers {
 // Per-batch buffers of the tensor-core coarse filter.
 template <typename Buf>
 struct TcWorkBuffers {
-    Buf qb, qnorm, gmin, seltop, selids, cand_cnt, cand, fail_list, scalars, fail_list2, retry_qb, retry_qnorm;
+    Buf whole, qb, qnorm, gmin, seltop, selids, cand_cnt, cand, fail_list, scalars, fail_list2, retry_qb, retry_qnorm;
     // own_queries: qb and qnorm are needed (not when the caller keeps prepared rows); bounded: rows come with a previous assignment
     // (launch_coarse_tc_assign), which needs group minima for the rows it searches again only.
     psb_status ensure(int nq, int nlist, int dim, int nprobe, int device, cudaStream_t st, bool own_queries = true, bool bounded = false) {
         const int dimp = coarse_tc_padded_dim(dim);
         const int groups = coarse_tc_tiles(nlist) * (256 / coarse_tc_group(nlist, nprobe));
-        if (own_queries) {
-            PSB_TRY(qb.reserve((size_t)2 * nq * dimp, device, st));
-            PSB_TRY(qnorm.reserve(sizeof(float) * 2 * (size_t)nq, device, st));
-        }
-        const int retry = std::min(nq, coarse_tc_retry_rows());
-        PSB_TRY(gmin.reserve(sizeof(float) * (size_t)coarse_tc_pitch(bounded ? retry : nq) * groups, device, st));
-        if (bounded) {
-            PSB_TRY(fail_list2.reserve(sizeof(int) * (size_t)nq, device, st));
-            PSB_TRY(retry_qb.reserve((size_t)2 * retry * dimp, device, st));
-            PSB_TRY(retry_qnorm.reserve(sizeof(float) * 2 * (size_t)retry, device, st));
-        }
-        PSB_TRY(seltop.reserve(sizeof(float) * (size_t)nq * nprobe, device, st));
-        if (nprobe > 1) PSB_TRY(selids.reserve(sizeof(int) * (size_t)nq * nprobe, device, st));
-        PSB_TRY(cand_cnt.reserve(sizeof(int) * (size_t)nq, device, st));
-        PSB_TRY(cand.reserve(sizeof(int) * (size_t)nq * (nprobe == 1 ? coarse_tc_list_cap() : coarse_tc_mask_words(nlist)), device, st));
-        PSB_TRY(fail_list.reserve(sizeof(int) * (size_t)nq, device, st));
+        const size_t n = (size_t)nq, own = own_queries ? n : 0, retry = bounded ? (size_t)std::min(nq, coarse_tc_retry_rows()) : 0;
+        PSB_TRY(reserve_together(&whole, {{&qb, 2 * own * dimp}, {&qnorm, sizeof(float) * 2 * own},
+                                          {&gmin, sizeof(float) * (size_t)coarse_tc_pitch(bounded ? (int)retry : nq) * groups},
+                                          {&fail_list2, bounded ? sizeof(int) * n : 0}, {&retry_qb, 2 * retry * dimp}, {&retry_qnorm, sizeof(float) * 2 * retry},
+                                          {&seltop, sizeof(float) * n * nprobe}, {&selids, nprobe > 1 ? sizeof(int) * n * nprobe : 0}, {&cand_cnt, sizeof(int) * n},
+                                          {&cand, sizeof(int) * n * (nprobe == 1 ? coarse_tc_list_cap() : coarse_tc_mask_words(nlist))},
+                                          {&fail_list, sizeof(int) * n}}, device, st));
         if (!scalars.p) {
             PSB_TRY(scalars.reserve(sizeof(int) * 8, device, st));
             PSB_CUDA(cudaMemsetAsync(scalars.p, 0, sizeof(int) * 8, st));
@@ -467,7 +494,7 @@ struct psb_session {
     // Rows of a large batch cross to the device once each: the slot of every row held here, the rows by slot, the number of slots and
     // where each sub-batch's begin (PartMarks).
     DevBuf slot_of, unique, marks;
-    bool slots_dirty = true;             // slot_of is not all -1 (never used, or a batch was left half done)
+    bool slots_dirty = true;             // slot_of is not all -1 (a batch was left half done)
     int* h_unique = nullptr;             // pinned: the slots the host threads fill
     size_t h_unique_count = 0;
     size_t slots = 0;                    // of the batch at work, at most
@@ -477,8 +504,8 @@ struct psb_session {
     cudaStream_t list_stream = nullptr;  // brings the slot lists to the host thread beside the row copies
     std::vector<long long> h_global_begin;  // striped shards: host copy of the slices' first rows
     // workspaces
-    DevBuf q, q_u8, dist_tile, probes, probe_dist, lut, vis_count, vis_off, vis_cursor, item_off, item_off_tc, visitors, q_rows, thr,
-        pool_cnt, pool, fail_list, fallback_partial, scalars, lut_h, lut_scale, cand_rows, cand_dist, cand_count, stage, score, out_rows, out_dist, out_ids;
+    DevBuf q, q_u8, dist_tile, probes, lut, vis_count, vis_off, vis_cursor, item_off, item_off_tc, visitors, q_rows, thr,
+        pool_cnt, pool, fail_list, fallback_partial, scan_whole, call_whole, rows_whole, scalars, lut_h, lut_scale, cand_rows, cand_dist, cand_count, stage, score, out_rows, out_dist, out_ids;
     int ws_scan_queries = 0;        // queries the scan workspace (visitors, pools, cutoffs) currently holds
     long long ws_scan_tables = 0;   // tables the fp16 table buffer currently holds
     int pool_cap = 0;
@@ -699,25 +726,17 @@ psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool
     if (row_form) return PSB_OK;
     const size_t tables = table_count(s, nq, nprobe);
     s->ws_scan_queries = 0; s->ws_scan_tables = 0;  // set again below once every buffer has its size
-    PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
-    PSB_TRY(s->vis_off.reserve(sizeof(int) * ((size_t)s->nlist + 1)));
-    PSB_TRY(s->vis_cursor.reserve(sizeof(int) * (size_t)s->nlist));
-    PSB_TRY(s->item_off.reserve(sizeof(long long) * ((size_t)s->nlist + 1)));
-    PSB_TRY(s->item_off_tc.reserve(sizeof(long long) * ((size_t)s->nlist + 1)));
-    PSB_TRY(s->visitors.reserve(sizeof(int) * (size_t)nq * nprobe));
-    PSB_TRY(s->q_rows.reserve(sizeof(long long) * (size_t)nq));
-    PSB_TRY(s->thr.reserve(sizeof(float) * (size_t)nq));
-    PSB_TRY(s->pool_cnt.reserve(sizeof(int) * (size_t)nq));
     const int cap = pool_capacity(stage1_k);
-    PSB_TRY(s->pool.reserve(sizeof(uint64_t) * (size_t)nq * cap));
-    s->pool_cap = cap;
-    PSB_TRY(s->fail_list.reserve(sizeof(int) * (size_t)nq));
-    PSB_TRY(s->fallback_partial.reserve(fallback_partial_bytes(stage1_k)));
     const bool half_tables = s->opt.scan_mode != 1 && !residual_table_free(s, stage1_k);
-    if (half_tables) {
-        PSB_TRY(s->lut_h.reserve(sizeof(unsigned short) * tables * s->m * s->k));
-        PSB_TRY(s->lut_scale.reserve(sizeof(float) * tables));
-    }
+    const size_t n = (size_t)nq, nl = (size_t)s->nlist;
+    PSB_TRY(reserve_together(&s->scan_whole, {{&s->vis_count, sizeof(int) * nl}, {&s->vis_off, sizeof(int) * (nl + 1)}, {&s->vis_cursor, sizeof(int) * nl},
+                                              {&s->item_off, sizeof(long long) * (nl + 1)}, {&s->item_off_tc, sizeof(long long) * (nl + 1)},
+                                              {&s->visitors, sizeof(int) * n * nprobe}, {&s->q_rows, sizeof(long long) * n}, {&s->thr, sizeof(float) * n},
+                                              {&s->pool_cnt, sizeof(int) * n}, {&s->pool, sizeof(uint64_t) * n * cap}, {&s->fail_list, sizeof(int) * n},
+                                              {&s->fallback_partial, fallback_partial_bytes(stage1_k)},
+                                              {&s->lut_h, half_tables ? sizeof(unsigned short) * tables * s->m * s->k : 0},
+                                              {&s->lut_scale, half_tables ? sizeof(float) * tables : 0}}));
+    s->pool_cap = cap;
     // what the buffers hold now (reserve() keeps a larger buffer from an earlier call)
     s->ws_scan_queries = (int)std::min<size_t>({s->q_rows.bytes / sizeof(long long), s->thr.bytes / sizeof(float),
                                                 s->pool_cnt.bytes / sizeof(int), s->fail_list.bytes / sizeof(int),
@@ -761,16 +780,13 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, con
 
 psb_status ensure_pipeline_ws(psb_session* s, int nq, int nprobe, int topk, int stage1_k) {
     const int sb = sub_batch_rows(s, nq, nprobe, overlap_enabled(s, nq, rerank_enabled(s, topk)));
-    PSB_TRY(s->q.reserve(sizeof(float) * (size_t)nq * s->dim));
-    PSB_TRY(s->probes.reserve(sizeof(int) * (size_t)nq * nprobe));
-    PSB_TRY(s->probe_dist.reserve(sizeof(float) * (size_t)nq * nprobe));
+    const size_t n = (size_t)nq;
+    PSB_TRY(reserve_together(&s->call_whole, {{&s->q, sizeof(float) * n * s->dim}, {&s->probes, sizeof(int) * n * nprobe},
+                                              {&s->cand_rows, sizeof(int) * n * stage1_k},
+                                              {&s->cand_dist, sizeof(float) * n * stage1_k}, {&s->cand_count, sizeof(int) * n},
+                                              {&s->out_rows, sizeof(int) * n * topk}, {&s->out_dist, sizeof(float) * n * topk},
+                                              {&s->out_ids, sizeof(long long) * n * topk}}));
     if (!residual_table_free(s, stage1_k) && !rows_form(s, sb, nprobe)) PSB_TRY(s->lut.reserve(sizeof(float) * table_count(s, sb, nprobe) * s->m * s->k));
-    PSB_TRY(s->cand_rows.reserve(sizeof(int) * (size_t)nq * stage1_k));
-    PSB_TRY(s->cand_dist.reserve(sizeof(float) * (size_t)nq * stage1_k));
-    PSB_TRY(s->cand_count.reserve(sizeof(int) * (size_t)nq));
-    PSB_TRY(s->out_rows.reserve(sizeof(int) * (size_t)nq * topk));
-    PSB_TRY(s->out_dist.reserve(sizeof(float) * (size_t)nq * topk));
-    PSB_TRY(s->out_ids.reserve(sizeof(long long) * (size_t)nq * topk));
     return ensure_scan_ws(s, sb, nprobe, stage1_k, rows_form(s, sb, nprobe));  // the scan runs one sub-batch at a time
 }
 
@@ -919,12 +935,11 @@ psb_status rows_begin(psb_session* s, long long requests, size_t parts, cudaStre
     const size_t slots = (size_t)std::max<long long>(1, std::min(requests, s->exact_count));
     s->slots = slots;
     s->parts = parts;
-    PSB_TRY(s->unique.reserve(sizeof(int) * slots));
-    PSB_TRY(s->marks.reserve(sizeof(int) * PartMarks::device_words(parts)));
-    PSB_TRY(s->stage.reserve(slots * s->dim * s->exact_elem));
-    const bool fresh = s->slot_of.p == nullptr;
-    PSB_TRY(s->slot_of.reserve(sizeof(int) * (size_t)std::max<long long>(1, s->exact_count)));
-    if (fresh || s->slots_dirty) PSB_CUDA(cudaMemsetAsync(s->slot_of.p, 0xff, s->slot_of.bytes, st));
+    bool moved = false;
+    PSB_TRY(reserve_together(&s->rows_whole, {{&s->unique, sizeof(int) * slots}, {&s->marks, sizeof(int) * PartMarks::device_words(parts)},
+                                              {&s->stage, slots * s->dim * s->exact_elem},
+                                              {&s->slot_of, sizeof(int) * (size_t)std::max<long long>(1, s->exact_count)}}, 0, nullptr, &moved));
+    if (moved || s->slots_dirty) PSB_CUDA(cudaMemsetAsync(s->slot_of.p, 0xff, s->slot_of.bytes, st));
     s->slots_dirty = true;
     PSB_CUDA(cudaMemsetAsync(s->marks.p, 0, sizeof(int) * PartMarks::device_words(parts), st));
     return PSB_OK;

@@ -50,3 +50,19 @@ def test_blocks_pass_between_sessions(psb):
     with psb.Session(ix, n_rerank=40, max_batch=64) as s:
         check(s, 0, 64, False)
     assert not wrong, wrong
+
+
+@pytest.mark.parametrize("mode", [0, 1, 4])       # mapped, staged, hybrid
+@pytest.mark.parametrize("scan_mode", [0, 2, 3])
+@pytest.mark.parametrize("residual", [False, True])
+def test_workspaces_follow_the_calls(psb, mode, scan_mode, residual):
+    """One session, calls that grow the buffers of one group at a time - queries, probes, results, candidate widths - and small ones between."""
+    ix = synth.make_index(6000, 32, 1100, 8, seed=15, residual=residual)   # enough lists for the tensor-core coarse filter
+    q = synth.make_queries(ix, 2500, seed=16)
+    search = oracle.ivfrespq_search if residual else oracle.ivfpq_search
+    with psb.Session(ix, n_rerank=60, exact_mode=mode, scan_mode=scan_mode, residual=residual, max_batch=2500) as s:
+        for n, nprobe, k in ((1, 2, 5), (300, 2, 5), (7, 16, 5), (300, 2, 50), (2500, 2, 5), (2500, 16, 50), (3, 16, 50), (1200, 24, 55), (1, 1, 1)):
+            got = s.search(q[:n], nprobe, k)
+            lo = max(0, n - 40)
+            want = search(ix, q[lo:n], nprobe, k, 60)
+            assert np.array_equal(got["indices"][lo:], want["indices"]) and np.array_equal(got["distances"][lo:], want["distances"]), (n, nprobe, k)
