@@ -138,14 +138,7 @@ k_adc_select(const AdcRows g, int buffer) {
 
 template <int M>
 psb_status run_rows(const AdcRows& g, int nq, cudaStream_t s) {
-    // Enough blocks for several per SM, at least one row per thread, at most 4,096 rows behind one table.
-    auto block_of = [&](double visits) {
-        const double want = visits / (g.sm_count * 6.0);
-        int b = kRowsThreads;
-        while (b < 4096 && b < want) b <<= 1;
-        return b;
-    };
-    const int block = block_of((double)nq * g.expected_rows);
+    const int block = adc_rows_block((double)nq * g.expected_rows, g.sm_count);
     const size_t tab = ((size_t)g.m * g.k + g.dim) * sizeof(float);
     if (g.residual) {
         const int chunks = (int)std::max<long long>(1, (g.longest_list + block - 1) / block);

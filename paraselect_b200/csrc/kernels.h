@@ -273,6 +273,12 @@ struct AdcRows {
     int sm_count;
 };
 psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s);
+// Rows behind one table: enough blocks for several per SM, at least one row per thread, at most 4,096 rows.
+inline int adc_rows_block(double visits, int sm_count) {
+    int b = 256;
+    while (b < 4096 && b < visits / (sm_count * 6.0)) b <<= 1;
+    return b;
+}
 
 // ---- IVF-Flat fine scan (flat.cu) ------------------------------------------------------------------------------
 // Exact fp32 distances of every query to the rows of its probed lists (device-resident rows, list-contiguous) and the topk

@@ -75,3 +75,18 @@ def test_row_form_takes_no_list_workspace(psb):
             used.append(before - torch.cuda.mem_get_info()[0])
         assert np.array_equal(got["indices"][:50], want["indices"]) and np.array_equal(got["distances"][:50], want["distances"])
     assert used[1] < 100e6, used
+
+
+@pytest.mark.parametrize("dim,M", [(128, 8), (100, 20), (64, 4)])   # shapes without a tensor-core form
+@pytest.mark.parametrize("mode", [0, 1, 3])                          # mapped, staged, on the device
+def test_both_sides_of_the_line_without_a_filter(psb, dim, M, mode):
+    """Batches from one query to overlapped sub-batches, on both sides of the line between the row form and the lists."""
+    ix = synth.make_index(40000, dim, 32, M, seed=dim, zipf=True)
+    q = synth.make_queries(ix, 2600, seed=12, weights=synth.zipf_weights(32))
+    with psb.Session(ix, n_rerank=80, exact_mode=mode) as s, psb.Session(ix, n_rerank=80, exact_mode=3, scan_mode=1) as ref:
+        for n in (1, 30, 300, 2600):
+            got, want = s.search(q[:n], 24, 10), ref.search(q[:n], 24, 10)
+            assert np.array_equal(got["indices"], want["indices"]) and np.array_equal(got["distances"], want["distances"]), n
+            assert got["stats"]["pq_scanned_codes"] == want["stats"]["pq_scanned_codes"]
+        some = oracle.ivfpq_search(ix, q[2500:], 24, 10, 80)
+    assert np.array_equal(got["indices"][2500:], some["indices"]) and np.array_equal(got["distances"][2500:], some["distances"])
