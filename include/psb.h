@@ -121,7 +121,8 @@ enum {
                                   sub-batch psb_options.zero_copy_pct percent of the rows fetched are gathered by a kernel
                                   over PCIe - on reserve_sms SMs of its own (default 32), which the scan's grid leaves free -
                                   while host threads stage the others through the pinned rings; neither the host cores nor
-                                  the kernel's reads fill the link alone */
+                                  the kernel's reads fill the link alone.  Where no scan runs beside the rerank the kernel
+                                  has the whole GPU and brings all rows, unless zero_copy_pct is given */
 };
 
 /* IVFPQSearchOptions (src/search/ivfpq/ivfpq_search_context.h:31-45) reduced to what this path uses,
@@ -167,7 +168,7 @@ typedef struct psb_options {
        memory and returns, and the call reports PSB_TIMEOUT. */
     int test_wait_limit;
     int test_skip_mma;
-    int zero_copy_pct;  /* PSB_EXACT_HOST_HYBRID: share of each sub-batch gathered by the kernel, 1..100 (0 = 45) */
+    int zero_copy_pct;  /* PSB_EXACT_HOST_HYBRID: share of each sub-batch gathered by the kernel, 1..100 (0 = 45 beside a scan, else 100) */
     /* Residual mode, optional: the per-row correction asset of the index, value[row] = |recon(row)|^2 + 2 <centroid[list(row)],
        recon(row)> (src/common/row_correction.h:37-45), as HOST arrays over the rows of the view - either fp32 or the affine u16
        form (value = rc_offset + rc_scale * u16, src/common/row_correction.h:7-20).  The residual cutoff estimate reads it;

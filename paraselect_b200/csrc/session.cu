@@ -884,7 +884,12 @@ psb_status validate_params(const psb_session* s, const psb_query_batch_view* qv,
     return PSB_OK;
 }
 
-constexpr long long kClaimRequests = 65536;   // candidates from which a batch's rows are fetched once each
+// Candidates from which a batch's rows are fetched once each.  Claiming them and fetching with 16-byte loads beside one another costs 10 to
+// 17 us more of launches; scoring in place reads every request, in order, over the link.  In place against claimed, whole search, us: 2,000
+// requests 82 / 91 (u8, dim 100) and 111 / 127 (fp32, dim 96), 8,000 119 / 98 and 246 / 246, 16,000 171 / 105 and 415 / 377, 65,000 544 / 186
+// and 1,168 / 886.  Where host threads bring a share, handing the work to them comes on top, 50 us for rows of 100 bytes and 2 ms for rows
+// of 512: the lines lie at 25,000 and 500,000 requests (measured with nothing beside them), this one between.
+constexpr long long kClaimRequests = 8192, kClaimRequestsThreads = 65536;
 
 // Staged rerank transport: host threads gather exact rows into two pinned buffers, and cudaMemcpyAsync moves each filled buffer
 // while the other is being filled.  h_rows: the rows of `count` consecutive slots; d_stage: the first slot's place; copies are queued
@@ -1017,15 +1022,21 @@ psb_status ensure_zc_stream(psb_session* s) {
     return PSB_OK;
 }
 
-// The host threads' share of the rows, in percent.
-int host_share(const psb_session* s) {
+// The host threads' share of the rows, in percent.  The hybrid transport's threads pay beside a scan, which leaves the kernel few SMs; with
+// all of them the kernel alone is faster at every size (serial search, 130,000 to 2 million requests: 1.5 - 11.6 ms against 5.4 - 16.2 for
+// fp32 rows of dim 96, 0.16 - 1.1 against 0.23 - 1.2 for u8 rows of dim 100), so it brings all rows there unless the caller names a share.
+int host_share(const psb_session* s, bool beside) {
     if (s->opt.exact_mode == PSB_EXACT_HOST_STAGED || !s->exact_dev) return 100;
-    return s->opt.exact_mode == PSB_EXACT_HOST_HYBRID ? 100 - (s->opt.zero_copy_pct > 0 ? s->opt.zero_copy_pct : 45) : 0;
+    if (s->opt.exact_mode != PSB_EXACT_HOST_HYBRID) return 0;
+    if (s->opt.zero_copy_pct > 0) return 100 - s->opt.zero_copy_pct;
+    return beside ? 55 : 0;
 }
 bool device_rows(const psb_session* s) { return s->opt.exact_mode == PSB_EXACT_RESIDENT || s->opt.exact_mode == PSB_EXACT_HOST_CACHED; }
 // Rows scored where they lie: in device memory, or so few that fetching each once would not pay for its launches.
-bool rows_in_place(const psb_session* s, long long requests) {
-    return device_rows(s) || (s->exact_dev && s->opt.exact_mode != PSB_EXACT_HOST_STAGED && requests < kClaimRequests);
+bool rows_in_place(const psb_session* s, long long requests, bool beside) {
+    if (device_rows(s)) return true;
+    if (!s->exact_dev || s->opt.exact_mode == PSB_EXACT_HOST_STAGED) return false;
+    return requests < (host_share(s, beside) > 0 ? kClaimRequestsThreads : kClaimRequests);
 }
 
 // Scores and selection of one part, the rows being in place or in their slots.  d_ids_out: original ids instead of rows.
@@ -1048,15 +1059,15 @@ psb_status rerank_impl(psb_session* s, const void* d_queries, int nq, const int*
         PSB_TRY(s->score.reserve(sizeof(float) * (size_t)nq * width));
         score = s->score.as<float>();
     }
-    const bool in_place = rows_in_place(s, (long long)nq * width);
+    const bool beside = s->background || (s->aux_stream != nullptr && s->stream == s->aux_stream);
+    const bool in_place = rows_in_place(s, (long long)nq * width, beside);
     if (!in_place) {
         PSB_TRY(rows_begin(s, (long long)nq * width, 1, s->stream));
         PSB_TRY(rows_claim(s, 0, d_cand, nq, width, stride, d_counts, s->stream));
-        const int host_pct = host_share(s);
+        const int host_pct = host_share(s, beside);
         const int row_bytes = s->dim * s->exact_elem;
         // Beside a scan on the other stream the gather kernel runs on SMs of its own: the ones the scan's persistent grid leaves free
         // (reserve_sms), or gather_ctas lean CTAs spread over all SMs when the caller asks for that.
-        const bool beside = s->background || (s->aux_stream != nullptr && s->stream == s->aux_stream);
         const int owned = beside && s->opt.gather_ctas == 0 ? (s->opt.reserve_sms > 0 ? s->opt.reserve_sms : 8) : 0;
         const int lean = beside ? s->opt.gather_ctas : 0;
         if (host_pct == 0) {
@@ -1678,9 +1689,9 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     std::thread worker;
     // The rows of the whole batch are claimed and fetched once each, sub-batch by sub-batch (a row an earlier sub-batch has fetched is
     // in its slot already), unless they are scored in place.
-    const int host_pct = host_share(s);
+    const int host_pct = host_share(s, true);
     const bool hybrid = staged_overlap && host_pct < 100;
-    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k));
+    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k, true));
     const int row_bytes = s->dim * s->exact_elem;
     if (hybrid) PSB_TRY(ensure_zc_stream(s));
     if (shared_rows) {

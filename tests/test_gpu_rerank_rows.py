@@ -71,3 +71,29 @@ def test_rows_of_whole_units(psb, dim, u8, nq, width):
         masked = np.where(np.arange(width)[None, :] < cnt[:, None], cand, -1)
         wi, wd = oracle.rerank(ix["vectors"], q, masked, 10)
         assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
+
+
+@pytest.mark.parametrize("how", ["alone", "share", "background"])
+@pytest.mark.parametrize("dim,u8,nq,width", [(32, False, 82, 100), (32, False, 81, 101), (100, True, 700, 100), (33, False, 700, 100)])
+def test_hybrid_shares(psb, how, dim, u8, nq, width):
+    """The hybrid transport by the kernel alone, with a share the caller names, and on a stream beside another: on both sides of the lines."""
+    import torch
+    ix = index(1500, dim, u8, dim)
+    rng = np.random.default_rng(nq + dim)
+    with psb.Session(ix, n_rerank=width, exact_mode=4, max_batch=nq, zero_copy_pct=40 if how == "share" else 0) as s:
+        other = torch.cuda.Stream()
+        if how == "background":
+            s.set_stream(other.cuda_stream, background=True)
+        for again in range(2):
+            q = rng.integers(0, 256, (nq, dim)).astype(np.uint8) if u8 else rng.standard_normal((nq, dim)).astype(np.float32)
+            cand = np.stack([rng.permutation(1500)[:width] for _ in range(nq)]).astype(np.int32)
+            dq, dc = torch.from_numpy(q).cuda(), torch.from_numpy(cand).cuda()
+            rows = torch.empty((nq, 10), dtype=torch.int32, device="cuda"); dist = torch.empty((nq, 10), device="cuda")
+            torch.cuda.synchronize()
+            s.stage_rerank(dq, nq, dc, width, width, None, 10, rows, dist)
+            s.sync()
+            torch.cuda.synchronize()
+            wi, wd = oracle.rerank(ix["vectors"], q, cand, 10)
+            assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
+        if how == "background":
+            s.set_stream(None)
