@@ -210,16 +210,19 @@ psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const lo
     return PSB_OK;
 }
 
-bool flat_list_form(int nq, int nprobe, int nlist, int dim) {
-    // From eight visitors per list on, a tile's rows serve enough queries to be worth the schedule's three small kernels; the tile's
-    // rows have to fit.
-    return (long long)nq * nprobe >= 8ll * nlist && small_tile_bytes(dim) <= (size_t)200 * 1024;
+bool flat_list_form(int nq, int nprobe, int nlist, long long rows, int dim) {
+    // The list form's tiles read a list's rows once for 32 visitors: 2.4e-7 us for each dimension of a visited row against 1.0e-6 in the row
+    // form, for 16 to 30 us more of launches.  Both forms at 1 to 32 visitors a list, dim 32 to 128, 20,000 to 300,000 rows: the lines lie
+    // between 3.5e7 and 7e7 dimensions visited - at 3 visitors of 586-row lists (dim 96: 120 us in lists, 131 in rows; 12 visitors 194 and
+    // 386), at 7 of the same lists (dim 32, a quarter of the probes), at 16 of 312-row ones (61 and 78 us at 32).  With one visitor a tile
+    // has no one to share with, whatever the batch visits.  The tile's rows have to fit.
+    return (double)nq * nprobe * rows / nlist * dim >= 6e7 && (long long)nq * nprobe >= 2ll * nlist && small_tile_bytes(dim) <= (size_t)200 * 1024;
 }
 
 psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
     if (f.topk <= 0 || f.topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "flat scan supports topk in 1..2048");
-    const bool lists = flat_list_form(nq, f.nprobe, f.nlist, f.dim);
+    const bool lists = flat_list_form(nq, f.nprobe, f.nlist, f.n_rows, f.dim);
     const long long pairs = (long long)nq * f.nprobe;
     if (lists) PSB_CUDA(cudaMemsetAsync(f.vis_count, 0, sizeof(int) * (size_t)f.nlist, s));
     PSB_TRY(launch_row_segments(f.probes, nq, f.nprobe, f.offsets, 0, f.nlist, f.seg, f.vis_count, lists ? f.slot : nullptr, f.counters, s));

@@ -286,7 +286,8 @@ inline int adc_rows_block(double visits, int sm_count) {
 struct FlatScan {
     const float* queries; int dim;             // [nq][dim]
     const int* probes; int nprobe;             // [nq][nprobe] list ids (outside [0, nlist): skipped)
-    const long long* offsets; int nlist;       // [nlist + 1]
+    const long long* offsets; int nlist;        // [nlist + 1]
+    long long n_rows;                          // of all lists
     const float* rows; const long long* ids;   // [n][dim], [n]
     int topk;
     long long* out_ids; float* out_dist;       // [nq][topk]
@@ -297,7 +298,7 @@ struct FlatScan {
     unsigned long long* counters;
     int sm_count;
 };
-bool flat_list_form(int nq, int nprobe, int nlist, int dim);
+bool flat_list_form(int nq, int nprobe, int nlist, long long rows, int dim);   // rows: of all lists
 psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s);
 
 // ---- rerank ------------------------------------------------------------------------------------------------

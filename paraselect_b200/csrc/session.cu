@@ -2073,14 +2073,14 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     const int parts = (int)((n + most - 1) / most), per = (n + parts - 1) / parts;
     PSB_TRY(s->row_dist.reserve(sizeof(float) * (size_t)per * f.stride));
     PSB_TRY(s->row_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
-    if (flat_list_form(per, nprobe, s->nlist, s->dim)) {
+    if (flat_list_form(per, nprobe, s->nlist, s->n_vectors, s->dim)) {
         PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
         PSB_TRY(s->flat_slot.reserve(sizeof(int) * (size_t)per * nprobe));
         PSB_TRY(s->vis_off.reserve(sizeof(int) * ((size_t)s->nlist + 1)));
         PSB_TRY(s->item_off.reserve(sizeof(long long) * ((size_t)s->nlist + 1)));
         PSB_TRY(s->visitors.reserve(sizeof(int) * (size_t)per * nprobe));
     }
-    f.dim = s->dim; f.nprobe = nprobe; f.offsets = s->offsets.as<long long>(); f.nlist = s->nlist; f.rows = s->flat_rows.as<float>();
+    f.dim = s->dim; f.nprobe = nprobe; f.offsets = s->offsets.as<long long>(); f.nlist = s->nlist; f.n_rows = s->n_vectors; f.rows = s->flat_rows.as<float>();
     f.ids = s->reordered.as<long long>(); f.topk = topk; f.dist = s->row_dist.as<float>(); f.seg = s->row_seg.as<int>();
     f.vis_count = s->vis_count.as<int>(); f.slot = s->flat_slot.as<int>(); f.vis_off = s->vis_off.as<int>(); f.item_off = s->item_off.as<long long>();
     f.visitors = s->visitors.as<int>(); f.counters = s->scalars.as<unsigned long long>(); f.sm_count = s->sm_count;

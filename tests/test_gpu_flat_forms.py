@@ -38,3 +38,24 @@ def test_coarse_small_batches(psb, nq, nlist, dim, k, equal):
     ids, dist = psb.coarse_host(q, c, k, coarse_mode=1)
     wi, wd = oracle.coarse(q, c, k)
     assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+
+
+@pytest.mark.parametrize("n,dim,nlist,nq,nprobe,topk,values", [
+    # enough to visit (6e7 dimensions, two visitors a list) for the list form
+    (3000, 33, 5, 700, 5, 10, "normal"), (3000, 100, 5, 251, 4, 7, "normal"), (4000, 64, 3, 385, 2, 300, "normal"), (9000, 16, 7, 449, 7, 300, "normal"),
+    (6000, 8, 4, 1300, 4, 1100, "normal"), (6000, 8, 4, 1251, 4, 2048, "normal"), (7000, 12, 3, 750, 3, 50, "grid"), (5000, 4, 2, 3200, 2, 20, "equal"),
+    (64, 300, 2, 3300, 2, 5, "normal"), (400, 7, 20, 22000, 20, 64, "normal"), (30000, 2, 4, 1100, 4, 300, "grid"), (30000, 1, 4, 2100, 4, 900, "grid"),
+    # more queries than one part of a call holds, in the row form and in the list form; more than 2^28 distances
+    (40, 7, 20, 33000, 20, 64, "normal"), (300, 16, 4, 33001, 4, 10, "normal"), (600001, 2, 3, 500, 3, 10, "normal")])
+def test_flat_list_form_and_parts(psb, n, dim, nlist, nq, nprobe, topk, values):
+    rng = np.random.default_rng(n + dim + nq)
+    draw = {"normal": lambda *s: rng.standard_normal(s), "grid": lambda *s: rng.integers(-1, 2, s), "equal": lambda *s: np.ones(s)}[values]
+    off = np.concatenate([[0], np.sort(rng.integers(0, n + 1, nlist - 1)), [n]]).astype(np.int64)
+    fx = dict(centroids=rng.standard_normal((nlist, dim)).astype(np.float32), offsets=off, reordered_ids=rng.permutation(n).astype(np.int64),
+              vectors=draw(n, dim).astype(np.float32))
+    q = draw(nq, dim).astype(np.float32)
+    with psb.FlatSession(fx, max_batch=nq) as s:
+        got = s.search(q, nprobe, topk, batch_size=nq)
+    some = np.unique(np.concatenate([np.arange(50), nq // 2 + np.arange(-25, 25), nq - 1 - np.arange(50), rng.integers(0, nq, 100)]))   # part borders among them
+    wi, wd = oracle.ivfflat_search(fx["centroids"], off, fx["reordered_ids"], fx["vectors"], q[some], nprobe, topk)
+    assert np.array_equal(got["indices"][some], wi) and np.array_equal(got["distances"][some], wd)

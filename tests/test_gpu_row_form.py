@@ -90,3 +90,15 @@ def test_both_sides_of_the_line_without_a_filter(psb, dim, M, mode):
             assert got["stats"]["pq_scanned_codes"] == want["stats"]["pq_scanned_codes"]
         some = oracle.ivfpq_search(ix, q[2500:], 24, 10, 80)
     assert np.array_equal(got["indices"][2500:], some["indices"]) and np.array_equal(got["distances"][2500:], some["distances"])
+
+
+@pytest.mark.parametrize("n,nq", [(600, 33000), (300001, 950)])   # more queries than a part holds; more than 2^28 distances
+def test_parts_of_a_call(psb, n, nq):
+    ix = synth.make_index(n, 20, 2, 4, seed=21, residual=True)
+    q = synth.make_queries(ix, nq, seed=22)
+    with psb.Session(ix, n_rerank=20, residual=True, exact_mode=3, serial_pipeline=True, max_batch=nq) as s:
+        got = s.search(q, 2, 10, batch_size=nq)
+    some = np.concatenate([np.arange(30), nq // 2 + np.arange(-15, 15), nq - 1 - np.arange(30)])
+    want = oracle.ivfrespq_search(ix, q[some], 2, 10, 20)
+    assert np.array_equal(got["indices"][some], want["indices"]) and np.array_equal(got["distances"][some], want["distances"])
+    assert got["stats"]["pq_scanned_codes"] == nq * n
