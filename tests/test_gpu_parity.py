@@ -185,18 +185,21 @@ def test_rerank_random_matches_checker(psb, dim):
 
 
 # ---------------------------------------------------------------------------------------------- whole search
+@pytest.mark.parametrize("scan_mode", [0, 2, 3])   # 0: batches this small take the row form
 @pytest.mark.parametrize("name", ["ivfpq_d32_m8", "ivfpq_d96_m48_zipf", "ivfpq_d100_m20"])
 @pytest.mark.parametrize("mode", [0, 1, 4])
-def test_search_matches_reference_golden(psb, name, mode):
+def test_search_matches_reference_golden(psb, name, mode, scan_mode):
+    if scan_mode == 3 and name == "ivfpq_d100_m20":
+        pytest.skip("five dimensions a sub-vector have no tensor-core scan")
     g = cases.load_golden(name)
     nprobe, topk, n_rerank = (int(x) for x in g["params"])
     ix = cases.golden_index(g)
-    with psb.Session(ix, n_rerank=n_rerank, exact_mode=mode) as s:
+    with psb.Session(ix, n_rerank=n_rerank, exact_mode=mode, scan_mode=scan_mode) as s:
         r = s.search(g["queries"], nprobe, topk, batch_size=7, want_coarse=True)  # tail batch on purpose
     assert np.array_equal(r["coarse"], g["ref_probes"])
     assert np.array_equal(r["indices"], g["ref_indices"])
     assert np.array_equal(r["distances"], g["ref_distances"])
-    with psb.Session(dict(ix, vectors=None)) as s:
+    with psb.Session(dict(ix, vectors=None), scan_mode=scan_mode) as s:
         r = s.search(g["queries"], nprobe, topk)
     assert np.array_equal(r["distances"], g["ref_norerank_distances"])
 
@@ -216,12 +219,13 @@ def test_plain_pq_pipeline_equals_exhaustive(psb, m, dim, rerank, empty):
     (80000, 96, 128, 48, 16, 100, 1000, True),  # IVF-PQ 100M sharded configuration, cut down
     (20000, 64, 32, 16, 32, 10, 0, False),      # no rerank: ADC distances out
 ])
-def test_search_matches_checker(psb, n, dim, nlist, M, nprobe, topk, n_rerank, zipf):
+@pytest.mark.parametrize("scan_mode", [0, 3])
+def test_search_matches_checker(psb, n, dim, nlist, M, nprobe, topk, n_rerank, zipf, scan_mode):
     ix = synth.make_index(n, dim, nlist, M, seed=n % 97, zipf=zipf)
     w = synth.zipf_weights(nlist) if zipf else None
     q = synth.make_queries(ix, 64, seed=17, weights=w)
     o = oracle.ivfpq_search(ix if n_rerank else dict(ix, vectors=None), q, nprobe, topk, n_rerank)
-    with psb.Session(ix if n_rerank else dict(ix, vectors=None), n_rerank=n_rerank) as s:
+    with psb.Session(ix if n_rerank else dict(ix, vectors=None), n_rerank=n_rerank, scan_mode=scan_mode) as s:
         r = s.search(q, nprobe, topk, batch_size=50, want_coarse=True)
     assert np.array_equal(r["coarse"], o["coarse"])
     assert np.array_equal(r["indices"], o["indices"])
@@ -407,7 +411,8 @@ def test_half_prefilter_scan_extreme_table_values(psb):
 
 
 # ---------------------------------------------------------------------------------------------- overlapped pipeline
-def test_overlapped_pipeline_equals_serial_pipeline(psb):
+@pytest.mark.parametrize("scan_mode", [0, 3])   # 0: batches this small take the row form; 3: the tensor-core scan, its tables and pools beside a transfer
+def test_overlapped_pipeline_equals_serial_pipeline(psb, scan_mode):
     """Batches of >= 2048 queries run as sub-batches whose rerank overlaps the next scan on a second stream; results
     must equal the serial pipeline's and the checker's."""
     torch = _torch()
@@ -415,7 +420,7 @@ def test_overlapped_pipeline_equals_serial_pipeline(psb):
     q = synth.make_queries(ix, 2600, seed=62, weights=synth.zipf_weights(64))
     res = {}
     for serial in (False, True):
-        with psb.Session(ix, n_rerank=120, serial_pipeline=serial) as s:
+        with psb.Session(ix, n_rerank=120, serial_pipeline=serial, scan_mode=scan_mode) as s:
             res[serial] = s.search(q, 8, 10, batch_size=2600, want_coarse=True)
     for k in ("indices", "distances", "coarse"):
         assert np.array_equal(res[False][k], res[True][k])
@@ -423,7 +428,7 @@ def test_overlapped_pipeline_equals_serial_pipeline(psb):
     assert np.array_equal(res[False]["indices"][:200], want["indices"])
     assert np.array_equal(res[False]["distances"][:200], want["distances"])
     # device-resident entry point
-    with psb.Session(ix, n_rerank=120, max_batch=2600) as s:
+    with psb.Session(ix, n_rerank=120, max_batch=2600, scan_mode=scan_mode) as s:
         ids = torch.empty((2600, 10), dtype=torch.int64, device="cuda")
         dd = torch.empty((2600, 10), dtype=torch.float32, device="cuda")
         s.search_device(dev(q), 2600, 8, 10, ids, dd)
@@ -432,8 +437,9 @@ def test_overlapped_pipeline_equals_serial_pipeline(psb):
         assert np.array_equal(dd.cpu().numpy(), res[True]["distances"])
 
 
+@pytest.mark.parametrize("scan_mode", [0, 3])
 @pytest.mark.parametrize("residual", [False, True])
-def test_short_tail_batch_after_an_overlapped_batch(psb, residual):
+def test_short_tail_batch_after_an_overlapped_batch(psb, residual, scan_mode):
     """batch_size 2600 with 2600 + 1500 queries: the full batch runs as four overlapped sub-batches of 650, the tail batch
     (below the overlap limit of 2048) runs in one piece of 1500 - larger than any sub-batch before it.  The workspaces
     must follow; results equal the serial pipeline's and the checker's."""
@@ -441,7 +447,7 @@ def test_short_tail_batch_after_an_overlapped_batch(psb, residual):
     q = synth.make_queries(ix, 4100, seed=162, weights=synth.zipf_weights(64))
     res = {}
     for serial in (False, True):
-        with psb.Session(ix, n_rerank=120, serial_pipeline=serial, residual=residual) as s:
+        with psb.Session(ix, n_rerank=120, serial_pipeline=serial, residual=residual, scan_mode=scan_mode) as s:
             res[serial] = s.search(q, 8, 10, batch_size=2600)
     for k in ("indices", "distances"):
         assert np.array_equal(res[False][k], res[True][k])
@@ -469,7 +475,8 @@ def test_knn_exact_short_last_tile(psb):
     assert np.array_equal(rows[:3].cpu().numpy(), want)
 
 
-def test_sharded_step_with_second_stream_equals_search(psb):
+@pytest.mark.parametrize("scan_mode", [0, 3])
+def test_sharded_step_with_second_stream_equals_search(psb, scan_mode):
     """The sharded step on one rank, cut into sub-batches whose exchange half (rerank, id map) runs on a second stream
     through psb_session_set_stream while the next sub-batch scans: same results as the session's own search."""
     torch = _torch()
@@ -480,7 +487,7 @@ def test_sharded_step_with_second_stream_equals_search(psb):
         want = s.search(q, 8, 10, batch_size=700)
     stream = torch.cuda.Stream()
     with torch.cuda.stream(stream):
-        with psb.Session(ix, n_rerank=120, max_batch=700, stream=stream.cuda_stream) as s:
+        with psb.Session(ix, n_rerank=120, max_batch=700, stream=stream.cuda_stream, scan_mode=scan_mode) as s:
             search = ShardedSearch(SessionEngine(s, torch), None, 1, 700, 64, 16, 256, 8, 10, 120, torch, rerank=True, parts=3)
             dq = dev(q)
             for parts in (1, 3, 3):
@@ -490,7 +497,8 @@ def test_sharded_step_with_second_stream_equals_search(psb):
                 assert np.array_equal(dd.cpu().numpy(), want["distances"])
 
 
-def test_staged_transport_overlapped_by_a_host_worker_equals_mapped(psb):
+@pytest.mark.parametrize("scan_mode", [0, 3])
+def test_staged_transport_overlapped_by_a_host_worker_equals_mapped(psb, scan_mode):
     """Host-staged rerank transport: batches of >= 2048 queries hand each sub-batch's candidates to a host worker thread that
     gathers rows into pinned rings while the next sub-batch scans; results must equal the mapped transport's."""
     ix = synth.make_index(60000, 64, 64, 16, seed=81, zipf=True)
@@ -501,7 +509,7 @@ def test_staged_transport_overlapped_by_a_host_worker_equals_mapped(psb):
                      ("hybrid", dict(exact_mode=psb.EXACT_HOST_HYBRID)),
                      ("hybrid_70", dict(exact_mode=psb.EXACT_HOST_HYBRID, zero_copy_pct=70)),
                      ("hybrid_serial", dict(exact_mode=psb.EXACT_HOST_HYBRID, serial_pipeline=True))):
-        with psb.Session(ix, n_rerank=120, **kw) as s:
+        with psb.Session(ix, n_rerank=120, scan_mode=scan_mode, **kw) as s:
             res[name] = s.search(q, 8, 10, batch_size=2600)
             again = s.search(q, 8, 10, batch_size=2600)  # buffers are reused across batches
             assert np.array_equal(again["indices"], res[name]["indices"])

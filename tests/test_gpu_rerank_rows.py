@@ -39,14 +39,15 @@ def test_rows_named_many_times(psb, mode, dim, u8, nq, width):
             assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
 
 
+@pytest.mark.parametrize("scan_mode", [0, 3])
 @pytest.mark.parametrize("mode", [0, 1, 4])
-def test_overlapped_batches_share_rows(psb, mode):
+def test_overlapped_batches_share_rows(psb, mode, scan_mode):
     ix = index(3000, 32, False, 7)
     q = np.random.default_rng(8).standard_normal((2500, 32)).astype(np.float32)
     want = oracle.ivfpq_search(ix, q[:200], 3, 10, 60)
     with psb.Session(ix, n_rerank=60, exact_mode=3) as s:
         ref = s.search(q, 3, 10, batch_size=2500)
-    with psb.Session(ix, n_rerank=60, exact_mode=mode) as s:
+    with psb.Session(ix, n_rerank=60, exact_mode=mode, scan_mode=scan_mode) as s:
         for _ in range(2):
             got = s.search(q, 3, 10, batch_size=2500)
             assert np.array_equal(got["indices"], ref["indices"]) and np.array_equal(got["distances"], ref["distances"])

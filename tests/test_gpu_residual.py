@@ -113,12 +113,13 @@ def test_residual_pq_pipeline_equals_exhaustive(psb, m, dim, rerank):
     (80000, 96, 128, 48, 16, 100, 1000, True),
     (20000, 64, 32, 16, 32, 10, 0, False),       # n_rerank below the floor: candidate width 512
 ])
-def test_residual_search_matches_checker(psb, n, dim, nlist, M, nprobe, topk, n_rerank, zipf):
+@pytest.mark.parametrize("scan_mode", [0, 3])
+def test_residual_search_matches_checker(psb, n, dim, nlist, M, nprobe, topk, n_rerank, zipf, scan_mode):
     ix = synth.make_index(n, dim, nlist, M, seed=n % 97, zipf=zipf, residual=True)
     w = synth.zipf_weights(nlist) if zipf else None
     q = synth.make_queries(ix, 64, seed=17, weights=w)
     o = oracle.ivfrespq_search(ix, q, nprobe, topk, n_rerank)
-    with psb.Session(ix, n_rerank=n_rerank, residual=True) as s:
+    with psb.Session(ix, n_rerank=n_rerank, residual=True, scan_mode=scan_mode) as s:
         r = s.search(q, nprobe, topk, batch_size=50, want_coarse=True)
     assert np.array_equal(r["coarse"], o["coarse"])
     assert np.array_equal(r["indices"], o["indices"])
@@ -126,21 +127,22 @@ def test_residual_search_matches_checker(psb, n, dim, nlist, M, nprobe, topk, n_
     assert r["stats"]["pq_scanned_codes"] == o["scanned"]
 
 
-def test_residual_overlapped_pipeline_and_device_entry(psb):
+@pytest.mark.parametrize("scan_mode", [0, 3])
+def test_residual_overlapped_pipeline_and_device_entry(psb, scan_mode):
     """2600 queries run as sub-batches whose rerank overlaps the next scan; same results as the serial pipeline."""
     torch = _torch()
     ix = synth.make_index(60000, 64, 64, 16, seed=61, zipf=True, residual=True)
     q = synth.make_queries(ix, 2600, seed=62, weights=synth.zipf_weights(64))
     res = {}
     for serial in (False, True):
-        with psb.Session(ix, n_rerank=120, serial_pipeline=serial, residual=True) as s:
+        with psb.Session(ix, n_rerank=120, serial_pipeline=serial, residual=True, scan_mode=scan_mode) as s:
             res[serial] = s.search(q, 8, 10, batch_size=2600, want_coarse=True)
     for k in ("indices", "distances", "coarse"):
         assert np.array_equal(res[False][k], res[True][k])
     want = oracle.ivfrespq_search(ix, q[:200], 8, 10, 120)
     assert np.array_equal(res[False]["indices"][:200], want["indices"])
     assert np.array_equal(res[False]["distances"][:200], want["distances"])
-    with psb.Session(ix, n_rerank=120, max_batch=2600, residual=True) as s:
+    with psb.Session(ix, n_rerank=120, max_batch=2600, residual=True, scan_mode=scan_mode) as s:
         ids = torch.empty((2600, 10), dtype=torch.int64, device="cuda")
         dd = torch.empty((2600, 10), dtype=torch.float32, device="cuda")
         s.search_device(dev(q), 2600, 8, 10, ids, dd)
