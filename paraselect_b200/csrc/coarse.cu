@@ -114,13 +114,13 @@ k_select_rows(const float* __restrict__ dist, int n, int k, int buffer, int* __r
 }  // namespace
 
 psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float* d_centroids, int nlist,
-                                    int dim, float* d_dist, cudaStream_t s) {
+                                    int dim, float* d_dist, int sm_count, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
     dim3 grid((nlist + BC - 1) / BC, (nq + BQ - 1) / BQ);
     // Small tiles while the large ones would leave SMs without one (two waves of small tiles still beat one of large ones), if
     // their rows fit.
     const size_t small = small_tile_bytes(dim);
-    if ((long long)grid.x * grid.y < 148 && small <= (size_t)200 * 1024) {
+    if ((long long)grid.x * grid.y < sm_count && small <= (size_t)200 * 1024) {
         const dim3 g2((nlist + SC - 1) / SC, (nq + SQ - 1) / SQ);
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_coarse_dist_small), small));
         k_coarse_dist_small<<<g2, kSmallThreads, small, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist);
@@ -185,6 +185,8 @@ extern "C" psb_status psb_coarse_search_static(const float* d_queries, int nq, c
     }
     float* tile = g_scratch_ptr[device];
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    PSB_TRY(launch_coarse_dist_exact(d_queries, nq, d_centroids, nlist, dim, tile, st));
+    int sms = 0;
+    PSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    PSB_TRY(launch_coarse_dist_exact(d_queries, nq, d_centroids, nlist, dim, tile, sms, st));
     return launch_select_rows(tile, nq, nlist, nprobe, d_ids, d_dist, st);
 }

@@ -28,7 +28,7 @@ inline int pool_capacity(int stage1_k) {
 // Exact fp32 distance matrix tile: dist[q][c] = sum_d (queries[q][d] - centroids[c][d])^2 evaluated as the
 // sequential non-fused sum.  dist is [nq][nlist].
 psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float* d_centroids, int nlist,
-                                    int dim, float* d_dist, cudaStream_t s);
+                                    int dim, float* d_dist, int sm_count, cudaStream_t s);
 // Per query the k smallest (distance, id) pairs of a [nq][n] distance matrix, sorted ascending.
 psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_ids, float* d_out,
                               cudaStream_t s);
@@ -204,7 +204,7 @@ bool scan_tc_supported(int dim, int m, int k);
 psb_status launch_row_bias(const uint8_t* d_codes, const long long* d_offsets, long long row_base, int list_begin, int list_end,
                            int dim, int m, int k, const float* d_codebook, const float* d_centroids, float* d_out, cudaStream_t s);
 psb_status launch_row_aug(const uint8_t* d_codes, long long rows, int dim, int m, int k, const float* d_codebook, void* d_out,
-                          cudaStream_t s);
+                          int sm_count, cudaStream_t s);
 struct ScanTcLaunch {
     const float* queries; const float* centroids; const float* codebook; const int* probes;
     const void* row_aug;
@@ -224,7 +224,7 @@ struct SelectRescoreLaunch {
     int m, k; bool residual, tree;
     int* out_rows; float* out_dist; int* out_count; int* fail_list; int* n_fail; unsigned long long* counters;
     bool shared_cut = false;
-    int sm_count = 148;
+    int sm_count;
 };
 psb_status launch_select_rescore(const SelectRescoreLaunch& L, int nq, cudaStream_t s);
 
@@ -344,11 +344,11 @@ psb_status launch_widen_ids(const int* d_in, long long n, long long* d_out, cuda
 
 // ---- training ------------------------------------------------------------------------------------------------
 psb_status launch_pq_encode(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
-                            uint8_t* d_codes, cudaStream_t s);
+                            uint8_t* d_codes, int sm_count, cudaStream_t s);
 // The assignment of PQ training's Lloyd iterations: |c|^2 - 2 x.c in fused multiply-adds for sub-vectors of 2, 4 or 8 (else the encoder's
 // arithmetic).
 psb_status launch_pq_assign_train(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
-                                  uint8_t* d_codes, cudaStream_t s);
+                                  uint8_t* d_codes, int sm_count, cudaStream_t s);
 psb_status launch_pq_accumulate(const float* d_data, long long n, int dim, const uint8_t* d_codes, int m, int k,
                                 double* d_sums, int* d_counts, cudaStream_t s);
 // Codewords = sums / counts (no rows: kept); leaves the sums and counts zeroed.

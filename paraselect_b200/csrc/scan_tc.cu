@@ -626,12 +626,12 @@ psb_status launch_row_bias(const uint8_t* d_codes, const long long* d_offsets, l
 }
 
 psb_status launch_row_aug(const uint8_t* d_codes, long long rows, int dim, int m, int k, const float* d_codebook, void* d_out,
-                          cudaStream_t s) {
+                          int sm_count, cudaStream_t s) {
     if (rows <= 0) return PSB_OK;
     const int dsub = dim / m;
     const float cw2 = kBeta * kBeta + scan_tc_eps(dim);
     const size_t smem = (size_t)m * k * sizeof(float);
-    const unsigned grid = (unsigned)std::min<long long>((rows + 255) / 256, 148 * 16);
+    const unsigned grid = (unsigned)std::min<long long>((rows + 255) / 256, (long long)sm_count * 16);
 #define PSB_AUG(D)                                                                                                      \
     do {                                                                                                                \
         if (smem > 32 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_row_aug<D>), smem)); \

@@ -444,7 +444,7 @@ struct psb_session {
     TcIndexBuffers<DevBuf> tc_index;
     TcWorkBuffers<DevBuf> tc_work;
     int device = 0;
-    int sm_count = 148;
+    int sm_count = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaStream_t aux_stream = nullptr;  // second stream of the overlapped pipeline (created on first use)
@@ -831,7 +831,7 @@ psb_status coarse_exact(psb_session* s, const float* d_queries, int nq, int npro
     for (int q0 = 0; q0 < nq; q0 += chunk) {
         const int n = std::min(chunk, nq - q0);
         PSB_TRY(launch_coarse_dist_exact(d_queries + (size_t)q0 * s->dim, n, s->centroids.as<float>(), s->nlist, s->dim,
-                                         s->dist_tile.as<float>(), s->stream));
+                                         s->dist_tile.as<float>(), s->sm_count, s->stream));
         PSB_TRY(launch_select_rows(s->dist_tile.as<float>(), n, s->nlist, nprobe, d_ids + (size_t)q0 * nprobe,
                                    d_dist ? d_dist + (size_t)q0 * nprobe : nullptr, s->stream));
     }
@@ -1216,7 +1216,7 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
     // per-row terms of the tensor-core scan (8 bytes per code row), once per index
     if ((opt.scan_mode == 0 || opt.scan_mode == 3) && s->shard_rows > 0 && scan_tc_supported(s->dim, s->m, s->k)) {
         PSB_TRY(s->row_aug.reserve((size_t)s->shard_rows * 8));
-        PSB_TRY(launch_row_aug(s->codes.as<uint8_t>(), s->shard_rows, s->dim, s->m, s->k, s->codebook.as<float>(), s->row_aug.p, st));
+        PSB_TRY(launch_row_aug(s->codes.as<uint8_t>(), s->shard_rows, s->dim, s->m, s->k, s->codebook.as<float>(), s->row_aug.p, s->sm_count, st));
         if (opt.adc_mode == 1 && opt.row_correction_u16) {  // the caller's row correction, affine u16
             if (!(opt.rc_scale > 0.f)) return fail(PSB_INVALID_ARGUMENT, "row_correction_u16 needs a positive rc_scale");
             PSB_TRY(s->row_bias.reserve(sizeof(uint16_t) * (size_t)s->shard_rows));
@@ -2260,7 +2260,7 @@ psb_status psb_coarse_host(const float* h_queries, int nq, const float* h_centro
         PSB_TRY(tile.reserve(row_bytes * (size_t)chunk));
         for (int q0 = 0; q0 < nq; q0 += chunk) {
             const int n = std::min(chunk, nq - q0);
-            PSB_TRY(launch_coarse_dist_exact(q.as<float>() + (size_t)q0 * dim, n, c.as<float>(), nlist, dim, tile.as<float>(), nullptr));
+            PSB_TRY(launch_coarse_dist_exact(q.as<float>() + (size_t)q0 * dim, n, c.as<float>(), nlist, dim, tile.as<float>(), sms, nullptr));
             PSB_TRY(launch_select_rows(tile.as<float>(), n, nlist, nprobe, ids.as<int>() + (size_t)q0 * nprobe,
                                        dist.as<float>() + (size_t)q0 * nprobe, nullptr));
         }
@@ -2277,7 +2277,8 @@ psb_status psb_knn_exact(const float* d_queries, int nq, const float* d_base, in
     if (k <= 0 || k > n) return fail(PSB_INVALID_ARGUMENT, "k must be in 1..n");
     if (k > kMaxProbe) return fail(PSB_UNSUPPORTED_SHAPE, "k above 4096 is not supported");
     if (n > INT_MAX) return fail(PSB_UNSUPPORTED_SHAPE, "more than 2^31-1 base rows");
-    PSB_TRY(check_device(device));
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // tiles of base rows, each at most 1 GiB of distances, then a merge of the per-tile winners.  A last tile with fewer
     // than k rows is folded into the tile before it, so every tile selects exactly k rows.
@@ -2300,7 +2301,7 @@ psb_status psb_knn_exact(const float* d_queries, int nq, const float* d_base, in
     for (int t = 0; t < tiles; ++t) {
         const long long r0 = spans[(size_t)t].first;
         const int rows = spans[(size_t)t].second;  // >= k: k <= n, and no span is shorter than k unless it is the only one
-        PSB_TRY(launch_coarse_dist_exact(d_queries, nq, d_base + (size_t)r0 * dim, rows, dim, dist.as<float>(), st));
+        PSB_TRY(launch_coarse_dist_exact(d_queries, nq, d_base + (size_t)r0 * dim, rows, dim, dist.as<float>(), sms, st));
         PSB_TRY(launch_select_rows(dist.as<float>(), nq, rows, k, trows.as<int>() + (size_t)t * nq * k,
                                    tdist.as<float>() + (size_t)t * nq * k, st));
         PSB_TRY(launch_offset_rows(trows.as<int>() + (size_t)t * nq * k, (long long)nq * k, (int)r0, st));
@@ -2366,7 +2367,7 @@ private:
         PSB_TRY(tile_.reserve(row_bytes * (size_t)chunk, device_, st_));
         for (int64_t r0 = 0; r0 < n_; r0 += chunk) {
             const int nn = (int)std::min<int64_t>(chunk, n_ - r0);
-            PSB_TRY(launch_coarse_dist_exact(data_ + (size_t)r0 * dim_, nn, d_centroids, k_, dim_, tile_.as<float>(), st_));
+            PSB_TRY(launch_coarse_dist_exact(data_ + (size_t)r0 * dim_, nn, d_centroids, k_, dim_, tile_.as<float>(), sms_, st_));
             PSB_TRY(launch_select_rows(tile_.as<float>(), nn, k_, 1, d_assign + r0, d_best + r0, st_));
         }
         return PSB_OK;
@@ -2555,7 +2556,8 @@ psb_status psb_pq_train(const float* d_data, int64_t n, int dim, int subvectors,
     if (!d_data || !d_codebook || n <= 0 || dim <= 0 || subvectors <= 0 || dim % subvectors || codebook_size <= 0 ||
         codebook_size > kMaxCodebook || iters < 0)
         return fail(PSB_INVALID_ARGUMENT, "invalid PQ training request");
-    PSB_TRY(check_device(device));
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
     if (n > INT_MAX) return fail(PSB_UNSUPPORTED_SHAPE, "PQ training on more than 2^31-1 rows");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int dsub = dim / subvectors, words = subvectors * codebook_size;
@@ -2617,7 +2619,7 @@ psb_status psb_pq_train(const float* d_data, int64_t n, int dim, int subvectors,
     }
     PSB_TRY(launch_pq_init_rows(d_data, dim, subvectors, codebook_size, d_rows, d_codebook, st));
     for (int it = 0; it < iters; ++it) {
-        PSB_TRY(launch_pq_assign_train(d_data, n, dim, d_codebook, subvectors, codebook_size, codes, st));
+        PSB_TRY(launch_pq_assign_train(d_data, n, dim, d_codebook, subvectors, codebook_size, codes, sms, st));
         PSB_TRY(launch_pq_accumulate(d_data, n, dim, codes, subvectors, codebook_size, sums, counts, st));
         PSB_TRY(launch_pq_update(sums, counts, subvectors, codebook_size, dsub, d_codebook, st));
     }
@@ -2630,8 +2632,9 @@ psb_status psb_pq_encode(const float* d_data, int64_t n, int dim, const float* d
     if (!d_data || !d_codebook || !d_codes || n < 0 || dim <= 0 || subvectors <= 0 || dim % subvectors ||
         codebook_size <= 0 || codebook_size > kMaxCodebook)
         return fail(PSB_INVALID_ARGUMENT, "invalid PQ encode request");
-    PSB_TRY(check_device(device));
-    return launch_pq_encode(d_data, n, dim, d_codebook, subvectors, codebook_size, d_codes, static_cast<cudaStream_t>(stream));
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
+    return launch_pq_encode(d_data, n, dim, d_codebook, subvectors, codebook_size, d_codes, sms, static_cast<cudaStream_t>(stream));
 }
 
 // ---- index-build glue (host) ---------------------------------------------------------------------------------

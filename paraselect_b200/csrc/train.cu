@@ -754,11 +754,11 @@ __global__ void k_gen_normal(uint64_t seed, long long first, long long n, float 
 
 namespace {
 template <int D, bool kTrain = false>
-psb_status run_pq_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, uint8_t* d_codes, cudaStream_t s) {
+psb_status run_pq_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, uint8_t* d_codes, int sm_count, cudaStream_t s) {
     // A CTA walks its sub-quantisers one after the other; with few row blocks they are cut into ranges so that two CTAs per SM
     // have work, down to one sub-quantiser each.
     const long long blocks = (n + kNearRows - 1) / kNearRows;
-    const int ranges = (int)std::max<long long>(1, std::min<long long>(m, (2 * 148 + blocks - 1) / blocks));
+    const int ranges = (int)std::max<long long>(1, std::min<long long>(m, (2ll * sm_count + blocks - 1) / blocks));
     const int per = (m + ranges - 1) / ranges;
     const size_t smem = near_smem<D>(per);
     PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_nearest<D, kTrain>), smem));
@@ -770,22 +770,22 @@ psb_status run_pq_nearest(const float* d_data, long long n, int dim, const float
 }  // namespace
 
 psb_status launch_pq_encode(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
-                            uint8_t* d_codes, cudaStream_t s) {
+                            uint8_t* d_codes, int sm_count, cudaStream_t s) {
     if (n <= 0) return PSB_OK;
     const int dsub = dim / m;
     // Few codewords or long sub-vectors: one by one (the filter pays from about 32 codewords on, and its operands hold 16
     // dimensions at most); m is bounded by the codes a CTA stages.
     if (k > 32 && m <= 192) {
         switch (dsub) {
-            case 2: return run_pq_nearest<2>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 3: return run_pq_nearest<3>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 4: return run_pq_nearest<4>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 5: return run_pq_nearest<5>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 6: return run_pq_nearest<6>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 8: return run_pq_nearest<8>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 10: return run_pq_nearest<10>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 12: return run_pq_nearest<12>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 16: return run_pq_nearest<16>(d_data, n, dim, d_codebook, m, k, d_codes, s);
+            case 2: return run_pq_nearest<2>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 3: return run_pq_nearest<3>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 4: return run_pq_nearest<4>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 5: return run_pq_nearest<5>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 6: return run_pq_nearest<6>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 8: return run_pq_nearest<8>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 10: return run_pq_nearest<10>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 12: return run_pq_nearest<12>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 16: return run_pq_nearest<16>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
             default: break;
         }
     }
@@ -805,17 +805,17 @@ psb_status launch_pq_encode(const float* d_data, long long n, int dim, const flo
 }
 
 psb_status launch_pq_assign_train(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
-                                  uint8_t* d_codes, cudaStream_t s) {
+                                  uint8_t* d_codes, int sm_count, cudaStream_t s) {
     if (n <= 0) return PSB_OK;
     if (k > 32 && m <= 192) {
         switch (dim / m) {
-            case 2: return run_pq_nearest<2, true>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 4: return run_pq_nearest<4, true>(d_data, n, dim, d_codebook, m, k, d_codes, s);
-            case 8: return run_pq_nearest<8, true>(d_data, n, dim, d_codebook, m, k, d_codes, s);
+            case 2: return run_pq_nearest<2, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 4: return run_pq_nearest<4, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 8: return run_pq_nearest<8, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
             default: break;
         }
     }
-    return launch_pq_encode(d_data, n, dim, d_codebook, m, k, d_codes, s);
+    return launch_pq_encode(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
 }
 
 psb_status launch_pq_accumulate(const float* d_data, long long n, int dim, const uint8_t* d_codes, int m, int k,
