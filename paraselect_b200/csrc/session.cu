@@ -86,6 +86,16 @@ psb_status kernel_carveout_max(const void* kernel) {
 
 namespace {
 
+// The library's memory pool of each device (work_pool).
+struct Pools { std::mutex mu; cudaMemPool_t pool[64] = {}; };
+Pools& pools() { static Pools* one = new Pools; return *one; }   // never destroyed: the driver may end first
+// What the pool holds and nobody uses goes back to the device.
+void trim_pool(int device) {
+    if (device < 0 || device >= 64) return;
+    std::lock_guard<std::mutex> lk(pools().mu);
+    if (pools().pool[device]) cudaMemPoolTrimTo(pools().pool[device], 0);
+}
+
 // Device buffer that grows on demand (contents are not preserved).
 struct DevBuf {
     void* p = nullptr;
@@ -96,7 +106,14 @@ struct DevBuf {
     psb_status reserve(size_t need) {
         if (need <= bytes) return PSB_OK;
         release();
-        PSB_CUDA(cudaMalloc(&p, need ? need : 1));
+        cudaError_t e = cudaMalloc(&p, need ? need : 1);
+        int device = 0;
+        if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess) {   // perhaps the pool holds what is missing
+            cudaGetLastError();
+            trim_pool(device);
+            e = cudaMalloc(&p, need ? need : 1);
+        }
+        if (e != cudaSuccess) { p = nullptr; return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__); }
         bytes = need;
         return PSB_OK;
     }
@@ -159,14 +176,13 @@ psb_status check_device(int device, int* sm_count = nullptr) {
 // Work memory of the operators that allocate, run and free within one call (training, one-shot searches): from a memory pool of
 // the library per device, stream-ordered, so that a call pays neither cudaMalloc nor the device synchronisation of cudaFree (about
 // a third of a small training call).  The pool keeps at most kPoolKeep bytes between calls; what is above goes back to the device at
-// the next synchronisation.
+// the next synchronisation, the rest with the last session of the device or when a session finds no memory.
 constexpr unsigned long long kPoolKeep = 1ull << 30;
 psb_status work_pool(int device, cudaMemPool_t* out) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     if (device < 0 || device >= 64) return fail(PSB_UNSUPPORTED_SHAPE, "device ordinal above 63");
-    std::lock_guard<std::mutex> lk(mu);
-    if (!pools[device]) {
+    std::lock_guard<std::mutex> lk(pools().mu);
+    cudaMemPool_t& known = pools().pool[device];
+    if (!known) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -175,9 +191,9 @@ psb_status work_pool(int device, cudaMemPool_t* out) {
         PSB_CUDA(cudaMemPoolCreate(&p, &props));
         unsigned long long keep = kPoolKeep;
         PSB_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
-        pools[device] = p;
+        known = p;
     }
-    *out = pools[device];
+    *out = known;
     return PSB_OK;
 }
 
@@ -517,6 +533,10 @@ struct psb_session {
     double gemm_ms_total = 0.0;
     long long gemm_launches_total = 0;
 
+    bool counted = false;           // among its device's sessions
+    static std::atomic<int>& sessions(int device) { static std::atomic<int> n[64]; return n[device & 63]; }
+    void count() { counted = true; sessions(device).fetch_add(1); }
+
     psb_session() = default;
     psb_session(const psb_session&) = delete;
     psb_session& operator=(const psb_session&) = delete;
@@ -545,6 +565,7 @@ struct psb_session {
         if (zc_ev_b) cudaEventDestroy(zc_ev_b);
 
         if (own_stream && stream) cudaStreamDestroy(stream);
+        if (counted && sessions(device).fetch_sub(1) == 1) trim_pool(device);
         cudaGetLastError();
     }
 
@@ -1274,6 +1295,7 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
         }
     }
     PSB_CUDA(cudaStreamSynchronize(st));
+    s->count();
     *out = s.release();
     return PSB_OK;
 }
@@ -2046,6 +2068,7 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
     PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
     PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, st));
     PSB_CUDA(cudaStreamSynchronize(st));
+    s->count();
     *out = s.release();
     return PSB_OK;
 }

@@ -66,3 +66,23 @@ def test_workspaces_follow_the_calls(psb, mode, scan_mode, residual):
             lo = max(0, n - 40)
             want = search(ix, q[lo:n], nprobe, k, 60)
             assert np.array_equal(got["indices"][lo:], want["indices"]) and np.array_equal(got["distances"][lo:], want["distances"]), (n, nprobe, k)
+
+
+def test_pool_goes_back_with_the_last_session(psb):
+    """Training keeps its work memory in the library's pool; the last session of the device to end gives it back."""
+    import torch
+    ix = synth.make_index(2000, 32, 16, 8, seed=5)
+    rows = torch.randn(600_000, 128, device="cuda")
+    cen = rows[:1024].clone()
+    assign = torch.empty(600_000, dtype=torch.int32, device="cuda")
+    with psb.Session(ix, n_rerank=40, max_batch=64) as first:
+        first.search(ix["vectors"][:1], 4, 10)
+        second = psb.Session(ix, n_rerank=40, max_batch=64)
+        psb.kmeans_train(rows, 600_000, 128, cen, 1024, 2, assign)
+        torch.cuda.synchronize()
+        kept = torch.cuda.mem_get_info()[0]
+        second.close()
+        assert abs(torch.cuda.mem_get_info()[0] - kept) < 32e6    # another session is there: the pool stays
+    assert torch.cuda.mem_get_info()[0] - kept > 100e6             # 154 MB of operands alone
+    psb.kmeans_train(rows, 600_000, 128, cen, 1024, 1, assign)     # and is taken anew
+    torch.cuda.synchronize()
