@@ -329,7 +329,7 @@ def main():
     ap.add_argument("--exact-mode", default="auto", choices=["auto", "mapped", "staged", "cached", "hybrid"],
                     help="rerank transport on one GPU: staged = host threads gather rows into pinned rings and cudaMemcpyAsync moves "
                          "them (no SM time spent on the transfer), mapped = kernels gather mapped host rows over PCIe; "
-                         "auto = hybrid when a batch gathers at least 2 GB (the scan is then long enough to run beside the transfer), else mapped; "
+                         "auto = hybrid when a batch asks for at least 2 GB of rows (the scan is then long enough to run beside the transfer), else mapped; "
                          "cached = the session copies the rows into device memory once (not the host-resident configuration the "
                          "headline metric names: an extra data point); hybrid = staged and mapped at once, --zero-copy-pct of every "
                          "sub-batch through the kernel")
@@ -514,6 +514,8 @@ def main():
                   recall_at_k_cpu=recall_at(ref["indices"][:gtn], gt_ids[:gtn], topk) if gtn else None,
                   recall_at_10_gpu=recall_at(e2e_ids[:gtn], gt_ids[:gtn], min(10, topk)) if gtn else None,
                   recall_at_10_cpu=recall_at(ref["indices"][:gtn], gt_ids[:gtn], min(10, topk)) if gtn else None)
+    host_pct = dict(staged=100, hybrid=100 - (args.zero_copy_pct or 45)).get(args.exact_mode, 0)   # the host threads' share of the rows
+    fetched = int(c["staged_gather_bytes"] / max(1, args.steps) * 100 / host_pct) or None if host_pct and R > topk else None
     line = dict(
         metric="QPS (IVF-PQ search, recall@k equal to the reference CPU path)", value=round(nq / (ms_dev * 1e-3), 1),
         unit="queries/s", n_gpus=1, steps=args.steps, warmup=max(args.warmup, 3), ms_per_step=round(ms_dev, 3),
@@ -523,13 +525,14 @@ def main():
                     l2="inputs larger than L2 (codes %.1f GB)" % (index["codes"].nbytes / 1e9)),
         e2e=dict(value=round(nq / (ms_e2e * 1e-3), 1), unit="queries/s", ms_per_step=round(ms_e2e, 3),
                  h2d_bytes_per_step=int(stats["h2d_bytes"]), d2h_bytes_per_step=int(stats["d2h_bytes"]),
-                 pcie_gather_bytes_per_step=int(nq * stage1 * dim * 4) if R > topk else 0),
+                 requested_row_bytes_per_step=int(nq * stage1 * dim * 4) if R > topk else 0),
         gpu_launches=launches, roofline=roofline,
-        # the exact rerank moves nq * n_rerank rows from host memory per batch: what the end-to-end step is bound by
-        transport=dict(bytes_per_step=int(nq * stage1 * dim * 4) if R > topk else 0,
-                       achieved_gbs=round(nq * stage1 * dim * 4 / max(1e-9, stats["pq_rerank_ms"] * 1e-3) / 1e9, 1) if R > topk and stats["pq_rerank_ms"] > 0 else None,
-                       pinned_h2d_copy_gbs=h2d_gbs, note="achieved = gathered bytes / rerank stage time (random rows of dim * 4 bytes); "
-                       "pinned_h2d_copy_gbs = one large pinned copy on this host, the link's ceiling"),
+        # the exact rerank asks for nq * n_rerank rows of host memory per batch and fetches each distinct one once: what the
+        # end-to-end step is bound by
+        transport=dict(requested_bytes_per_step=int(nq * stage1 * dim * 4) if R > topk else 0, fetched_bytes_per_step=fetched,
+                       achieved_gbs=round(fetched / max(1e-9, stats["pq_rerank_ms"] * 1e-3) / 1e9, 1) if fetched and stats["pq_rerank_ms"] > 0 else None,
+                       pinned_h2d_copy_gbs=h2d_gbs, note="fetched = distinct rows, from the host threads' share (none in the mapped transport); achieved = "
+                       "fetched bytes / rerank stage time (random rows of dim * 4 bytes); pinned_h2d_copy_gbs = one large pinned copy on this host, the link's ceiling"),
         cpu_baseline=dict(value=round(ns / dt, 2), unit="queries/s", cores=cores, kind=kind,
                           sample="first %d queries of the batch, all %d host threads" % (ns, cores)),
         stages_ms=dict(coarse=round(stats["coarse_search_ms"], 3), lut=round(stats["pq_lut_build_ms"], 3),
@@ -709,7 +712,7 @@ def multi_gpu_main(args, cfg, rank, world, local_rank):
                         l2="inputs larger than L2 (codes %.2f GB per rank)" % (index["codes"].nbytes / 1e9)),
             e2e=dict(value=round(nq / (ms_e2e * 1e-3), 1), unit="queries/s", ms_per_step=round(ms_e2e, 3),
                      h2d_bytes_per_step=int(nq * dim * 4), d2h_bytes_per_step=int(nq * topk * 12),
-                     pcie_gather_bytes_per_step=int(nq * width * dim * 4) if R > topk else 0),
+                     requested_row_bytes_per_step=int(nq * width * dim * 4) if R > topk else 0),
             gpu_launches=int(tot[3].item()),
             roofline=roofline,
             counters=dict(scanned_codes_per_step=int(S * launches_per_step), fallback_queries_per_step=tot[4].item() / max(1, args.steps),
