@@ -313,7 +313,7 @@ k_seed_threshold(const float* __restrict__ lut, const int* __restrict__ probes, 
     float* s_pk = reinterpret_cast<float*>(s_pref + nprobe + 1);  // [nprobe] |q - c|^2 per probe (flat_bias only)
     if (!per_probe) {
         const float* src = lut + (size_t)q * m * k;
-        if (((m * k) & 3) == 0) {
+        if (((m * k) & 3) == 0 && (reinterpret_cast<uintptr_t>(lut) & 15) == 0) {   // a caller's tables may start at any float
 #pragma unroll 4
             for (int e = threadIdx.x; e < m * k / 4; e += kSeedThreads) reinterpret_cast<float4*>(s_lut)[e] = __ldg(reinterpret_cast<const float4*>(src) + e);
         } else {

@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(T) k_select_rescore(const RescoreArgs g) {
     if (need < 0) return;
     const int mk = g.m * g.k;
     const float* lut = g.lut + (size_t)q * mk;
-    if ((mk & 3) == 0) {
+    if ((mk & 3) == 0 && (reinterpret_cast<uintptr_t>(g.lut) & 15) == 0) {   // a caller's tables may start at any float
 #pragma unroll 4
         for (int e = threadIdx.x; e < mk / 4; e += T) reinterpret_cast<float4*>(s_tab)[e] = __ldg(reinterpret_cast<const float4*>(lut) + e);
     } else {

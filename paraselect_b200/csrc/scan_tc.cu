@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
             if (!__all_sync(0xffffffffu, wait_or_abort(&a_empty[aslot], ((n / NA) & 1u) ^ 1u, abort_flag, limit))) { failed = true; break; }
             const float* cen = g.centroids + (size_t)d.list * g.dim;  // residual mode: the list's centroid (read through L1/L2)
             if (tid < 2 * TV) {  // query tile: two threads per visitor row
+                const bool qvec = (reinterpret_cast<uintptr_t>(g.queries) & 15) == 0;
                 const int i = tid >> 1, part = tid & 1;
                 unsigned char* arow = s_a + aslot * a_bytes + (size_t)i * 128;
                 const uint32_t axs = (uint32_t)(i & 7) << 4;
@@ -300,8 +301,15 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
                 if (pq >= 0) {
                     const float* qrow = g.queries + (size_t)pq * g.dim;
                     for (int c = part; c < nchunk_data; c += 2) {
-                        float4 x0 = __ldg(reinterpret_cast<const float4*>(qrow + c * 8));
-                        float4 x1 = __ldg(reinterpret_cast<const float4*>(qrow + c * 8 + 4));
+                        float4 x0, x1;
+                        if (qvec) {
+                            x0 = __ldg(reinterpret_cast<const float4*>(qrow + c * 8));
+                            x1 = __ldg(reinterpret_cast<const float4*>(qrow + c * 8 + 4));
+                        } else {   // a caller's queries may start at any float
+                            const float* x = qrow + c * 8;
+                            x0 = make_float4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
+                            x1 = make_float4(__ldg(x + 4), __ldg(x + 5), __ldg(x + 6), __ldg(x + 7));
+                        }
                         if (g.residual) {
                             const float4 c0 = __ldg(reinterpret_cast<const float4*>(cen + c * 8));
                             const float4 c1 = __ldg(reinterpret_cast<const float4*>(cen + c * 8 + 4));
