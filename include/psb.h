@@ -15,6 +15,10 @@
  *   - Distances are squared L2.  Missing results are id -1 / distance FLT_MAX
  *     (src/search/ivf_common/ivf_exact_topk.h:87-90).
  *   - A session serves one caller thread at a time (src/search/ivfrespq/ivfrespq_search.cuh:118-119).
+ *   - Memory: a session keeps its workspaces (sized for the largest call so far; up to 1 GiB of them are distances, in the scan's row
+ *     form and in IVF-Flat) until it is destroyed.  Operators without a session work in a pool of the library per device, which keeps at
+ *     most 1 GiB between calls until the device's last session is destroyed, a session finds no memory, or the process ends.  Up to eight
+ *     page-locked blocks of 260 KiB go from session to session and stay with the process.
  *   - There is no CPU fallback: every compute entry point fails with PSB_NO_DEVICE when no sm_100 GPU
  *     is usable.
  */
@@ -110,7 +114,9 @@ typedef struct psb_index_view {
 
 /* How the exact rows reach the GPU during the rerank. */
 enum {
-    PSB_EXACT_HOST_MAPPED = 0, /* register (pin + map) the caller's host rows once; kernels gather rows over PCIe */
+    PSB_EXACT_HOST_MAPPED = 0, /* register (pin + map) the caller's host rows once; kernels gather rows over PCIe.  Sessions over the same
+                                  rows, or over a part of them, share the mapping, which ends with the last of them; rows that overlap
+                                  mapped ones without lying inside them are refused */
     PSB_EXACT_HOST_STAGED = 1, /* host threads gather rows into pinned rings, cudaMemcpyAsync overlaps the copies */
     PSB_EXACT_RESIDENT = 2,    /* exact.fp32 / exact.u8 is already a device pointer (IVFExactStorageKind::Resident,
                                   src/search/ivf_common/ivf_storage.h:25-30) */

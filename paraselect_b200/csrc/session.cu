@@ -1665,8 +1665,8 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     const int sb = sub_batch_rows(s, n, nprobe, overlap || staged_overlap);
     const bool residual = s->opt.adc_mode == 1;
     // Sub-batch boundaries.  Equal cuts, except with the overlapped staged transport.  There the transfer costs the scan
-    // nothing and is the longer of the two (3.84 GB per 10,000-query batch at the host's ~30 GB/s of random row reads, against
-    // ~60 ms of scanning), so it should start as early as possible: the first sub-batch is the small one (10/30/30/30 %).
+    // nothing and is the longer of the two (100M x 96, 10,000 queries x 1,000 candidates: 3.1 GB of distinct rows at the
+    // host's ~30 GB/s of random row reads, against ~60 ms of scanning), so it should start as early as possible: the first sub-batch is the small one (10/30/30/30 %).
     std::vector<int> cuts;
     const int plan = s->opt.even_cuts;
     if (staged_overlap && (!residual || residual_table_free(s, stage1_k)) && sb * 4 >= n && n >= 4096 && plan != 1) {

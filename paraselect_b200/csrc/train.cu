@@ -383,7 +383,7 @@ k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* 
 // codeword so far, a draw r in [0, sum), and the first row at which the running sum reaches r.  On one host thread this took 0.5 s
 // for 32,768 rows x 24 sub-quantisers, 98 % of a codebook training.  Here a cluster of eight CTAs holds a sub-quantiser's rows and
 // their distances in shared memory (rows that do not fit are read through L2); a pick is one update of the distances, two cluster
-// barriers and a search in one warp's stretch of rows: 1.5 us, 255 picks, every sub-quantiser on SMs of its own.
+// barriers and a search in one warp's stretch of rows: 5.6 us (32,768 rows, 24 sub-quantisers), 255 picks, every sub-quantiser on SMs of its own.
 // The draws are made by the host (they do not depend on the data).  The rows picked are the reference's: its sequential sum and the
 // tree sum used here each stay within (n + 64) 2^-53 of the exact one, so when r is further than three times that from the
 // borders of the row found, the sequential search finds the same row; when it is not (about one draw in a million), one thread
