@@ -339,8 +339,8 @@ psb_status psb_stage_scan(psb_session* session, const float* d_lut, int nq, cons
  * query vectors besides their tables, or, for a small batch, score every row without a filter.  Same results as psb_stage_scan:
  * whichever form runs, distances are sums of entries of d_lut, so d_lut has to be the tables of d_queries (a filter that works
  * on the queries would otherwise drop rows by other distances than the tables give).  In residual mode d_lut may be NULL where
- * the tensor-core scan is possible for every list (scan_mode 0 or 3 on a supported shape): no per-(query, probe) table is then
- * materialised at all - the kernels build the entries they need from the query, the centroid and the codebook, with the same
+ * the tensor-core scan is possible for every list (scan_mode 0 or 3 on a supported shape) or where every batch is scored without a
+ * filter (scan_mode 0 on other shapes): no per-(query, probe) table is then materialised at all - the kernels build the entries they need from the query, the centroid and the codebook, with the same
  * rounding. */
 psb_status psb_stage_scan_queries(psb_session* session, const float* d_queries, const float* d_lut, int nq,
                                   const int* d_probes, int nprobe, int stage1_k, int* d_rows, float* d_dist, int* d_count);

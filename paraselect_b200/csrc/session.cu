@@ -673,13 +673,6 @@ bool residual_table_free(const psb_session* s, int stage1_k) {
            (size_t)pool_capacity(stage1_k) * 8 + (size_t)s->dim * 4 <= (size_t)226 * 1024;
 }
 
-// Whether a stage call may leave its tables out: residual mode on a shape the tensor-core scan takes (a shard without rows scans
-// nothing), whichever form the scan then runs in.
-bool tables_optional(const psb_session* s, int stage1_k) {
-    if (residual_table_free(s, stage1_k)) return true;
-    return s->opt.adc_mode == 1 && s->shard_rows == 0 && scan_tc_supported(s->dim, s->m, s->k);
-}
-
 // Tables one scan call needs for nq queries.
 size_t table_count(const psb_session* s, int nq, int nprobe) {
     return s->opt.adc_mode == 1 ? (size_t)nq * nprobe : (size_t)nq;
@@ -736,6 +729,12 @@ bool rows_form(const psb_session* s, int nq, int nprobe, bool any_probes = false
     }
     const double per_query = visits * (4e-6 + 3.2e-7 * s->m) + (residual ? nprobe * (0.008 + 2.3e-4 * s->m) - 0.35 : -0.1);   // us
     return nq * per_query <= (residual ? 170.0 : 130.0);
+}
+
+// Whether a stage call may leave its tables out, whatever the size of its batch: residual mode where the tensor-core scan takes every list,
+// or where the row form takes every batch (shapes without a filter, a shard without rows).
+bool tables_optional(const psb_session* s, int nprobe, int stage1_k) {
+    return residual_table_free(s, stage1_k) || (s->opt.adc_mode == 1 && s->row_aug.p == nullptr && rows_form(s, 1, nprobe, true));
 }
 
 // Queries per sub-batch of the pipeline: a quarter of the batch when the rerank overlaps the scan, and in residual mode
@@ -1448,8 +1447,8 @@ psb_status psb_stage_scan_queries(psb_session* s, const float* d_queries, const 
     if (nq < 0 || nprobe <= 0 || stage1_k <= 0) return fail(PSB_INVALID_ARGUMENT, "nprobe and stage1_k must be positive, nq not negative");
     if (nprobe > kMaxProbe || stage1_k > kMaxStage1) return fail(PSB_UNSUPPORTED_SHAPE, "nprobe above 4096 or stage1_k above 2048");
     if (nq == 0) return PSB_OK;
-    if (!d_lut && !tables_optional(s, stage1_k))
-        return fail(PSB_INVALID_ARGUMENT, "the scan needs the lookup tables (they may be left out only in residual mode with the tensor-core scan)");
+    if (!d_lut && !(d_queries && tables_optional(s, nprobe, stage1_k)))
+        return fail(PSB_INVALID_ARGUMENT, "the scan needs the lookup tables (they may be left out only in residual mode, with the queries at hand)");
     s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
     const bool rows_only = d_queries != nullptr && rows_form(s, nq, nprobe, true);
