@@ -212,11 +212,11 @@ psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const lo
 
 bool flat_list_form(int nq, int nprobe, int nlist, long long rows, int dim) {
     // The list form's tiles read a list's rows once for 32 visitors: 2.4e-7 us for each dimension of a visited row against 1.0e-6 in the row
-    // form, for 16 to 30 us more of launches.  Both forms at 1 to 32 visitors a list, dim 32 to 128, 20,000 to 300,000 rows: the lines lie
-    // between 3.5e7 and 7e7 dimensions visited - at 3 visitors of 586-row lists (dim 96: 120 us in lists, 131 in rows; 12 visitors 194 and
-    // 386), at 7 of the same lists (dim 32, a quarter of the probes), at 16 of 312-row ones (61 and 78 us at 32).  With one visitor a tile
-    // has no one to share with, whatever the batch visits.  The tile's rows have to fit.
-    return (double)nq * nprobe * rows / nlist * dim >= 6e7 && (long long)nq * nprobe >= 2ll * nlist && small_tile_bytes(dim) <= (size_t)200 * 1024;
+    // form, for 16 to 30 us more of launches.  Both forms of 225 drawn batches (dim 32 to 128, 20,000 to 300,000 rows in 64 to 512 lists, 4 to 32
+    // probes, 4 to 1,000 queries): with the line at 4e7 visited dimensions the form taken is on average 0.1 % and at most 7 % slower than the
+    // other, at 2e7 30 %, at 6e7 29, at eight visitors a list 42.  586-row lists of dim 96: 3 visitors 120 us in lists, 131 in rows, 12
+    // visitors 194 and 386.  With one visitor a tile has no one to share with, whatever the batch visits.  The tile's rows have to fit.
+    return (double)nq * nprobe * rows / nlist * dim >= 4e7 && (long long)nq * nprobe >= 2ll * nlist && small_tile_bytes(dim) <= (size_t)200 * 1024;
 }
 
 psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {

@@ -41,7 +41,7 @@ def test_coarse_small_batches(psb, nq, nlist, dim, k, equal):
 
 
 @pytest.mark.parametrize("n,dim,nlist,nq,nprobe,topk,values", [
-    # enough to visit (6e7 dimensions, two visitors a list) for the list form
+    # enough to visit (4e7 dimensions, two visitors a list) for the list form
     (3000, 33, 5, 700, 5, 10, "normal"), (3000, 100, 5, 251, 4, 7, "normal"), (4000, 64, 3, 385, 2, 300, "normal"), (9000, 16, 7, 449, 7, 300, "normal"),
     (6000, 8, 4, 1300, 4, 1100, "normal"), (6000, 8, 4, 1251, 4, 2048, "normal"), (7000, 12, 3, 750, 3, 50, "grid"), (5000, 4, 2, 3200, 2, 20, "equal"),
     (64, 300, 2, 3300, 2, 5, "normal"), (400, 7, 20, 22000, 20, 64, "normal"), (30000, 2, 4, 1100, 4, 300, "grid"), (30000, 1, 4, 2100, 4, 900, "grid"),
