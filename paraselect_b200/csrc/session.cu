@@ -904,12 +904,13 @@ psb_status validate_params(const psb_session* s, const psb_query_batch_view* qv,
     return PSB_OK;
 }
 
-// Candidates from which a batch's rows are fetched once each.  Claiming them and fetching with 16-byte loads beside one another costs 10 to
-// 17 us more of launches; scoring in place reads every request, in order, over the link.  In place against claimed, whole search, us: 2,000
-// requests 82 / 91 (u8, dim 100) and 111 / 127 (fp32, dim 96), 8,000 119 / 98 and 246 / 246, 16,000 171 / 105 and 415 / 377, 65,000 544 / 186
-// and 1,168 / 886.  Where host threads bring a share, handing the work to them comes on top, 50 us for rows of 100 bytes and 2 ms for rows
-// of 512: the lines lie at 25,000 and 500,000 requests (measured with nothing beside them), this one between.
-constexpr long long kClaimRequests = 8192, kClaimRequestsThreads = 65536;
+// Bytes of candidates' rows from which a batch's rows are fetched once each.  Claiming them costs 18 us more of launches and then saves what is
+// asked for more than once, and for rows longer than a line the slower reads of scoring in place.  In place against claimed, whole search, us:
+// 512-byte rows, 8,000 requests 205 / 209, 16,000 342 / 308, 64,000 1,158 / 856; 256-byte ones, 16,000 217 / 217, 64,000 631 / 521; 128-byte
+// ones, 32,000 236 / 246, 64,000 342 / 328, 260,000 1,219 / 898; 32-byte ones, 130,000 313 / 325, 260,000 579 / 485.
+// Where host threads bring a share, handing the work to them costs 2 ms more for long rows: with nothing beside them that pays from 200,000 to
+// 500,000 requests on.  That line counts requests and lies lower, for threads work beside a scan.
+constexpr long long kClaimBytes = 4500000, kClaimBytesShort = 6500000, kClaimRequestsThreads = 65536;
 
 // Staged rerank transport: host threads gather exact rows into two pinned buffers, and cudaMemcpyAsync moves each filled buffer
 // while the other is being filled.  h_rows: the rows of `count` consecutive slots; d_stage: the first slot's place; copies are queued
@@ -1043,8 +1044,8 @@ psb_status ensure_zc_stream(psb_session* s) {
 }
 
 // The host threads' share of the rows, in percent.  The hybrid transport's threads pay beside a scan, which leaves the kernel few SMs; with
-// all of them the kernel alone is faster at every size (serial search, 130,000 to 2 million requests: 1.5 - 11.6 ms against 5.4 - 16.2 for
-// fp32 rows of dim 96, 0.16 - 1.1 against 0.23 - 1.2 for u8 rows of dim 100), so it brings all rows there unless the caller names a share.
+// all of them the kernel alone is faster at every size (serial search, 130,000 to 2 million requests of fp32 rows of dim 96: 1.5 - 11.6
+// ms against 5.4 - 16.2), so it brings all rows there unless the caller names a share.
 int host_share(const psb_session* s, bool beside) {
     if (s->opt.exact_mode == PSB_EXACT_HOST_STAGED || !s->exact_dev) return 100;
     if (s->opt.exact_mode != PSB_EXACT_HOST_HYBRID) return 0;
@@ -1056,7 +1057,9 @@ bool device_rows(const psb_session* s) { return s->opt.exact_mode == PSB_EXACT_R
 bool rows_in_place(const psb_session* s, long long requests, bool beside) {
     if (device_rows(s)) return true;
     if (!s->exact_dev || s->opt.exact_mode == PSB_EXACT_HOST_STAGED) return false;
-    return requests < (host_share(s, beside) > 0 ? kClaimRequestsThreads : kClaimRequests);
+    if (host_share(s, beside) > 0) return requests < kClaimRequestsThreads;
+    const long long row_bytes = (long long)s->dim * s->exact_elem;
+    return requests * row_bytes < (row_bytes <= 128 ? kClaimBytesShort : kClaimBytes);
 }
 
 // Scores and selection of one part, the rows being in place or in their slots.  d_ids_out: original ids instead of rows.

@@ -75,7 +75,7 @@ def test_rows_of_whole_units(psb, dim, u8, nq, width):
 
 
 @pytest.mark.parametrize("how", ["alone", "share", "background"])
-@pytest.mark.parametrize("dim,u8,nq,width", [(32, False, 82, 100), (32, False, 81, 101), (100, True, 700, 100), (33, False, 700, 100)])
+@pytest.mark.parametrize("dim,u8,nq,width", [(32, False, 507, 100), (32, False, 508, 100), (100, True, 700, 100), (33, False, 340, 100), (33, False, 700, 100)])
 def test_hybrid_shares(psb, how, dim, u8, nq, width):
     """The hybrid transport by the kernel alone, with a share the caller names, and on a stream beside another: on both sides of the lines."""
     import torch
