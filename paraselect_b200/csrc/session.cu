@@ -703,11 +703,12 @@ double expected_rows(const psb_session* s, int nprobe) {
 // rows of m = 48 each, 1,200 for m = 8; lists so short that a query's rows cost less than its fixed share stay with the row form.
 // Shapes the filter does not take: in residual mode the row form at any size (0.2 to 0.95 of the list-centric scan's time over twelve
 // shapes of dim 60 to 960, m = 8 to 64, at 1 to 6,000 queries; 1.3 at 32 queries of dim 960).  In plain mode the list-centric scan starts
-// some 40 us later and takes 0.29 us more a query, but less a row (a list's visitors share its codes) and builds one table per query,
-// where the row form builds one per 4,096 rows or fewer - from codewords of other than 2, 4 or 8 elements by scalar loads, whose bank
-// conflicts are the common factor of that length and 32.  Fitted to both forms of 23 such shapes at 1 to 10,000 queries; the form chosen
-// is on average 1 % and at most 21 % slower than the other would have been.  10,000 queries of 31,000 rows each: rows 7.8 ms and lists 3.4 for
-// dim 128, m = 8, 13.2 and 4.5 for dim 256, m = 16; of 14,000 rows, dim 100, m = 20, 2.9 and 3.3.
+// some 40 us later, 0.1 more for a thousand rows a query visits, and takes 0.29 us more a query, but less a row (a list's visitors share
+// its codes) and builds one table per query, where the row form builds one per 4,096 rows or fewer - from codewords of other than 2, 4 or 8
+// elements by scalar loads, whose bank conflicts are the common factor of that length and 32.  Fitted to both forms of 29 such shapes
+// and 168 drawn batches, 1 to 10,000 queries: the form chosen is on average 0.7 % and at most 21 % slower than the other would have been.
+// 10,000 queries of 31,000 rows each: rows 7.8 ms and lists 3.4 for dim 128, m = 8, 13.2 and 4.5 for dim 256, m = 16; of 14,000 rows, dim
+// 100, m = 20, 2.9 and 3.3.
 // any_probes: the caller's own probes, which may name a list more than once.
 long long row_stride(const psb_session* s, int nprobe, bool any_probes) {
     return std::max<long long>(1, any_probes ? s->longest[1] * nprobe : s->longest[(size_t)nprobe]);
@@ -725,7 +726,7 @@ bool rows_form(const psb_session* s, int nq, int nprobe, bool any_probes = false
         const bool wide = dsub == 2 || dsub == 4 || dsub == 8;
         const double tables = wide ? 0.0 : std::max(1.0, std::ceil(visits / adc_rows_block(nq * visits, s->sm_count)));
         const double table = (double)s->dim * s->k * (8e-7 + 7e-8 * std::gcd(dsub, 32));   // us
-        return nq * (visits * (8e-6 - 4e-8 * s->m) + tables * table - 0.29) <= 40.0;
+        return nq * (visits * (8e-6 - 4e-8 * s->m) + tables * table - 0.29) <= 40.0 + 1e-4 * visits;
     }
     const double per_query = visits * (4e-6 + 3.2e-7 * s->m) + (residual ? nprobe * (0.008 + 2.3e-4 * s->m) - 0.35 : -0.1);   // us
     return nq * per_query <= (residual ? 170.0 : 130.0);
