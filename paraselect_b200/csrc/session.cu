@@ -689,6 +689,7 @@ void note_list_lengths(psb_session* s, const int64_t* offsets) {
 }
 
 constexpr long long kRowDistFloats = 1ll << 28;   // distances kept at a time in the row forms: 1 GiB
+constexpr long long kPartQueries = 32768;         // queries at a time: they are the grid's second dimension, which ends at 65,535
 
 // Rows a query is expected to scan: its own list's, found in proportion to its length, and those of nprobe - 1 others.
 double expected_rows(const psb_session* s, int nprobe) {
@@ -794,7 +795,7 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, con
         return launch_scan(s->scan_index(), ws, d_lut, nq, d_probes, nprobe, stage1_k, d_rows, d_dist, d_count, s->sm_count, st, d_queries);
     AdcRows g{};
     g.stride = row_stride(s, nprobe, any_probes);
-    const int most = (int)std::max<long long>(1, std::min<long long>(32768, kRowDistFloats / g.stride));
+    const int most = (int)std::max<long long>(1, std::min(kPartQueries, kRowDistFloats / g.stride));
     const int parts = (nq + most - 1) / most, per = (nq + parts - 1) / parts;
     PSB_TRY(s->row_dist.reserve(sizeof(float) * (size_t)per * g.stride));
     PSB_TRY(s->row_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
@@ -2095,7 +2096,7 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     // A row of distances per query, as long as the nprobe longest lists; queries in parts of at most 1 GiB of them.
     FlatScan f{};
     f.stride = std::max<long long>(1, s->longest[(size_t)nprobe]);
-    const long long most = std::max<long long>(1, std::min<long long>(32768, ((long long)1 << 28) / f.stride));
+    const long long most = std::max<long long>(1, std::min(kPartQueries, kRowDistFloats / f.stride));
     const int parts = (int)((n + most - 1) / most), per = (n + parts - 1) / parts;
     PSB_TRY(s->row_dist.reserve(sizeof(float) * (size_t)per * f.stride));
     PSB_TRY(s->row_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
