@@ -514,7 +514,7 @@ def main():
                   recall_at_k_cpu=recall_at(ref["indices"][:gtn], gt_ids[:gtn], topk) if gtn else None,
                   recall_at_10_gpu=recall_at(e2e_ids[:gtn], gt_ids[:gtn], min(10, topk)) if gtn else None,
                   recall_at_10_cpu=recall_at(ref["indices"][:gtn], gt_ids[:gtn], min(10, topk)) if gtn else None)
-    host_pct = dict(staged=100, hybrid=100 - (args.zero_copy_pct or 45)).get(args.exact_mode, 0)   # the host threads' share of the rows
+    host_pct = dict(staged=100, hybrid=100 - (args.zero_copy_pct or 100)).get(args.exact_mode, 0)   # the host threads' share of the rows
     fetched = int(c["staged_gather_bytes"] / max(1, args.steps) * 100 / host_pct) or None if host_pct and R > topk else None
     line = dict(
         metric="QPS (IVF-PQ search, recall@k equal to the reference CPU path)", value=round(nq / (ms_dev * 1e-3), 1),

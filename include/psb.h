@@ -123,12 +123,10 @@ enum {
     PSB_EXACT_HOST_CACHED = 3, /* the session copies the caller's host rows into device memory once at creation and reranks from
                                   there (refused with PSB_OUT_OF_MEMORY when they do not fit); no counterpart in the reference,
                                   whose rerank rows stay on the host */
-    PSB_EXACT_HOST_HYBRID = 4  /* both host transports at once: the rows are registered and mapped as in HOST_MAPPED, and of every
-                                  sub-batch psb_options.zero_copy_pct percent of the rows fetched are gathered by a kernel
-                                  over PCIe - on reserve_sms SMs of its own (default 32), which the scan's grid leaves free -
-                                  while host threads stage the others through the pinned rings; neither the host cores nor
-                                  the kernel's reads fill the link alone.  Where no scan runs beside the rerank the kernel
-                                  has the whole GPU and brings all rows, unless zero_copy_pct is given */
+    PSB_EXACT_HOST_HYBRID = 4  /* HOST_MAPPED with the option of host threads beside the kernel: zero_copy_pct = 0 or 100: a kernel brings
+                                  all rows a batch fetches over PCIe - beside a scan on reserve_sms SMs of its own (default 16), which the
+                                  scan's grid leaves free - as in HOST_MAPPED; 1..99: that many percent, while host threads stage the
+                                  others through the pinned rings.  The kernel reads rows in ascending order at the link's rate. */
 };
 
 /* IVFPQSearchOptions (src/search/ivfpq/ivfpq_search_context.h:31-45) reduced to what this path uses,
@@ -164,8 +162,9 @@ typedef struct psb_options {
     float seed_sigma;   /* margin of the sampled admission cutoff in standard deviations (default 4; accepted 2..10).  Results do
                            not depend on it: a too-tight cutoff only sends more queries to the exact fallback. */
     int pipeline_parts; /* sub-batches per batch of the overlapped pipeline (default 4; accepted 2..32) */
-    int even_cuts;      /* staged transport: 0 = a short first sub-batch (10/30/30/30 %: the transfer, the longer half, starts early),
-                           1 = equal sub-batches, 2 = a short last sub-batch (32/32/26/10 %) */
+    int even_cuts;      /* rows fetched from the host beside the scan: 0 = a short first sub-batch (by the kernel 12/18/22/26/22 %, by host
+                           threads 10/30/30/30 %), so that the transfer starts early, 1 = equal sub-batches, 2 = a short last sub-batch
+                           (32/32/26/10 %) */
     int gather_ctas;    /* 128-thread CTAs of the PCIe row-gather kernel when it runs beside a scan (default: two per SM) */
     int tc_min_visitors;/* lists with fewer visiting queries than this stay with the SIMT scan (default 1: none do) */
     /* Test hooks of the time-out paths of the tensor-core kernels (leave 0): test_wait_limit = polls before a device-side wait
@@ -174,7 +173,7 @@ typedef struct psb_options {
        memory and returns, and the call reports PSB_TIMEOUT. */
     int test_wait_limit;
     int test_skip_mma;
-    int zero_copy_pct;  /* PSB_EXACT_HOST_HYBRID: share of each sub-batch gathered by the kernel, 1..100 (0 = 45 beside a scan, else 100) */
+    int zero_copy_pct;  /* PSB_EXACT_HOST_HYBRID: share of each sub-batch gathered by the kernel, 1..100 (0 = 100) */
     /* Residual mode, optional: the per-row correction asset of the index, value[row] = |recon(row)|^2 + 2 <centroid[list(row)],
        recon(row)> (src/common/row_correction.h:37-45), as HOST arrays over the rows of the view - either fp32 or the affine u16
        form (value = rc_offset + rc_scale * u16, src/common/row_correction.h:7-20).  The residual cutoff estimate reads it;

@@ -313,10 +313,21 @@ struct RowMap {
     long long base = 0;
     long long count = 0;
 };
-// Each row a batch's candidates name gets a slot: d_slot_of [count] (-1: none yet), d_unique [slots] = the row of each, d_n_unique their
-// number so far (the caller zeroes it once per batch; a batch may claim in several launches).  launch_release_rows puts d_slot_of back.
+// Each row a batch's candidates name gets a slot, those of one launch in ascending order.  A batch may claim in several launches (parts): the
+// slots of each begin at *d_begin, which the part before left in its *d_end; *d_n_unique: their number so far.  launch_release_rows puts slot_of
+// back.
+struct ClaimBuffers {
+    long long count = 0;        // rows held here
+    int* slot_of = nullptr;     // [count] -1: none yet
+    int* unique = nullptr;      // [slots] the row of each
+    unsigned* bits = nullptr;   // [claim_words(count)] zero before the launch, not after it
+    unsigned* old_bits = nullptr;   // as long: those of the claim before, zero after the launch
+    int* sums = nullptr;        // [claim_sums(count)]
+};
+size_t claim_words(long long count);
+size_t claim_sums(long long count);
 psb_status launch_claim_rows(const RowMap& mp, const int* d_candidates, int nq, int candidate_count, int candidate_stride, const int* d_counts,
-                             int* d_slot_of, int* d_unique, int* d_n_unique, cudaStream_t s);
+                             const ClaimBuffers& b, const int* d_begin, int* d_end, int* d_n_unique, cudaStream_t s);
 psb_status launch_release_rows(const int* d_unique, const int* d_n_unique, int* d_slot_of, int sm_count, cudaStream_t s);
 // Of the slots [begin, end) the host threads fill those below this, the gather kernel the others.
 __host__ __device__ __forceinline__ int host_share_end(int begin, int end, int host_pct) { return begin + (int)((long long)(end - begin) * host_pct / 100); }

@@ -464,7 +464,7 @@ struct psb_session {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaStream_t aux_stream = nullptr;  // second stream of the overlapped pipeline (created on first use)
-    cudaStream_t zc_stream = nullptr;   // hybrid transport: the kernel gather runs here, beside the copies of aux_stream
+    cudaStream_t zc_stream = nullptr;   // the gather kernel beside a scan runs here
     cudaEvent_t zc_ev_a = nullptr, zc_ev_b = nullptr;  // stage-level hybrid rerank: fork to and join from zc_stream
 
     cudaStream_t home_stream = nullptr; // the stream the session was created with (psb_session_set_stream(NULL) returns to it)
@@ -510,8 +510,9 @@ struct psb_session {
     long long staged_gather_bytes = 0;
     // Rows of a large batch cross to the device once each: the slot of every row held here, the rows by slot, the number of slots and
     // where each sub-batch's begin (PartMarks).
-    DevBuf slot_of, unique, marks;
-    bool slots_dirty = true;             // slot_of is not all -1 (a batch was left half done)
+    DevBuf slot_of, unique, marks, row_bits, row_sums;
+    bool slots_dirty = true;             // slot_of is not all -1, or row_bits not as rows_claim expects them (a batch was left half done)
+    int bits_turn = 0;                   // the half of row_bits the next claim uses: all 0
     int* h_unique = nullptr;             // pinned: the slots the host threads fill
     size_t h_unique_count = 0;
     size_t slots = 0;                    // of the batch at work, at most
@@ -747,8 +748,10 @@ int sub_batch_rows(const psb_session* s, int n, int nprobe, bool overlap) {
     return part_rows(n, overlap ? pipeline_parts : 1, tables ? (double)nprobe * s->m * s->k * sizeof(float) : 0.0);
 }
 
+int host_share(const psb_session* s);
+bool device_rows(const psb_session* s);
 // The staged transport (host gather threads + pinned rings), alone or with the kernel gather beside it.
-bool staged_mode(const psb_session* s) { return s->opt.exact_mode == PSB_EXACT_HOST_STAGED || s->opt.exact_mode == PSB_EXACT_HOST_HYBRID; }
+bool staged_mode(const psb_session* s) { return !device_rows(s) && host_share(s) > 0; }
 
 bool overlap_enabled(const psb_session* s, int n, bool rerank) {
     return rerank && !staged_mode(s) && n >= 2048 && !s->opt.serial_pipeline;
@@ -910,8 +913,7 @@ psb_status validate_params(const psb_session* s, const psb_query_batch_view* qv,
 // asked for more than once, and for rows longer than a line the slower reads of scoring in place.  In place against claimed, whole search, us:
 // 512-byte rows, 8,000 requests 205 / 209, 16,000 342 / 308, 64,000 1,158 / 856; 256-byte ones, 16,000 217 / 217, 64,000 631 / 521; 128-byte
 // ones, 32,000 236 / 246, 64,000 342 / 328, 260,000 1,219 / 898; 32-byte ones, 130,000 313 / 325, 260,000 579 / 485.
-// Where host threads bring a share, handing the work to them costs 2 ms more for long rows: with nothing beside them that pays from 200,000 to
-// 500,000 requests on.  That line counts requests and lies lower, for threads work beside a scan.
+// Where a caller has host threads bring a share, handing the work to them costs 2 ms more: that line counts requests.
 constexpr long long kClaimBytes = 4500000, kClaimBytesShort = 6500000, kClaimRequestsThreads = 65536;
 
 // Staged rerank transport: host threads gather exact rows into two pinned buffers, and cudaMemcpyAsync moves each filled buffer
@@ -982,8 +984,13 @@ psb_status rows_begin(psb_session* s, long long requests, size_t parts, cudaStre
     bool moved = false;
     PSB_TRY(reserve_together(&s->rows_whole, {{&s->unique, sizeof(int) * slots}, {&s->marks, sizeof(int) * PartMarks::device_words(parts)},
                                               {&s->stage, slots * s->dim * s->exact_elem},
-                                              {&s->slot_of, sizeof(int) * (size_t)std::max<long long>(1, s->exact_count)}}, 0, nullptr, &moved));
-    if (moved || s->slots_dirty) PSB_CUDA(cudaMemsetAsync(s->slot_of.p, 0xff, s->slot_of.bytes, st));
+                                              {&s->slot_of, sizeof(int) * (size_t)std::max<long long>(1, s->exact_count)},
+                                              {&s->row_bits, sizeof(unsigned) * claim_words(s->exact_count) * 2},
+                                              {&s->row_sums, sizeof(int) * claim_sums(s->exact_count)}}, 0, nullptr, &moved));
+    if (moved || s->slots_dirty) {
+        PSB_CUDA(cudaMemsetAsync(s->slot_of.p, 0xff, s->slot_of.bytes, st));
+        PSB_CUDA(cudaMemsetAsync(s->row_bits.p, 0, s->row_bits.bytes, st));
+    }
     s->slots_dirty = true;
     PSB_CUDA(cudaMemsetAsync(s->marks.p, 0, sizeof(int) * PartMarks::device_words(parts), st));
     return PSB_OK;
@@ -991,9 +998,12 @@ psb_status rows_begin(psb_session* s, long long requests, size_t parts, cudaStre
 int* part_begin(const psb_session* s, int part) { return s->marks.as<int>() + PartMarks::device_begin((size_t)part); }
 int* part_end(const psb_session* s, int part) { return part_begin(s, part) + 1; }
 psb_status rows_claim(psb_session* s, int part, const int* d_cand, int nq, int width, int stride, const int* d_counts, cudaStream_t st) {
-    PSB_TRY(launch_claim_rows(s->row_map(), d_cand, nq, width, stride, d_counts, s->slot_of.as<int>(), s->unique.as<int>(), s->marks.as<int>(), st));
-    PSB_CUDA(cudaMemcpyAsync(part_end(s, part), s->marks.p, sizeof(int), cudaMemcpyDeviceToDevice, st));
-    return PSB_OK;
+    ClaimBuffers b;
+    b.count = s->exact_count; b.slot_of = s->slot_of.as<int>(); b.unique = s->unique.as<int>(); b.sums = s->row_sums.as<int>();
+    b.bits = s->row_bits.as<unsigned>() + s->bits_turn * claim_words(s->exact_count);
+    b.old_bits = s->row_bits.as<unsigned>() + (s->bits_turn ^ 1) * claim_words(s->exact_count);
+    s->bits_turn ^= 1;
+    return launch_claim_rows(s->row_map(), d_cand, nq, width, stride, d_counts, b, part_begin(s, part), part_end(s, part), s->marks.as<int>(), st);
 }
 psb_status rows_end(psb_session* s, cudaStream_t st) {
     PSB_TRY(launch_release_rows(s->unique.as<int>(), s->marks.as<int>(), s->slot_of.as<int>(), s->sm_count, st));
@@ -1035,7 +1045,7 @@ psb_status rows_from_host(psb_session* s, int part, int host_pct, cudaStream_t s
     return PSB_OK;
 }
 
-// The stream of the hybrid transport's gather kernel.  Highest priority: its few CTAs each need an SM to themselves and must be
+// The stream of the gather kernel beside a scan.  Highest priority: its few CTAs each need an SM to themselves and must be
 // placed before the large grids of the scan stage that become runnable at the same moment.
 psb_status ensure_zc_stream(psb_session* s) {
     if (s->zc_stream) return PSB_OK;
@@ -1045,21 +1055,23 @@ psb_status ensure_zc_stream(psb_session* s) {
     return PSB_OK;
 }
 
-// The host threads' share of the rows, in percent.  The hybrid transport's threads pay beside a scan, which leaves the kernel few SMs; with
-// all of them the kernel alone is faster at every size (serial search, 130,000 to 2 million requests of fp32 rows of dim 96: 1.5 - 11.6
-// ms against 5.4 - 16.2), so it brings all rows there unless the caller names a share.
-int host_share(const psb_session* s, bool beside) {
+// SMs of the gather kernel beside a scan: 16 read ascending rows at the link's rate (8: 51.1 GB/s from an array of 0.8 GB but 40.3 from 20 GB, 16
+// and 32: 51.0 from either), and the scan's persistent grid leaves them free.
+constexpr int kGatherSms = 16;
+int gather_sms(const psb_session* s) { return s->opt.gather_ctas > 0 ? 0 : s->opt.reserve_sms > 0 ? s->opt.reserve_sms : kGatherSms; }
+
+// The host threads' share of the rows, in percent.  The kernel reads a part's rows in ascending order at the link's rate, beside a scan
+// and alone, and the threads take from the same link: they bring rows only where no kernel can (rows that are not mapped) or where the caller names a share.
+int host_share(const psb_session* s) {
     if (s->opt.exact_mode == PSB_EXACT_HOST_STAGED || !s->exact_dev) return 100;
-    if (s->opt.exact_mode != PSB_EXACT_HOST_HYBRID) return 0;
-    if (s->opt.zero_copy_pct > 0) return 100 - s->opt.zero_copy_pct;
-    return beside ? 55 : 0;
+    return s->opt.exact_mode == PSB_EXACT_HOST_HYBRID && s->opt.zero_copy_pct > 0 ? 100 - s->opt.zero_copy_pct : 0;
 }
 bool device_rows(const psb_session* s) { return s->opt.exact_mode == PSB_EXACT_RESIDENT || s->opt.exact_mode == PSB_EXACT_HOST_CACHED; }
 // Rows scored where they lie: in device memory, or so few that fetching each once would not pay for its launches.
-bool rows_in_place(const psb_session* s, long long requests, bool beside) {
+bool rows_in_place(const psb_session* s, long long requests) {
     if (device_rows(s)) return true;
     if (!s->exact_dev || s->opt.exact_mode == PSB_EXACT_HOST_STAGED) return false;
-    if (host_share(s, beside) > 0) return requests < kClaimRequestsThreads;
+    if (host_share(s) > 0) return requests < kClaimRequestsThreads;
     const long long row_bytes = (long long)s->dim * s->exact_elem;
     return requests * row_bytes < (row_bytes <= 128 ? kClaimBytesShort : kClaimBytes);
 }
@@ -1085,15 +1097,15 @@ psb_status rerank_impl(psb_session* s, const void* d_queries, int nq, const int*
         score = s->score.as<float>();
     }
     const bool beside = s->background || (s->aux_stream != nullptr && s->stream == s->aux_stream);
-    const bool in_place = rows_in_place(s, (long long)nq * width, beside);
+    const bool in_place = rows_in_place(s, (long long)nq * width);
     if (!in_place) {
         PSB_TRY(rows_begin(s, (long long)nq * width, 1, s->stream));
         PSB_TRY(rows_claim(s, 0, d_cand, nq, width, stride, d_counts, s->stream));
-        const int host_pct = host_share(s, beside);
+        const int host_pct = host_share(s);
         const int row_bytes = s->dim * s->exact_elem;
         // Beside a scan on the other stream the gather kernel runs on SMs of its own: the ones the scan's persistent grid leaves free
         // (reserve_sms), or gather_ctas lean CTAs spread over all SMs when the caller asks for that.
-        const int owned = beside && s->opt.gather_ctas == 0 ? (s->opt.reserve_sms > 0 ? s->opt.reserve_sms : 8) : 0;
+        const int owned = beside ? gather_sms(s) : 0;
         const int lean = beside ? s->opt.gather_ctas : 0;
         if (host_pct == 0) {
             PSB_TRY(launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, 0), part_end(s, 0), 0, s->stage.p, s->stream,
@@ -1192,7 +1204,7 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
     if (opt.zero_copy_pct < 0 || opt.zero_copy_pct > 100) return fail(PSB_INVALID_ARGUMENT, "zero_copy_pct must be in 0..100");
     if (opt.host_threads < 0 || opt.host_threads > 64) return fail(PSB_INVALID_ARGUMENT, "host_threads must be in 0..64");
     // hybrid transport: the gather kernel runs beside the scan on SMs of its own, which the scan's grid has to leave free
-    if (opt.exact_mode == PSB_EXACT_HOST_HYBRID && opt.reserve_sms == 0 && opt.gather_ctas == 0) opt.reserve_sms = 32;
+    if (opt.exact_mode == PSB_EXACT_HOST_HYBRID && opt.reserve_sms == 0 && opt.gather_ctas == 0) opt.reserve_sms = kGatherSms;
     if (opt.gather_ctas < 0 || opt.gather_ctas > 1024) return fail(PSB_INVALID_ARGUMENT, "gather_ctas must be in 0..1024");
     if (opt.adc_mode == 1 && !index->exact.fp32 && !index->exact.u8)
         return fail(PSB_INVALID_ARGUMENT, "residual mode always reranks: exact rows are required");
@@ -1668,13 +1680,21 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     const bool staged_overlap = rerank && staged_mode(s) && n >= 2048 && !s->opt.serial_pipeline;
     const int sb = sub_batch_rows(s, n, nprobe, overlap || staged_overlap);
     const bool residual = s->opt.adc_mode == 1;
-    // Sub-batch boundaries.  Equal cuts, except with the overlapped staged transport.  There the transfer costs the scan
-    // nothing and is the longer of the two (100M x 96, 10,000 queries x 1,000 candidates: 3.1 GB of distinct rows at the
-    // host's ~30 GB/s of random row reads, against ~60 ms of scanning), so it should start as early as possible: the first sub-batch is the small one (10/30/30/30 %).
+    // The rows of the whole batch are claimed and fetched once each, sub-batch by sub-batch (a row an earlier sub-batch has fetched is
+    // in its slot already), unless they are scored in place.
+    const int host_pct = host_share(s);
+    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k));
+    const bool kernel_gather = shared_rows && host_pct < 100;   // on a stream of its own
+    // Sub-batch boundaries.  Equal cuts, except where rows of host memory are fetched beside the scan.  There the transfer is about as long as
+    // the scan and costs it little, so the first sub-batch is a small one: the transfer starts early.  Where the kernel fetches, the cuts grow so that
+    // a sub-batch's scan takes about as long as the transfer of the one before, and the last is small again, for nothing hides its transfer
+    // (100M x 96, 10,000 queries x 1,000 candidates: 12/18/22/26/22 % 84.3 ms, 10/20/20/25/25 86.1, 10/30/30/30 88.6, seven parts 90.3; no difference
+    // at 1M to 12M rows).  Host threads are slower than the scan: 10/30/30/30 %.
     std::vector<int> cuts;
     const int plan = s->opt.even_cuts;
-    if (staged_overlap && (!residual || residual_table_free(s, stage1_k)) && sb * 4 >= n && n >= 4096 && plan != 1) {
+    if (shared_rows && (!residual || residual_table_free(s, stage1_k)) && sb * 4 >= n && n >= 4096 && plan != 1) {
         if (plan == 2) cuts = {0, (int)(0.32 * n), (int)(0.64 * n), (int)(0.90 * n), n};  // short last sub-batch (scan-bound hosts)
+        else if (host_pct == 0) cuts = {0, (int)(0.12 * n), (int)(0.30 * n), (int)(0.52 * n), (int)(0.78 * n), n};
         else cuts = {0, (int)(0.10 * n), (int)(0.40 * n), (int)(0.70 * n), n};
     } else {
         cuts = even_cuts(n, sb);
@@ -1713,13 +1733,8 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     psb_status worker_rc = PSB_OK;
     std::string worker_msg;
     std::thread worker;
-    // The rows of the whole batch are claimed and fetched once each, sub-batch by sub-batch (a row an earlier sub-batch has fetched is
-    // in its slot already), unless they are scored in place.
-    const int host_pct = host_share(s, true);
-    const bool hybrid = staged_overlap && host_pct < 100;
-    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k, true));
     const int row_bytes = s->dim * s->exact_elem;
-    if (hybrid) PSB_TRY(ensure_zc_stream(s));
+    if (kernel_gather) PSB_TRY(ensure_zc_stream(s));
     if (shared_rows) {
         PSB_TRY(s->score.reserve(sizeof(float) * (size_t)sb_max * stage1_k));
         PSB_TRY(rows_begin(s, (long long)n * stage1_k, cuts.size() - 1, st));
@@ -1801,6 +1816,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         if (times) rc = times->begin(st);
         ScanWorkspace sws;
         if (rc == PSB_OK) rc = s->timed_scan_ws(&sws);
+        if (kernel_gather) sws.reserve_ctas = std::max(sws.reserve_ctas, gather_sms(s));   // the gather kernel gets SMs of its own
         if (rc == PSB_OK && !table_free) {
             PSB_RANGE("pq_lut_build");
             if (residual && residual_tables_fused(sws, s->m, s->k)) {  // fp32 and fp16 tables in one kernel
@@ -1822,35 +1838,35 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         }
         if (rc == PSB_OK && times) rc = times->end(StageTimes::kScan, st);
         if (rc != PSB_OK) break;
-        if (staged_overlap) {  // claim the sub-batch's rows and hand it to the worker: an event marks the slot range ready
-            cudaEvent_t e, gathered = nullptr;
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) { rc = fail(PSB_CUDA_ERROR, "event creation failed"); break; }
-            deps.push_back(e);
+        cudaEvent_t ready = nullptr, gathered = nullptr;
+        auto event = [&](cudaEvent_t* e) -> psb_status {
+            if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return fail(PSB_CUDA_ERROR, "event creation failed");
+            deps.push_back(*e);
+            return PSB_OK;
+        };
+        if (shared_rows) {
             rc = rows_claim(s, (int)ci, rows_out, m, stage1_k, stage1_k, cnt_out, st);
-            if (rc == PSB_OK) rc = rows_tell_host(s, (int)ci, st);
+            if (rc == PSB_OK && staged_overlap) rc = rows_tell_host(s, (int)ci, st);
             if (rc != PSB_OK) break;
-            cudaEventRecord(e, st);
-            if (hybrid) {   // the kernel's share of the transfer, queued now: it starts the moment the rows are claimed
-                if (cudaEventCreateWithFlags(&gathered, cudaEventDisableTiming) != cudaSuccess) { rc = fail(PSB_CUDA_ERROR, "event creation failed"); break; }
-                deps.push_back(gathered);
-                cudaStreamWaitEvent(s->zc_stream, e, 0);
-                // on the SMs the scan's grid leaves free (reserve_sms), unless the caller asked for lean CTAs on all SMs
-                rc = launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, (int)ci), part_end(s, (int)ci), host_pct, s->stage.p,
-                                          s->zc_stream, s->sm_count, s->opt.gather_ctas, s->opt.gather_ctas > 0 ? 0 : s->opt.reserve_sms);
-                if (rc != PSB_OK) break;
-                cudaEventRecord(gathered, s->zc_stream);
-            }
-            { std::lock_guard<std::mutex> lk(mu); jobs.push_back(Job{(int)ci, p0, m, e, gathered}); }
+        }
+        if (shared_rows || overlap) {
+            if ((rc = event(&ready)) != PSB_OK) break;
+            cudaEventRecord(ready, st);
+        }
+        if (kernel_gather) {   // queued now: the transfer starts the moment the rows are claimed
+            if ((rc = event(&gathered)) != PSB_OK) break;
+            cudaStreamWaitEvent(s->zc_stream, ready, 0);
+            rc = launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, (int)ci), part_end(s, (int)ci), host_pct, s->stage.p,
+                                      s->zc_stream, s->sm_count, s->opt.gather_ctas, gather_sms(s));
+            if (rc != PSB_OK) break;
+            cudaEventRecord(gathered, s->zc_stream);
+        }
+        if (staged_overlap) {  // the worker takes over: the event marks the slot range ready
+            { std::lock_guard<std::mutex> lk(mu); jobs.push_back(Job{(int)ci, p0, m, ready, gathered}); }
             cv.notify_all();
             continue;
         }
-        if (overlap) {
-            cudaEvent_t e;
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) { rc = fail(PSB_CUDA_ERROR, "event creation failed"); break; }
-            deps.push_back(e);
-            cudaEventRecord(e, st);
-            cudaStreamWaitEvent(sx, e, 0);
-        }
+        if (overlap) cudaStreamWaitEvent(sx, ready, 0);
         // second half of the sub-batch (on the second stream when overlapping)
         cudaStream_t keep = s->stream;
         s->stream = sx;  // rerank_impl and the launchers below run on s->stream
@@ -1861,11 +1877,8 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
             PSB_RANGE("pq_rerank");
             mapped_ids = !s->striped;
             if (shared_rows) {
-                rc = rows_claim(s, (int)ci, rows_out, m, stage1_k, stage1_k, cnt_out, sx);
-                if (rc == PSB_OK)
-                    rc = launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, (int)ci), part_end(s, (int)ci), 0, s->stage.p, sx,
-                                              s->sm_count, s->opt.gather_ctas, s->opt.gather_ctas > 0 ? 0 : (s->opt.reserve_sms > 0 ? s->opt.reserve_sms : 8));
-                if (rc == PSB_OK) rc = score_part(p0, m);
+                cudaStreamWaitEvent(sx, gathered, 0);
+                rc = score_part(p0, m);
             } else {
                 const unsigned char* qe = static_cast<const unsigned char*>(dq_exact) + (size_t)p0 * row_bytes;
                 rc = rerank_impl(s, qe, m, rows_out, stage1_k, stage1_k, cnt_out, topk, mapped_ids ? nullptr : s->out_rows.as<int>() + (size_t)p0 * topk,

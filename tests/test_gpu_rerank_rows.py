@@ -98,3 +98,24 @@ def test_hybrid_shares(psb, how, dim, u8, nq, width):
             assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
         if how == "background":
             s.set_stream(None)
+
+
+@pytest.mark.parametrize("count", [31, 32, 33, 32767, 32768, 32769, 70001])
+@pytest.mark.parametrize("mode", [0, 4])
+def test_slots_in_row_order(psb, mode, count):
+    """Row counts at the ends of a word of marks and of a CTA's stretch of them, the first and last rows among those asked for, every row and few."""
+    import torch
+    ix = index(count, 32, False, count)
+    rng = np.random.default_rng(count)
+    nq, width = 900, 64                                             # above the line from which rows are fetched once
+    with psb.Session(ix, n_rerank=width, exact_mode=mode, max_batch=nq) as s:
+        for pool in (np.arange(count), np.unique(np.concatenate([[0, count - 1], rng.integers(0, count, 50)]))):
+            q = rng.standard_normal((nq, 32)).astype(np.float32)
+            cand = pool[rng.integers(0, len(pool), (nq, width))].astype(np.int32)
+            cand[0, :2] = [0, count - 1]
+            cand[:, 9] = -1
+            rows = torch.empty((nq, 10), dtype=torch.int32, device="cuda"); dist = torch.empty((nq, 10), device="cuda")
+            s.stage_rerank(torch.from_numpy(q).cuda(), nq, torch.from_numpy(cand).cuda(), width, width, None, 10, rows, dist)
+            s.sync()
+            wi, wd = oracle.rerank(ix["vectors"], q, cand, 10)
+            assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
