@@ -354,6 +354,9 @@ psb_status launch_offset_rows(int* d_rows, long long n, int delta, cudaStream_t 
 psb_status launch_widen_ids(const int* d_in, long long n, long long* d_out, cudaStream_t s);
 
 // ---- training ------------------------------------------------------------------------------------------------
+bool pq_nearest_supported(int dsub, int k, bool train);   // pq_nearest.cu: the tensor-core filter takes sub-vectors of this length
+psb_status launch_pq_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, bool train, uint8_t* d_codes, int sm_count,
+                             cudaStream_t s);
 psb_status launch_pq_encode(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
                             uint8_t* d_codes, int sm_count, cudaStream_t s);
 // The assignment of PQ training's Lloyd iterations: |c|^2 - 2 x.c in fused multiply-adds for sub-vectors of 2, 4 or 8 (else the encoder's

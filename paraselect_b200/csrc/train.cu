@@ -1,11 +1,10 @@
-// Training and encoding kernels: PQ encode (nearest codeword per sub-vector), PQ codebook Lloyd updates,
+// Training and encoding kernels: PQ encode (the shapes pq_nearest.cu does not take), PQ codebook seeding and Lloyd updates,
 // k-means accumulation / update, and the counter-based synthetic data generators used by the bench.
 //
 // Semantics follow the reference trainers: assignment = argmin of squared L2 with strict '<' so the lowest
 // index wins ties (src/clustering/kmeans/kmeans_utils.cu:359-413, src/quantization/pq/pq_encode.cuh:24-40),
 // update = mean of members, empty cluster keeps its centroid (src/clustering/kmeans/kmeans_utils.cu:267-284).
 // Member sums are accumulated in fp64 so the result does not depend on the summation order.
-#include <cuda_bf16.h>
 #include <algorithm>
 
 #include "common.cuh"
@@ -89,293 +88,6 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
     }
     __syncthreads();
     for (long long i = threadIdx.x; i < rows_here * m; i += kEncThreads) codes[(size_t)row0 * m + i] = s_codes[i];
-}
-
-// ---- nearest codeword of every sub-vector: a bf16 matrix product that filters, exact distances that decide -----------------
-// Per (row, sub-quantiser) all k codewords have to be compared; evaluated one by one in the reference encoder's arithmetic (sub,
-// mul, add per dimension, compare, select) that is 13 instructions for each of n * m * k pairs and the whole cost: 7.6 ms for 1M
-// rows of 128 dimensions, m = 32, at the issue limit, against 83 us for the bytes.  Here w = x.c - |c|^2 / 2 (largest for the nearest
-// codeword) comes from mma.sync with the operands split into two bf16 terms each and the norm into three,
-//     K slots  [ xh  xh  xl  1 1 1 ] . [ ch  cl  ch  -n0 -n1 -n2 ],   3 dsub + 3 <= 16 * KS,
-// which is within E of the true value; only groups of four codewords that hold a value >= max - 2E are evaluated exactly.  The
-// accumulators of mma.sync lie in registers where the maximum is taken; the contraction is so short (one K step for dsub 4) that
-// a tcgen05 accumulator would have to be read back from tensor memory, one value per pair, for a single K step of work.
-//   E: bf16 splits 3.1 * 2^-18 |x||c|; accumulation and norm split (16 KS) 2^-22 (|x||c| + |c|^2 / 2); rounding of the exact fp32
-//   distance (2 dsub + 2) 2^-24 (|x| + |c|)^2: together 2E <= 2^-15 |x| cmax + (KS + 1) 2^-18 (|x| + cmax)^2, and where products
-//   are subnormal or vanish, 2^-126 for each of the 16 KS products and three norm terms: 2 (16 KS + 3) 2^-126 <= 2^-118.
-// The nearest codeword in the exact arithmetic and all its ties are among the evaluated ones; the lowest index wins a tie.
-// kTrain: the evaluated ones are compared by |c|^2 - 2 x.c in fused multiply-adds, as the trainer's Lloyd iterations always have (the
-// reference's trainer assigns with a TF32 GEMM: src/quantization/pq/pq_trainer.cu:97-170); its rounding is within the same bound.
-// A warp takes 32 rows at a time (two 16-row tiles share every B fragment); a group's maximum is kept, not its values, so that the
-// 256 products of a row cost 16 registers; hits are queued and evaluated by full warps, one group per lane.  Rows pass through a
-// shared-memory tile of 32 floats each (read by 8 rows per request straight from global memory they took two thirds of the
-// time in the cache's tag stage).
-constexpr int kNearWarps = 8;
-constexpr int kNearSets = 2;                     // sets of 32 rows a warp takes one after the other against one codebook
-constexpr int kNearRows = kNearWarps * 32 * kNearSets;   // rows per CTA
-constexpr float kNearTiny = 3.1e-36f;            // above 2^-118
-constexpr float kFarNorm = 3.0e38f;              // in place of |c|^2 / 2 for codewords past k: below every score a threshold is taken from
-constexpr int kNearQueue = 384;                  // hits a warp queues (32 rows: usually 33 or 34); any beyond are evaluated on the spot
-
-__device__ __forceinline__ uint32_t bf16_word(float lo, float hi) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-template <int D> constexpr int near_ksteps() { return (3 * D + 3 + 15) / 16; }
-template <int D> constexpr int near_subs() { return 32 / D; }                                      // sub-quantisers of a tile
-template <int D> constexpr int near_pitch() { return (near_subs<D>() * D + 3) / 4 * 4 + 4; }       // 4 (mod 8) words: rows spread over the banks
-template <int D> constexpr size_t near_smem(int per) {
-    return (size_t)256 * D * 4 + (size_t)256 * near_ksteps<D>() * 32 + (size_t)kNearRows * near_pitch<D>() * 4 + (size_t)kNearWarps * kNearQueue * 2 +
-           (size_t)kNearWarps * 32 * 8 + (size_t)kNearRows * per;
-}
-template <int D>
-__device__ __forceinline__ void near_load(float (&v)[D], const float* __restrict__ x) {   // a sub-vector from shared memory
-    if constexpr (D % 4 == 0) {
-#pragma unroll
-        for (int d = 0; d < D; d += 4) { const float4 w = *reinterpret_cast<const float4*>(x + d); v[d] = w.x; v[d + 1] = w.y; v[d + 2] = w.z; v[d + 3] = w.w; }
-    } else if constexpr (D % 2 == 0) {
-#pragma unroll
-        for (int d = 0; d < D; d += 2) { const float2 w = *reinterpret_cast<const float2*>(x + d); v[d] = w.x; v[d + 1] = w.y; }
-    } else {
-#pragma unroll
-        for (int d = 0; d < D; ++d) v[d] = x[d];
-    }
-}
-// This lane's words of a row's A operand: K slots ks * 16 + 2t, + 1 (lo) and + 8, + 9 (hi); and |x|^2.
-template <int D>
-__device__ __forceinline__ float near_a_words(const float* __restrict__ x, int t, uint32_t (&lo)[near_ksteps<D>()], uint32_t (&hi)[near_ksteps<D>()]) {
-    constexpr int KS = near_ksteps<D>();
-    constexpr uint32_t kOnes = 0x3F803F80u, kOne = 0x3F80u;
-    float n2 = 0.0f;
-    if constexpr (D == 4 || D == 8) {   // every lane needs one pair of the row and its remainder
-        const float2 v = *reinterpret_cast<const float2*>(x + (D == 4 ? 2 * (t & 1) : 2 * t));
-        const uint32_t h = bf16_word(v.x, v.y);
-        const uint32_t l = bf16_word(v.x - __uint_as_float(h << 16), v.y - __uint_as_float(h & 0xFFFF0000u));
-        n2 = fmaf(v.x, v.x, v.y * v.y);
-        n2 += __shfl_xor_sync(0xffffffffu, n2, 1);
-        if constexpr (D == 8) n2 += __shfl_xor_sync(0xffffffffu, n2, 2);
-        lo[0] = h;
-        if constexpr (D == 4) {
-            hi[0] = t < 2 ? l : (t == 2 ? kOnes : kOne);
-        } else {
-            hi[0] = h; lo[1] = l; hi[1] = t == 0 ? kOnes : (t == 1 ? kOne : 0u);
-        }
-    } else {
-        float v[D], slot[KS * 16];
-        near_load<D>(v, x);
-#pragma unroll
-        for (int s = 0; s < KS * 16; ++s) slot[s] = 0.0f;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            const float h = bf16_round(v[d]);
-            slot[d] = h; slot[D + d] = h; slot[2 * D + d] = v[d] - h;
-            n2 = fmaf(v[d], v[d], n2);
-        }
-        slot[3 * D] = slot[3 * D + 1] = slot[3 * D + 2] = 1.0f;
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t w = bf16_word(slot[ks * 16 + 8 * half], slot[ks * 16 + 8 * half + 1]);
-#pragma unroll
-                for (int tt = 1; tt < 4; ++tt) {
-                    const uint32_t o = bf16_word(slot[ks * 16 + 8 * half + 2 * tt], slot[ks * 16 + 8 * half + 2 * tt + 1]);
-                    w = t == tt ? o : w;
-                }
-                (half ? hi : lo)[ks] = w;
-            }
-    }
-    return n2;
-}
-
-template <int D, bool kTrain>
-__global__ void __launch_bounds__(kNearWarps * 32, 2)
-k_pq_nearest(const float* __restrict__ data, long long n, int dim, const float* __restrict__ codebook, int m, int k, int subs_per_cta,
-             uint8_t* __restrict__ codes) {
-    constexpr int KS = near_ksteps<D>(), SUBS = near_subs<D>(), PITCH = near_pitch<D>();
-    extern __shared__ __align__(16) unsigned char s_near[];
-    float* s_cb = reinterpret_cast<float*>(s_near);                                     // [256][D] this sub-quantiser's codewords
-    uint2* s_b = reinterpret_cast<uint2*>(s_cb + 256 * D);                              // [32 n-tiles][KS][32 lanes] B fragments
-    float* s_x = reinterpret_cast<float*>(s_b + 256 * KS * 4);                          // [kNearRows][PITCH] rows, SUBS sub-vectors each
-    unsigned long long* s_best = reinterpret_cast<unsigned long long*>(s_x + kNearRows * PITCH);   // [warps][32]
-    uint16_t* s_queue = reinterpret_cast<uint16_t*>(s_best + kNearWarps * 32);          // [warps][kNearQueue]
-    uint8_t* s_codes = reinterpret_cast<uint8_t*>(s_queue + kNearWarps * kNearQueue);   // [kNearRows][subs_per_cta]
-    __shared__ int s_cnt[kNearWarps];
-    __shared__ float s_cmax[kNearWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3, g = lane >> 2;
-    const long long row0 = (long long)blockIdx.x * kNearRows;
-    const int rows_here = (int)min((long long)kNearRows, n - row0);
-    const int sub0 = blockIdx.y * subs_per_cta, sub1 = min(m, sub0 + subs_per_cta);
-    uint16_t* queue = s_queue + warp * kNearQueue;
-    unsigned long long* best = s_best + warp * 32;
-    const bool vec = (D % 4 == 0) && (dim % 4 == 0) && (reinterpret_cast<uintptr_t>(data) % 16 == 0);
-    for (int sub = sub0; sub < sub1; ++sub) {
-        __syncthreads();   // the previous sub-quantiser's operands are no longer read
-        const int ts = (sub - sub0) % SUBS;
-        if (ts == 0) {     // the next tile of the rows (rows past the end are zeros and are not written)
-            const int width = min(SUBS, sub1 - sub) * D;
-            const float* src = data + (size_t)row0 * dim + (size_t)sub * D;
-            if (vec) {
-                const int w4 = width >> 2;
-                for (int r = warp * 4 + (lane >> 3); r < kNearRows; r += kNearWarps * 4)
-                    for (int c = lane & 7; c < w4; c += 8)
-                        *reinterpret_cast<float4*>(s_x + r * PITCH + c * 4) =
-                            r < rows_here ? __ldg(reinterpret_cast<const float4*>(src + (size_t)r * dim) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            } else {
-                for (int r = warp; r < kNearRows; r += kNearWarps)
-                    if (lane < width) s_x[r * PITCH + lane] = r < rows_here ? __ldg(src + (size_t)r * dim + lane) : 0.0f;
-            }
-        }
-        {   // thread c prepares codeword c
-            const int c = threadIdx.x;
-            float v[D], n2 = 0.0f;
-#pragma unroll
-            for (int d = 0; d < D; ++d) v[d] = c < k ? __ldg(codebook + ((size_t)sub * k + c) * D + d) : 0.0f;
-#pragma unroll
-            for (int d = 0; d < D; ++d) { s_cb[c * D + d] = v[d]; n2 = fmaf(v[d], v[d], n2); }
-            float slot[KS * 16];
-#pragma unroll
-            for (int s = 0; s < KS * 16; ++s) slot[s] = 0.0f;
-#pragma unroll
-            for (int d = 0; d < D; ++d) {
-                const float h = bf16_round(v[d]);
-                slot[d] = h; slot[D + d] = v[d] - h; slot[2 * D + d] = h;
-            }
-            float rest = c < k ? 0.5f * n2 : kFarNorm;   // codewords past k are never near
-#pragma unroll
-            for (int i = 0; i < 3; ++i) { const float h = bf16_round(rest); slot[3 * D + i] = -h; rest -= h; }
-            uint4* dst = reinterpret_cast<uint4*>(s_b + ((size_t)(c >> 3) * KS) * 32 + (c & 7) * 4);   // fragment lane = (column % 8) * 4 + t
-#pragma unroll
-            for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-                for (int tt = 0; tt < 4; tt += 2)
-                    dst[ks * 16 + tt / 2] = make_uint4(bf16_word(slot[ks * 16 + 2 * tt], slot[ks * 16 + 2 * tt + 1]),
-                                                       bf16_word(slot[ks * 16 + 2 * tt + 8], slot[ks * 16 + 2 * tt + 9]),
-                                                       bf16_word(slot[ks * 16 + 2 * tt + 2], slot[ks * 16 + 2 * tt + 3]),
-                                                       bf16_word(slot[ks * 16 + 2 * tt + 10], slot[ks * 16 + 2 * tt + 11]));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) n2 = fmaxf(n2, __shfl_xor_sync(0xffffffffu, n2, o));
-            if (lane == 0) s_cmax[warp] = n2;
-        }
-        __syncthreads();
-        float cmax = s_cmax[0];
-#pragma unroll
-        for (int w = 1; w < kNearWarps; ++w) cmax = fmaxf(cmax, s_cmax[w]);
-        cmax = sqrtf(cmax) * 1.000001f;
-        const float* xsub = s_x + ts * D;
-#pragma unroll 1
-        for (int set = 0; set < kNearSets; ++set) {
-            const int wr0 = (set * kNearWarps + warp) * 32;   // first of the warp's 32 rows
-            if (wr0 >= rows_here) break;
-            if (lane == 0) s_cnt[warp] = 0;
-            best[lane] = ~0ull;
-            // A fragments: tile r covers rows r * 16 .. + 15, this lane's are g and g + 8 of each
-            uint32_t a[2][KS][4];
-            float xn[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t lo[KS], hi[KS];
-                xn[i] = near_a_words<D>(xsub + (wr0 + i * 8 + g) * PITCH, t, lo, hi);
-#pragma unroll
-                for (int ks = 0; ks < KS; ++ks) { a[i >> 1][ks][i & 1] = lo[ks]; a[i >> 1][ks][(i & 1) + 2] = hi[ks]; }
-            }
-            // group u of this lane = columns 16u + 2t, + 1, 16u + 8 + 2t, + 1
-            float gm[4][16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                float acc[2][2][4];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                    for (int r = 0; r < 2; ++r)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) acc[h][r][j] = 0.0f;
-#pragma unroll
-                    for (int ks = 0; ks < KS; ++ks) {
-                        const uint2 b = s_b[((2 * u + h) * KS + ks) * 32 + lane];
-                        mma_16816(acc[h][0], a[0][ks], b.x, b.y);
-                        mma_16816(acc[h][1], a[1][ks], b.x, b.y);
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = i >> 1, j = (i & 1) * 2;
-                    gm[i][u] = fmaxf(fmaxf(acc[0][r][j], acc[0][r][j + 1]), fmaxf(acc[1][r][j], acc[1][r][j + 1]));
-                }
-            }
-            __syncwarp();
-            // one group of four codewords of one row, exactly
-            auto evaluate = [&](uint32_t w) {
-                const int r = w & 31, c0 = (int)(w >> 7) * 16 + (int)((w >> 5) & 3) * 2;
-                float xv[D];
-                near_load<D>(xv, xsub + (wr0 + r) * PITCH);
-                unsigned long long key = ~0ull;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int c = c0 + (j & 1) + (j >> 1) * 8;
-                    float cv[D], dist = 0.0f;
-                    near_load<D>(cv, s_cb + c * D);
-                    if constexpr (kTrain) {
-#pragma unroll
-                        for (int d = 0; d < D; ++d) dist = fmaf(cv[d], cv[d], dist);
-#pragma unroll
-                        for (int d = 0; d < D; ++d) dist = fmaf(xv[d], -2.0f * cv[d], dist);
-                    } else {
-#pragma unroll
-                        for (int d = 0; d < D; ++d) {
-                            const float diff = __fsub_rn(xv[d], cv[d]);
-                            dist = __fadd_rn(dist, __fmul_rn(diff, diff));
-                        }
-                    }
-                    if (c < k && dist < FLT_MAX) {
-                        const unsigned long long kk = make_key(dist, (unsigned)c);
-                        key = kk < key ? kk : key;
-                    }
-                }
-                if (key != ~0ull) atomicMin(&best[r], key);
-            };
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float mx = gm[i][0];
-#pragma unroll
-                for (int u = 1; u < 16; ++u) mx = fmaxf(mx, gm[i][u]);
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float nx = sqrtf(xn[i]) * 1.000001f, both = nx + cmax;
-                const float thr = mx - (3.0517578125e-5f * nx * cmax + (float)(KS + 1) * 3.814697265625e-6f * both * both + kNearTiny);
-                uint32_t hit = 0;
-#pragma unroll
-                for (int u = 0; u < 16; ++u) hit |= (gm[i][u] >= thr ? 1u : 0u) << u;
-                if (!(fabsf(thr) <= 0.9f * kFarNorm)) hit = 0xffffu;   // a product or a norm overflowed or is not a number, or the codewords past k came first: evaluate everything
-                while (hit) {
-                    const int u = __ffs((int)hit) - 1;
-                    hit &= hit - 1;
-                    const uint32_t w = (uint32_t)((i * 8 + g) | (t << 5) | (u << 7));
-                    const int pos = atomicAdd(&s_cnt[warp], 1);
-                    if (pos < kNearQueue) queue[pos] = (uint16_t)w; else evaluate(w);
-                }
-            }
-            __syncwarp();
-            const int cnt = min(s_cnt[warp], kNearQueue);
-            for (int e = lane; e < cnt; e += 32) evaluate(queue[e]);
-            __syncwarp();
-            const unsigned long long b = best[lane];
-            s_codes[(size_t)(wr0 + lane) * subs_per_cta + (sub - sub0)] = b == ~0ull ? 0 : (uint8_t)b;
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    const int w = sub1 - sub0;
-    for (int i = threadIdx.x; i < rows_here * w; i += kNearWarps * 32) {
-        const int r = i / w, j = i - r * w;
-        codes[(size_t)(row0 + r) * m + sub0 + j] = s_codes[(size_t)r * subs_per_cta + j];
-    }
 }
 
 // ---- k-means++ seeding of the PQ codebooks, all sub-quantisers at once ------------------------------------------------------
@@ -752,43 +464,12 @@ __global__ void k_gen_normal(uint64_t seed, long long first, long long n, float 
 
 }  // namespace
 
-namespace {
-template <int D, bool kTrain = false>
-psb_status run_pq_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, uint8_t* d_codes, int sm_count, cudaStream_t s) {
-    // A CTA walks its sub-quantisers one after the other; with few row blocks they are cut into ranges so that two CTAs per SM
-    // have work, down to one sub-quantiser each.
-    const long long blocks = (n + kNearRows - 1) / kNearRows;
-    const int ranges = (int)std::max<long long>(1, std::min<long long>(m, (2ll * sm_count + blocks - 1) / blocks));
-    const int per = (m + ranges - 1) / ranges;
-    const size_t smem = near_smem<D>(per);
-    PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_nearest<D, kTrain>), smem));
-    k_pq_nearest<D, kTrain><<<dim3((unsigned)blocks, (unsigned)((m + per - 1) / per)), kNearWarps * 32, smem, s>>>(d_data, n, dim, d_codebook, m, k, per, d_codes);
-    count_launch();
-    PSB_LAUNCH_CHECK();
-    return PSB_OK;
-}
-}  // namespace
-
 psb_status launch_pq_encode(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
                             uint8_t* d_codes, int sm_count, cudaStream_t s) {
     if (n <= 0) return PSB_OK;
     const int dsub = dim / m;
-    // Few codewords or long sub-vectors: one by one (the filter pays from about 32 codewords on, and its operands hold 16
-    // dimensions at most); m is bounded by the codes a CTA stages.
-    if (k > 32 && m <= 192) {
-        switch (dsub) {
-            case 2: return run_pq_nearest<2>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 3: return run_pq_nearest<3>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 4: return run_pq_nearest<4>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 5: return run_pq_nearest<5>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 6: return run_pq_nearest<6>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 8: return run_pq_nearest<8>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 10: return run_pq_nearest<10>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 12: return run_pq_nearest<12>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 16: return run_pq_nearest<16>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            default: break;
-        }
-    }
+    if (pq_nearest_supported(dsub, k, false)) return launch_pq_nearest(d_data, n, dim, d_codebook, m, k, false, d_codes, sm_count, s);
+    // Few codewords or long sub-vectors: one by one.
     const unsigned grid = (unsigned)((n + kEncThreads - 1) / kEncThreads);
     const size_t tile = (size_t)kEncThreads * (dim + 1) * sizeof(float) + (size_t)k * dsub * sizeof(float) + (size_t)kEncThreads * m;
     if (tile <= 200 * 1024) {  // rows staged in shared memory
@@ -807,14 +488,7 @@ psb_status launch_pq_encode(const float* d_data, long long n, int dim, const flo
 psb_status launch_pq_assign_train(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
                                   uint8_t* d_codes, int sm_count, cudaStream_t s) {
     if (n <= 0) return PSB_OK;
-    if (k > 32 && m <= 192) {
-        switch (dim / m) {
-            case 2: return run_pq_nearest<2, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 4: return run_pq_nearest<4, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 8: return run_pq_nearest<8, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            default: break;
-        }
-    }
+    if (pq_nearest_supported(dim / m, k, true)) return launch_pq_nearest(d_data, n, dim, d_codebook, m, k, true, d_codes, sm_count, s);
     return launch_pq_encode(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
 }
 

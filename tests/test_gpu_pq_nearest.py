@@ -80,3 +80,25 @@ def test_encode_where_products_underflow(dim, M, scale):
     api.pq_encode(torch.from_numpy(x).cuda(), n, dim, torch.from_numpy(cb).cuda(), M, K, codes)
     torch.cuda.synchronize()
     assert np.array_equal(codes.cpu().numpy(), oracle.pq_encode(x, cb))
+
+
+@pytest.mark.parametrize("n,dim,M,K", [(127, 16, 4, 256), (128, 16, 5, 256), (129, 20, 5, 255), (1921, 24, 6, 256), (5000, 64, 16, 256), (70000, 8, 2, 256),
+                                       (150, 400, 200, 40), (3000, 48, 4, 256), (2500, 33, 11, 33)])
+@pytest.mark.parametrize("at", [0, 1, 2])
+def test_encode_tiles_and_items(n, dim, M, K, at):
+    """Rows at the ends of a tile and of an item's tiles, sub-quantisers that do not fill an operand row, rows that start at any float."""
+    import torch
+    from paraselect_b200 import api
+    if dim % M:
+        dim = dim // M * M
+    rng = np.random.default_rng(n + dim + at)
+    x = rng.standard_normal((n, dim)).astype(np.float32)
+    cb = rng.standard_normal((M, K, dim // M)).astype(np.float32)
+    flat = torch.empty(n * dim + 4, device="cuda")
+    flat[at:at + n * dim] = torch.from_numpy(x).cuda().flatten()
+    codes = torch.full((n * M + 4,), 99, dtype=torch.uint8, device="cuda")
+    api.pq_encode(flat[at:at + n * dim], n, dim, torch.from_numpy(cb).cuda(), M, K, codes[at:at + n * M])
+    torch.cuda.synchronize()
+    got = codes.cpu().numpy()
+    assert np.array_equal(got[at:at + n * M].reshape(n, M), oracle.pq_encode(x, cb))
+    assert (got[:at] == 99).all() and (got[at + n * M:] == 99).all()
