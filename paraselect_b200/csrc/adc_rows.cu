@@ -5,7 +5,7 @@
 // memory (residual mode: the table of a (query, probe) pair; a caller's own tables are read instead), scores its share of the query's rows
 // with it and writes the distances out; nothing is sampled, scheduled or re-scored, and a query's rows spread over the chip.  Bound:
 // shared-memory gathers, m per row visit, about 3.5 cycles per warp-wide gather of random banks.  The selection is select.cuh's, reading
-// each distance twice.
+// each distance twice, or (plain mode) the minima of 32 and the distances of the runs that matter.
 // Same arithmetic and order as the other scans (reference: src/search/ivfpq/stage/ivfpq_fine_cpu_lut.cpp:51-63,76-80;
 // src/search/ivfrespq/stage/ivfrespq_cpu_rerank.cpp:87-130,226-259,440-451), so the same candidates.
 #include <algorithm>
@@ -79,11 +79,16 @@ k_adc_rows(const AdcRows g, int block_rows) {
     block_table(s_tab, s_q, g, q);
     __syncthreads();
     float* out = g.dist + (size_t)q * g.stride;
-    for (int i = i0 + threadIdx.x; i < i1; i += kRowsThreads) {
-        int lo = 0, hi = g.nprobe;   // largest p with seg[p] <= i
-        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s_seg[mid] <= i) lo = mid; else hi = mid; }
-        const long long row = g.offsets[g.probes[(size_t)q * g.nprobe + lo]] + (i - s_seg[lo]);
-        out[i] = adc_row<M>(g.codes + (size_t)(row - g.row_base) * g.m, s_tab, g.m, g.k, false);
+    const int lane = threadIdx.x & 31;
+    for (int i = i0 + threadIdx.x; i - lane < i1; i += kRowsThreads) {   // whole runs: i0 and the warps' strides are multiples of 32
+        float d = __int_as_float(0x7f800000);
+        if (i < i1) {
+            int lo = 0, hi = g.nprobe;   // largest p with seg[p] <= i
+            while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s_seg[mid] <= i) lo = mid; else hi = mid; }
+            const long long row = g.offsets[g.probes[(size_t)q * g.nprobe + lo]] + (i - s_seg[lo]);
+            out[i] = d = adc_row<M>(g.codes + (size_t)(row - g.row_base) * g.m, s_tab, g.m, g.k, false);
+        }
+        if (g.runs) sel::store_run(g.runs + (size_t)q * g.run_stride, i / sel::kRun, d);
     }
 }
 
@@ -114,17 +119,24 @@ k_adc_pair_rows(const AdcRows g, int block_rows, int chunks) {
 template <int T>
 __global__ void __launch_bounds__(T)
 k_adc_select(const AdcRows g, int buffer) {
-    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, then the group minima
+    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the selection's runs, the segments (where they fit)
     __shared__ sel::Words w;
     const int q = blockIdx.x;
     const int* s = g.seg + (size_t)q * (g.nprobe + 1);
+    if (g.nprobe <= sel::kSegShared) {   // a search for every key: not in global memory
+        int* s_seg = reinterpret_cast<int*>(s_key + buffer) + sel::kMaxGroups;
+        for (int p = threadIdx.x; p <= g.nprobe; p += T) s_seg[p] = s[p];
+        __syncthreads();
+        s = s_seg;
+    }
     auto row_of = [&](int i) -> uint32_t {
         int lo = 0, hi = g.nprobe;
         while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
         const int l = g.probes[(size_t)q * g.nprobe + lo];
         return (uint32_t)(g.offsets[l] + (i - s[lo]) + (g.row_delta ? g.row_delta[l] : 0));
     };
-    const int keep = sel::smallest<T>(g.dist + (size_t)q * g.stride, s[g.nprobe], g.stage1_k, row_of, s_key, buffer, reinterpret_cast<float*>(s_key + buffer), &w);
+    const int keep = sel::smallest<T>(g.dist + (size_t)q * g.stride, s[g.nprobe], g.stage1_k, row_of, s_key, buffer, reinterpret_cast<int*>(s_key + buffer), &w,
+                                      g.runs ? g.runs + (size_t)q * g.run_stride : nullptr);
     for (int i = threadIdx.x; i < g.stage1_k; i += T) {
         const bool ok = i < keep;
         g.out_rows[(size_t)q * g.stage1_k + i] = ok ? (int)key_idx(s_key[i]) : -1;
@@ -172,7 +184,7 @@ psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s) {
         default: PSB_TRY(run_rows<0>(g, nq, s)); break;
     }
     const int buffer = sel::buffer_entries(g.stage1_k);
-    const size_t smem = sel::shared_bytes(g.stage1_k);
+    const size_t smem = sel::shared_bytes(g.stage1_k) + (g.nprobe <= sel::kSegShared ? ((size_t)g.nprobe + 1) * sizeof(int) : 0);
     // Fewer queries than SMs: one selecting block per SM at most, so a large one.
     auto select = [&](auto kernel, int threads) -> psb_status {
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));

@@ -96,14 +96,29 @@ k_coarse_dist_small(const float* __restrict__ queries, int nq, const float* __re
     }
 }
 
+// The same for few pairs: a thread per centroid and query, the query in shared memory.  Of a tile most threads have no query, and the others
+// have four centroids each, one after the other.  With the selection behind it, tiles against this, us: 1,024 centroids x 96, 1 query 15.2 / 11.3,
+// 32 queries 17.2 / 14.3, 64 19.3 / 19.2, 128 19.1 / 25.3; 4,096, 8 queries 15.3 / 14.1, 16 16.3 / 17.2; 512 x 126, 64 queries 23.5 / 19.4; 256 x 96,
+// 128 queries 19.2 / 15.3: the line lies at 32,768 pairs.
+constexpr int kFewThreads = 64;
+constexpr long long kFewPairs = 32768;
+__global__ void __launch_bounds__(kFewThreads)
+k_coarse_dist_few(const float* __restrict__ queries, const float* __restrict__ centroids, int nlist, int dim, float* __restrict__ dist) {
+    extern __shared__ __align__(16) float s_q[];
+    const int q = blockIdx.y, c = blockIdx.x * kFewThreads + threadIdx.x;
+    for (int d = threadIdx.x; d < dim; d += kFewThreads) s_q[d] = queries[(size_t)q * dim + d];
+    __syncthreads();
+    if (c < nlist) dist[(size_t)q * nlist + c] = row_distance(s_q, centroids + (size_t)c * dim, dim, rows_vec(centroids, dim));
+}
+
 // Per row: the k smallest (value, index) pairs, ascending.
 constexpr int kSelThreads = 256;
 __global__ void __launch_bounds__(kSelThreads)
 k_select_rows(const float* __restrict__ dist, int n, int k, int buffer, int* __restrict__ out_ids, float* __restrict__ out_dist) {
-    extern __shared__ __align__(16) uint64_t s_sel[];  // [buffer] keys, then the group minima
+    extern __shared__ __align__(16) uint64_t s_sel[];  // [buffer] keys, then the selection's runs
     __shared__ sel::Words w;
     const int keep = sel::smallest<kSelThreads>(dist + (size_t)blockIdx.x * n, n, k, [](int i) { return (uint32_t)i; }, s_sel, buffer,
-                                   reinterpret_cast<float*>(s_sel + buffer), &w);
+                                   reinterpret_cast<int*>(s_sel + buffer), &w);
     for (int i = threadIdx.x; i < k; i += blockDim.x) {
         const bool ok = i < keep;
         out_ids[(size_t)blockIdx.x * k + i] = ok ? (int)key_idx(s_sel[i]) : -1;
@@ -116,6 +131,14 @@ k_select_rows(const float* __restrict__ dist, int n, int k, int buffer, int* __r
 psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float* d_centroids, int nlist,
                                     int dim, float* d_dist, int sm_count, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
+    const size_t smem = (size_t)((dim + 3) & ~3) * sizeof(float);
+    if ((long long)nq * nlist <= kFewPairs && nq <= 65535 && smem <= (size_t)200 * 1024) {
+        if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_coarse_dist_few), smem));
+        k_coarse_dist_few<<<dim3((unsigned)((nlist + kFewThreads - 1) / kFewThreads), (unsigned)nq), kFewThreads, smem, s>>>(d_queries, d_centroids, nlist, dim, d_dist);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        return PSB_OK;
+    }
     dim3 grid((nlist + BC - 1) / BC, (nq + BQ - 1) / BQ);
     // Small tiles while the large ones would leave SMs without one (two waves of small tiles still beat one of large ones), if
     // their rows fit.

@@ -41,6 +41,25 @@ __device__ __forceinline__ void stage_wait() {
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 }
+// Distance of q (shared memory, 16-byte aligned) to the row x, four elements at a time where vec.
+__device__ __forceinline__ float row_distance(const float* __restrict__ q, const float* __restrict__ x, int dim, bool vec) {
+    float sum = 0.0f;
+    if (vec) {
+#pragma unroll 8
+        for (int d = 0; d < dim; d += 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(x + d));
+            const float4 y = *reinterpret_cast<const float4*>(q + d);
+            float t = __fsub_rn(y.x, v.x); sum = __fadd_rn(sum, __fmul_rn(t, t));
+            t = __fsub_rn(y.y, v.y); sum = __fadd_rn(sum, __fmul_rn(t, t));
+            t = __fsub_rn(y.z, v.z); sum = __fadd_rn(sum, __fmul_rn(t, t));
+            t = __fsub_rn(y.w, v.w); sum = __fadd_rn(sum, __fmul_rn(t, t));
+        }
+    } else {
+#pragma unroll 8
+        for (int d = 0; d < dim; ++d) { const float t = __fsub_rn(q[d], __ldg(x + d)); sum = __fadd_rn(sum, __fmul_rn(t, t)); }
+    }
+    return sum;
+}
 // acc[i][j] = distance of q row i to c row 16 j; the zeros behind dim add exact zeros.
 __device__ __forceinline__ void tile_distances(const float* __restrict__ q, const float* __restrict__ c, int pitch, int dim, float (&acc)[4][4]) {
 #pragma unroll

@@ -145,7 +145,8 @@ k_flat_tiles(const float* __restrict__ queries, int dim, int nprobe, const long 
 // Few visitors per list: a thread per (query, row).  grid (row blocks, queries).
 __global__ void __launch_bounds__(128)
 k_flat_rows(const float* __restrict__ queries, int dim, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
-            const float* __restrict__ rows, const int* __restrict__ seg, long long stride, float* __restrict__ dist) {
+            const float* __restrict__ rows, const int* __restrict__ seg, long long stride, float* __restrict__ dist, float* __restrict__ runs,
+            long long run_stride) {
     extern __shared__ __align__(16) float s_q[];
     const int q = blockIdx.y;
     const int* s = seg + (size_t)q * (nprobe + 1);
@@ -154,26 +155,16 @@ k_flat_rows(const float* __restrict__ queries, int dim, const int* __restrict__ 
     for (int d = threadIdx.x; d < dim; d += 128) s_q[d] = queries[(size_t)q * dim + d];
     __syncthreads();
     const bool vec = rows_vec(rows, dim);
-    for (int i = blockIdx.x * 128 + threadIdx.x; i < n; i += gridDim.x * 128) {
-        int lo = 0, hi = nprobe;   // largest p with s[p] <= i
-        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
-        const float* x = rows + (size_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo])) * dim;
-        float sum = 0.0f;
-        if (vec) {
-#pragma unroll 8
-            for (int d = 0; d < dim; d += 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4*>(x + d));
-                const float4 y = *reinterpret_cast<const float4*>(s_q + d);
-                float t = __fsub_rn(y.x, v.x); sum = __fadd_rn(sum, __fmul_rn(t, t));
-                t = __fsub_rn(y.y, v.y); sum = __fadd_rn(sum, __fmul_rn(t, t));
-                t = __fsub_rn(y.z, v.z); sum = __fadd_rn(sum, __fmul_rn(t, t));
-                t = __fsub_rn(y.w, v.w); sum = __fadd_rn(sum, __fmul_rn(t, t));
-            }
-        } else {
-#pragma unroll 8
-            for (int d = 0; d < dim; ++d) { const float t = __fsub_rn(s_q[d], __ldg(x + d)); sum = __fadd_rn(sum, __fmul_rn(t, t)); }
+    float* out = dist + (size_t)q * stride;
+    for (int i = blockIdx.x * 128 + threadIdx.x; i - (int)(threadIdx.x & 31) < n; i += gridDim.x * 128) {   // whole runs
+        float sum = __int_as_float(0x7f800000);
+        if (i < n) {
+            int lo = 0, hi = nprobe;   // largest p with s[p] <= i
+            while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
+            const float* x = rows + (size_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo])) * dim;
+            out[i] = sum = row_distance(s_q, x, dim, vec);
         }
-        dist[(size_t)q * stride + i] = sum;
+        if (runs) sel::store_run(runs + (size_t)q * run_stride, i / sel::kRun, sum);
     }
 }
 
@@ -182,17 +173,24 @@ template <int T>
 __global__ void __launch_bounds__(T)
 k_flat_select(const float* __restrict__ dist, long long stride, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
               const int* __restrict__ seg, int topk, int buffer, const long long* __restrict__ ids, long long* __restrict__ out_ids,
-              float* __restrict__ out_dist) {
-    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, then the group minima
+              float* __restrict__ out_dist, const float* __restrict__ runs, long long run_stride) {
+    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the selection's runs, the segments (where they fit)
     __shared__ sel::Words w;
     const int q = blockIdx.x;
     const int* s = seg + (size_t)q * (nprobe + 1);
+    if (nprobe <= sel::kSegShared) {   // a search for every key: not in global memory
+        int* s_seg = reinterpret_cast<int*>(s_key + buffer) + sel::kMaxGroups;
+        for (int p = threadIdx.x; p <= nprobe; p += T) s_seg[p] = s[p];
+        __syncthreads();
+        s = s_seg;
+    }
     auto row_of = [&](int i) -> uint32_t {
         int lo = 0, hi = nprobe;
         while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
         return (uint32_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo]));
     };
-    const int keep = sel::smallest<T>(dist + (size_t)q * stride, s[nprobe], topk, row_of, s_key, buffer, reinterpret_cast<float*>(s_key + buffer), &w);
+    const int keep = sel::smallest<T>(dist + (size_t)q * stride, s[nprobe], topk, row_of, s_key, buffer, reinterpret_cast<int*>(s_key + buffer), &w,
+                                      runs ? runs + (size_t)q * run_stride : nullptr);
     for (int i = threadIdx.x; i < topk; i += T) {
         const bool ok = i < keep;
         out_ids[(size_t)q * topk + i] = ok ? ids[key_idx(s_key[i])] : -1;
@@ -243,15 +241,15 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
         const size_t smem = (size_t)((f.dim + 3) & ~3) * sizeof(float);
         if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_rows), smem));
         k_flat_rows<<<dim3((unsigned)std::max<long long>(1, blocks), (unsigned)nq), 128, smem, s>>>(f.queries, f.dim, f.probes, f.nprobe, f.offsets, f.rows,
-                                                                                                    f.seg, f.stride, f.dist);
+                                                                                                    f.seg, f.stride, f.dist, f.runs, f.run_stride);
     }
     count_launch();
     PSB_LAUNCH_CHECK();
-    const size_t smem = sel::shared_bytes(f.topk);
+    const size_t smem = sel::shared_bytes(f.topk) + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
     auto select = [&](auto kernel, int threads) -> psb_status {   // fewer queries than SMs: large blocks
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
         kernel<<<nq, threads, smem, s>>>(f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids,
-                                         f.out_dist);
+                                         f.out_dist, lists ? nullptr : f.runs, f.run_stride);
         return PSB_OK;
     };
     if (nq <= f.sm_count) PSB_TRY(select(k_flat_select<1024>, 1024));

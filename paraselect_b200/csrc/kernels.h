@@ -268,6 +268,7 @@ struct AdcRows {
     int stage1_k;
     int* out_rows; float* out_dist; int* out_count;
     int* seg; float* dist; long long stride;        // workspace: [nq][nprobe + 1], [nq][stride]
+    float* runs; long long run_stride;              // workspace, plain mode: [nq][run_stride], the minimum of every 32 distances
     double expected_rows; long long longest_list;   // rows a query is expected to scan; rows of the longest list
     unsigned long long* counters;
     int sm_count;
@@ -292,6 +293,7 @@ struct FlatScan {
     int topk;
     long long* out_ids; float* out_dist;       // [nq][topk]
     float* dist; long long stride;             // [nq][stride] workspace, stride >= the rows of any nprobe lists
+    float* runs; long long run_stride;         // [nq][run_stride] workspace of the row form: the minimum of every 32 distances
     int* seg;                                  // [nq][nprobe + 1]
     // list form only (flat_list_form): [nlist], [nq * nprobe], [nlist + 1], [nlist + 1], [nq * nprobe]
     int* vis_count; int* slot; int* vis_off; long long* item_off; int* visitors;

@@ -403,7 +403,7 @@ k_topk_select(const float* __restrict__ dist, const int* __restrict__ cand, int 
               const long long* __restrict__ ids, long long* __restrict__ out_ids) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_raw);            // [max(np, buffer)]
-    int* s_rank = reinterpret_cast<int*>(s_raw + (size_t)max(np, buffer) * 8);  // [max(np, kMaxGroups)]: ranks, or the group minima
+    int* s_rank = reinterpret_cast<int*>(s_raw + (size_t)max(np, buffer) * 8);  // [max(np, kMaxGroups)]: ranks, or the selection's runs
     __shared__ sel::Words w;
     __shared__ int s_warp[32];
     __shared__ int s_total, s_twice;
@@ -417,7 +417,7 @@ k_topk_select(const float* __restrict__ dist, const int* __restrict__ cand, int 
         out_dist[(size_t)q * topk + r] = key == KEY_MAX ? FLT_MAX : key_dist(key);
     };
     const int keep = sel::smallest<kSelectThreads>(dist + (size_t)q * candidate_count, n, topk, [&](int i) { return (uint32_t)rows[i]; }, s_keys, buffer,
-                                                   reinterpret_cast<float*>(s_rank), &w);
+                                                   s_rank, &w);
     if (threadIdx.x == 0) s_twice = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < keep; i += kSelectThreads)   // a row twice, or a distance without a row

@@ -6,7 +6,8 @@
 namespace psb {
 namespace sel {
 
-constexpr int kMaxGroups = 2048;  // group minima
+constexpr int kMaxGroups = 2048;  // minima looked at
+constexpr int kSegShared = 1024;  // probes whose segments the selections over lists keep in shared memory
 
 // Entries the key buffer needs: a power of two that holds the keys gathered at the usual cut several times over.
 inline int buffer_entries(int k) { return k <= 256 ? 1024 : (k <= 1024 ? 4096 : 8192); }
@@ -52,71 +53,136 @@ __device__ unsigned smallest_word(int n, unsigned rank, Get get, uint32_t* out, 
     return rank;
 }
 
-// Leaves the min(k, n) smallest keys (vals[i], payload(i)) of i = 0..n-1 at the front of s_keys, ascending, and returns their number.  s_keys [buffer], s_min [kMaxGroups], one Words in shared memory; k <= buffer.
-//
-// Reads the values twice.  First every thread takes the minima of a few of its strided subsets; the k-th smallest of all these
-// minima - there are at least 2 k of them - bounds the k-th smallest value from above, and not much more than k values lie below
-// it.  One warp finds it by bisection (14 rounds or until exactly k lie below; a little high does no harm).  Then the values up to
-// that cut are gathered and put in order by rank or, above 256, by a bitonic sort.  A radix selection is left for
-// the rows the cut does not serve: too many equal values, fewer than k comparable ones, or k above what the group minima cover.
+// A value with at least k of s_min[0..n-1] (infinite: none) at or below it and not many more, by bisection; infinity where fewer than k are finite.
+// One warp; a share of R words at most in registers, or (R = 0) all read from shared memory in every round.  (A count by the whole block, with a
+// barrier and one counter for its warps in every round, took four times as long.)
+template <int R>
+__device__ __forceinline__ float bound_of(const float* s_min, int n, int k) {
+    const int lane = threadIdx.x & 31;
+    const float inf = __int_as_float(0x7f800000);
+    float v[R > 0 ? R : 1], lo = inf, hi = -inf;
+    auto each = [&](auto&& f) {
+        if constexpr (R > 0) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) f(v[r]);
+        } else {
+            for (int i = lane; i < n; i += 32) f(s_min[i]);
+        }
+    };
+    if constexpr (R > 0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = r * 32 + lane < n ? s_min[r * 32 + lane] : inf;
+    }
+    each([&](float x) { lo = fminf(lo, x); if (x < inf) hi = fmaxf(hi, x); });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o)); hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o)); }
+    auto count = [&](float at) {
+        int c = 0;
+        each([&](float x) { c += x <= at ? 1 : 0; });
+        return (int)__reduce_add_sync(0xffffffffu, c);
+    };
+    if (!(lo < inf) || count(hi) < k) return inf;
+    for (int it = 0; it < 14; ++it) {
+        const float mid = lo + 0.5f * (hi - lo);
+        const int c = count(mid);
+        if (c >= k) hi = mid; else lo = mid;
+        if (c >= k && c <= k + (k >> 3)) break;
+    }
+    return hi;
+}
+
+// Minima of every 32 values, left by the kernel that computed them (one warp each), bound a row's k-th smallest value as well as the minima
+// of subsets do, and say which 32 values to look at again.
+constexpr int kRun = 32;
+constexpr int kRunQueries = 16;   // (they cost a large batch's scan more than they save its selection)
+inline long long run_count(long long values) { return (values + kRun - 1) / kRun; }
+// The warp's lanes hold the values of run r (+infinity: none).
+__device__ __forceinline__ void store_run(float* __restrict__ runs, int r, float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) runs[r] = v;
+}
+
+// Leaves the min(k, n) smallest keys (vals[i], payload(i)) of i = 0..n-1 at the front of s_keys, ascending, and returns their number.  s_keys
+// [buffer], s_runs [kMaxGroups], one Words in shared memory; k <= buffer.  runs: the minima of every kRun values, or null.
+// The k-th smallest of the minima of at least 2 k subsets of the values bounds the k-th smallest value from above.  Every thread takes the
+// minima of a few strided subsets, and not much more than k values lie below that bound, whatever the order of the values; a second read
+// gathers them, and they are put in order by rank or, above the block's size, by a bitonic sort.  With runs, the minima of these bound the k-th
+// value first, and only runs below that bound are read: a run's values belong together - rows of one list - so the bound alone is a loose one.
+// 18,750 distances, 20 wanted, four blocks of 1,024 threads: 12.6 us without runs and with payloads one by one -> 10.1; 14,300, 200 wanted, 333
+// blocks of 256 (no runs) 32.6 -> 24; 256, 16 wanted, 1,000 blocks, which used to be ranked whole, 25 -> 4.8.
+// A radix selection is left for the rows the bound does not serve: too many equal values, fewer than k comparable ones, or k above what the
+// minima cover.
 template <int kThreads, typename Payload>   // kThreads: the block's threads, 256 or more
-__device__ int smallest(const float* __restrict__ vals, int n, int k, Payload payload, uint64_t* s_keys, int buffer, float* s_min, Words* w) {
+__device__ int smallest(const float* __restrict__ vals, int n, int k, Payload payload, uint64_t* s_keys, int buffer, int* s_runs, Words* w,
+                        const float* __restrict__ runs = nullptr) {
+    constexpr int PER = kMaxGroups / kThreads;
     const int tid = threadIdx.x, lane = tid & 31;
     const float inf = __int_as_float(0x7f800000);
-    const int keep = k < n ? k : n;
-    int per = (2 * k + kThreads - 1) / kThreads;   // subsets per thread
-    if (tid == 0) { w->cnt = 0; w->cut = inf; }
-    if (n > 2 * kThreads && per <= kMaxGroups / kThreads) {
-        if (per == 1) {
-            float m = inf;
-#pragma unroll 8
-            for (int i = tid; i < n; i += kThreads) m = fminf(m, vals[i]);
-            s_min[tid] = m;
-        } else {
-            for (int g = 0; g < per; ++g) {
-                float m = inf;
-#pragma unroll 4
-                for (int i = tid + g * kThreads; i < n; i += per * kThreads) m = fminf(m, vals[i]);
-                s_min[g * kThreads + tid] = m;
-            }
-        }
+    const int keep = k < n ? k : n, nruns = (n + kRun - 1) / kRun;
+    const int per = (2 * k + kThreads - 1) / kThreads;   // subsets per thread
+    float* s_min = reinterpret_cast<float*>(s_keys);     // [kMaxGroups]: the keys come later
+    auto bound = [&](int groups) {   // of s_min
         __syncthreads();
         if (tid < 32) {
-            const int groups = per * kThreads;
-            float mn = inf, mx = -inf;
-            for (int i = lane; i < groups; i += 32) { const float v = s_min[i]; mn = fminf(mn, v); if (v < inf) mx = fmaxf(mx, v); }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) { mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o)); mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); }
-            float lo = mn, hi = mx;
-            int c = groups;
-            for (int it = 0; it < 14 && mn < inf; ++it) {
-                const float mid = lo + 0.5f * (hi - lo);
-                c = 0;
-                for (int i = lane; i < groups; i += 32) c += s_min[i] <= mid ? 1 : 0;
-                c = __reduce_add_sync(0xffffffffu, c);
-                if (c >= k) hi = mid; else lo = mid;
-                if (c == k) break;
-            }
-            c = 0;
-            for (int i = lane; i < groups; i += 32) c += s_min[i] <= hi ? 1 : 0;
-            c = __reduce_add_sync(0xffffffffu, c);
-            if (lane == 0) w->cut = c >= k && mn < inf ? hi : inf;
+            const float at = groups <= kThreads ? bound_of<kThreads / 32>(s_min, groups, k) : bound_of<0>(s_min, groups, k);
+            if (lane == 0) w->cut = at;
+        }
+        __syncthreads();
+        return w->cut;
+    };
+    if (tid == 0) { w->cnt = 0; w->done = 0; w->cut = inf; }
+    bool some = false;      // only the runs of s_runs are looked at
+    int looked = n;
+    if (runs && nruns >= 2 * k && nruns <= kMaxGroups) {
+        for (int r = tid; r < nruns; r += kThreads) s_min[r] = runs[r];
+        const float at = bound(nruns);
+        if (at < inf) {
+            for (int r = tid; r < nruns; r += kThreads)
+                if (s_min[r] <= at) s_runs[atomicAdd(&w->done, 1)] = r;
+            __syncthreads();
+            some = true;
+            looked = w->done * kRun;
         }
     }
-    __syncthreads();
-    const float cut = w->cut;
-    if (cut < inf || n <= buffer) {
+    auto gather = [&](auto index) {   // index(e): the place of the e-th value looked at, n or more for none
+        float cut = inf;
+        if (looked > 4 * k && looked >= 96 && per <= PER) {
+            if (per == 1) {
+                float m = inf;
 #pragma unroll 8
-        for (int i = tid; i < n; i += kThreads) {
-            const float v = vals[i];
-            if (cut == inf || v <= cut) {
+                for (int e = tid; e < looked; e += kThreads) { const int i = index(e); if (i < n) m = fminf(m, vals[i]); }
+                s_min[tid] = m;
+            } else {
+                for (int g = 0; g < per; ++g) {
+                    float m = inf;
+#pragma unroll 4
+                    for (int e = tid + g * kThreads; e < looked; e += per * kThreads) { const int i = index(e); if (i < n) m = fminf(m, vals[i]); }
+                    s_min[g * kThreads + tid] = m;
+                }
+            }
+            cut = bound(per * kThreads);
+        } else {
+            __syncthreads();
+        }
+        if (cut == inf && looked > buffer) return cut;
+#pragma unroll 8
+        for (int e = tid; e < looked; e += kThreads) {
+            const int i = index(e);
+            const float v = i < n ? vals[i] : inf;
+            if (cut == inf ? i < n : v <= cut) {
                 const int pos = atomicAdd(&w->cnt, 1);
-                if (pos < buffer) s_keys[pos] = make_key(v, payload(i));
+                if (pos < buffer) s_keys[pos] = make_key(v, (uint32_t)i);
             }
         }
-    }
+        return cut;
+    };
+    const float cut = some ? gather([&](int e) { return s_runs[e / kRun] * kRun + e % kRun; }) : gather([](int e) { return e; });
     __syncthreads();
     int c = w->cnt;
+    // Payloads, which may be a search and two loads each, for all kept values at once.
+    if (c >= keep && c <= buffer)
+        for (int e = tid; e < c; e += kThreads) s_keys[e] = (s_keys[e] & ~0xffffffffull) | (uint32_t)payload((int)key_idx(s_keys[e]));
     __syncthreads();
     if (c < keep || c > buffer) {
         // The keep-th smallest value by radix over the values up to the cut, then all below it and of the equal ones those with the

@@ -3,6 +3,7 @@
 #include "batch_parts.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "select.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -502,7 +503,7 @@ struct psb_session {
     Tail* h_tail = nullptr;
     static_assert(kSmallIo + sizeof(Tail) <= kHostBlock, "the tail lies behind the block's data");
     bool counters_known = false;           // h_tail->c is what the device's counters hold
-    DevBuf row_dist, row_seg;              // a row of distances per query (IVF-Flat, row form of the ADC scan)
+    DevBuf row_dist, row_seg, row_runs, row_whole;   // a row of distances per query (IVF-Flat, row form of the ADC scan), the minima of every 32
     std::vector<long long> longest;        // [p] = rows of this shard's p longest lists together
     double own_list_rows = 0.0;            // expected length of the list a random row lies in
     std::unique_ptr<HostPool> host_pool;   // gather threads of the staged transport (created on first use)
@@ -800,8 +801,9 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, con
     g.stride = row_stride(s, nprobe, any_probes);
     const int most = (int)std::max<long long>(1, std::min(kPartQueries, kRowDistFloats / g.stride));
     const int parts = (nq + most - 1) / most, per = (nq + parts - 1) / parts;
-    PSB_TRY(s->row_dist.reserve(sizeof(float) * (size_t)per * g.stride));
-    PSB_TRY(s->row_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
+    g.run_stride = sel::run_count(g.stride);
+    PSB_TRY(reserve_together(&s->row_whole, {{&s->row_dist, sizeof(float) * (size_t)per * g.stride}, {&s->row_seg, sizeof(int) * (size_t)per * ((size_t)nprobe + 1)},
+                                             {&s->row_runs, sizeof(float) * (size_t)per * g.run_stride}}));
     const ScanIndex ix = s->scan_index();
     g.nprobe = nprobe; g.centroids = ix.centroids; g.codebook = ix.codebook; g.codes = ix.codes; g.offsets = ix.offsets; g.row_base = ix.row_base;
     g.row_delta = ix.row_delta; g.list_begin = ix.list_begin; g.list_end = ix.list_end; g.dim = ix.dim; g.m = ix.m; g.k = ix.k;
@@ -813,6 +815,7 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, con
         g.lut = d_lut ? d_lut + (size_t)q0 * table_count(s, 1, nprobe) * s->m * s->k : nullptr;
         g.out_rows = d_rows + (size_t)q0 * stage1_k; g.out_dist = d_dist ? d_dist + (size_t)q0 * stage1_k : nullptr;
         g.out_count = d_count ? d_count + q0 : nullptr;
+        g.runs = !ix.residual && std::min(per, nq - q0) <= sel::kRunQueries ? s->row_runs.as<float>() : nullptr;
         PSB_TRY(launch_adc_rows(g, std::min(per, nq - q0), st));
     }
     if (ws.ev_end) PSB_CUDA(cudaEventRecord(ws.ev_end, st));
@@ -2111,8 +2114,9 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     f.stride = std::max<long long>(1, s->longest[(size_t)nprobe]);
     const long long most = std::max<long long>(1, std::min(kPartQueries, kRowDistFloats / f.stride));
     const int parts = (int)((n + most - 1) / most), per = (n + parts - 1) / parts;
-    PSB_TRY(s->row_dist.reserve(sizeof(float) * (size_t)per * f.stride));
-    PSB_TRY(s->row_seg.reserve(sizeof(int) * (size_t)per * ((size_t)nprobe + 1)));
+    f.run_stride = sel::run_count(f.stride);
+    PSB_TRY(reserve_together(&s->row_whole, {{&s->row_dist, sizeof(float) * (size_t)per * f.stride}, {&s->row_seg, sizeof(int) * (size_t)per * ((size_t)nprobe + 1)},
+                                             {&s->row_runs, sizeof(float) * (size_t)per * f.run_stride}}));
     if (flat_list_form(per, nprobe, s->nlist, s->n_vectors, s->dim)) {
         PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
         PSB_TRY(s->flat_slot.reserve(sizeof(int) * (size_t)per * nprobe));
@@ -2127,6 +2131,7 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     for (int q0 = 0; q0 < n; q0 += per) {
         f.queries = dq + (size_t)q0 * s->dim; f.probes = s->probes.as<int>() + (size_t)q0 * nprobe;
         f.out_ids = d_ids + (size_t)q0 * topk; f.out_dist = d_dist + (size_t)q0 * topk;
+        f.runs = std::min(per, n - q0) <= sel::kRunQueries ? s->row_runs.as<float>() : nullptr;
         PSB_TRY(launch_flat_scan(f, std::min(per, n - q0), s->stream));
     }
     if (ev1) PSB_CUDA(cudaEventRecord(ev1, s->stream));

@@ -107,3 +107,27 @@ def test_parts_of_a_call(psb, n, nq):
     want = oracle.ivfrespq_search(ix, q[some], 2, 10, 20)
     assert np.array_equal(got["indices"][some], want["indices"]) and np.array_equal(got["distances"][some], want["distances"])
     assert got["stats"]["pq_scanned_codes"] == nq * n
+
+
+@pytest.mark.parametrize("nq", [1, 16, 17])                        # with and without the minima of 32 distances
+@pytest.mark.parametrize("near", [31, 32, 33, 700, 6000])          # rows that lie together: their runs alone would bound loosely
+@pytest.mark.parametrize("k", [1, 10, 100, 700])
+def test_runs_of_distances(psb, nq, near, k):
+    """Selections over runs: IVF-Flat, where a distance row is what the test makes it; equal distances across a run's end, lists of odd length."""
+    rng = np.random.default_rng(near + k)
+    dim, n = 12, 9001
+    vec = rng.integers(-8, 9, (n, dim)).astype(np.float32) * 4
+    vec[1000:1000 + near] = rng.integers(-1, 2, (near, dim))[: n - 1000]
+    off = np.array([0, 17, 1000, 1033, 7000, n], np.int64)
+    cen = rng.standard_normal((5, dim)).astype(np.float32)
+    ix = dict(centroids=cen, offsets=off, reordered_ids=rng.permutation(n).astype(np.int64), vectors=vec)
+    q = rng.integers(-1, 2, (nq, dim)).astype(np.float32)
+    with psb.FlatSession(ix, max_batch=nq) as s:
+        got = s.search(q, 5, k, batch_size=nq)
+    d = np.zeros((nq, n), np.float32)
+    for j in range(dim):
+        t = q[:, None, j] - vec[None, :, j]
+        d += t * t
+    order = np.lexsort((np.broadcast_to(np.arange(n), d.shape), d), axis=1)[:, :k]   # whole numbers: exact; ties by row
+    assert np.array_equal(got["indices"], ix["reordered_ids"][order])
+    assert np.array_equal(got["distances"], np.take_along_axis(d, order, 1))
