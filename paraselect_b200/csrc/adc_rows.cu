@@ -172,7 +172,7 @@ psb_status run_rows(const AdcRows& g, int nq, cudaStream_t s) {
 
 psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
-    PSB_TRY(launch_row_segments(g.probes, nq, g.nprobe, g.offsets, g.list_begin, g.list_end, g.seg, nullptr, nullptr, g.counters, s));
+    PSB_TRY(launch_row_segments(g.probes, nq, g.nprobe, g.offsets, g.list_begin, g.list_end, g.seg, nullptr, nullptr, g.counters, s, g.mark));
     switch (g.m) {
         case 8: PSB_TRY(run_rows<8>(g, nq, s)); break;
         case 16: PSB_TRY(run_rows<16>(g, nq, s)); break;

@@ -18,7 +18,8 @@ constexpr int BQ = 64, BC = 128, KC = 16, kDistThreads = 256;
 // dist[q][c] for a BQ x BC tile; each thread owns 4 queries x 8 centroids.
 __global__ void __launch_bounds__(kDistThreads)
 k_coarse_dist_exact(const float* __restrict__ queries, int nq, const float* __restrict__ centroids, int nlist,
-                    int dim, float* __restrict__ dist) {
+                    int dim, float* __restrict__ dist, unsigned long long* mark) {
+    mark_start(mark);
     __shared__ __align__(16) float qs[KC][BQ];
     __shared__ __align__(16) float cs[KC][BC];
     const int q0 = blockIdx.y * BQ, c0 = blockIdx.x * BC;
@@ -71,7 +72,9 @@ k_coarse_dist_exact(const float* __restrict__ queries, int nq, const float* __re
 // dimensions staged at once by 16-byte loads, one barrier.  A batch of 333 queries x 700 centroids x 100 dimensions is 36 of the large
 // tiles, each a chain of load, barrier and compute steps (38 us); a single query against 1,024 centroids took 24 us the same way.
 __global__ void __launch_bounds__(kSmallThreads)
-k_coarse_dist_small(const float* __restrict__ queries, int nq, const float* __restrict__ centroids, int nlist, int dim, float* __restrict__ dist) {
+k_coarse_dist_small(const float* __restrict__ queries, int nq, const float* __restrict__ centroids, int nlist, int dim, float* __restrict__ dist,
+                    unsigned long long* mark) {
+    mark_start(mark);
     extern __shared__ __align__(16) float s_small[];
     const int pitch = small_pitch(dim);
     float* qs = s_small;                  // [SQ][pitch]
@@ -100,13 +103,19 @@ k_coarse_dist_small(const float* __restrict__ queries, int nq, const float* __re
 // have four centroids each, one after the other.  With the selection behind it, tiles against this, us: 1,024 centroids x 96, 1 query 15.2 / 11.3,
 // 32 queries 17.2 / 14.3, 64 19.3 / 19.2, 128 19.1 / 25.3; 4,096, 8 queries 15.3 / 14.1, 16 16.3 / 17.2; 512 x 126, 64 queries 23.5 / 19.4; 256 x 96,
 // 128 queries 19.2 / 15.3: the line lies at 32,768 pairs.
-constexpr int kFewThreads = 64;
+constexpr int kFewThreads = kCoarseFewBlock;
 constexpr long long kFewPairs = 32768;
 __global__ void __launch_bounds__(kFewThreads)
-k_coarse_dist_few(const float* __restrict__ queries, const float* __restrict__ centroids, int nlist, int dim, float* __restrict__ dist) {
+k_coarse_dist_few(const float* __restrict__ queries, const float* __restrict__ centroids, int nlist, int dim, float* __restrict__ dist,
+                  unsigned long long* mark, float* __restrict__ copy) {
     extern __shared__ __align__(16) float s_q[];
     const int q = blockIdx.y, c = blockIdx.x * kFewThreads + threadIdx.x;
-    for (int d = threadIdx.x; d < dim; d += kFewThreads) s_q[d] = queries[(size_t)q * dim + d];
+    mark_start(mark);
+    for (int d = threadIdx.x; d < dim; d += kFewThreads) {
+        const float v = queries[(size_t)q * dim + d];
+        s_q[d] = v;
+        if (copy && blockIdx.x == 0) copy[(size_t)q * dim + d] = v;
+    }
     __syncthreads();
     if (c < nlist) dist[(size_t)q * nlist + c] = row_distance(s_q, centroids + (size_t)c * dim, dim, rows_vec(centroids, dim));
 }
@@ -128,13 +137,17 @@ k_select_rows(const float* __restrict__ dist, int n, int k, int buffer, int* __r
 
 }  // namespace
 
+bool coarse_few(int nq, int nlist, int dim) { return (long long)nq * nlist <= kFewPairs && nq <= 65535 && (size_t)dim * sizeof(float) <= (size_t)200 * 1024; }
+
 psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float* d_centroids, int nlist,
-                                    int dim, float* d_dist, int sm_count, cudaStream_t s) {
+                                    int dim, float* d_dist, int sm_count, cudaStream_t s, unsigned long long* mark, float* d_copy) {
     if (nq <= 0) return PSB_OK;
+    if (d_copy && !coarse_few(nq, nlist, dim)) return fail(PSB_INTERNAL, "host queries are for few pairs");
     const size_t smem = (size_t)((dim + 3) & ~3) * sizeof(float);
-    if ((long long)nq * nlist <= kFewPairs && nq <= 65535 && smem <= (size_t)200 * 1024) {
+    if (coarse_few(nq, nlist, dim)) {
         if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_coarse_dist_few), smem));
-        k_coarse_dist_few<<<dim3((unsigned)((nlist + kFewThreads - 1) / kFewThreads), (unsigned)nq), kFewThreads, smem, s>>>(d_queries, d_centroids, nlist, dim, d_dist);
+        k_coarse_dist_few<<<dim3((unsigned)((nlist + kFewThreads - 1) / kFewThreads), (unsigned)nq), kFewThreads, smem, s>>>(d_queries, d_centroids, nlist, dim, d_dist, mark,
+                                                                                                                                  d_copy);
         count_launch();
         PSB_LAUNCH_CHECK();
         return PSB_OK;
@@ -146,12 +159,12 @@ psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float*
     if ((long long)grid.x * grid.y < sm_count && small <= (size_t)200 * 1024) {
         const dim3 g2((nlist + SC - 1) / SC, (nq + SQ - 1) / SQ);
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_coarse_dist_small), small));
-        k_coarse_dist_small<<<g2, kSmallThreads, small, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist);
+        k_coarse_dist_small<<<g2, kSmallThreads, small, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist, mark);
         count_launch();
         PSB_LAUNCH_CHECK();
         return PSB_OK;
     }
-    k_coarse_dist_exact<<<grid, kDistThreads, 0, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist);
+    k_coarse_dist_exact<<<grid, kDistThreads, 0, s>>>(d_queries, nq, d_centroids, nlist, dim, d_dist, mark);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

@@ -106,6 +106,11 @@ inline psb_status prefer_max_shared(F kernel) {
     return kernel_carveout_max(reinterpret_cast<const void*>(kernel));
 }
 
+// ---- device: a kernel's start on the device's clock (nanoseconds), by its first thread ------------
+__device__ __forceinline__ void mark_start(unsigned long long* mark) {
+    if (mark && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(*mark));
+}
+
 // ---- device: block-wide bitonic sort of n (power of two) keys in shared memory, ascending ---------
 template <typename K>
 __device__ __forceinline__ void block_bitonic_sort(K* s, int n) {

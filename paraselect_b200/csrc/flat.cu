@@ -30,7 +30,8 @@ namespace {
 // among its list's visitors.
 __global__ void __launch_bounds__(128) k_row_segments(const int* __restrict__ probes, int nq, int nprobe, const long long* __restrict__ offsets, int lb, int le,
                                                     int* __restrict__ seg, int* __restrict__ vis_count, int* __restrict__ slot,
-                                                    unsigned long long* __restrict__ counters) {
+                                                    unsigned long long* __restrict__ counters, unsigned long long* mark) {
+    mark_start(mark);
     const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (q >= nq) return;
     int* s = seg + (size_t)q * (nprobe + 1);
@@ -201,8 +202,8 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
 }  // namespace
 
 psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const long long* d_offsets, int list_begin, int list_end, int* d_seg,
-                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s) {
-    k_row_segments<<<(unsigned)((nq + 3) / 4), 128, 0, s>>>(d_probes, nq, nprobe, d_offsets, list_begin, list_end, d_seg, d_vis_count, d_slot, d_counters);
+                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s, unsigned long long* mark) {
+    k_row_segments<<<(unsigned)((nq + 3) / 4), 128, 0, s>>>(d_probes, nq, nprobe, d_offsets, list_begin, list_end, d_seg, d_vis_count, d_slot, d_counters, mark);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

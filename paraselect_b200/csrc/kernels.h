@@ -27,8 +27,12 @@ inline int pool_capacity(int stage1_k) {
 // ---- coarse ---------------------------------------------------------------------------------------
 // Exact fp32 distance matrix tile: dist[q][c] = sum_d (queries[q][d] - centroids[c][d])^2 evaluated as the
 // sequential non-fused sum.  dist is [nq][nlist].
+// mark: where the kernel notes its start.  d_copy (coarse_few shapes only): the queries lie in page-locked host memory, and the kernel leaves a
+// copy of them there.
 psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float* d_centroids, int nlist,
-                                    int dim, float* d_dist, int sm_count, cudaStream_t s);
+                                    int dim, float* d_dist, int sm_count, cudaStream_t s, unsigned long long* mark = nullptr, float* d_copy = nullptr);
+bool coarse_few(int nq, int nlist, int dim);   // so few pairs that a thread takes one each
+constexpr int kCoarseFewBlock = 64;            // centroids behind one read of a query
 // Per query the k smallest (distance, id) pairs of a [nq][n] distance matrix, sorted ascending.
 psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_ids, float* d_out,
                               cudaStream_t s);
@@ -257,7 +261,7 @@ psb_status launch_scan(const ScanIndex& ix, const ScanWorkspace& ws, const float
 // outside [list_begin, list_end) have none).  d_slot (may be null) [nq * nprobe]: the pair's place among its list's visitors, counted in
 // d_vis_count.  d_counters[0] += rows.
 psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const long long* d_offsets, int list_begin, int list_end, int* d_seg,
-                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s);
+                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s, unsigned long long* mark = nullptr);
 // The ADC scan in its row form: all distances, then the stage1_k smallest.
 struct AdcRows {
     const float* queries; const int* probes; int nprobe;
@@ -271,6 +275,7 @@ struct AdcRows {
     float* runs; long long run_stride;              // workspace, plain mode: [nq][run_stride], the minimum of every 32 distances
     double expected_rows; long long longest_list;   // rows a query is expected to scan; rows of the longest list
     unsigned long long* counters;
+    unsigned long long* mark;                       // the scan's start is noted there (may be null)
     int sm_count;
 };
 psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s);
@@ -342,7 +347,10 @@ psb_status launch_gather_unique(const void* src, int row_bytes, const int* d_uni
 // their number, else by their slot.
 psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
                                const int* d_candidates, int nq, int candidate_count, int candidate_stride,
-                               const int* d_counts, float* d_out_dist, cudaStream_t s);
+                               const int* d_counts, float* d_out_dist, cudaStream_t s, unsigned long long* mark = nullptr);
+// The end of a call: the session's 16 counter and status words, 8 words of the coarse stage (may be null) and the time go to page-locked host memory.
+struct CallTail { unsigned long long c[16]; int tc[8]; unsigned long long end; };
+psb_status launch_call_tail(const unsigned long long* d_words, const int* d_coarse, CallTail* h_tail, cudaStream_t s);
 // Per query the topk (distance,row) pairs without duplicates from d_dist [nq][candidate_count]; with d_ids (original ids by row)
 // d_out_ids [nq][topk] is written instead of d_out_rows.
 psb_status launch_topk_select(const float* d_dist, const int* d_candidates, int nq, int candidate_count,

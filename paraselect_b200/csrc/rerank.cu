@@ -126,6 +126,13 @@ __global__ void __launch_bounds__(kPlaceThreads) k_place_rows(const unsigned* __
     }
 }
 
+// A copy to the host behind the last kernel took 3 us of copy engine and 8 of waiting for it.
+__global__ void k_call_tail(const unsigned long long* __restrict__ words, const int* __restrict__ coarse, CallTail* tail) {
+    mark_start(&tail->end);
+    if (threadIdx.x < 16) tail->c[threadIdx.x] = words[threadIdx.x];
+    if (coarse && threadIdx.x < 8) tail->tc[threadIdx.x] = coarse[threadIdx.x];
+}
+
 __global__ void k_release_rows(const int* __restrict__ unique, const int* __restrict__ n_unique, int* __restrict__ slot_of) {
     const int n = *n_unique;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) slot_of[unique[i]] = -1;
@@ -258,7 +265,8 @@ __host__ __device__ __forceinline__ int score_pitch(int row_bytes) { return (row
 __global__ void __launch_bounds__(kScoreThreads)
 k_rerank_score(const unsigned char* __restrict__ src, const int* __restrict__ slot_of, RowMap mp, int dim, int elem_bytes, int through,
                const unsigned char* __restrict__ queries, const int* __restrict__ cand, int candidate_count,
-               int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist) {
+               int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist, unsigned long long* mark) {
+    mark_start(mark);
     extern __shared__ __align__(16) unsigned char s_score[];
     const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row_bytes = dim * elem_bytes, pitch = score_pitch(row_bytes);
@@ -327,7 +335,8 @@ template <bool U8>
 __global__ void __launch_bounds__(kScoreThreads, 6)
 k_rerank_score_wide(const unsigned char* __restrict__ src, const int* __restrict__ slot_of, RowMap mp, int dim,
                     const unsigned char* __restrict__ queries, const int* __restrict__ cand, int candidate_count,
-                    int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist) {
+                    int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist, unsigned long long* mark) {
+    mark_start(mark);
     extern __shared__ __align__(16) unsigned char s_score[];
     const int q = blockIdx.x, lane = threadIdx.x & 31, l = lane & 7;
     const int units = (U8 ? dim : dim * 4) >> 4;
@@ -558,7 +567,7 @@ psb_status launch_gather_unique(const void* src, int row_bytes, const int* d_uni
 
 psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
                                const int* d_candidates, int nq, int candidate_count, int candidate_stride,
-                               const int* d_counts, float* d_out_dist, cudaStream_t s) {
+                               const int* d_counts, float* d_out_dist, cudaStream_t s, unsigned long long* mark) {
     if (nq <= 0) return PSB_OK;
     const int row_bytes = dim * elem_bytes;
     const dim3 grid(nq, (candidate_count + kScoreBlock - 1) / kScoreBlock);
@@ -567,7 +576,7 @@ psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const Ro
         PSB_TRY(prefer_max_shared(kernel));
         kernel<<<grid, kScoreThreads, row_bytes, s>>>(
             static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, static_cast<const unsigned char*>(d_queries), d_candidates, candidate_count,
-            candidate_stride, d_counts, d_out_dist);
+            candidate_stride, d_counts, d_out_dist, mark);
         count_launch();
         PSB_LAUNCH_CHECK();
         return PSB_OK;
@@ -581,7 +590,15 @@ psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const Ro
     PSB_TRY(prefer_max_shared(k_rerank_score));
     k_rerank_score<<<grid, kScoreThreads, smem, s>>>(
         static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, elem_bytes, through, static_cast<const unsigned char*>(d_queries),
-        d_candidates, candidate_count, candidate_stride, d_counts, d_out_dist);
+        d_candidates, candidate_count, candidate_stride, d_counts, d_out_dist, mark);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+
+psb_status launch_call_tail(const unsigned long long* d_words, const int* d_coarse, CallTail* h_tail, cudaStream_t s) {
+    PSB_TRY(prefer_max_shared(k_call_tail));
+    k_call_tail<<<1, 32, 0, s>>>(d_words, d_coarse, h_tail);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

@@ -499,8 +499,13 @@ struct psb_session {
     // Host side of a search call: one pinned block through which a small batch's queries and results pass, and the device's counters
     // and status words with the results, so that a call waits for the GPU once.
     unsigned char* h_io = nullptr;         // a block of HostBlocks: kSmallIo bytes, then the tail
-    struct Tail { unsigned long long c[16]; int tc[8]; };
+    using Tail = CallTail;
     Tail* h_tail = nullptr;
+    // Of the call at work (CallMarks): words of `scalars` in which its kernels note the starts of the coarse stage, the scan and the rerank, and
+    // the queries, which the first kernel reads from the page-locked block, leaving a copy.  Null: events mark, a copy brings.
+    unsigned long long* call_marks = nullptr;
+    const float* host_queries = nullptr;
+    float* query_copy = nullptr;
     static_assert(kSmallIo + sizeof(Tail) <= kHostBlock, "the tail lies behind the block's data");
     bool counters_known = false;           // h_tail->c is what the device's counters hold
     DevBuf row_dist, row_seg, row_runs, row_whole;   // a row of distances per query (IVF-Flat, row form of the ADC scan), the minima of every 32
@@ -809,6 +814,7 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, con
     g.row_delta = ix.row_delta; g.list_begin = ix.list_begin; g.list_end = ix.list_end; g.dim = ix.dim; g.m = ix.m; g.k = ix.k;
     g.residual = ix.residual; g.tree = scan_tree_order(ix); g.stage1_k = stage1_k; g.seg = s->row_seg.as<int>(); g.dist = s->row_dist.as<float>();
     g.expected_rows = expected_rows(s, nprobe); g.longest_list = s->longest[1]; g.counters = ws.counters; g.sm_count = s->sm_count;
+    g.mark = s->call_marks ? s->call_marks + 1 : nullptr;
     if (ws.ev_begin) PSB_CUDA(cudaEventRecord(ws.ev_begin, st));
     for (int q0 = 0; q0 < nq; q0 += per) {
         g.queries = d_queries + (size_t)q0 * s->dim; g.probes = d_probes + (size_t)q0 * nprobe;
@@ -836,9 +842,10 @@ psb_status ensure_pipeline_ws(psb_session* s, int nq, int nprobe, int topk, int 
 
 // Coarse stage on device queries: exact distance tiles + row selection, query-chunked so the distance tile
 // stays below ~1 GiB.
+bool coarse_by_tc(const psb_session* s, int nq, int nprobe) { return s->tc_index.ready && coarse_tc_supported(nq, s->nlist, s->dim, nprobe); }
 psb_status coarse_exact(psb_session* s, const float* d_queries, int nq, int nprobe, int* d_ids, float* d_dist) {
     const int mode = s->opt.coarse_mode;
-    const bool tc_ok = s->tc_index.ready && coarse_tc_supported(nq, s->nlist, s->dim, nprobe);
+    const bool tc_ok = coarse_by_tc(s, nq, nprobe);
     if (mode == 2 && !tc_ok) return fail(PSB_UNSUPPORTED_SHAPE, "tensor-core coarse stage does not support this shape");
     if (mode != 1 && tc_ok) {
         PSB_TRY(s->tc_work.ensure(nq, s->nlist, s->dim, nprobe, s->device, s->stream));
@@ -858,8 +865,8 @@ psb_status coarse_exact(psb_session* s, const float* d_queries, int nq, int npro
     PSB_TRY(s->dist_tile.reserve(row_bytes * (size_t)chunk));
     for (int q0 = 0; q0 < nq; q0 += chunk) {
         const int n = std::min(chunk, nq - q0);
-        PSB_TRY(launch_coarse_dist_exact(d_queries + (size_t)q0 * s->dim, n, s->centroids.as<float>(), s->nlist, s->dim,
-                                         s->dist_tile.as<float>(), s->sm_count, s->stream));
+        PSB_TRY(launch_coarse_dist_exact(s->host_queries ? s->host_queries : d_queries + (size_t)q0 * s->dim, n, s->centroids.as<float>(), s->nlist, s->dim,
+                                         s->dist_tile.as<float>(), s->sm_count, s->stream, q0 == 0 ? s->call_marks : nullptr, s->query_copy));
         PSB_TRY(launch_select_rows(s->dist_tile.as<float>(), n, s->nlist, nprobe, d_ids + (size_t)q0 * nprobe,
                                    d_dist ? d_dist + (size_t)q0 * nprobe : nullptr, s->stream));
     }
@@ -1083,7 +1090,7 @@ bool rows_in_place(const psb_session* s, long long requests) {
 psb_status score_and_select(psb_session* s, bool in_place, const void* d_queries, int nq, const int* d_cand, int width, int stride, const int* d_counts,
                             int topk, int* d_out_rows, float* d_out_dist, long long* d_out_ids, float* d_score, cudaStream_t st) {
     PSB_TRY(launch_rerank_score(in_place ? s->exact_dev : s->stage.p, in_place ? nullptr : s->slot_of.as<int>(), s->row_map(), s->dim, s->exact_elem,
-                                d_queries, d_cand, nq, width, stride, d_counts, d_score, st));
+                                d_queries, d_cand, nq, width, stride, d_counts, d_score, st, s->call_marks ? s->call_marks + 2 : nullptr));
     if (!d_out_rows && !d_out_ids) return PSB_OK;  // partial rerank: the caller combines the scores of all shards
     return launch_topk_select(d_score, d_cand, nq, width, stride, d_counts, topk, d_out_rows, d_out_dist, st, s->reordered.as<long long>(), d_out_ids);
 }
@@ -1645,10 +1652,29 @@ psb_status ensure_host_io(psb_session* s) {
 }
 // Queues the device's counters and status words behind the work on `st`.
 psb_status queue_tail(psb_session* s, cudaStream_t st) {
-    PSB_CUDA(cudaMemcpyAsync(s->h_tail->c, s->scalars.p, sizeof(s->h_tail->c), cudaMemcpyDeviceToHost, st));
-    if (s->tc_work.scalars.p) PSB_CUDA(cudaMemcpyAsync(s->h_tail->tc, s->tc_work.scalars.p, sizeof(s->h_tail->tc), cudaMemcpyDeviceToHost, st));
-    return PSB_OK;
+    return launch_call_tail(s->scalars.as<unsigned long long>(), s->tc_work.scalars.as<int>(), s->h_tail, st);
 }
+// Small calls on one stream: the kernels note their starts themselves and the first reads the queries where they are.  A recorded event costs the
+// GPU five microseconds between two kernels and the host two, and a small copy to the device as much again.
+struct CallMarks {
+    psb_session* s;
+    bool on;
+    CallMarks(psb_session* s_, bool on_, const float* h_queries, int n) : s(s_), on(on_) {
+        if (!on) return;
+        s->call_marks = s->scalars.as<unsigned long long>() + 13;
+        // every 64 centroids are behind a read of the queries over PCIe: up to 64 KB of reads
+        if (coarse_few(n, s->nlist, s->dim) && (size_t)n * s->dim * sizeof(float) * ((s->nlist + kCoarseFewBlock - 1) / kCoarseFewBlock) <= 65536) {
+            s->host_queries = h_queries;
+            s->query_copy = s->q.as<float>();
+        }
+    }
+    ~CallMarks() { s->call_marks = nullptr; s->host_queries = nullptr; s->query_copy = nullptr; }
+    double ms(int from, int to) const {   // 0: coarse stage, 1: scan, 2: rerank, 3: end
+        const psb_session::Tail& t = *s->h_tail;
+        const unsigned long long a = t.c[13 + from], b = to == 3 ? t.end : t.c[13 + to];
+        return b > a ? (double)(b - a) * 1e-6 : 0.0;
+    }
+};
 // The counters as they are before a call: what the last call left, unless others have run in between.
 psb_status counters_before(psb_session* s, cudaStream_t st, unsigned long long (&c)[4]) {
     if (!s->counters_known) {
@@ -1962,6 +1988,10 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
                  b_ids = sizeof(long long) * (size_t)total * topk, b_dist = sizeof(float) * (size_t)total * topk;
     const bool small = batch == total && b_q + b_u8 + b_ids + b_dist <= kSmallIo;
     PSB_TRY(ensure_host_io(s));
+    const bool one_stream = total < 2048 && sub_batch_rows(s, total, nprobe, false) >= total;
+    CallMarks marks(s, small && one_stream && rows_form(s, total, nprobe) && !coarse_by_tc(s, total, nprobe) &&
+                           (!rerank || rows_in_place(s, (long long)total * stage1_k)), reinterpret_cast<const float*>(s->h_io), total);
+    const bool timed = stats && !marks.on;   // by events
     const long long launches0 = launches_total();
     unsigned long long c0[4] = {0, 0, 0, 0};
     if (stats) PSB_TRY(counters_before(s, st, c0));
@@ -1977,7 +2007,7 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
     for (int q0 = 0; q0 < total; q0 += batch, ++nb) {
         const int n = std::min(batch, total - q0);
         cudaEvent_t t_begin = nullptr, t_in = nullptr, t_done = nullptr;
-        if (stats) { PSB_TRY(times.mark(st)); t_begin = times.last; }
+        if (timed) { PSB_TRY(times.mark(st)); t_begin = times.last; }
         const void* from = queries->fp32 + (size_t)q0 * s->dim;
         const void* from_u8 = u8 ? queries->u8 + (size_t)q0 * s->dim : nullptr;
         if (small) {
@@ -1985,18 +2015,18 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
             from = s->h_io;
             if (u8) { std::memcpy(s->h_io + b_q, from_u8, (size_t)n * s->dim); from_u8 = s->h_io + b_q; }
         }
-        PSB_CUDA(cudaMemcpyAsync(s->q.p, from, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
+        if (!s->host_queries) PSB_CUDA(cudaMemcpyAsync(s->q.p, from, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
         h2d += (long long)sizeof(float) * n * s->dim;
         if (u8) {
             PSB_CUDA(cudaMemcpyAsync(s->q_u8.p, from_u8, (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
             h2d += (long long)n * s->dim;
         }
-        if (stats) { PSB_TRY(times.mark(st)); t_in = times.last; }
+        if (timed) { PSB_TRY(times.mark(st)); t_in = times.last; }
         const void* qe = s->exact_elem == 1 ? s->q_u8.p : s->q.p;
         long long* ids = small ? reinterpret_cast<long long*>(s->h_io + b_q + b_u8) : s->out_ids.as<long long>();
         float* dist = small ? reinterpret_cast<float*>(s->h_io + b_q + b_u8 + b_ids) : s->out_dist.as<float>();
-        PSB_TRY(search_device(s, s->q.as<float>(), qe, n, nprobe, topk, stage1_k, rerank, ids, dist, s->probes.as<int>(), stats ? &times : nullptr));
-        if (stats) { PSB_TRY(times.begin(st)); t_done = times.last; }
+        PSB_TRY(search_device(s, s->q.as<float>(), qe, n, nprobe, topk, stage1_k, rerank, ids, dist, s->probes.as<int>(), timed ? &times : nullptr));
+        if (timed) { PSB_TRY(times.begin(st)); t_done = times.last; }
         if (!small) {
             PSB_CUDA(cudaMemcpyAsync(output->indices + (size_t)q0 * topk, ids, sizeof(long long) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
             PSB_CUDA(cudaMemcpyAsync(output->distances + (size_t)q0 * topk, dist, sizeof(float) * (size_t)n * topk, cudaMemcpyDeviceToHost, st));
@@ -2007,19 +2037,25 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
             d2h += (long long)sizeof(int) * n * nprobe;
         }
         if (q0 + batch >= total) PSB_TRY(queue_tail(s, st));
-        if (stats) PSB_TRY(times.mark(st));
+        if (timed) PSB_TRY(times.mark(st));
         PSB_CUDA(cudaStreamSynchronize(st));
         if (small) {
             std::memcpy(output->indices, ids, b_ids);
             std::memcpy(output->distances, dist, b_dist);
         }
-        if (stats) {
+        if (timed) {
             auto span = [](cudaEvent_t a, cudaEvent_t b) { float t = 0.f; cudaEventElapsedTime(&t, a, b); return (double)t; };
             t_h2d += span(t_begin, t_in); t_d2h += span(t_done, times.last); t_total += span(t_begin, times.last);
             times.collect();
         }
     }
     PSB_TRY(check_tail(s));
+    if (stats && marks.on) {
+        times.ms[StageTimes::kCoarse] = marks.ms(0, 1);
+        times.ms[StageTimes::kScan] = marks.ms(1, rerank ? 2 : 3);
+        if (rerank) times.ms[StageTimes::kRerank] = marks.ms(2, 3);
+        t_total = marks.ms(0, 3);
+    }
     if (stats) {
         const unsigned long long* c1 = s->h_tail->c;
         stats->h2d_ms = t_h2d; stats->coarse_search_ms = times.ms[StageTimes::kCoarse]; stats->pq_lut_build_ms = times.ms[StageTimes::kLut];
@@ -2180,19 +2216,21 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
                  b_dist = sizeof(float) * (size_t)total * topk;
     const bool small = batch == total && b_q + b_ids + b_dist <= kSmallIo;   // through the pinned block, as psb_session_search
     PSB_TRY(ensure_host_io(s));
+    CallMarks marks(s, small && !coarse_by_tc(s, total, nprobe), reinterpret_cast<const float*>(s->h_io), total);
+    const bool timed = stats && !marks.on;   // by events
     const long long launches0 = launches_total();
     unsigned long long c0[4] = {0, 0, 0, 0};
     if (stats) PSB_TRY(counters_before(s, st, c0));
     s->counters_known = false;
     s->timing.used = 0;
     EventTimer tm(&s->timing);
-    if (stats) PSB_TRY(tm.mark(st));
+    if (timed) PSB_TRY(tm.mark(st));
     int nb = 0;
     for (int q0 = 0; q0 < total; q0 += batch, ++nb) {
         const int n = std::min(batch, total - q0);
         const void* from = queries->fp32 + (size_t)q0 * s->dim;
         if (small) { std::memcpy(s->h_io, from, sizeof(float) * (size_t)n * s->dim); from = s->h_io; }
-        PSB_CUDA(cudaMemcpyAsync(s->q.p, from, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
+        if (!s->host_queries) PSB_CUDA(cudaMemcpyAsync(s->q.p, from, sizeof(float) * (size_t)n * s->dim, cudaMemcpyHostToDevice, st));
         long long* ids = small ? reinterpret_cast<long long*>(s->h_io + b_q) : s->out_ids.as<long long>();
         float* dist = small ? reinterpret_cast<float*>(s->h_io + b_q + b_ids) : s->out_dist.as<float>();
         PSB_TRY(flat_search_device(s, s->q.as<float>(), n, nprobe, topk, ids, dist));
@@ -2204,7 +2242,7 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
             PSB_CUDA(cudaMemcpyAsync(output->coarse_ids + (size_t)q0 * nprobe, s->probes.p, sizeof(int) * (size_t)n * nprobe, cudaMemcpyDeviceToHost, st));
         if (q0 + batch >= total) {
             PSB_TRY(queue_tail(s, st));
-            if (stats) PSB_TRY(tm.mark(st));
+            if (timed) PSB_TRY(tm.mark(st));
         }
         PSB_CUDA(cudaStreamSynchronize(st));  // the batch buffers are reused
         if (small) {
@@ -2214,7 +2252,7 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
     }
     PSB_TRY(check_tail(s));
     if (stats) {
-        stats->total_ms = tm.ms(0, 1);
+        stats->total_ms = timed ? tm.ms(0, 1) : marks.ms(0, 3);
         stats->pq_scanned_codes = (long long)(s->h_tail->c[0] - c0[0]);  // rows scanned
         stats->h2d_bytes = (long long)sizeof(float) * total * s->dim;
         stats->d2h_bytes = (long long)(sizeof(long long) + sizeof(float)) * total * topk;

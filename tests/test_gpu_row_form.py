@@ -131,3 +131,18 @@ def test_runs_of_distances(psb, nq, near, k):
     order = np.lexsort((np.broadcast_to(np.arange(n), d.shape), d), axis=1)[:, :k]   # whole numbers: exact; ties by row
     assert np.array_equal(got["indices"], ix["reordered_ids"][order])
     assert np.array_equal(got["distances"], np.take_along_axis(d, order, 1))
+
+
+@pytest.mark.parametrize("nq", [1, 5, 90, 600])    # queries read where they are, copied for the coarse stage's threads, for its tiles
+@pytest.mark.parametrize("rerank", [0, 40])
+def test_small_calls_mark_their_own_times(psb, nq, rerank):
+    ix = synth.make_index(6000, 24, 70, 6, seed=5)
+    q = synth.make_queries(ix, nq, seed=nq)
+    want = oracle.ivfpq_search(ix, q, 6, 10, rerank)
+    with psb.Session(ix, n_rerank=rerank, max_batch=nq) as s:
+        for _ in range(2):
+            got = s.search(q, 6, 10, batch_size=nq)
+            assert np.array_equal(got["indices"], want["indices"]) and np.array_equal(got["distances"], want["distances"])
+            t = got["stats"]
+            stages = [t["coarse_search_ms"], t["pq_adc_scan_ms"]] + ([t["pq_rerank_ms"]] if rerank else [])
+            assert min(stages) > 0 and sum(stages) <= t["total_ms"] * 1.0001 + 0.01 and t["total_ms"] < 1000
