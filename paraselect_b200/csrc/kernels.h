@@ -33,6 +33,9 @@ psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float*
                                     int dim, float* d_dist, int sm_count, cudaStream_t s, unsigned long long* mark = nullptr, float* d_copy = nullptr);
 bool coarse_few(int nq, int nlist, int dim);   // so few pairs that a thread takes one each
 constexpr int kCoarseFewBlock = 64;            // centroids behind one read of a query
+// The nearest of k centroids to each of n rows, with the same distances; rows of up to nearest_rows_fit() dimensions.
+bool nearest_rows_fit(int dim);
+psb_status launch_nearest_rows(const float* d_rows, int n, const float* d_centroids, int k, int dim, int* d_ids, float* d_dist, cudaStream_t s);
 // Per query the k smallest (distance, id) pairs of a [nq][n] distance matrix, sorted ascending.
 psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_ids, float* d_out,
                               cudaStream_t s);

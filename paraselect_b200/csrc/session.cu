@@ -2445,6 +2445,11 @@ public:
 private:
     static constexpr size_t kKeepRows = (size_t)4 << 30;
     psb_status exact(const float* d_centroids, int* d_assign, float* d_best) {
+        if (nearest_rows_fit(dim_)) {
+            for (int64_t r0 = 0; r0 < n_; r0 += 1 << 30)
+                PSB_TRY(launch_nearest_rows(data_ + (size_t)r0 * dim_, (int)std::min<int64_t>(1 << 30, n_ - r0), d_centroids, k_, dim_, d_assign + r0, d_best + r0, st_));
+            return PSB_OK;
+        }
         const size_t row_bytes = sizeof(float) * (size_t)k_;
         const int64_t chunk = std::min<int64_t>((int64_t)std::max<size_t>(64, ((size_t)1 << 30) / row_bytes), n_);
         PSB_TRY(tile_.reserve(row_bytes * (size_t)chunk, device_, st_));

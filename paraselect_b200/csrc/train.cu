@@ -95,7 +95,9 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
 // codeword so far, a draw r in [0, sum), and the first row at which the running sum reaches r.  On one host thread this took 0.5 s
 // for 32,768 rows x 24 sub-quantisers, 98 % of a codebook training.  Here a cluster of eight CTAs holds a sub-quantiser's rows and
 // their distances in shared memory (rows that do not fit are read through L2); a pick is one update of the distances, two cluster
-// barriers and a search in one warp's stretch of rows: 5.6 us (32,768 rows, 24 sub-quantisers), 255 picks, every sub-quantiser on SMs of its own.
+// barriers and a search in one warp's stretch of rows, of which the lanes take eighths of 32 one after the other; the warp that finds the row
+// hands it round with its values: 4.3 us (32,768 rows, 24 sub-quantisers; 5.6 with values from global memory, rows read word by word and a
+// stretch walked 32 rows a step), 255 picks, every sub-quantiser on SMs of its own.
 // The draws are made by the host (they do not depend on the data).  The rows picked are the reference's: its sequential sum and the
 // tree sum used here each stay within (n + 64) 2^-53 of the exact one, so when r is further than three times that from the
 // borders of the row found, the sequential search finds the same row; when it is not (about one draw in a million), one thread
@@ -112,6 +114,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 __device__ __forceinline__ void cluster_store(uint32_t a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 __device__ __forceinline__ void cluster_store(uint32_t a, int v) { asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void cluster_store(uint32_t a, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
 __device__ __forceinline__ float cluster_load(uint32_t a) {
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
@@ -134,12 +137,13 @@ k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, in
     extern __shared__ __align__(16) float s_seed[];
     const int dsub = D > 0 ? D : dsub_rt;
     float* s_min = s_seed;                                  // [per] distance of each row to its nearest codeword so far
-    float* s_rows = s_seed + (per + 3) / 4 * 4;             // [per][dsub] when staged
+    float* s_rows = s_seed + (per + 511) / 256 * 256;       // [per][dsub] when staged; the search reads up to 255 places past a stretch's end
     __shared__ double s_sum[kSeedCluster * kSeedCtaWarps];  // every warp's sum, of all eight CTAs
     __shared__ int s_pick;
+    __shared__ float s_cen[D > 0 ? D : 1];
     const int sub = blockIdx.y, rank = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = min(n, rank * per), cnt = min(n, b + per) - b;
-    const int wper = ((per + kSeedCtaWarps - 1) / kSeedCtaWarps + 31) / 32 * 32;   // a warp's stretch of rows
+    const int wper = ((per + kSeedCtaWarps - 1) / kSeedCtaWarps + 31) / 32 * 32;   // a warp's stretch of rows: begins on a vector
     const int w0 = min(cnt, warp * wper), w1 = min(cnt, w0 + wper);
     const float* src = data + (size_t)sub * dsub;
     if (staged)
@@ -149,21 +153,44 @@ k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, in
     int pick = first[sub];
     if (rank == 0 && tid == 0) out[0] = pick;
     __syncthreads();
+    // A row's values: whole vectors where rows lie on their boundaries (staged ones of 2, 4, 8, 12, 16 dimensions).
+    auto row_of = [&](int r, float (&x)[D > 0 ? D : 1]) {
+        if constexpr (D > 0) {
+            if (!staged) {
+#pragma unroll
+                for (int d = 0; d < D; ++d) x[d] = __ldg(src + (size_t)(b + r) * dim + d);
+            } else if constexpr (D % 4 == 0) {
+#pragma unroll
+                for (int d = 0; d < D; d += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(s_rows + (size_t)r * D + d);
+                    x[d] = v.x; x[d + 1] = v.y; x[d + 2] = v.z; x[d + 3] = v.w;
+                }
+            } else if constexpr (D % 2 == 0) {
+#pragma unroll
+                for (int d = 0; d < D; d += 2) { const float2 v = *reinterpret_cast<const float2*>(s_rows + (size_t)r * D + d); x[d] = v.x; x[d + 1] = v.y; }
+            } else {
+#pragma unroll
+                for (int d = 0; d < D; ++d) x[d] = s_rows[(size_t)r * D + d];
+            }
+        }
+    };
+    float cv[D > 0 ? D : 1];
+    if constexpr (D > 0) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) cv[d] = __ldg(src + (size_t)pick * dim + d);
+    }
     for (int c = 1; c < keff; ++c) {
         const float* cen = src + (size_t)pick * dim;
-        float cv[D > 0 ? D : 1];
-        if constexpr (D > 0) {
-#pragma unroll
-            for (int d = 0; d < D; ++d) cv[d] = __ldg(cen + d);
-        }
         double sum = 0.0;
         for (int r = w0 + lane; r < w1; r += 32) {
-            const float* x = staged ? s_rows + (size_t)r * dsub : src + (size_t)(b + r) * dim;
             float acc = 0.0f;
             if constexpr (D > 0) {
+                float x[D];
+                row_of(r, x);
 #pragma unroll
                 for (int d = 0; d < D; ++d) { const float diff = __fsub_rn(x[d], cv[d]); acc = __fadd_rn(acc, __fmul_rn(diff, diff)); }
             } else {
+                const float* x = staged ? s_rows + (size_t)r * dsub : src + (size_t)(b + r) * dim;
                 for (int d = 0; d < dsub; ++d) { const float diff = __fsub_rn(x[d], __ldg(cen + d)); acc = __fadd_rn(acc, __fmul_rn(diff, diff)); }
             }
             float m = c == 1 ? acc : s_min[r];
@@ -198,18 +225,37 @@ k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, in
             int found = -1;
             bool sure = false;
             double run = before;
-            for (int r0 = w0; r0 < w1; r0 += 32) {
-                const int row = r0 + lane;
-                const double x = row < w1 ? (double)s_min[row] : 0.0;
-                const double in = warp_inclusive(x, lane) + run;
+            for (int r0 = w0; r0 < w1; r0 += 256) {   // eight rows a lane
+                const int row = r0 + lane * 8;
+                double x[8], mine = 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(s_min + row + i);   // (the last stretch may reach past the rows: into what lies behind them)
+                    x[i] = v.x; x[i + 1] = v.y; x[i + 2] = v.z; x[i + 3] = v.w;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { if (row + i >= w1) x[i] = 0.0; mine += x[i]; }
+                const double in = warp_inclusive(mine, lane) + run;
                 const unsigned hit = __ballot_sync(0xffffffffu, row < w1 && in >= r);
                 if (hit) {
                     const int l = __ffs((int)hit) - 1;
-                    const double hi = __shfl_sync(0xffffffffu, in, l);
-                    const double lo = __shfl_up_sync(0xffffffffu, in, 1);
-                    const double below = l ? __shfl_sync(0xffffffffu, lo, l) : run;
-                    found = b + r0 + l;
-                    sure = hi - r > slack && (r - below > slack || found == 0);
+                    const double upto = __shfl_up_sync(0xffffffffu, in, 1);
+                    if (lane == l) {   // one of this lane's rows
+                        double below = lane ? upto : run, hi = below;
+                        int i = 0;
+                        bool there = false;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (there) continue;
+                            const double next = below + x[j];
+                            if (next < r && j < 7 && row + j + 1 < w1) { below = next; i = j + 1; }
+                            else { hi = next; there = true; }
+                        }
+                        found = b + row + i;
+                        sure = hi - r > slack && (r - below > slack || found == 0);
+                    }
+                    found = __shfl_sync(0xffffffffu, found, l);
+                    sure = __shfl_sync(0xffffffffu, sure ? 1 : 0, l) != 0;
                     break;
                 }
                 run = __shfl_sync(0xffffffffu, in, 31);
@@ -228,56 +274,78 @@ k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, in
                 }
                 found = __shfl_sync(0xffffffffu, found, 0);
             }
-            if (lane < kSeedCluster) cluster_store(cluster_addr(&s_pick, lane), found);
+            if (lane < kSeedCluster) {
+                cluster_store(cluster_addr(&s_pick, lane), found);
+                if constexpr (D > 0) {
+                    float x[D];   // (the sequential search may have found a row of another CTA)
+                    if (found >= b && found < b + cnt) row_of(found - b, x);
+                    else {
+#pragma unroll
+                        for (int d = 0; d < D; ++d) x[d] = __ldg(src + (size_t)found * dim + d);
+                    }
+#pragma unroll
+                    for (int d = 0; d < D; ++d) cluster_store(cluster_addr(&s_cen[d], lane), x[d]);
+                }
+            }
             if (lane == 0) out[c] = found;
         }
         cluster_sync();
         pick = s_pick;
+        if constexpr (D > 0) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) cv[d] = s_cen[d];
+        }
     }
     for (int c = keff + tid; rank == 0 && c < k; c += kSeedCtaThreads) out[c] = first[sub];
 }
 
 // Codeword sums: a CTA takes one sub-quantiser's codes of a range of rows, orders the rows by codeword in shared memory (counts,
 // prefix, slots) and lets a warp sum each codeword's rows in fp64, so that only one fp64 atomic per non-empty codeword and
-// dimension leaves it.  (With fp64 atomics in shared memory per element, 12 CTAs for 32,768 rows, this was 459 us of a 0.8 ms iteration.)
-constexpr int kPqAccRows = 4096;
-__global__ void __launch_bounds__(256) k_pq_accumulate(const float* __restrict__ data, long long n, int dim, const uint8_t* __restrict__ codes,
+// dimension leaves it.  A lane keeps one dimension: P lanes read a row's sub-vector side by side, 32 / P rows at a time, and two to four
+// exchanges end it.  (A row per lane took five exchanges for each dimension: 44 us for 32,768 x 96, m = 24, 19 now; fp64 atomics in shared
+// memory per element 459.)
+constexpr int kPqAccRows = 4096, kPqAccThreads = 1024;   // threads: each warp's codewords follow one another, a list and a row's latency each
+__global__ void __launch_bounds__(kPqAccThreads) k_pq_accumulate(const float* __restrict__ data, long long n, int dim, const uint8_t* __restrict__ codes,
                                                        int m, int k, double* __restrict__ sums, int* __restrict__ counts) {
     __shared__ int s_off[257], s_cur[256], s_warp[32], s_total;
     __shared__ uint16_t s_row[kPqAccRows];
     const int dsub = dim / m, sub = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long r0 = (long long)blockIdx.x * kPqAccRows;
     const int rows = (int)min((long long)kPqAccRows, n - r0);
-    s_cur[threadIdx.x] = 0;
+    __shared__ uint8_t s_code[kPqAccRows];
+    if (threadIdx.x < 256) s_cur[threadIdx.x] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < rows; i += 256) atomicAdd(&s_cur[codes[(size_t)(r0 + i) * m + sub]], 1);
+#pragma unroll
+    for (int i = threadIdx.x; i < rows; i += kPqAccThreads) {
+        const uint8_t c = __ldg(codes + (size_t)(r0 + i) * m + sub);
+        s_code[i] = c;
+        atomicAdd(&s_cur[c], 1);
+    }
     __syncthreads();
-    const int mine = s_cur[threadIdx.x];
+    const int mine = threadIdx.x < 256 ? s_cur[threadIdx.x] : 0;
     const int ex = block_exclusive_scan(mine, s_warp, &s_total);
-    s_off[threadIdx.x] = ex;
-    s_cur[threadIdx.x] = ex;
+    if (threadIdx.x < 256) { s_off[threadIdx.x] = ex; s_cur[threadIdx.x] = ex; }
     if (threadIdx.x == 0) s_off[256] = rows;
     if (mine) atomicAdd(&counts[(size_t)sub * k + threadIdx.x], mine);
     __syncthreads();
-    for (int i = threadIdx.x; i < rows; i += 256) s_row[atomicAdd(&s_cur[codes[(size_t)(r0 + i) * m + sub]], 1)] = (uint16_t)i;
+    for (int i = threadIdx.x; i < rows; i += kPqAccThreads) s_row[atomicAdd(&s_cur[s_code[i]], 1)] = (uint16_t)i;   // (its own codes: no barrier needed)
     __syncthreads();
     const float* src = data + (size_t)r0 * dim + (size_t)sub * dsub;
-    for (int c = warp; c < k; c += 8) {
+    int p = 1;   // lanes of a row
+    while (p < dsub && p < 32) p <<= 1;
+    const int at = lane & (p - 1), first = lane / p, step = 32 / p;
+    for (int c = warp; c < k; c += kPqAccThreads / 32) {
         const int b = s_off[c], e = s_off[c + 1];
         if (b == e) continue;
-        for (int d0 = 0; d0 < dsub; d0 += 4) {   // four dimensions of the codeword's rows at a time
-            double acc[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int i = b + lane; i < e; i += 32) {
-                const float* x = src + (size_t)s_row[i] * dim + d0;
-#pragma unroll
-                for (int d = 0; d < 4; ++d) if (d0 + d < dsub) acc[d] += (double)__ldg(x + d);
+        for (int d0 = 0; d0 < dsub; d0 += p) {
+            const int d = d0 + at;
+            double acc = 0.0;
+            if (d < dsub) {
+#pragma unroll 4
+                for (int i = b + first; i < e; i += step) acc += (double)__ldg(src + (size_t)s_row[i] * dim + d);
             }
-#pragma unroll
-            for (int d = 0; d < 4; ++d) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
-                if (lane == d && d0 + d < dsub) atomicAdd(&sums[((size_t)sub * k + c) * dsub + d0 + d], acc[d]);
-            }
+            for (int o = p; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane < p && d < dsub) atomicAdd(&sums[((size_t)sub * k + c) * dsub + d], acc);
         }
     }
 }
@@ -495,7 +563,7 @@ psb_status launch_pq_assign_train(const float* d_data, long long n, int dim, con
 psb_status launch_pq_accumulate(const float* d_data, long long n, int dim, const uint8_t* d_codes, int m, int k,
                                 double* d_sums, int* d_counts, cudaStream_t s) {
     if (n <= 0) return PSB_OK;
-    k_pq_accumulate<<<dim3((unsigned)((n + kPqAccRows - 1) / kPqAccRows), (unsigned)m), 256, 0, s>>>(d_data, n, dim, d_codes, m, k, d_sums, d_counts);
+    k_pq_accumulate<<<dim3((unsigned)((n + kPqAccRows - 1) / kPqAccRows), (unsigned)m), kPqAccThreads, 0, s>>>(d_data, n, dim, d_codes, m, k, d_sums, d_counts);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
@@ -515,7 +583,7 @@ psb_status launch_pq_seed(const float* d_data, int n, int dim, int m, int k, con
                           int* d_status, cudaStream_t s) {
     const int dsub = dim / m;
     const int per = (n + kSeedCluster - 1) / kSeedCluster;
-    const size_t mins = (size_t)(per + 3) / 4 * 16, rows = (size_t)per * dsub * 4;
+    const size_t mins = (size_t)(per + 511) / 256 * 1024, rows = (size_t)per * dsub * 4;
     const int staged = mins + rows <= (size_t)200 * 1024 ? 1 : 0;
     const size_t smem = mins + (staged ? rows : 0);
     auto run = [&](auto kernel) -> psb_status {
@@ -525,7 +593,10 @@ psb_status launch_pq_seed(const float* d_data, int n, int dim, int m, int k, con
     };
     switch (dsub) {
         case 2: PSB_TRY(run(k_pq_seed<2>)); break;
+        case 3: PSB_TRY(run(k_pq_seed<3>)); break;
         case 4: PSB_TRY(run(k_pq_seed<4>)); break;
+        case 5: PSB_TRY(run(k_pq_seed<5>)); break;
+        case 6: PSB_TRY(run(k_pq_seed<6>)); break;
         case 8: PSB_TRY(run(k_pq_seed<8>)); break;
         default: PSB_TRY(run(k_pq_seed<0>)); break;
     }
