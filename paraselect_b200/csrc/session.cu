@@ -2405,7 +2405,10 @@ class Assigner {
 public:
     Assigner(const float* d_data, int64_t n, int dim, int k, int device, int sms, cudaStream_t st)
         : data_(d_data), n_(n), dim_(dim), k_(k), device_(device), sms_(sms), st_(st) {
-        tc_ = coarse_tc_supported((int)std::min<int64_t>(n, 1 << 30), k, dim, 1);
+        // The filter costs about 2 ns a row whatever the number of centroids, and its launches more than the row kernel's; that takes 1.2e-4 ns for
+        // each dimension of a pair.  Trainings of three iterations, rows / filter, us: 20,000 x 64, 256 centroids 548 / 631, 400 654 / 572; 20,000 x
+        // 128, 128 613 / 756, 200 749 / 673; 100,000 x 96, 128 1,218 / 1,239, 1,000 5,020 / 1,200; 400,000 x 100, 128 4,031 / 3,216, 1,000 19,369 / 3,233.
+        tc_ = n >= 64 && coarse_tc_padded_dim(dim) <= 128 && (!nearest_rows_fit(dim) || (double)k * dim >= 16384.0 + 1.6e8 / (double)n);
     }
     // d_assign [n], d_best [n] out; bounded: d_assign holds an assignment on entry, whose distances bound the nearest ones (one
     // filter pass instead of two).
