@@ -12,6 +12,7 @@
 //
 // Reference counterpart: the GPU-resident fine kernels of src/search/kernels/fine/gpu_fine/resident/resident_full_l2_topk.cu:19-178
 // behind ivfflat_search (src/search/ivfflat/ivfflat_search.cuh:41-51).
+#include <cuda_bf16.h>
 #include <algorithm>
 
 #include "common.cuh"
@@ -199,6 +200,255 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
     }
 }
 
+// ---- list form behind a filter --------------------------------------------------------------------------------------------------
+// The distances of a list's visitors to its rows are a matrix product; in the reference's arithmetic they are three instructions per
+// dimension and pair.  Where a selection follows anyway, the tiles are taken from mma.sync with both operands split into two bf16 terms
+// (|q|^2 + |x|^2 - 2 q.x in fp32), the selection keeps every row that the approximate distance cannot rule out, and those - a few more
+// than topk - are evaluated exactly.  (tcgen05 wants 128 visitors a tile; a list has sixty in the benchmark's configuration, and often ten.)
+// Bound: latency, a tile being a chain of look-ups, two stagings and a short product; four CTAs an SM.  1,000 queries x 16 lists of 390 rows x 128,
+// topk 10: tiles 163 -> 72 us, selection 14 -> 29, the whole call 244 -> 150.  Eight warps a tile 91, four rows' loads at a time 78.
+//   Error of an approximate distance against the exact arithmetic's, S = (|q| + max|x|)^2:  products, splits 3.1 * 2^-18 and 3 K additions of
+//   2^-22 each, of |q||x| <= S / 4, twice; norms (K + 4) 2^-24 S; their sum 2^-22 S; the exact arithmetic's own (K + 2) 2^-23 S; where products are
+//   subnormal, below 1e-35.  A row within twice that of the topk-th smallest approximate distance may be among the topk.
+constexpr int kFilterThreads = 128;   // four warps: 16 visitors x 32 rows each
+__host__ __device__ __forceinline__ int filter_dims(int dim) { return (dim + 15) / 16 * 16; }
+__host__ __device__ __forceinline__ int filter_pitch(int dim) { return filter_dims(dim) + 8; }   // bf16 between rows: eight rows' 16 bytes in different banks
+inline size_t filter_bytes(int dim) { return (size_t)(SQ + SC) * filter_pitch(dim) * 4; }
+__device__ __forceinline__ float filter_slack(float qn, float xmax2, int dim) {
+    const float s = sqrtf(qn) + sqrtf(xmax2), k = (float)filter_dims(dim);
+    return 2.0f * (s * s * 1.0001f * (5.913e-6f + k * (3.577e-7f + 5.97e-8f + 1.193e-7f) + 1.0e-6f) + 1.0e-35f);
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Squared norms of the rows, and the largest as the bits of a float (not a number: the largest of all).  A warp per row.
+__global__ void __launch_bounds__(256) k_flat_norms(const float* __restrict__ rows, long long n, int dim, float* __restrict__ norms, unsigned* __restrict__ most) {
+    const int lane = threadIdx.x & 31;
+    unsigned top = 0;
+    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < n; r += (long long)gridDim.x * 8) {
+        float s = 0.0f;
+        for (int d = lane; d < dim; d += 32) { const float v = rows[(size_t)r * dim + d]; s = fmaf(v, v, s); }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) norms[r] = s;
+        top = max(top, __float_as_uint(s) & 0x7fffffffu);
+    }
+    if (lane == 0 && top) atomicMax(most, top);
+}
+
+__global__ void __launch_bounds__(kFilterThreads)
+k_flat_tiles_filter(const float* __restrict__ queries, int dim, int nprobe, const long long* __restrict__ offsets, int nlist, const float* __restrict__ rows,
+                    const float* __restrict__ norms, const int* __restrict__ vis_off, const long long* __restrict__ item_off,
+                    const int* __restrict__ visitors, const int* __restrict__ seg, long long stride, float* __restrict__ dist) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ int s_list, s_pair[SQ];
+    __shared__ long long s_dst[SQ];
+    __shared__ float s_qn[SQ];
+    const int pitch = filter_pitch(dim), dims = filter_dims(dim);
+    __nv_bfloat16* qh = reinterpret_cast<__nv_bfloat16*>(s_raw);   // [SQ][pitch] visitors, high terms
+    __nv_bfloat16* ql = qh + SQ * pitch;
+    __nv_bfloat16* xh = ql + SQ * pitch;                           // [SC][pitch] rows
+    __nv_bfloat16* xl = xh + SC * pitch;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long total = item_off[nlist];
+    // One row by a warp, four elements a lane, several rows' loads before the first is used: two bf16 terms of each, and the squares' sum.
+    auto stage = [&](auto src_of, int count, __nv_bfloat16* high, __nv_bfloat16* low, bool vec, auto sum_of) {
+        constexpr int U = 8;
+        for (int r0 = warp; r0 < count; r0 += U * (kFilterThreads / 32)) {
+            float sums[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) sums[u] = 0.0f;
+            for (int d = lane * 4; d < dims; d += 128) {
+                float4 v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int r = r0 + u * (kFilterThreads / 32);
+                    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (r >= count) continue;
+                    const float* x = src_of(r) + d;
+                    if (vec) { if (d < dim) v[u] = __ldg(reinterpret_cast<const float4*>(x)); }
+                    else {
+                        if (d < dim) v[u].x = __ldg(x);
+                        if (d + 1 < dim) v[u].y = __ldg(x + 1);
+                        if (d + 2 < dim) v[u].z = __ldg(x + 2);
+                        if (d + 3 < dim) v[u].w = __ldg(x + 3);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int r = r0 + u * (kFilterThreads / 32);
+                    if (r >= count) continue;
+                    const __nv_bfloat162 h0 = __floats2bfloat162_rn(v[u].x, v[u].y), h1 = __floats2bfloat162_rn(v[u].z, v[u].w);
+                    const __nv_bfloat162 l0 = __floats2bfloat162_rn(v[u].x - __low2float(h0), v[u].y - __high2float(h0)),
+                                         l1 = __floats2bfloat162_rn(v[u].z - __low2float(h1), v[u].w - __high2float(h1));
+                    uint2 w;
+                    w.x = *reinterpret_cast<const uint32_t*>(&h0); w.y = *reinterpret_cast<const uint32_t*>(&h1);
+                    *reinterpret_cast<uint2*>(high + (size_t)r * pitch + d) = w;
+                    w.x = *reinterpret_cast<const uint32_t*>(&l0); w.y = *reinterpret_cast<const uint32_t*>(&l1);
+                    *reinterpret_cast<uint2*>(low + (size_t)r * pitch + d) = w;
+                    sums[u] = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, fmaf(v[u].w, v[u].w, sums[u]))));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) sum_of(r0 + u * (kFilterThreads / 32), sums[u]);
+        }
+    };
+    for (long long item = blockIdx.x; item < total; item += gridDim.x) {
+        __syncthreads();   // the previous tile is done with shared memory
+        if (warp == 0) { const int l = scan::find_list(item_off, nlist, item); if (lane == 0) s_list = l; }
+        __syncthreads();
+        const int l = s_list;
+        const int v0 = vis_off[l], nvis = vis_off[l + 1] - v0;
+        const int groups = (nvis + SQ - 1) / SQ;
+        const long long local = item - item_off[l];
+        const int g = (int)(local % groups);
+        const long long r0 = local / groups * SC, len = offsets[l + 1] - offsets[l], first = offsets[l] + r0;
+        const int nv = min(SQ, nvis - g * SQ), nr = (int)min((long long)SC, len - r0);
+        if (threadIdx.x < SQ) {
+            const int pair = threadIdx.x < nv ? visitors[v0 + g * SQ + threadIdx.x] : -1;
+            s_pair[threadIdx.x] = pair;
+            if (pair >= 0) { const int q = pair / nprobe; s_dst[threadIdx.x] = (long long)q * stride + seg[(size_t)q * (nprobe + 1) + (pair - q * nprobe)] + r0; }
+        }
+        stage([&](int r) { return rows + (size_t)(first + r) * dim; }, nr, xh, xl, rows_vec(rows, dim), [](int, float) {});
+        __syncthreads();
+        stage([&](int r) { return queries + (size_t)(s_pair[r] / nprobe) * dim; }, nv, qh, ql, rows_vec(queries, dim), [&](int r, float sum) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane == 0 && r < nv) s_qn[r] = sum;
+        });
+        __syncthreads();
+        const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 32;   // the warp's visitors and rows
+        if (m0 >= nv || n0 >= nr) continue;
+        float acc[4][4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[t][j] = 0.0f;
+        const int arow = (m0 + (lane & 15)) * pitch + (lane >> 4) * 8, brow = (n0 + (lane & 7) + (lane >> 4) * 8) * pitch + ((lane >> 3) & 1) * 8;
+#pragma unroll 2
+        for (int k0 = 0; k0 < dims; k0 += 16) {   // (rows past nv and nr hold what an earlier tile left: their sums are not written)
+            uint32_t ah[4], al[4], bh[2][4], bl[2][4];
+            ldmatrix4(ah, qh + arow + k0);
+            ldmatrix4(al, ql + arow + k0);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) { ldmatrix4(bh[h], xh + brow + h * 16 * pitch + k0); ldmatrix4(bl[h], xl + brow + h * 16 * pitch + k0); }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                mma_bf16(acc[t], ah, bl[t >> 1][(t & 1) * 2], bl[t >> 1][(t & 1) * 2 + 1]);
+                mma_bf16(acc[t], al, bh[t >> 1][(t & 1) * 2], bh[t >> 1][(t & 1) * 2 + 1]);
+                mma_bf16(acc[t], ah, bh[t >> 1][(t & 1) * 2], bh[t >> 1][(t & 1) * 2 + 1]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int c = n0 + t * 8 + (lane & 3) * 2;
+            const float x0 = c < nr ? __ldg(norms + first + c) : 0.0f, x1 = c + 1 < nr ? __ldg(norms + first + c + 1) : 0.0f;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int v = m0 + (lane >> 2) + h * 8;
+                if (v >= nv) continue;
+                float* out = dist + s_dst[v] + c;
+                const float qn = s_qn[v];
+                if (c < nr) out[0] = fmaf(-2.0f, acc[t][h * 2], qn + x0);
+                if (c + 1 < nr) out[1] = fmaf(-2.0f, acc[t][h * 2 + 1], qn + x1);
+            }
+        }
+    }
+}
+
+// One CTA per query: the topk nearest of its approximate distances' candidates, evaluated exactly; ties by row; original ids out.  A query whose
+// bound does not hold (values out of range, too many rows within it) has all its distances computed and selected from.
+template <int T>
+__global__ void __launch_bounds__(T)
+k_flat_select_filter(float* __restrict__ dist, long long stride, const float* __restrict__ queries, int dim, const float* __restrict__ rows,
+                     const unsigned* __restrict__ most, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
+                     const int* __restrict__ seg, int topk, int buffer, const long long* __restrict__ ids, long long* __restrict__ out_ids,
+                     float* __restrict__ out_dist) {
+    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the selection's runs, the query, the segments (where they fit)
+    __shared__ sel::Words w;
+    int* s_runs = reinterpret_cast<int*>(s_key + buffer);
+    float* s_q = reinterpret_cast<float*>(s_runs + sel::kMaxGroups);
+    const int q = blockIdx.x, lane = threadIdx.x & 31;
+    const int* s = seg + (size_t)q * (nprobe + 1);
+    for (int d = threadIdx.x; d < dim; d += T) s_q[d] = queries[(size_t)q * dim + d];
+    if (nprobe <= sel::kSegShared) {
+        int* s_seg = reinterpret_cast<int*>(s_q + ((dim + 3) & ~3));
+        for (int p = threadIdx.x; p <= nprobe; p += T) s_seg[p] = s[p];
+        s = s_seg;
+    }
+    if (threadIdx.x == 0) w.cnt = 0;
+    __syncthreads();
+    auto row_of = [&](int i) -> uint32_t {
+        int lo = 0, hi = nprobe;
+        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s[mid] <= i) lo = mid; else hi = mid; }
+        return (uint32_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo]));
+    };
+    const bool vec = rows_vec(rows, dim);
+    float* vals = dist + (size_t)q * stride;
+    const int n = s[nprobe];
+    int keep = min(topk, n);
+    float qn = 0.0f;
+    for (int d = lane; d < dim; d += 32) qn = fmaf(s_q[d], s_q[d], qn);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) qn += __shfl_xor_sync(0xffffffffu, qn, o);   // the same in every warp
+    const float inf = __int_as_float(0x7f800000), slack = filter_slack(qn, __uint_as_float(*most), dim);
+    bool sure = slack < 1.0e37f;
+    if (sure) {
+        float cut = inf;
+        if (n > 4 * topk && n >= 96) {   // as sel::smallest does
+            float* s_min = reinterpret_cast<float*>(s_key);
+            const int per = (2 * topk + T - 1) / T;
+            for (int g = 0; g < per; ++g) {
+                float m = inf;
+#pragma unroll 8
+                for (int i = threadIdx.x + g * T; i < n; i += per * T) m = fminf(m, vals[i]);
+                s_min[g * T + threadIdx.x] = m;
+            }
+            __syncthreads();
+            if (threadIdx.x < 32) {
+                const float at = per == 1 ? sel::bound_of<T / 32>(s_min, T, topk) : sel::bound_of<0>(s_min, per * T, topk);
+                if (lane == 0) w.cut = at;
+            }
+            __syncthreads();
+            cut = w.cut + slack;
+        }
+#pragma unroll 8
+        for (int i = threadIdx.x; i < n; i += T)
+            if (cut == inf || vals[i] <= cut) {
+                const int pos = atomicAdd(&w.cnt, 1);
+                if (pos < buffer) s_key[pos] = (uint64_t)i;
+            }
+        __syncthreads();
+        const int c = w.cnt;
+        sure = c >= keep && c <= buffer;
+        if (sure) {
+            for (int e = threadIdx.x; e < c; e += T) {
+                const uint32_t r = row_of((int)s_key[e]);
+                s_key[e] = make_key(row_distance(s_q, rows + (size_t)r * dim, dim, vec), r);
+            }
+            __syncthreads();
+            sel::put_in_order<T>(s_key, c, topk);
+        }
+    }
+    if (!sure) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += T) vals[i] = row_distance(s_q, rows + (size_t)row_of(i) * dim, dim, vec);
+        __syncthreads();
+        keep = sel::smallest<T>(vals, n, topk, row_of, s_key, buffer, s_runs, &w);
+    }
+    for (int i = threadIdx.x; i < topk; i += T) {
+        const bool ok = i < keep;
+        out_ids[(size_t)q * topk + i] = ok ? ids[key_idx(s_key[i])] : -1;
+        out_dist[(size_t)q * topk + i] = ok ? key_dist(s_key[i]) : FLT_MAX;
+    }
+}
+
 }  // namespace
 
 psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const long long* d_offsets, int list_begin, int list_end, int* d_seg,
@@ -218,6 +468,18 @@ bool flat_list_form(int nq, int nprobe, int nlist, long long rows, int dim) {
     return (double)nq * nprobe * rows / nlist * dim >= 4e7 && (long long)nq * nprobe >= 2ll * nlist && small_tile_bytes(dim) <= (size_t)200 * 1024;
 }
 
+// The list form's tiles from the filter: its operands fit, and the selection's buffer holds topk and what the slack lets through.
+bool flat_filter_form(int dim, int topk) { return topk <= 256 && filter_bytes(dim) <= (size_t)100 * 1024; }
+
+psb_status launch_flat_norms(const float* d_rows, long long n, int dim, float* d_norms, unsigned* d_most, cudaStream_t s) {
+    PSB_CUDA(cudaMemsetAsync(d_most, 0, sizeof(unsigned), s));
+    if (n <= 0) return PSB_OK;
+    k_flat_norms<<<(unsigned)std::min<long long>((n + 7) / 8, 4096), 256, 0, s>>>(d_rows, n, dim, d_norms, d_most);
+    count_launch();
+    PSB_LAUNCH_CHECK();
+    return PSB_OK;
+}
+
 psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
     if (f.topk <= 0 || f.topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "flat scan supports topk in 1..2048");
@@ -232,6 +494,27 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
         k_flat_visitors<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(f.probes, pairs, f.slot, f.vis_off, f.visitors);
         count_launch();
         PSB_LAUNCH_CHECK();
+        if (flat_filter_form(f.dim, f.topk)) {
+            const size_t smem = filter_bytes(f.dim);
+            PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_tiles_filter), smem));
+            const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)220 * 1024 / (smem + 2048)));
+            k_flat_tiles_filter<<<(unsigned)(f.sm_count * per_sm), kFilterThreads, smem, s>>>(f.queries, f.dim, f.nprobe, f.offsets, f.nlist, f.rows, f.norms,
+                                                                                              f.vis_off, f.item_off, f.visitors, f.seg, f.stride, f.dist);
+            count_launch();
+            PSB_LAUNCH_CHECK();
+            const size_t keys = sel::shared_bytes(f.topk) + (size_t)((f.dim + 3) & ~3) * 4 + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
+            auto select = [&](auto kernel, int threads) -> psb_status {
+                PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), keys));
+                kernel<<<nq, threads, keys, s>>>(f.dist, f.stride, f.queries, f.dim, f.rows, f.most, f.probes, f.nprobe, f.offsets, f.seg, f.topk,
+                                                 sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist);
+                return PSB_OK;
+            };
+            if (nq <= f.sm_count) PSB_TRY(select(k_flat_select_filter<1024>, 1024));
+            else PSB_TRY(select(k_flat_select_filter<256>, 256));
+            count_launch();
+            PSB_LAUNCH_CHECK();
+            return PSB_OK;
+        }
         const size_t smem = small_tile_bytes(f.dim);
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_tiles), smem));
         const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)220 * 1024 / (smem + 1024)));

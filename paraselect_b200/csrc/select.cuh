@@ -103,6 +103,29 @@ __device__ __forceinline__ void store_run(float* __restrict__ runs, int r, float
     if ((threadIdx.x & 31) == 0) runs[r] = v;
 }
 
+// The first c keys of s_keys in ascending order, and nothing (KEY_MAX) in the places up to k.
+template <int kThreads>
+__device__ __forceinline__ void put_in_order(uint64_t* s_keys, int c, int k) {
+    const int tid = threadIdx.x;
+    if (c <= kThreads) {   // a key's place is the number of smaller ones
+        const uint64_t mine = tid < c ? s_keys[tid] : KEY_MAX;
+        int rank = 0;
+        if ((tid & ~31) < c) {
+#pragma unroll 4
+            for (int j = 0; j < c; ++j) { const uint64_t o = s_keys[j]; rank += o < mine || (o == mine && j < tid) ? 1 : 0; }   // a key may occur twice
+        }
+        __syncthreads();
+        if (tid < c) s_keys[rank] = mine;
+        for (int i = c + tid; i < k; i += kThreads) s_keys[i] = KEY_MAX;
+        __syncthreads();
+    } else {
+        const int np = next_pow2(c);
+        for (int i = c + tid; i < np || i < k; i += kThreads) s_keys[i] = KEY_MAX;
+        __syncthreads();
+        block_bitonic_sort(s_keys, np);
+    }
+}
+
 // Leaves the min(k, n) smallest keys (vals[i], payload(i)) of i = 0..n-1 at the front of s_keys, ascending, and returns their number.  s_keys
 // [buffer], s_runs [kMaxGroups], one Words in shared memory; k <= buffer.  runs: the minima of every kRun values, or null.
 // The k-th smallest of the minima of at least 2 k subsets of the values bounds the k-th smallest value from above.  Every thread takes the
@@ -230,23 +253,7 @@ __device__ int smallest(const float* __restrict__ vals, int n, int k, Payload pa
         }
         __syncthreads();
     }
-    if (c <= kThreads) {   // a key's place is the number of smaller ones
-        const uint64_t mine = tid < c ? s_keys[tid] : KEY_MAX;
-        int rank = 0;
-        if ((tid & ~31) < c) {
-#pragma unroll 4
-            for (int j = 0; j < c; ++j) { const uint64_t o = s_keys[j]; rank += o < mine || (o == mine && j < tid) ? 1 : 0; }   // a key may occur twice
-        }
-        __syncthreads();
-        if (tid < c) s_keys[rank] = mine;
-        for (int i = c + tid; i < k; i += kThreads) s_keys[i] = KEY_MAX;
-        __syncthreads();
-    } else {
-        const int np = next_pow2(c);
-        for (int i = c + tid; i < np || i < k; i += kThreads) s_keys[i] = KEY_MAX;
-        __syncthreads();
-        block_bitonic_sort(s_keys, np);
-    }
+    put_in_order<kThreads>(s_keys, c, k);
     return keep;
 }
 

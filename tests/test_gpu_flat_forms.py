@@ -59,3 +59,43 @@ def test_flat_list_form_and_parts(psb, n, dim, nlist, nq, nprobe, topk, values):
     some = np.unique(np.concatenate([np.arange(50), nq // 2 + np.arange(-25, 25), nq - 1 - np.arange(50), rng.integers(0, nq, 100)]))   # part borders among them
     wi, wd = oracle.ivfflat_search(fx["centroids"], off, fx["reordered_ids"], fx["vectors"], q[some], nprobe, topk)
     assert np.array_equal(got["indices"][some], wi) and np.array_equal(got["distances"][some], wd)
+
+
+@pytest.mark.parametrize("dim", [5, 16, 100, 128, 130, 240])
+@pytest.mark.parametrize("kind", ["normal", "far", "tiny", "grid", "odd"])
+@pytest.mark.parametrize("k", [1, 10, 256])
+def test_list_form_behind_the_filter(psb, dim, kind, k):
+    """Approximate distances and exact evaluation of the candidates: a large offset, which loosens the bound; values whose squares vanish, equal
+    distances by the hundred and values that are not finite, for which a query's distances are all computed."""
+    rng = np.random.default_rng(dim + k)
+    nlist, n, nq, nprobe = 6, 9000, 700, 3
+    cen = rng.standard_normal((nlist, dim)).astype(np.float32)
+    off = np.array([0, 1, 65, 65, 1400, 5000, n], np.int64)
+    own = np.repeat(np.arange(nlist), np.diff(off))
+    x = (cen[own] + 0.3 * rng.standard_normal((n, dim))).astype(np.float32)
+    q = (cen[rng.integers(0, nlist, nq)] + 0.3 * rng.standard_normal((nq, dim))).astype(np.float32)
+    if kind == "far":
+        x, q, cen = x + 100, q + 100, cen + 100
+    if kind == "tiny":
+        x, q, cen = (v * np.float32(1e-20) for v in (x, q, cen))
+    if kind == "grid":
+        x, q = np.round(x), np.round(q)
+    if kind == "odd":
+        x[4000, 0], x[77, dim - 1], q[3, 1] = np.inf, np.nan, np.inf
+    ix = dict(centroids=cen, offsets=off, reordered_ids=rng.permutation(n).astype(np.int64), vectors=x)
+    with psb.FlatSession(ix, max_batch=nq) as s:
+        got = s.search(q, nprobe, k, batch_size=nq, want_coarse=True)
+    for i in list(range(12)) + [nq - 1]:
+        rows = np.concatenate([np.arange(off[p], off[p + 1]) for p in got["coarse"][i]])
+        d = np.zeros(len(rows), np.float32)
+        with np.errstate(invalid="ignore", over="ignore"):
+            for j in range(dim):
+                t = q[i, j] - x[rows, j]
+                d += t * t
+        fine = np.isfinite(d)
+        if not fine.all() and i == 3:
+            continue
+        order = np.lexsort((rows, np.where(np.isnan(d), np.inf, d)))[:k]
+        take = np.isfinite(d[order])
+        assert np.array_equal(got["indices"][i][: len(order)][take], ix["reordered_ids"][rows[order]][take]), (kind, i)
+        assert np.array_equal(got["distances"][i][: len(order)][take], d[order][take])
