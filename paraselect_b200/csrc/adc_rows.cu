@@ -64,6 +64,7 @@ __device__ __forceinline__ void block_table(float* __restrict__ s_tab, const flo
 template <int M>
 __global__ void __launch_bounds__(kRowsThreads)
 k_adc_rows(const AdcRows g, int block_rows) {
+    behind();
     extern __shared__ __align__(16) float s_rows[];
     float* s_tab = s_rows;                                      // [m * k]
     float* s_q = s_rows + g.m * g.k;                            // [dim]
@@ -96,6 +97,7 @@ k_adc_rows(const AdcRows g, int block_rows) {
 template <int M>
 __global__ void __launch_bounds__(kRowsThreads)
 k_adc_pair_rows(const AdcRows g, int block_rows, int chunks) {
+    behind();
     extern __shared__ __align__(16) float s_rows[];
     float* s_tab = s_rows;
     float* s_q = s_rows + g.m * g.k;
@@ -119,6 +121,7 @@ k_adc_pair_rows(const AdcRows g, int block_rows, int chunks) {
 template <int T>
 __global__ void __launch_bounds__(T)
 k_adc_select(const AdcRows g, int buffer) {
+    behind();
     extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the selection's runs, the segments (where they fit)
     __shared__ sel::Words w;
     const int q = blockIdx.x;
@@ -157,11 +160,11 @@ psb_status run_rows(const AdcRows& g, int nq, cudaStream_t s) {
         const long long blocks = (long long)nq * g.nprobe * chunks;
         if (blocks > 0x7fffffffLL) return fail(PSB_UNSUPPORTED_SHAPE, "too many (query, probe) pairs in one batch");
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_adc_pair_rows<M>), tab));
-        k_adc_pair_rows<M><<<(unsigned)blocks, kRowsThreads, tab, s>>>(g, block, chunks);
+        PSB_TRY(launch_behind(true, k_adc_pair_rows<M>, dim3((unsigned)blocks), kRowsThreads, tab, s, g, block, chunks));
     } else {
         const size_t smem = tab + ((size_t)g.nprobe + 1) * sizeof(int);
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_adc_rows<M>), smem));
-        k_adc_rows<M><<<dim3((unsigned)((g.stride + block - 1) / block), (unsigned)nq), kRowsThreads, smem, s>>>(g, block);
+        PSB_TRY(launch_behind(true, k_adc_rows<M>, dim3((unsigned)((g.stride + block - 1) / block), (unsigned)nq), kRowsThreads, smem, s, g, block));
     }
     count_launch();
     PSB_LAUNCH_CHECK();
@@ -172,7 +175,7 @@ psb_status run_rows(const AdcRows& g, int nq, cudaStream_t s) {
 
 psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
-    PSB_TRY(launch_row_segments(g.probes, nq, g.nprobe, g.offsets, g.list_begin, g.list_end, g.seg, nullptr, nullptr, g.counters, s, g.mark));
+    PSB_TRY(launch_row_segments(g.probes, nq, g.nprobe, g.offsets, g.list_begin, g.list_end, g.seg, nullptr, nullptr, g.counters, s, g.chained, g.mark));
     switch (g.m) {
         case 8: PSB_TRY(run_rows<8>(g, nq, s)); break;
         case 16: PSB_TRY(run_rows<16>(g, nq, s)); break;
@@ -188,8 +191,7 @@ psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s) {
     // Fewer queries than SMs: one selecting block per SM at most, so a large one.
     auto select = [&](auto kernel, int threads) -> psb_status {
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
-        kernel<<<nq, threads, smem, s>>>(g, buffer);
-        return PSB_OK;
+        return launch_behind(true, kernel, dim3((unsigned)nq), (unsigned)threads, smem, s, g, buffer);
     };
     if (nq <= g.sm_count) PSB_TRY(select(k_adc_select<1024>, 1024));
     else PSB_TRY(select(k_adc_select<256>, 256));

@@ -74,6 +74,7 @@ k_coarse_dist_exact(const float* __restrict__ queries, int nq, const float* __re
 __global__ void __launch_bounds__(kSmallThreads)
 k_coarse_dist_small(const float* __restrict__ queries, int nq, const float* __restrict__ centroids, int nlist, int dim, float* __restrict__ dist,
                     unsigned long long* mark) {
+    behind();
     mark_start(mark);
     extern __shared__ __align__(16) float s_small[];
     const int pitch = small_pitch(dim);
@@ -110,6 +111,7 @@ k_coarse_dist_few(const float* __restrict__ queries, const float* __restrict__ c
                   unsigned long long* mark, float* __restrict__ copy) {
     extern __shared__ __align__(16) float s_q[];
     const int q = blockIdx.y, c = blockIdx.x * kFewThreads + threadIdx.x;
+    behind();
     mark_start(mark);
     for (int d = threadIdx.x; d < dim; d += kFewThreads) {
         const float v = queries[(size_t)q * dim + d];
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(kSelThreads)
 k_select_rows(const float* __restrict__ dist, int n, int k, int buffer, int* __restrict__ out_ids, float* __restrict__ out_dist) {
     extern __shared__ __align__(16) uint64_t s_sel[];  // [buffer] keys, then the selection's runs
     __shared__ sel::Words w;
+    behind();
     const int keep = sel::smallest<kSelThreads>(dist + (size_t)blockIdx.x * n, n, k, [](int i) { return (uint32_t)i; }, s_sel, buffer,
                                    reinterpret_cast<int*>(s_sel + buffer), &w);
     for (int i = threadIdx.x; i < k; i += blockDim.x) {
@@ -240,7 +243,7 @@ psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_
     if (k <= 0 || k > kMaxProbe) return fail(PSB_UNSUPPORTED_SHAPE, "row selection supports 1..4096 results");
     const size_t smem = sel::shared_bytes(k);
     PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_select_rows), smem));
-    k_select_rows<<<nq, kSelThreads, smem, s>>>(d_dist, n, k, sel::buffer_entries(k), d_ids, d_out);
+    PSB_TRY(launch_behind(true, k_select_rows, dim3((unsigned)nq), kSelThreads, smem, s, d_dist, n, k, sel::buffer_entries(k), d_ids, d_out));
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

@@ -106,6 +106,26 @@ inline psb_status prefer_max_shared(F kernel) {
     return kernel_carveout_max(reinterpret_cast<const void*>(kernel));
 }
 
+// ---- kernels of a small call, one behind the other on a stream --------------------------------------
+// launch_behind lets a kernel's blocks be placed while the kernel before it still runs: behind(), which each of them begins with, waits for its end and
+// its writes, and lets the next be placed.  That takes the 1 to 2 us between two kernels' work; for a kernel launched in the usual way behind()
+// does nothing.  Only where the stream's last work is a kernel of the same call, not a wait for another stream.  Every kernel launched so waits before its first access to memory, so that the end of one is the end of all before it.
+template <typename... P, typename... A>
+inline psb_status launch_behind(bool chained, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr; cfg.numAttrs = chained ? 1 : 0;   // not chained: an ordinary launch
+    PSB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return PSB_OK;
+}
+__device__ __forceinline__ void behind() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---- device: a kernel's start on the device's clock (nanoseconds), by its first thread ------------
 __device__ __forceinline__ void mark_start(unsigned long long* mark) {
     if (mark && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(*mark));

@@ -32,6 +32,7 @@ namespace {
 __global__ void __launch_bounds__(128) k_row_segments(const int* __restrict__ probes, int nq, int nprobe, const long long* __restrict__ offsets, int lb, int le,
                                                     int* __restrict__ seg, int* __restrict__ vis_count, int* __restrict__ slot,
                                                     unsigned long long* __restrict__ counters, unsigned long long* mark) {
+    behind();
     mark_start(mark);
     const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (q >= nq) return;
@@ -150,6 +151,7 @@ k_flat_rows(const float* __restrict__ queries, int dim, const int* __restrict__ 
             const float* __restrict__ rows, const int* __restrict__ seg, long long stride, float* __restrict__ dist, float* __restrict__ runs,
             long long run_stride) {
     extern __shared__ __align__(16) float s_q[];
+    behind();
     const int q = blockIdx.y;
     const int* s = seg + (size_t)q * (nprobe + 1);
     const int n = s[nprobe];
@@ -178,6 +180,7 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
               float* __restrict__ out_dist, const float* __restrict__ runs, long long run_stride) {
     extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the selection's runs, the segments (where they fit)
     __shared__ sel::Words w;
+    behind();
     const int q = blockIdx.x;
     const int* s = seg + (size_t)q * (nprobe + 1);
     if (nprobe <= sel::kSegShared) {   // a search for every key: not in global memory
@@ -452,8 +455,9 @@ k_flat_select_filter(float* __restrict__ dist, long long stride, const float* __
 }  // namespace
 
 psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const long long* d_offsets, int list_begin, int list_end, int* d_seg,
-                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s, unsigned long long* mark) {
-    k_row_segments<<<(unsigned)((nq + 3) / 4), 128, 0, s>>>(d_probes, nq, nprobe, d_offsets, list_begin, list_end, d_seg, d_vis_count, d_slot, d_counters, mark);
+                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s, bool chained, unsigned long long* mark) {
+    PSB_TRY(launch_behind(chained, k_row_segments, dim3((unsigned)((nq + 3) / 4)), 128, 0, s, d_probes, nq, nprobe, d_offsets, list_begin, list_end, d_seg, d_vis_count, d_slot,
+                          d_counters, mark));
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
@@ -486,7 +490,7 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     const bool lists = flat_list_form(nq, f.nprobe, f.nlist, f.n_rows, f.dim);
     const long long pairs = (long long)nq * f.nprobe;
     if (lists) PSB_CUDA(cudaMemsetAsync(f.vis_count, 0, sizeof(int) * (size_t)f.nlist, s));
-    PSB_TRY(launch_row_segments(f.probes, nq, f.nprobe, f.offsets, 0, f.nlist, f.seg, f.vis_count, lists ? f.slot : nullptr, f.counters, s));
+    PSB_TRY(launch_row_segments(f.probes, nq, f.nprobe, f.offsets, 0, f.nlist, f.seg, f.vis_count, lists ? f.slot : nullptr, f.counters, s, true));
     if (lists) {
         k_flat_lists<<<1, 1024, 0, s>>>(f.vis_count, f.offsets, f.nlist, f.vis_off, f.item_off);
         count_launch();
@@ -524,17 +528,14 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
         const long long blocks = std::min<long long>((f.stride + 127) / 128, 8192);
         const size_t smem = (size_t)((f.dim + 3) & ~3) * sizeof(float);
         if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_rows), smem));
-        k_flat_rows<<<dim3((unsigned)std::max<long long>(1, blocks), (unsigned)nq), 128, smem, s>>>(f.queries, f.dim, f.probes, f.nprobe, f.offsets, f.rows,
-                                                                                                    f.seg, f.stride, f.dist, f.runs, f.run_stride);
+        PSB_TRY(launch_behind(true, k_flat_rows, dim3((unsigned)std::max<long long>(1, blocks), (unsigned)nq), 128, smem, s, f.queries, f.dim, f.probes, f.nprobe, f.offsets, f.rows, f.seg, f.stride, f.dist, f.runs, f.run_stride));
     }
     count_launch();
     PSB_LAUNCH_CHECK();
     const size_t smem = sel::shared_bytes(f.topk) + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
     auto select = [&](auto kernel, int threads) -> psb_status {   // fewer queries than SMs: large blocks
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
-        kernel<<<nq, threads, smem, s>>>(f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids,
-                                         f.out_dist, lists ? nullptr : f.runs, f.run_stride);
-        return PSB_OK;
+        return launch_behind(true, kernel, dim3((unsigned)nq), (unsigned)threads, smem, s, f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist, lists ? nullptr : f.runs, f.run_stride);
     };
     if (nq <= f.sm_count) PSB_TRY(select(k_flat_select<1024>, 1024));
     else PSB_TRY(select(k_flat_select<256>, 256));

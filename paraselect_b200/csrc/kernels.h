@@ -264,7 +264,7 @@ psb_status launch_scan(const ScanIndex& ix, const ScanWorkspace& ws, const float
 // outside [list_begin, list_end) have none).  d_slot (may be null) [nq * nprobe]: the pair's place among its list's visitors, counted in
 // d_vis_count.  d_counters[0] += rows.
 psb_status launch_row_segments(const int* d_probes, int nq, int nprobe, const long long* d_offsets, int list_begin, int list_end, int* d_seg,
-                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s, unsigned long long* mark = nullptr);
+                               int* d_vis_count, int* d_slot, unsigned long long* d_counters, cudaStream_t s, bool chained, unsigned long long* mark = nullptr);
 // The ADC scan in its row form: all distances, then the stage1_k smallest.
 struct AdcRows {
     const float* queries; const int* probes; int nprobe;
@@ -279,6 +279,7 @@ struct AdcRows {
     double expected_rows; long long longest_list;   // rows a query is expected to scan; rows of the longest list
     unsigned long long* counters;
     unsigned long long* mark;                       // the scan's start is noted there (may be null)
+    bool chained;                                   // behind a kernel of the same call (launch_behind)
     int sm_count;
 };
 psb_status launch_adc_rows(const AdcRows& g, int nq, cudaStream_t s);
@@ -352,15 +353,15 @@ psb_status launch_gather_unique(const void* src, int row_bytes, const int* d_uni
 // their number, else by their slot.
 psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
                                const int* d_candidates, int nq, int candidate_count, int candidate_stride,
-                               const int* d_counts, float* d_out_dist, cudaStream_t s, unsigned long long* mark = nullptr);
+                               const int* d_counts, float* d_out_dist, cudaStream_t s, unsigned long long* mark = nullptr, bool chained = false);
 // The end of a call: the session's 16 counter and status words, 8 words of the coarse stage (may be null) and the time go to page-locked host memory.
 struct CallTail { unsigned long long c[16]; int tc[8]; unsigned long long end; };
-psb_status launch_call_tail(const unsigned long long* d_words, const int* d_coarse, CallTail* h_tail, cudaStream_t s);
+psb_status launch_call_tail(const unsigned long long* d_words, const int* d_coarse, CallTail* h_tail, cudaStream_t s, bool chained);
 // Per query the topk (distance,row) pairs without duplicates from d_dist [nq][candidate_count]; with d_ids (original ids by row)
 // d_out_ids [nq][topk] is written instead of d_out_rows.
 psb_status launch_topk_select(const float* d_dist, const int* d_candidates, int nq, int candidate_count,
                               int candidate_stride, const int* d_counts, int topk, int* d_out_rows,
-                              float* d_out_dist, cudaStream_t s, const long long* d_ids = nullptr, long long* d_out_ids = nullptr);
+                              float* d_out_dist, cudaStream_t s, const long long* d_ids = nullptr, long long* d_out_ids = nullptr, bool chained = false);
 psb_status launch_map_ids(const int* d_rows, long long n, const long long* d_reordered, const RowMap& mp,
                           long long* d_out, cudaStream_t s);
 psb_status launch_merge(const int* d_rows, const float* d_dist, int parts, int nq, int k, int* d_out_rows,

@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kPlaceThreads) k_place_rows(const unsigned* __
     if (sums) {
         for (int b = threadIdx.x; b < (int)blockIdx.x; b += kPlaceThreads) before += sums[b];
     } else {
+#pragma unroll 8
         for (int b = 0; b < (int)blockIdx.x; ++b) before += __popc(bits[b * kPlaceThreads + threadIdx.x]);
     }
     if (w < words) old_bits[w] = 0u;
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(kPlaceThreads) k_place_rows(const unsigned* __
 
 // A copy to the host behind the last kernel took 3 us of copy engine and 8 of waiting for it.
 __global__ void k_call_tail(const unsigned long long* __restrict__ words, const int* __restrict__ coarse, CallTail* tail) {
+    behind();
     mark_start(&tail->end);
     if (threadIdx.x < 16) tail->c[threadIdx.x] = words[threadIdx.x];
     if (coarse && threadIdx.x < 8) tail->tc[threadIdx.x] = coarse[threadIdx.x];
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(kScoreThreads)
 k_rerank_score(const unsigned char* __restrict__ src, const int* __restrict__ slot_of, RowMap mp, int dim, int elem_bytes, int through,
                const unsigned char* __restrict__ queries, const int* __restrict__ cand, int candidate_count,
                int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist, unsigned long long* mark) {
+    behind();
     mark_start(mark);
     extern __shared__ __align__(16) unsigned char s_score[];
     const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -336,6 +339,7 @@ __global__ void __launch_bounds__(kScoreThreads, 6)
 k_rerank_score_wide(const unsigned char* __restrict__ src, const int* __restrict__ slot_of, RowMap mp, int dim,
                     const unsigned char* __restrict__ queries, const int* __restrict__ cand, int candidate_count,
                     int candidate_stride, const int* __restrict__ counts, float* __restrict__ out_dist, unsigned long long* mark) {
+    behind();
     mark_start(mark);
     extern __shared__ __align__(16) unsigned char s_score[];
     const int q = blockIdx.x, lane = threadIdx.x & 31, l = lane & 7;
@@ -416,6 +420,7 @@ k_topk_select(const float* __restrict__ dist, const int* __restrict__ cand, int 
     __shared__ sel::Words w;
     __shared__ int s_warp[32];
     __shared__ int s_total, s_twice;
+    behind();
     const int q = blockIdx.x;
     const int n = cand_count(counts, q, candidate_count);
     const int* rows = cand + (size_t)q * candidate_stride;
@@ -567,16 +572,14 @@ psb_status launch_gather_unique(const void* src, int row_bytes, const int* d_uni
 
 psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const RowMap& mp, int dim, int elem_bytes, const void* d_queries,
                                const int* d_candidates, int nq, int candidate_count, int candidate_stride,
-                               const int* d_counts, float* d_out_dist, cudaStream_t s, unsigned long long* mark) {
+                               const int* d_counts, float* d_out_dist, cudaStream_t s, unsigned long long* mark, bool chained) {
     if (nq <= 0) return PSB_OK;
     const int row_bytes = dim * elem_bytes;
     const dim3 grid(nq, (candidate_count + kScoreBlock - 1) / kScoreBlock);
     if (((reinterpret_cast<uintptr_t>(d_src) | reinterpret_cast<uintptr_t>(d_queries) | row_bytes) & 15) == 0 && row_bytes <= 48 * 1024) {
         auto kernel = elem_bytes == 4 ? k_rerank_score_wide<false> : k_rerank_score_wide<true>;
         PSB_TRY(prefer_max_shared(kernel));
-        kernel<<<grid, kScoreThreads, row_bytes, s>>>(
-            static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, static_cast<const unsigned char*>(d_queries), d_candidates, candidate_count,
-            candidate_stride, d_counts, d_out_dist, mark);
+        PSB_TRY(launch_behind(chained, kernel, grid, kScoreThreads, row_bytes, s, static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, static_cast<const unsigned char*>(d_queries), d_candidates, candidate_count, candidate_stride, d_counts, d_out_dist, mark));
         count_launch();
         PSB_LAUNCH_CHECK();
         return PSB_OK;
@@ -588,17 +591,15 @@ psb_status launch_rerank_score(const void* d_src, const int* d_slot_of, const Ro
     if (smem > (size_t)220 * 1024) return fail(PSB_UNSUPPORTED_SHAPE, "rows too long for the exact rerank");
     if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_rerank_score), smem));
     PSB_TRY(prefer_max_shared(k_rerank_score));
-    k_rerank_score<<<grid, kScoreThreads, smem, s>>>(
-        static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, elem_bytes, through, static_cast<const unsigned char*>(d_queries),
-        d_candidates, candidate_count, candidate_stride, d_counts, d_out_dist, mark);
+    PSB_TRY(launch_behind(chained, k_rerank_score, grid, kScoreThreads, smem, s, static_cast<const unsigned char*>(d_src), d_slot_of, mp, dim, elem_bytes, through, static_cast<const unsigned char*>(d_queries), d_candidates, candidate_count, candidate_stride, d_counts, d_out_dist, mark));
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
 }
 
-psb_status launch_call_tail(const unsigned long long* d_words, const int* d_coarse, CallTail* h_tail, cudaStream_t s) {
+psb_status launch_call_tail(const unsigned long long* d_words, const int* d_coarse, CallTail* h_tail, cudaStream_t s, bool chained) {
     PSB_TRY(prefer_max_shared(k_call_tail));
-    k_call_tail<<<1, 32, 0, s>>>(d_words, d_coarse, h_tail);
+    PSB_TRY(launch_behind(chained, k_call_tail, dim3(1), 32, 0, s, d_words, d_coarse, h_tail));
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
@@ -606,7 +607,7 @@ psb_status launch_call_tail(const unsigned long long* d_words, const int* d_coar
 
 psb_status launch_topk_select(const float* d_dist, const int* d_candidates, int nq, int candidate_count,
                               int candidate_stride, const int* d_counts, int topk, int* d_out_rows,
-                              float* d_out_dist, cudaStream_t s, const long long* d_ids, long long* d_out_ids) {
+                              float* d_out_dist, cudaStream_t s, const long long* d_ids, long long* d_out_ids, bool chained) {
     if (nq <= 0) return PSB_OK;
     if (candidate_count > kMaxRerankWidth) return fail(PSB_UNSUPPORTED_SHAPE, "rerank accepts at most 4096 candidates per query");
     int np = 32;
@@ -616,8 +617,7 @@ psb_status launch_topk_select(const float* d_dist, const int* d_candidates, int 
     if (smem > 32 * 1024)
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_topk_select), smem));
     PSB_TRY(prefer_max_shared(k_topk_select));
-    k_topk_select<<<nq, kSelectThreads, smem, s>>>(d_dist, d_candidates, candidate_count, candidate_stride, d_counts,
-                                                   topk, np, buffer, d_out_rows, d_out_dist, d_ids, d_out_ids);
+    PSB_TRY(launch_behind(chained, k_topk_select, dim3((unsigned)nq), kSelectThreads, smem, s, d_dist, d_candidates, candidate_count, candidate_stride, d_counts, topk, np, buffer, d_out_rows, d_out_dist, d_ids, d_out_ids));
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

@@ -506,6 +506,7 @@ struct psb_session {
     unsigned long long* call_marks = nullptr;
     const float* host_queries = nullptr;
     float* query_copy = nullptr;
+    bool one_stream = false;               // the call at work has no second stream: its kernels follow one another (launch_behind)
     static_assert(kSmallIo + sizeof(Tail) <= kHostBlock, "the tail lies behind the block's data");
     bool counters_known = false;           // h_tail->c is what the device's counters hold
     DevBuf row_dist, row_seg, row_runs, row_whole;   // a row of distances per query (IVF-Flat, row form of the ADC scan), the minima of every 32
@@ -814,7 +815,7 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, con
     g.row_delta = ix.row_delta; g.list_begin = ix.list_begin; g.list_end = ix.list_end; g.dim = ix.dim; g.m = ix.m; g.k = ix.k;
     g.residual = ix.residual; g.tree = scan_tree_order(ix); g.stage1_k = stage1_k; g.seg = s->row_seg.as<int>(); g.dist = s->row_dist.as<float>();
     g.expected_rows = expected_rows(s, nprobe); g.longest_list = s->longest[1]; g.counters = ws.counters; g.sm_count = s->sm_count;
-    g.mark = s->call_marks ? s->call_marks + 1 : nullptr;
+    g.mark = s->call_marks ? s->call_marks + 1 : nullptr; g.chained = s->one_stream;
     if (ws.ev_begin) PSB_CUDA(cudaEventRecord(ws.ev_begin, st));
     for (int q0 = 0; q0 < nq; q0 += per) {
         g.queries = d_queries + (size_t)q0 * s->dim; g.probes = d_probes + (size_t)q0 * nprobe;
@@ -1090,9 +1091,9 @@ bool rows_in_place(const psb_session* s, long long requests) {
 psb_status score_and_select(psb_session* s, bool in_place, const void* d_queries, int nq, const int* d_cand, int width, int stride, const int* d_counts,
                             int topk, int* d_out_rows, float* d_out_dist, long long* d_out_ids, float* d_score, cudaStream_t st) {
     PSB_TRY(launch_rerank_score(in_place ? s->exact_dev : s->stage.p, in_place ? nullptr : s->slot_of.as<int>(), s->row_map(), s->dim, s->exact_elem,
-                                d_queries, d_cand, nq, width, stride, d_counts, d_score, st, s->call_marks ? s->call_marks + 2 : nullptr));
+                                d_queries, d_cand, nq, width, stride, d_counts, d_score, st, s->call_marks ? s->call_marks + 2 : nullptr, s->one_stream && in_place));
     if (!d_out_rows && !d_out_ids) return PSB_OK;  // partial rerank: the caller combines the scores of all shards
-    return launch_topk_select(d_score, d_cand, nq, width, stride, d_counts, topk, d_out_rows, d_out_dist, st, s->reordered.as<long long>(), d_out_ids);
+    return launch_topk_select(d_score, d_cand, nq, width, stride, d_counts, topk, d_out_rows, d_out_dist, st, s->reordered.as<long long>(), d_out_ids, s->one_stream);
 }
 
 psb_status rerank_impl(psb_session* s, const void* d_queries, int nq, const int* d_cand, int width, int stride,
@@ -1652,7 +1653,7 @@ psb_status ensure_host_io(psb_session* s) {
 }
 // Queues the device's counters and status words behind the work on `st`.
 psb_status queue_tail(psb_session* s, cudaStream_t st) {
-    return launch_call_tail(s->scalars.as<unsigned long long>(), s->tc_work.scalars.as<int>(), s->h_tail, st);
+    return launch_call_tail(s->scalars.as<unsigned long long>(), s->tc_work.scalars.as<int>(), s->h_tail, st, s->call_marks != nullptr);
 }
 // Small calls on one stream: the kernels note their starts themselves and the first reads the queries where they are.  A recorded event costs the
 // GPU five microseconds between two kernels and the host two, and a small copy to the device as much again.
@@ -1741,6 +1742,11 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         PSB_CUDA(cudaStreamCreateWithPriority(&s->aux_stream, cudaStreamNonBlocking, lo));
     }
     cudaStream_t sx = (overlap || staged_overlap) ? s->aux_stream : st;
+    struct OneStream {
+        psb_session* s;
+        OneStream(psb_session* s_, bool one) : s(s_) { s->one_stream = one; }
+        ~OneStream() { s->one_stream = false; }
+    } one_stream(s, !overlap && !staged_overlap);
     struct EventList {  // destroyed on every way out of this function (an event may be destroyed once the waits on it are queued)
         std::vector<cudaEvent_t> v;
         ~EventList() { for (auto e : v) cudaEventDestroy(e); }
