@@ -1,6 +1,7 @@
 // The re-scoring selection behind the tensor-core scan (scan_tc.cu): exact distances of the filter's survivors and the stage1_k
 // smallest of each query.
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "common.cuh"
@@ -37,6 +38,7 @@ struct RescoreArgs {
     int shared_cut;   // the cutoff covers the rows of all shards: this shard need not reach stage1_k rows
     int sort_n;       // next_pow2(stage1_k)
     int staged;       // residual mode: codebook and residuals fit shared memory (else they are read through L1)
+    int above, upto;  // residual mode: the launch takes the queries with more pooled rows than this, and at most that many
 };
 
 __host__ __device__ __forceinline__ int residual_pitch(int dim, int dsub) { return dim + dsub; }   // residuals of different probes in different banks
@@ -204,22 +206,26 @@ __global__ void __launch_bounds__(T) k_select_rescore(const RescoreArgs g) {
     select_keys<T, KPT>(g, q, need, key, s_keys, s_cnt, s_pos);
 }
 
+// Takes the queries with more than g.above and at most g.upto pooled rows.
 template <int DSUB, int TREE, int T, int KPT>
-__global__ void __launch_bounds__(T) k_select_rescore_residual(const RescoreArgs g) {
+__global__ void __launch_bounds__(T, T == 512 && KPT <= 8 ? 2 : 1) k_select_rescore_residual(const RescoreArgs g) {
     extern __shared__ __align__(16) unsigned char s_sel[];
     const int pitch = residual_pitch(g.dim, DSUB);
     float* s_book = reinterpret_cast<float*>(s_sel);                            // [m][k][DSUB] when staged
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_book + (g.staged ? (size_t)g.m * g.k * DSUB : 0));   // [sort_n]
     float* s_res = reinterpret_cast<float*>(s_keys + g.sort_n);                 // staged: [nprobe][pitch] residuals, else the query [dim]
     __shared__ int s_cnt[64], s_pos[3];
-    if (g.staged) {
-        const int n4 = g.m * g.k * DSUB / 4;
-#pragma unroll 4
-        for (int i = threadIdx.x; i < n4; i += T) reinterpret_cast<float4*>(s_book)[i] = __ldg(reinterpret_cast<const float4*>(g.codebook) + i);
-    }
+    bool there = !g.staged;   // the codebook
     for (int q = blockIdx.x; q < g.nq; q += gridDim.x) {
-        __syncthreads();   // the previous query is done with shared memory
         const int c = g.pool_cnt[q];
+        if (c <= g.above || c > g.upto) continue;   // uniform
+        if (!there) {
+            const int n4 = g.m * g.k * DSUB / 4;
+#pragma unroll 4
+            for (int i = threadIdx.x; i < n4; i += T) reinterpret_cast<float4*>(s_book)[i] = __ldg(reinterpret_cast<const float4*>(g.codebook) + i);
+            there = true;
+        }
+        __syncthreads();   // the previous query is done with shared memory
         const long long need = rescore_need(g, q, c);
         if (need < 0) continue;   // uniform
         const float* qv = g.queries + (size_t)q * g.dim;
@@ -281,15 +287,29 @@ psb_status run_select_rescore_residual(RescoreArgs g, int sm_count, cudaStream_t
     const size_t keys = (size_t)g.sort_n * 8, book = (size_t)g.m * g.k * DSUB * 4, res = (size_t)g.nprobe * residual_pitch(g.dim, DSUB) * 4;
     g.staged = keys + book + res <= (size_t)220 * 1024 && ((size_t)g.m * g.k * DSUB) % 4 == 0 ? 1 : 0;
     const size_t smem = keys + (g.staged ? book + res : (size_t)g.dim * 4);
-    return by_capacity(g.pool_cap, [&](auto t, auto kpt) -> psb_status {
+    auto run = [&](auto t, auto kpt) -> psb_status {
         constexpr int T = decltype(t)::value, KPT = decltype(kpt)::value;
         auto kernel = k_select_rescore_residual<DSUB, TREE, T, KPT>;
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
         PSB_TRY(prefer_max_shared(kernel));
-        const int per_sm = (int)std::max<size_t>(1, std::min<size_t>((size_t)220 * 1024 / (smem + 1024), 1024 / T));
+        // An SM's 228 KB, of which a block takes one for itself, and the static words.
+        const int per_sm = (int)std::max<size_t>(1, std::min<size_t>((size_t)228 * 1024 / (smem + 1024 + 272), 1024 / T));
         kernel<<<(unsigned)std::min(g.nq, sm_count * per_sm), T, smem, s>>>(g);
         return PSB_OK;
-    });
+    };
+    g.above = -1; g.upto = INT_MAX;
+    // A pool is sized for sixteen times the rows wanted, and rarely holds twice as many: with room for 2,048 (4,096) keys a thread needs half the registers,
+    // and two blocks of 512 share an SM, one's latencies behind the other's work.  The few queries with more go to a launch of their own.
+    const int usual = g.stage1_k <= 512 ? 2048 : 4096;
+    if (g.pool_cap > usual) {
+        g.upto = usual;
+        if (usual == 2048) PSB_TRY(run(std::integral_constant<int, 512>(), std::integral_constant<int, 4>()));
+        else PSB_TRY(run(std::integral_constant<int, 512>(), std::integral_constant<int, 8>()));
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        g.above = usual; g.upto = INT_MAX;
+    }
+    return by_capacity(g.pool_cap, run);
 }
 template <int DSUB>
 psb_status run_select_rescore_tree(const RescoreArgs& g, int sm_count, cudaStream_t s) {
