@@ -38,7 +38,7 @@ struct RescoreArgs {
     int shared_cut;   // the cutoff covers the rows of all shards: this shard need not reach stage1_k rows
     int sort_n;       // next_pow2(stage1_k)
     int staged;       // residual mode: codebook and residuals fit shared memory (else they are read through L1)
-    int above, upto;  // residual mode: the launch takes the queries with more pooled rows than this, and at most that many
+    int above, upto;  // the launch takes the queries with more pooled rows than this, and at most that many
 };
 
 __host__ __device__ __forceinline__ int residual_pitch(int dim, int dsub) { return dim + dsub; }   // residuals of different probes in different banks
@@ -173,13 +173,14 @@ __device__ __forceinline__ long long rescore_need(const RescoreArgs& g, int q, i
 }
 
 template <int M, int T, int KPT>
-__global__ void __launch_bounds__(T) k_select_rescore(const RescoreArgs g) {
+__global__ void __launch_bounds__(T, T == 512 && KPT <= 8 ? 2 : 1) k_select_rescore(const RescoreArgs g) {
     extern __shared__ __align__(16) unsigned char s_sel[];
     uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_sel);                      // [sort_n]
     float* s_tab = reinterpret_cast<float*>(s_sel + (size_t)g.sort_n * 8);      // [m * k]
     __shared__ int s_cnt[64], s_pos[3];
     const int q = blockIdx.x;
     const int c = g.pool_cnt[q];
+    if (c <= g.above || c > g.upto) return;
     const long long need = rescore_need(g, q, c);
     if (need < 0) return;
     const int mk = g.m * g.k;
@@ -270,11 +271,27 @@ psb_status by_capacity(int cap, F run) {
     if (cap <= 8192) return run(std::integral_constant<int, 512>(), std::integral_constant<int, 16>());
     return run(std::integral_constant<int, 1024>(), std::integral_constant<int, 16>());
 }
+// A pool is sized for sixteen times the rows wanted, and rarely holds twice as many: with room for 2,048 (4,096) keys a thread needs half the
+// registers, and two blocks of 512 share an SM, one's latencies behind the other's work.  The few queries with more go to a launch of their own.
+template <typename F>
+psb_status by_pool(RescoreArgs& g, F run) {
+    const int usual = g.stage1_k <= 512 ? 2048 : 4096;
+    g.above = -1; g.upto = INT_MAX;
+    if (g.pool_cap > usual) {
+        g.upto = usual;
+        if (usual == 2048) PSB_TRY(run(std::integral_constant<int, 512>(), std::integral_constant<int, 4>()));
+        else PSB_TRY(run(std::integral_constant<int, 512>(), std::integral_constant<int, 8>()));
+        count_launch();
+        PSB_LAUNCH_CHECK();
+        g.above = usual; g.upto = INT_MAX;
+    }
+    return by_capacity(g.pool_cap, run);
+}
 template <int M>
-psb_status run_select_rescore(const RescoreArgs& g, cudaStream_t s) {
+psb_status run_select_rescore(RescoreArgs g, cudaStream_t s) {
     const size_t smem = (size_t)g.sort_n * 8 + (size_t)g.m * g.k * 4;
     if (smem > (size_t)220 * 1024) return fail(PSB_UNSUPPORTED_SHAPE, "re-scoring selection does not fit shared memory");
-    return by_capacity(g.pool_cap, [&](auto t, auto kpt) -> psb_status {
+    return by_pool(g, [&](auto t, auto kpt) -> psb_status {
         constexpr int T = decltype(t)::value, KPT = decltype(kpt)::value;
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_select_rescore<M, T, KPT>), smem));
         PSB_TRY(prefer_max_shared(k_select_rescore<M, T, KPT>));
@@ -297,19 +314,7 @@ psb_status run_select_rescore_residual(RescoreArgs g, int sm_count, cudaStream_t
         kernel<<<(unsigned)std::min(g.nq, sm_count * per_sm), T, smem, s>>>(g);
         return PSB_OK;
     };
-    g.above = -1; g.upto = INT_MAX;
-    // A pool is sized for sixteen times the rows wanted, and rarely holds twice as many: with room for 2,048 (4,096) keys a thread needs half the registers,
-    // and two blocks of 512 share an SM, one's latencies behind the other's work.  The few queries with more go to a launch of their own.
-    const int usual = g.stage1_k <= 512 ? 2048 : 4096;
-    if (g.pool_cap > usual) {
-        g.upto = usual;
-        if (usual == 2048) PSB_TRY(run(std::integral_constant<int, 512>(), std::integral_constant<int, 4>()));
-        else PSB_TRY(run(std::integral_constant<int, 512>(), std::integral_constant<int, 8>()));
-        count_launch();
-        PSB_LAUNCH_CHECK();
-        g.above = usual; g.upto = INT_MAX;
-    }
-    return by_capacity(g.pool_cap, run);
+    return by_pool(g, run);
 }
 template <int DSUB>
 psb_status run_select_rescore_tree(const RescoreArgs& g, int sm_count, cudaStream_t s) {

@@ -241,3 +241,17 @@ def test_tc_scan_bounded_wait_gives_up_cleanly(psb):
     rows, dist, cnt, _ = run_scan(psb, ix, q, probes, 50, 3)
     orow, odist, ocnt, _ = oracle.pq_scan(q, probes, ix["offsets"], ix["codes"], ix["codebook"], 50)
     assert np.array_equal(rows, orow) and np.array_equal(dist, odist) and np.array_equal(cnt, ocnt)
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("width", [512, 513, 1000])          # pools of 8,192 and 16,384 keys, the usual 2,048 and 4,096
+@pytest.mark.parametrize("sigma", [2.0, 10.0])               # pools on both sides of the usual size
+def test_usual_and_large_pools(psb, residual, width, sigma):
+    import synth
+    ix = synth.make_index(90000, 32, 10, 8, seed=12, zipf=True, residual=residual) if residual else synth.make_index(90000, 32, 10, 8, seed=12, zipf=True)
+    q = synth.make_queries(ix, 70, seed=13)
+    got = {}
+    for mode in (1, 3):
+        with psb.Session(ix, n_rerank=width, scan_mode=mode, residual=residual, seed_sigma=sigma, exact_mode=psb.EXACT_HOST_CACHED, max_batch=70) as s:
+            got[mode] = s.search(q, 7, 20, batch_size=70)
+    assert np.array_equal(got[1]["indices"], got[3]["indices"]) and np.array_equal(got[1]["distances"], got[3]["distances"])
