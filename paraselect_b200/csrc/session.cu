@@ -757,11 +757,40 @@ int sub_batch_rows(const psb_session* s, int n, int nprobe, bool overlap) {
 
 int host_share(const psb_session* s);
 bool device_rows(const psb_session* s);
+bool rows_in_place(const psb_session* s, long long requests);
 // The staged transport (host gather threads + pinned rings), alone or with the kernel gather beside it.
 bool staged_mode(const psb_session* s) { return !device_rows(s) && host_share(s) > 0; }
 
 bool overlap_enabled(const psb_session* s, int n, bool rerank) {
     return rerank && !staged_mode(s) && n >= 2048 && !s->opt.serial_pipeline;
+}
+
+bool staged_overlap_enabled(const psb_session* s, int n, bool rerank) { return rerank && staged_mode(s) && n >= 2048 && !s->opt.serial_pipeline; }
+
+// Whether the rows of a whole batch are claimed and fetched once each, sub-batch by sub-batch.
+bool rows_shared(const psb_session* s, int n, int stage1_k, bool rerank) {
+    return staged_overlap_enabled(s, n, rerank) || (overlap_enabled(s, n, rerank) && !rows_in_place(s, (long long)n * stage1_k));
+}
+
+// Sub-batch boundaries of a batch.  Equal cuts, except where rows of host memory are fetched beside the scan.  There the transfer is about as
+// long as the scan and costs it little, so the first sub-batch is a small one: the transfer starts early.  Where the kernel fetches, the cuts grow so
+// that a sub-batch's scan takes about as long as the transfer of the one before, and the last is small again, for nothing hides its transfer
+// (100M x 96, 10,000 queries x 1,000 candidates: 12/18/22/26/22 % 84.3 ms, 10/20/20/25/25 86.1, 10/30/30/30 88.6, seven parts 90.3; no difference
+// at 1M to 12M rows).  Host threads are slower than the scan: 10/30/30/30 %.
+std::vector<int> batch_cuts(const psb_session* s, int n, int nprobe, int stage1_k, bool rerank) {
+    const int sb = sub_batch_rows(s, n, nprobe, overlap_enabled(s, n, rerank) || staged_overlap_enabled(s, n, rerank));
+    const int plan = s->opt.even_cuts;
+    if (rows_shared(s, n, stage1_k, rerank) && (s->opt.adc_mode != 1 || residual_table_free(s, stage1_k)) && sb * 4 >= n && n >= 4096 && plan != 1) {
+        if (plan == 2) return {0, (int)(0.32 * n), (int)(0.64 * n), (int)(0.90 * n), n};  // short last sub-batch (scan-bound hosts)
+        if (host_share(s) == 0) return {0, (int)(0.12 * n), (int)(0.30 * n), (int)(0.52 * n), (int)(0.78 * n), n};
+        return {0, (int)(0.10 * n), (int)(0.40 * n), (int)(0.70 * n), n};
+    }
+    return even_cuts(n, sb);
+}
+int longest_cut(const std::vector<int>& cuts) {
+    int most = 0;
+    for (size_t i = 0; i + 1 < cuts.size(); ++i) most = std::max(most, cuts[i + 1] - cuts[i]);
+    return most;
 }
 
 // Grows the scan workspace to hold nq queries (never shrinks; a growing buffer is freed first, which waits for the device).
@@ -830,7 +859,9 @@ psb_status run_scan(psb_session* s, const ScanWorkspace& ws, bool rows_only, con
 }
 
 psb_status ensure_pipeline_ws(psb_session* s, int nq, int nprobe, int topk, int stage1_k) {
-    const int sb = sub_batch_rows(s, nq, nprobe, overlap_enabled(s, nq, rerank_enabled(s, topk)));
+    // For the longest sub-batch: a session's first call lays its workspace out once (for a quarter of the batch where a cut is longer, it was freed and
+    // laid out anew within the call, 1.5 ms of 10.1).
+    const int sb = longest_cut(batch_cuts(s, nq, nprobe, stage1_k, rerank_enabled(s, topk)));
     const size_t n = (size_t)nq;
     PSB_TRY(reserve_together(&s->call_whole, {{&s->q, sizeof(float) * n * s->dim}, {&s->probes, sizeof(int) * n * nprobe},
                                               {&s->cand_rows, sizeof(int) * n * stage1_k},
@@ -1707,30 +1738,15 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     // Staged transport, overlapped: a host worker thread takes each sub-batch's candidates as soon as its scan has finished,
     // gathers the rows with the host cores into the pinned rings and queues copies + exact scoring on the second stream,
     // while this thread goes on queueing the next sub-batch's scan.  No SM is spent on the transfer.
-    const bool staged_overlap = rerank && staged_mode(s) && n >= 2048 && !s->opt.serial_pipeline;
-    const int sb = sub_batch_rows(s, n, nprobe, overlap || staged_overlap);
+    const bool staged_overlap = staged_overlap_enabled(s, n, rerank);
     const bool residual = s->opt.adc_mode == 1;
     // The rows of the whole batch are claimed and fetched once each, sub-batch by sub-batch (a row an earlier sub-batch has fetched is
     // in its slot already), unless they are scored in place.
     const int host_pct = host_share(s);
-    const bool shared_rows = staged_overlap || (overlap && !rows_in_place(s, (long long)n * stage1_k));
+    const bool shared_rows = rows_shared(s, n, stage1_k, rerank);
     const bool kernel_gather = shared_rows && host_pct < 100;   // on a stream of its own
-    // Sub-batch boundaries.  Equal cuts, except where rows of host memory are fetched beside the scan.  There the transfer is about as long as
-    // the scan and costs it little, so the first sub-batch is a small one: the transfer starts early.  Where the kernel fetches, the cuts grow so that
-    // a sub-batch's scan takes about as long as the transfer of the one before, and the last is small again, for nothing hides its transfer
-    // (100M x 96, 10,000 queries x 1,000 candidates: 12/18/22/26/22 % 84.3 ms, 10/20/20/25/25 86.1, 10/30/30/30 88.6, seven parts 90.3; no difference
-    // at 1M to 12M rows).  Host threads are slower than the scan: 10/30/30/30 %.
-    std::vector<int> cuts;
-    const int plan = s->opt.even_cuts;
-    if (shared_rows && (!residual || residual_table_free(s, stage1_k)) && sb * 4 >= n && n >= 4096 && plan != 1) {
-        if (plan == 2) cuts = {0, (int)(0.32 * n), (int)(0.64 * n), (int)(0.90 * n), n};  // short last sub-batch (scan-bound hosts)
-        else if (host_pct == 0) cuts = {0, (int)(0.12 * n), (int)(0.30 * n), (int)(0.52 * n), (int)(0.78 * n), n};
-        else cuts = {0, (int)(0.10 * n), (int)(0.40 * n), (int)(0.70 * n), n};
-    } else {
-        cuts = even_cuts(n, sb);
-    }
-    int sb_max = 0;
-    for (size_t ci = 0; ci + 1 < cuts.size(); ++ci) sb_max = std::max(sb_max, cuts[ci + 1] - cuts[ci]);
+    const std::vector<int> cuts = batch_cuts(s, n, nprobe, stage1_k, rerank);
+    const int sb_max = longest_cut(cuts);
     // The sub-batch size depends on this batch's own n (a short tail batch may run in one piece where the full batch ran
     // in four), so the tables and the scan workspace are sized here, for the largest sub-batch of THIS batch.
     const bool rows_only = rows_form(s, sb_max, nprobe), table_free = residual_table_free(s, stage1_k) || rows_only;
