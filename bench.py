@@ -328,12 +328,12 @@ def main():
     ap.add_argument("--cpu-sample", type=int, default=0, help="queries in the CPU baseline sample (0 = auto)")
     ap.add_argument("--exact-mode", default="auto", choices=["auto", "mapped", "staged", "cached", "hybrid"],
                     help="rerank transport on one GPU: staged = host threads gather rows into pinned rings and cudaMemcpyAsync moves "
-                         "them (no SM time spent on the transfer), mapped = kernels gather mapped host rows over PCIe; "
+                         "them (no SM time spent on the transfer), mapped = a kernel gathers mapped host rows over PCIe in ascending order; "
                          "auto = hybrid when a batch asks for at least 2 GB of rows (the scan is then long enough to run beside the transfer), else mapped; "
                          "cached = the session copies the rows into device memory once (not the host-resident configuration the "
-                         "headline metric names: an extra data point); hybrid = staged and mapped at once, --zero-copy-pct of every "
-                         "sub-batch through the kernel")
-    ap.add_argument("--zero-copy-pct", type=int, default=0, help="hybrid transport: share of each sub-batch gathered by the kernel (0 = library default)")
+                         "headline metric names: an extra data point); hybrid = mapped, or with --zero-copy-pct both at once: that "
+                         "share of every sub-batch through the kernel, the others through the host threads")
+    ap.add_argument("--zero-copy-pct", type=int, default=0, help="hybrid transport: share of each sub-batch gathered by the kernel (0 = all of it)")
     ap.add_argument("--reserve-sms", type=int, default=24, help="N > 1: SMs the scan's persistent grid leaves to the exchange half "
                     "(the PCIe gather of the exact rows runs on that many SMs of its own, the collectives beside it)")
     ap.add_argument("--parts", type=int, default=4, help="N > 1: sub-batches per batch")
