@@ -87,6 +87,24 @@ def test_tc_filter_does_the_work_not_the_fallback(psb):
     assert np.array_equal(out[2][0], oi) and np.array_equal(out[2][1], od)
 
 
+@pytest.mark.parametrize("nlist", [1024, 2148])
+def test_tc_coarse_batches_one_after_the_other(psb, nlist):
+    """The candidate masks of one batch must not reach the next: batches of falling and ragged size on one session."""
+    import torch
+    import synth
+    ix = synth.make_index(6000, 64, nlist, 16, seed=21)
+    with psb.Session(dict(ix, vectors=None), coarse_mode=2) as s:
+        for seed, nq in ((1, 203), (2, 203), (3, 65), (4, 129)):
+            q = synth.make_queries(ix, nq, seed=seed)
+            ids = torch.empty((nq, 24), dtype=torch.int32, device="cuda")
+            dist = torch.empty((nq, 24), dtype=torch.float32, device="cuda")
+            s.stage_coarse(torch.from_numpy(q).cuda(), nq, 24, ids, dist)
+            s.sync()
+            oi, od = oracle.coarse(q, ix["centroids"], 24)
+            assert np.array_equal(ids.cpu().numpy(), oi) and np.array_equal(dist.cpu().numpy(), od)
+            assert s.counters()["coarse_fallback_queries"] == 0
+
+
 def test_kmeans_assignment_on_the_tensor_core_filter(psb):
     """k = 1024 centroids takes the tensor-core filter with exact refinement for the assignment step (the coarse stage
     with nprobe 1); assignments, objective and centroids must equal the exact SIMT path's, i.e. the checker's."""
