@@ -399,13 +399,15 @@ __host__ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 //                  takes most of the pass.  The rows of a group of at most 1,024 are put in order first (each finds its rank among the others: one barrier where a bitonic sort of
 //                  64 rows has 21), so that the sum does not depend on the order the slots were taken
 constexpr int kKmSplit = 8;
-__global__ void k_km_count(const int* __restrict__ assign, const float* __restrict__ best, long long n, int* __restrict__ counts,
+// Of the four kernels below each passes over a row whose assignment is no centroid (a row that is not a number has no nearest one).
+__global__ void k_km_count(const int* __restrict__ assign, const float* __restrict__ best, long long n, int k, int* __restrict__ counts,
                            double* __restrict__ obj) {
     __shared__ double s_part[8];
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double b = 0.0;
     if (i < n) {
-        atomicAdd(&counts[assign[i]], 1);
+        const int c = assign[i];
+        if ((unsigned)c < (unsigned)k) atomicAdd(&counts[c], 1);
         if (best) b = (double)best[i];
     }
     if (!obj) return;
@@ -433,11 +435,12 @@ __global__ void __launch_bounds__(1024) k_km_offsets(const int* __restrict__ cou
     }
     if (threadIdx.x == 0) offsets[k] = carry;
 }
-__global__ void k_km_fill(const int* __restrict__ assign, long long n, const int* __restrict__ offsets, int* __restrict__ cursor,
+__global__ void k_km_fill(const int* __restrict__ assign, long long n, int k, const int* __restrict__ offsets, int* __restrict__ cursor,
                           int* __restrict__ order) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int c = assign[i];
+    if ((unsigned)c >= (unsigned)k) return;
     order[offsets[c] + atomicAdd(&cursor[c], 1)] = (int)i;
 }
 // The same two for few centroids, whose counters all rows would queue at: a block counts its kFewRows rows in shared memory first, and takes the
@@ -455,7 +458,8 @@ __global__ void __launch_bounds__(1024) k_km_count_few(const int* __restrict__ a
     for (int t = 0; t < kFewRows / 1024; ++t) {
         const long long i = (long long)blockIdx.x * kFewRows + t * 1024 + threadIdx.x;
         if (i < n) {
-            atomicAdd(&s_count[assign[i]], 1);
+            const int c = assign[i];
+            if ((unsigned)c < (unsigned)k) atomicAdd(&s_count[c], 1);
             if (best) b += (double)best[i];
         }
     }
@@ -482,6 +486,7 @@ __global__ void __launch_bounds__(1024) k_km_fill_few(const int* __restrict__ as
     for (int t = 0; t < kFewRows / 1024; ++t) {
         const long long i = (long long)blockIdx.x * kFewRows + t * 1024 + threadIdx.x;
         own[t] = i < n ? assign[i] : -1;
+        if (own[t] >= k) own[t] = -1;
         slot[t] = own[t] >= 0 ? atomicAdd(&s_count[own[t]], 1) : 0;
     }
     __syncthreads();
@@ -686,7 +691,7 @@ psb_status launch_kmeans_accumulate(const float* d_data, long long n, int dim, c
     // d_counts and *d_obj were zeroed by the caller; d_sums is written whole
     if (n > 0) {
         if (k <= kFewCentroids) k_km_count_few<<<(unsigned)((n + kFewRows - 1) / kFewRows), 1024, 0, s>>>(d_assign, d_best, n, k, d_counts, d_obj);
-        else k_km_count<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_assign, d_best, n, d_counts, d_obj);
+        else k_km_count<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_assign, d_best, n, k, d_counts, d_obj);
         count_launch();
         PSB_LAUNCH_CHECK();
     }
@@ -695,7 +700,7 @@ psb_status launch_kmeans_accumulate(const float* d_data, long long n, int dim, c
     PSB_LAUNCH_CHECK();
     if (n > 0) {
         if (k <= kFewCentroids) k_km_fill_few<<<(unsigned)((n + kFewRows - 1) / kFewRows), 1024, 0, s>>>(d_assign, n, k, ws.offsets, ws.cursor, ws.order);
-        else k_km_fill<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_assign, n, ws.offsets, ws.cursor, ws.order);
+        else k_km_fill<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_assign, n, k, ws.offsets, ws.cursor, ws.order);
         count_launch();
         PSB_LAUNCH_CHECK();
     }
