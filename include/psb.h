@@ -537,6 +537,12 @@ psb_status psb_pq_train(const float* d_data, int64_t n, int dim, int subvectors,
  * d_codes [n][subvectors] out. */
 psb_status psb_pq_encode(const float* d_data, int64_t n, int dim, const float* d_codebook, int subvectors,
                          int codebook_size, uint8_t* d_codes, int device, void* stream);
+/* Test hook of the time-out path of the encoder's tensor-core filter: psb_pq_encode for shapes that have one, of whose work items only the
+ * first `items` get their products (-1: all).  A block with another waits in vain; it then waits for the products it has issued, frees its
+ * tensor memory and evaluates its rows without the filter, so that the codes are the same.  *d_gave_up (device, may be null) grows by one
+ * for each such block. */
+psb_status psb_pq_encode_limited(const float* d_data, int64_t n, int dim, const float* d_codebook, int subvectors, int codebook_size,
+                                 uint8_t* d_codes, int64_t items, int* d_gave_up, int device, void* stream);
 
 /* ---- index-build glue (host side: layout only, no arithmetic) ------------------------------------------------ */
 

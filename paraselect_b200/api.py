@@ -105,7 +105,7 @@ EXPORTS = [
     "psb_sizeof", "psb_kmeans_assign_bounded", "psb_group_create", "psb_group_set", "psb_group_search_device", "psb_group_searched_again", "psb_group_destroy",
     "psb_sign_padded_dim", "psb_sign_rotation_scale", "psb_sign_rotate", "psb_sign_encode_database", "psb_sign_encode_queries", "psb_sign_search_candidates",
     "psb_kmeans_init", "psb_rotate_rows", "psb_stage_rotate_queries", "psb_scan_sample_words", "psb_stage_scan_sample", "psb_stage_scan_shared",
-    "psb_ivf_layout_from_assignment", "psb_reorder_rows", "psb_coarse_host", "psb_coarse_search_static", "psb_knn_exact", "psb_kmeans_train", "psb_kmeans_assign", "psb_kmeans_accumulate", "psb_kmeans_update", "psb_residual_rows", "psb_pq_train", "psb_pq_encode", "psb_gen_mixture_rows", "psb_gen_normal",
+    "psb_ivf_layout_from_assignment", "psb_reorder_rows", "psb_coarse_host", "psb_coarse_search_static", "psb_knn_exact", "psb_kmeans_train", "psb_kmeans_assign", "psb_kmeans_accumulate", "psb_kmeans_update", "psb_residual_rows", "psb_pq_train", "psb_pq_encode", "psb_pq_encode_limited", "psb_gen_mixture_rows", "psb_gen_normal",
 ]
 
 _lib = None
@@ -819,6 +819,12 @@ def pq_train(d_data, n, dim, M, K, iters, seed, d_codebook, device=0, stream=Non
 def pq_encode(d_data, n, dim, d_codebook, M, K, d_codes, device=0, stream=None):
     _check(lib().psb_pq_encode(C.c_void_p(_p(d_data)), C.c_int64(n), dim, C.c_void_p(_p(d_codebook)), M, K,
                                C.c_void_p(_p(d_codes)), device, _stream_ptr(stream)))
+
+
+def pq_encode_limited(d_data, n, dim, d_codebook, M, K, d_codes, items=-1, d_gave_up=None, device=0, stream=None):
+    """Test hook of the time-out path of pq_encode's filter; see include/psb.h."""
+    _check(lib().psb_pq_encode_limited(C.c_void_p(_p(d_data)), C.c_int64(n), dim, C.c_void_p(_p(d_codebook)), M, K, C.c_void_p(_p(d_codes)),
+                                       C.c_int64(items), C.c_void_p(_p(d_gave_up)), device, _stream_ptr(stream)))
 
 
 def gen_mixture_rows(d_centres, d_offsets, ncomp, dim, sigma, seed, row_begin, n, d_out, device=0, stream=None):

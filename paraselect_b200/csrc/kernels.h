@@ -371,8 +371,11 @@ psb_status launch_widen_ids(const int* d_in, long long n, long long* d_out, cuda
 
 // ---- training ------------------------------------------------------------------------------------------------
 bool pq_nearest_supported(int dsub, int k, bool train);   // pq_nearest.cu: the tensor-core filter takes sub-vectors of this length
+// Test hook of its time-out path: the work items that get their products (-1: all; a CTA with others waits for them in vain), and the count of CTAs
+// that gave up and evaluated their rows without the filter.
+struct NearTest { long long items = -1; int* gave_up = nullptr; };
 psb_status launch_pq_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, bool train, uint8_t* d_codes, int sm_count,
-                             cudaStream_t s);
+                             cudaStream_t s, const NearTest& test = {});
 psb_status launch_pq_encode(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k,
                             uint8_t* d_codes, int sm_count, cudaStream_t s);
 // The assignment of PQ training's Lloyd iterations: |c|^2 - 2 x.c in fused multiply-adds for sub-vectors of 2, 4 or 8 (else the encoder's

@@ -206,6 +206,8 @@ struct NearArgs {
     int vec;                 // sub-vectors may be loaded V floats at a time
     int step_atom;           // from one item of a CTA to its next: atoms, and tiles
     long long step_tiles;
+    long long issued;        // the items below this one get their products: all, or fewer in the test of the time-out path
+    int* gave_up;            // the test's count of CTAs that gave up, or null
 };
 
 // The items of a CTA in order; every role walks them on its own.
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pq_nearest(const NearArgs g) {
     unsigned char* s_a = s_b + 2 * P::B;                                   // [kRingA] operand of a row tile
     float* s_cb = reinterpret_cast<float*>(s_a + kRingA * P::A);            // [2][SPA][kCodes][D] the codewords
     float* s_x = s_cb + 2 * P::CB / 4;                                     // [kRingX][kTile][PITCH]
-    __shared__ __align__(8) uint64_t b_full[2], b_empty[2], a_full[kRingX], a_empty[kRingA], x_empty[kRingX], acc_full[kGroups][kAcc], acc_empty[kAcc];
+    __shared__ __align__(8) uint64_t b_full[2], b_empty[2], a_full[kRingX], a_empty[kRingA], x_empty[kRingX], acc_full[kGroups][kAcc], acc_empty[kAcc], drained;
     __shared__ __align__(16) float s_cmax[2][SPA][kCodes / 32];   // largest |c|^2 of every 32 codewords
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
@@ -277,6 +279,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pq_nearest(const NearArgs g) {
             for (int p = 0; p < kGroups; ++p) mbar_init(&acc_full[p][i], 1);
             mbar_init(&acc_empty[i], 4);
         }
+        mbar_init(&drained, 1);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pq_nearest(const NearArgs g) {
         const uint32_t idesc = idesc_bf16(kTile, kCodes);
         const uint64_t da0 = make_sw128_desc(smem_u32(s_a)), db0 = make_sw128_desc(smem_u32(s_b));   // the address field counts 16-byte units
         uint32_t seq = 0;
-        for (NearItem o(g); o.live(g) && !failed; o.next(g)) {
+        for (NearItem o(g); o.id < g.issued && !failed; o.next(g)) {
             const int nsub = o.subs<SPA>(g), ntiles = o.tiles(g);
             const uint32_t bs = o.it & 1u;
             if (!near_wait_warp(&b_full[bs], (o.it >> 1) & 1u, abort_flag)) { failed = true; break; }
@@ -509,9 +512,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_pq_nearest(const NearArgs g) {
             }
             if (!failed && elected) umma_commit(&b_empty[bs]);
             __syncwarp();
-            // Before it leaves: the last commits have arrived, so that none is left to write to this CTA's shared memory.
-            if (!failed && o.id + gridDim.x >= g.items && !near_wait_warp(&b_empty[bs], (o.it >> 1) & 1u, abort_flag)) failed = true;
         }
+        // Whether or not a wait gave up: the products issued are done before the tensor memory that they write and the operands that they read go to
+        // someone else.  No other role has a part in this wait, so the flag does not end it.
+        if (elected) umma_commit(&drained);
+        __syncwarp();
+        if (!__all_sync(0xffffffffu, mbar_wait(&drained, 0, kNearWaitLimit))) failed = true;
     }
     if (failed) *abort_flag = 1;
     tc_fence_before();
@@ -519,6 +525,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pq_nearest(const NearArgs g) {
     if (warp == 0) tmem_dealloc(tmem, kTmemCols);
     if (!s_abort) return;
     // A bounded wait gave up: the CTA's items are evaluated one codeword after the other.
+    if (g.gave_up && tid == 0) atomicAdd(g.gave_up, 1);
     for (long long id = blockIdx.x; id < g.items; id += gridDim.x) {
         const int atom = (int)(id % g.atoms), nsub = min(SPA, g.m - atom * SPA);
         const long long r0 = id / g.atoms * g.per * kTile, r1 = min(g.n, r0 + (long long)g.per * kTile);
@@ -539,7 +546,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_pq_nearest(const NearArgs g) {
 }
 
 template <int D, bool kTrain>
-psb_status run_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, uint8_t* d_codes, int sm_count, cudaStream_t s) {
+psb_status run_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, uint8_t* d_codes, int sm_count, cudaStream_t s,
+                       const NearTest& test) {
     using P = Near<D>;
     NearArgs g;
     g.data = d_data; g.codebook = d_codebook; g.codes = d_codes; g.n = n; g.dim = dim; g.m = m; g.k = k;
@@ -551,6 +559,7 @@ psb_status run_nearest(const float* d_data, long long n, int dim, const float* d
     g.items = (g.tiles + g.per - 1) / g.per * g.atoms;
     const unsigned grid = (unsigned)std::min<long long>(g.items, sm_count);
     g.step_atom = (int)(grid % (unsigned)g.atoms); g.step_tiles = (long long)(grid / (unsigned)g.atoms) * g.per;
+    g.issued = test.items >= 0 ? std::min<long long>(test.items, g.items) : g.items; g.gave_up = test.gave_up;
     g.vec = dim % P::V == 0 && reinterpret_cast<uintptr_t>(d_data) % (4 * P::V) == 0 ? 1 : 0;
     PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_pq_nearest<D, kTrain>), P::SMEM));
     k_pq_nearest<D, kTrain><<<grid, kThreads, P::SMEM, s>>>(g);
@@ -569,26 +578,26 @@ bool pq_nearest_supported(int dsub, int k, bool train) {
 }
 
 psb_status launch_pq_nearest(const float* d_data, long long n, int dim, const float* d_codebook, int m, int k, bool train, uint8_t* d_codes, int sm_count,
-                             cudaStream_t s) {
+                             cudaStream_t s, const NearTest& test) {
     if (n <= 0) return PSB_OK;
     if (train) {
         switch (dim / m) {
-            case 2: return run_nearest<2, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 4: return run_nearest<4, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 8: return run_nearest<8, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 2: return run_nearest<2, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 4: return run_nearest<4, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 8: return run_nearest<8, true>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
             default: break;
         }
     } else {
         switch (dim / m) {
-            case 2: return run_nearest<2, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 3: return run_nearest<3, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 4: return run_nearest<4, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 5: return run_nearest<5, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 6: return run_nearest<6, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 8: return run_nearest<8, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 10: return run_nearest<10, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 12: return run_nearest<12, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
-            case 16: return run_nearest<16, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s);
+            case 2: return run_nearest<2, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 3: return run_nearest<3, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 4: return run_nearest<4, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 5: return run_nearest<5, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 6: return run_nearest<6, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 8: return run_nearest<8, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 10: return run_nearest<10, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 12: return run_nearest<12, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
+            case 16: return run_nearest<16, false>(d_data, n, dim, d_codebook, m, k, d_codes, sm_count, s, test);
             default: break;
         }
     }

@@ -2753,6 +2753,19 @@ psb_status psb_pq_encode(const float* d_data, int64_t n, int dim, const float* d
     return launch_pq_encode(d_data, n, dim, d_codebook, subvectors, codebook_size, d_codes, sms, static_cast<cudaStream_t>(stream));
 }
 
+psb_status psb_pq_encode_limited(const float* d_data, int64_t n, int dim, const float* d_codebook, int subvectors, int codebook_size,
+                                 uint8_t* d_codes, int64_t items, int* d_gave_up, int device, void* stream) {
+    if (!d_data || !d_codebook || !d_codes || n < 0 || dim <= 0 || subvectors <= 0 || dim % subvectors ||
+        codebook_size <= 0 || codebook_size > kMaxCodebook)
+        return fail(PSB_INVALID_ARGUMENT, "invalid PQ encode request");
+    if (!pq_nearest_supported(dim / subvectors, codebook_size, false)) return fail(PSB_UNSUPPORTED_SHAPE, "no filter takes codewords of this shape");
+    int sms = 0;
+    PSB_TRY(check_device(device, &sms));
+    NearTest test;
+    test.items = items; test.gave_up = d_gave_up;
+    return launch_pq_nearest(d_data, n, dim, d_codebook, subvectors, codebook_size, false, d_codes, sms, static_cast<cudaStream_t>(stream), test);
+}
+
 // ---- index-build glue (host) ---------------------------------------------------------------------------------
 
 psb_status psb_ivf_layout_from_assignment(const int* h_assign, int64_t n, int nlist, int64_t* h_offsets, int64_t* h_reordered_ids) {

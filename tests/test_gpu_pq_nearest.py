@@ -102,3 +102,27 @@ def test_encode_tiles_and_items(n, dim, M, K, at):
     got = codes.cpu().numpy()
     assert np.array_equal(got[at:at + n * M].reshape(n, M), oracle.pq_encode(x, cb))
     assert (got[:at] == 99).all() and (got[at + n * M:] == 99).all()
+
+
+@pytest.mark.parametrize("n,dim,M,K,items", [
+    (20000, 64, 16, 256, 0), (20000, 64, 16, 256, 50),      # 108 items, a block each: two turns of three tiles
+    (200000, 64, 16, 256, 0), (200000, 64, 16, 256, 149), (200000, 64, 16, 256, 419),   # 420 items: no product, some or nearly all before the wait
+    (300, 64, 4, 40, 0), (5000, 96, 24, 255, 1), (700, 32, 4, 256, 1)])
+def test_encode_when_a_wait_gives_up(n, dim, M, K, items):
+    """The time-out path: blocks whose items get no products wait for them until the limit; they then wait for the products they have issued,
+    free their tensor memory and evaluate their rows without the filter.  The codes are the same, the device stays usable."""
+    import torch
+    from paraselect_b200 import api
+    rng = np.random.default_rng(n + items)
+    x = rng.standard_normal((n, dim)).astype(np.float32)
+    cb = rng.standard_normal((M, K, dim // M)).astype(np.float32)
+    want = oracle.pq_encode(x, cb)
+    dx, dcb, gave_up = torch.from_numpy(x).cuda(), torch.from_numpy(cb).cuda(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    for few in (items, -1):
+        codes = torch.full((n, M), 99, dtype=torch.uint8, device="cuda")
+        gave_up.zero_()
+        torch.cuda.synchronize()
+        api.pq_encode_limited(dx, n, dim, dcb, M, K, codes, items=few, d_gave_up=gave_up)
+        torch.cuda.synchronize()
+        assert np.array_equal(codes.cpu().numpy(), want)
+        assert (int(gave_up) > 0) == (few >= 0)
