@@ -149,7 +149,7 @@ struct ScanWorkspace {
     unsigned long long* work_cursor_tc = nullptr;
     int* tc_status = nullptr;                    // [1] != 0 after a bounded wait of the tensor-core kernel gave up
     int tc_min_visitors = 0;                     // lists with at least this many visiting queries go to the tensor-core kernel (0 = 1)
-    int tc_wait_limit = 0, tc_skip_mma = 0;      // test hooks of the time-out path
+    int tc_wait_limit = 0, tc_issue_tiles = -1;  // test hooks of the time-out path: polls, tiles of a CTA that get their products (-1: all)
     int pool_cap;
     void* lut_h = nullptr;       // [tables][m*k] fp16 tables (tables = max_batch, x nprobe in residual mode) for the half pre-filter scan (null = fp32 scan only)
     float* lut_scale = nullptr;  // [tables]
@@ -220,7 +220,7 @@ struct ScanTcLaunch {
     const int* vis_count; const int* vis_off; const int* visitors; const long long* item_off;
     const float* thr; int* pool_cnt; uint64_t* pool; int pool_cap;
     unsigned long long* work_cursor; unsigned long long* counters; int* status;
-    int chunk_rows, reserve_ctas, sm_count, wait_limit, skip_mma;
+    int chunk_rows, reserve_ctas, sm_count, wait_limit, issue_tiles;
 };
 psb_status launch_scan_tc(const ScanTcLaunch& L, cudaStream_t s);
 // Selection over pools that may hold unscored survivors of the tensor-core filter (re-scored exactly here).

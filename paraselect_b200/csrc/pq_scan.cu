@@ -1515,7 +1515,7 @@ psb_status launch_scan(const ScanIndex& ix, const ScanWorkspace& ws, const float
         L.lut_div = a.lut_div; L.residual = ix.residual; L.vis_count = ws.vis_count; L.vis_off = ws.vis_off; L.visitors = ws.visitors;
         L.item_off = ws.item_off_tc; L.thr = ws.thr; L.pool_cnt = ws.pool_cnt; L.pool = ws.pool; L.pool_cap = ws.pool_cap;
         L.work_cursor = ws.work_cursor_tc; L.counters = ws.counters; L.status = ws.tc_status; L.chunk_rows = kScanChunkRows;
-        L.reserve_ctas = ws.reserve_ctas; L.sm_count = sm_count; L.wait_limit = ws.tc_wait_limit; L.skip_mma = ws.tc_skip_mma;
+        L.reserve_ctas = ws.reserve_ctas; L.sm_count = sm_count; L.wait_limit = ws.tc_wait_limit; L.issue_tiles = ws.tc_issue_tiles;
         PSB_TRY(launch_scan_tc(L, s));
     }
     if (simt_needed) {

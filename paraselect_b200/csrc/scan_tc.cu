@@ -77,7 +77,7 @@ struct ScanTcArgs {
     float eps;                // accumulation slack e
     int* status;              // != 0 after a bounded wait gave up
     int wait_limit;           // polls before a wait gives up (tests shorten it)
-    int skip_mma;             // test hook: the MMA warp issues nothing, so every role waiting for a result runs into its limit
+    uint32_t issue_tiles;     // tiles of a CTA that get their products: all, or fewer in tests, where the roles that wait for the next run into their limit
 };
 
 // Bounded wait that also leaves when another role of the CTA has given up.
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
     unsigned char* s_b = s_a + g.na * a_bytes;               // [ns][katoms][TN][128 B]
     unsigned char* s_tab = s_b + g.ns * b_bytes;             // [m][k] entries of DSUB bf16: the codebook rounded to bf16
     __shared__ __align__(8) uint64_t item_full[kItemRing], item_empty[kItemRing], vis_full[kItemRing];
-    __shared__ __align__(8) uint64_t a_full[2], a_empty[2], b_full[4], b_empty[4], acc_full[4], acc_empty[4];
+    __shared__ __align__(8) uint64_t a_full[2], a_empty[2], b_full[4], b_empty[4], acc_full[4], acc_empty[4], drained;
     __shared__ ItemDesc s_desc[kItemRing];
     __shared__ float s_P[kItemRing][TV];
     __shared__ int s_pq[kItemRing][TV], s_hi[kItemRing][TV];
@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
             mbar_init(&b_full[i], TN); mbar_init(&b_empty[i], 1);
             mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 128);  // the four warps of one epilogue group
         }
+        mbar_init(&drained, 1);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
                     const long long t1 = clock64();
                     if (!wait_or_abort(&acc_empty[st], (use & 1u) ^ 1u, abort_flag, limit)) { failed = true; break; }
                     w_rows += t1 - t0; w_acc += clock64() - t1;
-                    if (g.skip_mma) continue;  // test hook: nothing is issued or committed, so the waiting roles give up
+                    if (gi >= g.issue_tiles) continue;  // tests: nothing is issued or committed, so the waiting roles give up
                     tc_fence_after();
                     const uint64_t db = st == 0 ? db0 : (st == 1 ? db1 : db2);
                     const uint32_t tacc = tmem + st * TN;
@@ -520,10 +521,14 @@ __global__ void __launch_bounds__(kTcScanThreads, 1) k_scan_tc(const ScanTcArgs 
                     umma_commit(&b_empty[st]);
                 }
                 if (failed) break;
-                if (!g.skip_mma) umma_commit(&a_empty[aslot]);  // the query tile may be rebuilt once these MMAs have read it
+                if (it0 + (uint32_t)ntiles <= g.issue_tiles) umma_commit(&a_empty[aslot]);  // the query tile may be rebuilt once these MMAs have read it
                 it0 += (uint32_t)ntiles;
                 mbar_arrive(&item_empty[islot]);
             }
+            // Whether or not a wait gave up: the products issued are done before the CTA gives back the tensor memory that they write and the operands
+            // that they read.  No other role has a part in this wait, so the flag does not end it.
+            umma_commit(&drained);
+            if (!mbar_wait(&drained, 0)) failed = true;
             // where the issuer's time went (diagnostics, summed over CTAs): waiting for items, decoded rows, accumulators; tiles
             atomicAdd(&a.counters[4], (unsigned long long)w_item);
             atomicAdd(&a.counters[5], (unsigned long long)w_rows);
@@ -681,7 +686,7 @@ psb_status launch_scan_tc(const ScanTcLaunch& L, cudaStream_t s) {
     g.dim = L.dim; g.kp = (L.dim + kAugSlots + 15) / 16 * 16; g.katoms = (g.kp + 63) / 64; g.na = na; g.ns = ns;
     g.residual = L.residual ? 1 : 0;
     g.eps = scan_tc_eps(L.dim);
-    g.status = L.status; g.wait_limit = L.wait_limit > 0 ? L.wait_limit : kWaitLimit; g.skip_mma = L.skip_mma;
+    g.status = L.status; g.wait_limit = L.wait_limit > 0 ? L.wait_limit : kWaitLimit; g.issue_tiles = L.issue_tiles >= 0 ? (uint32_t)L.issue_tiles : 0xffffffffu;
     const unsigned grid = scan_grid(L.sm_count, L.reserve_ctas);
     const int dsub = L.dim / L.m;
     if (dsub == 2) {

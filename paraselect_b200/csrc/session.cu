@@ -625,7 +625,7 @@ struct psb_session {
         w.reserve_ctas = opt.reserve_sms;
         w.seed_sigma = opt.seed_sigma;
         w.item_off_tc = item_off_tc.as<long long>(); w.work_cursor_tc = sc + 11; w.tc_status = reinterpret_cast<int*>(sc + 12);
-        w.tc_min_visitors = opt.tc_min_visitors; w.tc_wait_limit = opt.test_wait_limit; w.tc_skip_mma = opt.test_skip_mma & 1;
+        w.tc_min_visitors = opt.tc_min_visitors; w.tc_wait_limit = opt.test_wait_limit; w.tc_issue_tiles = opt.test_skip_mma & 1 ? 0 : opt.test_skip_mma & 4 ? 3 : -1;
         w.cap_queries = ws_scan_queries; w.cap_tables = ws_scan_tables;
         return w;
     }

@@ -228,15 +228,16 @@ def test_search_with_tc_scan_matches_checker(psb, residual):
     assert np.array_equal(got["indices"], ref["indices"]) and np.array_equal(got["distances"], ref["distances"])
 
 
-def test_tc_scan_bounded_wait_gives_up_cleanly(psb):
-    """The time-out path: with the issuing warp told to skip its tcgen05.mma (nothing is left in flight) every role that
-    waits for a result runs into the shortened poll limit, the kernel frees its tensor memory and returns, and the call
+@pytest.mark.parametrize("skip", [1, 4])   # no products at all, those of a block's first three tiles
+def test_tc_scan_bounded_wait_gives_up_cleanly(psb, skip):
+    """The time-out path: with the issuing warp told to skip its tcgen05.mma every role that waits for a result runs into the
+    shortened poll limit, the kernel waits for the products it has issued, frees its tensor memory and returns, and the call
     reports PSB_TIMEOUT.  The device stays usable: the next session's scan gives the right answer."""
     ix = synth.make_index(9000, 96, 12, 48, seed=41, zipf=True)
     q = synth.make_queries(ix, 64, seed=42)
     probes, _ = oracle.coarse(q, ix["centroids"], 4)
     with pytest.raises(psb.PsbError) as e:
-        run_scan(psb, ix, q, probes, 50, 3, test_skip_mma=1, test_wait_limit=4096)
+        run_scan(psb, ix, q, probes, 50, 3, test_skip_mma=skip, test_wait_limit=4096)
     assert e.value.status == 7
     rows, dist, cnt, _ = run_scan(psb, ix, q, probes, 50, 3)
     orow, odist, ocnt, _ = oracle.pq_scan(q, probes, ix["offsets"], ix["codes"], ix["codebook"], 50)
