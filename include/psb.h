@@ -169,7 +169,7 @@ typedef struct psb_options {
     int tc_min_visitors;/* lists with fewer visiting queries than this stay with the SIMT scan (default 1: none do) */
     /* Test hooks of the time-out paths of the tensor-core kernels (leave 0): test_wait_limit = polls before a device-side wait
        gives up; test_skip_mma bit 0 makes the scan's issuing warp skip its tcgen05.mma (bit 2: those past a block's third tile), bit 1
-       makes the coarse kernel's producer skip its loads - every waiting role then runs into the limit, the kernel waits for what it has
+       makes the coarse kernel's producer skip its loads (bit 3: those past a block's third query tile) - every waiting role then runs into the limit, the kernel waits for what it has
        issued, frees its tensor memory and returns, and the call reports PSB_TIMEOUT. */
     int test_wait_limit;
     int test_skip_mma;

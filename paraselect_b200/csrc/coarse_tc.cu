@@ -94,8 +94,7 @@ struct TcArgs {
     int cand_cap;
     float band;             // pass 2: cut = T + band * E; 2, or 1 when T bounds the exact distance itself (a previous assignment)
     int wait_limit;         // polls before a wait gives up (0: kWaitLimit)
-    int skip_loads;         // test hook of the time-out path: the producer issues no load at all, so nothing is in flight when
-                            // the other roles give up
+    uint32_t load_tiles;    // query tiles a CTA loads before its producer gives up: all, or fewer in the test of the time-out path (0: no load at all)
 };
 
 // Work split: the (centroid block, query tile) pairs are numbered block-major and CTA b takes the contiguous range
@@ -144,7 +143,7 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     const size_t a_bytes = (size_t)a.katoms * TQ * 128, b_bytes = (size_t)a.katoms * TCOL * 128;
     unsigned char* s_a = s_base;                         // [kStagesA][katoms][TQ][128 B]
     unsigned char* s_b = s_base + kStagesA * a_bytes;    // [2][katoms][TCOL][128 B]
-    __shared__ __align__(8) uint64_t a_full[kStagesA], a_empty[kStagesA], b_full, b_empty, acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t a_full[kStagesA], a_empty[kStagesA], b_full, b_empty, acc_full[2], acc_empty[2], drained;
     __shared__ uint32_t s_tmem;
     __shared__ __align__(16) float s_cn2[kBlockCols];
     __shared__ __align__(16) float s_top[kBlockCols / 8];   // the largest s_cn2 of every eight columns
@@ -152,7 +151,7 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
 
     if (tid == 0) {
         for (int i = 0; i < kStagesA; ++i) { mbar_init(&a_full[i], 1); mbar_init(&a_empty[i], 1); }
-        mbar_init(&b_full, 1); mbar_init(&b_empty, 1);
+        mbar_init(&b_full, 1); mbar_init(&b_empty, 1); mbar_init(&drained, 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpiWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -170,9 +169,9 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     int failed = 0;
 
     if (warp == kEpiWarps) {
-        if (lane == 0 && !a.skip_loads) {
+        if (lane == 0 && a.load_tiles) {
             uint32_t it = 0, un = 0;  // query tiles issued, units issued
-            for (; (int)un < nunits && !failed; ++un) {
+            while ((int)un < nunits && !failed) {
                 int cblock, t0, t1;
                 seg_get(a, l0, l1, (int)un, cblock, t0, t1);
                 if (!mbar_wait(&b_empty, (un & 1u) ^ 1u, wl)) { failed = 1; break; }
@@ -180,14 +179,20 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
                 for (int h = 0; h < 2; ++h)
                     for (int ka = 0; ka < a.katoms; ++ka)
                         tma_load_2d(s_b + h * b_bytes + (size_t)ka * TCOL * 128, &map_c, ka * KATOM, cblock * kBlockCols + h * TCOL, &b_full);
+                ++un;
                 for (int t = t0; t < t1; ++t, ++it) {
                     const uint32_t st = it % kStagesA;
-                    if (!mbar_wait(&a_empty[st], ((it / kStagesA) & 1u) ^ 1u, wl)) { failed = 1; break; }
+                    if (it >= a.load_tiles || !mbar_wait(&a_empty[st], ((it / kStagesA) & 1u) ^ 1u, wl)) { failed = 1; break; }
                     mbar_expect_tx(&a_full[st], (uint32_t)a_bytes);
                     for (int ka = 0; ka < a.katoms; ++ka)
                         tma_load_2d(s_a + st * a_bytes + (size_t)ka * TQ * 128, &map_q, ka * KATOM, t * TQ, &a_full[st]);
                 }
             }
+            // Whether or not a wait gave up: the loads issued have landed before the CTA gives back the memory they write to.  (A barrier's phase is
+            // never more than one behind its last load.)
+            if (un && !mbar_wait(&b_full, (un - 1) & 1u)) failed = 1;
+            for (uint32_t st = 0; st < kStagesA; ++st)
+                if (it > st && !mbar_wait(&a_full[st], ((it - st - 1) / kStagesA) & 1u)) failed = 1;
         }
     } else if (warp == kEpiWarps + 1) {
         if (lane == 0) {
@@ -215,6 +220,9 @@ k_coarse_tc(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
                 }
                 umma_commit(&b_empty);
             }
+            // So it is with the products and the tensor memory.
+            umma_commit(&drained);
+            if (!mbar_wait(&drained, 0)) failed = 1;
         }
     } else {
         // epilogue warps
@@ -937,7 +945,7 @@ psb_status plan_tc(const CoarseTcIndex& ix, const CoarseTcWorkspace& ws, int nq,
     a.nprobe = nprobe; a.cn2 = ix.cn2; a.qnorm = static_cast<const float2*>(ws.qnorm); a.cmax = ix.cmax; a.gmin = ws.gmin; a.seltop = ws.seltop;
     a.mwords = coarse_tc_mask_words(ix.nlist); a.status = ws.status;
     a.mask = nullptr; a.cand_cnt = nullptr; a.cand_list = nullptr; a.cand_cap = 0; a.band = 2.0f;
-    a.wait_limit = ws.test_wait_limit; a.skip_loads = ws.test_skip_loads;
+    a.wait_limit = ws.test_wait_limit; a.load_tiles = ws.test_load_tiles >= 0 ? (uint32_t)ws.test_load_tiles : 0xffffffffu;
     a.gmin_q = 1; a.gmin_g = coarse_tc_pitch(nq);
     a.qtiles = (nq + TQ - 1) / TQ;
     a.cblocks = a.ntiles / 2;

@@ -68,7 +68,7 @@ struct CoarseTcWorkspace {
     int* fail_cursor = nullptr;   // null: n_fail + 1
     int* status;     // [1]
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // optional: begin/end of GEMM pass 1 and pass 2
-    int test_wait_limit = 0, test_skip_loads = 0;              // test hooks of the time-out path (0: off)
+    int test_wait_limit = 0, test_load_tiles = -1;             // test hooks of the time-out path: polls (0: the usual), query tiles a CTA loads (-1: all)
 };
 int coarse_tc_padded_dim(int dim);
 int coarse_tc_tiles(int nlist);

@@ -882,7 +882,7 @@ psb_status coarse_exact(psb_session* s, const float* d_queries, int nq, int npro
     if (mode != 1 && tc_ok) {
         PSB_TRY(s->tc_work.ensure(nq, s->nlist, s->dim, nprobe, s->device, s->stream));
         CoarseTcWorkspace tw = s->tc_work.view();
-        tw.test_wait_limit = s->opt.test_wait_limit; tw.test_skip_loads = (s->opt.test_skip_mma & 2) ? 1 : 0;
+        tw.test_wait_limit = s->opt.test_wait_limit; tw.test_load_tiles = s->opt.test_skip_mma & 2 ? 0 : s->opt.test_skip_mma & 8 ? 3 : -1;
         if (s->opt.time_kernels) {
             for (int i = 0; i < 4; ++i) PSB_CUDA(cudaEventCreate(&tw.ev[i]));
             s->gemm_events.emplace_back(tw.ev[0], tw.ev[1]);

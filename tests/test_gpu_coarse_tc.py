@@ -145,22 +145,24 @@ def test_three_call_lloyd_iteration_equals_kmeans_train(psb):
     assert np.mean(assign_a.cpu().numpy() == assign_b.cpu().numpy()) > 0.9999
 
 
-def test_coarse_tc_bounded_wait_gives_up_cleanly(psb):
-    """The time-out path of the coarse kernel: its producer lane told to issue no load at all (nothing is left in flight), the
-    MMA lane and the epilogue warps run into the shortened poll limit, the kernel frees its tensor memory and returns, and the
-    call reports PSB_TIMEOUT.  The device stays usable: the next session's coarse stage gives the right answer."""
+@pytest.mark.parametrize("skip", [2, 8])   # no load at all, those of a block's first three query tiles
+def test_coarse_tc_bounded_wait_gives_up_cleanly(psb, skip):
+    """The time-out path of the coarse kernel: its producer lane told to stop loading, the MMA lane and the epilogue warps run into the
+    shortened poll limit, the kernel waits for the loads and products it has issued, frees its tensor memory and returns, and the call
+    reports PSB_TIMEOUT.  The device stays usable: the next session's coarse stage gives the right answer."""
     import torch
     import synth
     ix = synth.make_index(30000, 64, 2048, 8, seed=71)
-    q = synth.make_queries(ix, 300, seed=72)
-    out = torch.empty((300, 16), dtype=torch.int32, device="cuda")
-    with psb.Session(dict(ix, vectors=None), coarse_mode=2, test_skip_mma=2, test_wait_limit=4096) as s:
-        s.stage_coarse(torch.from_numpy(q).cuda(), 300, 16, out)
+    n = 20000   # a block has four query tiles and more
+    q = synth.make_queries(ix, n, seed=72)
+    out = torch.empty((n, 16), dtype=torch.int32, device="cuda")
+    with psb.Session(dict(ix, vectors=None), coarse_mode=2, max_batch=n, test_skip_mma=skip, test_wait_limit=4096) as s:
+        s.stage_coarse(torch.from_numpy(q).cuda(), n, 16, out)
         with pytest.raises(psb.PsbError) as e:
             s.sync()
         assert e.value.status == 7
-    with psb.Session(dict(ix, vectors=None), coarse_mode=2) as s:
-        s.stage_coarse(torch.from_numpy(q).cuda(), 300, 16, out)
+    with psb.Session(dict(ix, vectors=None), max_batch=n, coarse_mode=2) as s:
+        s.stage_coarse(torch.from_numpy(q).cuda(), n, 16, out)
         s.sync()
-        want, _ = oracle.coarse(q, ix["centroids"], 16)
-        assert np.array_equal(out.cpu().numpy(), want)
+        want, _ = oracle.coarse(q[-500:], ix["centroids"], 16)
+        assert np.array_equal(out[-500:].cpu().numpy(), want)
