@@ -170,7 +170,7 @@ typedef struct psb_options {
     /* Test hooks of the time-out paths of the tensor-core kernels (leave 0): test_wait_limit = polls before a device-side wait
        gives up; test_skip_mma bit 0 makes the scan's issuing warp skip its tcgen05.mma (bit 2: those past a block's third tile), bit 1
        makes the coarse kernel's producer skip its loads (bit 3: those past a block's third query tile) - every waiting role then runs into the limit, the kernel waits for what it has
-       issued, frees its tensor memory and returns, and the call reports PSB_TIMEOUT. */
+       issued, frees its tensor memory and returns, and the call reports PSB_TIMEOUT.  Bit 4 makes a search whose rows are being gathered beside it end with an error. */
     int test_wait_limit;
     int test_skip_mma;
     int zero_copy_pct;  /* PSB_EXACT_HOST_HYBRID: share of each sub-batch gathered by the kernel, 1..100 (0 = 100) */

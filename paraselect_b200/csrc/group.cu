@@ -249,9 +249,10 @@ psb_status group_step(psb_group* g, const float* dq, int nq, int nprobe, int top
             if (rc == PSB_OK) rc = back;
         }
     }
+    // also after an error: what the second stream still does with the session's buffers comes before the main stream's next work
+    const cudaError_t rec = cudaEventRecord(g->ev_back, g->aux), join = rec == cudaSuccess ? cudaStreamWaitEvent(g->main, g->ev_back, 0) : rec;
     PSB_TRY(rc);
-    PSB_CUDA(cudaEventRecord(g->ev_back, g->aux));
-    PSB_CUDA(cudaStreamWaitEvent(g->main, g->ev_back, 0));
+    PSB_CUDA(join);
     // every rank wrote the ids of the rows it holds, -1 elsewhere
     PSB_NCCL(g, all_reduce(d_ids, d_ids, (size_t)nq * topk, kNcclInt64, kNcclMax, g->comm, g->main), "all-reduce of the ids");
     return PSB_OK;

@@ -1097,6 +1097,24 @@ psb_status ensure_zc_stream(psb_session* s) {
     return PSB_OK;
 }
 
+// A call's gathers on zc_stream.  Their results are waited for one by one where rows are scored; a call that ends before that, with an error, leaves
+// gathers that still read the slot lists and write the slots.  Whatever way the call ends, its stream goes on behind them.
+struct Gathers {
+    psb_session* s;
+    cudaStream_t to;
+    bool open = false;   // some may not have been waited for
+    ~Gathers() {
+        if (!open) return;
+        cudaEvent_t e = nullptr;
+        const bool joined = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess && cudaEventRecord(e, s->zc_stream) == cudaSuccess &&
+                            cudaStreamWaitEvent(to, e, 0) == cudaSuccess;
+        if (e) cudaEventDestroy(e);
+        if (!joined) cudaStreamSynchronize(s->zc_stream);
+    }
+};
+// Test hook of that: an error where a call has gathers under way.
+psb_status gather_error(const psb_session* s) { return s->opt.test_skip_mma & 16 ? fail(PSB_INTERNAL, "test hook: an error beside a gather") : PSB_OK; }
+
 // SMs of the gather kernel beside a scan: 16 read ascending rows at the link's rate (8: 51.1 GB/s from an array of 0.8 GB but 40.3 from 20 GB, 16
 // and 32: 51.0 from either), and the scan's persistent grid leaves them free.
 constexpr int kGatherSms = 16;
@@ -1156,19 +1174,23 @@ psb_status rerank_impl(psb_session* s, const void* d_queries, int nq, const int*
             // This thread and the host pool bring their share while the kernel, on a stream of its own, brings the rest.  The call
             // blocks for the host gather; a caller that overlaps it with a scan queues that scan first.
             PSB_TRY(rows_tell_host(s, 0, s->stream));
+            Gathers gathers{s, s->stream};
             if (host_pct < 100) {
                 PSB_TRY(ensure_zc_stream(s));
                 if (!s->zc_ev_a) PSB_CUDA(cudaEventCreateWithFlags(&s->zc_ev_a, cudaEventDisableTiming));
                 if (!s->zc_ev_b) PSB_CUDA(cudaEventCreateWithFlags(&s->zc_ev_b, cudaEventDisableTiming));
                 PSB_CUDA(cudaEventRecord(s->zc_ev_a, s->stream));
                 PSB_CUDA(cudaStreamWaitEvent(s->zc_stream, s->zc_ev_a, 0));
+                gathers.open = true;
                 PSB_TRY(launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, 0), part_end(s, 0), host_pct, s->stage.p,
                                              s->zc_stream, s->sm_count, 0, owned));
                 PSB_CUDA(cudaEventRecord(s->zc_ev_b, s->zc_stream));
             }
             PSB_CUDA(cudaStreamSynchronize(s->stream));
+            PSB_TRY(gather_error(s));
             PSB_TRY(rows_from_host(s, 0, host_pct, s->stream));
             if (host_pct < 100) PSB_CUDA(cudaStreamWaitEvent(s->stream, s->zc_ev_b, 0));
+            gathers.open = false;
         }
     }
     PSB_TRY(score_and_select(s, in_place, d_queries, nq, d_cand, width, stride, d_counts, topk, d_out_rows, d_out_dist, d_out_ids, score, s->stream));
@@ -1776,6 +1798,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         PSB_CUDA(cudaStreamWaitEvent(sx, e0, 0));
     }
     psb_status rc = PSB_OK;
+    Gathers gathers{s, st};
     struct Job { int part, p0, m; cudaEvent_t ready; cudaEvent_t gathered; };
     std::mutex mu;
     std::condition_variable cv;
@@ -1812,6 +1835,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
                 // Hybrid transport: the kernel's share of the slots comes through the gather kernel, which the main thread queued right
                 // behind this sub-batch's claim (j.gathered marks its end); the host threads and the copy engine bring the others; the
                 // scoring waits for both.
+                PSB_TRY(gather_error(s));
                 PSB_TRY(rows_from_host(s, j.part, host_pct, sx));
                 if (j.gathered) PSB_CUDA(cudaStreamWaitEvent(sx, j.gathered, 0));
                 PSB_TRY(score_part(j.p0, j.m));
@@ -1907,10 +1931,12 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
         if (kernel_gather) {   // queued now: the transfer starts the moment the rows are claimed
             if ((rc = event(&gathered)) != PSB_OK) break;
             cudaStreamWaitEvent(s->zc_stream, ready, 0);
+            gathers.open = true;
             rc = launch_gather_unique(s->exact_dev, row_bytes, s->unique.as<int>(), part_begin(s, (int)ci), part_end(s, (int)ci), host_pct, s->stage.p,
                                       s->zc_stream, s->sm_count, s->opt.gather_ctas, gather_sms(s));
             if (rc != PSB_OK) break;
             cudaEventRecord(gathered, s->zc_stream);
+            if (!staged_overlap && (rc = gather_error(s)) != PSB_OK) break;
         }
         if (staged_overlap) {  // the worker takes over: the event marks the slot range ready
             { std::lock_guard<std::mutex> lk(mu); jobs.push_back(Job{(int)ci, p0, m, ready, gathered}); }
@@ -1949,6 +1975,7 @@ psb_status search_device(psb_session* s, const float* dq, const void* dq_exact, 
     }
     finish_worker();
     if (worker_rc != PSB_OK && rc == PSB_OK) rc = fail(worker_rc, "rerank worker: " + worker_msg);
+    if (rc == PSB_OK) gathers.open = false;   // the second stream has waited for each, and the main stream waits for that below
     if (shared_rows && rc == PSB_OK) rc = rows_end(s, sx);
     if (times && (overlap || staged_overlap)) times->last = nullptr;
     if (overlap || staged_overlap) {  // the main stream continues only after the second stream has finished this batch

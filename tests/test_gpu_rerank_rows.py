@@ -119,3 +119,36 @@ def test_slots_in_row_order(psb, mode, count):
             s.sync()
             wi, wd = oracle.rerank(ix["vectors"], q, cand, 10)
             assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
+
+
+@pytest.mark.parametrize("mode,pct,call", [(0, 0, "search"), (4, 90, "search"), (4, 90, "stage")])   # the kernel alone; host threads beside it
+def test_error_beside_a_gather(psb, mode, pct, call):
+    """A call that ends with an error while a kernel on a stream of its own gathers its rows: the session's stream goes on behind the gather, so
+    that the next call, or the owner of its buffers, does not meet it.  The transfer takes 7 ms; nothing is left of it once the stream has drained."""
+    import time
+    import torch
+    n, dim, nq, width = 100000, 1024, 2100, 400
+    ix = index(n, dim, False, 1)
+    q = np.random.default_rng(2).standard_normal((nq, dim)).astype(np.float32)
+    st = torch.cuda.Stream()
+    with psb.Session(ix, n_rerank=width, exact_mode=mode, zero_copy_pct=pct, max_batch=nq, test_skip_mma=16, stream=st.cuda_stream) as s:
+        dq = torch.from_numpy(q).cuda()
+        ids, dist = torch.empty((nq, 10), dtype=torch.int64, device="cuda"), torch.empty((nq, 10), device="cuda")
+        cand = torch.randint(n, (nq, width), dtype=torch.int32, device="cuda")
+        rows = torch.empty((nq, 10), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(2):
+            with pytest.raises(psb.PsbError) as e:
+                if call == "search":
+                    s.search_device(dq, nq, 3, 10, ids, dist)
+                else:
+                    s.stage_rerank(dq, nq, cand, width, width, None, 10, rows, dist)
+            assert e.value.status == 6 and "gather" in str(e.value)
+            st.synchronize()
+            t = time.perf_counter()
+            torch.cuda.synchronize()
+            assert time.perf_counter() - t < 2.5e-3
+    with psb.Session(ix, n_rerank=width, exact_mode=mode, zero_copy_pct=pct, max_batch=nq) as s:   # the rows are mapped anew
+        got = s.search(q, 3, 10, batch_size=nq)
+    want = oracle.ivfpq_search(ix, q[-8:], 3, 10, width)
+    assert np.array_equal(got["indices"][-8:], want["indices"]) and np.array_equal(got["distances"][-8:], want["distances"])
