@@ -97,11 +97,14 @@ __global__ void k_flat_visitors(const int* __restrict__ probes, long long pairs,
     visitors[vis_off[probes[i]] + slot[i]] = (int)i;
 }
 
-// Persistent CTAs over the tiles: (list, 32 of its visitors, 64 of its rows).
+// Persistent CTAs over the tiles: (list, 32 of its visitors, 64 of its rows).  again: only the visitors of the queries it names, of which there are
+// *n_again (null: all); a tile without one costs its look-ups.
 __global__ void __launch_bounds__(kSmallThreads)
 k_flat_tiles(const float* __restrict__ queries, int dim, int nprobe, const long long* __restrict__ offsets, int nlist, const float* __restrict__ rows,
              const int* __restrict__ vis_off, const long long* __restrict__ item_off, const int* __restrict__ visitors, const int* __restrict__ seg,
-             long long stride, float* __restrict__ dist) {
+             long long stride, float* __restrict__ dist, const int* __restrict__ again, const int* __restrict__ n_again) {
+    behind();
+    if (again && *n_again == 0) return;
     extern __shared__ __align__(16) float s_flat[];
     __shared__ int s_list, s_pair[SQ];
     __shared__ long long s_dst[SQ];
@@ -122,21 +125,26 @@ k_flat_tiles(const float* __restrict__ queries, int dim, int nprobe, const long 
         const int g = (int)(local % groups);
         const long long r0 = local / groups * SC, len = offsets[l + 1] - offsets[l];
         const int nv = min(SQ, nvis - g * SQ), nr = (int)min((long long)SC, len - r0);
+        bool live = false;
         if (threadIdx.x < SQ) {
-            const int pair = threadIdx.x < nv ? visitors[v0 + g * SQ + threadIdx.x] : -1;
+            int pair = threadIdx.x < nv ? visitors[v0 + g * SQ + threadIdx.x] : -1;
+            const int q = pair >= 0 ? pair / nprobe : 0;
+            if (again && pair >= 0 && !again[q]) pair = -1;
+            live = pair >= 0;
             s_pair[threadIdx.x] = pair;
-            if (pair >= 0) { const int q = pair / nprobe; s_dst[threadIdx.x] = (long long)q * stride + seg[(size_t)q * (nprobe + 1) + (pair - q * nprobe)] + r0; }
+            if (live) s_dst[threadIdx.x] = (long long)q * stride + seg[(size_t)q * (nprobe + 1) + (pair - q * nprobe)] + r0;
         }
+        if (again && !__syncthreads_or(live)) continue;
         stage_rows<kSmallThreads>(cs, pitch, rows + (size_t)(offsets[l] + r0) * dim, nr, dim);
         __syncthreads();
-        for (int i = warp; i < nv; i += kSmallThreads / 32) stage_row(qs + i * pitch, queries + (size_t)(s_pair[i] / nprobe) * dim, dim, vec, lane);
+        for (int i = warp; i < nv; i += kSmallThreads / 32) if (s_pair[i] >= 0) stage_row(qs + i * pitch, queries + (size_t)(s_pair[i] / nprobe) * dim, dim, vec, lane);
         stage_wait();
-        if (ty * 4 < nv) {
+        if ((s_pair[ty * 4] & s_pair[ty * 4 + 1] & s_pair[ty * 4 + 2] & s_pair[ty * 4 + 3]) >= 0) {   // one of the four visitors is wanted
             float acc[4][4];
             tile_distances(qs + ty * 4 * pitch, cs + tx * pitch, pitch, dim, acc);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                if (ty * 4 + i >= nv) continue;
+                if (s_pair[ty * 4 + i] < 0) continue;
                 float* out = dist + s_dst[ty * 4 + i];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) if (tx + 16 * j < nr) out[tx + 16 * j] = acc[i][j];
@@ -172,16 +180,17 @@ k_flat_rows(const float* __restrict__ queries, int dim, const int* __restrict__ 
     }
 }
 
-// One CTA per query: the topk nearest of its distances, ties by row; original ids out.
+// One CTA per query: the topk nearest of its distances, ties by row; original ids out.  again: of the queries it names (null: of all).
 template <int T>
 __global__ void __launch_bounds__(T)
 k_flat_select(const float* __restrict__ dist, long long stride, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
               const int* __restrict__ seg, int topk, int buffer, const long long* __restrict__ ids, long long* __restrict__ out_ids,
-              float* __restrict__ out_dist, const float* __restrict__ runs, long long run_stride) {
+              float* __restrict__ out_dist, const float* __restrict__ runs, long long run_stride, const int* __restrict__ again) {
     extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the selection's runs, the segments (where they fit)
     __shared__ sel::Words w;
     behind();
     const int q = blockIdx.x;
+    if (again && !again[q]) return;
     const int* s = seg + (size_t)q * (nprobe + 1);
     if (nprobe <= sel::kSegShared) {   // a search for every key: not in global memory
         int* s_seg = reinterpret_cast<int*>(s_key + buffer) + sel::kMaxGroups;
@@ -210,16 +219,25 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
 // than topk - are evaluated exactly.  (tcgen05 wants 128 visitors a tile; a list has sixty in the benchmark's configuration, and often ten.)
 // Bound: latency, a tile being a chain of look-ups, two stagings and a short product; four CTAs an SM.  1,000 queries x 16 lists of 390 rows x 128,
 // topk 10: tiles 163 -> 72 us, selection 14 -> 29, the whole call 244 -> 150.  Eight warps a tile 91, four rows' loads at a time 78.
-//   Error of an approximate distance against the exact arithmetic's, S = (|q| + max|x|)^2:  products, splits 3.1 * 2^-18 and 3 K additions of
-//   2^-22 each, of |q||x| <= S / 4, twice; norms (K + 4) 2^-24 S; their sum 2^-22 S; the exact arithmetic's own (K + 2) 2^-23 S; where products are
-//   subnormal, below 1e-35.  A row within twice that of the topk-th smallest approximate distance may be among the topk.
+//   Error of an approximate distance against the exact arithmetic's, S = (|q| + |x|)^2 <= 2 (|q|^2 + |x|^2):  products, splits 3.1 * 2^-18 and 3 K
+//   additions of 2^-22 each, of |q||x| <= S / 4, twice; norms (K + 4) 2^-24 S; their sum 2^-22 S; the exact arithmetic's own (K + 2) 2^-23 S; where
+//   products are subnormal, below 1e-35.  Together e = slack (|q|^2 + |x|^2) + 1e-35, and the tiles leave the lower bound, approximation - e.
+//   The topk rows of the smallest lower bounds, t at most, lie within t + 2 e: of all rows in the visited lists |x|^2 is at most `most`, and of rows
+//   with |x| >= 3 |q| the lower bound is at least ((2/3)^2 - 2 * 10/9 slack) |x|^2 >= 0.4 |x|^2, so that |x|^2 <= max(9 |q|^2, 2.5 t) for the topk: one row far
+//   out does not loosen the bound for the others.  Only rows whose lower bound is below that can be among the topk.
+//   A row whose norm is too large for a bound, or not a number, is evaluated for every query that visits its list.
+// Where more than 1,024 rows are left - all rows far from the origin, or equally near by the thousand - the bound is no help: such queries are noted, and
+// two more launches, which leave at once where there are none, take them through the exact tiles.  1,000 queries x 16 lists of 390 rows x 128, us: exact tiles
+// for all
+// 227, behind the filter 131; one row of 1,000 times the norm, or not a number, 131; an offset of 100 with a spread of 0.3 301; all rows the same 488 (exact
+// tiles 376).  With one norm for the whole index and the way back in the selection's own block these were 926, 917 and 1,237.
 constexpr int kFilterThreads = 128;   // four warps: 16 visitors x 32 rows each
 __host__ __device__ __forceinline__ int filter_dims(int dim) { return (dim + 15) / 16 * 16; }
 __host__ __device__ __forceinline__ int filter_pitch(int dim) { return filter_dims(dim) + 8; }   // bf16 between rows: eight rows' 16 bytes in different banks
 inline size_t filter_bytes(int dim) { return (size_t)(SQ + SC) * filter_pitch(dim) * 4; }
-__device__ __forceinline__ float filter_slack(float qn, float xmax2, int dim) {
-    const float s = sqrtf(qn) + sqrtf(xmax2), k = (float)filter_dims(dim);
-    return 2.0f * (s * s * 1.0001f * (5.913e-6f + k * (3.577e-7f + 5.97e-8f + 1.193e-7f) + 1.0e-6f) + 1.0e-35f);
+__device__ __forceinline__ float filter_slack(int dim) {   // <= 3.2e-4: operands of 256 dimensions at most
+    const float k = (float)filter_dims(dim);
+    return 2.0002f * (5.913e-6f + k * (3.577e-7f + 5.97e-8f + 1.193e-7f) + 1.0e-6f);
 }
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -230,11 +248,22 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Squared norms of the rows, and the largest as the bits of a float (not a number: the largest of all).  A warp per row.
-__global__ void __launch_bounds__(256) k_flat_norms(const float* __restrict__ rows, long long n, int dim, float* __restrict__ norms, unsigned* __restrict__ most) {
+// Squared norms of the rows, and the largest of each list as the bits of a float (not a number: the largest of all).  A warp takes `per` rows, one
+// after the other.
+__global__ void __launch_bounds__(256) k_flat_norms(const float* __restrict__ rows, long long n, int dim, const long long* __restrict__ offsets, int nlist,
+                                                    int per, float* __restrict__ norms, unsigned* __restrict__ most) {
     const int lane = threadIdx.x & 31;
+    const long long r0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * per, r1 = min(n, r0 + per);
+    if (r0 >= r1) return;
+    int l = scan::find_list(offsets, nlist, r0);
+    long long end = offsets[l + 1];
     unsigned top = 0;
-    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < n; r += (long long)gridDim.x * 8) {
+    for (long long r = r0; r < r1; ++r) {
+        if (r >= end) {
+            if (lane == 0 && top) atomicMax(&most[l], top);
+            top = 0;
+            while (r >= end) end = offsets[++l + 1];
+        }
         float s = 0.0f;
         for (int d = lane; d < dim; d += 32) { const float v = rows[(size_t)r * dim + d]; s = fmaf(v, v, s); }
 #pragma unroll
@@ -242,7 +271,7 @@ __global__ void __launch_bounds__(256) k_flat_norms(const float* __restrict__ ro
         if (lane == 0) norms[r] = s;
         top = max(top, __float_as_uint(s) & 0x7fffffffu);
     }
-    if (lane == 0 && top) atomicMax(most, top);
+    if (lane == 0 && top) atomicMax(&most[l], top);
 }
 
 __global__ void __launch_bounds__(kFilterThreads)
@@ -260,6 +289,8 @@ k_flat_tiles_filter(const float* __restrict__ queries, int dim, int nprobe, cons
     __nv_bfloat16* xl = xh + SC * pitch;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long total = item_off[nlist];
+    const float less = 1.0f - filter_slack(dim), none = __int_as_float(0x7fffffff);
+    auto lower = [&](float dot, float norms2) { return norms2 < 1.0e36f ? fmaf(-2.0f, dot, fmaf(norms2, less, -1.0e-35f)) : none; };
     // One row by a warp, four elements a lane, several rows' loads before the first is used: two bf16 terms of each, and the squares' sum.
     auto stage = [&](auto src_of, int count, __nv_bfloat16* high, __nv_bfloat16* low, bool vec, auto sum_of) {
         constexpr int U = 8;
@@ -358,26 +389,32 @@ k_flat_tiles_filter(const float* __restrict__ queries, int dim, int nprobe, cons
                 if (v >= nv) continue;
                 float* out = dist + s_dst[v] + c;
                 const float qn = s_qn[v];
-                if (c < nr) out[0] = fmaf(-2.0f, acc[t][h * 2], qn + x0);
-                if (c + 1 < nr) out[1] = fmaf(-2.0f, acc[t][h * 2 + 1], qn + x1);
+                if (c < nr) out[0] = lower(acc[t][h * 2], qn + x0);
+                if (c + 1 < nr) out[1] = lower(acc[t][h * 2 + 1], qn + x1);
             }
         }
     }
 }
 
-// One CTA per query: the topk nearest of its approximate distances' candidates, evaluated exactly; ties by row; original ids out.  A query whose
-// bound does not hold (values out of range, too many rows within it) has all its distances computed and selected from.
+// One CTA per query: the topk nearest of the rows that their lower bounds do not rule out, evaluated exactly; ties by row; original ids out.  A query
+// with too many of them is noted in `again` and counted, and left.
 template <int T>
 __global__ void __launch_bounds__(T)
-k_flat_select_filter(float* __restrict__ dist, long long stride, const float* __restrict__ queries, int dim, const float* __restrict__ rows,
-                     const unsigned* __restrict__ most, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets,
+k_flat_select_filter(const float* __restrict__ dist, long long stride, const float* __restrict__ queries, int dim, const float* __restrict__ rows,
+                     const unsigned* __restrict__ most, const int* __restrict__ probes, int nprobe, const long long* __restrict__ offsets, int nlist,
                      const int* __restrict__ seg, int topk, int buffer, const long long* __restrict__ ids, long long* __restrict__ out_ids,
-                     float* __restrict__ out_dist) {
-    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the selection's runs, the query, the segments (where they fit)
+                     float* __restrict__ out_dist, int* __restrict__ again, int* __restrict__ n_again) {
+    extern __shared__ __align__(16) uint64_t s_key[];   // [buffer] keys, the query, the segments (where they fit)
     __shared__ sel::Words w;
-    int* s_runs = reinterpret_cast<int*>(s_key + buffer);
-    float* s_q = reinterpret_cast<float*>(s_runs + sel::kMaxGroups);
+    behind();
+    float* s_q = reinterpret_cast<float*>(s_key + buffer);
     const int q = blockIdx.x, lane = threadIdx.x & 31;
+    unsigned top = 0;   // the largest norm in the lists the query visits; the same in every warp
+    for (int p = lane; p < nprobe; p += 32) {
+        const int l = probes[(size_t)q * nprobe + p];
+        if (l >= 0 && l < nlist) top = max(top, most[l]);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
     const int* s = seg + (size_t)q * (nprobe + 1);
     for (int d = threadIdx.x; d < dim; d += T) s_q[d] = queries[(size_t)q * dim + d];
     if (nprobe <= sel::kSegShared) {
@@ -393,58 +430,53 @@ k_flat_select_filter(float* __restrict__ dist, long long stride, const float* __
         return (uint32_t)(offsets[probes[(size_t)q * nprobe + lo]] + (i - s[lo]));
     };
     const bool vec = rows_vec(rows, dim);
-    float* vals = dist + (size_t)q * stride;
+    const float* vals = dist + (size_t)q * stride;
     const int n = s[nprobe];
-    int keep = min(topk, n);
+    const int keep = min(topk, n);
     float qn = 0.0f;
     for (int d = lane; d < dim; d += 32) qn = fmaf(s_q[d], s_q[d], qn);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) qn += __shfl_xor_sync(0xffffffffu, qn, o);   // the same in every warp
-    const float inf = __int_as_float(0x7f800000), slack = filter_slack(qn, __uint_as_float(*most), dim);
-    bool sure = slack < 1.0e37f;
-    if (sure) {
-        float cut = inf;
-        if (n > 4 * topk && n >= 96) {   // as sel::smallest does
-            float* s_min = reinterpret_cast<float*>(s_key);
-            const int per = (2 * topk + T - 1) / T;
-            for (int g = 0; g < per; ++g) {
-                float m = inf;
+    const float inf = __int_as_float(0x7f800000);
+    float cut = inf;
+    if (n > 4 * topk && n >= 96) {   // as sel::smallest does
+        float* s_min = reinterpret_cast<float*>(s_key);
+        const int per = (2 * topk + T - 1) / T;
+        for (int g = 0; g < per; ++g) {
+            float m = inf;
 #pragma unroll 8
-                for (int i = threadIdx.x + g * T; i < n; i += per * T) m = fminf(m, vals[i]);
-                s_min[g * T + threadIdx.x] = m;
-            }
-            __syncthreads();
-            if (threadIdx.x < 32) {
-                const float at = per == 1 ? sel::bound_of<T / 32>(s_min, T, topk) : sel::bound_of<0>(s_min, per * T, topk);
-                if (lane == 0) w.cut = at;
-            }
-            __syncthreads();
-            cut = w.cut + slack;
+            for (int i = threadIdx.x + g * T; i < n; i += per * T) m = fminf(m, vals[i]);
+            s_min[g * T + threadIdx.x] = m;
         }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const float at = per == 1 ? sel::bound_of<T / 32>(s_min, T, topk) : sel::bound_of<0>(s_min, per * T, topk);
+            if (lane == 0) w.cut = at;
+        }
+        __syncthreads();
+        const float t = w.cut;
+        cut = fmaf(2.0002f * filter_slack(dim), qn + fminf(__uint_as_float(top), fmaxf(9.0f * qn, 2.5f * t)), fmaf(fabsf(t), 1.0e-6f, t)) + 4.0e-35f;
+    }
 #pragma unroll 8
-        for (int i = threadIdx.x; i < n; i += T)
-            if (cut == inf || vals[i] <= cut) {
-                const int pos = atomicAdd(&w.cnt, 1);
-                if (pos < buffer) s_key[pos] = (uint64_t)i;
-            }
-        __syncthreads();
-        const int c = w.cnt;
-        sure = c >= keep && c <= buffer;
-        if (sure) {
-            for (int e = threadIdx.x; e < c; e += T) {
-                const uint32_t r = row_of((int)s_key[e]);
-                s_key[e] = make_key(row_distance(s_q, rows + (size_t)r * dim, dim, vec), r);
-            }
-            __syncthreads();
-            sel::put_in_order<T>(s_key, c, topk);
+    for (int i = threadIdx.x; i < n; i += T)
+        if (!(vals[i] > cut)) {   // not a number: no bound
+            const int pos = atomicAdd(&w.cnt, 1);
+            if (pos < buffer) s_key[pos] = (uint64_t)i;
         }
+    __syncthreads();
+    const int c = w.cnt;
+    const bool sure = c >= keep && c <= buffer;
+    if (threadIdx.x == 0) {
+        again[q] = sure ? 0 : 1;
+        if (!sure) atomicAdd(n_again, 1);
     }
-    if (!sure) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += T) vals[i] = row_distance(s_q, rows + (size_t)row_of(i) * dim, dim, vec);
-        __syncthreads();
-        keep = sel::smallest<T>(vals, n, topk, row_of, s_key, buffer, s_runs, &w);
+    if (!sure) return;
+    for (int e = threadIdx.x; e < c; e += T) {
+        const uint32_t r = row_of((int)s_key[e]);
+        s_key[e] = make_key(row_distance(s_q, rows + (size_t)r * dim, dim, vec), r);
     }
+    __syncthreads();
+    sel::put_in_order<T>(s_key, c, topk);
     for (int i = threadIdx.x; i < topk; i += T) {
         const bool ok = i < keep;
         out_ids[(size_t)q * topk + i] = ok ? ids[key_idx(s_key[i])] : -1;
@@ -475,10 +507,11 @@ bool flat_list_form(int nq, int nprobe, int nlist, long long rows, int dim) {
 // The list form's tiles from the filter: its operands fit, and the selection's buffer holds topk and what the slack lets through.
 bool flat_filter_form(int dim, int topk) { return topk <= 256 && filter_bytes(dim) <= (size_t)100 * 1024; }
 
-psb_status launch_flat_norms(const float* d_rows, long long n, int dim, float* d_norms, unsigned* d_most, cudaStream_t s) {
-    PSB_CUDA(cudaMemsetAsync(d_most, 0, sizeof(unsigned), s));
+psb_status launch_flat_norms(const float* d_rows, long long n, int dim, const long long* d_offsets, int nlist, float* d_norms, unsigned* d_most, cudaStream_t s) {
+    PSB_CUDA(cudaMemsetAsync(d_most, 0, sizeof(unsigned) * (size_t)nlist, s));
     if (n <= 0) return PSB_OK;
-    k_flat_norms<<<(unsigned)std::min<long long>((n + 7) / 8, 4096), 256, 0, s>>>(d_rows, n, dim, d_norms, d_most);
+    const int per = (int)((n + 32767) / 32768);
+    k_flat_norms<<<(unsigned)((n + 8ll * per - 1) / (8ll * per)), 256, 0, s>>>(d_rows, n, dim, d_offsets, nlist, per, d_norms, d_most);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;
@@ -488,8 +521,10 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     if (nq <= 0) return PSB_OK;
     if (f.topk <= 0 || f.topk > kMaxTopk) return fail(PSB_UNSUPPORTED_SHAPE, "flat scan supports topk in 1..2048");
     const bool lists = flat_list_form(nq, f.nprobe, f.nlist, f.n_rows, f.dim);
+    bool filtered = false;   // the exact tiles and the selection take the queries for which the filter's bound did not hold
     const long long pairs = (long long)nq * f.nprobe;
-    if (lists) PSB_CUDA(cudaMemsetAsync(f.vis_count, 0, sizeof(int) * (size_t)f.nlist, s));
+    int* n_again = lists ? f.vis_count + f.nlist : nullptr;
+    if (lists) PSB_CUDA(cudaMemsetAsync(f.vis_count, 0, sizeof(int) * ((size_t)f.nlist + 1), s));
     PSB_TRY(launch_row_segments(f.probes, nq, f.nprobe, f.offsets, 0, f.nlist, f.seg, f.vis_count, lists ? f.slot : nullptr, f.counters, s, true));
     if (lists) {
         k_flat_lists<<<1, 1024, 0, s>>>(f.vis_count, f.offsets, f.nlist, f.vis_off, f.item_off);
@@ -498,7 +533,8 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
         k_flat_visitors<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(f.probes, pairs, f.slot, f.vis_off, f.visitors);
         count_launch();
         PSB_LAUNCH_CHECK();
-        if (flat_filter_form(f.dim, f.topk)) {
+        filtered = flat_filter_form(f.dim, f.topk);
+        if (filtered) {
             const size_t smem = filter_bytes(f.dim);
             PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_tiles_filter), smem));
             const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)220 * 1024 / (smem + 2048)));
@@ -506,24 +542,22 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
                                                                                               f.vis_off, f.item_off, f.visitors, f.seg, f.stride, f.dist);
             count_launch();
             PSB_LAUNCH_CHECK();
-            const size_t keys = sel::shared_bytes(f.topk) + (size_t)((f.dim + 3) & ~3) * 4 + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
+            const size_t keys = (size_t)sel::buffer_entries(f.topk) * 8 + (size_t)((f.dim + 3) & ~3) * 4 + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
             auto select = [&](auto kernel, int threads) -> psb_status {
                 PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), keys));
-                kernel<<<nq, threads, keys, s>>>(f.dist, f.stride, f.queries, f.dim, f.rows, f.most, f.probes, f.nprobe, f.offsets, f.seg, f.topk,
-                                                 sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist);
-                return PSB_OK;
+                return launch_behind(true, kernel, dim3((unsigned)nq), (unsigned)threads, keys, s, f.dist, f.stride, f.queries, f.dim, f.rows, f.most, f.probes, f.nprobe, f.offsets,
+                                     f.nlist, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist, f.again, n_again);
             };
             if (nq <= f.sm_count) PSB_TRY(select(k_flat_select_filter<1024>, 1024));
             else PSB_TRY(select(k_flat_select_filter<256>, 256));
             count_launch();
             PSB_LAUNCH_CHECK();
-            return PSB_OK;
         }
         const size_t smem = small_tile_bytes(f.dim);
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_tiles), smem));
         const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)220 * 1024 / (smem + 1024)));
-        k_flat_tiles<<<(unsigned)(f.sm_count * per_sm), kSmallThreads, smem, s>>>(f.queries, f.dim, f.nprobe, f.offsets, f.nlist, f.rows, f.vis_off,
-                                                                                  f.item_off, f.visitors, f.seg, f.stride, f.dist);
+        PSB_TRY(launch_behind(true, k_flat_tiles, dim3((unsigned)(f.sm_count * per_sm)), kSmallThreads, smem, s, f.queries, f.dim, f.nprobe, f.offsets, f.nlist, f.rows, f.vis_off,
+                              f.item_off, f.visitors, f.seg, f.stride, f.dist, filtered ? f.again : nullptr, n_again));
     } else {
         const long long blocks = std::min<long long>((f.stride + 127) / 128, 8192);
         const size_t smem = (size_t)((f.dim + 3) & ~3) * sizeof(float);
@@ -535,7 +569,8 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
     const size_t smem = sel::shared_bytes(f.topk) + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
     auto select = [&](auto kernel, int threads) -> psb_status {   // fewer queries than SMs: large blocks
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
-        return launch_behind(true, kernel, dim3((unsigned)nq), (unsigned)threads, smem, s, f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist, lists ? nullptr : f.runs, f.run_stride);
+        return launch_behind(true, kernel, dim3((unsigned)nq), (unsigned)threads, smem, s, f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist, lists ? nullptr : f.runs, f.run_stride,
+                             filtered ? f.again : nullptr);
     };
     if (nq <= f.sm_count) PSB_TRY(select(k_flat_select<1024>, 1024));
     else PSB_TRY(select(k_flat_select<256>, 256));

@@ -299,20 +299,20 @@ struct FlatScan {
     const long long* offsets; int nlist;        // [nlist + 1]
     long long n_rows;                          // of all lists
     const float* rows; const long long* ids;   // [n][dim], [n]
-    const float* norms; const unsigned* most;  // squared norms of the rows and the largest's bits (launch_flat_norms)
+    const float* norms; const unsigned* most;  // squared norms of the rows and each list's largest's bits (launch_flat_norms)
     int topk;
     long long* out_ids; float* out_dist;       // [nq][topk]
     float* dist; long long stride;             // [nq][stride] workspace, stride >= the rows of any nprobe lists
     float* runs; long long run_stride;         // [nq][run_stride] workspace of the row form: the minimum of every 32 distances
     int* seg;                                  // [nq][nprobe + 1]
-    // list form only (flat_list_form): [nlist], [nq * nprobe], [nlist + 1], [nlist + 1], [nq * nprobe]
-    int* vis_count; int* slot; int* vis_off; long long* item_off; int* visitors;
+    // list form only (flat_list_form): [nlist + 1], [nq * nprobe], [nlist + 1], [nlist + 1], [nq * nprobe], [nq]
+    int* vis_count; int* slot; int* vis_off; long long* item_off; int* visitors; int* again;
     unsigned long long* counters;
     int sm_count;
 };
 bool flat_list_form(int nq, int nprobe, int nlist, long long rows, int dim);   // rows: of all lists
 psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s);
-psb_status launch_flat_norms(const float* d_rows, long long n, int dim, float* d_norms, unsigned* d_most, cudaStream_t s);
+psb_status launch_flat_norms(const float* d_rows, long long n, int dim, const long long* d_offsets, int nlist, float* d_norms, unsigned* d_most, cudaStream_t s);
 
 // ---- rerank ------------------------------------------------------------------------------------------------
 // Which rows of the index-wide (list-contiguous) numbering a session's exact store and id table hold.

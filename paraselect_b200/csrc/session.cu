@@ -494,7 +494,7 @@ struct psb_session {
     DevBuf opq, q_rot;                     // OPQ rotation [dim][dim] and the rotated queries of the batch in flight
     bool row_bias_is_u16 = false;          // row_bias holds the caller's affine u16 row correction
     bool flat = false;                     // IVF-Flat session: exact rows resident in flat_rows, no PQ parts
-    DevBuf flat_rows, flat_slot, flat_norms;   // norms: of every row, then the largest
+    DevBuf flat_rows, flat_slot, flat_norms, flat_again;   // norms: of every row, then the largest of each list
     EventPool timing, timing_aux;          // events of the main stream's marks and of the second stream's (set from one thread each)
     // Host side of a search call: one pinned block through which a small batch's queries and results pass, and the device's counters
     // and status words with the results, so that a call waits for the GPU once.
@@ -2170,8 +2170,9 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
         PSB_CUDA(cudaMemcpyAsync(s->flat_rows.p, index->rowmajor_fp32, sizeof(float) * n * s->dim, cudaMemcpyHostToDevice, st));
     }
     note_list_lengths(s.get(), index->lists.offsets);
-    PSB_TRY(s->flat_norms.reserve(sizeof(float) * (n + 1)));
-    PSB_TRY(launch_flat_norms(s->flat_rows.as<float>(), s->n_vectors, s->dim, s->flat_norms.as<float>(), s->flat_norms.as<unsigned>() + n, st));
+    PSB_TRY(s->flat_norms.reserve(sizeof(float) * (n + nl)));
+    PSB_TRY(launch_flat_norms(s->flat_rows.as<float>(), s->n_vectors, s->dim, s->offsets.as<long long>(), s->nlist, s->flat_norms.as<float>(),
+                              s->flat_norms.as<unsigned>() + n, st));
     PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
     PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, st));
     PSB_CUDA(cudaStreamSynchronize(st));
@@ -2205,7 +2206,8 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     PSB_TRY(reserve_together(&s->row_whole, {{&s->row_dist, sizeof(float) * (size_t)per * f.stride}, {&s->row_seg, sizeof(int) * (size_t)per * ((size_t)nprobe + 1)},
                                              {&s->row_runs, sizeof(float) * (size_t)per * f.run_stride}}));
     if (flat_list_form(per, nprobe, s->nlist, s->n_vectors, s->dim)) {
-        PSB_TRY(s->vis_count.reserve(sizeof(int) * (size_t)s->nlist));
+        PSB_TRY(s->vis_count.reserve(sizeof(int) * ((size_t)s->nlist + 1)));
+        PSB_TRY(s->flat_again.reserve(sizeof(int) * (size_t)per));
         PSB_TRY(s->flat_slot.reserve(sizeof(int) * (size_t)per * nprobe));
         PSB_TRY(s->vis_off.reserve(sizeof(int) * ((size_t)s->nlist + 1)));
         PSB_TRY(s->item_off.reserve(sizeof(long long) * ((size_t)s->nlist + 1)));
@@ -2215,7 +2217,7 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     f.norms = s->flat_norms.as<float>(); f.most = s->flat_norms.as<unsigned>() + std::max<long long>(1, s->n_vectors);
     f.ids = s->reordered.as<long long>(); f.topk = topk; f.dist = s->row_dist.as<float>(); f.seg = s->row_seg.as<int>();
     f.vis_count = s->vis_count.as<int>(); f.slot = s->flat_slot.as<int>(); f.vis_off = s->vis_off.as<int>(); f.item_off = s->item_off.as<long long>();
-    f.visitors = s->visitors.as<int>(); f.counters = s->scalars.as<unsigned long long>(); f.sm_count = s->sm_count;
+    f.visitors = s->visitors.as<int>(); f.again = s->flat_again.as<int>(); f.counters = s->scalars.as<unsigned long long>(); f.sm_count = s->sm_count;
     for (int q0 = 0; q0 < n; q0 += per) {
         f.queries = dq + (size_t)q0 * s->dim; f.probes = s->probes.as<int>() + (size_t)q0 * nprobe;
         f.out_ids = d_ids + (size_t)q0 * topk; f.out_dist = d_dist + (size_t)q0 * topk;

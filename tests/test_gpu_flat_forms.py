@@ -62,11 +62,12 @@ def test_flat_list_form_and_parts(psb, n, dim, nlist, nq, nprobe, topk, values):
 
 
 @pytest.mark.parametrize("dim", [5, 16, 100, 128, 130, 240])
-@pytest.mark.parametrize("kind", ["normal", "far", "tiny", "grid", "odd"])
+@pytest.mark.parametrize("kind", ["normal", "far", "tiny", "grid", "odd", "one", "spread", "crowd", "large"])
 @pytest.mark.parametrize("k", [1, 10, 256])
 def test_list_form_behind_the_filter(psb, dim, kind, k):
     """Approximate distances and exact evaluation of the candidates: a large offset, which loosens the bound; values whose squares vanish, equal
-    distances by the hundred and values that are not finite, for which a query's distances are all computed."""
+    distances by the hundred and values that are not finite; a row and rows of many times the others' norm; a list of equal rows, whose visitors
+    alone go back to the exact tiles; norms on both sides of the largest that a bound is given for."""
     rng = np.random.default_rng(dim + k)
     nlist, n, nq, nprobe = 6, 9000, 700, 3
     cen = rng.standard_normal((nlist, dim)).astype(np.float32)
@@ -80,6 +81,15 @@ def test_list_form_behind_the_filter(psb, dim, kind, k):
         x, q, cen = (v * np.float32(1e-20) for v in (x, q, cen))
     if kind == "grid":
         x, q = np.round(x), np.round(q)
+    if kind == "one":
+        x[2000] *= 1000
+    if kind == "spread":
+        x[::3] *= np.exp(rng.uniform(-7, 7, (len(x[::3]), 1))).astype(np.float32)
+    if kind == "crowd":
+        x[1400:5000] = cen[4]
+    if kind == "large":
+        x, q, cen = (v * np.float32(4e17 / np.sqrt(dim)) for v in (x, q, cen))
+        x[::2] *= 3
     if kind == "odd":
         x[4000, 0], x[77, dim - 1], q[3, 1] = np.inf, np.nan, np.inf
     ix = dict(centroids=cen, offsets=off, reordered_ids=rng.permutation(n).astype(np.int64), vectors=x)
@@ -99,3 +109,42 @@ def test_list_form_behind_the_filter(psb, dim, kind, k):
         take = np.isfinite(d[order])
         assert np.array_equal(got["indices"][i][: len(order)][take], ix["reordered_ids"][rows[order]][take]), (kind, i)
         assert np.array_equal(got["distances"][i][: len(order)][take], d[order][take])
+
+
+@pytest.mark.parametrize("kind,times", [("one", 2.0), ("nan", 2.0), ("far", 4.0), ("same", 6.0)])   # measured 1.0, 1.0, 2.3, 3.7
+def test_cost_where_the_bound_is_loose(psb, kind, times):
+    """Rows that loosen the filter's bound cost the queries that it cannot serve the exact tiles, and the others nothing."""
+    import torch
+    rng = np.random.default_rng(1)
+    n, dim, nlist, nq = 100000, 128, 256, 1000
+    cen = rng.standard_normal((nlist, dim)).astype(np.float32)
+    own = np.sort(rng.integers(0, nlist, n))
+    off = np.concatenate([[0], np.cumsum(np.bincount(own, minlength=nlist))]).astype(np.int64)
+    x = (cen[own] + 0.3 * rng.standard_normal((n, dim))).astype(np.float32)
+    q = (cen[rng.integers(0, nlist, nq)] + 0.3 * rng.standard_normal((nq, dim))).astype(np.float32)
+
+    def cost(x, q, cen):
+        st = torch.cuda.Stream()
+        with psb.FlatSession(dict(centroids=cen, offsets=off, reordered_ids=np.arange(n), vectors=x), max_batch=nq, stream=st.cuda_stream) as s:
+            dq, ids, dist = torch.from_numpy(q).cuda(), torch.empty(nq, 10, dtype=torch.int64, device="cuda"), torch.empty(nq, 10, device="cuda")
+            torch.cuda.synchronize()
+            ms = []
+            for _ in range(9):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record(st)
+                for _ in range(4):
+                    s.search_device(dq, nq, 16, 10, ids, dist)
+                b.record(st)
+                torch.cuda.synchronize()
+                ms.append(a.elapsed_time(b))
+        return sorted(ms)[4]
+    plain = cost(x, q, cen)
+    if kind == "one":
+        x[n // 2] *= 1000
+    if kind == "nan":
+        x[n // 2, 0] = np.nan
+    if kind == "far":
+        x, q, cen = x + 100, q + 100, cen + 100
+    if kind == "same":
+        x[:] = 1.0
+    assert cost(x, q, cen) < times * plain
