@@ -3,6 +3,7 @@
 #include "batch_parts.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "mapped_rows.h"
 #include "select.cuh"
 
 #include <algorithm>
@@ -220,52 +221,39 @@ struct PoolBuf {
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
-// Host rows mapped for the device, counted over the sessions that read them: several sessions may lie over one array (a session per
-// query thread, or per view of it), and the mapping ends with the last of them, whichever made it.
-class MappedRows {
-public:
-    static MappedRows& get() { static MappedRows* one = new MappedRows; return *one; }   // never destroyed: the driver may end first
-    // *counted: give() has to follow.  False when the caller itself has the range registered, which is then the caller's to end.
-    psb_status take(const void* rows, size_t bytes, bool* counted) {
-        const uintptr_t b = reinterpret_cast<uintptr_t>(rows), e = b + bytes;
-        std::lock_guard<std::mutex> lk(mu_);
-        *counted = false;
-        for (Range& r : ranges_) {
-            if (r.begin <= b && e <= r.end) { ++r.users; *counted = true; return PSB_OK; }
-            if (r.begin < e && b < r.end)
-                return fail(PSB_CUDA_ERROR, "the exact rows overlap rows another session has mapped; use PSB_EXACT_HOST_STAGED");
-        }
+struct HostPages {
+    static Mapping map(const void* rows, size_t bytes, int* code) {
         cudaError_t err = cudaHostRegister(const_cast<void*>(rows), bytes, cudaHostRegisterMapped | cudaHostRegisterReadOnly);
-        if (err == cudaErrorHostMemoryAlreadyRegistered) { cudaGetLastError(); return PSB_OK; }
+        if (err == cudaErrorHostMemoryAlreadyRegistered) { cudaGetLastError(); return Mapping::kOthers; }
         if (err != cudaSuccess) {
             cudaGetLastError();
             err = cudaHostRegister(const_cast<void*>(rows), bytes, cudaHostRegisterMapped);
         }
-        if (err != cudaSuccess) {
-            cudaGetLastError();
-            return fail(PSB_CUDA_ERROR, std::string("cannot map the exact rows into the device address space (") + cudaGetErrorString(err) +
-                                            "); use PSB_EXACT_HOST_STAGED");
-        }
-        ranges_.push_back(Range{b, e, 1});
-        *counted = true;
-        return PSB_OK;
+        if (err == cudaSuccess) return Mapping::kMapped;
+        cudaGetLastError();
+        *code = (int)err;
+        return Mapping::kNot;
     }
-    void give(const void* rows, size_t bytes) {
-        const uintptr_t b = reinterpret_cast<uintptr_t>(rows), e = b + bytes;
-        std::lock_guard<std::mutex> lk(mu_);
-        for (size_t i = 0; i < ranges_.size(); ++i) {
-            if (b < ranges_[i].begin || ranges_[i].end < e) continue;
-            if (--ranges_[i].users == 0) {
-                cudaHostUnregister(reinterpret_cast<void*>(ranges_[i].begin));
-                ranges_.erase(ranges_.begin() + (ptrdiff_t)i);
-            }
-            return;
-        }
-    }
-private:
-    struct Range { uintptr_t begin, end; int users; };
-    std::mutex mu_;
-    std::vector<Range> ranges_;
+    static void unmap(void* rows) { cudaHostUnregister(rows); }
+};
+MappedRows<HostPages>& mapped_rows() { static auto* one = new MappedRows<HostPages>; return *one; }   // never destroyed: the driver may end first
+psb_status map_rows(const void* rows, size_t bytes, bool* counted) {
+    int code = 0;
+    const Mapping got = mapped_rows().take(rows, bytes, &code);
+    *counted = got == Mapping::kMapped;
+    if (got == Mapping::kOverlaps) return fail(PSB_CUDA_ERROR, "the exact rows overlap rows another session has mapped; use PSB_EXACT_HOST_STAGED");
+    if (got == Mapping::kNot)
+        return fail(PSB_CUDA_ERROR, std::string("cannot map the exact rows into the device address space (") + cudaGetErrorString((cudaError_t)code) +
+                                        "); use PSB_EXACT_HOST_STAGED");
+    return PSB_OK;
+}
+// The caller's arrays that a call copies to or from the device.  On a way out with an error the copies may still be under way on `st`.
+struct HostCopies {
+    cudaStream_t st;
+    MappedRows<HostPages>::Copies noted;
+    bool ended = false;
+    HostCopies(cudaStream_t st_, std::initializer_list<std::pair<const void*, size_t>> spans) : st(st_), noted(mapped_rows(), spans) {}
+    ~HostCopies() { if (noted.any() && !ended) cudaStreamSynchronize(st); }
 };
 
 // Page-locked blocks through which small calls pass, one to a session from its first search to its end, handed on from session to
@@ -483,7 +471,7 @@ struct psb_session {
     int exact_elem = 0;            // 4 = fp32, 1 = u8, 0 = rerank disabled
     const void* exact_host = nullptr;
     const void* exact_dev = nullptr;  // device-visible pointer (mapped host or resident)
-    bool mapped = false;           // exact_host is counted in MappedRows
+    bool mapped = false;           // exact_host is counted in mapped_rows()
     long long exact_count = 0;
     // staged mode
     void* pinned[2] = {nullptr, nullptr};
@@ -561,7 +549,7 @@ struct psb_session {
         for (cudaStream_t other : {list_stream, aux_stream, zc_stream})
             if (other) { cudaStreamSynchronize(other); cudaStreamDestroy(other); }
         collect_scan_events();
-        if (mapped) MappedRows::get().give(exact_host, (size_t)exact_count * dim * exact_elem);
+        if (mapped) mapped_rows().give(exact_host, (size_t)exact_count * dim * exact_elem);
         for (int i = 0; i < 2; ++i) {
             if (pinned[i]) cudaFreeHost(pinned[i]);
             if (pinned_ev[i]) cudaEventDestroy(pinned_ev[i]);
@@ -1284,6 +1272,24 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
     if (opt.stream) s->stream = static_cast<cudaStream_t>(opt.stream);
     else { PSB_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)); s->own_stream = true; }
     cudaStream_t st = s->stream;
+    const auto& E = index->exact;
+    if (E.fp32 || E.u8) {
+        s->exact_elem = E.fp32 ? 4 : 1;
+        s->exact_host = E.fp32 ? static_cast<const void*>(E.fp32) : static_cast<const void*>(E.u8);
+        s->exact_count = E.count;
+    }
+    const size_t exact_bytes = (size_t)s->exact_count * s->dim * s->exact_elem;
+    if ((opt.exact_mode == PSB_EXACT_HOST_MAPPED || opt.exact_mode == PSB_EXACT_HOST_HYBRID) && exact_bytes > 0) {   // before the copies are noted
+        PSB_TRY(map_rows(s->exact_host, exact_bytes, &s->mapped));
+        void* dp = nullptr;
+        PSB_CUDA(cudaHostGetDevicePointer(&dp, const_cast<void*>(s->exact_host), 0));
+        s->exact_dev = dp;
+    }
+    HostCopies copies(st, {{index->coarse.centroids, sizeof(float) * (size_t)nlist * s->dim}, {index->lists.offsets, sizeof(long long) * ((size_t)nlist + 1)},
+                           {index->lists.reordered_ids, sizeof(long long) * (size_t)s->n_vectors}, {index->pq.codes, (size_t)s->n_vectors * s->m},
+                           {index->pq.codebook, sizeof(float) * (size_t)s->k * s->dim}, {opt.opq_matrix, sizeof(float) * (size_t)s->dim * s->dim},
+                           {opt.row_correction_u16, sizeof(uint16_t) * (size_t)s->n_vectors}, {opt.row_correction_fp32, sizeof(float) * (size_t)s->n_vectors},
+                           {opt.exact_mode == PSB_EXACT_HOST_CACHED ? s->exact_host : nullptr, exact_bytes}});
     if (gb) {
         s->striped = true;
         s->h_global_begin.assign(gb, gb + nlist);
@@ -1346,12 +1352,8 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
     }
     note_list_lengths(s.get(), index->lists.offsets);
     // exact rows
-    const auto& E = index->exact;
-    if (E.fp32 || E.u8) {
-        s->exact_elem = E.fp32 ? 4 : 1;
-        s->exact_host = E.fp32 ? static_cast<const void*>(E.fp32) : static_cast<const void*>(E.u8);
-        s->exact_count = E.count;
-        const size_t bytes = (size_t)E.count * E.dim * s->exact_elem;
+    if (s->exact_host) {
+        const size_t bytes = exact_bytes;
         if (opt.exact_mode == PSB_EXACT_RESIDENT) {
             s->exact_dev = s->exact_host;
         } else if (opt.exact_mode == PSB_EXACT_HOST_CACHED && bytes > 0) {
@@ -1367,14 +1369,10 @@ psb_status psb_session_create(const psb_index_view* index, const psb_options* op
                                          static_cast<const unsigned char*>(s->exact_host) + off, std::min(chunk, bytes - off),
                                          cudaMemcpyHostToDevice, st));
             s->exact_dev = s->exact_cache.p;
-        } else if ((opt.exact_mode == PSB_EXACT_HOST_MAPPED || opt.exact_mode == PSB_EXACT_HOST_HYBRID) && bytes > 0) {
-            PSB_TRY(MappedRows::get().take(s->exact_host, bytes, &s->mapped));
-            void* dp = nullptr;
-            PSB_CUDA(cudaHostGetDevicePointer(&dp, const_cast<void*>(s->exact_host), 0));
-            s->exact_dev = dp;
         }
     }
     PSB_CUDA(cudaStreamSynchronize(st));
+    copies.ended = true;
     s->count();
     *out = s.release();
     return PSB_OK;
@@ -2037,6 +2035,8 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
                  b_ids = sizeof(long long) * (size_t)total * topk, b_dist = sizeof(float) * (size_t)total * topk;
     const bool small = batch == total && b_q + b_u8 + b_ids + b_dist <= kSmallIo;
     PSB_TRY(ensure_host_io(s));
+    HostCopies copies(st, {{small ? nullptr : queries->fp32, sizeof(float) * (size_t)total * s->dim}, {small || !u8 ? nullptr : queries->u8, (size_t)total * s->dim},
+                           {small ? nullptr : output->indices, b_ids}, {small ? nullptr : output->distances, b_dist}, {output->coarse_ids, sizeof(int) * (size_t)total * nprobe}});
     const bool one_stream = total < 2048 && sub_batch_rows(s, total, nprobe, false) >= total;
     CallMarks marks(s, small && one_stream && rows_form(s, total, nprobe) && !coarse_by_tc(s, total, nprobe) &&
                            (!rerank || rows_in_place(s, (long long)total * stage1_k)), reinterpret_cast<const float*>(s->h_io), total);
@@ -2098,6 +2098,7 @@ psb_status psb_session_search(psb_session* s, const psb_query_batch_view* querie
             times.collect();
         }
     }
+    copies.ended = true;
     PSB_TRY(check_tail(s));
     if (stats && marks.on) {
         times.ms[StageTimes::kCoarse] = marks.ms(0, 1);
@@ -2157,6 +2158,8 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
     else { PSB_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)); s->own_stream = true; }
     cudaStream_t st = s->stream;
     const size_t nl = (size_t)s->nlist, n = (size_t)std::max<long long>(1, s->n_vectors);
+    HostCopies copies(st, {{index->coarse.centroids, sizeof(float) * nl * s->dim}, {index->lists.offsets, sizeof(long long) * (nl + 1)},
+                           {index->lists.reordered_ids, sizeof(long long) * (size_t)s->n_vectors}, {index->rowmajor_fp32, sizeof(float) * (size_t)s->n_vectors * s->dim}});
     PSB_TRY(s->centroids.reserve(sizeof(float) * nl * s->dim));
     PSB_CUDA(cudaMemcpyAsync(s->centroids.p, index->coarse.centroids, sizeof(float) * nl * s->dim, cudaMemcpyHostToDevice, st));
     if (opt.coarse_mode != 1 && s->nlist >= 1024 && coarse_tc_padded_dim(s->dim) <= 128)
@@ -2176,6 +2179,7 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
     PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
     PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, st));
     PSB_CUDA(cudaStreamSynchronize(st));
+    copies.ended = true;
     s->count();
     *out = s.release();
     return PSB_OK;
@@ -2270,6 +2274,8 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
                  b_dist = sizeof(float) * (size_t)total * topk;
     const bool small = batch == total && b_q + b_ids + b_dist <= kSmallIo;   // through the pinned block, as psb_session_search
     PSB_TRY(ensure_host_io(s));
+    HostCopies copies(st, {{small ? nullptr : queries->fp32, sizeof(float) * (size_t)total * s->dim}, {small ? nullptr : output->indices, b_ids},
+                           {small ? nullptr : output->distances, b_dist}, {output->coarse_ids, sizeof(int) * (size_t)total * nprobe}});
     CallMarks marks(s, small && !coarse_by_tc(s, total, nprobe), reinterpret_cast<const float*>(s->h_io), total);
     const bool timed = stats && !marks.on;   // by events
     const long long launches0 = launches_total();
@@ -2304,6 +2310,7 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
             std::memcpy(output->distances, dist, b_dist);
         }
     }
+    copies.ended = true;
     PSB_TRY(check_tail(s));
     if (stats) {
         stats->total_ms = timed ? tm.ms(0, 1) : marks.ms(0, 3);
@@ -2343,6 +2350,10 @@ psb_status psb_rerank_host(const psb_host_storage_view* storage, const uint8_t* 
     PSB_TRY(cand.reserve(sizeof(int) * (size_t)batch_n * candidate_stride));
     PSB_TRY(out_rows.reserve(sizeof(int) * (size_t)batch_n * topk)); PSB_TRY(out_dist.reserve(sizeof(float) * (size_t)batch_n * topk));
     cudaStream_t st = nullptr;
+    HostCopies copies(st, {{use_float ? (const void*)storage->fp32 : (const void*)storage->u8, base_bytes},
+                           {use_float ? (const void*)h_queries_fp32 : (const void*)h_queries_u8, (size_t)batch_n * dim * elem},
+                           {h_candidates, sizeof(int) * (size_t)batch_n * candidate_stride}, {h_candidate_counts, sizeof(int) * (size_t)batch_n},
+                           {h_output_ids, sizeof(int) * (size_t)batch_n * topk}, {h_output_distances, sizeof(float) * (size_t)batch_n * topk}});
     PSB_CUDA(cudaMemcpy(base.p, use_float ? (const void*)storage->fp32 : (const void*)storage->u8, base_bytes, cudaMemcpyHostToDevice));
     PSB_CUDA(cudaMemcpy(q.p, use_float ? (const void*)h_queries_fp32 : (const void*)h_queries_u8, (size_t)batch_n * dim * elem, cudaMemcpyHostToDevice));
     PSB_CUDA(cudaMemcpy(cand.p, h_candidates, sizeof(int) * (size_t)batch_n * candidate_stride, cudaMemcpyHostToDevice));
@@ -2377,6 +2388,8 @@ psb_status psb_coarse_host(const float* h_queries, int nq, const float* h_centro
     PSB_TRY(q.reserve(sizeof(float) * (size_t)nq * dim)); PSB_TRY(c.reserve(sizeof(float) * (size_t)nlist * dim));
     PSB_TRY(ids.reserve(sizeof(int) * (size_t)nq * nprobe)); PSB_TRY(ids64.reserve(sizeof(long long) * (size_t)nq * nprobe));
     PSB_TRY(dist.reserve(sizeof(float) * (size_t)nq * nprobe));
+    HostCopies copies(nullptr, {{h_queries, sizeof(float) * (size_t)nq * dim}, {h_centroids, sizeof(float) * (size_t)nlist * dim},
+                                {h_ids, sizeof(long long) * (size_t)nq * nprobe}, {h_dist, sizeof(float) * (size_t)nq * nprobe}});
     PSB_CUDA(cudaMemcpy(q.p, h_queries, sizeof(float) * (size_t)nq * dim, cudaMemcpyHostToDevice));
     PSB_CUDA(cudaMemcpy(c.p, h_centroids, sizeof(float) * (size_t)nlist * dim, cudaMemcpyHostToDevice));
     const bool tc_ok = coarse_tc_supported(nq, nlist, dim, nprobe);
@@ -2556,6 +2569,7 @@ psb_status psb_kmeans_train(const float* d_data, int64_t n, int dim, float* d_ce
                                          obj.as<double>() + it, acc_ws, st));
         if (it < iters) PSB_TRY(launch_kmeans_update(sums.as<double>(), counts.as<int>(), k, dim, d_centroids, st));
     }
+    HostCopies copies(st, {{h_objective, sizeof(double) * ((size_t)iters + 1)}});
     if (h_objective) PSB_CUDA(cudaMemcpyAsync(h_objective, obj.p, sizeof(double) * ((size_t)iters + 1), cudaMemcpyDeviceToHost, st));
     PSB_CUDA(cudaStreamSynchronize(st));
     return assigner.check_status();
