@@ -860,9 +860,16 @@ psb_status ensure_pipeline_ws(psb_session* s, int nq, int nprobe, int topk, int 
     return ensure_scan_ws(s, sb, nprobe, stage1_k, rows_form(s, sb, nprobe));  // the scan runs one sub-batch at a time
 }
 
+bool coarse_by_tc(const psb_session* s, int nq, int nprobe) { return s->tc_index.ready && coarse_tc_supported(nq, s->nlist, s->dim, nprobe); }
+// Queries whose distances to all centroids the exact coarse stage keeps at a time, and the bytes they take (0: the tensor cores search).
+int exact_coarse_chunk(const psb_session* s, int nq) {
+    return std::min(nq, (int)std::max<size_t>(64, ((size_t)1 << 30) / (sizeof(float) * (size_t)s->nlist)));
+}
+size_t exact_coarse_bytes(const psb_session* s, int nq, int nprobe) {
+    return s->opt.coarse_mode != 1 && coarse_by_tc(s, nq, nprobe) ? 0 : sizeof(float) * (size_t)s->nlist * exact_coarse_chunk(s, nq);
+}
 // Coarse stage on device queries: exact distance tiles + row selection, query-chunked so the distance tile
 // stays below ~1 GiB.
-bool coarse_by_tc(const psb_session* s, int nq, int nprobe) { return s->tc_index.ready && coarse_tc_supported(nq, s->nlist, s->dim, nprobe); }
 psb_status coarse_exact(psb_session* s, const float* d_queries, int nq, int nprobe, int* d_ids, float* d_dist) {
     const int mode = s->opt.coarse_mode;
     const bool tc_ok = coarse_by_tc(s, nq, nprobe);
@@ -879,10 +886,8 @@ psb_status coarse_exact(psb_session* s, const float* d_queries, int nq, int npro
         return launch_coarse_tc(s->tc_index.view(s->centroids.as<float>(), s->nlist, s->dim), tw, d_queries,
                                 nq, nprobe, d_ids, d_dist, s->sm_count, s->stream);
     }
-    const size_t row_bytes = sizeof(float) * (size_t)s->nlist;
-    int chunk = (int)std::max<size_t>(64, ((size_t)1 << 30) / row_bytes);
-    chunk = std::min(chunk, nq);
-    PSB_TRY(s->dist_tile.reserve(row_bytes * (size_t)chunk));
+    const int chunk = exact_coarse_chunk(s, nq);
+    PSB_TRY(s->dist_tile.reserve(sizeof(float) * (size_t)s->nlist * chunk));
     for (int q0 = 0; q0 < nq; q0 += chunk) {
         const int n = std::min(chunk, nq - q0);
         PSB_TRY(launch_coarse_dist_exact(s->host_queries ? s->host_queries : d_queries + (size_t)q0 * s->dim, n, s->centroids.as<float>(), s->nlist, s->dim,
@@ -2192,7 +2197,21 @@ psb_status psb_flat_session_destroy(psb_flat_session* s) {
 
 namespace {
 psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe, int topk, long long* d_ids, float* d_dist) {
-    PSB_TRY(s->probes.reserve(sizeof(int) * (size_t)n * nprobe));
+    // A row of distances per query, as long as the nprobe longest lists; queries in parts of at most 1 GiB of them.
+    FlatScan f{};
+    f.stride = std::max<long long>(1, s->longest[(size_t)nprobe]);
+    const long long most = std::max<long long>(1, std::min(kPartQueries, kRowDistFloats / f.stride));
+    const int parts = (int)((n + most - 1) / most), per = (n + parts - 1) / parts;
+    f.run_stride = sel::run_count(f.stride);
+    // All that the call needs in one allocation, before anything is queued (a first call of 1,000 queries x 16 lists of 390 rows x 128: 900 -> 543 us).
+    const bool lists = flat_list_form(per, nprobe, s->nlist, s->n_vectors, s->dim);
+    const size_t pairs = lists ? (size_t)per * nprobe : 0, nl = lists ? (size_t)s->nlist + 1 : 0;
+    PSB_TRY(reserve_together(&s->row_whole, {{&s->probes, sizeof(int) * (size_t)n * nprobe}, {&s->dist_tile, exact_coarse_bytes(s, n, nprobe)},
+                                             {&s->row_dist, sizeof(float) * (size_t)per * f.stride}, {&s->row_seg, sizeof(int) * (size_t)per * ((size_t)nprobe + 1)},
+                                             {&s->row_runs, sizeof(float) * (size_t)per * f.run_stride},
+                                             {&s->vis_count, sizeof(int) * nl}, {&s->vis_off, sizeof(int) * nl}, {&s->item_off, sizeof(long long) * nl},
+                                             {&s->visitors, sizeof(int) * pairs}, {&s->flat_slot, sizeof(int) * pairs},
+                                             {&s->flat_again, lists ? sizeof(int) * (size_t)per : 0}}));
     PSB_TRY(coarse_exact(s, dq, n, nprobe, s->probes.as<int>(), nullptr));
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (s->opt.time_kernels) {  // bracket the fine scan (read back by psb_session_counters)
@@ -2200,22 +2219,6 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
         PSB_CUDA(cudaEventCreate(&ev1));
         s->scan_events.emplace_back(ev0, ev1);
         PSB_CUDA(cudaEventRecord(ev0, s->stream));
-    }
-    // A row of distances per query, as long as the nprobe longest lists; queries in parts of at most 1 GiB of them.
-    FlatScan f{};
-    f.stride = std::max<long long>(1, s->longest[(size_t)nprobe]);
-    const long long most = std::max<long long>(1, std::min(kPartQueries, kRowDistFloats / f.stride));
-    const int parts = (int)((n + most - 1) / most), per = (n + parts - 1) / parts;
-    f.run_stride = sel::run_count(f.stride);
-    PSB_TRY(reserve_together(&s->row_whole, {{&s->row_dist, sizeof(float) * (size_t)per * f.stride}, {&s->row_seg, sizeof(int) * (size_t)per * ((size_t)nprobe + 1)},
-                                             {&s->row_runs, sizeof(float) * (size_t)per * f.run_stride}}));
-    if (flat_list_form(per, nprobe, s->nlist, s->n_vectors, s->dim)) {
-        PSB_TRY(s->vis_count.reserve(sizeof(int) * ((size_t)s->nlist + 1)));
-        PSB_TRY(s->flat_again.reserve(sizeof(int) * (size_t)per));
-        PSB_TRY(s->flat_slot.reserve(sizeof(int) * (size_t)per * nprobe));
-        PSB_TRY(s->vis_off.reserve(sizeof(int) * ((size_t)s->nlist + 1)));
-        PSB_TRY(s->item_off.reserve(sizeof(long long) * ((size_t)s->nlist + 1)));
-        PSB_TRY(s->visitors.reserve(sizeof(int) * (size_t)per * nprobe));
     }
     f.dim = s->dim; f.nprobe = nprobe; f.offsets = s->offsets.as<long long>(); f.nlist = s->nlist; f.n_rows = s->n_vectors; f.rows = s->flat_rows.as<float>();
     f.norms = s->flat_norms.as<float>(); f.most = s->flat_norms.as<unsigned>() + std::max<long long>(1, s->n_vectors);
@@ -2267,9 +2270,8 @@ psb_status psb_flat_session_search(psb_flat_session* s, const psb_query_batch_vi
     if (total == 0) return PSB_OK;
     const int batch = std::min(std::min(params->batch_size, s->opt.max_batch), total);
     cudaStream_t st = s->stream;
-    PSB_TRY(s->q.reserve(sizeof(float) * (size_t)batch * s->dim));
-    PSB_TRY(s->out_ids.reserve(sizeof(long long) * (size_t)batch * topk));
-    PSB_TRY(s->out_dist.reserve(sizeof(float) * (size_t)batch * topk));
+    PSB_TRY(reserve_together(&s->call_whole, {{&s->q, sizeof(float) * (size_t)batch * s->dim}, {&s->out_ids, sizeof(long long) * (size_t)batch * topk},
+                                              {&s->out_dist, sizeof(float) * (size_t)batch * topk}}));
     const size_t b_q = (sizeof(float) * (size_t)total * s->dim + 255) / 256 * 256, b_ids = sizeof(long long) * (size_t)total * topk,
                  b_dist = sizeof(float) * (size_t)total * topk;
     const bool small = batch == total && b_q + b_ids + b_dist <= kSmallIo;   // through the pinned block, as psb_session_search

@@ -111,6 +111,21 @@ def test_list_form_behind_the_filter(psb, dim, kind, k):
         assert np.array_equal(got["distances"][i][: len(order)][take], d[order][take])
 
 
+def test_calls_of_changing_size(psb):
+    """A session's buffers are one allocation, laid out anew when a call needs more: both forms, more and fewer queries, probes and results."""
+    rng = np.random.default_rng(3)
+    n, dim, nlist = 20000, 64, 32
+    off = np.concatenate([[0], np.sort(rng.integers(0, n + 1, nlist - 1)), [n]]).astype(np.int64)
+    fx = dict(centroids=rng.standard_normal((nlist, dim)).astype(np.float32), offsets=off, reordered_ids=rng.permutation(n).astype(np.int64),
+              vectors=rng.standard_normal((n, dim)).astype(np.float32))
+    with psb.FlatSession(fx, max_batch=900) as s:
+        for nq, nprobe, topk in ((3, 8, 10), (700, 4, 10), (5, 32, 300), (900, 2, 256), (64, 20, 7), (900, 9, 300), (1, 1, 1), (850, 3, 20)):
+            q = rng.standard_normal((nq, dim)).astype(np.float32)
+            got = s.search(q, nprobe, topk, batch_size=nq)
+            wi, wd = oracle.ivfflat_search(fx["centroids"], off, fx["reordered_ids"], fx["vectors"], q, nprobe, topk)
+            assert np.array_equal(got["indices"], wi) and np.array_equal(got["distances"], wd)
+
+
 @pytest.mark.parametrize("kind,times", [("one", 2.0), ("nan", 2.0), ("far", 4.0), ("same", 6.0)])   # measured 1.0, 1.0, 2.3, 3.7
 def test_cost_where_the_bound_is_loose(psb, kind, times):
     """Rows that loosen the filter's bound cost the queries that it cannot serve the exact tiles, and the others nothing."""
