@@ -445,8 +445,12 @@ __global__ void k_km_fill(const int* __restrict__ assign, long long n, int k, co
 }
 // The same two for few centroids, whose counters all rows would queue at: a block counts its kFewRows rows in shared memory first, and takes the
 // places of each centroid's with one atomic (400,000 rows, 64
-// centroids, five iterations: 4.7 -> 3.3 ms).
+// centroids, five iterations: 4.7 -> 3.3 ms).  A block's own part, which it does whatever the rows, costs 2 to 3 us more in all, so that there have to be rows enough
+// and rows enough a centroid.  Whole accumulation of 64 dimensions, us, rows by themselves / by blocks: 512 centroids, 20 rows each 33.0 / 36.2, 32 37.4 / 37.0, 96
+// 49.0 / 40.6; 1,024, 16 35.9 / 39.3, 32 40.4 / 39.7; 2,048, 16 46.2 / 46.9, 32 50.1 / 50.1, 48 54.8 / 51.9; 256, 32 32.6 / 36.1, 64 37.8 / 38.3, 160 53.3 / 44.7; 64, 96
+// 35.8 / 38.1, 400 50.6 / 41.8.
 constexpr int kFewCentroids = 2048, kFewRows = 4096;
+constexpr long long kFewPerCentroid = 32, kFewLeast = 16384;
 __global__ void __launch_bounds__(1024) k_km_count_few(const int* __restrict__ assign, const float* __restrict__ best, long long n, int k, int* __restrict__ counts,
                                                        double* __restrict__ obj) {
     __shared__ int s_count[kFewCentroids];
@@ -689,8 +693,9 @@ psb_status launch_kmeans_accumulate(const float* d_data, long long n, int dim, c
     if (n > 0x7fffffffLL) return fail(PSB_UNSUPPORTED_SHAPE, "more than 2^31-1 rows in one accumulation");
     if (!ws.order || !ws.offsets || !ws.cursor) return fail(PSB_INTERNAL, "k-means accumulation workspace missing");
     // d_counts and *d_obj were zeroed by the caller; d_sums is written whole
+    const bool few = k <= kFewCentroids && n >= kFewLeast && n >= kFewPerCentroid * k;
     if (n > 0) {
-        if (k <= kFewCentroids) k_km_count_few<<<(unsigned)((n + kFewRows - 1) / kFewRows), 1024, 0, s>>>(d_assign, d_best, n, k, d_counts, d_obj);
+        if (few) k_km_count_few<<<(unsigned)((n + kFewRows - 1) / kFewRows), 1024, 0, s>>>(d_assign, d_best, n, k, d_counts, d_obj);
         else k_km_count<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_assign, d_best, n, k, d_counts, d_obj);
         count_launch();
         PSB_LAUNCH_CHECK();
@@ -699,7 +704,7 @@ psb_status launch_kmeans_accumulate(const float* d_data, long long n, int dim, c
     count_launch();
     PSB_LAUNCH_CHECK();
     if (n > 0) {
-        if (k <= kFewCentroids) k_km_fill_few<<<(unsigned)((n + kFewRows - 1) / kFewRows), 1024, 0, s>>>(d_assign, n, k, ws.offsets, ws.cursor, ws.order);
+        if (few) k_km_fill_few<<<(unsigned)((n + kFewRows - 1) / kFewRows), 1024, 0, s>>>(d_assign, n, k, ws.offsets, ws.cursor, ws.order);
         else k_km_fill<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_assign, n, k, ws.offsets, ws.cursor, ws.order);
         count_launch();
         PSB_LAUNCH_CHECK();
