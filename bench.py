@@ -514,14 +514,15 @@ def main():
                   recall_at_k_cpu=recall_at(ref["indices"][:gtn], gt_ids[:gtn], topk) if gtn else None,
                   recall_at_10_gpu=recall_at(e2e_ids[:gtn], gt_ids[:gtn], min(10, topk)) if gtn else None,
                   recall_at_10_cpu=recall_at(ref["indices"][:gtn], gt_ids[:gtn], min(10, topk)) if gtn else None)
-    host_pct = dict(staged=100, hybrid=100 - (args.zero_copy_pct or 100)).get(args.exact_mode, 0)   # the host threads' share of the rows
-    fetched = int(c["staged_gather_bytes"] / max(1, args.steps) * 100 / host_pct) or None if host_pct and R > topk else None
+    fetched = int(c["rerank_rows_fetched"] / max(1, args.steps) * dim * 4) or None   # each distinct row of a batch once
+    rows_by = {"hybrid": "host-hybrid fp32" + (", %d %% by the gather kernel" % args.zero_copy_pct if args.zero_copy_pct else " (all by the gather kernel over mapped memory)"),
+               "cached": "device-cached fp32"}.get(args.exact_mode, "host-%s fp32" % args.exact_mode)
     line = dict(
         metric="QPS (IVF-PQ search, recall@k equal to the reference CPU path)", value=round(nq / (ms_dev * 1e-3), 1),
         unit="queries/s", n_gpus=1, steps=args.steps, warmup=max(args.warmup, 3), ms_per_step=round(ms_dev, 3),
         higher_is_better=True, scaling="strong", vs_baseline=None, dtype="f32", data="synthetic",
         config=dict(workload=args.workload, desc=cfg["desc"], rows=cfg["n"], dim=dim, nlist=cfg["nlist"], M=cfg["M"],
-                    batch=nq, nprobe=nprobe, topk=topk, n_rerank=R, exact_rows="host-%s fp32" % args.exact_mode,
+                    batch=nq, nprobe=nprobe, topk=topk, n_rerank=R, exact_rows=rows_by,
                     l2="inputs larger than L2 (codes %.1f GB)" % (index["codes"].nbytes / 1e9)),
         e2e=dict(value=round(nq / (ms_e2e * 1e-3), 1), unit="queries/s", ms_per_step=round(ms_e2e, 3),
                  h2d_bytes_per_step=int(stats["h2d_bytes"]), d2h_bytes_per_step=int(stats["d2h_bytes"]),
@@ -531,8 +532,8 @@ def main():
         # end-to-end step is bound by
         transport=dict(requested_bytes_per_step=int(nq * stage1 * dim * 4) if R > topk else 0, fetched_bytes_per_step=fetched,
                        achieved_gbs=round(fetched / max(1e-9, stats["pq_rerank_ms"] * 1e-3) / 1e9, 1) if fetched and stats["pq_rerank_ms"] > 0 else None,
-                       pinned_h2d_copy_gbs=h2d_gbs, note="fetched = distinct rows, from the host threads' share (none in the mapped transport); achieved = "
-                       "fetched bytes / rerank stage time (random rows of dim * 4 bytes); pinned_h2d_copy_gbs = one large pinned copy on this host, the link's ceiling"),
+                       pinned_h2d_copy_gbs=h2d_gbs, note="fetched = distinct rows of a batch; achieved = fetched bytes / rerank stage time "
+                       "(rows of dim * 4 bytes, in ascending order; the stage has gaps between its parts); pinned_h2d_copy_gbs = one large pinned copy on this host, the link's ceiling"),
         cpu_baseline=dict(value=round(ns / dt, 2), unit="queries/s", cores=cores, kind=kind,
                           sample="first %d queries of the batch, all %d host threads" % (ns, cores)),
         stages_ms=dict(coarse=round(stats["coarse_search_ms"], 3), lut=round(stats["pq_lut_build_ms"], 3),

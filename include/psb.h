@@ -224,7 +224,8 @@ typedef struct psb_stats {
        bytes gathered, since the last reset. */
     double staged_gather_ms;
     long long staged_gather_bytes;
-    int reserved[4];
+    long long rerank_rows_fetched; /* session counters: rows that crossed from host memory, each distinct row of a batch once (rows scored in place are not counted) */
+    int reserved[2];
 } psb_stats;
 
 typedef struct psb_session psb_session;

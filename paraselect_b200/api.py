@@ -89,7 +89,8 @@ class Stats(C.Structure):
                 ("batches", C.c_int), ("coarse_fallback_queries", C.c_int), ("prefilter_survivors", C.c_longlong),
                 ("tc_wait_item_cycles", C.c_longlong), ("tc_wait_rows_cycles", C.c_longlong), ("tc_wait_acc_cycles", C.c_longlong),
                 ("tc_tiles", C.c_longlong), ("staged_gather_ms", C.c_double), ("staged_gather_bytes", C.c_longlong),
-                ("reserved", C.c_int * 4)]
+                ("rerank_rows_fetched", C.c_longlong),
+                ("reserved", C.c_int * 2)]
 
     def as_dict(self):
         return {n: getattr(self, n) for n, _ in self._fields_ if n != "reserved"}

@@ -328,7 +328,7 @@ struct RowMap {
 };
 // Each row a batch's candidates name gets a slot, those of one launch in ascending order.  A batch may claim in several launches (parts): the
 // slots of each begin at *d_begin, which the part before left in its *d_end; *d_n_unique: their number so far.  launch_release_rows puts slot_of
-// back.
+// back and adds the number of rows to *d_fetched.
 struct ClaimBuffers {
     long long count = 0;        // rows held here
     int* slot_of = nullptr;     // [count] -1: none yet
@@ -341,7 +341,7 @@ size_t claim_words(long long count);
 size_t claim_sums(long long count);
 psb_status launch_claim_rows(const RowMap& mp, const int* d_candidates, int nq, int candidate_count, int candidate_stride, const int* d_counts,
                              const ClaimBuffers& b, const int* d_begin, int* d_end, int* d_n_unique, cudaStream_t s);
-psb_status launch_release_rows(const int* d_unique, const int* d_n_unique, int* d_slot_of, int sm_count, cudaStream_t s);
+psb_status launch_release_rows(const int* d_unique, const int* d_n_unique, int* d_slot_of, unsigned long long* d_fetched, int sm_count, cudaStream_t s);
 // Of the slots [begin, end) the host threads fill those below this, the gather kernel the others.
 __host__ __device__ __forceinline__ int host_share_end(int begin, int end, int host_pct) { return begin + (int)((long long)(end - begin) * host_pct / 100); }
 // Copies the rows (src: device-visible, by row) of slots [*d_begin, *d_end) to d_stage (by slot).  compact_ctas > 0: the kernel runs

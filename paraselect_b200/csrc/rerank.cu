@@ -135,8 +135,10 @@ __global__ void k_call_tail(const unsigned long long* __restrict__ words, const 
     if (coarse && threadIdx.x < 8) tail->tc[threadIdx.x] = coarse[threadIdx.x];
 }
 
-__global__ void k_release_rows(const int* __restrict__ unique, const int* __restrict__ n_unique, int* __restrict__ slot_of) {
+// *fetched grows by the number of rows.
+__global__ void k_release_rows(const int* __restrict__ unique, const int* __restrict__ n_unique, int* __restrict__ slot_of, unsigned long long* __restrict__ fetched) {
     const int n = *n_unique;
+    if ((blockIdx.x | threadIdx.x) == 0) *fetched += (unsigned long long)n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) slot_of[unique[i]] = -1;
 }
 
@@ -541,9 +543,9 @@ psb_status launch_claim_rows(const RowMap& mp, const int* d_candidates, int nq, 
     return PSB_OK;
 }
 
-psb_status launch_release_rows(const int* d_unique, const int* d_n_unique, int* d_slot_of, int sm_count, cudaStream_t s) {
+psb_status launch_release_rows(const int* d_unique, const int* d_n_unique, int* d_slot_of, unsigned long long* d_fetched, int sm_count, cudaStream_t s) {
     PSB_TRY(prefer_max_shared(k_release_rows));
-    k_release_rows<<<sm_count * 2, 256, 0, s>>>(d_unique, d_n_unique, d_slot_of);
+    k_release_rows<<<sm_count * 2, 256, 0, s>>>(d_unique, d_n_unique, d_slot_of, d_fetched);
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

@@ -684,6 +684,8 @@ void note_list_lengths(psb_session* s, const int64_t* offsets) {
     s->own_list_rows = s->shard_rows > 0 ? sq / (double)s->shard_rows : 0.0;
 }
 
+// Words of a session's `scalars`: counters [0..7], work words of the scan and its status [8..12], call marks [13..15], rows fetched.
+constexpr size_t kScalars = 24, kRowsFetched = 16;
 constexpr long long kRowDistFloats = 1ll << 28;   // distances kept at a time in the row forms: 1 GiB
 constexpr long long kPartQueries = 32768;         // queries at a time: they are the grid's second dimension, which ends at 65,535
 
@@ -781,13 +783,16 @@ int longest_cut(const std::vector<int>& cuts) {
     return most;
 }
 
+psb_status ensure_scalars(psb_session* s, cudaStream_t st) {
+    if (s->scalars.p) return PSB_OK;
+    PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * kScalars));
+    PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * kScalars, st));
+    return PSB_OK;
+}
 // Grows the scan workspace to hold nq queries (never shrinks; a growing buffer is freed first, which waits for the device).
 // row_form: the scan's row form takes this call.  It uses the counters alone of all that follows; its distances are run_scan's.
 psb_status ensure_scan_ws(psb_session* s, int nq, int nprobe, int stage1_k, bool row_form) {
-    if (!s->scalars.p) {
-        PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
-        PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, s->stream));
-    }
+    PSB_TRY(ensure_scalars(s, s->stream));
     if (row_form) return PSB_OK;
     const size_t tables = table_count(s, nq, nprobe);
     s->ws_scan_queries = 0; s->ws_scan_tables = 0;  // set again below once every buffer has its size
@@ -1017,6 +1022,7 @@ psb_status rows_begin(psb_session* s, long long requests, size_t parts, cudaStre
     s->slots = slots;
     s->parts = parts;
     bool moved = false;
+    PSB_TRY(ensure_scalars(s, st));
     PSB_TRY(reserve_together(&s->rows_whole, {{&s->unique, sizeof(int) * slots}, {&s->marks, sizeof(int) * PartMarks::device_words(parts)},
                                               {&s->stage, slots * s->dim * s->exact_elem},
                                               {&s->slot_of, sizeof(int) * (size_t)std::max<long long>(1, s->exact_count)},
@@ -1041,7 +1047,7 @@ psb_status rows_claim(psb_session* s, int part, const int* d_cand, int nq, int w
     return launch_claim_rows(s->row_map(), d_cand, nq, width, stride, d_counts, b, part_begin(s, part), part_end(s, part), s->marks.as<int>(), st);
 }
 psb_status rows_end(psb_session* s, cudaStream_t st) {
-    PSB_TRY(launch_release_rows(s->unique.as<int>(), s->marks.as<int>(), s->slot_of.as<int>(), s->sm_count, st));
+    PSB_TRY(launch_release_rows(s->unique.as<int>(), s->marks.as<int>(), s->slot_of.as<int>(), s->scalars.as<unsigned long long>() + kRowsFetched, s->sm_count, st));
     s->slots_dirty = false;
     return PSB_OK;
 }
@@ -1634,10 +1640,13 @@ psb_status psb_session_counters(psb_session* s, psb_stats* stats, int reset) {
     if (!s || !stats) return fail(PSB_INVALID_ARGUMENT, "null argument");
     s->counters_known = false;
     PSB_CUDA(cudaSetDevice(s->device));
-    unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    unsigned long long h[kScalars] = {};
     if (s->scalars.p) {
         PSB_CUDA(cudaMemcpyAsync(h, s->scalars.p, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
-        if (reset) PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(h), s->stream));
+        if (reset) {
+            PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 8, s->stream));
+            PSB_CUDA(cudaMemsetAsync(s->scalars.as<unsigned long long>() + kRowsFetched, 0, sizeof(unsigned long long), s->stream));
+        }
         PSB_CUDA(cudaStreamSynchronize(s->stream));
     }
     stats->pq_scanned_codes = (long long)h[0];
@@ -1647,6 +1656,7 @@ psb_status psb_session_counters(psb_session* s, psb_stats* stats, int reset) {
     stats->prefilter_survivors = (long long)h[3];
     stats->tc_wait_item_cycles = (long long)h[4]; stats->tc_wait_rows_cycles = (long long)h[5];
     stats->tc_wait_acc_cycles = (long long)h[6]; stats->tc_tiles = (long long)h[7];
+    stats->rerank_rows_fetched = (long long)h[kRowsFetched];
     stats->staged_gather_ms = s->staged_gather_s * 1e3; stats->staged_gather_bytes = s->staged_gather_bytes;
     if (reset) { s->staged_gather_s = 0.0; s->staged_gather_bytes = 0; }
     stats->kernel_launches = launches_total();
@@ -2181,8 +2191,7 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
     PSB_TRY(s->flat_norms.reserve(sizeof(float) * (n + nl)));
     PSB_TRY(launch_flat_norms(s->flat_rows.as<float>(), s->n_vectors, s->dim, s->offsets.as<long long>(), s->nlist, s->flat_norms.as<float>(),
                               s->flat_norms.as<unsigned>() + n, st));
-    PSB_TRY(s->scalars.reserve(sizeof(unsigned long long) * 16));
-    PSB_CUDA(cudaMemsetAsync(s->scalars.p, 0, sizeof(unsigned long long) * 16, st));
+    PSB_TRY(ensure_scalars(s.get(), st));
     PSB_CUDA(cudaStreamSynchronize(st));
     copies.ended = true;
     s->count();

@@ -121,6 +121,29 @@ def test_slots_in_row_order(psb, mode, count):
             assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
 
 
+@pytest.mark.parametrize("mode,pct", [(0, 0), (4, 0), (4, 50)])
+def test_rows_fetched_are_counted(psb, mode, pct):
+    """Each distinct row of a batch once, whoever brings it; rows that are scored in place are not counted."""
+    import torch
+    ix = index(1500, 32, False, 5)
+    rng = np.random.default_rng(6)
+    nq, width = 700, 100
+    with psb.Session(ix, n_rerank=width, exact_mode=mode, zero_copy_pct=pct, max_batch=nq) as s:
+        assert s.counters(reset=True)["rerank_rows_fetched"] == 0
+        want = 0
+        q = torch.from_numpy(rng.standard_normal((nq, 32)).astype(np.float32)).cuda()
+        rows = torch.empty((nq, 10), dtype=torch.int32, device="cuda"); dist = torch.empty((nq, 10), device="cuda")
+        for top in (300, 1500):
+            cand = rng.integers(-1, top, (nq, width)).astype(np.int32)
+            s.stage_rerank(q, nq, torch.from_numpy(cand).cuda(), width, width, None, 10, rows, dist)
+            s.sync()
+            want += len(np.unique(cand[cand >= 0]))
+        s.stage_rerank(q, 3, torch.from_numpy(cand[:3].copy()).cuda(), width, width, None, 10, rows, dist)   # in place
+        s.sync()
+        assert s.counters(reset=True)["rerank_rows_fetched"] == want
+        assert s.counters()["rerank_rows_fetched"] == 0
+
+
 @pytest.mark.parametrize("mode,pct,call", [(0, 0, "search"), (4, 90, "search"), (4, 90, "stage")])   # the kernel alone; host threads beside it
 def test_error_beside_a_gather(psb, mode, pct, call):
     """A call that ends with an error while a kernel on a stream of its own gathers its rows: the session's stream goes on behind the gather, so
