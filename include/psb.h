@@ -192,7 +192,7 @@ typedef struct psb_options {
 /* Counters and stage times of the last psb_session_search call; names follow the reference's
  * IVFSearchStatsCollector fields (src/search/ivfpq/pipeline/ivfpq_pipeline.cu:41-71,84-103).  Stage times are the device's.  In small calls
  * (queries and results of 256 KiB at most, one stream) the kernels note their own starts, a stage lasts until the next one's, queries and
- * results pass without copies (h2d_ms = d2h_ms = 0), and total_ms begins with the first kernel. */
+ * results pass without copies of their own (h2d_ms = d2h_ms = 0), and total_ms, which has the transfers in it all the same, is the host's clock. */
 typedef struct psb_stats {
     double total_ms;
     double coarse_search_ms;

@@ -146,3 +146,22 @@ def test_small_calls_mark_their_own_times(psb, nq, rerank):
             t = got["stats"]
             stages = [t["coarse_search_ms"], t["pq_adc_scan_ms"]] + ([t["pq_rerank_ms"]] if rerank else [])
             assert min(stages) > 0 and sum(stages) <= t["total_ms"] * 1.0001 + 0.01 and t["total_ms"] < 1000
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("nq", [1, 300, 3000])   # 3,000: by events, as calls that do not pass through the page-locked block
+def test_total_time_is_the_whole_call(psb, flat, nq):
+    """The transfers among it: never longer than the call takes by the wall clock, and most of that."""
+    import time
+    ix = synth.make_index(6000, 24, 70, 6, seed=5)
+    q = synth.make_queries(ix, nq, seed=nq)
+    fx = dict(centroids=ix["centroids"], offsets=ix["offsets"], reordered_ids=ix["reordered_ids"], vectors=ix["vectors"])
+    with (psb.FlatSession(fx, max_batch=nq) if flat else psb.Session(ix, n_rerank=40, max_batch=nq)) as s:
+        share = []
+        for _ in range(40):
+            t = time.perf_counter()
+            got = s.search(q, 6, 10, batch_size=nq)
+            wall = (time.perf_counter() - t) * 1e3
+            assert 0 < got["stats"]["total_ms"] <= wall
+            share.append(got["stats"]["total_ms"] / wall)
+    assert sorted(share)[20] > 0.4     # the rest: the binding's arrays and checks
