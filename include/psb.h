@@ -510,6 +510,11 @@ psb_status psb_kmeans_assign(const float* d_data, int64_t n, int dim, const floa
  * centroid bounds its nearest distance, and the tensor-core filter runs once instead of twice; the result is the same. */
 psb_status psb_kmeans_assign_bounded(const float* d_data, int64_t n, int dim, const float* d_centroids, int k, int* d_assign,
                                      float* d_best, int have_previous, int device, void* stream);
+/* psb_kmeans_assign_bounded by a given form, as psb_options.coarse_mode names one for the coarse stage: 0 = as the size says, 1 = exact kernels
+ * only, 2 = tensor-core filter required (PSB_UNSUPPORTED_SHAPE below 64 rows, below 128 centroids or above 128
+ * dimensions).  The result is the same. */
+psb_status psb_kmeans_assign_form(const float* d_data, int64_t n, int dim, const float* d_centroids, int k, int* d_assign,
+                                  float* d_best, int have_previous, int form, int device, void* stream);
 psb_status psb_kmeans_accumulate(const float* d_data, int64_t n, int dim, const int* d_assign, const float* d_best, int k,
                                  double* d_sums, int* d_counts, double* d_objective, int device, void* stream);
 psb_status psb_kmeans_update(const double* d_sums, const int* d_counts, int k, int dim, float* d_centroids, int device,

@@ -2488,13 +2488,15 @@ namespace {
 // centroid - any point will do) and kept when it takes at most kKeepRows bytes, and nothing is copied to the host in between.
 class Assigner {
 public:
-    Assigner(const float* d_data, int64_t n, int dim, int k, int device, int sms, cudaStream_t st)
+    // form: 0 = the rule below, 1 = without the filter, 2 = with it (filter_takes)
+    Assigner(const float* d_data, int64_t n, int dim, int k, int device, int sms, cudaStream_t st, int form = 0)
         : data_(d_data), n_(n), dim_(dim), k_(k), device_(device), sms_(sms), st_(st) {
         // The filter costs about 2 ns a row whatever the number of centroids, and its launches more than the row kernel's; that takes 1.2e-4 ns for
         // each dimension of a pair.  Trainings of three iterations, rows / filter, us: 20,000 x 64, 256 centroids 548 / 631, 400 654 / 572; 20,000 x
         // 128, 128 613 / 756, 200 749 / 673; 100,000 x 96, 128 1,218 / 1,239, 1,000 5,020 / 1,200; 400,000 x 100, 128 4,031 / 3,216, 1,000 19,369 / 3,233.
-        tc_ = n >= 64 && coarse_tc_padded_dim(dim) <= 128 && (!nearest_rows_fit(dim) || (double)k * dim >= 16384.0 + 1.6e8 / (double)n);
+        tc_ = form == 2 || (form == 0 && filter_takes(n, dim, k) && (!nearest_rows_fit(dim) || (double)k * dim >= 16384.0 + 1.6e8 / (double)n));
     }
+    static bool filter_takes(int64_t n, int dim, int k) { return n >= 64 && k >= 128 && coarse_tc_padded_dim(dim) <= 128; }
     // d_assign [n], d_best [n] out; bounded: d_assign holds an assignment on entry, whose distances bound the nearest ones (one
     // filter pass instead of two).
     psb_status run(const float* d_centroids, int* d_assign, float* d_best, bool bounded) {
@@ -2602,12 +2604,18 @@ psb_status psb_kmeans_assign(const float* d_data, int64_t n, int dim, const floa
 
 psb_status psb_kmeans_assign_bounded(const float* d_data, int64_t n, int dim, const float* d_centroids, int k, int* d_assign,
                                      float* d_best, int have_previous, int device, void* stream) {
-    if (!d_data || !d_centroids || !d_assign || !d_best || n <= 0 || dim <= 0 || k <= 0)
+    return psb_kmeans_assign_form(d_data, n, dim, d_centroids, k, d_assign, d_best, have_previous, 0, device, stream);
+}
+
+psb_status psb_kmeans_assign_form(const float* d_data, int64_t n, int dim, const float* d_centroids, int k, int* d_assign,
+                                  float* d_best, int have_previous, int form, int device, void* stream) {
+    if (!d_data || !d_centroids || !d_assign || !d_best || n <= 0 || dim <= 0 || k <= 0 || form < 0 || form > 2)
         return fail(PSB_INVALID_ARGUMENT, "invalid k-means assignment request");
+    if (form == 2 && !Assigner::filter_takes(n, dim, k)) return fail(PSB_UNSUPPORTED_SHAPE, "the tensor-core filter does not take this shape");
     int sms = 0;
     PSB_TRY(check_device(device, &sms));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    Assigner assigner(d_data, n, dim, k, device, sms, st);
+    Assigner assigner(d_data, n, dim, k, device, sms, st, form);
     PSB_TRY(assigner.run(d_centroids, d_assign, d_best, have_previous != 0));
     PSB_CUDA(cudaStreamSynchronize(st));
     return assigner.check_status();

@@ -35,6 +35,43 @@ def test_useless_bounds(psb, n, dim, k, prev):
     assert torch.equal(best, want_d) and torch.equal(assign.long(), want)
 
 
+@pytest.mark.parametrize("n,dim,k", [(300, 64, 1024), (1000, 100, 1500), (64, 37, 2048), (65, 37, 128), (5000, 100, 131), (4097, 128, 255), (3000, 5, 256),
+                                     (2500, 37, 257), (6000, 128, 511), (6000, 64, 512), (1025, 100, 513), (9000, 96, 700), (3333, 126, 1023)])
+@pytest.mark.parametrize("prev", [None, "zeros", "far", "outside", "same"])
+@pytest.mark.parametrize("form", [1, 2])
+def test_either_form(psb, n, dim, k, prev, form):
+    """The same through the form that is asked for, wherever the line between them lies: loose bounds, rows near nothing, ties, rows that are not
+    numbers, centroids that fill a part of a block or a little of a second."""
+    import torch
+    g = torch.Generator(device="cuda"); g.manual_seed(n + dim + k)
+    c = torch.randn(k, dim, device="cuda", generator=g)
+    x = c[torch.randint(k, (n,), device="cuda", generator=g)] + 0.2 * torch.randn(n, dim, device="cuda", generator=g)
+    x[1:20] = c[5] * 0.0
+    x[20:30] = 40 * x[20:30]
+    c[7] = c[6]
+    c[k - 1] = c[3]
+    x[30:40] = c[6]
+    want_d, want = nearest(x, c)
+    x[50, dim - 1], x[51, 0] = float("nan"), float("inf")
+    fine = torch.ones(n, dtype=torch.bool, device="cuda"); fine[50:52] = False
+    assign = {None: torch.full((n,), 77, dtype=torch.int32, device="cuda"), "zeros": torch.zeros(n, dtype=torch.int32, device="cuda"),
+              "far": ((want + k // 2) % k).to(torch.int32), "outside": torch.full((n,), -1, dtype=torch.int32, device="cuda"),
+              "same": want.to(torch.int32)}[prev].contiguous()
+    best = torch.empty(n, device="cuda")
+    psb.kmeans_assign(x, n, dim, c, k, assign, best, have_previous=prev is not None, form=form)
+    assert torch.equal(best[fine], want_d[fine]) and torch.equal(assign.long()[fine], want[fine])
+    assert bool(((assign >= 0) & (assign < k))[50:52].all())
+
+
+def test_form_that_does_not_take_the_shape(psb):
+    import torch
+    x, c = torch.randn(100, 130, device="cuda"), torch.randn(200, 130, device="cuda")
+    assign, best = torch.empty(100, dtype=torch.int32, device="cuda"), torch.empty(100, device="cuda")
+    for n, dim, k in ((100, 130, 200), (63, 64, 200), (100, 64, 127)):
+        with pytest.raises(psb.PsbError):
+            psb.kmeans_assign(x, n, dim, c, k, assign, best, form=2)
+
+
 @pytest.mark.parametrize("n,dim,k,big", [(5000, 128, 40, 3000), (9000, 100, 7, 1025), (1024, 33, 1, 1024), (2000, 300, 5, 1500)])
 def test_sums_of_large_groups(psb, n, dim, k, big):
     import torch
