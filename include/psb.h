@@ -161,8 +161,8 @@ typedef struct psb_options {
     /* Tuning, all optional (0 = the default): */
     float seed_sigma;   /* margin of the sampled admission cutoff in standard deviations (default 4; accepted 2..10).  Results do
                            not depend on it: a too-tight cutoff only sends more queries to the exact fallback. */
-    int pipeline_parts; /* sub-batches per batch of the overlapped pipeline (default 4; accepted 2..32) */
-    int even_cuts;      /* rows fetched from the host beside the scan: 0 = a short first sub-batch (by the kernel 12/18/22/26/22 %, by host
+    int pipeline_parts; /* sub-batches per batch of the overlapped pipeline, of equal size (default 4, or as even_cuts says; accepted 2..32) */
+    int even_cuts;      /* rows fetched from the host beside the scan (without pipeline_parts, or by host threads in 4 sub-batches at most): 0 = a short first sub-batch (by the kernel 12/18/22/26/22 %, by host
                            threads 10/30/30/30 %), so that the transfer starts early, 1 = equal sub-batches, 2 = a short last sub-batch
                            (32/32/26/10 %) */
     int gather_ctas;    /* 128-thread CTAs of the PCIe row-gather kernel when it runs beside a scan (default: two per SM) */

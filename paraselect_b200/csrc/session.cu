@@ -766,10 +766,11 @@ bool rows_shared(const psb_session* s, int n, int stage1_k, bool rerank) {
 // long as the scan and costs it little, so the first sub-batch is a small one: the transfer starts early.  Where the kernel fetches, the cuts grow so
 // that a sub-batch's scan takes about as long as the transfer of the one before, and the last is small again, for nothing hides its transfer
 // (100M x 96, 10,000 queries x 1,000 candidates: 12/18/22/26/22 % 84.3 ms, 10/20/20/25/25 86.1, 10/30/30/30 88.6, seven parts 90.3; no difference
-// at 1M to 12M rows).  Host threads are slower than the scan: 10/30/30/30 %.
+// at 1M to 12M rows).  Host threads are slower than the scan: 10/30/30/30 %.  Where the kernel fetches, a number of sub-batches that the caller gives
+// means that many equal ones.
 std::vector<int> batch_cuts(const psb_session* s, int n, int nprobe, int stage1_k, bool rerank) {
     const int sb = sub_batch_rows(s, n, nprobe, overlap_enabled(s, n, rerank) || staged_overlap_enabled(s, n, rerank));
-    const int plan = s->opt.even_cuts;
+    const int plan = s->opt.pipeline_parts != 0 && host_share(s) == 0 ? 1 : s->opt.even_cuts;
     if (rows_shared(s, n, stage1_k, rerank) && (s->opt.adc_mode != 1 || residual_table_free(s, stage1_k)) && sb * 4 >= n && n >= 4096 && plan != 1) {
         if (plan == 2) return {0, (int)(0.32 * n), (int)(0.64 * n), (int)(0.90 * n), n};  // short last sub-batch (scan-bound hosts)
         if (host_share(s) == 0) return {0, (int)(0.12 * n), (int)(0.30 * n), (int)(0.52 * n), (int)(0.78 * n), n};

@@ -121,6 +121,29 @@ def test_slots_in_row_order(psb, mode, count):
             assert np.array_equal(rows.cpu().numpy(), wi) and np.array_equal(dist.cpu().numpy(), wd)
 
 
+@pytest.mark.parametrize("mode,pct", [(0, 0), (4, 0), (4, 60), (1, 0)])   # the kernel, without and with the option of host threads; with them; they alone
+def test_cuts_of_a_large_batch(psb, mode, pct):
+    """Batches large enough for uneven sub-batches, whatever the cuts: the results of one piece.  A number of sub-batches that the caller gives holds
+    where the kernel fetches the rows: as many launches as of equal sub-batches."""
+    ix = index(3000, 32, False, 9)
+    q = np.random.default_rng(10).standard_normal((4201, 32)).astype(np.float32)
+    with psb.Session(ix, n_rerank=60, exact_mode=3, serial_pipeline=True) as s:
+        ref = s.search(q, 3, 10, batch_size=4201)
+
+    def launches(**how):
+        with psb.Session(ix, n_rerank=60, exact_mode=mode, zero_copy_pct=pct, **how) as s:
+            for _ in range(2):
+                got = s.search(q, 3, 10, batch_size=4201)
+                assert np.array_equal(got["indices"], ref["indices"]) and np.array_equal(got["distances"], ref["distances"])
+            return got["stats"]["kernel_launches"]
+    own = [launches(even_cuts=e) for e in (0, 1, 2)]
+    assert own[1] <= own[0] and own[1] == own[2]
+    for parts in (2, 3, 4, 6):
+        equal = launches(pipeline_parts=parts, even_cuts=1)
+        assert mode not in (0, 4) or pct or launches(pipeline_parts=parts) == launches(pipeline_parts=parts, even_cuts=2) == equal
+        assert parts <= 4 or launches(pipeline_parts=parts) == equal
+
+
 @pytest.mark.parametrize("mode,pct", [(0, 0), (4, 0), (4, 50)])
 def test_rows_fetched_are_counted(psb, mode, pct):
     """Each distinct row of a batch once, whoever brings it; rows that are scored in place are not counted."""
