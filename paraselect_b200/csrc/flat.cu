@@ -220,8 +220,9 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
 // Bound: latency, a tile being a chain of look-ups, two stagings and a short product; four CTAs an SM.  1,000 queries x 16 lists of 390 rows x 128,
 // topk 10: tiles 163 -> 72 us, selection 14 -> 29, the whole call 244 -> 150.  Eight warps a tile 91, four rows' loads at a time 78.
 //   Error of an approximate distance against the exact arithmetic's, S = (|q| + |x|)^2 <= 2 (|q|^2 + |x|^2):  products, splits 3.1 * 2^-18 and 3 K
-//   additions of 2^-22 each, of |q||x| <= S / 4, twice; norms (K + 4) 2^-24 S; their sum 2^-22 S; the exact arithmetic's own (K + 2) 2^-23 S; where
-//   products are subnormal, below 1e-35.  Together e = slack (|q|^2 + |x|^2) + 1e-35, and the tiles leave the lower bound, approximation - e.
+//   additions of 2^-22 each, of |q||x| <= S / 4, twice; norms (K + 4) 2^-24 S; their sum 2^-22 S; the exact arithmetic's own (K + 2) 2^-23 S; and
+//   2^-126 for each of 3 K products and 3 K partial sums that are subnormal and may vanish, twice: 12 K 2^-126 <= 3.7e-35 for the 256 dimensions the operands hold.
+//   Together e = slack (|q|^2 + |x|^2) + 3.7e-35, and the tiles leave the lower bound, approximation - e.
 //   The topk rows of the smallest lower bounds, t at most, lie within t + 2 e: of all rows in the visited lists |x|^2 is at most `most`, and of rows
 //   with |x| >= 3 |q| the lower bound is at least ((2/3)^2 - 2 * 10/9 slack) |x|^2 >= 0.4 |x|^2, so that |x|^2 <= max(9 |q|^2, 2.5 t) for the topk: one row far
 //   out does not loosen the bound for the others.  Only rows whose lower bound is below that can be among the topk.
@@ -232,6 +233,7 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
 // 227, behind the filter 131; one row of 1,000 times the norm, or not a number, 131; an offset of 100 with a spread of 0.3 301; all rows the same 488 (exact
 // tiles 376).  With one norm for the whole index and the way back in the selection's own block these were 926, 917 and 1,237.
 constexpr int kFilterThreads = 128;   // four warps: 16 visitors x 32 rows each
+constexpr float kFilterTiny = 3.7e-35f;
 __host__ __device__ __forceinline__ int filter_dims(int dim) { return (dim + 15) / 16 * 16; }
 __host__ __device__ __forceinline__ int filter_pitch(int dim) { return filter_dims(dim) + 8; }   // bf16 between rows: eight rows' 16 bytes in different banks
 inline size_t filter_bytes(int dim) { return (size_t)(SQ + SC) * filter_pitch(dim) * 4; }
@@ -290,7 +292,7 @@ k_flat_tiles_filter(const float* __restrict__ queries, int dim, int nprobe, cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long total = item_off[nlist];
     const float less = 1.0f - filter_slack(dim), none = __int_as_float(0x7fffffff);
-    auto lower = [&](float dot, float norms2) { return norms2 < 1.0e36f ? fmaf(-2.0f, dot, fmaf(norms2, less, -1.0e-35f)) : none; };
+    auto lower = [&](float dot, float norms2) { return norms2 < 1.0e36f ? fmaf(-2.0f, dot, fmaf(norms2, less, -kFilterTiny)) : none; };
     // One row by a warp, four elements a lane, several rows' loads before the first is used: two bf16 terms of each, and the squares' sum.
     auto stage = [&](auto src_of, int count, __nv_bfloat16* high, __nv_bfloat16* low, bool vec, auto sum_of) {
         constexpr int U = 8;
@@ -455,7 +457,7 @@ k_flat_select_filter(const float* __restrict__ dist, long long stride, const flo
         }
         __syncthreads();
         const float t = w.cut;
-        cut = fmaf(2.0002f * filter_slack(dim), qn + fminf(__uint_as_float(top), fmaxf(9.0f * qn, 2.5f * t)), fmaf(fabsf(t), 1.0e-6f, t)) + 4.0e-35f;
+        cut = fmaf(2.0002f * filter_slack(dim), qn + fminf(__uint_as_float(top), fmaxf(9.0f * qn, 2.5f * t)), fmaf(fabsf(t), 1.0e-6f, t)) + 2.0f * 1.01f * kFilterTiny;
     }
 #pragma unroll 8
     for (int i = threadIdx.x; i < n; i += T)

@@ -61,12 +61,12 @@ def test_flat_list_form_and_parts(psb, n, dim, nlist, nq, nprobe, topk, values):
     assert np.array_equal(got["indices"][some], wi) and np.array_equal(got["distances"][some], wd)
 
 
-@pytest.mark.parametrize("dim", [5, 16, 100, 128, 130, 240])
-@pytest.mark.parametrize("kind", ["normal", "far", "tiny", "grid", "odd", "one", "spread", "crowd", "large"])
+@pytest.mark.parametrize("dim", [5, 16, 100, 128, 130, 240, 256])
+@pytest.mark.parametrize("kind", ["normal", "far", "tiny", "vanish", "grid", "odd", "one", "spread", "crowd", "large"])
 @pytest.mark.parametrize("k", [1, 10, 256])
 def test_list_form_behind_the_filter(psb, dim, kind, k):
-    """Approximate distances and exact evaluation of the candidates: a large offset, which loosens the bound; values whose squares vanish, equal
-    distances by the hundred and values that are not finite; a row and rows of many times the others' norm; a list of equal rows, whose visitors
+    """Approximate distances and exact evaluation of the candidates: a large offset, which loosens the bound; values whose squares vanish, and
+    ones whose products with the query lie on both sides of the smallest normal number; equal distances by the hundred and values that are not finite; a row and rows of many times the others' norm; a list of equal rows, whose visitors
     alone go back to the exact tiles; norms on both sides of the largest that a bound is given for."""
     rng = np.random.default_rng(dim + k)
     nlist, n, nq, nprobe = 6, 9000, 700, 3
@@ -79,6 +79,8 @@ def test_list_form_behind_the_filter(psb, dim, kind, k):
         x, q, cen = x + 100, q + 100, cen + 100
     if kind == "tiny":
         x, q, cen = (v * np.float32(1e-20) for v in (x, q, cen))
+    if kind == "vanish":
+        x, cen, q = x * np.float32(1e-17), cen * np.float32(1e-17), q * np.float32(1e-21)
     if kind == "grid":
         x, q = np.round(x), np.round(q)
     if kind == "one":
