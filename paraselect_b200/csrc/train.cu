@@ -647,7 +647,7 @@ psb_status launch_pq_seed(const float* d_data, int n, int dim, int m, int k, con
     const int dsub = dim / m;
     const int per = (n + kSeedCluster - 1) / kSeedCluster;
     const size_t mins = (size_t)(per + 511) / 256 * 1024, rows = (size_t)per * dsub * 4;
-    const int staged = mins + rows <= (size_t)200 * 1024 ? 1 : 0;
+    const int staged = mins + rows <= (size_t)202 * 1024 ? 1 : 0;   // 2 KB for the places past a stretch's end
     const size_t smem = mins + (staged ? rows : 0);
     auto run = [&](auto kernel) -> psb_status {
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
