@@ -103,6 +103,10 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
 // borders of the row found, the sequential search finds the same row; when it is not (about one draw in a million), one thread
 // repeats the search sequentially.  A sum that is not a positive finite number is left to the host's own initialisation (status).
 constexpr int kSeedCluster = 8, kSeedCtaThreads = 512, kSeedCtaWarps = kSeedCtaThreads / 32;
+// Rows of a warp's stretch up to which the search takes a row a lane, in a kernel of its own: a lane's eight rows are two chains of sums, and the warps of a
+// round share an instruction cache that it finds cold.  Eight / one, us, four sub-quantisers of 4: 2,000 rows 710 / 626, 4,096 747 / 657, 8,192
+// (stretches of 64) 785 / 733, 16,384 (128) 832 / 843.  Both searches in one kernel: 646, 673, 745.
+constexpr int kSeedShort = 64;
 
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
     uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
@@ -130,7 +134,7 @@ __device__ __forceinline__ double warp_inclusive(double v, int lane) {
 }
 
 // draws [m][k - 1] uniform in [0, 1); first [m]; rows_out [m][k]; status [m] = 1: left to the host.  per = rows per CTA.
-template <int D>
+template <int D, bool SHORT>
 __global__ void __launch_bounds__(kSeedCtaThreads) __cluster_dims__(kSeedCluster, 1, 1)
 k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, int per, int staged, const double* __restrict__ draws,
           const int* __restrict__ first, long long* __restrict__ rows_out, int* __restrict__ status) {
@@ -225,7 +229,21 @@ k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, in
             int found = -1;
             bool sure = false;
             double run = before;
-            for (int r0 = w0; r0 < w1; r0 += 256) {   // eight rows a lane
+            if constexpr (SHORT) {   // a row a lane
+                for (int r0 = w0; r0 < w1; r0 += 32) {
+                    const int row = r0 + lane;
+                    const double in = warp_inclusive(row < w1 ? (double)s_min[row] : 0.0, lane) + run;
+                    const unsigned hit = __ballot_sync(0xffffffffu, row < w1 && in >= r);
+                    if (hit) {
+                        const int l = __ffs((int)hit) - 1;
+                        const double hi = __shfl_sync(0xffffffffu, in, l), lo = __shfl_sync(0xffffffffu, in, l ? l - 1 : 0), below = l ? lo : run;
+                        found = b + r0 + l;
+                        sure = hi - r > slack && (r - below > slack || found == 0);
+                        break;
+                    }
+                    run = __shfl_sync(0xffffffffu, in, 31);
+                }
+            } else for (int r0 = w0; r0 < w1; r0 += 256) {   // eight rows a lane
                 const int row = r0 + lane * 8;
                 double x[8], mine = 0.0;
 #pragma unroll
@@ -263,10 +281,12 @@ k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, in
             if (!sure) {   // too close to a border, or beyond the stretch: the sequential sums decide
                 if (lane == 0) {
                     double t = 0.0;
+#pragma unroll 1
                     for (int i = 0; i < n; ++i) t += (double)cluster_load(cluster_addr(&s_min[i % per], i / per));
                     const double rs = __dmul_rn(draws[(size_t)sub * (k - 1) + (c - 1)], t);
                     double cum = 0.0;
                     found = n - 1;
+#pragma unroll 1
                     for (int i = 0; i < n; ++i) {
                         cum += (double)cluster_load(cluster_addr(&s_min[i % per], i / per));
                         if (cum >= rs) { found = i; break; }
@@ -649,19 +669,20 @@ psb_status launch_pq_seed(const float* d_data, int n, int dim, int m, int k, con
     const size_t mins = (size_t)(per + 511) / 256 * 1024, rows = (size_t)per * dsub * 4;
     const int staged = mins + rows <= (size_t)202 * 1024 ? 1 : 0;   // 2 KB for the places past a stretch's end
     const size_t smem = mins + (staged ? rows : 0);
-    auto run = [&](auto kernel) -> psb_status {
+    auto run = [&](auto few, auto many) -> psb_status {
+        auto kernel = per <= kSeedShort * kSeedCtaWarps ? few : many;
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
         kernel<<<dim3(kSeedCluster, (unsigned)m), kSeedCtaThreads, smem, s>>>(d_data, n, dim, dsub, k, per, staged, d_draws, d_first, d_rows, d_status);
         return PSB_OK;
     };
     switch (dsub) {
-        case 2: PSB_TRY(run(k_pq_seed<2>)); break;
-        case 3: PSB_TRY(run(k_pq_seed<3>)); break;
-        case 4: PSB_TRY(run(k_pq_seed<4>)); break;
-        case 5: PSB_TRY(run(k_pq_seed<5>)); break;
-        case 6: PSB_TRY(run(k_pq_seed<6>)); break;
-        case 8: PSB_TRY(run(k_pq_seed<8>)); break;
-        default: PSB_TRY(run(k_pq_seed<0>)); break;
+        case 2: PSB_TRY(run(k_pq_seed<2, true>, k_pq_seed<2, false>)); break;
+        case 3: PSB_TRY(run(k_pq_seed<3, true>, k_pq_seed<3, false>)); break;
+        case 4: PSB_TRY(run(k_pq_seed<4, true>, k_pq_seed<4, false>)); break;
+        case 5: PSB_TRY(run(k_pq_seed<5, true>, k_pq_seed<5, false>)); break;
+        case 6: PSB_TRY(run(k_pq_seed<6, true>, k_pq_seed<6, false>)); break;
+        case 8: PSB_TRY(run(k_pq_seed<8, true>, k_pq_seed<8, false>)); break;
+        default: PSB_TRY(run(k_pq_seed<0, true>, k_pq_seed<0, false>)); break;
     }
     count_launch();
     PSB_LAUNCH_CHECK();

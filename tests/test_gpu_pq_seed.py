@@ -30,10 +30,10 @@ def test_first_codewords_are_the_hosts(psb, n, dim, M, K, kind):
         assert np.array_equal(got[s].view(np.uint32), want.view(np.uint32)), "subspace %d" % s
 
 
-@pytest.mark.parametrize("n,dim,M,K", [(2049, 15, 5, 256), (8193, 30, 6, 200), (600, 18, 3, 256), (32769, 20, 4, 256), (4095, 8, 4, 256),
+@pytest.mark.parametrize("n,dim,M,K", [(2049, 15, 5, 256), (8193, 30, 6, 200), (600, 18, 3, 256), (32769, 20, 4, 256), (4095, 8, 4, 256), (8192, 16, 4, 256), (600, 8, 2, 256),
                                        (68256, 10, 2, 256), (45504, 16, 2, 256)])   # the most rows that shared memory holds
 def test_stretches_of_the_search(psb, n, dim, M, K):
-    """Sub-vectors of two, three, five and six; stretches that end within a lane's eight rows."""
+    """Sub-vectors of two, three, five and six; stretches that end within a lane's eight rows; both searches at the line between them."""
     test_first_codewords_are_the_hosts(psb, n, dim, M, K, "normal")
 
 
