@@ -29,6 +29,28 @@ def test_static_coarse_matches_allocating_coarse_twice(psb):
         assert np.array_equal(dist.cpu().numpy(), want_dist)
 
 
+@pytest.mark.parametrize("nq,nlist,dim,nprobe", [(1, 1024, 96, 32), (100, 700, 33, 20), (300, 4096, 96, 64)])   # each kernel for the distances
+def test_static_coarse_in_a_captured_graph(psb, nq, nlist, dim, nprobe):
+    import torch
+    rng = np.random.default_rng(nlist)
+    c = rng.standard_normal((nlist, dim)).astype(np.float32)
+    dq, dc = torch.zeros(nq, dim, device="cuda"), torch.from_numpy(c).cuda()
+    ids, dist = torch.empty((nq, nprobe), dtype=torch.int32, device="cuda"), torch.empty(nq, nprobe, device="cuda")
+    psb.coarse_search_static(dq, nq, dc, nlist, dim, nprobe, ids, dist)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        for _ in range(2):   # the second call works in the array of the first
+            psb.coarse_search_static(dq, nq, dc, nlist, dim, nprobe, ids, dist, stream=torch.cuda.current_stream().cuda_stream)
+    for _ in range(3):
+        q = rng.standard_normal((nq, dim)).astype(np.float32)
+        dq.copy_(torch.from_numpy(q))
+        g.replay()
+        torch.cuda.synchronize()
+        want_ids, want_dist = psb.coarse_host(q, c, nprobe, coarse_mode=1)
+        assert np.array_equal(ids.cpu().numpy(), want_ids) and np.array_equal(dist.cpu().numpy(), want_dist)
+
+
 def test_static_coarse_rejects_shapes_beyond_its_scratch(psb):
     import torch
     dq = torch.zeros((4097, 8), dtype=torch.float32, device="cuda")
