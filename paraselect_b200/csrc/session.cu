@@ -482,7 +482,7 @@ struct psb_session {
     DevBuf opq, q_rot;                     // OPQ rotation [dim][dim] and the rotated queries of the batch in flight
     bool row_bias_is_u16 = false;          // row_bias holds the caller's affine u16 row correction
     bool flat = false;                     // IVF-Flat session: exact rows resident in flat_rows, no PQ parts
-    DevBuf flat_rows, flat_slot, flat_norms, flat_again;   // norms: of every row, then the largest of each list
+    DevBuf flat_rows, flat_norms, flat_whole, flat_slot, flat_again;   // norms: of every row, then the largest of each list
     EventPool timing, timing_aux;          // events of the main stream's marks and of the second stream's (set from one thread each)
     // Host side of a search call: one pinned block through which a small batch's queries and results pass, and the device's counters
     // and status words with the results, so that a call waits for the GPU once.
@@ -2200,13 +2200,14 @@ psb_status psb_flat_session_create(const psb_flat_index_view* index, const psb_o
     PSB_TRY(s->offsets.reserve(sizeof(long long) * (nl + 1)));
     PSB_CUDA(cudaMemcpyAsync(s->offsets.p, index->lists.offsets, sizeof(long long) * (nl + 1), cudaMemcpyHostToDevice, st));
     PSB_TRY(s->reordered.reserve(sizeof(long long) * n));
-    PSB_TRY(s->flat_rows.reserve(sizeof(float) * n * s->dim));
+    // One allocation: the norms of their own took the room in a block of the driver's that the first call's workspace then lacked (21 queries x 7 lists
+    // of 1,000 rows, first call 85 -> 480 us).
+    PSB_TRY(reserve_together(&s->flat_whole, {{&s->flat_rows, sizeof(float) * n * s->dim}, {&s->flat_norms, sizeof(float) * (n + nl)}}));
     if (s->n_vectors > 0) {
         PSB_CUDA(cudaMemcpyAsync(s->reordered.p, index->lists.reordered_ids, sizeof(long long) * n, cudaMemcpyHostToDevice, st));
         PSB_CUDA(cudaMemcpyAsync(s->flat_rows.p, index->rowmajor_fp32, sizeof(float) * n * s->dim, cudaMemcpyHostToDevice, st));
     }
     note_list_lengths(s.get(), index->lists.offsets);
-    PSB_TRY(s->flat_norms.reserve(sizeof(float) * (n + nl)));
     PSB_TRY(launch_flat_norms(s->flat_rows.as<float>(), s->n_vectors, s->dim, s->offsets.as<long long>(), s->nlist, s->flat_norms.as<float>(),
                               s->flat_norms.as<unsigned>() + n, st));
     PSB_TRY(ensure_scalars(s.get(), st));
