@@ -216,9 +216,10 @@ k_flat_select(const float* __restrict__ dist, long long stride, const int* __res
 // The distances of a list's visitors to its rows are a matrix product; in the reference's arithmetic they are three instructions per
 // dimension and pair.  Where a selection follows anyway, the tiles are taken from mma.sync with both operands split into two bf16 terms
 // (|q|^2 + |x|^2 - 2 q.x in fp32), the selection keeps every row that the approximate distance cannot rule out, and those - a few more
-// than topk - are evaluated exactly.  (tcgen05 wants 128 visitors a tile; a list has sixty in the benchmark's configuration, and often ten.)
+// than topk - are evaluated exactly.  (A list has sixty visitors in the benchmark's configuration, and
+// often ten: too few for the M of a tcgen05 product.  With its rows as M and the visitors as N they would do; that form is not built.)
 // Bound: latency, a tile being a chain of look-ups, two stagings and a short product; four CTAs an SM.  1,000 queries x 16 lists of 390 rows x 128,
-// topk 10: tiles 163 -> 72 us, selection 14 -> 29, the whole call 244 -> 150.  Eight warps a tile 91, four rows' loads at a time 78.
+// topk 10: tiles 163 -> 71 us, selection 14 -> 23, the whole call 244 -> 140.  Eight warps a tile 91, four rows' loads at a time 78.
 //   Error of an approximate distance against the exact arithmetic's, S = (|q| + |x|)^2 <= 2 (|q|^2 + |x|^2):  products, splits 3.1 * 2^-18 and 3 K
 //   additions of 2^-22 each, of |q||x| <= S / 4, twice; norms (K + 4) 2^-24 S; their sum 2^-22 S; the exact arithmetic's own (K + 2) 2^-23 S; and
 //   2^-126 for each of 3 K products and 3 K partial sums that are subnormal and may vanish, twice: 12 K 2^-126 <= 3.7e-35 for the 256 dimensions the operands hold.

@@ -45,9 +45,11 @@ __device__ __forceinline__ long long local_row(const RowMap& mp, long long r) {
 }
 
 // The claim of a part of a batch: k_mark_rows sets the bit of every row the part names and no earlier part has a slot for, k_count_rows counts the
-// bits of each stretch of rows, k_place_rows gives the marked rows the next slots in the order of their numbers.  The order is what makes the fetch fast: rows read over PCIe at random places of a large array are bound by the translation of their
-// addresses, in ascending order by the link.  A million rows of 384 bytes on 16 SMs: from an array of 0.8 GB 50.8 GB/s in random order, 50.9 sorted;
-// of 4.6 GB 18.9 and 51.0; of 20 GB 12.9 and 51.0 (one large copy: 55.5).  The bits cost one read of count / 8 bytes: 12.5 MB for 100M rows.
+// bits of each stretch of rows, k_place_rows gives the marked rows the next slots in the order of their numbers.  The order is what makes the fetch
+// fast: rows read over PCIe at random places of a large array are bound by the translation of their addresses, in ascending order by the link.  A
+// million rows of 384 bytes on 16 SMs: from an array of 0.8 GB 50.8 GB/s in random order, 50.9 sorted; of 4.6 GB 18.9 and 51.0; of 20 GB 12.9 and
+// 51.0 (one large copy: 55.5).  The bits, count / 8 bytes of them (12.5 MB for 100M rows), are read by k_count_rows and by k_place_rows, which also
+// clears as many of the claim before, for every part of a batch.
 // Up to kSelfCountWords words each CTA counts the marks before its stretch itself, and k_count_rows is not launched (27,000 requests of 510,000
 // rows: 10 us less per call).  The other CTAs read a CTA's words while it places them: the marks of the claim before are what it takes back.
 constexpr int kPlaceThreads = 1024;                // words of 32 rows a CTA places: each warp 32 of them, one row per lane at a time

@@ -95,7 +95,7 @@ k_pq_encode_tile(const float* __restrict__ data, long long n, int dim, const flo
 // codeword so far, a draw r in [0, sum), and the first row at which the running sum reaches r.  On one host thread this took 0.5 s
 // for 32,768 rows x 24 sub-quantisers, 98 % of a codebook training.  Here a cluster of eight CTAs holds a sub-quantiser's rows and
 // their distances in shared memory (rows that do not fit are read through L2); a pick is one update of the distances, two cluster
-// barriers and a search in one warp's stretch of rows, of which the lanes take eighths of 32 one after the other; the warp that finds the row
+// barriers and a search in one warp's stretch of rows, of which a lane takes eight at a time (kSeedShort: one); the warp that finds the row
 // hands it round with its values: 4.3 us (32,768 rows, 24 sub-quantisers; 5.6 with values from global memory, rows read word by word and a
 // stretch walked 32 rows a step), 255 picks, every sub-quantiser on SMs of its own.
 // The draws are made by the host (they do not depend on the data).  The rows picked are the reference's: its sequential sum and the
@@ -157,7 +157,7 @@ k_pq_seed(const float* __restrict__ data, int n, int dim, int dsub_rt, int k, in
     int pick = first[sub];
     if (rank == 0 && tid == 0) out[0] = pick;
     __syncthreads();
-    // A row's values: whole vectors where rows lie on their boundaries (staged ones of 2, 4, 8, 12, 16 dimensions).
+    // A row's values: whole vectors where rows lie on their boundaries (staged ones of 2, 4, 6, 8 dimensions).
     auto row_of = [&](int r, float (&x)[D > 0 ? D : 1]) {
         if constexpr (D > 0) {
             if (!staged) {
