@@ -149,7 +149,8 @@ typedef struct psb_options {
     int scan_mode;      /* which ADC scan runs; all give identical results.  0 = auto: the tensor-core pre-filter (bf16 tcgen05
                            GEMM of visiting queries against code rows decoded on the fly, survivors re-scored exactly in fp32)
                            when the shape fits, else the SIMT fp16 pre-filter scan, else the fp32 scan; 1 = fp32 SIMT scan only;
-                           2 = SIMT scans only; 3 = tensor-core pre-filter required (PSB_UNSUPPORTED_SHAPE when it cannot run) */
+                           2 = SIMT scans only; 3 = tensor-core pre-filter required (PSB_UNSUPPORTED_SHAPE when it cannot run).  An IVF-Flat
+                           session's list form: 1 and 2 = exact tiles, 3 = behind the filter where that fits, else as the batch says */
     int adc_mode;       /* PQAdcDistanceMode (src/search/kernels/fine/fine_search_strategy.h:21-24): 0 = Plain (codes
                            encode the row), 1 = Residual (codes encode row - centroid[list]).  Residual mode follows
                            cpu_fine_kernel_pq_resid_cpu_lut_timed (src/search/ivfrespq/stage/ivfrespq_cpu_rerank.cpp:594-735):

@@ -364,7 +364,7 @@ class FlatSession:
     index: dict with centroids [nlist,dim] f32, offsets [nlist+1] i64, reordered_ids [n] i64, vectors [n,dim] f32 (list-contiguous).
     """
 
-    def __init__(self, index, device=0, max_batch=0, stream=None, coarse_mode=0, time_kernels=False):
+    def __init__(self, index, device=0, max_batch=0, stream=None, coarse_mode=0, time_kernels=False, scan_mode=0):
         cen = _np(index["centroids"], np.float32)
         off = _np(index["offsets"], np.int64)
         rid = _np(index["reordered_ids"], np.int64)
@@ -375,7 +375,8 @@ class FlatSession:
         fv.lists = ListLayoutView(_p(off), _p(rid), cen.shape[0], int(vec.shape[0]))
         fv.rowmajor_fp32 = _p(vec)
         self.dim, self.nlist = cen.shape[1], cen.shape[0]
-        opt = Options(device=device, max_batch=max_batch, stream=stream, coarse_mode=coarse_mode, time_kernels=int(time_kernels))
+        opt = Options(device=device, max_batch=max_batch, stream=stream, coarse_mode=coarse_mode, time_kernels=int(time_kernels),
+                      scan_mode=scan_mode)
         self._h = C.c_void_p()
         _check(lib().psb_flat_session_create(C.byref(fv), C.byref(opt), C.byref(self._h)))
 

@@ -301,6 +301,7 @@ struct FlatScan {
     const float* rows; const long long* ids;   // [n][dim], [n]
     const float* norms; const unsigned* most;  // squared norms of the rows and each list's largest's bits (launch_flat_norms)
     int topk;
+    int form;                                  // of the list form's tiles: 1, 2 = exact, 3 = behind the filter where that fits, else by the batch
     long long* out_ids; float* out_dist;       // [nq][topk]
     float* dist; long long stride;             // [nq][stride] workspace, stride >= the rows of any nprobe lists
     float* runs; long long run_stride;         // [nq][run_stride] workspace of the row form: the minimum of every 32 distances

@@ -2250,7 +2250,7 @@ psb_status flat_search_device(psb_session* s, const float* dq, int n, int nprobe
     }
     f.dim = s->dim; f.nprobe = nprobe; f.offsets = s->offsets.as<long long>(); f.nlist = s->nlist; f.n_rows = s->n_vectors; f.rows = s->flat_rows.as<float>();
     f.norms = s->flat_norms.as<float>(); f.most = s->flat_norms.as<unsigned>() + std::max<long long>(1, s->n_vectors);
-    f.ids = s->reordered.as<long long>(); f.topk = topk; f.dist = s->row_dist.as<float>(); f.seg = s->row_seg.as<int>();
+    f.ids = s->reordered.as<long long>(); f.topk = topk; f.form = s->opt.scan_mode; f.dist = s->row_dist.as<float>(); f.seg = s->row_seg.as<int>();
     f.vis_count = s->vis_count.as<int>(); f.slot = s->flat_slot.as<int>(); f.vis_off = s->vis_off.as<int>(); f.item_off = s->item_off.as<long long>();
     f.visitors = s->visitors.as<int>(); f.again = s->flat_again.as<int>(); f.counters = s->scalars.as<unsigned long long>(); f.sm_count = s->sm_count;
     for (int q0 = 0; q0 < n; q0 += per) {

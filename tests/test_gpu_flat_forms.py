@@ -95,7 +95,7 @@ def test_list_form_behind_the_filter(psb, dim, kind, k):
     if kind == "odd":
         x[4000, 0], x[77, dim - 1], q[3, 1] = np.inf, np.nan, np.inf
     ix = dict(centroids=cen, offsets=off, reordered_ids=rng.permutation(n).astype(np.int64), vectors=x)
-    with psb.FlatSession(ix, max_batch=nq) as s:
+    with psb.FlatSession(ix, max_batch=nq, scan_mode=3) as s:
         got = s.search(q, nprobe, k, batch_size=nq, want_coarse=True)
     for i in list(range(12)) + [nq - 1]:
         rows = np.concatenate([np.arange(off[p], off[p + 1]) for p in got["coarse"][i]])
@@ -111,6 +111,22 @@ def test_list_form_behind_the_filter(psb, dim, kind, k):
         take = np.isfinite(d[order])
         assert np.array_equal(got["indices"][i][: len(order)][take], ix["reordered_ids"][rows[order]][take]), (kind, i)
         assert np.array_equal(got["distances"][i][: len(order)][take], d[order][take])
+
+
+@pytest.mark.parametrize("form", [0, 1, 3])
+@pytest.mark.parametrize("nprobe,k", [(1, 10), (1, 11), (1, 256), (2, 200), (3, 256), (3, 200)])   # either side of the line: rows, and rows for each wanted
+def test_both_forms_of_the_tiles(psb, form, nprobe, k):
+    rng = np.random.default_rng(k)
+    n, dim, nlist, nq = 9300, 64, 7, 1100
+    off = np.linspace(0, n, nlist + 1).astype(np.int64)
+    fx = dict(centroids=rng.standard_normal((nlist, dim)).astype(np.float32), offsets=off, reordered_ids=rng.permutation(n).astype(np.int64),
+              vectors=rng.standard_normal((n, dim)).astype(np.float32))
+    q = rng.standard_normal((nq, dim)).astype(np.float32)
+    with psb.FlatSession(fx, max_batch=nq, scan_mode=form) as s:
+        got = s.search(q, nprobe, k, batch_size=nq)
+    some = rng.integers(0, nq, 60)
+    wi, wd = oracle.ivfflat_search(fx["centroids"], off, fx["reordered_ids"], fx["vectors"], q[some], nprobe, k)
+    assert np.array_equal(got["indices"][some], wi) and np.array_equal(got["distances"][some], wd)
 
 
 def test_calls_of_changing_size(psb):
