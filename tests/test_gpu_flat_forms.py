@@ -170,7 +170,7 @@ def test_cost_where_the_bound_is_loose(psb, kind, times):
                 b.record(st)
                 torch.cuda.synchronize()
                 ms.append(a.elapsed_time(b))
-        return sorted(ms)[4]
+        return min(ms)   # the host's other work only adds
     plain = cost(x, q, cen)
     if kind == "one":
         x[n // 2] *= 1000

@@ -189,4 +189,6 @@ def test_first_call_lays_its_workspace_out_once(psb):
             torch.cuda.synchronize()
             return time.perf_counter() - t
     first(0), first(1)
-    assert sorted(first(0) for _ in range(9))[4] < 1.4 * sorted(first(1) for _ in range(9))[4]   # measured 1.0; laid out anew for each sub-batch 2.1
+    took = [(first(0), first(1)) for _ in range(15)]   # in turn, and the least of each: the host's other work only adds
+    grow, equal = (min(t) for t in zip(*took))
+    assert grow < 1.5 * equal   # measured 1.0; laid out anew for each sub-batch 1.8 to 2.0
