@@ -243,7 +243,7 @@ psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_
     if (k <= 0 || k > kMaxProbe) return fail(PSB_UNSUPPORTED_SHAPE, "row selection supports 1..4096 results");
     const size_t smem = sel::shared_bytes(k);
     PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_select_rows), smem));
-    PSB_TRY(launch_behind(true, k_select_rows, dim3((unsigned)nq), kSelThreads, smem, s, d_dist, n, k, sel::buffer_entries(k), d_ids, d_out));
+    PSB_TRY(launch_behind(select_behind(nq, (long long)nq * n <= 8192 ? nq : 2, k, 32), k_select_rows, dim3((unsigned)nq), kSelThreads, smem, s, d_dist, n, k, sel::buffer_entries(k), d_ids, d_out));
     count_launch();
     PSB_LAUNCH_CHECK();
     return PSB_OK;

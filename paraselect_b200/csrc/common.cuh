@@ -121,6 +121,11 @@ inline psb_status launch_behind(bool chained, void (*kernel)(P...), dim3 grid, u
     PSB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
     return PSB_OK;
 }
+// Whether a selection of k by a block per query is launched so: a few queries' (few), or a short one.  A block that is placed early stays where the kernel
+// before had room first, perhaps beside others like it while SMs are without one, and a long selection loses more by that than the launch costs.  Coarse stage, us,
+// behind / not: 64 queries x 256 centroids, 32 wanted 6.7 / 9.2, 64 29.8 / 12.4; 17 x 1,024, 256 wanted 53 / 18.5; 4 x 1,024, 64 wanted 9.2 / 10.3; 8 x 4,000, 128
+// wanted 28.6 / 16.5.  The selections over lists: 333 queries x 4 of 700 lists, 200 wanted 93 / 89; 1,000 x 16, 100 wanted 106 / 115.
+inline bool select_behind(int nq, int few, int k, int short_k) { return nq <= few || k <= short_k; }
 __device__ __forceinline__ void behind() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

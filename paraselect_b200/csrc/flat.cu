@@ -555,7 +555,7 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
             const size_t keys = (size_t)sel::buffer_entries(f.topk) * 8 + (size_t)((f.dim + 3) & ~3) * 4 + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
             auto select = [&](auto kernel, int threads) -> psb_status {
                 PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), keys));
-                return launch_behind(true, kernel, dim3((unsigned)nq), (unsigned)threads, keys, s, f.dist, f.stride, f.queries, f.dim, f.rows, f.most, f.probes, f.nprobe, f.offsets,
+                return launch_behind(select_behind(nq, f.sm_count, f.topk, 128), kernel, dim3((unsigned)nq), (unsigned)threads, keys, s, f.dist, f.stride, f.queries, f.dim, f.rows, f.most, f.probes, f.nprobe, f.offsets,
                                      f.nlist, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist, f.again, n_again);
             };
             if (nq <= f.sm_count) PSB_TRY(select(k_flat_select_filter<1024>, 1024));
@@ -572,14 +572,15 @@ psb_status launch_flat_scan(const FlatScan& f, int nq, cudaStream_t s) {
         const long long blocks = std::min<long long>((f.stride + 127) / 128, 8192);
         const size_t smem = (size_t)((f.dim + 3) & ~3) * sizeof(float);
         if (smem > 48 * 1024) PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_flat_rows), smem));
-        PSB_TRY(launch_behind(true, k_flat_rows, dim3((unsigned)std::max<long long>(1, blocks), (unsigned)nq), 128, smem, s, f.queries, f.dim, f.probes, f.nprobe, f.offsets, f.rows, f.seg, f.stride, f.dist, f.runs, f.run_stride));
+        // (behind: 8 queries x 8 lists of 428 rows of 64 25.4 us against 26.7, 32 29.4 and 31.3, 64 45.0 and 41.0, 128 62.9 and 55.4)
+        PSB_TRY(launch_behind(nq <= 32, k_flat_rows, dim3((unsigned)std::max<long long>(1, blocks), (unsigned)nq), 128, smem, s, f.queries, f.dim, f.probes, f.nprobe, f.offsets, f.rows, f.seg, f.stride, f.dist, f.runs, f.run_stride));
     }
     count_launch();
     PSB_LAUNCH_CHECK();
     const size_t smem = sel::shared_bytes(f.topk) + (f.nprobe <= sel::kSegShared ? ((size_t)f.nprobe + 1) * sizeof(int) : 0);
     auto select = [&](auto kernel, int threads) -> psb_status {   // fewer queries than SMs: large blocks
         PSB_TRY(kernel_shared(reinterpret_cast<const void*>(kernel), smem));
-        return launch_behind(true, kernel, dim3((unsigned)nq), (unsigned)threads, smem, s, f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist, lists ? nullptr : f.runs, f.run_stride,
+        return launch_behind(select_behind(nq, f.sm_count, f.topk, 128), kernel, dim3((unsigned)nq), (unsigned)threads, smem, s, f.dist, f.stride, f.probes, f.nprobe, f.offsets, f.seg, f.topk, sel::buffer_entries(f.topk), f.ids, f.out_ids, f.out_dist, lists ? nullptr : f.runs, f.run_stride,
                              filtered ? f.again : nullptr);
     };
     if (nq <= f.sm_count) PSB_TRY(select(k_flat_select<1024>, 1024));
