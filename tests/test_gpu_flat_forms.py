@@ -27,7 +27,8 @@ def test_flat_forms(psb, n, dim, nlist, nq, nprobe, topk, values):
     assert np.array_equal(got["indices"], wi) and np.array_equal(got["distances"], wd)
 
 
-@pytest.mark.parametrize("nq,nlist,dim,k", [(1, 3, 5, 3), (33, 65, 12, 20), (2, 3000, 40, 1), (3, 5000, 8, 700), (40, 513, 6, 130), (2, 9000, 4, 1500)])
+@pytest.mark.parametrize("nq,nlist,dim,k", [(1, 3, 5, 3), (33, 65, 12, 20), (2, 3000, 40, 1), (3, 5000, 8, 700), (40, 513, 6, 130), (2, 9000, 4, 1500),
+                                           (30, 600, 5, 256), (30, 513, 5, 228), (30, 2000, 5, 900), (30, 2000, 5, 400), (3, 4000, 5, 512), (30, 1024, 5, 900)])   # the bound with few values for each wanted
 @pytest.mark.parametrize("equal", [False, True])
 def test_coarse_small_batches(psb, nq, nlist, dim, k, equal):
     rng = np.random.default_rng(nlist)
