@@ -126,15 +126,19 @@ k_coarse_dist_few(const float* __restrict__ queries, const float* __restrict__ c
 // tile on its way while one is compared; every thread keeps the nearest of its own centroids for its four rows.  The same distances; ties go to
 // the lower id.  Bound: fp32 issue, three instructions per dimension and pair.  (Distances to memory and a selecting block per row: 70,338 x 96, 237
 // centroids, two iterations of a training 5,688 us, now 1,071; 400,000 x 128, 64 centroids, five 14,450 and 6,030.)
+// So few rows that CTAs of them leave SMs idle: the centroids are cut into ranges, a CTA each, and the smallest key of a row is taken in `keys` (a chain of
+// all tiles took 272 us for 700 x 64, 3,000 centroids, where the distances to memory took 91; in ranges 34).
 constexpr int kNearThreads = 256, kNearRows = 64;
 inline size_t near_bytes(int dim) { return (size_t)(kNearRows + 2 * SC) * small_pitch(dim) * 4; }
 __global__ void __launch_bounds__(kNearThreads)
-k_nearest_rows(const float* __restrict__ rows, int n, const float* __restrict__ centroids, int k, int dim, int* __restrict__ out_ids, float* __restrict__ out_dist) {
+k_nearest_rows(const float* __restrict__ rows, int n, const float* __restrict__ centroids, int k_all, int dim, int range, unsigned long long* __restrict__ keys,
+               int* __restrict__ out_ids, float* __restrict__ out_dist) {
     extern __shared__ __align__(16) float s_near[];
     const int pitch = small_pitch(dim), tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     float* rs = s_near;
     float* cs = s_near + kNearRows * pitch;   // [2][SC][pitch]
-    const int r0 = blockIdx.x * kNearRows;
+    const int r0 = blockIdx.x * kNearRows, first = blockIdx.y * range, k = min(range, k_all - first);   // of this CTA's centroids
+    centroids += (size_t)first * dim;
     stage_rows<kNearThreads>(rs, pitch, rows + (size_t)r0 * dim, min(kNearRows, n - r0), dim);
     stage_rows<kNearThreads>(cs, pitch, centroids, min(SC, k), dim);
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -160,19 +164,26 @@ k_nearest_rows(const float* __restrict__ rows, int n, const float* __restrict__ 
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        uint64_t key = id[i] >= 0 ? make_key(best[i], (uint32_t)id[i]) : KEY_MAX;
+        uint64_t key = id[i] >= 0 ? make_key(best[i], (uint32_t)(first + id[i])) : KEY_MAX;
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) { const uint64_t other = __shfl_xor_sync(0xffffffffu, key, o); key = other < key ? other : key; }
         const int r = r0 + ty * 4 + i;
         if (r >= n) continue;   // (the same for the sixteen lanes of a row, which alone exchange)
         if (key == KEY_MAX && tx == 0) {   // no distance is a finite number: the smallest all the same, infinity before what is not a number
             for (int c = 0; c < k; ++c) {
-                const uint64_t other = make_key(row_distance(rs + (ty * 4 + i) * pitch, centroids + (size_t)c * dim, dim, rows_vec(centroids, dim)), (uint32_t)c);
+                const uint64_t other = make_key(row_distance(rs + (ty * 4 + i) * pitch, centroids + (size_t)c * dim, dim, rows_vec(centroids, dim)), (uint32_t)(first + c));
                 key = other < key ? other : key;
             }
         }
-        if (tx == 0) { out_ids[r] = (int)key_idx(key); out_dist[r] = key_dist(key); }
+        if (tx != 0) continue;
+        if (keys) atomicMin(keys + r, (unsigned long long)key);
+        else { out_ids[r] = (int)key_idx(key); out_dist[r] = key_dist(key); }
     }
+}
+
+__global__ void __launch_bounds__(256) k_nearest_out(const unsigned long long* __restrict__ keys, int n, int* __restrict__ out_ids, float* __restrict__ out_dist) {
+    const int r = blockIdx.x * 256 + threadIdx.x;
+    if (r < n) { out_ids[r] = (int)key_idx(keys[r]); out_dist[r] = key_dist(keys[r]); }
 }
 
 // Per row: the k smallest (value, index) pairs, ascending.
@@ -227,14 +238,33 @@ psb_status launch_coarse_dist_exact(const float* d_queries, int nq, const float*
 }
 
 bool nearest_rows_fit(int dim) { return near_bytes(dim) <= (size_t)200 * 1024; }
+// Whether it beats distances to memory and a selection.  Not for few rows and pairs (700 x 128 to 100 centroids, three iterations, 223 us, distances to memory 196), nor for long
+// rows, which leave an SM one CTA, and many centroids (20,000 x 200, trainings of three iterations, ms: 600 centroids 2.06, distances to memory 1.96, 3,000 8.3 and 7.0).
+bool nearest_rows_pays(int n, int k, int dim) { return nearest_rows_fit(dim) && (n >= 1024 || (long long)n * k >= 98304) && (dim <= 128 || k < 512 || n < 2048); }
 
-psb_status launch_nearest_rows(const float* d_rows, int n, const float* d_centroids, int k, int dim, int* d_ids, float* d_dist, cudaStream_t s) {
+// Cut until there are two CTAs an SM; two tiles of short rows are not worth the keys' passes.
+int nearest_rows_range(int n, int k, int dim, int sm_count) {
+    const int tiles = (k + SC - 1) / SC, blocks = (n + kNearRows - 1) / kNearRows;
+    if (tiles < (dim >= 96 ? 2 : 3) || blocks >= 2 * sm_count) return k;
+    const int parts = std::min(tiles, (2 * sm_count + blocks - 1) / blocks), each = (tiles + parts - 1) / parts;
+    return each < tiles ? each * SC : k;
+}
+
+psb_status launch_nearest_rows(const float* d_rows, int n, const float* d_centroids, int k, int dim, int range, unsigned long long* d_keys, int* d_ids, float* d_dist,
+                               cudaStream_t s) {
     if (n <= 0) return PSB_OK;
+    if (range < k) PSB_CUDA(cudaMemsetAsync(d_keys, 0xff, sizeof(unsigned long long) * (size_t)n, s));   // KEY_MAX
     const size_t smem = near_bytes(dim);
     PSB_TRY(kernel_shared(reinterpret_cast<const void*>(k_nearest_rows), smem));
-    k_nearest_rows<<<(unsigned)((n + kNearRows - 1) / kNearRows), kNearThreads, smem, s>>>(d_rows, n, d_centroids, k, dim, d_ids, d_dist);
+    k_nearest_rows<<<dim3((unsigned)((n + kNearRows - 1) / kNearRows), (unsigned)((k + range - 1) / range)), kNearThreads, smem, s>>>(
+        d_rows, n, d_centroids, k, dim, range, range < k ? d_keys : nullptr, d_ids, d_dist);
     count_launch();
     PSB_LAUNCH_CHECK();
+    if (range < k) {
+        k_nearest_out<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_keys, n, d_ids, d_dist);
+        count_launch();
+        PSB_LAUNCH_CHECK();
+    }
     return PSB_OK;
 }
 

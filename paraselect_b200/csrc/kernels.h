@@ -35,7 +35,11 @@ bool coarse_few(int nq, int nlist, int dim);   // so few pairs that a thread tak
 constexpr int kCoarseFewBlock = 64;            // centroids behind one read of a query
 // The nearest of k centroids to each of n rows, with the same distances; rows of up to nearest_rows_fit() dimensions.
 bool nearest_rows_fit(int dim);
-psb_status launch_nearest_rows(const float* d_rows, int n, const float* d_centroids, int k, int dim, int* d_ids, float* d_dist, cudaStream_t s);
+bool nearest_rows_pays(int n, int k, int dim);
+// range: centroids of a CTA (nearest_rows_range); below k the rows' smallest keys pass through d_keys [n].
+int nearest_rows_range(int n, int k, int dim, int sm_count);
+psb_status launch_nearest_rows(const float* d_rows, int n, const float* d_centroids, int k, int dim, int range, unsigned long long* d_keys, int* d_ids, float* d_dist,
+                               cudaStream_t s);
 // Per query the k smallest (distance, id) pairs of a [nq][n] distance matrix, sorted ascending.
 psb_status launch_select_rows(const float* d_dist, int nq, int n, int k, int* d_ids, float* d_out,
                               cudaStream_t s);

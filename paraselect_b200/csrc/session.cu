@@ -2549,9 +2549,12 @@ public:
 private:
     static constexpr size_t kKeepRows = (size_t)4 << 30;
     psb_status exact(const float* d_centroids, int* d_assign, float* d_best) {
-        if (nearest_rows_fit(dim_)) {
-            for (int64_t r0 = 0; r0 < n_; r0 += 1 << 30)
-                PSB_TRY(launch_nearest_rows(data_ + (size_t)r0 * dim_, (int)std::min<int64_t>(1 << 30, n_ - r0), d_centroids, k_, dim_, d_assign + r0, d_best + r0, st_));
+        if (nearest_rows_pays((int)std::min<int64_t>(n_, INT_MAX), k_, dim_)) {
+            for (int64_t r0 = 0; r0 < n_; r0 += 1 << 30) {
+                const int nn = (int)std::min<int64_t>(1 << 30, n_ - r0), range = nearest_rows_range(nn, k_, dim_, sms_);
+                if (range < k_) PSB_TRY(keys_.reserve(sizeof(unsigned long long) * (size_t)nn, device_, st_));
+                PSB_TRY(launch_nearest_rows(data_ + (size_t)r0 * dim_, nn, d_centroids, k_, dim_, range, keys_.as<unsigned long long>(), d_assign + r0, d_best + r0, st_));
+            }
             return PSB_OK;
         }
         const size_t row_bytes = sizeof(float) * (size_t)k_;
@@ -2571,7 +2574,7 @@ private:
     bool tc_;
     TcIndexBuffers<PoolBuf> index_;
     TcWorkBuffers<PoolBuf> work_;
-    PoolBuf rows_, norms_, tile_;
+    PoolBuf rows_, norms_, tile_, keys_;
 };
 }  // namespace
 

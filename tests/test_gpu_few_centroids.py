@@ -15,6 +15,8 @@ def distances(x, c):
 
 @pytest.mark.parametrize("n,dim,k", [(1, 8, 1), (63, 8, 1), (64, 5, 64), (65, 33, 65), (4096, 20, 63), (4097, 12, 129), (300, 200, 70), (8193, 3, 7),
                                      (5000, 48, 700), (3000, 130, 300), (20000, 16, 2049), (12289, 8, 2048),
+                                     # few rows: centroids in ranges, or a thread for each pair; long rows and many centroids
+                                     (1, 100, 3000), (40, 16, 900), (51, 128, 1000), (701, 64, 1500), (9001, 20, 321), (2047, 200, 513), (2049, 200, 513),
                                      # both sides of the line to counts by blocks of rows
                                      (16383, 8, 512), (16384, 8, 512), (16385, 8, 513), (20481, 5, 1), (33000, 6, 1031),
                                      # above the line to the filter, whose blocks are of 512 centroids
