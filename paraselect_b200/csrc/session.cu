@@ -2506,9 +2506,10 @@ public:
     Assigner(const float* d_data, int64_t n, int dim, int k, int device, int sms, cudaStream_t st, int form = 0)
         : data_(d_data), n_(n), dim_(dim), k_(k), device_(device), sms_(sms), st_(st) {
         // The filter costs about 2 ns a row whatever the number of centroids, and its launches more than the row kernel's; that takes 1.2e-4 ns for
-        // each dimension of a pair.  Trainings of three iterations, rows / filter, us: 20,000 x 64, 256 centroids 548 / 631, 400 654 / 572; 20,000 x
-        // 128, 128 613 / 756, 200 749 / 673; 100,000 x 96, 128 1,218 / 1,239, 1,000 5,020 / 1,200; 400,000 x 100, 128 4,031 / 3,216, 1,000 19,369 / 3,233.
-        tc_ = form == 2 || (form == 0 && filter_takes(n, dim, k) && (!nearest_rows_fit(dim) || (double)k * dim >= 16384.0 + 1.6e8 / (double)n));
+        // each dimension of a pair and as much as 20 of them besides.  Trainings of three iterations, rows / filter, us: 20,000 x 64, 256 centroids 548 / 631, 400 654 / 572; 20,000 x
+        // 128, 128 613 / 756, 200 749 / 673; 100,000 x 96, 128 1,218 / 1,239, 1,000 5,020 / 1,200; 400,000 x 100, 128 4,031 / 3,216, 1,000 19,369 / 3,233; 100,000 x 3, 600
+        // 784 / 827, 3,000 2,516 / 1,270; 10,000 x 16, 3,000 552 / 512.  Of 200 trainings (700 to 300,000 rows of 3 to 128 dimensions) the form taken is on average 0.5 % slower than the other.
+        tc_ = form == 2 || (form == 0 && filter_takes(n, dim, k) && (!nearest_rows_fit(dim) || (double)k * (dim + 20) >= 8000.0 + 3.0e8 / (double)n));
     }
     static bool filter_takes(int64_t n, int dim, int k) { return n >= 64 && k >= 128 && coarse_tc_padded_dim(dim) <= 128; }
     // d_assign [n], d_best [n] out; bounded: d_assign holds an assignment on entry, whose distances bound the nearest ones (one
