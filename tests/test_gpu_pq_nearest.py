@@ -83,7 +83,8 @@ def test_encode_where_products_underflow(dim, M, scale):
 
 
 @pytest.mark.parametrize("n,dim,M,K", [(127, 16, 4, 256), (128, 16, 5, 256), (129, 20, 5, 255), (1921, 24, 6, 256), (5000, 64, 16, 256), (70000, 8, 2, 256),
-                                       (150, 400, 200, 40), (3000, 48, 4, 256), (2500, 33, 11, 33)])
+                                       (150, 400, 200, 40), (3000, 48, 4, 256), (2500, 33, 11, 33),
+                                       (57600, 20, 5, 256), (113700, 20, 5, 256), (38000, 32, 16, 40)])   # items of nine and of fifteen tiles
 @pytest.mark.parametrize("at", [0, 1, 2])
 def test_encode_tiles_and_items(n, dim, M, K, at):
     """Rows at the ends of a tile and of an item's tiles, sub-quantisers that do not fill an operand row, rows that start at any float."""
